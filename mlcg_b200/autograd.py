@@ -654,35 +654,39 @@ class SchNetEval(torch.autograd.Function):
 
 class SchNetForceMatching(torch.autograd.Function):
     """``(energies, forces)`` of a standard SchNet in training mode, differentiable with respect to the weights: ``forward_pass`` holds
-    both with the state of the pass (one library call), the backward is one more.  Positions are constants here (the caller takes the
+    both with the state of the pass (one library call), the backward is one more.  The buffers of the state are saved tensors like the
+    weights: freed by the backward, checked for changes, open to saved-tensor hooks.  Positions are constants here (the caller takes the
     composable operators where they require a gradient).  A backward pass that is itself differentiated (``create_graph``) goes
     through the composable operators."""
 
     @staticmethod
     def forward(ctx, forward_pass, composable, *params):
-        energy, forces, ctx.state = forward_pass
-        ctx.composable = composable
-        ctx.save_for_backward(*params)
+        energy, forces, state = forward_pass
+        ctx.state, ctx.composable = state, composable
+        ctx.save_for_backward(*params, *state.tensors)
+        state.tensors = None
         ctx.set_materialize_grads(False)
         return energy, forces
 
     @staticmethod
     def backward(ctx, gE, gF):
-        params, state = ctx.saved_tensors, ctx.state
+        state, wanted = ctx.state, ctx.needs_input_grad[2:]
         if gE is None and gF is None:
-            return (None,) * (2 + len(params))
+            return (None,) * (2 + len(wanted))
+        kept = ctx.saved_tensors
+        params, saved = kept[:len(wanted)], kept[len(wanted):]
         if torch.is_grad_enabled():
-            pairs = [(v, g) for v, g in zip(ctx.composable(state), (gE, gF)) if g is not None]
-            wanted = [p for p, need in zip(params, ctx.needs_input_grad[2:]) if need]
-            got = iter(torch.autograd.grad([v for v, _ in pairs], wanted, [g for _, g in pairs], create_graph=True, allow_unused=True))
-            return (None, None) + tuple(next(got) if need else None for need in ctx.needs_input_grad[2:])
+            pairs = [(v, g) for v, g in zip(ctx.composable(state, saved), (gE, gF)) if g is not None]
+            got = iter(torch.autograd.grad([v for v, _ in pairs], [p for p, need in zip(params, wanted) if need], [g for _, g in pairs],
+                                           create_graph=True, allow_unused=True))
+            return (None, None) + tuple(next(got) if need else None for need in wanted)
         gE = None if gE is None else gE.contiguous()
-        gF = torch.zeros_like(state.pos) if gF is None else gF.contiguous()
-        grads = get_backend().schnet_train_backward(state, gE, gF)
+        gF = torch.zeros_like(state.view(saved, "pos")) if gF is None else gF.contiguous()
+        grads = get_backend().schnet_train_backward(state, saved, params, gE, gF)
         tensors = state.weights[1][1]
         if tensors[4] is not None:                     # the last bias enters every bead's energy once, and no force
-            struct_ptr = state.views()[1]
+            struct_ptr = state.view(saved, "struct_ptr")
             n = struct_ptr[1:] - struct_ptr[:-1]
             grads[4] = torch.zeros_like(tensors[4]) if gE is None else (gE * n).sum().reshape(tensors[4].shape)
         grads = [g for g, t in zip(grads, tensors) if t is not None]
-        return (None, None) + tuple(g if need else None for g, need in zip(grads, ctx.needs_input_grad[2:]))
+        return (None, None) + tuple(g if need else None for g, need in zip(grads, wanted))

@@ -5,7 +5,7 @@ back end is :class:`CudaBackend`; it refuses tensors that are not on a CUDA devi
 raises if ``libmlcg_b200.so`` is missing.
 """
 import ctypes
-from dataclasses import dataclass
+from dataclasses import dataclass, replace
 from typing import Optional
 
 import numpy as np
@@ -53,8 +53,16 @@ class _WeightPlaces:
                                         *(None if h < 0 else base + h for h in self.head), None), addresses
 
 
+def weights_struct(sizes, tensors):
+    """``mlcgb_schnet_weights`` over ``tensors`` (in the packed order; None: absent) with the widths and counts of ``sizes``, another such
+    structure or anything with its fields, and the block array it points to."""
+    ptr = [None if t is None else t.data_ptr() for t in tensors]
+    arr = (_lib.SchnetBlockStruct * sizes.num_blocks)(*(_lib.SchnetBlockStruct(*ptr[k: k + 8]) for k in range(5, len(ptr), 8)))
+    return _lib.SchnetWeightsStruct(sizes.hidden, sizes.filters, sizes.conv_out, sizes.head_width, sizes.num_blocks, sizes.num_types, arr, *ptr[:5]), arr
+
+
 def _weights_places(weights):
-    struct, (_, tensors, _) = weights
+    struct, (_, tensors, *_) = weights
     places = struct.__dict__.get("places")
     if places is None:
         places = struct.places = _WeightPlaces(tensors)
@@ -62,14 +70,24 @@ def _weights_places(weights):
 
 
 class ForceMatchingState:
-    """What the backward of a force-matching step needs of its forward pass: device pointers into buffers that it keeps alive.
-    ``views()``: the edge lists ``(row0, row1, offsets, twin, sel, pair_of)`` or an edge plan, and the structure boundaries."""
+    """What the backward of a force-matching step needs of its forward pass.  ``tensors``: the device buffers, which the pass's autograd
+    node takes over as saved tensors; everything else says where in them things lie.  No address outlives the forward pass: saved-tensor
+    hooks may bring the buffers back elsewhere.  ``places``: name -> (index in ``tensors``, byte offset, entries, dtype; offset None: the
+    tensor itself)."""
 
-    __slots__ = ("pos", "types", "struct_ptr", "N", "B", "E", "lists", "forward_ws", "spec", "conv_cut", "weights", "views", "keep")
+    __slots__ = ("N", "B", "E", "tensors", "places", "spec", "conv_cut", "weights")
 
     def __init__(self, *values):
         for name, value in zip(self.__slots__, values):
             setattr(self, name, value)
+
+    def view(self, saved, name):
+        k, at, n, dtype = self.places[name]
+        return saved[k] if at is None else saved[k][at: at + n * dtype.itemsize].view(dtype)
+
+    def address(self, saved, name):
+        k, at, _, _ = self.places[name]
+        return saved[k].data_ptr() + (at or 0)
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -833,18 +851,12 @@ class CudaBackend:
             return energy, grad, E, None
         at = (ctypes.c_int64 * 8)()
         lib.mlcgb_schnet_evaluate_lists(N, B, E, at)
-        g, p = graph_ws.data_ptr(), ws.data_ptr()
-        lists = (p + at[2], p + at[3], g + at[1], p + at[6], p + at[5])       # row0, row1, offsets, sel, pair_of
-
-        def views():
-            def part(t, k, n, dtype=torch.int32):
-                return t[at[k]: at[k] + n * dtype.itemsize].view(dtype)
-            row0, row1, twin, pair_of = (part(ws, k, E) for k in (2, 3, 4, 5))
-            offsets = part(graph_ws, 1, N + 1, torch.int64)
-            return (row0, row1, offsets, twin, part(ws, 6, E // 2), pair_of), part(graph_ws, 0, B + 1, torch.int64) if ptr is None else ptr
-
-        return energy, grad, E, ForceMatchingState(pos, types, (g + at[0]) if ptr is None else ptr.data_ptr(), N, B, E, lists, p + at[7], spec, conv_cut,
-                                                   weights, views, (graph_ws, ws, ptr))
+        i32, i64 = torch.int32, torch.int64
+        places = {"pos": (0, None, 0, None), "types": (1, None, 0, None), "p0": (2, None, 0, None), "p1": (3, None, 0, None),
+                  "struct_ptr": (5, at[0], B + 1, i64) if ptr is None else (6, None, 0, None), "offsets": (5, at[1], N + 1, i64),
+                  "row0": (4, at[2], E, i32), "row1": (4, at[3], E, i32), "twin": (4, at[4], E, i32), "pair_of": (4, at[5], E, i32),
+                  "sel": (4, at[6], E // 2, i32), "forward_ws": (4, at[7], 0, None)}
+        return energy, grad, E, ForceMatchingState(N, B, E, (pos, types, spec.p0, spec.p1, ws, graph_ws, ptr), places, spec, conv_cut, weights)
 
     # ------------------------------------------------------------------ one force-matching step
     @staticmethod
@@ -871,29 +883,36 @@ class CudaBackend:
                 _ptr(plan.perm_in), plan.E, sel.numel(), ctypes.byref(s), int(conv_cut[0]), float(conv_cut[1]), float(conv_cut[2]), ctypes.byref(wstruct), 1,
                 _ptr(ws), wsb, _ptr(energy), _ptr(forces), _ptr(status), _stream()), "schnet_train_forward")
         self.defer_status(status, "SchNet force matching")
-        lists = tuple(t.data_ptr() for t in (plan.row0, plan.row1, plan.ptr_out, sel, pair_of))
-        return energy, forces, ForceMatchingState(pos, types, struct_ptr.data_ptr(), N, B, plan.E, lists, ws.data_ptr(), spec, conv_cut, weights,
-                                                  lambda: (plan, struct_ptr), (ws, plan, struct_ptr))
+        names = ("pos", "types", "p0", "p1", "struct_ptr", "offsets", "row0", "row1", "twin", "pair_of", "sel", "forward_ws")
+        tensors = (pos, types, spec.p0, spec.p1, struct_ptr, plan.ptr_out, plan.row0, plan.row1, plan.perm_in, pair_of, sel, ws)
+        return energy, forces, ForceMatchingState(N, B, plan.E, tensors, {n: (k, None, 0, None) for k, n in enumerate(names)}, spec, conv_cut, weights)
 
-    def schnet_train_backward(self, state, gE, gF):
+    def schnet_train_backward(self, state, saved, params, gE, gF):
         """Gradients of a loss on the energies and forces of the forward pass that ``state`` came from with respect to the weights, as
-        views of one buffer in the order of the packed weights (``None`` for the output network's second bias)."""
-        wstruct, (_, tensors, live) = state.weights
-        N, B, E, dev = state.N, state.B, state.E, state.pos.device
-        s, keep = self._spec(state.spec, torch.float32)
+        views of one buffer in the order of the packed weights (``None`` for the output network's second bias).  ``saved``, ``params``:
+        the buffers of the state and the weights (without the absent ones) as the autograd node's saved tensors hand them back."""
+        wstruct, (_, tensors, live, addresses) = state.weights
+        params = iter(params)
+        weights = [None if t is None else next(params) for t in tensors]
+        if tuple(0 if t is None else t.data_ptr() for t in weights) != addresses:       # (moved by a saved-tensor hook)
+            weights = [None if t is None else t.contiguous() for t in weights]
+            wstruct, _keep = weights_struct(wstruct, weights)
+        N, B, E, dev = state.N, state.B, state.E, gF.device
+        s, keep = self._spec(replace(state.spec, p0=state.view(saved, "p0"), p1=state.view(saved, "p1")), torch.float32)
         wsb = self.lib.mlcgb_schnet_train_workspace_bytes(1, N, E, E // 2, state.spec.num_rbf, wstruct.head_width, wstruct.num_blocks, wstruct.num_types)
         ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
         places = _weights_places(state.weights)
         flat = torch.empty(places.total, dtype=torch.float32, device=dev)
         gs, arr = places.struct(wstruct, flat.data_ptr())
         status = self._sticky_status(dev)
-        row0, row1, offsets, sel, pair_of = state.lists
+        pos, types, struct_ptr, row0, row1, offsets, sel, pair_of, forward_ws = [
+            state.address(saved, n) for n in ("pos", "types", "struct_ptr", "row0", "row1", "offsets", "sel", "pair_of", "forward_ws")]
         cut = state.conv_cut
         with _on(dev):
             _lib.check(self.lib.mlcgb_schnet_train_backward(
-                state.pos.data_ptr(), state.types.data_ptr(), state.struct_ptr, N, B, row0, row1, offsets, sel, pair_of, E, E // 2, ctypes.byref(s),
-                int(cut[0]), float(cut[1]), float(cut[2]), ctypes.byref(wstruct), 1, _ptr(gE), _ptr(gF), state.forward_ws, ws.data_ptr(), wsb,
-                ctypes.byref(gs), status.data_ptr(), _stream()), "schnet_train_backward")
+                pos, types, struct_ptr, N, B, row0, row1, offsets, sel, pair_of, E, E // 2, ctypes.byref(s), int(cut[0]), float(cut[1]), float(cut[2]),
+                ctypes.byref(wstruct), 1, _ptr(gE), _ptr(gF), forward_ws, ws.data_ptr(), wsb, ctypes.byref(gs), status.data_ptr(), _stream()),
+                "schnet_train_backward")
         self.defer_status(status, "SchNet force matching")
         views = iter(torch._C._nn.unflatten_dense_tensors(flat, live))        # (behind the launches: the device is busy by now)
         return [None if t is None or k == 4 else next(views) for k, t in enumerate(tensors)]

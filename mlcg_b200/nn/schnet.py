@@ -4,15 +4,15 @@
 ``SchNet`` :32-192, ``InteractionBlock`` :195-262, ``CFConv`` :265-368, ``StandardSchNet`` :371-475.
 """
 import warnings
+from types import SimpleNamespace
 from typing import Final, List
 
 import torch
 
-from .. import _lib
 from ..autograd import (attach_plan, EdgeDiff, EdgeDistanceOnce, EdgePlan, FusedFilterConv, FusedInteraction, PairSelect, RowScale, SchNetEval, SchNetForceMatching, SegIn, SegmentSum, SegPair,
                         edge_distances, plan_of)
 from ..autograd import tanh as tanh_op
-from ..backend import get_backend
+from ..backend import get_backend, weights_struct
 from ..data import ENERGY_KEY, AtomicData
 from ..neighbor_list import atomic_data2neighbor_list, bare_edge_plan, make_neighbor_list, sizes_or_pointer, validate_neighborlist
 from .cutoff import cutoff_kind
@@ -302,15 +302,10 @@ class SchNet(torch.nn.Module):
         ok = ok and all(v % 4 == 0 and v <= 128 for v in (H, H2, Wh))
         result = None
         if ok:
-            ptr = lambda t: None if t is None else t.data_ptr()
-            arr = (_lib.SchnetBlockStruct * len(blocks))()
-            for i in range(len(blocks)):
-                for f, t in zip(("lin1_w", "filter_w1", "filter_b1", "filter_w2", "lin2_w", "lin2_b", "lin_w", "lin_b"), tensors[5 + 8 * i: 13 + 8 * i]):
-                    setattr(arr[i], f, ptr(t))
-            ws = _lib.SchnetWeightsStruct(H, F, H2, Wh, len(blocks), self.embedding_layer.num_embeddings, arr, ptr(tensors[0]), ptr(tensors[1]),
-                                          ptr(tensors[2]), ptr(tensors[3]), ptr(tensors[4]))
+            sizes = SimpleNamespace(hidden=H, filters=F, conv_out=H2, head_width=Wh, num_blocks=len(blocks), num_types=self.embedding_layer.num_embeddings)
+            ws, arr = weights_struct(sizes, tensors)
             live = [t for k, t in enumerate(tensors) if t is not None and k != 4]
-            result = (ws, (arr, tensors, live))
+            result = (ws, (arr, tensors, live, key))
         self.__dict__["_mlcgb_packed"] = (key, result)
         return result
 
@@ -444,19 +439,18 @@ class SchNet(torch.nn.Module):
             result = self._from_positions(data, setup, True, True)
             if result is None:
                 return None
-        batch = getattr(data, "batch", None)
 
         # (holds nothing that leads to the outputs: `data` would, and its autograd graph would never be freed)
-        def composable(state):  # the same two values through operators that can be differentiated to any order
-            p, (lists, ptr) = state.pos.detach().clone().requires_grad_(True), state.views()
-            plan = lists if isinstance(lists, EdgePlan) else EdgePlan.from_graph(
-                dict(zip(("row0", "row1", "offsets", "twin", "sel", "pair_of"), lists)), p.shape[0], symmetric=True)
+        def composable(state, saved):  # the same two values through operators that can be differentiated to any order
+            lists = {name: state.view(saved, name) for name in ("row0", "row1", "offsets", "twin", "sel", "pair_of")}
+            p, ptr = state.view(saved, "pos").detach().clone().requires_grad_(True), state.view(saved, "struct_ptr")
+            plan = EdgePlan.from_graph(lists, p.shape[0], symmetric=True)
             nl = make_neighbor_list(tag="", order=2, index_mapping=attach_plan(torch.stack([plan.row0, plan.row1]).to(torch.int64), plan),
                                     rcut=self.rbf_layer.cutoff.cutoff_upper, self_interaction=False)
             nl["_mlcgb_zero_shifts"], nl["_mlcgb_ptr"] = True, ptr
             sizes = ptr[1:] - ptr[:-1]
-            owner = torch.repeat_interleave(torch.arange(sizes.numel(), device=p.device), sizes, output_size=p.shape[0]) if batch is None else batch
-            again = AtomicData(pos=p, atom_types=state.types, batch=owner, n_atoms=sizes, neighbor_list={self.name: nl})
+            owner = torch.repeat_interleave(torch.arange(sizes.numel(), device=p.device), sizes, output_size=p.shape[0])
+            again = AtomicData(pos=p, atom_types=state.view(saved, "types"), batch=owner, n_atoms=sizes, neighbor_list={self.name: nl})
             energy = self(again).out[self.name][ENERGY_KEY]
             return energy, -torch.autograd.grad(energy.sum(), p, create_graph=True)[0]
 

@@ -106,3 +106,64 @@ def test_a_step_leaves_nothing_behind():
         del data
         used.append(torch.cuda.memory_allocated())
     assert used[1] == used[2] == used[3]
+
+
+def _data(pos, types_, sizes, **more):
+    n = torch.tensor(sizes)
+    return mlcg_b200.AtomicData(pos=pos.to(DEV, copy=True), atom_types=types_.to(DEV, copy=True), batch=torch.arange(len(n)).repeat_interleave(n).to(DEV),
+                                n_atoms=n.to(DEV), **more)
+
+
+def _fused(value):
+    return type(value.grad_fn).__name__ == "SchNetForceMatchingBackward"
+
+
+def _grads(net):
+    return {n: p.grad.clone() for n, p in net.named_parameters() if p.grad is not None}
+
+
+def _step(m, data, target):
+    m.zero_grad(set_to_none=True)
+    out = m(data).out["SchNet"]
+    ((out["forces"] - target.to(DEV)) ** 2).mean().backward()
+    return out
+
+
+def _close(a, b, rtol=1e-4):
+    assert a.keys() == b.keys()
+    for n in a:
+        assert float((a[n] - b[n]).abs().max()) <= rtol * float(b[n].abs().max()) + 1e-9, n
+
+
+@pytest.mark.parametrize("given_list", [False, True])
+def test_the_backward_frees_what_the_forward_kept(given_list):
+    """The state of a forward pass belongs to its autograd node: gone after the backward although the outputs live on, and seen by
+    saved-tensor hooks, which may bring it back at another address."""
+    sizes = [40] * 8
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 7)
+    m = bnn.GradientsOut(net.to(DEV), "forces").train()
+    more = {}
+    if given_list:
+        more["neighbor_list"] = net.neighbor_list(_data(pos, types_, sizes), 9.0)
+    kept = 4 * 2 * 512 * 2000          # W, W', h and z of two blocks and at least 2000 pairs
+    _step(m, _data(pos, types_, sizes, **more), target)
+    plain = _grads(net)
+    before = torch.cuda.memory_allocated()
+    out = _step(m, _data(pos, types_, sizes, **more), target)
+    assert _fused(out["forces"])
+    assert torch.cuda.memory_allocated() - before < kept // 8
+    seen = []
+
+    def pack(t):
+        seen.append(t.numel() * t.element_size())
+        return t.cpu()
+
+    m.zero_grad(set_to_none=True)
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.to(DEV)):
+        out = m(_data(pos, types_, sizes, **more)).out["SchNet"]
+        loss = ((out["forces"] - target.to(DEV)) ** 2).mean()
+    assert sum(seen) > kept
+    junk = [torch.full((sum(seen) // 4,), float("nan"), device=DEV) for _ in range(2)]     # (where the forward's buffers were)
+    loss.backward()
+    _close(_grads(net), plain, 1e-6)
+    del junk
