@@ -117,6 +117,12 @@ def _on(device):
     return torch.cuda.device(device)
 
 
+def _own(t: torch.Tensor, given: torch.Tensor) -> torch.Tensor:
+    """``t`` where it does not share memory with ``given``, else a copy: for what a backward pass reads of inputs that the caller may
+    have overwritten by then."""
+    return t.clone() if t.data_ptr() == given.data_ptr() else t
+
+
 def _need_cuda(*ts):
     for t in ts:
         if t is not None and not t.is_cuda:
@@ -816,7 +822,7 @@ class CudaBackend:
         guess at the edge count that sizes the workspace (too low costs a second call).  ``training``: the forward pass of
         :meth:`schnet_train_forward` (forces), its state as the last value."""
         w, _keep = weights
-        pos = pos.detach().contiguous()
+        given, pos = pos, pos.detach().contiguous()
         N, dev = pos.shape[0], pos.device
         B = ptr.numel() - 1 if n_atoms is None else n_atoms.numel()
         s, keep = self._spec(spec, torch.float32)
@@ -849,6 +855,7 @@ class CudaBackend:
         self.defer_status(status, "SchNet force matching" if training else "SchNet evaluation")
         if not training:
             return energy, grad, E, None
+        pos = _own(pos, given)
         at = (ctypes.c_int64 * 8)()
         lib.mlcgb_schnet_evaluate_lists(N, B, E, at)
         i32, i64 = torch.int32, torch.int64
@@ -869,6 +876,7 @@ class CudaBackend:
     def schnet_train_forward(self, pos, types, struct_ptr, plan, spec: RbfSpec, conv_cut, weights):
         """(energies [B], forces [N,3], state for :meth:`schnet_train_backward`) of a standard SchNet on a given edge plan."""
         wstruct, _keep = weights
+        given, pos = pos, pos.detach().contiguous()
         N, B, dev = pos.shape[0], struct_ptr.numel() - 1, pos.device
         sel, pair_of = plan.half_selection(), plan.pair_index()
         s, keep = self._spec(spec, torch.float32)
@@ -884,7 +892,7 @@ class CudaBackend:
                 _ptr(ws), wsb, _ptr(energy), _ptr(forces), _ptr(status), _stream()), "schnet_train_forward")
         self.defer_status(status, "SchNet force matching")
         names = ("pos", "types", "p0", "p1", "struct_ptr", "offsets", "row0", "row1", "twin", "pair_of", "sel", "forward_ws")
-        tensors = (pos, types, spec.p0, spec.p1, struct_ptr, plan.ptr_out, plan.row0, plan.row1, plan.perm_in, pair_of, sel, ws)
+        tensors = (_own(pos, given), types, spec.p0, spec.p1, struct_ptr, plan.ptr_out, plan.row0, plan.row1, plan.perm_in, pair_of, sel, ws)
         return energy, forces, ForceMatchingState(N, B, plan.E, tensors, {n: (k, None, 0, None) for k, n in enumerate(names)}, spec, conv_cut, weights)
 
     def schnet_train_backward(self, state, saved, params, gE, gF):

@@ -432,7 +432,7 @@ class SchNet(torch.nn.Module):
                 return None
             if ptr is None or ptr.device != data.pos.device:
                 ptr = self._structure_ptr(data)
-            result = be.schnet_train_forward(data.pos.detach().contiguous(), self._types(data), ptr, plan, *setup[:3])
+            result = be.schnet_train_forward(data.pos, self._types(data), ptr, plan, *setup[:3])
         elif getattr(data, "pbc", None) is not None and bool(torch.any(data.pbc)):
             return None
         else:

@@ -167,3 +167,30 @@ def test_the_backward_frees_what_the_forward_kept(given_list):
     loss.backward()
     _close(_grads(net), plain, 1e-6)
     del junk
+
+
+def test_inputs_overwritten_before_the_backward():
+    """The next batch copied over the positions leaves the gradients alone; bead types that changed are an error, as anywhere in torch."""
+    sizes = [23, 40, 9]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 8)
+    m = bnn.GradientsOut(net.to(DEV), "forces").train()
+    _step(m, _data(pos, types_, sizes), target)
+    expected = _grads(net)
+    for given_list in (False, True):
+        data = _data(pos, types_, sizes)
+        if given_list:
+            data.neighbor_list = net.neighbor_list(data, 9.0)
+        mine = data.pos
+        m.zero_grad(set_to_none=True)
+        out = m(data).out["SchNet"]
+        assert _fused(out["forces"])
+        with torch.no_grad():
+            mine.copy_(mine.flip(0) * 1.5)
+        data.n_atoms.zero_()
+        ((out["forces"] - target.to(DEV)) ** 2).mean().backward()
+        _close(_grads(net), expected, 1e-6)
+    data = _data(pos, types_, sizes)
+    out = m(data).out["SchNet"]
+    data.atom_types.zero_()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out["forces"].sum().backward()
