@@ -111,7 +111,8 @@ class CFConv(torch.nn.Module):
         if cached is not None and cached[0] == key:
             return cached[1]
         result = self._fused_spec_uncached(rbf_layer)
-        self.__dict__["_fused_spec_cache"] = (key, result)
+        # (the objects of the key are held too, so that no other takes over one's id)
+        self.__dict__["_fused_spec_cache"] = (key, result, (rbf_layer, self.cutoff, rc, *net.layers, *rbf_layer._parameters.values(), *rbf_layer._buffers.values()))
         return result
 
     def _fused_spec_uncached(self, rbf_layer):
@@ -281,11 +282,21 @@ class SchNet(torch.nn.Module):
                       (c.lin2, "bias"), (b.lin, "weight"), (b.lin, "bias")]
         return slots
 
+    def _layers(self):
+        """(all modules, :meth:`_whole_model_slots`), worked out again when a module has been put in, taken out or replaced."""
+        cached = self.__dict__.get("_mlcgb_layers")
+        if cached is None or [child for children in cached[0] for child in children.values()] != cached[1]:
+            modules = list(self.modules())
+            children = [m._modules for m in modules]
+            cached = (children, [child for c in children for child in c.values()], modules, self._whole_model_slots())
+            self.__dict__["_mlcgb_layers"] = cached
+            self.__dict__.pop("_mlcgb_packed", None)
+            self.__dict__.pop("_mlcgb_setup", None)
+        return cached[2], cached[3]
+
     def packed_weights(self):
         """``mlcgb_schnet_weights`` over the current parameters (rebuilt whenever a parameter's storage has moved), or None."""
-        slots = self.__dict__.get("_mlcgb_slots", False)
-        if slots is False:
-            slots = self.__dict__["_mlcgb_slots"] = self._whole_model_slots()
+        slots = self._layers()[1]
         if slots is None:
             return None
         tensors = [m._parameters[n] for m, n in slots]

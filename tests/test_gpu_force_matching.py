@@ -1,4 +1,6 @@
 """The one-call force-matching step (values, forces, weight gradients) against a float64 evaluation of the same float32 weights."""
+import copy
+
 import pytest
 import torch
 
@@ -194,3 +196,24 @@ def test_inputs_overwritten_before_the_backward():
     data.atom_types.zero_()
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         out["forces"].sum().backward()
+
+
+@pytest.mark.parametrize("training", [True, False])
+def test_a_layer_replaced_after_a_call(training):
+    sizes = [23, 40]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 15)
+    m = bnn.GradientsOut(net.to(DEV), "forces").train(training)
+    before = m(_data(pos, types_, sizes)).out["SchNet"]["forces"].detach()
+    for path, layer in (("interaction_blocks.0.conv.lin1", torch.nn.Linear(128, 128, bias=False)),
+                        ("interaction_blocks.1.conv.filter_network.layers.0", torch.nn.Linear(32, 128)), ("output_network.layers.0", torch.nn.Linear(128, 128)),
+                        ("interaction_blocks.0.activation", torch.nn.SiLU())):
+        parent, _, name = path.rpartition(".")
+        setattr(net.get_submodule(parent), name, layer.to(DEV))
+        got = m(_data(pos, types_, sizes)).out["SchNet"]["forces"].detach()
+        net2, *_ = _setup("expnormal", 32, 9.0, 2, sizes, 128, 15)
+        net2.interaction_blocks[0].activation = copy.deepcopy(net.interaction_blocks[0].activation)
+        net2.load_state_dict(net.state_dict())
+        fresh = bnn.GradientsOut(net2.to(DEV), "forces").train(training)(_data(pos, types_, sizes)).out["SchNet"]["forces"].detach()
+        scale = float(fresh.abs().max())
+        assert torch.allclose(got, fresh, rtol=1e-4, atol=1e-4 * scale) and float((got - before).abs().max()) > 1e-3 * scale, path
+        before = got
