@@ -19,6 +19,8 @@ from .cutoff import cutoff_kind
 from .mlp import MLP, init_xavier_uniform, node_linear
 
 FILTER_PRECISIONS = {"fp32": 0, "bf16": 1}
+_hooks = torch.nn.modules.module
+_EVERY_MODULES_HOOKS = (_hooks._global_forward_hooks, _hooks._global_forward_pre_hooks, _hooks._global_backward_hooks, _hooks._global_backward_pre_hooks)
 
 
 class LazyRadialBasis:
@@ -264,19 +266,19 @@ class SchNet(torch.nn.Module):
         """(module, parameter name) of every tensor ``mlcgb_schnet_eval`` reads, or None if the layout is not the standard
         one: nn.Embedding, InteractionBlock(CFConv) blocks with tanh, output network MLP([H, w, 1]) with tanh."""
         emb, head = self.embedding_layer, self.output_network
-        if type(emb) is not torch.nn.Embedding or not isinstance(head, MLP) or len(head.layers) != 3:
+        if type(emb) is not torch.nn.Embedding or type(head) is not MLP or len(head.layers) != 3:
             return None
         h0, hact, h1 = head.layers
-        if not (isinstance(h0, torch.nn.Linear) and isinstance(hact, torch.nn.Tanh) and isinstance(h1, torch.nn.Linear)):
+        if not (isinstance(h0, torch.nn.Linear) and type(hact) is torch.nn.Tanh and isinstance(h1, torch.nn.Linear)):
             return None
         if h0.bias is None or h1.out_features != 1 or h0.in_features != emb.embedding_dim:
             return None
         slots = [(emb, "weight"), (h0, "weight"), (h0, "bias"), (h1, "weight"), (h1, "bias")]
         for b in self.interaction_blocks:
-            if type(b) is not InteractionBlock or type(b.conv) is not CFConv or not isinstance(b.activation, torch.nn.Tanh):
+            if type(b) is not InteractionBlock or type(b.conv) is not CFConv or type(b.activation) is not torch.nn.Tanh:
                 return None
             c, net = b.conv, b.conv.filter_network
-            if not isinstance(net, MLP) or len(net.layers) != 3 or c.lin1.bias is not None or c.lin2.bias is None or b.lin.bias is None:
+            if type(net) is not MLP or len(net.layers) != 3 or c.lin1.bias is not None or c.lin2.bias is None or b.lin.bias is None:
                 return None
             slots += [(c.lin1, "weight"), (net.layers[0], "weight"), (net.layers[0], "bias"), (net.layers[2], "weight"), (c.lin2, "weight"),
                       (c.lin2, "bias"), (b.lin, "weight"), (b.lin, "bias")]
@@ -293,6 +295,17 @@ class SchNet(torch.nn.Module):
             self.__dict__.pop("_mlcgb_packed", None)
             self.__dict__.pop("_mlcgb_setup", None)
         return cached[2], cached[3]
+
+    def _forward_of_ones_own(self) -> bool:
+        """A ``forward`` of a subclass or an instance, which the routes past it may not leave out."""
+        return type(self).forward is not SchNet.forward or "forward" in self.__dict__
+
+    def _calls_are_watched(self) -> bool:
+        """Whether somebody would notice that a training step does not call the modules one by one: hooks on any of them or on all
+        modules of the program, or a ``forward`` put in place of theirs."""
+        return self._forward_of_ones_own() or any(_EVERY_MODULES_HOOKS) or any([
+            m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__
+            for m in self._layers()[0]])
 
     def packed_weights(self):
         """``mlcgb_schnet_weights`` over the current parameters (rebuilt whenever a parameter's storage has moved), or None."""
@@ -382,7 +395,7 @@ class SchNet(torch.nn.Module):
         return self._evaluate_whole_model(data, forces=True)
 
     def _evaluate_whole_model(self, data, forces):
-        setup = self._whole_model_setup(data.pos)
+        setup = None if self._forward_of_ones_own() else self._whole_model_setup(data.pos)
         if setup is None:
             return None
         neighbor_list = data.neighbor_list.get(self.name)
@@ -424,9 +437,9 @@ class SchNet(torch.nn.Module):
     def energy_and_forces_training(self, data):
         """(energy [B], forces [N,3]) in training mode, differentiable with respect to the weights: one library call forward and one
         backward (:class:`mlcg_b200.autograd.SchNetForceMatching`); None where that route does not apply — other layouts or widths,
-        trained basis parameters, periodic or asymmetric lists, no edges, gradients off."""
+        trained basis parameters, periodic or asymmetric lists, no edges, gradients off, hooks or a ``forward`` of one's own."""
         be = get_backend()
-        if not torch.is_grad_enabled() or self.edge_capacity:
+        if not torch.is_grad_enabled() or self.edge_capacity or self._calls_are_watched():
             return None
         setup = self._whole_model_setup(data.pos, training=True)
         if setup is None or not be.train_ok(setup):

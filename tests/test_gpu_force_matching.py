@@ -217,3 +217,38 @@ def test_a_layer_replaced_after_a_call(training):
         scale = float(fresh.abs().max())
         assert torch.allclose(got, fresh, rtol=1e-4, atol=1e-4 * scale) and float((got - before).abs().max()) > 1e-3 * scale, path
         before = got
+
+
+@pytest.mark.parametrize("where", ["", "interaction_blocks.0", "interaction_blocks.1.conv", "embedding_layer", "output_network"])
+def test_hooks_run_in_training(where):
+    sizes = [23, 40]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 9)
+    net = net.to(DEV)
+    m = bnn.GradientsOut(net, "forces").train()
+    _step(m, _data(pos, types_, sizes), target)
+    expected, calls = _grads(net), []
+    handles = [net.get_submodule(where).register_forward_hook(lambda *a: calls.append("after")),
+               net.get_submodule(where).register_forward_pre_hook(lambda *a: calls.append("before"))]
+    _step(m, _data(pos, types_, sizes), target)
+    assert calls == ["before", "after"]
+    _close(_grads(net), expected)
+    for h in handles:
+        h.remove()
+    assert _fused(_step(m, _data(pos, types_, sizes), target)["forces"])
+
+
+@pytest.mark.parametrize("training", [True, False])
+def test_a_forward_of_ones_own_runs(training):
+    sizes = [23, 40]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 9)
+
+    class Shifted(bnn.StandardSchNet):
+        def forward(self, data):
+            data = super().forward(data)
+            data.out[self.name]["energy"] = 2.0 * data.out[self.name]["energy"]
+            return data
+
+    m = bnn.GradientsOut(net.to(DEV), "forces").train(training)
+    once = m(_data(pos, types_, sizes)).out["SchNet"]["energy"]
+    net.__class__ = Shifted
+    assert torch.allclose(m(_data(pos, types_, sizes)).out["SchNet"]["energy"], 2.0 * once, rtol=1e-5)
