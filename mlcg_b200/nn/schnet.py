@@ -271,7 +271,7 @@ class SchNet(torch.nn.Module):
         h0, hact, h1 = head.layers
         if not (isinstance(h0, torch.nn.Linear) and type(hact) is torch.nn.Tanh and isinstance(h1, torch.nn.Linear)):
             return None
-        if h0.bias is None or h1.out_features != 1 or h0.in_features != emb.embedding_dim:
+        if h0.bias is None or h1.out_features != 1 or h0.in_features != emb.embedding_dim or emb.max_norm is not None:
             return None
         slots = [(emb, "weight"), (h0, "weight"), (h0, "bias"), (h1, "weight"), (h1, "bias")]
         for b in self.interaction_blocks:
@@ -444,6 +444,9 @@ class SchNet(torch.nn.Module):
         setup = self._whole_model_setup(data.pos, training=True)
         if setup is None or not be.train_ok(setup):
             return None
+        table = self.embedding_layer
+        if table.padding_idx is not None or table.max_norm is not None or table.scale_grad_by_freq or table.sparse:
+            return None             # (options that change the table's gradient or its rows)
         params = [t for t in setup[2][1][1] if t is not None]
         if not any(p.requires_grad for p in params):
             return None

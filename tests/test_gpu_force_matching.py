@@ -252,3 +252,20 @@ def test_a_forward_of_ones_own_runs(training):
     once = m(_data(pos, types_, sizes)).out["SchNet"]["energy"]
     net.__class__ = Shifted
     assert torch.allclose(m(_data(pos, types_, sizes)).out["SchNet"]["energy"], 2.0 * once, rtol=1e-5)
+
+
+@pytest.mark.parametrize("option", [dict(padding_idx=2), dict(scale_grad_by_freq=True), dict(sparse=True), dict(max_norm=0.5)])
+def test_options_of_the_embedding(option):
+    sizes = [23, 40]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 10)
+    net = net.to(DEV)
+    weight = net.embedding_layer.weight.detach().clone()
+    grads = []
+    for asked in (False, True):            # the composable operators, then what the model takes by itself
+        net.embedding_layer = torch.nn.Embedding(7, 128, _weight=weight.clone(), **option)
+        m = bnn.GradientsOut(net, "forces").train()
+        data = _data(pos, types_, sizes)
+        data.pos.requires_grad_(not asked)
+        _step(m, data, target)
+        grads.append({n: p.grad.to_dense().clone() for n, p in net.named_parameters()} | {"table": net.embedding_layer.weight.detach().clone()})
+    _close(grads[1], grads[0])
