@@ -676,7 +676,7 @@ class SchNetForceMatching(torch.autograd.Function):
         kept = ctx.saved_tensors
         params, saved = kept[:len(wanted)], kept[len(wanted):]
         if torch.is_grad_enabled():
-            pairs = [(v, g) for v, g in zip(ctx.composable(state, saved), (gE, gF)) if g is not None]
+            pairs = [(v, g) for v, g in zip(ctx.composable(state, params, saved), (gE, gF)) if g is not None]
             got = iter(torch.autograd.grad([v for v, _ in pairs], [p for p, need in zip(params, wanted) if need], [g for _, g in pairs],
                                            create_graph=True, allow_unused=True))
             return (None, None) + tuple(next(got) if need else None for need in wanted)

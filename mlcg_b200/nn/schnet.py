@@ -447,7 +447,8 @@ class SchNet(torch.nn.Module):
         table = self.embedding_layer
         if table.padding_idx is not None or table.max_norm is not None or table.scale_grad_by_freq or table.sparse:
             return None             # (options that change the table's gradient or its rows)
-        params = [t for t in setup[2][1][1] if t is not None]
+        # (the tensors that the modules hold in this call: the packed weights may be others over the same memory)
+        params = [t for t in (m._parameters[n] for m, n in self._layers()[1]) if t is not None]
         if not any(p.requires_grad for p in params):
             return None
         neighbor_list = data.neighbor_list.get(self.name)
@@ -468,7 +469,7 @@ class SchNet(torch.nn.Module):
                 return None
 
         # (holds nothing that leads to the outputs: `data` would, and its autograd graph would never be freed)
-        def composable(state, saved):  # the same two values through operators that can be differentiated to any order
+        def composable(state, params, saved):  # the same two values through operators that can be differentiated to any order
             lists = {name: state.view(saved, name) for name in ("row0", "row1", "offsets", "twin", "sel", "pair_of")}
             p, ptr = state.view(saved, "pos").detach().clone().requires_grad_(True), state.view(saved, "struct_ptr")
             plan = EdgePlan.from_graph(lists, p.shape[0], symmetric=True)
@@ -478,7 +479,9 @@ class SchNet(torch.nn.Module):
             sizes = ptr[1:] - ptr[:-1]
             owner = torch.repeat_interleave(torch.arange(sizes.numel(), device=p.device), sizes, output_size=p.shape[0])
             again = AtomicData(pos=p, atom_types=state.view(saved, "types"), batch=owner, n_atoms=sizes, neighbor_list={self.name: nl})
-            energy = self(again).out[self.name][ENERGY_KEY]
+            paths = {m: path for path, m in self.named_modules()}
+            given = {f"{paths[m]}.{n}": t for (m, n), t in zip(((m, n) for m, n in self._layers()[1] if m._parameters[n] is not None), params)}
+            energy = torch.func.functional_call(self, given, (again,)).out[self.name][ENERGY_KEY]
             return energy, -torch.autograd.grad(energy.sum(), p, create_graph=True)[0]
 
         return SchNetForceMatching.apply(result, composable, *params)

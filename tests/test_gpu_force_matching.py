@@ -269,3 +269,28 @@ def test_options_of_the_embedding(option):
         _step(m, data, target)
         grads.append({n: p.grad.to_dense().clone() for n, p in net.named_parameters()} | {"table": net.embedding_layer.weight.detach().clone()})
     _close(grads[1], grads[0])
+
+
+@pytest.mark.parametrize("create_graph", [False, True])
+def test_parameters_handed_in_for_a_call(create_graph):
+    """``torch.func.functional_call`` with aliases of the weights, and with other values than the module's."""
+    sizes = [23, 40]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 11)
+    m = bnn.GradientsOut(net.to(DEV), "forces").train()
+    _step(m, _data(pos, types_, sizes), target)
+    own = {n: p.grad.clone() for n, p in m.named_parameters() if p.grad is not None}
+    m.zero_grad(set_to_none=True)
+    for scale in (1.0, 1.1):
+        given = {n: (p.detach() if scale == 1.0 else p.detach() * scale).requires_grad_() for n, p in m.named_parameters()}
+        out = torch.func.functional_call(m, given, (_data(pos, types_, sizes),)).out["SchNet"]
+        loss = ((out["forces"] - target.to(DEV)) ** 2).mean()
+        got = torch.autograd.grad(loss, list(given.values()), create_graph=create_graph, allow_unused=True)
+        got = {n: g.detach() for n, g in zip(given, got) if g is not None}
+        if scale != 1.0:
+            with torch.no_grad():
+                for p in m.parameters():
+                    p.mul_(scale)
+            _step(m, _data(pos, types_, sizes), target)
+            own = {n: p.grad.clone() for n, p in m.named_parameters() if p.grad is not None}
+        assert set(own) <= set(got) | {"model.output_network.layers.2.bias"}
+        _close({n: got[n] for n in own}, own)
