@@ -663,6 +663,7 @@ class SchNetForceMatching(torch.autograd.Function):
     def forward(ctx, forward_pass, composable, *params):
         energy, forces, state = forward_pass
         ctx.state, ctx.composable = state, composable
+        ctx.ids = tuple(map(id, params))          # (which of the inputs are one and the same)
         ctx.save_for_backward(*params, *state.tensors)
         state.tensors = None
         ctx.set_materialize_grads(False)
@@ -677,9 +678,11 @@ class SchNetForceMatching(torch.autograd.Function):
         params, saved = kept[:len(wanted)], kept[len(wanted):]
         if torch.is_grad_enabled():
             pairs = [(v, g) for v, g in zip(ctx.composable(state, params, saved), (gE, gF)) if g is not None]
-            got = iter(torch.autograd.grad([v for v, _ in pairs], [p for p, need in zip(params, wanted) if need], [g for _, g in pairs],
-                                           create_graph=True, allow_unused=True))
-            return (None, None) + tuple(next(got) if need else None for need in wanted)
+            # (a weight that several blocks share is an input of this node for each of them, and has one gradient)
+            asked = [k for k, need in enumerate(wanted) if need and ctx.ids.index(ctx.ids[k]) == k]
+            got = dict(zip(asked, torch.autograd.grad([v for v, _ in pairs], [params[k] for k in asked], [g for _, g in pairs], create_graph=True,
+                                                      allow_unused=True)))
+            return (None, None) + tuple(got.get(k) for k in range(len(wanted)))
         gE = None if gE is None else gE.contiguous()
         gF = torch.zeros_like(state.view(saved, "pos")) if gF is None else gF.contiguous()
         grads = get_backend().schnet_train_backward(state, saved, params, gE, gF)

@@ -294,3 +294,18 @@ def test_parameters_handed_in_for_a_call(create_graph):
             own = {n: p.grad.clone() for n, p in m.named_parameters() if p.grad is not None}
         assert set(own) <= set(got) | {"model.output_network.layers.2.bias"}
         _close({n: got[n] for n in own}, own)
+
+
+def test_second_derivatives_of_a_shared_layer():
+    """A filter network that two blocks share enters the step twice: its gradient is one sum, differentiable or not."""
+    sizes = [23, 40]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 16)
+    net.interaction_blocks[1].conv.filter_network = net.interaction_blocks[0].conv.filter_network
+    m = bnn.GradientsOut(net.to(DEV), "forces").train()
+    _step(m, _data(pos, types_, sizes), target)
+    expected = _grads(net)
+    names = list(expected)
+    for create_graph in (False, True):
+        loss = ((m(_data(pos, types_, sizes)).out["SchNet"]["forces"] - target.to(DEV)) ** 2).mean()
+        got = torch.autograd.grad(loss, [dict(net.named_parameters())[n] for n in names], create_graph=create_graph)
+        _close(dict(zip(names, (g.detach() for g in got))), expected)
