@@ -445,6 +445,8 @@ class SchNet(torch.nn.Module):
         if setup is None or not be.train_ok(setup):
             return None
         table = self.embedding_layer
+        if any(p.requires_grad for p in self.rbf_layer.parameters()):
+            return None             # trained basis parameters
         if table.padding_idx is not None or table.max_norm is not None or table.scale_grad_by_freq or table.sparse:
             return None             # (options that change the table's gradient or its rows)
         # (the tensors that the modules hold in this call: the packed weights may be others over the same memory)
@@ -561,8 +563,6 @@ class SchNet(torch.nn.Module):
         if cached is not None and cached[0] == key:
             return cached[1]
         specs = [b.conv.fused_spec(self.rbf_layer, training) for b in blocks]
-        if training and any(p.requires_grad for p in rbf.parameters()):
-            specs = [None]                   # trained basis parameters: the composable operators
         precisions = {FILTER_PRECISIONS[b.conv.filter_precision] for b in blocks}
         result = None
         if all(s is not None for s in specs) and all(s[1] == specs[0][1] for s in specs[1:]) and len(precisions) == 1:

@@ -309,3 +309,17 @@ def test_second_derivatives_of_a_shared_layer():
         loss = ((m(_data(pos, types_, sizes)).out["SchNet"]["forces"] - target.to(DEV)) ** 2).mean()
         got = torch.autograd.grad(loss, [dict(net.named_parameters())[n] for n in names], create_graph=create_graph)
         _close(dict(zip(names, (g.detach() for g in got))), expected)
+
+
+def test_a_basis_unfrozen_later_is_trained():
+    sizes = [23, 40]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 12)
+    basis = bnn.ExpNormalBasis(net.rbf_layer.cutoff, 32, trainable=True).requires_grad_(False)
+    net.rbf_layer = basis
+    m = bnn.GradientsOut(net.to(DEV), "forces").train()
+    assert _fused(_step(m, _data(pos, types_, sizes), target)["forces"]) and basis.means.grad is None
+    basis.requires_grad_(True)
+    _step(m, _data(pos, types_, sizes), target)
+    assert basis.means.grad is not None and float(basis.means.grad.abs().max()) > 0
+    basis.requires_grad_(False)
+    assert _fused(_step(m, _data(pos, types_, sizes), target)["forces"])
