@@ -312,6 +312,8 @@ class SchNet(torch.nn.Module):
         slots = self._layers()[1]
         if slots is None:
             return None
+        if not all([n in m._parameters for m, n in slots]):     # (parametrized or pruned: worked out anew by the module itself)
+            return None
         tensors = [m._parameters[n] for m, n in slots]
         key = tuple(0 if t is None else t.data_ptr() for t in tensors)
         packed = self.__dict__.get("_mlcgb_packed")

@@ -323,3 +323,32 @@ def test_a_basis_unfrozen_later_is_trained():
     assert basis.means.grad is not None and float(basis.means.grad.abs().max()) > 0
     basis.requires_grad_(False)
     assert _fused(_step(m, _data(pos, types_, sizes), target)["forces"])
+
+
+class _Doubled(torch.nn.Module):
+    def forward(self, w):
+        return 2.0 * w
+
+
+@pytest.mark.parametrize("ran_before", [False, True])
+@pytest.mark.parametrize("layer", ["interaction_blocks.0.conv.lin1", "interaction_blocks.1.conv.filter_network.layers.2", "output_network.layers.0"])
+def test_parametrized_weights(layer, ran_before):
+    sizes = [23, 40]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 14)
+    net = net.to(DEV)
+    m = bnn.GradientsOut(net, "forces").train()
+    doubled = copy.deepcopy(net)
+    with torch.no_grad():
+        doubled.get_submodule(layer).weight.mul_(2.0)
+    md = bnn.GradientsOut(doubled, "forces").train()
+    expected = _step(md, _data(pos, types_, sizes), target)["forces"].detach()
+    if ran_before:
+        _step(m, _data(pos, types_, sizes), target)
+    torch.nn.utils.parametrize.register_parametrization(net.get_submodule(layer), "weight", _Doubled())
+    got = _step(m, _data(pos, types_, sizes), target)["forces"].detach()
+    assert torch.allclose(got, expected, rtol=1e-4, atol=1e-4 * float(expected.abs().max()))
+    w = net.get_submodule(layer).parametrizations.weight.original.grad
+    assert torch.allclose(w, 2.0 * doubled.get_submodule(layer).weight.grad, rtol=1e-3, atol=1e-4 * float(w.abs().max()))
+    for mode, ref in ((m.eval(), md.eval()),):
+        assert torch.allclose(mode(_data(pos, types_, sizes)).out["SchNet"]["forces"], ref(_data(pos, types_, sizes)).out["SchNet"]["forces"],
+                              rtol=1e-4, atol=1e-4 * float(expected.abs().max()))
