@@ -13,6 +13,12 @@ ENERGY_KEY = "energy"
 FORCE_KEY = "forces"
 
 
+def without_kept(module: torch.nn.Module) -> Dict[str, Any]:
+    """What ``copy`` and ``pickle`` take of a module: not what this package keeps on it between calls (``_mlcgb_...``: device
+    addresses, and lists made for tensors that the copy does not hold)."""
+    return {k: v for k, v in torch.nn.Module.__getstate__(module).items() if not k.startswith("_mlcgb_")}
+
+
 class AtomicData:
     def __init__(self, pos: torch.Tensor, atom_types: torch.Tensor, batch: torch.Tensor = None, n_atoms: torch.Tensor = None,
                  neighbor_list: Dict[str, Dict[str, Any]] = None, **extra):

@@ -13,7 +13,7 @@ from ..autograd import (attach_plan, EdgeDiff, EdgeDistanceOnce, EdgePlan, Fused
                         edge_distances, plan_of)
 from ..autograd import tanh as tanh_op
 from ..backend import get_backend, weights_struct
-from ..data import ENERGY_KEY, AtomicData
+from ..data import ENERGY_KEY, AtomicData, without_kept
 from ..neighbor_list import atomic_data2neighbor_list, bare_edge_plan, make_neighbor_list, sizes_or_pointer, validate_neighborlist
 from .cutoff import cutoff_kind
 from .mlp import MLP, init_xavier_uniform, node_linear
@@ -109,13 +109,16 @@ class CFConv(torch.nn.Module):
                getattr(self.cutoff, "cutoff_lower", None), getattr(self.cutoff, "cutoff_upper", None),
                getattr(rc, "cutoff_lower", None), getattr(rc, "cutoff_upper", None),
                tuple(map(id, net.layers)), tuple(map(id, rbf_layer._parameters.values())), tuple(map(id, rbf_layer._buffers.values())))
-        cached = self.__dict__.get("_fused_spec_cache")
+        cached = self.__dict__.get("_mlcgb_fused_spec")
         if cached is not None and cached[0] == key:
             return cached[1]
         result = self._fused_spec_uncached(rbf_layer)
         # (the objects of the key are held too, so that no other takes over one's id)
-        self.__dict__["_fused_spec_cache"] = (key, result, (rbf_layer, self.cutoff, rc, *net.layers, *rbf_layer._parameters.values(), *rbf_layer._buffers.values()))
+        self.__dict__["_mlcgb_fused_spec"] = (key, result, (rbf_layer, self.cutoff, rc, *net.layers, *rbf_layer._parameters.values(), *rbf_layer._buffers.values()))
         return result
+
+    def __getstate__(self):
+        return without_kept(self)
 
     def _fused_spec_uncached(self, rbf_layer):
         net = self.filter_network
@@ -231,6 +234,9 @@ class SchNet(torch.nn.Module):
         self.nls_distance_method = nls_distance_method
         self.output_network = output_network
         self.reset_parameters()
+
+    def __getstate__(self):
+        return without_kept(self)
 
     def reset_parameters(self):
         self.embedding_layer.reset_parameters()

@@ -1,5 +1,6 @@
 """The one-call force-matching step (values, forces, weight gradients) against a float64 evaluation of the same float32 weights."""
 import copy
+import io
 
 import pytest
 import torch
@@ -352,3 +353,18 @@ def test_parametrized_weights(layer, ran_before):
     for mode, ref in ((m.eval(), md.eval()),):
         assert torch.allclose(mode(_data(pos, types_, sizes)).out["SchNet"]["forces"], ref(_data(pos, types_, sizes)).out["SchNet"]["forces"],
                               rtol=1e-4, atol=1e-4 * float(expected.abs().max()))
+
+
+def test_a_model_that_has_run_can_be_copied_and_saved():
+    sizes = [23, 40]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 13)
+    m = bnn.GradientsOut(net.to(DEV), "forces").train()
+    _step(m, _data(pos, types_, sizes), target)
+    expected = _grads(net)
+    m.eval()(_data(pos, types_, sizes))
+    file = io.BytesIO()
+    torch.save(m, file)
+    file.seek(0)
+    for other in (copy.deepcopy(m), torch.load(file, weights_only=False)):
+        _step(other.train(), _data(pos, types_, sizes), target)
+        _close(_grads(other.model), expected, 1e-6)

@@ -264,6 +264,18 @@ def test_sumout_additivity(golden):
     assert torch.allclose(out.out["energy"], e, rtol=1e-6) and torch.allclose(out.out["forces"], f, rtol=1e-6)
 
 
+def test_copies_of_a_prior_start_without_its_kept_lists():
+    import copy
+    data, priors = prior_setup(12, 2, 3, torch.Generator().manual_seed(6))
+    for p in priors.values():
+        p.eval()(data)
+        assert any(k.startswith("_mlcgb_") for k in p.__dict__)
+        other = copy.deepcopy(p)
+        assert not any(k.startswith("_mlcgb_") for k in other.__dict__)
+        energy = data.out[p.name]["energy"]
+        assert torch.equal(other(data).out[p.name]["energy"], energy)
+
+
 def test_no_cpu_fallback(monkeypatch):
     """Without the test substitution the package refuses CPU tensors instead of computing on the host."""
     monkeypatch.setattr(backend, "_backend", None)
