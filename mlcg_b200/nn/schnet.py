@@ -321,11 +321,13 @@ class SchNet(torch.nn.Module):
         if not all([n in m._parameters for m, n in slots]):     # (parametrized or pruned: worked out anew by the module itself)
             return None
         tensors = [m._parameters[n] for m, n in slots]
-        key = tuple(0 if t is None else t.data_ptr() for t in tensors)
+        if not all([t is None or t.is_contiguous() for t in tensors]):
+            return None
+        key = tuple([0 if t is None else t.data_ptr() for t in tensors])
         packed = self.__dict__.get("_mlcgb_packed")
         if packed is not None and packed[0] == key:
             return packed[1]
-        ok = all(t is None or (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()) for t in tensors)
+        ok = all(t is None or (t.is_cuda and t.dtype == torch.float32) for t in tensors)
         H = self.embedding_layer.embedding_dim
         blocks = list(self.interaction_blocks)
         F, H2, Wh = blocks[0].conv.lin1.out_features, blocks[0].conv.lin2.out_features, self.output_network.layers[0].out_features

@@ -368,3 +368,18 @@ def test_a_model_that_has_run_can_be_copied_and_saved():
     for other in (copy.deepcopy(m), torch.load(file, weights_only=False)):
         _step(other.train(), _data(pos, types_, sizes), target)
         _close(_grads(other.model), expected, 1e-6)
+
+
+@pytest.mark.parametrize("training", [True, False])
+def test_a_weight_turned_in_place_after_a_call(training):
+    sizes = [23, 40]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 17)
+    net = net.to(DEV)
+    m = bnn.GradientsOut(net, "forces").train(training)
+    m(_data(pos, types_, sizes))
+    w = net.interaction_blocks[1].conv.lin1.weight
+    w.data = w.data.t()                            # same storage, other strides
+    got = m(_data(pos, types_, sizes)).out["SchNet"]["forces"].detach()
+    w.data = w.data.contiguous()
+    expected = m(_data(pos, types_, sizes)).out["SchNet"]["forces"].detach()
+    assert torch.allclose(got, expected, rtol=1e-4, atol=1e-4 * float(expected.abs().max()))
