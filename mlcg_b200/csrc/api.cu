@@ -6,6 +6,7 @@
 
 namespace mlcgb {
 thread_local int g_last_cuda_error = 0;
+thread_local int g_chain_depth = 0;
 
 namespace {
 struct TimelineRecord {

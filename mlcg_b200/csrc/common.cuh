@@ -38,12 +38,24 @@ struct TimelineScope {
 // already left) before that kernel has finished as a whole; it runs its own set-up — weight tiles, barriers, tensor-memory
 // allocation, nothing that depends on the previous kernel — and calls pdl_wait() before it touches any activation.
 // pdl_wait() returns once the previous kernel has completed and its writes are visible; it is a no-op for a plain launch.
+//
+// Weights read before pdl_wait() are only there if whatever wrote them had completed before the previous kernel of the stream
+// began or got past its own wait.  That holds behind a kernel of the same library call, whose kernels all wait (or are launched
+// plainly), and not for the first launch of a call, which may follow an optimiser's kernel or a copy: launch_with_weights() starts
+// early only inside a ChainScope, which a call opens once its first kernel is launched.
+extern thread_local int g_chain_depth;
+struct ChainScope {
+    ChainScope() { ++g_chain_depth; }
+    ~ChainScope() { --g_chain_depth; }
+    ChainScope(const ChainScope &) = delete;
+    ChainScope &operator=(const ChainScope &) = delete;
+};
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
-inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+inline void launch_early(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -53,8 +65,18 @@ inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);      // errors surface through cudaGetLastError() in check_launch()
+}
+// a kernel that reads nothing before its pdl_wait()
+template <typename... KArgs, typename... Args>
+inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    launch_early(true, kernel, grid, block, smem, st, args...);
+}
+// a kernel that reads weights (constants of the whole call) before it
+template <typename... KArgs, typename... Args>
+inline void launch_with_weights(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    launch_early(g_chain_depth > 0, kernel, grid, block, smem, st, args...);
 }
 #endif
 

@@ -65,6 +65,7 @@ int mlcgb_schnet_evaluate(const void *pos, const int64_t *types, const int64_t *
     int rc = mlcgb_graph_finish(pos, MLCGB_F32, ptr, N, B, r, 0, nullptr, nullptr, g, G.graph, offsets, E, nullptr, nullptr, nullptr, row0, row1, twin, sel,
                                 pair_of, host[3] != 0, status, stream);
     if (rc) return rc;
+    ChainScope chain;
     if (training)
         rc = precision ? MLCGB_E_ARG
                        : mlcgb_schnet_train_forward(pos, types, ptr, N, B, row0, row1, offsets, sel, pair_of, twin, E, E / 2, rbf, conv_cutoff_kind,

@@ -238,7 +238,7 @@ static int filter_fwd_launch(const FilterFwdParams &p, cudaStream_t st) {
     const int use_map = (make_rows_map(&wmap, p.W, p.E, kF) && !(p.sel && p.twin)) ? 1 : 0;
     const int64_t ntiles = (p.E + tc::kRows - 1) / tc::kRows;
     const int grid = (int)(ntiles < kNumSM ? ntiles : kNumSM);
-    launch_pdl(filter_fwd_pipe_kernel<SPLIT, kTcThreads>, dim3(grid), dim3(kTcThreads + 32), L::kTotal, st, p, wmap, use_map);
+    launch_with_weights(filter_fwd_pipe_kernel<SPLIT, kTcThreads>, dim3(grid), dim3(kTcThreads + 32), L::kTotal, st, p, wmap, use_map);
     return check_launch();
 }
 
@@ -920,7 +920,7 @@ static int filter_bwd_saved_launch(const FilterBwdParams &q, cudaStream_t st) {
     }
     const int64_t ntiles = (q.f.E + tc::kRows - 1) / tc::kRows;
     const int grid = (int)(ntiles < kNumSM ? ntiles : kNumSM);
-    launch_pdl(filter_bwd_saved_kernel<SPLIT>, dim3(grid), dim3(kSavedThreads), L::kTotalExtra, st, q);
+    launch_with_weights(filter_bwd_saved_kernel<SPLIT>, dim3(grid), dim3(kSavedThreads), L::kTotalExtra, st, q);
     return check_launch();
 }
 
@@ -937,7 +937,7 @@ static int filter_bwd_launch(const FilterBwdParams &q, cudaStream_t st) {
     }
     const int64_t ntiles = (q.f.E + tc::kRows - 1) / tc::kRows;
     const int grid = (int)(ntiles < kNumSM ? ntiles : kNumSM);
-    launch_pdl(filter_bwd_pipe_kernel<SPLIT>, dim3(grid), dim3(kTcThreads), L::kTotal, st, q);
+    launch_with_weights(filter_bwd_pipe_kernel<SPLIT>, dim3(grid), dim3(kTcThreads), L::kTotal, st, q);
     return check_launch();
 }
 

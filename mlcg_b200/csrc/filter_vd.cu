@@ -380,7 +380,7 @@ static int filter_vd_launch(const FilterVdParams &q, int64_t num_blocks, cudaStr
     if (!make_rows_map(&wmap, q.f.W, rows, kF, 32) || !make_rows_map(&dmap, q.Wd, rows, kF, 32)) return MLCGB_E_LIMIT;
     const int64_t ntiles = (q.f.E + tc::kRows - 1) / tc::kRows, per_block = num_blocks < kNumSM ? kNumSM / num_blocks : 1;
     const int grid = (int)(ntiles < per_block ? ntiles : per_block);
-    launch_pdl(filter_vd_kernel<SPLIT>, dim3(grid, (unsigned)num_blocks), dim3(kTcThreads + 32), kVdSmem<SPLIT>, st, q, wmap, dmap);
+    launch_with_weights(filter_vd_kernel<SPLIT>, dim3(grid, (unsigned)num_blocks), dim3(kTcThreads + 32), kVdSmem<SPLIT>, st, q, wmap, dmap);
     return check_launch();
 }
 

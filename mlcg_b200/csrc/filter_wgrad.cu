@@ -433,7 +433,7 @@ int filter_wgrad_blocks(const float *d, const float *dd, int64_t P, const int32_
         if (cudaFuncSetAttribute(filter_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FilterGradSmem::kTotal) != cudaSuccess) return check_launch();
         done[dev] = true;
     }
-    launch_pdl(filter_wgrad_kernel, dim3(filter_wgrad_parts(P, num_blocks), (unsigned)num_blocks), dim3(kTcThreads), FilterGradSmem::kTotal, st, q);
+    launch_with_weights(filter_wgrad_kernel, dim3(filter_wgrad_parts(P, num_blocks), (unsigned)num_blocks), dim3(kTcThreads), FilterGradSmem::kTotal, st, q);
     return check_launch();
 }
 

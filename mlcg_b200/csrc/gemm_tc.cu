@@ -998,11 +998,11 @@ static int rows_pipe_launch(int mode, const void *A, const void *B, const void *
     static bool p0[64] = {false}, p1[64] = {false};
     if (mode == 0) {
         if (int rc = set_smem(gemm_tc_rows_pipe_kernel<0>, p0)) return rc;
-        launch_pdl(gemm_tc_rows_pipe_kernel<0>, dim3(grid), dim3(kGT), GemmTcSmem::kTotal, st, (const float *)A, (const float *)B, (const float *)bias, M,
+        launch_with_weights(gemm_tc_rows_pipe_kernel<0>, dim3(grid), dim3(kGT), GemmTcSmem::kTotal, st, (const float *)A, (const float *)B, (const float *)bias, M,
                    (int)N, (int)K, (const float *)aux, epi, cmap, status);
     } else {
         if (int rc = set_smem(gemm_tc_rows_pipe_kernel<1>, p1)) return rc;
-        launch_pdl(gemm_tc_rows_pipe_kernel<1>, dim3(grid), dim3(kGT), GemmTcSmem::kTotal, st, (const float *)A, (const float *)B, (const float *)bias, M,
+        launch_with_weights(gemm_tc_rows_pipe_kernel<1>, dim3(grid), dim3(kGT), GemmTcSmem::kTotal, st, (const float *)A, (const float *)B, (const float *)bias, M,
                    (int)N, (int)K, (const float *)aux, epi, cmap, status);
     }
     return check_launch();
@@ -1021,7 +1021,7 @@ static int chain2_launch(const void *A, const void *Wa, const void *ba, const vo
             return check_launch();
         done[dev] = true;
     }
-    launch_pdl(gemm_tc_chain2_kernel<KIND>, dim3(grid), dim3(kGT), ChainSmem::kTotal, st, (const float *)A, (const float *)Wa, (const float *)ba,
+    launch_with_weights(gemm_tc_chain2_kernel<KIND>, dim3(grid), dim3(kGT), ChainSmem::kTotal, st, (const float *)A, (const float *)Wa, (const float *)ba,
                (const float *)Wb, (const float *)bb, (const float *)aux, M, (float *)mid_out, (float *)C, status, (const float *)ext0,
                (const float *)ext1, (float *)q_out);
     return check_launch();

@@ -49,6 +49,7 @@ static int interaction_forward_counted(const void *x, const void *d, const int64
     if ((H & 3) || (F & 3) || (H2 & 3) || H > 128 || F != 128 || H2 > 128) return MLCGB_E_LIMIT;
     int rc = mlcgb_gemm_tc_fused(0, x, W1, nullptr, nullptr, 0, N, F, H, xl, status, stream);                 // lin1 (no bias)
     if (rc) return rc;
+    ChainScope chain;
     rc = mlcgb_filter_forward_counted(d, P, pairs_dev, sel, nullptr, rbf, conv_cutoff_kind, conv_lower, conv_upper, fA1, fb1, fA2, F, precision,
                                       Wp, hsave, status, stream);
     if (rc) return rc;
@@ -97,6 +98,7 @@ static int interaction_backward_counted(const void *g, const void *a, const void
         rc = mlcgb_gemm_tc_fused(1, gy, W2, nullptr, nullptr, 0, N, F, H2, gagg, status, stream);              // through lin2
     }
     if (rc) return rc;
+    ChainScope chain;
     if (gx) {
         rc = mlcgb_seg_mul_sum(gagg, Wp, MLCGB_F32, ptr_out, nbr_out, pair_of, N, P, F, gxl, stream);          // to the gathered features
         if (rc) return rc;
@@ -254,6 +256,7 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
         }
         f.ah = nullptr; f.en = ws + lay.en; f.s = ws + lay.gd; f.want_grad = grad_pos != nullptr; f.status = status;
         if ((rc = small_start(f, st))) return rc;
+        ChainScope chain;
         if ((rc = filters(0, L))) return rc;       // (of all blocks at once: they depend on the distances alone)
         if ((rc = small_forward(f, st))) return rc;
         return small_finish(f, twin, struct_ptr, (float *)energy, (float *)grad_pos, grad_sign, st);
@@ -263,6 +266,7 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
         TimelineScope timeline_scope("embedding", stream);
         launch_pdl(embedding_rows_kernel, dim3(grid_for(N * (H >> 2), 256)), dim3(256), 0, st, (const float *)w->embedding, types, N, H, w->num_types, ws + lay.x[0], status);
     }
+    ChainScope chain;
     int cur = 0;
     for (int64_t l = 0; l < L; l++) {
         const mlcgb_schnet_block &bw = w->blocks[l];

@@ -534,7 +534,7 @@ static int small_launch_rt(const SmallNet &p, cudaStream_t st) {
     static bool done[64] = {false};
     if (int rc = small_configure(small_block_kernel<KIND, RT>, SmallSmem<RT>::kBytes, done)) return rc;
     const int64_t tiles = (p.N + RT - 1) / RT;
-    launch_pdl(small_block_kernel<KIND, RT>, dim3((unsigned)(tiles < kNumSM ? tiles : kNumSM)), dim3(kST), SmallSmem<RT>::kBytes, st, p);
+    launch_with_weights(small_block_kernel<KIND, RT>, dim3((unsigned)(tiles < kNumSM ? tiles : kNumSM)), dim3(kST), SmallSmem<RT>::kBytes, st, p);
     return check_launch();
 }
 template <int KIND>
@@ -550,7 +550,7 @@ int small_start(const SmallForward &f, cudaStream_t st) {
     int64_t grid = (f.N + 7) / 8;
     if (grid < (f.E + kST - 1) / kST) grid = (f.E + kST - 1) / kST;
     if (grid > kNumSM) grid = kNumSM;
-    launch_pdl(small_start_kernel, dim3((unsigned)grid), dim3(kST), SmallSmem<8>::kBytes, st, f.pos, f.types, f.row0, f.row1, f.N, f.E, f.w->num_types,
+    launch_with_weights(small_start_kernel, dim3((unsigned)grid), dim3(kST), SmallSmem<8>::kBytes, st, f.pos, f.types, f.row0, f.row1, f.N, f.E, f.w->num_types,
                (const float *)f.w->embedding, (const float *)f.w->blocks[0].lin1_w, f.d, f.x[0], f.xl[0], f.status);
     return check_launch();
 }

@@ -190,6 +190,7 @@ int mlcgb_schnet_train_forward(const void *pos, const int64_t *types, const int6
     if (N <= kSmallNodes) {
         const SmallForward f = small_view(o, ws, pos, types, row0, row1, pair_of, offsets, N, E, B, w, status);
         int rs = small_start(f, st);
+        ChainScope chain;
         if (!rs) rs = filters(0, L);
         if (!rs) rs = small_forward(f, st);
         return rs ? rs : small_finish(f, twin, struct_ptr, (float *)energy, (float *)grad_pos, negate ? -1.f : 1.f, st);
@@ -201,6 +202,7 @@ int mlcgb_schnet_train_forward(const void *pos, const int64_t *types, const int6
         launch_pdl(embedding_rows_kernel, dim3(grid_for(N * (kH >> 2), 256)), dim3(256), 0, st, (const float *)w->embedding, types, N, kH, w->num_types,
                    blk(0) + o.x, status);
     }
+    ChainScope chain;
     for (int64_t l = 0; l < L; l++) {
         const mlcgb_schnet_block &bw = w->blocks[l];
         float *b = blk(l), *xout = l + 1 < L ? blk(l + 1) + o.x : ws + o.block0 + L * o.stride;
@@ -251,6 +253,7 @@ int mlcgb_schnet_train_backward(const void *pos, const int64_t *types, const int
     float *xb0 = ws + v.block0 + L * v.stride;         // gradient of the first block's input
     int rc = mlcgb_edge_tangent(pos, gG, d, row0, row1, E, negate, dd, stream);
     if (rc) return rc;
+    ChainScope chain;
     float *yb = ws + v.yb, *gy = ws + v.gy, *r = ws + v.r;
     if (N <= kSmallNodes) {
         const SmallForward f = small_view(o, const_cast<float *>(fw), pos, types, row0, row1, pair_of, offsets, N, E, B, w, status);

@@ -49,3 +49,36 @@ def test_evaluation_from_positions_keeps_up_with_changing_sizes():
         given.neighbor_list = net.neighbor_list(given, 8.0)
         want = model(given).out["SchNet"]
         assert torch.equal(got["energy"], want["energy"]) and torch.equal(got["forces"], want["forces"]), sizes
+
+
+@pytest.mark.parametrize("sizes", [[40, 30], [2500]])
+def test_weights_written_by_the_launch_before(sizes):
+    """A call whose first kernels read weights sees what the kernel launched just before it wrote to them, and so does one product
+    whose second operand the product before it has made."""
+    from mlcg_b200.backend import get_backend
+    torch.manual_seed(0)
+    cut = bnn.CosineCutoff(0.0, 8.0)
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, 32, trainable=False), cut, [128], embedding_size=5, num_interactions=2).eval().to(DEV)
+    model = bnn.GradientsOut(net, "forces").eval()
+    n = sum(sizes)
+    data = mlcg_b200.AtomicData(pos=torch.rand(n, 3, device=DEV).mul(20.0), atom_types=torch.zeros(n, dtype=torch.int64, device=DEV),
+                                batch=torch.repeat_interleave(torch.arange(len(sizes)), torch.tensor(sizes)).to(DEV), n_atoms=torch.tensor(sizes, device=DEV))
+    data.neighbor_list = net.neighbor_list(data, 8.0)
+    params = [p.data for p in net.parameters()]
+    versions, want = [[p * s for p in params] for s in (1.0, 0.5, 1.5)], []
+    write = lambda v: torch._foreach_copy_(params, v)  # noqa: E731
+    for v in versions:
+        write(v)
+        torch.cuda.synchronize()
+        want.append({k: t.clone() for k, t in model(data).out["SchNet"].items()})
+    for k in [1, 0, 2] * 10:
+        write(versions[k])
+        got = model(data).out["SchNet"]
+        assert torch.equal(got["forces"], want[k]["forces"]) and torch.equal(got["energy"], want[k]["energy"])
+    be = get_backend()
+    x, w = torch.randn(128, 128, device=DEV), torch.randn(128, 128, device=DEV) / 11
+    y = be.gemm_fused(0, x, w)
+    torch.cuda.synchronize()
+    z = be.gemm_fused(0, x, y)
+    for _ in range(20):
+        assert torch.equal(be.gemm_fused(0, x, be.gemm_fused(0, x, w)), z)
