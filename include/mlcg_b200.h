@@ -523,7 +523,8 @@ int mlcgb_schnet_evaluate(const void *pos, const int64_t *types, const int64_t *
 void mlcgb_schnet_evaluate_lists(int64_t N, int64_t B, int64_t E, int64_t *at /* [8] */);
 
 /* One force-matching step of the same model, all widths 128 except the output network's (MLCGB_E_LIMIT otherwise), E > 0:
- *   forward:  energies and d(sum of energies)/d(pos) as mlcgb_schnet_eval gives them; `workspace` keeps what the backward reads
+ *   forward:  energies and d(sum of energies)/d(pos) as mlcgb_schnet_eval gives them; `workspace` keeps what the backward reads, a
+ *             copy of the positions (its first 3 N floats) among it
  *   backward: for a loss L(energies, grad_pos) with gE [B] (or NULL: zero) and gG [N,3] its derivatives, dL/d(every weight): the
  *             derivative along the displacement gG of the positions and its way back (src/mlcg/nn/gradients.py:216-222 with
  *             create_graph, then loss.backward()).  `grads` holds device pointers shaped like the weights (head_out_b ignored; its
@@ -537,7 +538,7 @@ int mlcgb_schnet_train_forward(const void *pos, const int64_t *types, const int6
                                int64_t E, int64_t P, const mlcgb_rbf_spec *rbf, int conv_cutoff_kind, double conv_lower, double conv_upper,
                                const mlcgb_schnet_weights *w, int negate, void *workspace, size_t workspace_bytes, void *energy, void *grad_pos,
                                int32_t *status, void *stream);
-int mlcgb_schnet_train_backward(const void *pos, const int64_t *types, const int64_t *struct_ptr, int64_t N, int64_t B, const int32_t *row0,
+int mlcgb_schnet_train_backward(const int64_t *types, const int64_t *struct_ptr, int64_t N, int64_t B, const int32_t *row0,
                                 const int32_t *row1, const int64_t *offsets, const int32_t *sel, const int32_t *pair_of, int64_t E, int64_t P,
                                 const mlcgb_rbf_spec *rbf, int conv_cutoff_kind, double conv_lower, double conv_upper,
                                 const mlcgb_schnet_weights *w, int negate, const void *gE, const void *gG, const void *forward_workspace, void *workspace,

@@ -129,7 +129,7 @@ SIGNATURES = {
     "mlcgb_gemm_tc_chain2_tangent": (c_int, [c_int] + [c_vp] * 6 + [c_i64] + [c_vp] * 5),
     "mlcgb_schnet_train_workspace_bytes": (c_sz, [c_int] + [c_i64] * 7),
     "mlcgb_schnet_train_forward": (c_int, [c_vp] * 3 + [c_i64, c_i64] + [c_vp] * 6 + [c_i64, c_i64, c_vp, c_int, c_dbl, c_dbl, c_vp, c_int, c_vp, c_sz] + [c_vp] * 4),
-    "mlcgb_schnet_train_backward": (c_int, [c_vp] * 3 + [c_i64, c_i64] + [c_vp] * 5 + [c_i64, c_i64, c_vp, c_int, c_dbl, c_dbl, c_vp, c_int] + [c_vp] * 4 + [c_sz]
+    "mlcgb_schnet_train_backward": (c_int, [c_vp] * 2 + [c_i64, c_i64] + [c_vp] * 5 + [c_i64, c_i64, c_vp, c_int, c_dbl, c_dbl, c_vp, c_int] + [c_vp] * 4 + [c_sz]
                                     + [c_vp] * 3),
     "mlcgb_seg_force": (c_int, [c_vp] * 7 + [c_i64, c_i64, c_vp, c_vp, c_int, c_vp]),
     "mlcgb_seg_tangent": (c_int, [c_vp] * 8 + [c_i64, c_i64, c_vp, c_vp]),

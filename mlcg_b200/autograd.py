@@ -684,7 +684,7 @@ class SchNetForceMatching(torch.autograd.Function):
                                                       allow_unused=True)))
             return (None, None) + tuple(got.get(k) for k in range(len(wanted)))
         gE = None if gE is None else gE.contiguous()
-        gF = torch.zeros_like(state.view(saved, "pos")) if gF is None else gF.contiguous()
+        gF = torch.zeros_like(state.positions(saved)) if gF is None else gF.contiguous()
         grads = get_backend().schnet_train_backward(state, saved, params, gE, gF)
         tensors = state.weights[1][1]
         if tensors[4] is not None:                     # the last bias enters every bead's energy once, and no force

@@ -5,7 +5,7 @@ back end is :class:`CudaBackend`; it refuses tensors that are not on a CUDA devi
 raises if ``libmlcg_b200.so`` is missing.
 """
 import ctypes
-from dataclasses import dataclass, replace
+from dataclasses import dataclass
 from typing import Optional
 
 import numpy as np
@@ -72,22 +72,28 @@ def _weights_places(weights):
 class ForceMatchingState:
     """What the backward of a force-matching step needs of its forward pass.  ``tensors``: the device buffers, which the pass's autograd
     node takes over as saved tensors; everything else says where in them things lie.  No address outlives the forward pass: saved-tensor
-    hooks may bring the buffers back elsewhere.  ``places``: name -> (index in ``tensors``, byte offset, entries, dtype; offset None: the
-    tensor itself)."""
+    hooks may bring the buffers back elsewhere.  ``places``: (index in ``tensors``, byte offset) of each of :attr:`NAMES`."""
 
+    NAMES = ("types", "struct_ptr", "row0", "row1", "offsets", "sel", "pair_of", "forward_ws", "twin", "p0", "p1")
     __slots__ = ("N", "B", "E", "tensors", "places", "spec", "conv_cut", "weights")
 
     def __init__(self, *values):
-        for name, value in zip(self.__slots__, values):
-            setattr(self, name, value)
+        self.N, self.B, self.E, self.tensors, self.places, self.spec, self.conv_cut, self.weights = values
+
+    def addresses(self, saved):
+        base = [0 if t is None else t.data_ptr() for t in saved]
+        return [base[k] + at for k, at in self.places]
 
     def view(self, saved, name):
-        k, at, n, dtype = self.places[name]
-        return saved[k] if at is None else saved[k][at: at + n * dtype.itemsize].view(dtype)
+        k, at = self.places[self.NAMES.index(name)]
+        if saved[k].dtype != torch.uint8:             # (a tensor of its own)
+            return saved[k]
+        entries, dtype = {"struct_ptr": (self.B + 1, torch.int64), "offsets": (self.N + 1, torch.int64), "sel": (self.E // 2, torch.int32),
+                          "forward_ws": (3 * self.N, torch.float32)}.get(name, (self.E, torch.int32))
+        return saved[k][at: at + entries * dtype.itemsize].view(dtype)
 
-    def address(self, saved, name):
-        k, at, _, _ = self.places[name]
-        return saved[k].data_ptr() + (at or 0)
+    def positions(self, saved):
+        return self.view(saved, "forward_ws").view(self.N, 3)
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -115,12 +121,6 @@ def _on(device):
     if device.index is None or device.index == torch._C._cuda_getDevice():
         return _NO_GUARD
     return torch.cuda.device(device)
-
-
-def _own(t: torch.Tensor, given: torch.Tensor) -> torch.Tensor:
-    """``t`` where it does not share memory with ``given``, else a copy: for what a backward pass reads of inputs that the caller may
-    have overwritten by then."""
-    return t.clone() if t.data_ptr() == given.data_ptr() else t
 
 
 def _need_cuda(*ts):
@@ -530,8 +530,8 @@ class CudaBackend:
         return out
 
     # ------------------------------------------------------------------ radial basis
-    def _spec(self, spec: RbfSpec, dtype):
-        p0, p1 = spec.p0, spec.p1
+    def _spec(self, spec: RbfSpec, dtype, p0=None, p1=None):
+        p0, p1 = spec.p0 if p0 is None else p0, spec.p1 if p1 is None else p1
         if p0.dtype != dtype or p1.dtype != dtype or not (p0.is_contiguous() and p1.is_contiguous()):
             p0 = p0.detach().to(dtype).contiguous()
             p1 = p1.detach().to(dtype).reshape(-1).contiguous()
@@ -822,7 +822,7 @@ class CudaBackend:
         guess at the edge count that sizes the workspace (too low costs a second call).  ``training``: the forward pass of
         :meth:`schnet_train_forward` (forces), its state as the last value."""
         w, _keep = weights
-        given, pos = pos, pos.detach().contiguous()
+        pos = pos.detach().contiguous()
         N, dev = pos.shape[0], pos.device
         B = ptr.numel() - 1 if n_atoms is None else n_atoms.numel()
         s, keep = self._spec(spec, torch.float32)
@@ -855,15 +855,10 @@ class CudaBackend:
         self.defer_status(status, "SchNet force matching" if training else "SchNet evaluation")
         if not training:
             return energy, grad, E, None
-        pos = _own(pos, given)
         at = (ctypes.c_int64 * 8)()
         lib.mlcgb_schnet_evaluate_lists(N, B, E, at)
-        i32, i64 = torch.int32, torch.int64
-        places = {"pos": (0, None, 0, None), "types": (1, None, 0, None), "p0": (2, None, 0, None), "p1": (3, None, 0, None),
-                  "struct_ptr": (5, at[0], B + 1, i64) if ptr is None else (6, None, 0, None), "offsets": (5, at[1], N + 1, i64),
-                  "row0": (4, at[2], E, i32), "row1": (4, at[3], E, i32), "twin": (4, at[4], E, i32), "pair_of": (4, at[5], E, i32),
-                  "sel": (4, at[6], E // 2, i32), "forward_ws": (4, at[7], 0, None)}
-        return energy, grad, E, ForceMatchingState(N, B, E, (pos, types, spec.p0, spec.p1, ws, graph_ws, ptr), places, spec, conv_cut, weights)
+        places = ((0, 0), (4, at[0]) if ptr is None else (5, 0), (3, at[2]), (3, at[3]), (4, at[1]), (3, at[6]), (3, at[5]), (3, at[7]), (3, at[4]), (1, 0), (2, 0))
+        return energy, grad, E, ForceMatchingState(N, B, E, (types, spec.p0, spec.p1, ws, graph_ws, ptr), places, spec, conv_cut, weights)
 
     # ------------------------------------------------------------------ one force-matching step
     @staticmethod
@@ -876,7 +871,7 @@ class CudaBackend:
     def schnet_train_forward(self, pos, types, struct_ptr, plan, spec: RbfSpec, conv_cut, weights):
         """(energies [B], forces [N,3], state for :meth:`schnet_train_backward`) of a standard SchNet on a given edge plan."""
         wstruct, _keep = weights
-        given, pos = pos, pos.detach().contiguous()
+        pos = pos.detach().contiguous()
         N, B, dev = pos.shape[0], struct_ptr.numel() - 1, pos.device
         sel, pair_of = plan.half_selection(), plan.pair_index()
         s, keep = self._spec(spec, torch.float32)
@@ -891,34 +886,31 @@ class CudaBackend:
                 _ptr(plan.perm_in), plan.E, sel.numel(), ctypes.byref(s), int(conv_cut[0]), float(conv_cut[1]), float(conv_cut[2]), ctypes.byref(wstruct), 1,
                 _ptr(ws), wsb, _ptr(energy), _ptr(forces), _ptr(status), _stream()), "schnet_train_forward")
         self.defer_status(status, "SchNet force matching")
-        names = ("pos", "types", "p0", "p1", "struct_ptr", "offsets", "row0", "row1", "twin", "pair_of", "sel", "forward_ws")
-        tensors = (_own(pos, given), types, spec.p0, spec.p1, struct_ptr, plan.ptr_out, plan.row0, plan.row1, plan.perm_in, pair_of, sel, ws)
-        return energy, forces, ForceMatchingState(N, B, plan.E, tensors, {n: (k, None, 0, None) for k, n in enumerate(names)}, spec, conv_cut, weights)
+        tensors = (types, struct_ptr, plan.row0, plan.row1, plan.ptr_out, sel, pair_of, ws, plan.perm_in, spec.p0, spec.p1)
+        return energy, forces, ForceMatchingState(N, B, plan.E, tensors, tuple((k, 0) for k in range(len(tensors))), spec, conv_cut, weights)
 
     def schnet_train_backward(self, state, saved, params, gE, gF):
         """Gradients of a loss on the energies and forces of the forward pass that ``state`` came from with respect to the weights, as
         views of one buffer in the order of the packed weights (``None`` for the output network's second bias).  ``saved``, ``params``:
         the buffers of the state and the weights (without the absent ones) as the autograd node's saved tensors hand them back."""
         wstruct, (_, tensors, live, addresses) = state.weights
-        params = iter(params)
-        weights = [None if t is None else next(params) for t in tensors]
-        if tuple(0 if t is None else t.data_ptr() for t in weights) != addresses:       # (moved by a saved-tensor hook)
-            weights = [None if t is None else t.contiguous() for t in weights]
+        if tuple([t.data_ptr() for t in params]) != addresses:       # (moved by a saved-tensor hook)
+            moved = iter([t.contiguous() for t in params])
+            weights = [None if t is None else next(moved) for t in tensors]
             wstruct, _keep = weights_struct(wstruct, weights)
         N, B, E, dev = state.N, state.B, state.E, gF.device
-        s, keep = self._spec(replace(state.spec, p0=state.view(saved, "p0"), p1=state.view(saved, "p1")), torch.float32)
+        types, struct_ptr, row0, row1, offsets, sel, pair_of, forward_ws = state.addresses(saved)[:8]
+        s, keep = self._spec(state.spec, torch.float32, saved[state.places[-2][0]], saved[state.places[-1][0]])
         wsb = self.lib.mlcgb_schnet_train_workspace_bytes(1, N, E, E // 2, state.spec.num_rbf, wstruct.head_width, wstruct.num_blocks, wstruct.num_types)
         ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
         places = _weights_places(state.weights)
         flat = torch.empty(places.total, dtype=torch.float32, device=dev)
         gs, arr = places.struct(wstruct, flat.data_ptr())
         status = self._sticky_status(dev)
-        pos, types, struct_ptr, row0, row1, offsets, sel, pair_of, forward_ws = [
-            state.address(saved, n) for n in ("pos", "types", "struct_ptr", "row0", "row1", "offsets", "sel", "pair_of", "forward_ws")]
         cut = state.conv_cut
         with _on(dev):
             _lib.check(self.lib.mlcgb_schnet_train_backward(
-                pos, types, struct_ptr, N, B, row0, row1, offsets, sel, pair_of, E, E // 2, ctypes.byref(s), int(cut[0]), float(cut[1]), float(cut[2]),
+                types, struct_ptr, N, B, row0, row1, offsets, sel, pair_of, E, E // 2, ctypes.byref(s), int(cut[0]), float(cut[1]), float(cut[2]),
                 ctypes.byref(wstruct), 1, _ptr(gE), _ptr(gF), forward_ws, ws.data_ptr(), wsb, ctypes.byref(gs), status.data_ptr(), _stream()),
                 "schnet_train_backward")
         self.defer_status(status, "SchNet force matching")

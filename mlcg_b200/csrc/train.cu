@@ -77,10 +77,18 @@ embedding_grad_kernel(const float *__restrict__ xb, const int64_t *__restrict__ 
     for (int t = 0; t < T; t++) partial[(me * T + t) * 128 + c] = tab[t * 128];
 }
 
+// Before anything else of a forward pass: the positions as the backward will want them (the caller may overwrite his), zmax cleared
+__global__ void __launch_bounds__(256)
+train_begin_kernel(const float *__restrict__ pos, int64_t n, float *__restrict__ kept, float *__restrict__ zmax, int64_t L) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < L) zmax[t] = 0.f;
+    for (int64_t i = t; i < n; i += (int64_t)gridDim.x * blockDim.x) kept[i] = pos[i];
+}
+
 constexpr int64_t kH = 128;
 
 struct TrainForward {                                 // offsets in floats
-    int64_t d, gd, en, ah, zmax, W, Wd, Hs, Zs, wstride, hstride, block0, stride, total;      // W .. Zs: of all blocks
+    int64_t pos, d, gd, en, ah, zmax, W, Wd, Hs, Zs, wstride, hstride, block0, stride, total;      // W .. Zs: of all blocks
     int64_t x, xl, agg, a, gu, gagg, gxl, g;          // of a block; g: the gradient of the block's output
 };
 struct TrainBackward {
@@ -95,6 +103,7 @@ static TrainForward train_forward_layout(int64_t N, int64_t E, int64_t P, int64_
     int64_t at = 0;
     auto take = [&](int64_t n) { const int64_t r = at; at += (n + 3) & ~(int64_t)3; return r; };
     const int64_t hidden = (int64_t)(mlcgb_filter_hidden_bytes(P) / sizeof(float));
+    o.pos = take(3 * N);
     o.d = take(E); o.gd = take(E); o.en = take(N); o.ah = take(N * Wh); o.zmax = take(L);
     o.wstride = padded_rows(P) * kH;
     o.hstride = hidden;
@@ -182,7 +191,8 @@ int mlcgb_schnet_train_forward(const void *pos, const int64_t *types, const int6
     float *ws = (float *)workspace, *d = ws + o.d;
     auto st = (cudaStream_t)stream;
     auto blk = [&](int64_t l) { return ws + o.block0 + l * o.stride; };
-    cudaMemsetAsync(ws + o.zmax, 0, L * sizeof(float), st);
+    train_begin_kernel<<<grid_for(3 * N, 256), 256, 0, st>>>((const float *)pos, 3 * N, ws + o.pos, ws + o.zmax, L);
+    ChainScope chain;
     auto filters = [&](int64_t l, int64_t n) {
         return filter_vd_blocks(d, P, nullptr, sel, rbf, conv_cutoff_kind, conv_lower, conv_upper, w->blocks + l, n, 0, ws + o.W + l * o.wstride,
                                 ws + o.Wd + l * o.wstride, ws + o.Hs + l * o.hstride, ws + o.Zs + l * o.hstride, ws + o.zmax + l, status, st);
@@ -190,7 +200,6 @@ int mlcgb_schnet_train_forward(const void *pos, const int64_t *types, const int6
     if (N <= kSmallNodes) {
         const SmallForward f = small_view(o, ws, pos, types, row0, row1, pair_of, offsets, N, E, B, w, status);
         int rs = small_start(f, st);
-        ChainScope chain;
         if (!rs) rs = filters(0, L);
         if (!rs) rs = small_forward(f, st);
         return rs ? rs : small_finish(f, twin, struct_ptr, (float *)energy, (float *)grad_pos, negate ? -1.f : 1.f, st);
@@ -202,7 +211,6 @@ int mlcgb_schnet_train_forward(const void *pos, const int64_t *types, const int6
         launch_pdl(embedding_rows_kernel, dim3(grid_for(N * (kH >> 2), 256)), dim3(256), 0, st, (const float *)w->embedding, types, N, kH, w->num_types,
                    blk(0) + o.x, status);
     }
-    ChainScope chain;
     for (int64_t l = 0; l < L; l++) {
         const mlcgb_schnet_block &bw = w->blocks[l];
         float *b = blk(l), *xout = l + 1 < L ? blk(l + 1) + o.x : ws + o.block0 + L * o.stride;
@@ -232,19 +240,19 @@ int mlcgb_schnet_train_forward(const void *pos, const int64_t *types, const int6
     return finish_launch((const float *)pos, ws + o.gd, d, row1, offsets, twin, N, (float *)grad_pos, negate ? -1.f : 1.f, ws + o.en, struct_ptr, B, (float *)energy, st);
 }
 
-int mlcgb_schnet_train_backward(const void *pos, const int64_t *types, const int64_t *struct_ptr, int64_t N, int64_t B, const int32_t *row0,
+int mlcgb_schnet_train_backward(const int64_t *types, const int64_t *struct_ptr, int64_t N, int64_t B, const int32_t *row0,
                                 const int32_t *row1, const int64_t *offsets, const int32_t *sel, const int32_t *pair_of, int64_t E, int64_t P,
                                 const mlcgb_rbf_spec *rbf, int conv_cutoff_kind, double conv_lower, double conv_upper,
                                 const mlcgb_schnet_weights *w, int negate, const void *gE, const void *gG, const void *forward_workspace, void *workspace,
                                 size_t workspace_bytes, const mlcgb_schnet_weights *grads, int32_t *status, void *stream) {
     if (!rbf || !w || !grads || N <= 0 || B <= 0 || E <= 0 || 2 * P != E) return MLCGB_E_ARG;
-    if (!pos || !types || !struct_ptr || !row0 || !row1 || !offsets || !sel || !pair_of || !gG || !forward_workspace || !workspace || !status) return MLCGB_E_ARG;
+    if (!types || !struct_ptr || !row0 || !row1 || !offsets || !sel || !pair_of || !gG || !forward_workspace || !workspace || !status) return MLCGB_E_ARG;
     const int64_t R = rbf->num_rbf, Wh = w->head_width, L = w->num_blocks, T = w->num_types;
     if (!train_supported(w, R)) return MLCGB_E_LIMIT;
     const TrainForward o = train_forward_layout(N, E, P, Wh, L);
     const TrainBackward v = train_backward_layout(N, E, P, R, Wh, L, T);
     if (workspace_bytes < (size_t)v.total * sizeof(float)) return MLCGB_E_WORKSPACE;
-    const float *fw = (const float *)forward_workspace, *d = fw + o.d;
+    const float *fw = (const float *)forward_workspace, *d = fw + o.d, *pos = fw + o.pos;
     float *ws = (float *)workspace, *dd = ws + v.dd;
     auto st = (cudaStream_t)stream;
     auto fblk = [&](int64_t l) { return fw + o.block0 + l * o.stride; };

@@ -323,7 +323,7 @@ class SchNet(torch.nn.Module):
         tensors = [m._parameters[n] for m, n in slots]
         if not all([t is None or t.is_contiguous() for t in tensors]):
             return None
-        key = tuple([0 if t is None else t.data_ptr() for t in tensors])
+        key = tuple([t.data_ptr() for t in tensors if t is not None])
         packed = self.__dict__.get("_mlcgb_packed")
         if packed is not None and packed[0] == key:
             return packed[1]
@@ -483,7 +483,7 @@ class SchNet(torch.nn.Module):
         # (holds nothing that leads to the outputs: `data` would, and its autograd graph would never be freed)
         def composable(state, params, saved):  # the same two values through operators that can be differentiated to any order
             lists = {name: state.view(saved, name) for name in ("row0", "row1", "offsets", "twin", "sel", "pair_of")}
-            p, ptr = state.view(saved, "pos").detach().clone().requires_grad_(True), state.view(saved, "struct_ptr")
+            p, ptr = state.positions(saved).clone().requires_grad_(True), state.view(saved, "struct_ptr")
             plan = EdgePlan.from_graph(lists, p.shape[0], symmetric=True)
             nl = make_neighbor_list(tag="", order=2, index_mapping=attach_plan(torch.stack([plan.row0, plan.row1]).to(torch.int64), plan),
                                     rcut=self.rbf_layer.cutoff.cutoff_upper, self_interaction=False)
