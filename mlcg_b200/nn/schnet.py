@@ -23,6 +23,62 @@ _hooks = torch.nn.modules.module
 _EVERY_MODULES_HOOKS = (_hooks._global_forward_hooks, _hooks._global_forward_pre_hooks, _hooks._global_backward_hooks, _hooks._global_backward_pre_hooks)
 
 
+def _all_modules(module):
+    """``module.modules()`` in another order and a third of the time."""
+    found, todo = {}, [module]
+    while todo:
+        m = todo.pop()
+        if m is not None and m not in found:
+            found[m] = None
+            todo.extend(m._modules.values())
+    return list(found)
+
+
+class _Layers:
+    """The modules of a SchNet by direct reference, for what its one-call routes look at in every call (attribute access through
+    ``torch.nn.Module`` takes half a microsecond a step).  Made anew when a module has been put in, taken out or replaced."""
+
+    def __init__(self, net):
+        modules = _all_modules(net)
+        self._children = [m._modules for m in modules if m._modules]
+        self._found = [child for c in self._children for child in c.values()]
+        self._states = [m.__dict__ for m in modules]
+        basis = net.rbf_layer
+        self._basis = [m._parameters for m in _all_modules(basis)]
+        self._basis_tensors = (basis._parameters, basis._buffers)
+        self.slots = net._whole_model_slots()         # (module, parameter name) of every weight, or None
+        self._places = None if self.slots is None else [(m._parameters, n) for m, n in self.slots]
+        self._cutoffs = None if self.slots is None else [(b.conv, b.conv.cutoff) for b in net.interaction_blocks]
+        self._basis_cutoff = getattr(basis, "cutoff", None)
+
+    def still_there(self) -> bool:
+        return [child for c in self._children for child in c.values()] == self._found
+
+    def weights(self):
+        """The tensor of every slot (None: a bias that is absent); None for other layouts and for parametrized or pruned layers, whose
+        weights are worked out anew by the modules themselves."""
+        try:
+            return None if self._places is None else [p[n] for p, n in self._places]
+        except KeyError:
+            return None
+
+    def watched(self) -> bool:
+        """Whether somebody would notice that a training step does not call the modules one by one: hooks on any of them or on all
+        modules of the program, or a ``forward`` put in place of theirs."""
+        return any(_EVERY_MODULES_HOOKS) or any([d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]
+                                                 or "forward" in d for d in self._states])
+
+    def trained_basis(self) -> bool:
+        return any([t is not None and t.requires_grad for p in self._basis for t in p.values()])
+
+    def description(self):
+        """What the filter description of the model is worked out from, beside the modules and the weights."""
+        lo, hi = getattr(self._basis_cutoff, "cutoff_lower", None), getattr(self._basis_cutoff, "cutoff_upper", None)
+        parameters, buffers = self._basis_tensors
+        return (*map(id, parameters.values()), *map(id, buffers.values()), lo, hi,
+                *[(getattr(c, "cutoff_lower", None), getattr(c, "cutoff_upper", None), conv.filter_precision) for conv, c in self._cutoffs])
+
+
 class LazyRadialBasis:
     """Stands for ``rbf_layer(distances)`` without computing it.  In eval mode the fused tensor-core kernel
     evaluates the basis inside its GEMM prologue, so the ``[E, R]`` expansion never has to exist; a consumer
@@ -290,38 +346,22 @@ class SchNet(torch.nn.Module):
                       (c.lin2, "bias"), (b.lin, "weight"), (b.lin, "bias")]
         return slots
 
-    def _layers(self):
-        """(all modules, :meth:`_whole_model_slots`), worked out again when a module has been put in, taken out or replaced."""
+    def _layers(self) -> "_Layers":
         cached = self.__dict__.get("_mlcgb_layers")
-        if cached is None or [child for children in cached[0] for child in children.values()] != cached[1]:
-            modules = list(self.modules())
-            children = [m._modules for m in modules]
-            cached = (children, [child for c in children for child in c.values()], modules, self._whole_model_slots())
-            self.__dict__["_mlcgb_layers"] = cached
+        if cached is None or not cached.still_there():
+            cached = self.__dict__["_mlcgb_layers"] = _Layers(self)
             self.__dict__.pop("_mlcgb_packed", None)
             self.__dict__.pop("_mlcgb_setup", None)
-        return cached[2], cached[3]
+        return cached
 
     def _forward_of_ones_own(self) -> bool:
         """A ``forward`` of a subclass or an instance, which the routes past it may not leave out."""
         return type(self).forward is not SchNet.forward or "forward" in self.__dict__
 
-    def _calls_are_watched(self) -> bool:
-        """Whether somebody would notice that a training step does not call the modules one by one: hooks on any of them or on all
-        modules of the program, or a ``forward`` put in place of theirs."""
-        return self._forward_of_ones_own() or any(_EVERY_MODULES_HOOKS) or any([
-            m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__
-            for m in self._layers()[0]])
-
-    def packed_weights(self):
+    def packed_weights(self, layers=None):
         """``mlcgb_schnet_weights`` over the current parameters (rebuilt whenever a parameter's storage has moved), or None."""
-        slots = self._layers()[1]
-        if slots is None:
-            return None
-        if not all([n in m._parameters for m, n in slots]):     # (parametrized or pruned: worked out anew by the module itself)
-            return None
-        tensors = [m._parameters[n] for m, n in slots]
-        if not all([t is None or t.is_contiguous() for t in tensors]):
+        tensors = (self._layers() if layers is None else layers).weights()
+        if tensors is None or not all([t is None or t.is_contiguous() for t in tensors]):
             return None
         key = tuple([t.data_ptr() for t in tensors if t is not None])
         packed = self.__dict__.get("_mlcgb_packed")
@@ -449,19 +489,20 @@ class SchNet(torch.nn.Module):
         backward (:class:`mlcg_b200.autograd.SchNetForceMatching`); None where that route does not apply — other layouts or widths,
         trained basis parameters, periodic or asymmetric lists, no edges, gradients off, hooks or a ``forward`` of one's own."""
         be = get_backend()
-        if not torch.is_grad_enabled() or self.edge_capacity or self._calls_are_watched():
+        if not torch.is_grad_enabled() or self.edge_capacity or self._forward_of_ones_own():
             return None
-        setup = self._whole_model_setup(data.pos, training=True)
-        if setup is None or not be.train_ok(setup):
+        layers = self._layers()
+        if layers.slots is None or layers.watched():
             return None
-        table = self.embedding_layer
-        if any(p.requires_grad for p in self.rbf_layer.parameters()):
-            return None             # trained basis parameters
+        setup = self._whole_model_setup(data.pos, True, layers)
+        if setup is None or not be.train_ok(setup) or layers.trained_basis():
+            return None
+        table = layers.slots[0][0]
         if table.padding_idx is not None or table.max_norm is not None or table.scale_grad_by_freq or table.sparse:
             return None             # (options that change the table's gradient or its rows)
         # (the tensors that the modules hold in this call: the packed weights may be others over the same memory)
-        params = [t for t in (m._parameters[n] for m, n in self._layers()[1]) if t is not None]
-        if not any(p.requires_grad for p in params):
+        params = [t for t in layers.weights() if t is not None]
+        if not any([p.requires_grad for p in params]):
             return None
         neighbor_list = data.neighbor_list.get(self.name)
         if self.is_nl_compatible(neighbor_list):
@@ -492,7 +533,7 @@ class SchNet(torch.nn.Module):
             owner = torch.repeat_interleave(torch.arange(sizes.numel(), device=p.device), sizes, output_size=p.shape[0])
             again = AtomicData(pos=p, atom_types=state.view(saved, "types"), batch=owner, n_atoms=sizes, neighbor_list={self.name: nl})
             paths = {m: path for path, m in self.named_modules()}
-            given = {f"{paths[m]}.{n}": t for (m, n), t in zip(((m, n) for m, n in self._layers()[1] if m._parameters[n] is not None), params)}
+            given = {f"{paths[m]}.{n}": t for (m, n), t in zip(((m, n) for m, n in layers.slots if m._parameters[n] is not None), params)}
             energy = torch.func.functional_call(self, given, (again,)).out[self.name][ENERGY_KEY]
             return energy, -torch.autograd.grad(energy.sum(), p, create_graph=True)[0]
 
@@ -550,7 +591,7 @@ class SchNet(torch.nn.Module):
             types = types.to(torch.int64).contiguous()
         return types
 
-    def _whole_model_setup(self, pos, training=False):
+    def _whole_model_setup(self, pos, training=False, layers=None):
         """(basis spec, CFConv cutoff, packed weights, filter precision) for ``mlcgb_schnet_eval``, or None: eval mode, no kernel
         profiler attached, float32 positions on CUDA, standard layout with every block on the fused filter
         kernel, one cutoff and one filter precision for all blocks.  The model-dependent part is worked out once per set of
@@ -559,19 +600,15 @@ class SchNet(torch.nn.Module):
         if (self.training != training or getattr(be, "profiler", True) is not None or not getattr(be, "tensor_core_gemm", False) or not pos.is_cuda
                 or pos.dtype != torch.float32 or pos.shape[0] == 0):
             return None
-        weights = self.packed_weights()
+        layers = self._layers() if layers is None else layers
+        weights = self.packed_weights(layers)
         if weights is None or weights[1][1][0].device != pos.device:
             return None
-        blocks = self.interaction_blocks
-        rc = self.rbf_layer.cutoff
-        rbf = self.rbf_layer
-        key = (training, id(weights), id(rbf), tuple(map(id, rbf._parameters.values())), tuple(map(id, rbf._buffers.values())),
-               getattr(rc, "cutoff_lower", None), getattr(rc, "cutoff_upper", None),
-               tuple((getattr(b.conv.cutoff, "cutoff_lower", None), getattr(b.conv.cutoff, "cutoff_upper", None), b.conv.filter_precision)
-                     for b in blocks))
+        key = (training, id(weights), layers.description())
         cached = self.__dict__.get("_mlcgb_setup")
         if cached is not None and cached[0] == key:
             return cached[1]
+        blocks = self.interaction_blocks
         specs = [b.conv.fused_spec(self.rbf_layer, training) for b in blocks]
         precisions = {FILTER_PRECISIONS[b.conv.filter_precision] for b in blocks}
         result = None
