@@ -2816,14 +2816,16 @@ struct HostSlot {
 };
 static thread_local HostSlot g_host_slot;
 
+// (acquire: the caller reads the other words of the line behind this; publish() has them out before the sequence number)
+static bool published(int64_t seq, const int64_t *slot) { return __atomic_load_n(slot, __ATOMIC_ACQUIRE) == seq; }
+
 static int wait_published(int64_t seq, const int64_t *slot, cudaStream_t st) {
-    const volatile int64_t *h = slot;
     for (uint64_t it = 1;; it++) {
-        if (h[0] == seq) return MLCGB_OK;
+        if (published(seq, slot)) return MLCGB_OK;
         if ((it & 4095) == 0) {                        // a stream that has stopped without publishing has failed
             const cudaError_t e = cudaStreamQuery(st);
             if (e == cudaErrorNotReady) continue;
-            if (e == cudaSuccess && h[0] == seq) return MLCGB_OK;
+            if (e == cudaSuccess && published(seq, slot)) return MLCGB_OK;
             g_last_cuda_error = (int)(e == cudaSuccess ? cudaErrorUnknown : e);
             cudaGetLastError();
             return MLCGB_E_LAUNCH;

@@ -72,3 +72,28 @@ def test_fixed_capacity(n, room):
     for k in ("row0", "row1", "twin", "pair_of"):
         assert torch.equal(res[k][:live], ref[k]), k
     assert torch.equal(res["sel"][:live // 2], ref["sel"])
+
+
+def test_counts_read_by_several_threads():
+    """Each host thread reads its own counts from the line that its graph's kernels write, on its own stream."""
+    from concurrent.futures import ThreadPoolExecutor
+    be = get_backend()
+    rng = np.random.default_rng(5)
+    work = []
+    for n in (50, 700, 3000, 41, 2100, 900):
+        pos = (rng.random((n, 3)) * n ** (1 / 3) * 2).astype(np.float32)
+        ptr = np.array([0, n // 2, n], dtype=np.int64)
+        work.append((torch.as_tensor(pos, device=DEV), torch.as_tensor(ptr, device=DEV), radius_ref.radius_graph_c(pos, ptr, 4.0, 1000, False, "cluster").shape[1]))
+    torch.cuda.synchronize()
+
+    def run(k):
+        stream, got = torch.cuda.Stream(), []
+        with torch.cuda.device(0), torch.cuda.stream(stream):
+            for i in range(60):
+                pos, ptr, want = work[(i * (k + 1) + k) % len(work)]
+                got.append(be.radius_graph(pos, ptr, 4.0, 1000, False, 1, want_plan=True)["edge_index"].shape[1] == want)
+        stream.synchronize()
+        return all(got)
+
+    with ThreadPoolExecutor(4) as pool:
+        assert all(pool.map(run, range(4)))
