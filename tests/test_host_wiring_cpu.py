@@ -264,6 +264,18 @@ def test_sumout_additivity(golden):
     assert torch.allclose(out.out["energy"], e, rtol=1e-6) and torch.allclose(out.out["forces"], f, rtol=1e-6)
 
 
+def test_kept_parameters_follow_the_strides():
+    """Bead types (or an index list) that are another view of the same memory, of the same shape, are another input."""
+    data, priors = prior_setup(10, 2, 3, torch.Generator().manual_seed(7))
+    storage = torch.randint(0, 3, (40,), generator=torch.Generator().manual_seed(8))
+    p = priors["bonds"].eval()
+    for types_ in (storage[:20], storage[::2]):
+        data.atom_types = types_
+        got = p(data).out["bonds"]["energy"].clone()
+        data.atom_types = types_.clone()
+        assert torch.equal(got, prior_setup(10, 2, 3, torch.Generator().manual_seed(7))[1]["bonds"].eval()(data).out["bonds"]["energy"])
+
+
 def test_copies_of_a_prior_start_without_its_kept_lists():
     import copy
     data, priors = prior_setup(12, 2, 3, torch.Generator().manual_seed(6))
