@@ -577,7 +577,7 @@ typedef struct {
     const int32_t *idx;
     const void *params;
     /* n_slices = 0, or a symmetric list once more in slices of 32 runs of terms that share their first bead (idx and params are then
-       not read).  slices [n_slices][4] = {first step, steps, base, span}; slice_beads [n_slices][32] = first bead of each run (~bead:
+       not read and may be NULL).  slices [n_slices][4] = {first step, steps, base, span}; slice_beads [n_slices][32] = first bead of each run (~bead:
        none, the lane adds nothing); offsets [steps][32][4] = second bead minus the slice's base, at most its span; slice_params
        [n_params][steps][32][4], all 0 where a run has no term (offsets then name a bead that is not the first one). */
     int64_t n_slices, steps;

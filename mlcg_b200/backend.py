@@ -1032,8 +1032,8 @@ class CudaBackend:
 
     def prior_eval(self, lists, pos, batch, B, deterministic=True, forces=False, totals=False):
         """Every prior list of a model in one call.  ``lists``: sequence of ``(kind, idx32 [order, M], params [P, M], symmetric,
-        sliced | None)`` (at most ``_lib.MAX_PRIOR_SEGMENTS``; ``sliced``: ``(slices, beads, offsets, params)`` of a symmetric pair list,
-        as ``mlcgb_prior_list`` describes them).  Returns ``(energy [n, B], dE/dpos [n, N, 3])``, one row / block
+        None)``, or ``(kind, None, None, True, (slices, beads, offsets, params))`` for a symmetric pair list in slices as
+        ``mlcgb_prior_list`` describes them (at most ``_lib.MAX_PRIOR_SEGMENTS``).  Returns ``(energy [n, B], dE/dpos [n, N, 3])``, one row / block
         per list (``forces``: the negative gradient), and with ``totals`` their sums ``(energy [B], gradient [N, 3])`` over the lists.
         ``deterministic``: sums formed as 64-bit fixed-point integers (bit-identical from run to run)."""
         _need_cuda(pos, batch)
@@ -1048,20 +1048,26 @@ class CudaBackend:
         keep = []
         M_total = moved = 0
         for k, (kind, idx, params, symmetric, sliced) in enumerate(lists):
-            _need_cuda(idx, params)
-            if idx.dtype != torch.int32 or params.dtype != pos.dtype:
-                raise TypeError("prior lists take int32 indices and parameters of the positions' dtype")
-            idx, params = idx.contiguous(), params.contiguous()
-            M = idx.shape[1]
-            keep += [idx, params]
             a = arr[k]
-            a.kind, a.n_params, a.symmetric, a.M, a.idx, a.params = kind, params.shape[0], bool(symmetric), M, idx.data_ptr(), params.data_ptr()
             if sliced is not None:
-                slices, beads, offsets, slice_params = sliced
+                slices, beads, offsets, params = sliced
+                _need_cuda(*sliced)
+                M, per_term = offsets.shape[0] * 128, 2
                 a.n_slices, a.steps, a.slices, a.slice_beads = slices.shape[0], offsets.shape[0], slices.data_ptr(), beads.data_ptr()
-                a.offsets, a.slice_params = offsets.data_ptr(), slice_params.data_ptr()
+                a.offsets, a.slice_params = offsets.data_ptr(), params.data_ptr()
+            else:
+                _need_cuda(idx, params)
+                if idx.dtype != torch.int32:
+                    raise TypeError("prior lists take int32 indices")
+                idx, params = idx.contiguous(), params.contiguous()
+                M, per_term = idx.shape[1], 4 * idx.shape[0]
+                keep += [idx, params]
+                a.idx, a.params = idx.data_ptr(), params.data_ptr()
+            if params.dtype != pos.dtype:
+                raise TypeError("prior lists take parameters of the positions' dtype")
+            a.kind, a.n_params, a.symmetric, a.M = kind, params.shape[0], bool(symmetric), M
             M_total += M
-            moved += M * (params.shape[0] * pos.element_size() + (2 if sliced is not None else 4 * idx.shape[0]))
+            moved += M * (params.shape[0] * pos.element_size() + per_term)
         rows = n + 1 if totals else n
         buf = torch.empty(rows * (3 * N + B), dtype=pos.dtype, device=dev)
         grad, energy = buf[: rows * 3 * N].view(rows, N, 3), buf[rows * 3 * N:].view(rows, B)

@@ -648,7 +648,6 @@ extern "C" int mlcgb_prior_eval(int n_lists, const mlcgb_prior_list *lists, cons
         const mlcgb_prior_list &l = lists[i];
         const int need = l.kind == 3 ? 1 : (l.kind == 2 ? 3 : 2);
         if (l.kind < 0 || l.kind > 3 || l.M < 0 || l.n_params < need || (l.kind == 2 && (l.n_params - 1) % 2 != 0)) return MLCGB_E_ARG;
-        if (l.M > 0 && (!l.idx || !l.params)) return MLCGB_E_ARG;
         seg.kind[i] = l.kind;
         seg.n_params[i] = l.n_params;
         seg.symmetric[i] = (l.kind == 0 || l.kind == 3) && l.symmetric ? 1 : 0;
@@ -656,6 +655,7 @@ extern "C" int mlcgb_prior_eval(int n_lists, const mlcgb_prior_list *lists, cons
         seg.idx[i] = l.idx;
         seg.params[i] = l.params;
         const bool sliced = seg.symmetric[i] && l.n_slices > 0;
+        if (l.M > 0 && !sliced && (!l.idx || !l.params)) return MLCGB_E_ARG;
         if (sliced) {
             if (!l.slices || !l.slice_beads || !l.offsets || !l.slice_params || l.steps <= 0 || l.n_slices >= ((int64_t)1 << 31)) return MLCGB_E_ARG;
             if (((uintptr_t)l.slices | (uintptr_t)l.offsets | (uintptr_t)l.slice_params) & 31) return MLCGB_E_ARG;

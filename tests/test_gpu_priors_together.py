@@ -42,6 +42,26 @@ def test_forces_and_totals(n, B, dtype):
         assert float((forces.double() - f_sum).abs().max()) <= tol * (1 + float(f_sum.abs().max()))
 
 
+def test_a_sliced_list_is_kept_once():
+    """The slices of a pair list take the place of the 32-bit list and of the gathered parameters: 6 bytes a term and the padding."""
+    data, priors = prior_setup(150, 20, 4, torch.Generator().manual_seed(3))
+    gen = torch.Generator().manual_seed(3)      # (beads that do not overlap, as above)
+    data.pos = torch.cat([random_walk_chain(150, gen, min_dist=3.0) for _ in range(20)]).float()
+    p = priors["repulsion"]
+    with torch.no_grad():
+        p.sigma.copy_(0.5 * (p.sigma + p.sigma.t()))
+    data, p = data.to(DEV), p.to(DEV).eval()
+    M = data.neighbor_list["repulsion"]["index_mapping"].shape[1]
+    before = torch.cuda.memory_allocated()
+    assert p._cached_list(data)[4] is not None
+    kept = torch.cuda.memory_allocated() - before
+    assert 6 * M <= kept <= 1.3 * 6 * M
+    together, alone = _evaluate_together([p], data, forces=True)[0]["repulsion"], bnn.GradientsOut(p, "forces").eval()(data).out["repulsion"]
+    # (float32 sums of up to 300 terms in two orders: the bar of the test above, on both sides)
+    assert torch.allclose(together[0], alone["energy"], rtol=2e-5, atol=2e-5)
+    assert float((together[1] - alone["forces"]).abs().max()) <= 2e-5 * (1 + float(alone["forces"].abs().max()))
+
+
 def test_pair_slices_of_beads_that_lie_far_apart():
     near = torch.arange(9, device=DEV, dtype=torch.int32)
     pairs = torch.stack([torch.zeros_like(near), near + 65535 - 8] ).repeat(1, 20)
