@@ -345,16 +345,8 @@ int mlcgb_row_dot(const void *a /* [E,F] */, const void *b /* [E,F] */, int dtyp
  * respect to y: the second-order pass of force matching).  G is ignored in mode 0. */
 int mlcgb_tanh_grad(int mode, const void *G, const void *g, const void *y, int dtype, int64_t n, void *out, void *stream);
 
-/* Filter rows and their distance derivatives in one launch, one row per unordered pair (sel[P]: the pair's edge): W[p,:] as
- * mlcgb_filter_forward gives it, Wd[p,:] = dW/dd.  rows_dev: NULL or the live row count in device memory.  h_save / z_save
- * (mlcgb_filter_hidden_bytes(P) bytes each, or NULL): the hidden layer and z' = phi'(d) A1^T, kept for mlcgb_filter_weight_grad, and
- * zmax, one float that is zero before, the largest |z'|. */
-int mlcgb_filter_value_derivative(const void *d, int64_t P, const int64_t *rows_dev, const int32_t *sel, const mlcgb_rbf_spec *rbf,
-                                  int conv_cutoff_kind, double conv_lower, double conv_upper, const void *A1, const void *b1,
-                                  const void *A2, int64_t F, int precision, void *W, void *Wd, void *h_save, void *z_save,
-                                  void *zmax, int32_t *status, void *stream);
-
-/* Aggregations over such rows (float32, F = 128, symmetric centre-sorted list ptr / nbr with its pair index):
+/* Aggregations over filter rows W [P,F], one per unordered pair, and their distance derivatives Wd = dW/dd (float32, F = 128,
+ * symmetric centre-sorted list ptr / nbr with its pair index pair_of):
  *   seg_force:    out[i] = sum_j a[j] W[p] (out NULL: not wanted),  s[e] = (accumulate ? s[e] : 0) + sum_f (x[i] a[j] Wd[p])_f
  *   seg_tangent:  out[i] = sum_j a[j] W[p] + b[j] (dd[e] Wd[p])   (a NULL: zero)
  *   edge_tangent: dd[e] = change of the distance of edge e when the positions move along v */
@@ -362,16 +354,6 @@ int mlcgb_seg_force(const void *a, const void *x, const void *W, const void *Wd,
                     int64_t N, int64_t F, void *out, void *s, int accumulate, void *stream);
 int mlcgb_seg_tangent(const void *a, const void *b, const void *W, const void *Wd, const void *dd, const int64_t *ptr, const int32_t *nbr,
                       const int32_t *pair_of, int64_t N, int64_t F, void *out, void *stream);
-/* Weight gradients of the filter network of one block from the second-order pass of force matching (the derivative of
- * src/mlcg/nn/gradients.py:216-222 with respect to the parameters): partial sums of dA2 [F,F] | dA1 [F,R] | db1 [F], one set per CTA
- * (mlcgb_filter_weight_grad_parts(P) of them, F F + F R + F floats each), to be added in order.  dd: distance tangents; xl / xt:
- * features gathered by the aggregation and their tangent (NULL: zero); agb / gagg: gradients of the aggregate and of its tangent. */
-int64_t mlcgb_filter_weight_grad_parts(int64_t P);
-int mlcgb_filter_weight_grad(const void *d, const void *dd, int64_t P, const int32_t *sel, const int32_t *row0, const int32_t *row1,
-                             const mlcgb_rbf_spec *rbf, int conv_cutoff_kind, double conv_lower, double conv_upper, const void *A2, int64_t F,
-                             const void *h_saved, const void *z_saved, const void *zmax, const void *xl, const void *xt, const void *gagg,
-                             const void *agb, void *partial, int32_t *status, void *stream);
-
 int mlcgb_edge_tangent(const void *pos, const void *v, const void *d, const int32_t *row0, const int32_t *row1, int64_t E, int negate, void *dd,
                        void *stream);
 

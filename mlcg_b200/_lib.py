@@ -122,10 +122,6 @@ SIGNATURES = {
                                      c_vp]),
     "mlcgb_filter_backward": (c_int, [c_vp, c_i64, c_vp, c_vp, ctypes.POINTER(RbfSpecStruct), c_int, c_dbl, c_dbl, c_vp, c_vp, c_vp, c_i64, c_int,
                                       c_vp, c_vp, c_vp, c_vp, c_i64, c_vp, c_vp, c_vp, c_vp]),
-    "mlcgb_filter_value_derivative": (c_int, [c_vp, c_i64, c_vp, c_vp, ctypes.POINTER(RbfSpecStruct), c_int, c_dbl, c_dbl, c_vp, c_vp, c_vp, c_i64, c_int,
-                                              c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
-    "mlcgb_filter_weight_grad_parts": (c_i64, [c_i64]),
-    "mlcgb_filter_weight_grad": (c_int, [c_vp, c_vp, c_i64, c_vp, c_vp, c_vp, ctypes.POINTER(RbfSpecStruct), c_int, c_dbl, c_dbl, c_vp, c_i64] + [c_vp] * 10),
     "mlcgb_gemm_tc_chain2_tangent": (c_int, [c_int] + [c_vp] * 6 + [c_i64] + [c_vp] * 5),
     "mlcgb_schnet_train_workspace_bytes": (c_sz, [c_int] + [c_i64] * 7),
     "mlcgb_schnet_train_forward": (c_int, [c_vp] * 3 + [c_i64, c_i64] + [c_vp] * 6 + [c_i64, c_i64, c_vp, c_int, c_dbl, c_dbl, c_vp, c_int, c_vp, c_sz] + [c_vp] * 4),

@@ -421,18 +421,3 @@ int filter_vd_blocks(const float *d, int64_t P, const int64_t *rows_dev, const i
 }
 
 }  // namespace mlcgb
-
-using namespace mlcgb;
-
-extern "C" int mlcgb_filter_value_derivative(const void *d, int64_t P, const int64_t *rows_dev, const int32_t *sel, const mlcgb_rbf_spec *rbf,
-                                             int conv_cutoff_kind, double conv_lower, double conv_upper, const void *A1, const void *b1,
-                                             const void *A2, int64_t F, int precision, void *W, void *Wd, void *h_save, void *z_save, void *zmax,
-                                             int32_t *status, void *stream) {
-    if (F != kF) return MLCGB_E_LIMIT;
-    mlcgb_schnet_block block = {};
-    block.filter_w1 = A1;
-    block.filter_b1 = b1;
-    block.filter_w2 = A2;
-    return filter_vd_blocks((const float *)d, P, rows_dev, sel, rbf, conv_cutoff_kind, conv_lower, conv_upper, &block, 1, precision, (float *)W, (float *)Wd,
-                            (float *)h_save, (float *)z_save, (float *)zmax, status, (cudaStream_t)stream);
-}

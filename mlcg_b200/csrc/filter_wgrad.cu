@@ -438,21 +438,3 @@ int filter_wgrad_blocks(const float *d, const float *dd, int64_t P, const int32_
 }
 
 }  // namespace mlcgb
-
-using namespace mlcgb;
-
-extern "C" {
-
-int64_t mlcgb_filter_weight_grad_parts(int64_t P) { return filter_wgrad_parts(P, 1); }
-
-int mlcgb_filter_weight_grad(const void *d, const void *dd, int64_t P, const int32_t *sel, const int32_t *row0, const int32_t *row1,
-                             const mlcgb_rbf_spec *rbf, int conv_cutoff_kind, double conv_lower, double conv_upper, const void *A2, int64_t F,
-                             const void *h_saved, const void *z_saved, const void *zmax, const void *xl, const void *xt, const void *gagg,
-                             const void *agb, void *partial, int32_t *status, void *stream) {
-    if (F != kF) return MLCGB_E_LIMIT;
-    const FilterGradBlock block = {(const float *)A2, (const float *)xl, (const float *)xt, (const float *)gagg, (const float *)agb};
-    return filter_wgrad_blocks((const float *)d, (const float *)dd, P, sel, row0, row1, rbf, conv_cutoff_kind, conv_lower, conv_upper, &block, 1,
-                               (const float *)h_saved, (const float *)z_saved, (const float *)zmax, (float *)partial, status, (cudaStream_t)stream);
-}
-
-}  // extern "C"

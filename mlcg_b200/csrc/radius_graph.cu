@@ -1866,10 +1866,9 @@ __global__ void struct_of_kernel(const int64_t *__restrict__ ptr, int64_t B, int
         for (int64_t i = ptr[b] + threadIdx.x; i < ptr[b + 1]; i += blockDim.x) struct_of[i] = (int32_t)b;
 }
 
-// parts: kPartScan: the scan of the degrees follows the count
-enum { kPartScan = 1 };
+// scan: the scan of the degrees follows the count
 template <typename T>
-static int radius_launch(int parts, bool fill, const void *pos_, const int64_t *ptr, int64_t N, int64_t B, double r, int64_t max_nn,
+static int radius_launch(bool scan, bool fill, const void *pos_, const int64_t *ptr, int64_t N, int64_t B, double r, int64_t max_nn,
                          int loop, int rule, void *ws, size_t ws_bytes, int dtype, int32_t *deg, int64_t *offsets,
                          FillOut out, int32_t *status, cudaStream_t st, Exclusion ex = Exclusion{}, int brute_max = kBruteMax, int brute_tile = 0, int32_t *upper = nullptr) {
     const WsLayout L = ws_layout(N, B, dtype);
@@ -1911,7 +1910,7 @@ static int radius_launch(int parts, bool fill, const void *pos_, const int64_t *
         else
             neighbours_kernel<T, false, false><<<nbr_grid, kNbrWarps * 32, 0, st>>>(pos, ptr, N, B, r2, max_nn, loop, rule, spos, cellparam,
                                                                                     cell_of, cell_start, struct_of, deg, nullptr, out, ex, status, n_plain, upper);
-        if (parts & kPartScan) launch_scan(deg, N, bsum, offsets, st);
+        if (scan) launch_scan(deg, N, bsum, offsets, st);
     } else {
         if (tiles) {
             int grid = 0;
@@ -1966,7 +1965,7 @@ static int radius_count_impl(const void *pos, int dtype, const int64_t *ptr, int
     }
     if (!pos || !deg || B == 0) return MLCGB_E_ARG;
     return MLCGB_DISPATCH_DTYPE(dtype, [&] {
-        return radius_launch<scalar_t>(kPartScan, false, pos, ptr, N, B, r, max_nn, loop, rule, workspace, workspace_bytes, dtype, deg,
+        return radius_launch<scalar_t>(true, false, pos, ptr, N, B, r, max_nn, loop, rule, workspace, workspace_bytes, dtype, deg,
                                        offsets, FillOut{}, status, (cudaStream_t)stream, ex);
     });
 }
@@ -1998,7 +1997,7 @@ static int radius_fill_impl(const void *pos, int dtype, const int64_t *ptr, int6
     if (!pos || !edge_index) return MLCGB_E_ARG;
     FillOut out{edge_index, edge_index + E, mapping_batch, distance, row0_i32, row1_i32};
     return MLCGB_DISPATCH_DTYPE(dtype, [&] {
-        return radius_launch<scalar_t>(kPartScan, true, pos, ptr, N, B, r, 0, loop, 0, const_cast<void *>(workspace), workspace_bytes, dtype,
+        return radius_launch<scalar_t>(true, true, pos, ptr, N, B, r, 0, loop, 0, const_cast<void *>(workspace), workspace_bytes, dtype,
                                        nullptr, const_cast<int64_t *>(offsets), out, status, (cudaStream_t)stream, ex);
     });
 }
@@ -2172,7 +2171,7 @@ extern "C" int mlcgb_radius_graph_capacity(const void *pos, int dtype, const int
     if (capacity == 0) return check_launch();
     FillOut out{edge_index, edge_index ? edge_index + capacity : nullptr, nullptr, nullptr, row0_i32, row1_i32};
     return MLCGB_DISPATCH_DTYPE(dtype, [&] {
-        return radius_launch<scalar_t>(kPartScan, true, pos, ptr, N, B, r, 0, loop, 0, workspace, workspace_bytes, dtype, nullptr, offsets, out, status,
+        return radius_launch<scalar_t>(true, true, pos, ptr, N, B, r, 0, loop, 0, workspace, workspace_bytes, dtype, nullptr, offsets, out, status,
                                        st);
     });
 }
@@ -2205,7 +2204,7 @@ extern "C" int mlcgb_radius_graph_static(const void *pos, int dtype, const int64
     // rows of the caller's [2, capacity] buffer
     FillOut out{edge_index, edge_index + capacity, nullptr, nullptr, nullptr, nullptr};
     return MLCGB_DISPATCH_DTYPE(dtype, [&] {
-        return radius_launch<scalar_t>(kPartScan, true, pos, ptr, N, B, r, 0, loop, 0, scratch, kStaticScratchBytes, dtype, nullptr, offsets, out,
+        return radius_launch<scalar_t>(true, true, pos, ptr, N, B, r, 0, loop, 0, scratch, kStaticScratchBytes, dtype, nullptr, offsets, out,
                                        status, st);
     });
 }
@@ -2884,7 +2883,7 @@ int mlcgb_graph_begin(const void *pos, int dtype, const int64_t *n_atoms, int64_
         const WsLayout W = ws_layout(N, B, dtype);
         char *cw = w + L.cells;
         auto *deg = (int32_t *)(w + L.deg), *upper = (int32_t *)(w + L.upper), *status = (int32_t *)(w + L.header);
-        const int rl = radius_launch<scalar_t>(0, false, pos, ptr, N, B, r, max_nn, loop, rule, cw, W.total, dtype, deg, offsets, FillOut{}, status, st, ex,
+        const int rl = radius_launch<scalar_t>(false, false, pos, ptr, N, B, r, max_nn, loop, rule, cw, W.total, dtype, deg, offsets, FillOut{}, status, st, ex,
                                                rows ? kMaskMax : kBruteMax, rows ? 2 : 0, upper);
         if (rl) return rl;
         if (rows) mask_rows_kernel<scalar_t><<<grid_for((N + 3) / 4 * 32, 256), 256, 0, st>>>(
@@ -2931,7 +2930,7 @@ int mlcgb_graph_finish(const void *pos, int dtype, const int64_t *ptr, int64_t N
         const auto *cellparam = (const CellParam *)(cw + W.cellparam);
         const auto *seg = (const int4 *)(w + L.seg);
         if (cells) {
-            const int rl = radius_launch<scalar_t>(0, true, pos, ptr, N, B, r, 0, loop, 0, cw, W.total, dtype, nullptr, const_cast<int64_t *>(offsets), out,
+            const int rl = radius_launch<scalar_t>(false, true, pos, ptr, N, B, r, 0, loop, 0, cw, W.total, dtype, nullptr, const_cast<int64_t *>(offsets), out,
                                                    (int32_t *)(w + L.header), st, ex, rows ? kMaskMax : kBruteMax, rows ? 2 : 0);
             if (rl) return rl;
             if (twin && ((uintptr_t)row1 & 31) != 0) {
