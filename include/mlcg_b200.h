@@ -40,6 +40,13 @@ extern "C" {
 
 const char *mlcgb_strerror(int code);
 int mlcgb_last_cuda_error(void); /* cudaError_t of the last failed launch on this host thread */
+/* MLCGB_VERSION of the library.  The hundreds move when an entry point that existed before takes other arguments or means something
+ * else (or is gone); a binding checks them.  Since 101:
+ *   200  mlcgb_prior_list: run_ptr, n_runs gone, the slice fields new.  mlcgb_prior_eval: the int32 struct_of became batch (int64 or
+ *        NULL), negate and the totals are new, fixed_point = 0 writes its outputs too (it added to them), the workspace is wanted in
+ *        both modes and mlcgb_prior_eval_workspace_bytes takes the dtype where it took fixed_point.  mlcgb_gemm_tc_chain2 with
+ *        backward = 1 writes mid_out unless it is NULL. */
+#define MLCGB_VERSION 200
 int mlcgb_version(void);
 
 /* Device time per entry point, without a profiler.  No counterpart in the reference (mlcg times whole steps on the host).

@@ -44,6 +44,7 @@ class PriorListStruct(ctypes.Structure):
 
 
 MAX_PRIOR_SEGMENTS = 8
+VERSION = 200                  # MLCGB_VERSION of the header that the tables below follow
 EVALUATE_DONE, EVALUATE_MORE = 1, 2
 
 # name -> (restype, argtypes); one entry per symbol declared in include/mlcg_b200.h
@@ -164,6 +165,9 @@ def load():
     for name, (res, args) in SIGNATURES.items():
         fn = getattr(lib, name)  # AttributeError here means header and library disagree
         fn.restype, fn.argtypes = res, args
+    if lib.mlcgb_version() // 100 != VERSION // 100:
+        _load_error = f"{LIB_PATH} has interface version {lib.mlcgb_version()}, this binding is written for {VERSION}; rebuild it"
+        raise ExtensionMissing(_load_error)
     _lib = lib
     return lib
 

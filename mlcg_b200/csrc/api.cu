@@ -72,7 +72,7 @@ const char *mlcgb_strerror(int code) {
 
 int mlcgb_last_cuda_error(void) { return mlcgb::g_last_cuda_error; }
 
-int mlcgb_version(void) { return 101; }
+int mlcgb_version(void) { return MLCGB_VERSION; }
 
 int mlcgb_timeline_begin(void) {
     mlcgb::Timeline &t = mlcgb::g_timeline;

@@ -37,7 +37,19 @@ def test_library_exports_every_declared_symbol():
         assert hasattr(lib, name), name
     lib.mlcgb_strerror.restype = ctypes.c_char_p
     assert lib.mlcgb_strerror(0) == b"ok" and b"workspace" in lib.mlcgb_strerror(-2)
-    assert lib.mlcgb_version() >= 100
+    header = open(os.path.join(ROOT, "include", "mlcg_b200.h")).read()
+    assert lib.mlcgb_version() == _lib.VERSION == int(re.search(r"#define MLCGB_VERSION (\d+)", header).group(1))
+
+
+def test_a_library_of_another_interface_is_refused(monkeypatch):
+    """Entry points keep their names when their arguments change: the version is what tells a binding."""
+    lib = _lib.load()
+    monkeypatch.setattr(_lib, "_lib", None)
+    monkeypatch.setattr(_lib, "VERSION", _lib.VERSION - 100)
+    with pytest.raises(_lib.ExtensionMissing, match="interface version"):
+        _lib.load()
+    monkeypatch.undo()
+    assert _lib.load() is lib
 
 
 def test_workspace_size_queries_are_host_only():
