@@ -544,7 +544,7 @@ def training_step_measurement(dev, world, steps=10, warmup=3):
     walk, 20 types), SchNet 3 blocks / 128 / 128 exp-normal functions / 10 A, ``model.train()`` so that the force pass keeps its graph,
     MSE on forces against N(0,1) targets, gradient all-reduce over the ranks (NCCL; mean), AdamW(lr 1e-4, weight decay 0) — the step
     of src/mlcg/pl/model.py:113-131 under examples/input_yamls/slurm_example/train.yaml:9.  Returns this rank's
-    (ms per step, ms in the all-reduce per step, last loss)."""
+    (ms per step: mean, median, least and most; ms in the all-reduce per step, last loss, ...)."""
     import mlcg_b200
     from mlcg_b200 import nn as bnn
     from mlcg_b200.distributed import allreduce_gradients
@@ -580,16 +580,18 @@ def training_step_measurement(dev, world, steps=10, warmup=3):
     for _ in range(warmup):
         step(False)
     torch.cuda.synchronize()
-    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    a.record()
-    for _ in range(steps):
+    marks = [torch.cuda.Event(enable_timing=True) for _ in range(steps + 1)]
+    marks[0].record()
+    for k in range(steps):
         loss = step(True)
-    b.record()
+        marks[k + 1].record()
     torch.cuda.synchronize()
     from mlcg_b200.backend import get_backend
     get_backend().check_pending()
     ar_ms = sum(x.elapsed_time(y) for x, y in ar_events) / steps if ar_events else 0.0
-    return a.elapsed_time(b) / steps, ar_ms, float(loss.detach()), B, sum(p.numel() for p in params)
+    each = sorted(x.elapsed_time(y) for x, y in zip(marks, marks[1:]))
+    times = dict(mean=marks[0].elapsed_time(marks[-1]) / steps, median=each[steps // 2], least=each[0], most=each[-1])
+    return times, ar_ms, float(loss.detach()), B, sum(p.numel() for p in params)
 
 
 def training_cpu_leg(arm, steps=2):
@@ -822,14 +824,14 @@ def run_ours(args):
         torch.cuda.empty_cache()
         bnn.set_edge_capacity(model, None)
         tr_ms, ar_ms, tr_loss, tr_B, n_params = training_step_measurement(dev, world)
-        tt = torch.tensor([tr_ms, ar_ms], dtype=torch.float64, device=dev)
+        tt = torch.tensor([tr_ms["mean"], ar_ms, tr_ms["median"], tr_ms["least"], tr_ms["most"]], dtype=torch.float64, device=dev)
         if world > 1:
             dist.all_reduce(tt, op=dist.ReduceOp.MAX)
-        training = dict(ms_per_step=float(tt[0]), structures_per_s=world * tr_B / (float(tt[0]) / 1e3), allreduce_ms_per_step=float(tt[1]),
-                        allreduce_bytes=4 * n_params, structures_per_gpu=tr_B, n_gpus=world, loss=tr_loss,
+        training = dict(ms_per_step=float(tt[0]), ms_median=float(tt[2]), ms_least=float(tt[3]), ms_most=float(tt[4]),
+                        structures_per_s=world * tr_B / (float(tt[0]) / 1e3), allreduce_ms_per_step=float(tt[1]), allreduce_bytes=4 * n_params, structures_per_gpu=tr_B, n_gpus=world, loss=tr_loss,
                         note="256 structures x 73 beads per GPU, SchNet 3 blocks / 128 / 128 expnorm / 10 A, train mode (second-order pass), "
-                             "MSE on forces, gradient all-reduce (mean) over the ranks, AdamW(1e-4); 10 steps after 3 warm-ups, CUDA events, "
-                             "maximum over ranks")
+                             "MSE on forces, gradient all-reduce (mean) over the ranks, AdamW(1e-4); 10 steps after 3 warm-ups, CUDA events (mean, "
+                             "and median, least and most of the steps), maximum over ranks")
         flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
         bnn.set_edge_capacity(model, int(1.1 * n_edges))
     # the ranks part here: everything below is rank 0's own reporting (no collective may follow)
@@ -995,7 +997,8 @@ def run_only(args):
         rec = measure_priors_and_dynamics(dev, hbm_peak, arm, dynamics=args.only == "dynamics")
     else:
         ms, ar, loss, B, n_params = training_step_measurement(dev, 1, steps=max(args.steps, 1) if args.steps != 50 else 10, warmup=max(args.warmup, 1) if args.warmup != 10 else 3)
-        rec = {"training_step_256x73": dict(ms_per_step=ms, structures_per_s=B / (ms / 1e3), loss=loss, parameters=n_params)}
+        rec = {"training_step_256x73": dict(ms_per_step=ms["mean"], ms_median=ms["median"], ms_least=ms["least"], ms_most=ms["most"],
+                                            structures_per_s=B / (ms["mean"] / 1e3), loss=loss, parameters=n_params)}
     print(json.dumps(rec))
 
 
