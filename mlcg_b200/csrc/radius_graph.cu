@@ -2224,8 +2224,15 @@ namespace mlcgb {
 constexpr int64_t kMaskNodes = 2048;
 constexpr int kMaskStructs = 2048;             // structure boundaries held in shared memory
 
-// larger batches whose structures have at most 768 points on average: those that do go the same way (mask_rows_kernel); in a batch of
-// large structures the bit rows (192 bytes per point) would be room for nothing
+// Larger batches whose structures have at most 768 points on average: those that do go the same way (mask_rows_kernel); in a batch of
+// large structures the bit rows (192 bytes per point) would be room for nothing.  Graph and plan of 40 000 points in structures of
+// one size, us, bit rows : cells,
+//   points            400        576        768       1024
+//   uniform, 10 A     117 : 165  135 : 161  154 : 157  173 : 168
+//   chains, 12 A       85 : 210   89 : 184   93 : 229   98 : 211
+//   chains, 15 A, f64  93 : 198   99 : 498  105 : 993  116 : 1257
+// In a uniform cube the two meet at the limit; chains, which crowd few cells of their grid, would still gain up to the 1024 points that
+// a warp's row of bits can hold.
 constexpr int kMaskWordsPerRow = 24;
 static inline bool mask_rows_route(int64_t N, int64_t B) { return N > kMaskNodes && N <= 32 * kMaskWordsPerRow * B; }
 

@@ -12,7 +12,7 @@
 // memory before the kernel waits for its predecessor.  A 128-column layer over 8 rows is 1300 issue slots per scheduler (four
 // k-ranges by 128 columns; partial sums through shared memory).  Launches per evaluation of L blocks: 2 L + 3 where the tensor-core
 // sequence takes 7 L + 7; one evaluation of 64 x 10 beads, two blocks: 154 us of kernels before.
-// Above kSmallNodes the rows per SM make the tensor-core kernels the faster ones.
+// For many more rows per SM the tensor-core kernels are the faster ones (figures at kSmallNodes).
 #include "schnet_internal.cuh"
 #include "tc_common.cuh"
 
