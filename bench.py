@@ -442,13 +442,14 @@ def measure_priors_and_dynamics(dev, hbm_peak, arm, seed=2, dynamics=True):
     data = mlcg_b200.AtomicData(pos=ppos.clone(), atom_types=types5_h.to(dev), batch=torch.arange(Bp, device=dev).repeat_interleave(npb),
                                 n_atoms=torch.full((Bp,), npb, device=dev), neighbor_list=nls)
     M_all = sum(int(m.shape[1]) for m, _ in lists.values())
-    moved = sum(int(m.numel()) * 4 + int(m.shape[1]) * 4 * n_par[name] for name, (m, _) in lists.items()) + 2 * ppos.numel() * 4
+    # (repulsion in slices: a 16-bit offset and a parameter per term; the others four bytes per index and parameter)
+    moved = sum(int(m.shape[1]) * (6 if name == "repulsion" else 4 * (m.shape[0] + n_par[name])) for name, (m, _) in lists.items()) + 2 * ppos.numel() * 4
     for mode, flag in (("fixed_point", True), ("float_atomics", False)):
         bnn.set_prior_determinism(flag)
         ms = time_cuda(lambda: bnn.evaluate_priors(list(pri.values()), data), iters=5, warm=2)
         out[f"priors_together_1024x268_{mode}"] = dict(terms=M_all, ms=ms, terms_per_s=M_all / (ms / 1e3), moved_GBps=moved / ms / 1e6,
                                                         frac_of_hbm=moved / ms / 1e6 / hbm_peak,
-                                                        note="bonds + angles + dihedrals + repulsion in one launch; bytes moved: int32 indices, "
+                                                        note="bonds + angles + dihedrals + repulsion in one call; bytes moved: the lists as they are kept, "
                                                              "float32 per-term parameters, positions in, gradients out")
     bnn.set_prior_determinism(True)
     if not dynamics:
@@ -667,6 +668,11 @@ def kernel_work(name, E, P, N, F, R):
         return P * (8 * F + 4), 4 * E * F * (R + F)
     if name == "seg_mul_sum":           # one filter row per pair, neighbour index and pair index per edge, node rows in and out
         return P * F * 4 + 8 * E + 2 * N * F * 4 + 8 * N, 2 * E * F
+    if name == "seg_force":             # mean of its launches: a filter and a derivative row per pair (the first block's dot product: the latter
+        #                                 alone), two indices and a dot product per edge (read too where it adds), two node rows in, one out
+        L = WORKLOAD["interactions"]
+        rows, nodes, dots = (2 * L - 1) / L, (3 * L - 1) / L, (2 * L - 1) / L
+        return rows * P * F * 4 + (8 + 4 * dots) * E + nodes * N * F * 4 + 8 * N, (4 * L - 2) / L * E * F
     if name.startswith("gemm_tc"):      # node-sized Linear layers, 128 wide
         return (2 * N * F + F * F) * 4, 2 * N * F * F
     if name == "radius_graph_capacity":
