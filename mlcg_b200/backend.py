@@ -124,9 +124,17 @@ def _on(device):
 
 
 def _need_cuda(*ts):
+    """Every tensor whose address a kernel gets is on the device of the first one."""
+    device = None
     for t in ts:
-        if t is not None and not t.is_cuda:
+        if t is None:
+            continue
+        if not t.is_cuda:
             raise RuntimeError("mlcg_b200 operators run on CUDA tensors only (there is no CPU fallback)")
+        if device is None:
+            device = t.get_device()
+        elif t.get_device() != device:
+            raise RuntimeError(f"mlcg_b200: tensors on different devices (cuda:{device} and {t.device})")
 
 
 def _raise_for_status(word: int, what: str) -> None:
@@ -795,6 +803,7 @@ class CudaBackend:
         """Energies [B] and d(sum of energies)/d(pos) [N,3] (its negative with ``forces``) of a standard SchNet in one library call.  ``weights`` is what
         :func:`mlcg_b200.nn.schnet.packed_weights` returns: ``(SchnetWeightsStruct, keep-alive objects)``.  ``counts``: the
         device-side (edges, pairs) of a fixed-capacity graph, whose plan is sized by the capacity."""
+        _need_cuda(pos, types, struct_ptr, plan.row0)
         wstruct, _keep = weights
         N, dev = pos.shape[0], pos.device
         B = struct_ptr.numel() - 1
@@ -821,6 +830,7 @@ class CudaBackend:
         [N,3], edge count, None)``; None for a list without edges or cut short.  ``n_atoms`` or ``ptr`` (the other None); ``edges``: a
         guess at the edge count that sizes the workspace (too low costs a second call).  ``training``: the forward pass of
         :meth:`schnet_train_forward` (forces), its state as the last value."""
+        _need_cuda(pos, types, n_atoms, ptr)
         w, _keep = weights
         pos = pos.detach().contiguous()
         N, dev = pos.shape[0], pos.device
@@ -870,6 +880,7 @@ class CudaBackend:
 
     def schnet_train_forward(self, pos, types, struct_ptr, plan, spec: RbfSpec, conv_cut, weights):
         """(energies [B], forces [N,3], state for :meth:`schnet_train_backward`) of a standard SchNet on a given edge plan."""
+        _need_cuda(pos, types, struct_ptr, plan.row0)
         wstruct, _keep = weights
         pos = pos.detach().contiguous()
         N, B, dev = pos.shape[0], struct_ptr.numel() - 1, pos.device
@@ -1009,6 +1020,7 @@ class CudaBackend:
         """The slices of a pair list (int32 [2, M], runs of equal first bead from ``starts`` on) as ``mlcgb_prior_list`` takes them:
         ``(slices, beads, offsets, params)``; None where the second beads of a slice lie too far apart or ``worth(slots)`` says that
         the padding takes too many (``slots``: those of lanes with a run)."""
+        _need_cuda(idx, params, starts)
         idx, params, starts = idx.contiguous(), params.contiguous(), starts.contiguous()
         M, R, dev = idx.shape[1], starts.numel(), idx.device
         n = (R + 31) // 32
@@ -1041,9 +1053,11 @@ class CudaBackend:
         if n == 0 or n > _lib.MAX_PRIOR_SEGMENTS:
             raise ValueError(f"between 1 and {_lib.MAX_PRIOR_SEGMENTS} prior lists per launch")
         pos = pos.detach().contiguous()
+        N, dev, dt = pos.shape[0], pos.device, _dt(pos)
         if batch is not None:
             batch = batch.to(torch.int64).contiguous()
-        N, dev, dt = pos.shape[0], pos.device, _dt(pos)
+            if batch.numel() != N:
+                raise ValueError("batch must have one entry per bead")
         arr = (_lib.PriorListStruct * n)()
         keep = []
         M_total = moved = 0
@@ -1051,12 +1065,12 @@ class CudaBackend:
             a = arr[k]
             if sliced is not None:
                 slices, beads, offsets, params = sliced
-                _need_cuda(*sliced)
+                _need_cuda(pos, *sliced)
                 M, per_term = offsets.shape[0] * 128, 2
                 a.n_slices, a.steps, a.slices, a.slice_beads = slices.shape[0], offsets.shape[0], slices.data_ptr(), beads.data_ptr()
                 a.offsets, a.slice_params = offsets.data_ptr(), params.data_ptr()
             else:
-                _need_cuda(idx, params)
+                _need_cuda(pos, idx, params)
                 if idx.dtype != torch.int32:
                     raise TypeError("prior lists take int32 indices")
                 idx, params = idx.contiguous(), params.contiguous()

@@ -587,6 +587,8 @@ class SchNet(torch.nn.Module):
     @staticmethod
     def _types(data):
         types = data.atom_types
+        if types.numel() != data.pos.shape[0]:
+            raise ValueError("atom_types must have one entry per bead")
         if types.dtype != torch.int64 or not types.is_contiguous():
             types = types.to(torch.int64).contiguous()
         return types

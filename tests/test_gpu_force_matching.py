@@ -383,3 +383,19 @@ def test_a_weight_turned_in_place_after_a_call(training):
     w.data = w.data.contiguous()
     expected = m(_data(pos, types_, sizes)).out["SchNet"]["forces"].detach()
     assert torch.allclose(got, expected, rtol=1e-4, atol=1e-4 * float(expected.abs().max()))
+
+
+@pytest.mark.parametrize("training", [True, False])
+def test_inputs_a_kernel_could_not_read_are_refused(training):
+    """Bead types on the host, or fewer of them than beads, end in an error on the host."""
+    sizes = [23, 40]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 18)
+    m = bnn.GradientsOut(net.to(DEV), "forces").train(training)
+    for wrong in (types_, types_.to(DEV)[:-1]):
+        for given_list in (False, True):
+            data = _data(pos, types_, sizes)
+            if given_list:
+                data.neighbor_list = net.neighbor_list(data, 9.0)
+            data.atom_types = wrong
+            with pytest.raises((RuntimeError, ValueError)):
+                m(data)

@@ -62,6 +62,21 @@ def test_a_sliced_list_is_kept_once():
     assert float((together[1] - alone["forces"]).abs().max()) <= 2e-5 * (1 + float(alone["forces"].abs().max()))
 
 
+def test_lists_a_kernel_could_not_read_are_refused():
+    data, priors = prior_setup(40, 2, 4, torch.Generator().manual_seed(4))
+    with torch.no_grad():
+        priors["repulsion"].sigma.copy_(0.5 * (priors["repulsion"].sigma + priors["repulsion"].sigma.t()))
+    on_host = data.neighbor_list["repulsion"]["index_mapping"]
+    data, p = data.to(DEV), priors["repulsion"].to(DEV).eval()
+    _evaluate_together([p], data, forces=True)
+    batch, data.batch = data.batch, data.batch[:-1]
+    with pytest.raises(ValueError, match="one entry per bead"):
+        _evaluate_together([p], data, forces=True)
+    data.batch, data.neighbor_list["repulsion"]["index_mapping"] = batch, on_host
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        _evaluate_together([p], data, forces=True)
+
+
 def test_pair_slices_of_beads_that_lie_far_apart():
     near = torch.arange(9, device=DEV, dtype=torch.int32)
     pairs = torch.stack([torch.zeros_like(near), near + 65535 - 8] ).repeat(1, 20)
