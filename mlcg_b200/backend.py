@@ -223,8 +223,20 @@ class CudaBackend:
         pending, self._pending = self._pending, []
         if not pending:
             return
-        words = torch.stack([s[0] for s, _ in pending]).cpu().tolist()
+        words = [0] * len(pending)
+        for dev in {s.device for s, _ in pending}:         # one read per device
+            here = [k for k, (s, _) in enumerate(pending) if s.device == dev]
+            for k, word in zip(here, torch.stack([pending[k][0][0] for k in here]).cpu().tolist()):
+                words[k] = word
         self._raise_pending(words, pending)
+
+    def _take_pending(self, dev):
+        """The one status word that waits to be read, for a kernel on ``dev`` to hand over with its own result; more than one, or one of
+        another device, are read here."""
+        if len(self._pending) > 1 or (self._pending and self._pending[0][0].device != dev):
+            self.check_pending()
+        pend, self._pending = self._pending, []
+        return pend
 
     @staticmethod
     def _raise_pending(words, pending):
@@ -342,9 +354,7 @@ class CudaBackend:
                 return dict(edge_index=torch.empty((2, 0), dtype=torch.int64, device=dev), distance=pos.new_empty(0) if want_distance else None,
                             mapping_batch=torch.empty(0, dtype=torch.int64, device=dev) if want_batch else None, row0=empty, row1=empty.clone(),
                             offsets=torch.zeros(N + 1, dtype=torch.int64, device=dev), status=0, ptr=ptr, twin=None, sel=None, pair_of=None)
-            if len(self._pending) > 1:
-                self.check_pending()
-            pend, self._pending = self._pending, []
+            pend = self._take_pending(dev)
             wsb = self.lib.mlcgb_graph_workspace_bytes(N, B, dt)
             ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
             offsets = torch.empty(N + 1, dtype=torch.int64, device=dev)
@@ -836,9 +846,7 @@ class CudaBackend:
         N, dev = pos.shape[0], pos.device
         B = ptr.numel() - 1 if n_atoms is None else n_atoms.numel()
         s, keep = self._spec(spec, torch.float32)
-        if len(self._pending) > 1:
-            self.check_pending()
-        pend, self._pending = self._pending, []
+        pend = self._take_pending(dev)
         status = self._sticky_status(dev)
         lib, ref, size = self.lib, ctypes.byref(w), self.lib.mlcgb_schnet_evaluate_workspace_bytes
         with _on(dev):

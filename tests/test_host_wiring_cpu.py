@@ -288,6 +288,21 @@ def test_copies_of_a_prior_start_without_its_kept_lists():
         assert torch.equal(other(data).out[p.name]["energy"], energy)
 
 
+def test_a_status_word_is_handed_over_on_its_own_device_only():
+    """A graph's kernel reads the status word of earlier work; one of another device, or a second one, is read by the host first."""
+    be = object.__new__(backend.CudaBackend)
+    word = torch.zeros(4, dtype=torch.int32)
+    be._pending = [(word, "here")]
+    assert be._take_pending(word.device) == [(word, "here")] and be._pending == []
+    be._pending = [(word, "elsewhere")]
+    assert be._take_pending(torch.device("cuda", 0)) == [] and be._pending == []
+    be._pending = [(word, "a"), (word.clone(), "b")]
+    assert be._take_pending(word.device) == []
+    be._pending = [(word, "a"), (torch.tensor([16, 0, 0, 0], dtype=torch.int32), "b")]
+    with pytest.raises(RuntimeError, match="b: a weight is beyond"):
+        be.check_pending()
+
+
 def test_no_cpu_fallback(monkeypatch):
     """Without the test substitution the package refuses CPU tensors instead of computing on the host."""
     monkeypatch.setattr(backend, "_backend", None)
