@@ -333,6 +333,7 @@ class CudaBackend:
         ``want_plan``: also twin, sel and pair_of as :meth:`pair_plan` gives them, or None under these keys where a list was cut short,
         has loops or exclusions, or has no edges; ``want_index=False``: no int64 edge index."""
         _need_cuda(pos, ptr, n_atoms)
+        ptr, n_atoms = (None if t is None else t.contiguous() for t in (ptr, n_atoms))
         ex_xs = ex_ptr = None
         if exclude is not None:
             if int(rule) != 0:
@@ -386,7 +387,7 @@ class CudaBackend:
         """Radius graph of periodic structures: dict(edge_index [2,E] i64 (row 0 = centre), cell_shifts [E,3], distance|None,
         mapping_batch|None, status int).  ``cells`` [B,3,3] in the dtype of ``pos``, ``repeats`` [B,3] copies per cell vector."""
         _need_cuda(pos, ptr, cells, repeats)
-        pos = pos.detach().contiguous()
+        pos, ptr = pos.detach().contiguous(), ptr.contiguous()
         cells = cells.detach().to(pos.dtype).contiguous()
         repeats = repeats.to(torch.int32).contiguous()
         N, B, dev = pos.shape[0], ptr.numel() - 1, pos.device
@@ -418,7 +419,7 @@ class CudaBackend:
         ``[2, capacity]`` buffer to reuse, whose entries are valid point indices (zeros at first).  An overflow sets bit 5 of the
         backend's accumulating status words (reported by :meth:`check_pending`)."""
         _need_cuda(pos, ptr)
-        pos = pos.detach().contiguous()
+        pos, ptr = pos.detach().contiguous(), ptr.contiguous()
         N, B, dev = pos.shape[0], ptr.numel() - 1, pos.device
         dt = _dt(pos)
         capacity = int(capacity)
@@ -443,6 +444,7 @@ class CudaBackend:
         """:meth:`radius_graph_capacity` and :meth:`pair_plan` together, from ``n_atoms`` (int64 [B]; ``ptr`` None) or ``ptr``:
         dict(row0, row1, offsets, counts, ptr, twin, sel, pair_of)."""
         _need_cuda(pos, ptr, n_atoms)
+        ptr, n_atoms = (None if t is None else t.contiguous() for t in (ptr, n_atoms))
         pos = pos.detach().contiguous()
         N, dev, dt = pos.shape[0], pos.device, _dt(pos)
         B = ptr.numel() - 1 if n_atoms is None else n_atoms.numel()

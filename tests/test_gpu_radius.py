@@ -296,3 +296,15 @@ def test_reverse_edge_map_of_a_list_with_self_pairs():
     assert int(st[0]) == 0
     t = twin.long()
     assert torch.equal(res["row0"][t], res["row1"]) and torch.equal(res["row1"][t], res["row0"])
+
+
+def test_boundaries_of_any_stride():
+    """Structure boundaries that are a column of a larger tensor, positions that are a transposed view."""
+    rng = np.random.default_rng(2)
+    pos = (rng.random((90, 3)) * 9).astype(np.float32)
+    ptr = np.array([0, 20, 65, 90], dtype=np.int64)
+    wide = torch.stack([torch.as_tensor(ptr), torch.zeros(4, dtype=torch.int64)], dim=1).to(DEV)
+    turned = torch.as_tensor(np.ascontiguousarray(pos.T), device=DEV).t()
+    ei, dist = mlcg_b200.neighbor_list.radius_cuda(turned, wide[:, 0], 3.0, 1000, True)
+    want, want_d = radius_ref.radius_graph_c(pos, ptr, 3.0, 1000, False, "native", with_distance=True)
+    assert np.array_equal(ei.cpu().numpy(), want) and np.array_equal(dist.cpu().numpy(), want_d)
