@@ -29,12 +29,24 @@ class GraphedForceField:
         self.data.pos = data.pos.detach().contiguous().clone()
         self._pos = self.data.pos
         be = get_backend()
+        self._release_rows()                      # (a row buffer of its own, not one that other recordings or calls write)
         for _ in range(max(1, warmup)):           # lazily created buffers and kernel attributes exist before the recording
             self._evaluate()
         be.check_pending()
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph):
             self.energy, self.forces = self._evaluate()
+        # The recording holds addresses only.  What lies there is kept with it: the storage of weights and buffers, and what the modules
+        # made of this data's lists, which evaluations of other data replace on the modules.
+        self._kept = [[t.detach() for t in (*model.parameters(), *model.buffers())],
+                      [v for m in model.modules() for k, v in m.__dict__.items() if k.startswith("_mlcgb_")],
+                      [getattr(self.data, k, None) for k in ("atom_types", "batch", "n_atoms")],
+                      [list(nl.values()) for nl in (getattr(self.data, "neighbor_list", None) or {}).values()]]
+        self._release_rows()
+
+    def _release_rows(self):
+        for m in self.model.modules():
+            m.__dict__.pop("_mlcgb_rows", None)
 
     def _evaluate(self) -> Tuple[torch.Tensor, torch.Tensor]:
         data = self.data

@@ -82,3 +82,39 @@ def test_weights_written_by_the_launch_before(sizes):
     z = be.gemm_fused(0, x, y)
     for _ in range(20):
         assert torch.equal(be.gemm_fused(0, x, be.gemm_fused(0, x, w)), z)
+
+
+def test_recordings_of_one_model_stand_by_themselves():
+    """Two recordings and plain evaluations of one model over different data: the row buffers and the prior lists that a recording
+    reads stay its own, and nothing of it writes memory that has been given back."""
+    from helpers import prior_setup
+    torch.manual_seed(0)
+    cut = bnn.CosineCutoff(0.0, 9.0)
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, 32, trainable=False), cut, [128], embedding_size=4, num_interactions=2)
+    sets = []
+    for k, (n, B) in enumerate(((30, 6), (45, 5))):
+        data, priors = prior_setup(n, B, 4, torch.Generator().manual_seed(k))
+        gen = torch.Generator().manual_seed(k)
+        data.pos = torch.cat([random_walk_chain(n, gen, min_dist=3.0) for _ in range(B)]).float()
+        sets.append(data.to(DEV))
+    with torch.no_grad():
+        priors["repulsion"].sigma.copy_(0.5 * (priors["repulsion"].sigma + priors["repulsion"].sigma.t()))
+    model = bnn.SumOut(torch.nn.ModuleDict({"SchNet": bnn.GradientsOut(net, "forces"), **{k: bnn.GradientsOut(p, "forces") for k, p in priors.items()}}))
+    model = bnn.set_edge_capacity(model.eval().to(DEV), 9000)
+    fresh = lambda d: mlcg_b200.AtomicData(pos=d.pos.clone(), atom_types=d.atom_types, batch=d.batch, n_atoms=d.n_atoms,  # noqa: E731
+                                           neighbor_list={k: dict(v) for k, v in d.neighbor_list.items()})
+    want = []
+    for d in sets:
+        out = model(fresh(d)).out
+        want.append((out["energy"].clone(), out["forces"].clone()))
+    fields = [mlcg_b200.GraphedForceField(model, fresh(d)) for d in sets]
+    rows = [[v for v in f._kept[1] if isinstance(v, tuple) and len(v) == 2 and torch.is_tensor(v[1])] for f in fields]
+    assert len(rows[0]) == len(rows[1]) == 1 and rows[0][0][1].data_ptr() != rows[1][0][1].data_ptr()
+    model(fresh(sets[1]))
+    junk = [torch.full((2, 9000), 7, dtype=torch.int32, device=DEV) for _ in range(64)] + [torch.full((2 ** 16,), 7, dtype=torch.int32, device=DEV) for _ in range(64)]
+    for _ in range(2):
+        for f, d, (e, g) in zip(fields, sets, want):
+            got = f(d.pos)
+            assert torch.equal(got[0], e) and torch.equal(got[1], g)
+    fields[0].check()
+    assert all(bool((j == 7).all()) for j in junk)
