@@ -878,6 +878,7 @@ class CudaBackend:
         at = (ctypes.c_int64 * 8)()
         lib.mlcgb_schnet_evaluate_lists(N, B, E, at)
         places = ((0, 0), (4, at[0]) if ptr is None else (5, 0), (3, at[2]), (3, at[3]), (4, at[1]), (3, at[6]), (3, at[5]), (3, at[7]), (3, at[4]), (1, 0), (2, 0))
+        ws = ws[:size(N, B, E, spec.num_rbf, ref, 1)]          # (saved with the size that its edges ask for, not that of the guess)
         return energy, grad, E, ForceMatchingState(N, B, E, (types, spec.p0, spec.p1, ws, graph_ws, ptr), places, spec, conv_cut, weights)
 
     # ------------------------------------------------------------------ one force-matching step

@@ -399,3 +399,23 @@ def test_inputs_a_kernel_could_not_read_are_refused(training):
             data.atom_types = wrong
             with pytest.raises((RuntimeError, ValueError)):
                 m(data)
+
+
+def test_a_checkpointed_step():
+    """What a pass saves has the sizes of its edges, not of the guess before it: a checkpoint's second forward saves the same."""
+    from torch.utils.checkpoint import checkpoint
+    net, *_ = _setup("expnormal", 32, 9.0, 2, [40], 128, 19)
+    m = bnn.GradientsOut(net.to(DEV), "forces").train()
+    for sizes in ([40] * 4, [23, 40, 9], [73] * 3, [300]):
+        _, pos, types_, _, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 20)
+        m.zero_grad(set_to_none=True)
+        forces = checkpoint(lambda p: m(_data(p, types_, sizes)).out["SchNet"]["forces"], pos.to(DEV), use_reentrant=False)
+        ((forces - target.to(DEV)) ** 2).mean().backward()
+        got = _grads(net)
+        loss = ((m(_data(pos, types_, sizes)).out["SchNet"]["forces"] - target.to(DEV)) ** 2).mean()
+        m.zero_grad(set_to_none=True)
+        loss.backward(retain_graph=True)
+        _close(got, _grads(net), 1e-6)
+        m.zero_grad(set_to_none=True)
+        loss.backward()                            # (a second backward over the same state)
+        _close(_grads(net), got, 1e-6)
