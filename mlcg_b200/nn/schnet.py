@@ -42,7 +42,7 @@ class _Layers:
         modules = _all_modules(net)
         self._children = [m._modules for m in modules if m._modules]
         self._found = [child for c in self._children for child in c.values()]
-        self._states = [m.__dict__ for m in modules]
+        self._states = [m.__dict__ for m in modules if m is not net]       # (its own would tie a knot: `net` holds this object)
         basis = net.rbf_layer
         self._basis = [m._parameters for m in _all_modules(basis)]
         self._basis_tensors = (basis._parameters, basis._buffers)
@@ -62,11 +62,11 @@ class _Layers:
         except KeyError:
             return None
 
-    def watched(self) -> bool:
-        """Whether somebody would notice that a training step does not call the modules one by one: hooks on any of them or on all
-        modules of the program, or a ``forward`` put in place of theirs."""
+    def watched(self, net) -> bool:
+        """Whether somebody would notice that a training step of ``net`` does not call the modules one by one: hooks on any of them or
+        on all modules of the program, or a ``forward`` put in place of theirs."""
         return any(_EVERY_MODULES_HOOKS) or any([d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]
-                                                 or "forward" in d for d in self._states])
+                                                 or "forward" in d for d in (net.__dict__, *self._states)])
 
     def trained_basis(self) -> bool:
         return any([t is not None and t.requires_grad for p in self._basis for t in p.values()])
@@ -492,7 +492,7 @@ class SchNet(torch.nn.Module):
         if not torch.is_grad_enabled() or self.edge_capacity or self._forward_of_ones_own():
             return None
         layers = self._layers()
-        if layers.slots is None or layers.watched():
+        if layers.slots is None or layers.watched(self):
             return None
         setup = self._whole_model_setup(data.pos, True, layers)
         if setup is None or not be.train_ok(setup) or layers.trained_basis():

@@ -288,6 +288,23 @@ def test_copies_of_a_prior_start_without_its_kept_lists():
         assert torch.equal(other(data).out[p.name]["energy"], energy)
 
 
+def test_a_model_goes_with_its_last_reference():
+    """What a SchNet keeps on itself between calls holds no way back to it: its memory does not wait for the cycle collector."""
+    import gc
+    import weakref
+    cut = bnn.CosineCutoff(0.0, 8.0)
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, 16), cut, [16], hidden_channels=16, embedding_size=4, num_filters=16, num_interactions=2)
+    assert net.packed_weights() is None and net._layers().slots is not None
+    gc.collect()
+    gc.disable()
+    try:
+        gone = [weakref.ref(net), weakref.ref(net.embedding_layer), weakref.ref(net.interaction_blocks[0].lin.weight)]
+        del net
+        assert [g() for g in gone] == [None, None, None]
+    finally:
+        gc.enable()
+
+
 def test_a_status_word_is_handed_over_on_its_own_device_only():
     """A graph's kernel reads the status word of earlier work; one of another device, or a second one, is read by the host first."""
     be = object.__new__(backend.CudaBackend)
