@@ -339,11 +339,15 @@ class SchNet(torch.nn.Module):
         for b in self.interaction_blocks:
             if type(b) is not InteractionBlock or type(b.conv) is not CFConv or type(b.activation) is not torch.nn.Tanh:
                 return None
-            c, net = b.conv, b.conv.filter_network
-            if type(net) is not MLP or len(net.layers) != 3 or c.lin1.bias is not None or c.lin2.bias is None or b.lin.bias is None:
+            c, lin = b.conv, b.lin
+            net, lin1, lin2 = c.filter_network, c.lin1, c.lin2
+            if type(net) is not MLP or lin1.bias is not None or lin2.bias is None or lin.bias is None:
                 return None
-            slots += [(c.lin1, "weight"), (net.layers[0], "weight"), (net.layers[0], "bias"), (net.layers[2], "weight"), (c.lin2, "weight"),
-                      (c.lin2, "bias"), (b.lin, "weight"), (b.lin, "bias")]
+            layers = list(net.layers)
+            if len(layers) != 3:
+                return None
+            slots += [(lin1, "weight"), (layers[0], "weight"), (layers[0], "bias"), (layers[2], "weight"), (lin2, "weight"), (lin2, "bias"), (lin, "weight"),
+                      (lin, "bias")]
         return slots
 
     def _layers(self) -> "_Layers":
