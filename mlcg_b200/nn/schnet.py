@@ -68,6 +68,10 @@ class _Layers:
         return any(_EVERY_MODULES_HOOKS) or any([d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]
                                                  or "forward" in d for d in (net.__dict__, *self._states)])
 
+    def in_mode(self, training: bool) -> bool:
+        """Whether all modules are in the same mode as the model (each takes its weights as constants or not by its own)."""
+        return all([d["training"] is training for d in self._states])
+
     def trained_basis(self) -> bool:
         return any([t is not None and t.requires_grad for p in self._basis for t in p.values()])
 
@@ -608,7 +612,7 @@ class SchNet(torch.nn.Module):
             return None
         layers = self._layers() if layers is None else layers
         weights = self.packed_weights(layers)
-        if weights is None or weights[1][1][0].device != pos.device:
+        if weights is None or weights[1][1][0].device != pos.device or not layers.in_mode(training):
             return None
         key = (training, id(weights), layers.description())
         cached = self.__dict__.get("_mlcgb_setup")

@@ -419,3 +419,25 @@ def test_a_checkpointed_step():
         m.zero_grad(set_to_none=True)
         loss.backward()                            # (a second backward over the same state)
         _close(_grads(net), got, 1e-6)
+
+
+@pytest.mark.parametrize("training", [True, False])
+def test_a_part_of_the_model_in_the_other_mode(training):
+    """A block switched to the other mode after a call: its layers act as they do in a model that has had it so from the start."""
+    sizes = [23, 40]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 21)
+    m = bnn.GradientsOut(net.to(DEV), "forces").train(training)
+    other = copy.deepcopy(m)
+    m(_data(pos, types_, sizes))
+    results = []
+    for model in (m, other):
+        model.model.interaction_blocks[0].train(not training)
+        out = model(_data(pos, types_, sizes)).out["SchNet"]
+        if training:
+            assert not _fused(out["forces"])
+            ((out["forces"] - target.to(DEV)) ** 2).mean().backward()
+        results.append((out["forces"].detach(), _grads(model.model)))
+    assert torch.equal(results[0][0], results[1][0]) and results[0][1].keys() == results[1][1].keys()
+    _close(results[0][1], results[1][1], 1e-6)
+    if training:
+        assert "interaction_blocks.0.conv.lin1.weight" not in results[0][1]
