@@ -49,7 +49,7 @@ class _Layers:
         self.slots = net._whole_model_slots()         # (module, parameter name) of every weight, or None
         self._places = None if self.slots is None else [(m._parameters, n) for m, n in self.slots]
         self._cutoffs = None if self.slots is None else [(b.conv, b.conv.cutoff) for b in net.interaction_blocks]
-        self._basis_cutoff = getattr(basis, "cutoff", None)
+        self._basis_layer, self._basis_cutoff = basis, getattr(basis, "cutoff", None)
 
     def still_there(self) -> bool:
         return [child for c in self._children for child in c.values()] == self._found
@@ -79,7 +79,7 @@ class _Layers:
         """What the filter description of the model is worked out from, beside the modules and the weights."""
         lo, hi = getattr(self._basis_cutoff, "cutoff_lower", None), getattr(self._basis_cutoff, "cutoff_upper", None)
         parameters, buffers = self._basis_tensors
-        return (*map(id, parameters.values()), *map(id, buffers.values()), lo, hi,
+        return (*map(id, parameters.values()), *map(id, buffers.values()), lo, hi, self._basis_layer.__dict__.get("alpha"),
                 *[(getattr(c, "cutoff_lower", None), getattr(c, "cutoff_upper", None), conv.filter_precision) for conv, c in self._cutoffs])
 
 
@@ -167,7 +167,7 @@ class CFConv(torch.nn.Module):
         rc = rbf_layer.cutoff
         key = (id(rbf_layer), net.layers[0].weight.device, net.layers[0].weight.dtype, id(self.cutoff), id(rc),
                getattr(self.cutoff, "cutoff_lower", None), getattr(self.cutoff, "cutoff_upper", None),
-               getattr(rc, "cutoff_lower", None), getattr(rc, "cutoff_upper", None),
+               getattr(rc, "cutoff_lower", None), getattr(rc, "cutoff_upper", None), getattr(rbf_layer, "alpha", None),
                tuple(map(id, net.layers)), tuple(map(id, rbf_layer._parameters.values())), tuple(map(id, rbf_layer._buffers.values())))
         cached = self.__dict__.get("_mlcgb_fused_spec")
         if cached is not None and cached[0] == key:

@@ -441,3 +441,15 @@ def test_a_part_of_the_model_in_the_other_mode(training):
     _close(results[0][1], results[1][1], 1e-6)
     if training:
         assert "interaction_blocks.0.conv.lin1.weight" not in results[0][1]
+
+
+@pytest.mark.parametrize("training", [True, False])
+def test_a_basis_whose_scale_changes_after_a_call(training):
+    sizes = [23, 40]
+    net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, sizes, 128, 22)
+    m = bnn.GradientsOut(net.to(DEV), "forces").train(training)
+    before = m(_data(pos, types_, sizes)).out["SchNet"]["forces"].detach()
+    net.rbf_layer.alpha *= 0.8
+    got = m(_data(pos, types_, sizes)).out["SchNet"]["forces"].detach()
+    fresh = copy.deepcopy(m)(_data(pos, types_, sizes)).out["SchNet"]["forces"].detach()
+    assert torch.equal(got, fresh) and not torch.allclose(got, before, rtol=1e-2)
