@@ -123,16 +123,22 @@ def _ptr_from_index(idx: torch.Tensor, N: int) -> torch.Tensor:
 
 
 def attach_plan(edge_index: torch.Tensor, plan: EdgePlan) -> torch.Tensor:
-    edge_index._mlcgb_plan = plan
+    edge_index._mlcgb_plan = plan, None if edge_index.is_inference() else edge_index._version
     return edge_index
+
+
+def attached_plan(edge_index: torch.Tensor) -> Optional[EdgePlan]:
+    """The plan that travels with an edge list, None where the list has been written to since."""
+    plan, version = getattr(edge_index, "_mlcgb_plan", (None, None))
+    return plan if version is None or version == edge_index._version else None
 
 
 def plan_of(edge_index: torch.Tensor, N: int) -> EdgePlan:
     """The plan travelling with an edge list built by this package, else one derived on the spot."""
-    plan = getattr(edge_index, "_mlcgb_plan", None)
+    plan = attached_plan(edge_index)
     if plan is None or plan.N != N or plan.E != edge_index.shape[1]:
         plan = EdgePlan.from_edge_index(edge_index, N)
-        edge_index._mlcgb_plan = plan
+        attach_plan(edge_index, plan)
     return plan
 
 

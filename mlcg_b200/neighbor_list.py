@@ -10,11 +10,10 @@ from typing import Dict, Mapping, Optional, Tuple
 
 import torch
 
-from .autograd import EdgePlan, attach_plan, edge_distances
+from .autograd import EdgePlan, attach_plan, attached_plan, edge_distances
 from .backend import STATUS_TRUNCATED, get_backend
 
 RULE_NATIVE, RULE_CLUSTER = 0, 1
-PLAN_KEY = "_mlcgb_plan"
 
 
 def _as_3d(x: torch.Tensor) -> torch.Tensor:
@@ -132,7 +131,7 @@ def make_neighbor_list(tag: str, order: int, index_mapping: torch.Tensor, mappin
         raise RuntimeError(f"index_mapping shape does not match the order:{index_mapping.shape[0]} != {order}")
     if mapping_batch is None:
         mapping_batch = torch.zeros((index_mapping.shape[1],) if len(index_mapping) > 0 else (0,), dtype=torch.long)
-    plan = getattr(index_mapping, "_mlcgb_plan", None)
+    plan = attached_plan(index_mapping) if torch.is_tensor(index_mapping) else None
     im = torch.as_tensor(index_mapping, dtype=torch.long)
     if plan is not None:
         attach_plan(im, plan)

@@ -264,6 +264,23 @@ def test_sumout_additivity(golden):
     assert torch.allclose(out.out["energy"], e, rtol=1e-6) and torch.allclose(out.out["forces"], f, rtol=1e-6)
 
 
+@pytest.mark.parametrize("training", [False, True])
+def test_an_edge_list_written_to_is_planned_anew(golden, training):
+    """Edges changed in place after the list was built: the energies are those of the list as it is."""
+    c = golden["schnet_gaussian_f32"]
+    net = schnet_from_case(c)
+    model = bnn.GradientsOut(net, "forces").train(training)
+    data = data_from_case(c)
+    data.neighbor_list = net.neighbor_list(data, c["upper"])
+    edges = data.neighbor_list["SchNet"]["index_mapping"]
+    before = model(data).out["SchNet"]["energy"].detach()
+    edges[:, :8] = edges[:, 8:16].clone()
+    changed = model(data).out["SchNet"]["energy"].detach()
+    data.neighbor_list["SchNet"] = mlcg_b200.make_neighbor_list("", 2, edges.clone(), rcut=c["upper"], self_interaction=False)
+    fresh = model(data).out["SchNet"]["energy"].detach()
+    assert torch.allclose(changed, fresh, rtol=1e-5) and not torch.allclose(before, fresh, rtol=1e-5)
+
+
 def test_kept_parameters_follow_the_strides():
     """Bead types (or an index list) that are another view of the same memory, of the same shape, are another input."""
     data, priors = prior_setup(10, 2, 3, torch.Generator().manual_seed(7))
