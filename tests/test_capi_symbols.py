@@ -37,6 +37,7 @@ def test_library_exports_every_declared_symbol():
         assert hasattr(lib, name), name
     lib.mlcgb_strerror.restype = ctypes.c_char_p
     assert lib.mlcgb_strerror(0) == b"ok" and b"workspace" in lib.mlcgb_strerror(-2)
+    assert lib.mlcgb_version() >= 100
     header = open(os.path.join(ROOT, "include", "mlcg_b200.h")).read()
     assert lib.mlcgb_version() == _lib.VERSION == int(re.search(r"#define MLCGB_VERSION (\d+)", header).group(1))
 
