@@ -46,7 +46,7 @@ int mlcgb_last_cuda_error(void); /* cudaError_t of the last failed launch on thi
  *        NULL), negate and the totals are new, fixed_point = 0 writes its outputs too (it added to them), the workspace is wanted in
  *        both modes and mlcgb_prior_eval_workspace_bytes takes the dtype where it took fixed_point.  mlcgb_gemm_tc_chain2 with
  *        backward = 1 writes mid_out unless it is NULL. */
-#define MLCGB_VERSION 200
+#define MLCGB_VERSION 201
 int mlcgb_version(void);
 
 /* Device time per entry point, without a profiler.  No counterpart in the reference (mlcg times whole steps on the host).
@@ -141,7 +141,8 @@ int mlcgb_pair_index(const int32_t *sel /* [P] */, const int32_t *twin /* [E] */
  *   graph_begin: structure boundaries (n_atoms [B] given: ptr [B+1] is written; NULL: ptr is read), degrees, offsets [N+1]; waits for
  *     the result on the host and leaves host_out[0] = edges, [1] = status (bit 0: list cut short), [2] = *pending_status (a status
  *     word of earlier work, or NULL), [3] for with_cells.  Never while the stream is being captured.
- *   graph_finish: the edges (edge_index [2,E] int64 or NULL, distance, mapping_batch or NULL, row0 / row1 int32) and the plan (twin, sel,
+ *   graph_finish: the edges (edge_index [2,E] int64 or NULL, distance, mapping_batch or NULL, row0 / row1 int32, or NULL with edge_index
+ *     and no plan) and the plan (twin, sel,
  *     pair_of together, E < 2^31 and row1 on a 32-byte
  *     boundary then; or all NULL: with loop, excluded pairs or a list that was cut short) with the same workspace and offsets.
  *   graph_capacity: both without a host read into buffers of `capacity` edges (an even number), counts as in
@@ -149,6 +150,14 @@ int mlcgb_pair_index(const int32_t *sel /* [P] */, const int32_t *twin /* [E] */
  * N, B > 0.  Excluded pairs go with rule 0 and are given to both calls. */
 /* Structures of a sorted batch vector (batch[N-1] + 1), read on the host as above. */
 int mlcgb_batch_structures(const int64_t *batch, int64_t N, int64_t *host_out, void *stream);
+/* The same and the boundaries ptr [most + 1] of up to `most` structures, in one launch (more of them: mlcgb_batch_to_ptr). */
+int mlcgb_batch_boundaries(const int64_t *batch, int64_t N, int64_t most, int64_t *ptr, int64_t *host_out, void *stream);
+/* graph_begin / graph_finish for up to 2048 points given with their batch vector (sorted; NULL: one structure): edges and distances
+ * (or NULL), no plan.  Workspace: mlcgb_graph_workspace_bytes(N, 1, dtype). */
+int mlcgb_graph_small_begin(const void *pos, int dtype, const int64_t *batch, int64_t N, double r, int64_t max_nn, int loop, int rule, void *workspace,
+                            size_t workspace_bytes, int64_t *offsets, const int32_t *pending_status, int64_t *host_out, void *stream);
+int mlcgb_graph_small_finish(const void *pos, int dtype, const int64_t *batch, int64_t N, void *workspace, size_t workspace_bytes, const int64_t *offsets,
+                             int64_t E, int64_t *edge_index /* [2,E] */, void *distance /* [E] or NULL */, void *stream);
 size_t mlcgb_graph_workspace_bytes(int64_t N, int64_t B, int dtype);
 int mlcgb_graph_begin(const void *pos, int dtype, const int64_t *n_atoms, int64_t *ptr, int64_t N, int64_t B, double r, int64_t max_nn, int loop,
                       int rule, const int64_t *exclude_pair_xs, const int64_t *ptr_exclude_pair_xs, void *workspace, size_t workspace_bytes,

@@ -44,7 +44,7 @@ class PriorListStruct(ctypes.Structure):
 
 
 MAX_PRIOR_SEGMENTS = 8
-VERSION = 200                  # MLCGB_VERSION of the header that the tables below follow
+VERSION = 201                  # MLCGB_VERSION of the header that the tables below follow
 EVALUATE_DONE, EVALUATE_MORE = 1, 2
 
 # name -> (restype, argtypes); one entry per symbol declared in include/mlcg_b200.h
@@ -114,6 +114,9 @@ SIGNATURES = {
                                       ctypes.POINTER(SchnetWeightsStruct), c_int, c_int, c_int, c_vp, c_sz, c_vp, c_sz, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "mlcgb_graph_workspace_bytes": (c_sz, [c_i64, c_i64, c_int]),
     "mlcgb_graph_begin": (c_int, [c_vp, c_int, c_vp, c_vp, c_i64, c_i64, c_dbl, c_i64, c_int, c_int, c_vp, c_vp, c_vp, c_sz, c_vp, c_vp, c_vp, c_vp]),
+    "mlcgb_batch_boundaries": (c_int, [c_vp, c_i64, c_i64, c_vp, c_vp, c_vp]),
+    "mlcgb_graph_small_begin": (c_int, [c_vp, c_int, c_vp, c_i64, c_dbl, c_i64, c_int, c_int, c_vp, c_sz, c_vp, c_vp, c_vp, c_vp]),
+    "mlcgb_graph_small_finish": (c_int, [c_vp, c_int, c_vp, c_i64, c_vp, c_sz, c_vp, c_i64, c_vp, c_vp, c_vp]),
     "mlcgb_graph_finish": (c_int, [c_vp, c_int, c_vp, c_i64, c_i64, c_dbl, c_int, c_vp, c_vp, c_vp, c_sz, c_vp, c_i64] + [c_vp] * 8 + [c_int, c_vp, c_vp]),
     "mlcgb_graph_capacity": (c_int, [c_vp, c_int, c_vp, c_vp, c_i64, c_i64, c_dbl, c_i64, c_int, c_vp, c_sz, c_vp, c_i64] + [c_vp] * 8),
     "mlcgb_schnet_eval": (c_int, [c_vp, c_vp, c_vp, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_i64, c_i64, c_vp, c_int, c_dbl, c_dbl,

@@ -122,15 +122,47 @@ def _ptr_from_index(idx: torch.Tensor, N: int) -> torch.Tensor:
     return ptr
 
 
-def attach_plan(edge_index: torch.Tensor, plan: EdgePlan) -> torch.Tensor:
+class DeferredPlan:
+    """The plan of a centre-sorted list whose caller asked for the edges alone: made when an operator is first given the list.  It is
+    kept for the stream that it was made on (another one makes its own, there is no order between the two) and never out of a
+    recording, whose buffers hold nothing until it is replayed."""
+
+    __slots__ = ("index", "offsets", "N", "symmetric", "loops", "_made", "_stream")
+
+    def __init__(self, edge_index: torch.Tensor, offsets: torch.Tensor, N: int, symmetric: bool, loops: bool):
+        # (an alias: the list carries this object, which must not hold the list)
+        self.index, self.offsets, self.N, self.symmetric, self.loops = edge_index.detach(), offsets, N, symmetric, loops
+        self._made = self._stream = None
+
+    def plan(self) -> EdgePlan:
+        cuda = self.index.is_cuda
+        stream = torch.cuda.current_stream(self.index.device).cuda_stream if cuda else 0
+        recording = cuda and torch.cuda.is_current_stream_capturing()
+        if self._made is not None and self._stream == stream and not recording:
+            return self._made
+        row0, row1 = self.index.to(torch.int32).unbind(0)
+        plan = EdgePlan.from_centre_sorted(row0, row1, self.offsets, self.N, self.symmetric, self.loops)
+        if not recording:
+            self._made, self._stream = plan, stream
+        return plan
+
+
+def attach_plan(edge_index: torch.Tensor, plan) -> torch.Tensor:
+    """``plan``: an :class:`EdgePlan` or a :class:`DeferredPlan`."""
     edge_index._mlcgb_plan = plan, None if edge_index.is_inference() else edge_index._version
     return edge_index
 
 
-def attached_plan(edge_index: torch.Tensor) -> Optional[EdgePlan]:
-    """The plan that travels with an edge list, None where the list has been written to since."""
+def carried_plan(edge_index: torch.Tensor):
+    """What :func:`attach_plan` left with an edge list, None where the list has been written to since."""
     plan, version = getattr(edge_index, "_mlcgb_plan", (None, None))
     return plan if version is None or version == edge_index._version else None
+
+
+def attached_plan(edge_index: torch.Tensor) -> Optional[EdgePlan]:
+    """The plan that travels with an edge list, None where the list has been written to since."""
+    plan = carried_plan(edge_index)
+    return plan.plan() if isinstance(plan, DeferredPlan) else plan
 
 
 def plan_of(edge_index: torch.Tensor, N: int) -> EdgePlan:

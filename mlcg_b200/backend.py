@@ -316,22 +316,25 @@ class CudaBackend:
             self._run("batch_to_ptr", self.lib.mlcgb_batch_to_ptr, (_ptr(batch), batch.numel(), B, _ptr(ptr), _stream(),), **self._work("batch_to_ptr", locals()))
         return ptr
 
-    def batch_structures(self, batch: torch.Tensor) -> int:
-        """``int(batch[-1]) + 1`` of a sorted int64 batch vector."""
+    def batch_boundaries(self, batch: torch.Tensor) -> torch.Tensor:
+        """The boundaries of the ``int(batch[-1]) + 1`` structures of a sorted int64 batch vector."""
         _need_cuda(batch)
         batch = batch.contiguous()
-        host = ctypes.c_int64()
+        N, host = batch.numel(), ctypes.c_int64()
+        ptr = torch.empty(N + 1, dtype=torch.int64, device=batch.device)
         with _on(batch.device):
-            _lib.check(self.lib.mlcgb_batch_structures(_ptr(batch), batch.numel(), ctypes.addressof(host), _stream()), "batch_structures")
-        return host.value
+            _lib.check(self.lib.mlcgb_batch_boundaries(_ptr(batch), N, N, _ptr(ptr), ctypes.addressof(host), _stream()), "batch_boundaries")
+        B = host.value
+        return ptr[:B + 1] if 0 <= B <= N else self.batch_to_ptr(batch, B)
 
     def radius_graph(self, pos, ptr, r, max_num_neighbors, loop, rule, want_distance=False, want_batch=True, exclude=None, n_atoms=None, want_index=True,
-                     want_plan=False):
+                     want_plan=False, want_rows=True):
         """Returns dict(edge_index[2,E] i64, distance|None, mapping_batch|None, row0, row1 (i32), offsets[N+1] i64, status int).
         ``exclude``: ``(exclude_pair_xs, ptr_exclude_pair_xs)`` int64 as ``mlcg::radius_cuda`` takes them (rule "native" only).
         ``n_atoms`` (int64 [B] on the device) in place of ``ptr`` (None then; the boundaries come back under ``"ptr"``).
         ``want_plan``: also twin, sel and pair_of as :meth:`pair_plan` gives them, or None under these keys where a list was cut short,
-        has loops or exclusions, or has no edges; ``want_index=False``: no int64 edge index."""
+        has loops or exclusions, or has no edges; ``want_index=False``: no int64 edge index; ``want_rows=False`` (an index and no plan
+        then): None for row0 and row1."""
         _need_cuda(pos, ptr, n_atoms)
         ptr, n_atoms = (None if t is None else t.contiguous() for t in (ptr, n_atoms))
         ex_xs = ex_ptr = None
@@ -376,12 +379,40 @@ class CudaBackend:
                 pad = -E % 8        # (row1 on a 32-byte boundary)
                 r0, _, r1, twin, pair_of, sel = torch.empty(4 * E + pad + E // 2, dtype=torch.int32, device=dev).split((E, pad, E, E, E, E // 2))
             else:
-                r0, r1 = torch.empty(2 * E, dtype=torch.int32, device=dev).split((E, E))
+                r0, r1 = torch.empty(2 * E, dtype=torch.int32, device=dev).split((E, E)) if want_rows else (None, None)
             self._run("radius_fill", self.lib.mlcgb_graph_finish, common + (
                 _ptr(ptr), N, B, float(r), loop, _ptr(ex_xs), _ptr(ex_ptr), _ptr(ws), wsb, _ptr(offsets), E, _ptr(ei), _ptr(dist), _ptr(mb), _ptr(r0),
                 _ptr(r1), _ptr(twin), _ptr(sel), _ptr(pair_of), int(host[3] != 0), _ptr(self._sticky_status(dev)), _stream()), **self._work("radius_fill", locals()))
         return dict(edge_index=ei, distance=dist, mapping_batch=mb, row0=r0, row1=r1, offsets=offsets, status=st, ptr=ptr, twin=twin, sel=sel,
                     pair_of=pair_of)
+
+    small_graph_points = 2048       # what mlcgb_graph_small_begin takes
+
+    def radius_graph_small(self, pos, batch, r, max_num_neighbors, loop, rule, want_distance=False):
+        """:meth:`radius_graph` of 1 to 2048 points with their sorted batch vector (int64; None: one structure): edge_index, distance,
+        offsets and status, nothing else."""
+        _need_cuda(pos, batch)
+        batch = None if batch is None else batch.contiguous()
+        pos = pos.detach().contiguous()
+        N, dev = pos.shape[0], pos.device
+        dt, loop = _dt(pos), int(bool(loop))
+        with _on(dev):
+            pend = self._take_pending(dev)
+            wsb = self.lib.mlcgb_graph_workspace_bytes(N, 1, dt)
+            ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
+            offsets = torch.empty(N + 1, dtype=torch.int64, device=dev)
+            host = (ctypes.c_int64 * 4)()
+            self._run("radius_count", self.lib.mlcgb_graph_small_begin, (
+                _ptr(pos), dt, _ptr(batch), N, float(r), int(max_num_neighbors), loop, int(rule), _ptr(ws), wsb, _ptr(offsets),
+                _ptr(pend[0][0]) if pend else None, host, _stream()))
+            E = host[0]
+            if pend and host[2]:
+                self._raise_pending([int(host[2])], pend)
+            ei = torch.empty((2, E), dtype=torch.int64, device=dev)
+            dist = torch.empty(E, dtype=pos.dtype, device=dev) if want_distance else None
+            self._run("radius_fill", self.lib.mlcgb_graph_small_finish, (_ptr(pos), dt, _ptr(batch), N, _ptr(ws), wsb, _ptr(offsets), E, _ptr(ei), _ptr(dist),
+                                                                         _stream()))
+        return dict(edge_index=ei, distance=dist, offsets=offsets, status=int(host[1]))
 
     def radius_graph_pbc(self, pos, ptr, cells, repeats, r, max_num_neighbors, loop, want_distance=False, want_batch=True):
         """Radius graph of periodic structures: dict(edge_index [2,E] i64 (row 0 = centre), cell_shifts [E,3], distance|None,

@@ -1573,15 +1573,18 @@ extern "C" int mlcgb_debug_radius_phase_cycles(unsigned long long *out, int n, i
 }
 #endif
 
-__global__ void batch_to_ptr_kernel(const int64_t *__restrict__ batch, int64_t N, int64_t B, int64_t *__restrict__ ptr) {
-    const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b > B) return;
+__device__ __forceinline__ int64_t first_at_least(const int64_t *__restrict__ batch, int64_t N, int64_t b) {
     int64_t lo = 0, hi = N;  // first index with batch[idx] >= b
     while (lo < hi) {
         const int64_t mid = (lo + hi) >> 1;
         if (batch[mid] < b) lo = mid + 1; else hi = mid;
     }
-    ptr[b] = lo;
+    return lo;
+}
+__global__ void batch_to_ptr_kernel(const int64_t *__restrict__ batch, int64_t N, int64_t B, int64_t *__restrict__ ptr) {
+    const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (b > B) return;
+    ptr[b] = first_at_least(batch, N, b);
 }
 
 __global__ void edge_twin_kernel(const int32_t *__restrict__ row0, const int32_t *__restrict__ row1,
@@ -2275,6 +2278,14 @@ __device__ __forceinline__ void publish(const Publish &p, int64_t edges, int sta
 
 __global__ void last_of_kernel(const int64_t *__restrict__ last, Publish p) { publish(p, *last, 0); }
 
+// The same and the boundaries, for up to `most` structures: the host reads on while they are looked for
+__global__ void batch_boundaries_kernel(const int64_t *__restrict__ batch, int64_t N, int64_t most, int64_t *__restrict__ ptr, Publish p) {
+    const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, last = batch[N - 1];
+    if (b == 0) publish(p, last, 0);
+    if (b > last + 1 || b > most) return;
+    ptr[b] = first_at_least(batch, N, b);
+}
+
 __global__ void __launch_bounds__(kScanBlock) sizes_to_ptr_kernel(const int64_t *__restrict__ sizes, int64_t B, int64_t *__restrict__ ptr) {
     __shared__ int64_t s_warp[33];
     int64_t carry = 0;
@@ -2331,18 +2342,53 @@ __device__ __forceinline__ int structure_of(const int *s_ptr, int64_t B, int i) 
     return lo;
 }
 
-template <typename T>
+// The structure of point i as the run of its entry in a sorted batch vector of at most kMaskNodes points, by the whole warp: 32 probes,
+// then the stretch between two of them.  Two rounds of loads, and neither the number of structures nor their boundaries are needed (a
+// host read and two launches: 320 points in 16 structures took 80 us with them).  An unsorted vector gives some range inside [0, N].
+__device__ __forceinline__ void structure_run(const int64_t *__restrict__ batch, int N, int i, int lane, int &lo, int &hi) {
+    static_assert(kMaskNodes <= 32 * 64, "a stretch is two entries per lane");
+    const unsigned full = 0xffffffffu;
+    const int step = (N + 31) >> 5;
+    const int64_t b = batch[i];
+    const bool in = lane * step < N;
+    const int64_t v = in ? batch[lane * step] : 0;
+    const int c0 = __popc(__ballot_sync(full, in && v < b)), c1 = __popc(__ballot_sync(full, in && v <= b));
+    // entries before stretch c - 1 are below, those from probe c on are not: what lies between is looked at one by one
+    const int s0 = c0 ? (c0 - 1) * step + 1 : 0, s1 = c1 ? (c1 - 1) * step + 1 : 0;
+    const int t0 = c0 ? min(c0 * step, N) : 0, t1 = c1 ? min(c1 * step, N) : 0;
+    bool f[4];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int q0 = s0 + 32 * u + lane, q1 = s1 + 32 * u + lane;
+        f[u] = q0 < t0 && batch[q0] < b;
+        f[2 + u] = q1 < t1 && batch[q1] <= b;
+    }
+    lo = s0 + __popc(__ballot_sync(full, f[0])) + __popc(__ballot_sync(full, f[1]));
+    hi = s1 + __popc(__ballot_sync(full, f[2])) + __popc(__ballot_sync(full, f[3]));
+}
+
+// BATCH: `ptr` is the batch vector (NULL: one structure) and B means nothing
+template <typename T, bool BATCH>
 __global__ void __launch_bounds__(256)
 mask_count_kernel(const T *__restrict__ pos, const int64_t *__restrict__ sizes, int64_t *__restrict__ ptr, int64_t N, int64_t B, T r2, int64_t max_nn,
                   int loop, int rule, uint2 *__restrict__ masks, int words, int32_t *__restrict__ deg, int32_t *__restrict__ upper,
                   int32_t *__restrict__ uoff, int64_t *__restrict__ offsets, unsigned *__restrict__ ticket, int32_t *__restrict__ status,
                   int64_t capacity /* < 0: none */, int64_t *__restrict__ counts, int32_t *__restrict__ sticky, Publish pub) {
-    __shared__ int s_ptr[kMaskStructs + 1];
+    __shared__ int s_ptr[BATCH ? 1 : kMaskStructs + 1];
     __shared__ int s_last, s_wd[8], s_wu[8];
-    load_boundaries(s_ptr, sizes, ptr, B);
+    if constexpr (!BATCH) load_boundaries(s_ptr, sizes, ptr, B);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int64_t ci = (int64_t)blockIdx.x * 8 + warp; ci < N; ci += (int64_t)gridDim.x * 8) {
-        const int i = (int)ci, b = structure_of(s_ptr, B, i), lo = s_ptr[b], n = min(s_ptr[b + 1], (int)N) - lo, il = i - lo;
+        const int i = (int)ci;
+        int lo = 0, hi = (int)N;
+        if constexpr (BATCH) {
+            if (ptr) structure_run(ptr, (int)N, i, lane, lo, hi);
+        } else {
+            const int b = structure_of(s_ptr, B, i);
+            lo = s_ptr[b];
+            hi = min(s_ptr[b + 1], (int)N);
+        }
+        const int n = hi - lo, il = i - lo;
         const T xi = pos[3 * ci], yi = pos[3 * ci + 1], zi = pos[3 * ci + 2];
         unsigned m0 = 0, m1 = 0;                       // words `lane` and `32 + lane` of the row
         for (int jb = 0; jb < n; jb += 32) {
@@ -2447,19 +2493,28 @@ mask_count_kernel(const T *__restrict__ pos, const int64_t *__restrict__ sizes, 
     }
 }
 
-template <typename T>
+template <typename T, bool BATCH>
 __global__ void __launch_bounds__(256)
 mask_fill_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, int64_t N, int64_t B, const uint2 *__restrict__ masks, int words,
                  const int32_t *__restrict__ upper, const int32_t *__restrict__ uoff, const int64_t *__restrict__ offsets, FillOut out,
                  int32_t *__restrict__ twin, int32_t *__restrict__ sel, int32_t *__restrict__ pair_of, int32_t *__restrict__ sticky) {
-    __shared__ int s_ptr[kMaskStructs + 1];
-    load_boundaries(s_ptr, nullptr, const_cast<int64_t *>(ptr), B);
+    __shared__ int s_ptr[BATCH ? 1 : kMaskStructs + 1];
+    if constexpr (!BATCH) load_boundaries(s_ptr, nullptr, const_cast<int64_t *>(ptr), B);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt = lanemask_lt();
     const int64_t P = offsets[N] >> 1;
     if (twin && (offsets[N] & 1) && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(sticky, (int)kAsymmetric);
     for (int64_t ci = (int64_t)blockIdx.x * 8 + warp; ci < N; ci += (int64_t)gridDim.x * 8) {
-        const int i = (int)ci, b = structure_of(s_ptr, B, i), lo = s_ptr[b], n = min(s_ptr[b + 1], (int)N) - lo, il = i - lo;
+        const int i = (int)ci;
+        int b = 0, lo = 0, hi = (int)N;
+        if constexpr (BATCH) {
+            if (ptr) structure_run(ptr, (int)N, i, lane, lo, hi);
+        } else {
+            b = structure_of(s_ptr, B, i);
+            lo = s_ptr[b];
+            hi = min(s_ptr[b + 1], (int)N);
+        }
+        const int n = hi - lo, il = i - lo;
         const int64_t off = offsets[i];
         const int kept = (int)(offsets[i + 1] - off), nw = (n + 31) >> 5;
         if (kept == 0) continue;
@@ -2790,19 +2845,19 @@ __global__ void __launch_bounds__(kScanBlock) scan2_apply_kernel(const int32_t *
     }
 }
 
-template <typename T>
+template <typename T, bool BATCH = false>
 static int mask_count_launch(const void *pos, const int64_t *sizes, int64_t *ptr, int64_t N, int64_t B, double r, int64_t max_nn, int loop, int rule,
                              char *w, const GraphLayout &L, int64_t *offsets, int64_t capacity, int64_t *counts, int32_t *sticky, const Publish &pub,
                              cudaStream_t st) {
-    mask_count_kernel<T><<<grid_for(N, 8, 1), 256, 0, st>>>((const T *)pos, sizes, ptr, N, B, (T)(r * r), max_nn, loop, rule, (uint2 *)(w + L.masks),
+    mask_count_kernel<T, BATCH><<<grid_for(N, 8, 1), 256, 0, st>>>((const T *)pos, sizes, ptr, N, B, (T)(r * r), max_nn, loop, rule, (uint2 *)(w + L.masks),
                                                          (int)((N + 31) / 32), (int32_t *)(w + L.deg), (int32_t *)(w + L.upper), (int32_t *)(w + L.uoff),
                                                          offsets, (unsigned *)(w + L.header + 16), (int32_t *)(w + L.header), capacity, counts, sticky, pub);
     return check_launch();
 }
-template <typename T>
+template <typename T, bool BATCH = false>
 static int mask_fill_launch(const void *pos, const int64_t *ptr, int64_t N, int64_t B, char *w, const GraphLayout &L, const int64_t *offsets,
                             const FillOut &out, int32_t *twin, int32_t *sel, int32_t *pair_of, int32_t *sticky, cudaStream_t st) {
-    mask_fill_kernel<T><<<grid_for(N, 8, 2), 256, 0, st>>>((const T *)pos, ptr, N, B, (const uint2 *)(w + L.masks), (int)((N + 31) / 32),
+    mask_fill_kernel<T, BATCH><<<grid_for(N, 8, 2), 256, 0, st>>>((const T *)pos, ptr, N, B, (const uint2 *)(w + L.masks), (int)((N + 31) / 32),
                                                         (const int32_t *)(w + L.upper), (const int32_t *)(w + L.uoff), offsets, out, twin, sel, pair_of, sticky);
     return check_launch();
 }
@@ -2855,6 +2910,59 @@ int mlcgb_batch_structures(const int64_t *batch, int64_t N, int64_t *host_out, v
     if (int rc = wait_published(pub.seq, pub.host, st)) return rc;
     *host_out = pub.host[1] + 1;
     return MLCGB_OK;
+}
+
+int mlcgb_batch_boundaries(const int64_t *batch, int64_t N, int64_t most, int64_t *ptr, int64_t *host_out, void *stream) {
+    if (N <= 0 || most < 0 || !batch || !ptr || !host_out) return MLCGB_E_ARG;
+    auto st = (cudaStream_t)stream;
+    Publish pub;
+    pub.host = g_host_slot.get();
+    if (!pub.host) return check_launch();
+    pub.seq = ++g_host_slot.seq;
+    batch_boundaries_kernel<<<(unsigned)((most + 256) / 256), 256, 0, st>>>(batch, N, most, ptr, pub);
+    if (int rc = check_launch()) return rc;
+    if (int rc = wait_published(pub.seq, pub.host, st)) return rc;
+    *host_out = pub.host[1] + 1;
+    return MLCGB_OK;
+}
+
+int mlcgb_graph_small_begin(const void *pos, int dtype, const int64_t *batch, int64_t N, double r, int64_t max_nn, int loop, int rule, void *workspace,
+                            size_t workspace_bytes, int64_t *offsets, const int32_t *pending_status, int64_t *host_out, void *stream) {
+    TimelineScope timeline_scope("radius_count", stream);
+    if (N <= 0 || max_nn < 0 || !pos || !workspace || !offsets || !host_out) return MLCGB_E_ARG;
+    if (N > kMaskNodes) return MLCGB_E_LIMIT;
+    if ((rule != MLCGB_RULE_NATIVE && rule != MLCGB_RULE_CLUSTER) || (dtype != MLCGB_F32 && dtype != MLCGB_F64)) return MLCGB_E_ARG;
+    const GraphLayout L = graph_layout(N, 1, dtype);
+    if (workspace_bytes < L.total) return MLCGB_E_WORKSPACE;
+    auto st = (cudaStream_t)stream;
+    char *w = (char *)workspace;
+    Publish pub;
+    pub.host = g_host_slot.get();
+    if (!pub.host) return check_launch();
+    pub.seq = ++g_host_slot.seq;
+    pub.pending = pending_status;
+    cudaMemsetAsync(w + L.header, 0, 32, st);
+    int rc = MLCGB_DISPATCH_DTYPE(dtype, [&] {
+        return mask_count_launch<scalar_t, true>(pos, nullptr, const_cast<int64_t *>(batch), N, 1, r, max_nn, loop, rule, w, L, offsets, -1, nullptr, nullptr, pub, st);
+    });
+    if (rc || (rc = wait_published(pub.seq, pub.host, st))) return rc;
+    for (int i = 0; i < 4; i++) host_out[i] = pub.host[1 + i];
+    return MLCGB_OK;
+}
+
+int mlcgb_graph_small_finish(const void *pos, int dtype, const int64_t *batch, int64_t N, void *workspace, size_t workspace_bytes, const int64_t *offsets,
+                             int64_t E, int64_t *edge_index, void *distance, void *stream) {
+    TimelineScope timeline_scope("radius_fill", stream);
+    if (N <= 0 || E < 0) return MLCGB_E_ARG;
+    if (N > kMaskNodes) return MLCGB_E_LIMIT;
+    if (E == 0) return MLCGB_OK;
+    if (!pos || !workspace || !offsets || !edge_index) return MLCGB_E_ARG;
+    const GraphLayout L = graph_layout(N, 1, dtype);
+    if (workspace_bytes < L.total) return MLCGB_E_WORKSPACE;
+    return MLCGB_DISPATCH_DTYPE(dtype, [&] {
+        return mask_fill_launch<scalar_t, true>(pos, batch, N, 1, (char *)workspace, L, offsets, FillOut{edge_index, edge_index + E, nullptr, distance, nullptr, nullptr},
+                                                nullptr, nullptr, nullptr, nullptr, (cudaStream_t)stream);
+    });
 }
 
 size_t mlcgb_graph_workspace_bytes(int64_t N, int64_t B, int dtype) {
@@ -2917,7 +3025,7 @@ int mlcgb_graph_finish(const void *pos, int dtype, const int64_t *ptr, int64_t N
     TimelineScope timeline_scope("radius_fill", stream);
     if (N <= 0 || B <= 0 || E < 0) return MLCGB_E_ARG;
     if (E == 0) return MLCGB_OK;
-    if (!pos || !ptr || !workspace || !offsets || !row0 || !row1 || !sticky_status) return MLCGB_E_ARG;
+    if (!pos || !ptr || !workspace || !offsets || !sticky_status || !row0 != !row1 || (!row0 && (twin || !edge_index))) return MLCGB_E_ARG;
     if ((!twin != !sel) || (!twin != !pair_of) || (twin && (loop || exclude_pair_xs || (E & 1)))) return MLCGB_E_ARG;
     if (twin && E >= (int64_t)1 << 31) return MLCGB_E_LIMIT;
     const GraphLayout L = graph_layout(N, B, dtype);

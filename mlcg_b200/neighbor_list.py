@@ -10,7 +10,7 @@ from typing import Dict, Mapping, Optional, Tuple
 
 import torch
 
-from .autograd import EdgePlan, attach_plan, attached_plan, edge_distances
+from .autograd import DeferredPlan, EdgePlan, attach_plan, carried_plan, edge_distances
 from .backend import STATUS_TRUNCATED, get_backend
 
 RULE_NATIVE, RULE_CLUSTER = 0, 1
@@ -34,8 +34,9 @@ def _structure_ptr(x, batch, batch_size):
         raise ValueError("batch must have one entry per point")
     batch = batch.to(torch.int64)
     if batch_size is None:                                # sorted batch vector: last entry is the maximum
-        count = getattr(be, "batch_structures", None)
-        batch_size = 1 if N == 0 else int(batch[-1]) + 1 if count is None else count(batch)
+        if N > 0 and hasattr(be, "batch_boundaries"):
+            return be.batch_boundaries(batch)
+        batch_size = 1 if N == 0 else int(batch[-1]) + 1
     return be.batch_to_ptr(batch, batch_size)
 
 
@@ -57,14 +58,34 @@ def _graph(x, r, ptr, loop, max_num_neighbors, rule, want_distance=False, exclud
     return res
 
 
+def _edges(x, r, batch, batch_size, ptr, loop, max_num_neighbors, rule, want_distance=False, exclude=None):
+    """``(edge_index, distance | None)`` for callers that return edges: their plan is made if an operator is given the list (plan and int32
+    rows with the list: 1815 us for 65 M edges, without them 1004).  Structures from ``ptr``, or from ``batch`` and ``batch_size``."""
+    be, N = get_backend(), x.shape[0]
+    small = getattr(be, "small_graph_points", 0)
+    if ptr is None and 0 < N <= small and exclude is None and batch_size is None and (batch is None or batch.numel() == N):
+        res = be.radius_graph_small(_as_3d(x), None if batch is None else batch.to(torch.int64), r, max_num_neighbors, loop, rule, want_distance)
+    else:
+        more = {"want_rows": False} if small else {}
+        ptr = _structure_ptr(x, batch, batch_size) if ptr is None else ptr
+        res = be.radius_graph(_as_3d(x), ptr, r, max_num_neighbors, loop, rule, want_distance=want_distance, want_batch=False, exclude=exclude, **more)
+    # an exclusion list need not hold both directions of a pair: such a graph is not taken to be symmetric
+    symmetric = exclude is None and not res["status"] & STATUS_TRUNCATED
+    return attach_plan(res["edge_index"], DeferredPlan(res["edge_index"], res["offsets"], N, symmetric, bool(loop))), res["distance"]
+
+
+def _differentiated(x) -> bool:
+    """Whether somebody may differentiate through ``x``, backward or forward."""
+    return (x.requires_grad and torch.is_grad_enabled()) or torch.autograd.forward_ad._current_level >= 0
+
+
 def radius_graph(x: torch.Tensor, r: float, batch: Optional[torch.Tensor] = None, loop: bool = False,
                  max_num_neighbors: int = 32, flow: str = "source_to_target", num_workers: int = 1,
                  batch_size: Optional[int] = None) -> torch.Tensor:
     """Same call and result as ``torch_cluster.radius_graph`` (torch_impl.py:216-224 passes
     ``flow="target_to_source"``: row 0 = centre, row 1 = neighbour, centre-major, neighbours ascending)."""
     assert flow in ("source_to_target", "target_to_source")
-    res = _graph(x, r, _structure_ptr(x, batch, batch_size), loop, max_num_neighbors, RULE_CLUSTER)
-    ei = res["edge_index"]
+    ei, _ = _edges(x, r, batch, batch_size, None, loop, max_num_neighbors, RULE_CLUSTER)
     if flow == "target_to_source":
         return ei
     out = ei.flip(0)
@@ -84,10 +105,7 @@ def radius_cuda(x: torch.Tensor, ptr_x: Optional[torch.Tensor], r: float, max_nu
     exclude = None
     if exclude_pair_xs is not None and exclude_pair_xs.numel() > 0:
         exclude = (exclude_pair_xs, ptr_exclude_pair_xs)
-    if ptr_x is None:
-        ptr_x = torch.tensor([0, x.shape[0]], dtype=torch.int64, device=x.device)
-    res = _graph(x, r, ptr_x.to(torch.int64), not ignore_same_index, max_num_neighbors, RULE_NATIVE, want_distance=True, exclude=exclude)
-    return res["edge_index"], res["distance"]
+    return _edges(x, r, None, None, None if ptr_x is None else ptr_x.to(torch.int64), not ignore_same_index, max_num_neighbors, RULE_NATIVE, want_distance=True, exclude=exclude)
 
 
 def exclusion_pair_to_ptr(exc_pair_index: torch.Tensor, num_nodes: int) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -117,6 +135,9 @@ def radius_distance(x: torch.Tensor, r: float, batch: Optional[torch.Tensor] = N
     exclude = None
     if exclude_pair_indices is not None and exclude_pair_indices.numel() > 0:
         exclude = exclusion_pair_to_ptr(exclude_pair_indices.to(x.device), x.shape[0])
+    if not _differentiated(x):
+        edge_index, distance = _edges(x, r, batch, batch_size, None, loop, max_num_neighbors, RULE_NATIVE, want_distance=True, exclude=exclude)
+        return distance, edge_index
     res = _graph(x, r, _structure_ptr(x, batch, batch_size), loop, max_num_neighbors, RULE_NATIVE, exclude=exclude)
     # the distance goes through the differentiable geometry operators, so that derivatives of any
     # order with respect to x exist (the reference hand-writes two orders, radius.py:123-158)
@@ -131,7 +152,7 @@ def make_neighbor_list(tag: str, order: int, index_mapping: torch.Tensor, mappin
         raise RuntimeError(f"index_mapping shape does not match the order:{index_mapping.shape[0]} != {order}")
     if mapping_batch is None:
         mapping_batch = torch.zeros((index_mapping.shape[1],) if len(index_mapping) > 0 else (0,), dtype=torch.long)
-    plan = attached_plan(index_mapping) if torch.is_tensor(index_mapping) else None
+    plan = carried_plan(index_mapping) if torch.is_tensor(index_mapping) else None
     im = torch.as_tensor(index_mapping, dtype=torch.long)
     if plan is not None:
         attach_plan(im, plan)

@@ -308,3 +308,54 @@ def test_boundaries_of_any_stride():
     ei, dist = mlcg_b200.neighbor_list.radius_cuda(turned, wide[:, 0], 3.0, 1000, True)
     want, want_d = radius_ref.radius_graph_c(pos, ptr, 3.0, 1000, False, "native", with_distance=True)
     assert np.array_equal(ei.cpu().numpy(), want) and np.array_equal(dist.cpu().numpy(), want_d)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("sizes", [[1], [31, 33], [1, 0, 2, 0], [63] * 4 + [1], [2048], [1] * 2048, [2047, 1], [1024, 0, 1024], [2049], [500, 0, 1800]])
+def test_edges_from_a_batch_vector(sizes, dtype):
+    """Up to 2048 points structures are found in the batch vector itself (at most 64 entries between two probes of a warp); above, their
+    boundaries come with the number of structures.  The plan that an operator asks for later is the one of the list."""
+    from mlcg_b200.autograd import attached_plan
+    rng = np.random.default_rng(sum(sizes) + len(sizes))
+    ptr = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    pos = (rng.random((int(ptr[-1]), 3)) * max(sizes) ** (1 / 3) * 1.7).astype(dtype)
+    batch = np.repeat(np.arange(len(sizes)), sizes)
+    x, b = torch.as_tensor(pos, device=DEV), torch.as_tensor(batch, device=DEV)
+    for loop, cap in ((False, 1000), (True, 1000), (False, 3)):
+        ei = mlcg_b200.radius_graph(x, 3.0, b, loop, cap, flow="target_to_source")
+        want = radius_ref.radius_graph_c(pos, ptr, 3.0, cap, loop, "cluster")
+        assert np.array_equal(ei.cpu().numpy(), want)
+        plan = attached_plan(ei)
+        assert plan is attached_plan(ei) and torch.equal(torch.stack([plan.row0, plan.row1]).long(), ei)
+        if plan.symmetric:
+            assert torch.equal(ei.flip(0), ei[:, plan.perm_in.long()])
+    d, ei = mlcg_b200.radius_distance(x, 3.0, b, False, 1000)
+    want, wd = radius_ref.radius_graph_c(pos, ptr, 3.0, 1000, False, "native", with_distance=True)
+    assert np.array_equal(ei.cpu().numpy(), want) and np.array_equal(d.cpu().numpy(), wd)
+    y = x.clone().requires_grad_()
+    dg, eg = mlcg_b200.radius_distance(y, 3.0, b, False, 1000)
+    # (the differentiable distance sums its squares in another order: two roundings more)
+    assert dg.requires_grad and torch.equal(eg, ei) and torch.allclose(dg, d, rtol=4 * np.finfo(dtype).eps, atol=0)
+    if len(sizes) == 1:
+        assert torch.equal(mlcg_b200.radius_graph(x, 3.0, None, False, 1000), mlcg_b200.radius_graph(x, 3.0, b, False, 1000))
+        assert torch.equal(mlcg_b200.neighbor_list.radius_cuda(x, None, 3.0, 1000, True)[0], ei)
+
+
+def test_plan_of_edges_on_another_stream():
+    """What was made on one stream is not handed to another that nothing orders behind it, nor kept out of a recording."""
+    from mlcg_b200.autograd import attached_plan
+    x = torch.rand(300, 3, device=DEV) * 9
+    ei = mlcg_b200.radius_graph(x, 3.0, torch.zeros(300, dtype=torch.int64, device=DEV), max_num_neighbors=1000, flow="target_to_source")
+    here = attached_plan(ei)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        there = attached_plan(ei)
+    torch.cuda.synchronize()
+    assert there is not here and torch.equal(there.perm_in, here.perm_in) and torch.equal(there.pair_index(), here.pair_index())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        recorded = attached_plan(ei)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(recorded.perm_in, here.perm_in) and attached_plan(ei) is not recorded
