@@ -516,6 +516,15 @@ int mlcgb_schnet_evaluate(const void *pos, const int64_t *types, const int64_t *
                           const mlcgb_schnet_weights *w, int precision, int negate, int training, void *graph_workspace, size_t graph_bytes,
                           void *workspace, size_t workspace_bytes, void *energy, void *grad_pos, const int32_t *pending_status, int32_t *status,
                           int64_t *host, void *stream);
+/* The same for batches that mlcgb_schnet_evaluate_fixed_ok takes (1) without reading anything on the host: lists of `capacity` edges (an
+ * even number; the workspaces are sized with it in place of E), the neighbours in the caller's buffer where one is given.  A list that has more, or was cut short, sets its bit in status and is
+ * evaluated as one without edges. */
+int mlcgb_schnet_evaluate_fixed_ok(int64_t N, int64_t B, const mlcgb_schnet_weights *w);
+int mlcgb_schnet_evaluate_fixed(const void *pos, const int64_t *types, const int64_t *n_atoms, const int64_t *struct_ptr, int64_t N, int64_t B, double r,
+                                int64_t max_nn, const mlcgb_rbf_spec *rbf, int conv_cutoff_kind, double conv_lower, double conv_upper,
+                                const mlcgb_schnet_weights *w, int precision, int negate, int64_t capacity, int32_t *neighbours /* [capacity] or NULL */,
+                                void *graph_workspace, size_t graph_bytes,
+                                void *workspace, size_t workspace_bytes, void *energy, void *grad_pos, int32_t *status, void *stream);
 /* Byte offsets: at [0, 1] structure boundaries (where n_atoms was given) and CSR offsets in graph_workspace; at [2..7] row0, row1,
  * twin, pair_of, sel and the forward workspace in workspace. */
 void mlcgb_schnet_evaluate_lists(int64_t N, int64_t B, int64_t E, int64_t *at /* [8] */);

@@ -112,6 +112,9 @@ SIGNATURES = {
     "mlcgb_schnet_evaluate_lists": (None, [c_i64, c_i64, c_i64, c_vp]),
     "mlcgb_schnet_evaluate": (c_int, [c_vp, c_vp, c_vp, c_vp, c_i64, c_i64, c_dbl, c_i64, ctypes.POINTER(RbfSpecStruct), c_int, c_dbl, c_dbl,
                                       ctypes.POINTER(SchnetWeightsStruct), c_int, c_int, c_int, c_vp, c_sz, c_vp, c_sz, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "mlcgb_schnet_evaluate_fixed_ok": (c_int, [c_i64, c_i64, ctypes.POINTER(SchnetWeightsStruct)]),
+    "mlcgb_schnet_evaluate_fixed": (c_int, [c_vp, c_vp, c_vp, c_vp, c_i64, c_i64, c_dbl, c_i64, ctypes.POINTER(RbfSpecStruct), c_int, c_dbl, c_dbl,
+                                            ctypes.POINTER(SchnetWeightsStruct), c_int, c_int, c_i64, c_vp, c_vp, c_sz, c_vp, c_sz, c_vp, c_vp, c_vp, c_vp]),
     "mlcgb_graph_workspace_bytes": (c_sz, [c_i64, c_i64, c_int]),
     "mlcgb_graph_begin": (c_int, [c_vp, c_int, c_vp, c_vp, c_i64, c_i64, c_dbl, c_i64, c_int, c_int, c_vp, c_vp, c_vp, c_sz, c_vp, c_vp, c_vp, c_vp]),
     "mlcgb_batch_boundaries": (c_int, [c_vp, c_i64, c_i64, c_vp, c_vp, c_vp]),

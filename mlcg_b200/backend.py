@@ -912,6 +912,34 @@ class CudaBackend:
         ws = ws[:size(N, B, E, spec.num_rbf, ref, 1)]          # (saved with the size that its edges ask for, not that of the guess)
         return energy, grad, E, ForceMatchingState(N, B, E, (types, spec.p0, spec.p1, ws, graph_ws, ptr), places, spec, conv_cut, weights)
 
+    def schnet_fixed_ok(self, N, B, weights) -> bool:
+        return bool(self.lib.mlcgb_schnet_evaluate_fixed_ok(N, B, ctypes.byref(weights[0])))
+
+    def schnet_fixed(self, pos, types, n_atoms, ptr, r, max_num_neighbors, spec: RbfSpec, conv_cut, weights, precision, forces, rows):
+        """:meth:`schnet_from_positions` for batches that :meth:`schnet_fixed_ok` takes without a host read: lists of as many edges as the int32
+        ``rows`` [2, capacity] hold (the neighbours go there), more of them are reported by the deferred status check.  ``(energy, gradient or
+        forces)``."""
+        _need_cuda(pos, types, n_atoms, ptr, rows)
+        capacity = rows.shape[1]
+        w, _keep = weights
+        pos = pos.detach().contiguous()
+        N, dev = pos.shape[0], pos.device
+        B = ptr.numel() - 1 if n_atoms is None else n_atoms.numel()
+        s, keep = self._spec(spec, torch.float32)
+        status, lib, ref = self._sticky_status(dev), self.lib, ctypes.byref(w)
+        with _on(dev):
+            energy = torch.empty(B, dtype=torch.float32, device=dev)
+            grad = torch.empty((N, 3), dtype=torch.float32, device=dev)
+            size = lib.mlcgb_schnet_evaluate_workspace_bytes
+            gb, wsb = size(N, B, -1, 0, ref, 0), size(N, B, capacity, spec.num_rbf, ref, 0)
+            graph_ws, ws = torch.empty(gb, dtype=torch.uint8, device=dev), torch.empty(wsb, dtype=torch.uint8, device=dev)
+            _lib.check(lib.mlcgb_schnet_evaluate_fixed(
+                pos.data_ptr(), types.data_ptr(), _ptr(n_atoms), _ptr(ptr), N, B, r, max_num_neighbors, ctypes.byref(s), conv_cut[0], conv_cut[1], conv_cut[2],
+                ref, precision, int(forces), capacity, rows[1].data_ptr(), graph_ws.data_ptr(), gb, ws.data_ptr(), wsb, energy.data_ptr(), grad.data_ptr(), status.data_ptr(),
+                _stream()), "schnet_evaluate_fixed")
+        self.defer_status(status, "SchNet evaluation with a fixed edge capacity")
+        return energy, grad
+
     # ------------------------------------------------------------------ one force-matching step
     @staticmethod
     def train_ok(setup) -> bool:

@@ -217,14 +217,14 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
                               const int32_t *pair_of, const int32_t *twin, int64_t E, int64_t P, const int64_t *counts,
                               const mlcgb_rbf_spec *rbf, int conv_cutoff_kind, double conv_lower, double conv_upper,
                               const mlcgb_schnet_weights *w, int precision, void *workspace, size_t workspace_bytes, void *energy,
-                              void *grad_pos, float grad_sign, int32_t *status, void *stream) {
+                              void *grad_pos, float grad_sign, int32_t *status, void *stream, const SmallGraph *graph = nullptr) {
     const int64_t *pairs_dev = counts ? counts + 1 : nullptr;
     if (N < 0 || B < 0 || E < 0 || P < 0 || !w || !status || !energy || !struct_ptr) return MLCGB_E_ARG;
     if (B == 0) return MLCGB_OK;
     const int64_t H = w->hidden, F = w->filters, H2 = w->conv_out, Wh = w->head_width, L = w->num_blocks;
     if (F != 128 || H > 128 || H2 > 128 || Wh > 128 || (H & 3) || (H2 & 3) || (Wh & 3) || L < 1) return MLCGB_E_LIMIT;
     if (!pos || !types || !offsets || !w->embedding || !w->blocks || !w->head_W || !w->head_b || !w->head_out || !workspace) return MLCGB_E_ARG;
-    if (E > 0 && (!row0 || !row1 || !sel || !pair_of || !twin || 2 * P != E)) return MLCGB_E_ARG;
+    if (E > 0 && ((!row0 && !graph) || !row1 || !sel || !pair_of || !twin || 2 * P != E)) return MLCGB_E_ARG;
     const SchnetLayout lay = schnet_layout(N, E, P, H, F, H2, Wh, L);
     if (workspace_bytes < (size_t)lay.total * sizeof(float)) return MLCGB_E_WORKSPACE;
     float *ws = (float *)workspace;
@@ -255,7 +255,7 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
             f.gagg[l] = ws + (l & 1 ? lay.agg : lay.gxl);
         }
         f.ah = nullptr; f.en = ws + lay.en; f.s = ws + lay.gd; f.want_grad = grad_pos != nullptr; f.status = status;
-        if ((rc = small_start(f, st))) return rc;
+        if ((rc = graph ? small_graph_start(f, *graph, st) : small_start(f, st))) return rc;
         ChainScope chain;
         if ((rc = filters(0, L))) return rc;       // (of all blocks at once: they depend on the distances alone)
         if ((rc = small_forward(f, st))) return rc;
@@ -312,6 +312,18 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
     }
     return finish_launch((const float *)pos, ws + lay.gd, d, row1, offsets, twin, N, (float *)grad_pos, grad_sign, ws + lay.en, struct_ptr, B, (float *)energy, st);
 }
+
+}  // extern "C"
+
+int mlcgb::schnet_eval_small(const void *pos, const int64_t *types, int64_t N, int64_t B, const SmallGraph &g, const mlcgb_rbf_spec *rbf, int conv_cutoff_kind,
+                             double conv_lower, double conv_upper, const mlcgb_schnet_weights *w, int precision, void *workspace, size_t workspace_bytes,
+                             void *energy, void *grad_pos, float grad_sign, int32_t *status, cudaStream_t st) {
+    if (!grad_pos || !small_graph_ok(N, B, w)) return MLCGB_E_LIMIT;
+    return schnet_eval_impl(pos, types, g.ptr, N, B, nullptr, g.row1, g.offsets, g.sel, g.pair_of, g.twin, g.capacity, g.capacity / 2, g.counts, rbf,
+                            conv_cutoff_kind, conv_lower, conv_upper, w, precision, workspace, workspace_bytes, energy, grad_pos, grad_sign, status, st, &g);
+}
+
+extern "C" {
 
 int mlcgb_schnet_eval_counted(const void *pos, const int64_t *types, const int64_t *struct_ptr, int64_t N, int64_t B, const int32_t *row0,
                               const int32_t *row1, const int64_t *offsets, const int32_t *sel, const int32_t *pair_of, const int32_t *twin, int64_t E,

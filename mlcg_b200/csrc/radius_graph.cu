@@ -20,6 +20,7 @@
 //        leaves at once when there are none), and neighbours<FILL> (hits are marked in a bitmask in
 //        shared memory indexed by local point index, per centre, then emitted in ascending order).
 #include "common.cuh"
+#include "small_graph.cuh"
 
 #include <atomic>
 
@@ -2224,8 +2225,6 @@ extern "C" int mlcgb_radius_graph_static(const void *pos, int dtype, const int64
 // ------------------------------------------------------------------------------------------------
 namespace mlcgb {
 
-constexpr int64_t kMaskNodes = 2048;
-constexpr int kMaskStructs = 2048;             // structure boundaries held in shared memory
 
 // Larger batches whose structures have at most 768 points on average: those that do go the same way (mask_rows_kernel); in a batch of
 // large structures the bit rows (192 bytes per point) would be room for nothing.  Graph and plan of 40 000 points in structures of
@@ -2259,23 +2258,6 @@ static GraphLayout graph_layout(int64_t N, int64_t B, int dtype) {
 }
 static inline bool mask_route(int64_t N, int64_t B, const Exclusion &ex) { return N <= kMaskNodes && B <= kMaskStructs && !ex.ptr; }
 
-// Where a kernel leaves {sequence number, edges, status word, another status word} for the waiting host (mapped pinned memory)
-struct Publish {
-    int64_t *host = nullptr;
-    int64_t seq = 0;
-    const int32_t *pending = nullptr;
-    bool cells_known = false;                  // h[4] = 0: no structure of the batch belongs to the cell or warp kernels
-};
-__device__ __forceinline__ void publish(const Publish &p, int64_t edges, int status) {
-    volatile int64_t *h = p.host;
-    h[1] = edges;
-    h[2] = status;
-    if (!p.cells_known) h[4] = 1;
-    h[3] = p.pending ? *reinterpret_cast<const volatile int32_t *>(p.pending) : 0;
-    __threadfence_system();
-    h[0] = p.seq;
-}
-
 __global__ void last_of_kernel(const int64_t *__restrict__ last, Publish p) { publish(p, *last, 0); }
 
 // The same and the boundaries, for up to `most` structures: the host reads on while they are looked for
@@ -2298,48 +2280,6 @@ __global__ void __launch_bounds__(kScanBlock) sizes_to_ptr_kernel(const int64_t 
         __syncthreads();
     }
     if (threadIdx.x == 0) ptr[B] = carry;
-}
-
-// structure boundaries into shared memory: from the sizes (whose prefix sums block 0 also writes out) or from ptr
-__device__ __forceinline__ void load_boundaries(int *s_ptr, const int64_t *sizes, int64_t *ptr, int64_t B) {
-    __shared__ int s_part[8];
-    if (!sizes) {
-        for (int b = threadIdx.x; b <= B; b += 256) s_ptr[b] = (int)ptr[b];
-        __syncthreads();
-        return;
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int carry = 0;
-    for (int64_t b0 = 0; b0 < B; b0 += 256) {
-        const int64_t b = b0 + threadIdx.x;
-        const int v = b < B ? (int)sizes[b] : 0;
-        int inc = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += t;
-        }
-        if (lane == 31) s_part[warp] = inc;
-        __syncthreads();
-        int before = carry;
-        for (int w = 0; w < warp; w++) before += s_part[w];
-        if (b < B) s_ptr[b] = before + inc - v;
-        for (int w = 0; w < 8; w++) carry += s_part[w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) s_ptr[B] = carry;
-    __syncthreads();
-    if (blockIdx.x == 0)
-        for (int b = threadIdx.x; b <= B; b += 256) ptr[b] = s_ptr[b];
-}
-__device__ __forceinline__ int structure_of(const int *s_ptr, int64_t B, int i) {     // last b with s_ptr[b] <= i (empty structures skipped)
-    int lo = 0, hi = (int)B - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (s_ptr[mid] <= i) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
 }
 
 // The structure of point i as the run of its entry in a sorted batch vector of at most kMaskNodes points, by the whole warp: 32 probes,
@@ -2376,7 +2316,7 @@ mask_count_kernel(const T *__restrict__ pos, const int64_t *__restrict__ sizes, 
                   int64_t capacity /* < 0: none */, int64_t *__restrict__ counts, int32_t *__restrict__ sticky, Publish pub) {
     __shared__ int s_ptr[BATCH ? 1 : kMaskStructs + 1];
     __shared__ int s_last, s_wd[8], s_wu[8];
-    if constexpr (!BATCH) load_boundaries(s_ptr, sizes, ptr, B);
+    if constexpr (!BATCH) load_boundaries<256>(s_ptr, sizes, ptr, B);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int64_t ci = (int64_t)blockIdx.x * 8 + warp; ci < N; ci += (int64_t)gridDim.x * 8) {
         const int i = (int)ci;
@@ -2499,7 +2439,7 @@ mask_fill_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, int
                  const int32_t *__restrict__ upper, const int32_t *__restrict__ uoff, const int64_t *__restrict__ offsets, FillOut out,
                  int32_t *__restrict__ twin, int32_t *__restrict__ sel, int32_t *__restrict__ pair_of, int32_t *__restrict__ sticky) {
     __shared__ int s_ptr[BATCH ? 1 : kMaskStructs + 1];
-    if constexpr (!BATCH) load_boundaries(s_ptr, nullptr, const_cast<int64_t *>(ptr), B);
+    if constexpr (!BATCH) load_boundaries<256>(s_ptr, nullptr, const_cast<int64_t *>(ptr), B);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt = lanemask_lt();
     const int64_t P = offsets[N] >> 1;
@@ -2894,6 +2834,14 @@ static int wait_published(int64_t seq, const int64_t *slot, cudaStream_t st) {
     }
 }
 
+int publish_begin(Publish *p) {
+    p->host = g_host_slot.get();
+    if (!p->host) return check_launch();
+    p->seq = ++g_host_slot.seq;
+    return MLCGB_OK;
+}
+int publish_wait(const Publish &p, cudaStream_t st) { return wait_published(p.seq, p.host, st); }
+
 }  // namespace mlcgb
 
 extern "C" {
@@ -2902,12 +2850,10 @@ int mlcgb_batch_structures(const int64_t *batch, int64_t N, int64_t *host_out, v
     if (N <= 0 || !batch || !host_out) return MLCGB_E_ARG;
     auto st = (cudaStream_t)stream;
     Publish pub;
-    pub.host = g_host_slot.get();
-    if (!pub.host) return check_launch();
-    pub.seq = ++g_host_slot.seq;
+    if (int rc = publish_begin(&pub)) return rc;
     last_of_kernel<<<1, 1, 0, st>>>(batch + N - 1, pub);
     if (int rc = check_launch()) return rc;
-    if (int rc = wait_published(pub.seq, pub.host, st)) return rc;
+    if (int rc = publish_wait(pub, st)) return rc;
     *host_out = pub.host[1] + 1;
     return MLCGB_OK;
 }
@@ -2916,12 +2862,10 @@ int mlcgb_batch_boundaries(const int64_t *batch, int64_t N, int64_t most, int64_
     if (N <= 0 || most < 0 || !batch || !ptr || !host_out) return MLCGB_E_ARG;
     auto st = (cudaStream_t)stream;
     Publish pub;
-    pub.host = g_host_slot.get();
-    if (!pub.host) return check_launch();
-    pub.seq = ++g_host_slot.seq;
+    if (int rc = publish_begin(&pub)) return rc;
     batch_boundaries_kernel<<<(unsigned)((most + 256) / 256), 256, 0, st>>>(batch, N, most, ptr, pub);
     if (int rc = check_launch()) return rc;
-    if (int rc = wait_published(pub.seq, pub.host, st)) return rc;
+    if (int rc = publish_wait(pub, st)) return rc;
     *host_out = pub.host[1] + 1;
     return MLCGB_OK;
 }
@@ -2937,15 +2881,13 @@ int mlcgb_graph_small_begin(const void *pos, int dtype, const int64_t *batch, in
     auto st = (cudaStream_t)stream;
     char *w = (char *)workspace;
     Publish pub;
-    pub.host = g_host_slot.get();
-    if (!pub.host) return check_launch();
-    pub.seq = ++g_host_slot.seq;
+    if (int rc = publish_begin(&pub)) return rc;
     pub.pending = pending_status;
     cudaMemsetAsync(w + L.header, 0, 32, st);
     int rc = MLCGB_DISPATCH_DTYPE(dtype, [&] {
         return mask_count_launch<scalar_t, true>(pos, nullptr, const_cast<int64_t *>(batch), N, 1, r, max_nn, loop, rule, w, L, offsets, -1, nullptr, nullptr, pub, st);
     });
-    if (rc || (rc = wait_published(pub.seq, pub.host, st))) return rc;
+    if (rc || (rc = publish_wait(pub, st))) return rc;
     for (int i = 0; i < 4; i++) host_out[i] = pub.host[1 + i];
     return MLCGB_OK;
 }
@@ -2985,9 +2927,7 @@ int mlcgb_graph_begin(const void *pos, int dtype, const int64_t *n_atoms, int64_
     auto st = (cudaStream_t)stream;
     char *w = (char *)workspace;
     Publish pub;
-    pub.host = g_host_slot.get();
-    if (!pub.host) return check_launch();
-    pub.seq = ++g_host_slot.seq;
+    if (int rc = publish_begin(&pub)) return rc;
     pub.pending = pending_status;
     cudaMemsetAsync(w + L.header, 0, 32, st);
     int rc = MLCGB_DISPATCH_DTYPE(dtype, [&] {
@@ -3013,7 +2953,7 @@ int mlcgb_graph_begin(const void *pos, int dtype, const int64_t *n_atoms, int64_
         return check_launch();
     });
     if (rc) return rc;
-    if ((rc = wait_published(pub.seq, pub.host, st))) return rc;
+    if ((rc = publish_wait(pub, st))) return rc;
     for (int i = 0; i < 4; i++) host_out[i] = pub.host[1 + i];
     return MLCGB_OK;
 }

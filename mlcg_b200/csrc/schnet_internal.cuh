@@ -1,6 +1,7 @@
 // Pieces of the whole-model sequences (interaction.cu, train.cu) that live in files of their own.
 #pragma once
 #include "common.cuh"
+#include "small_graph.cuh"
 
 namespace mlcgb {
 
@@ -47,6 +48,29 @@ struct SmallForward {                      // per node unless said otherwise; NU
     int want_grad;
     int32_t *status;
 };
+// The radius graph and pair plan of up to kMaskNodes beads into lists of `capacity` edges, made in front of an evaluation without the
+// host: more edges, an odd number of them or a list cut short leave a graph without edges, which is reported.
+struct SmallGraph {
+    const int64_t *sizes;                  // [B], or NULL: ptr is read
+    int64_t *ptr;
+    double r;
+    int64_t max_nn, capacity;
+    uint2 *masks;                          // [N][(N + 31) / 32]
+    int32_t *deg, *upper;                  // [N]
+    int32_t *row1, *twin, *pair_of, *sel;  // [capacity], sel [capacity / 2]
+    int64_t *offsets, *counts;             // [N + 1]; {edges, pairs}
+    Publish pub;                           // host NULL: reported in the evaluation's status word
+};
+inline size_t small_graph_scratch(int64_t N) { return (size_t)N * ((N + 31) / 32) * 8 + (size_t)N * 8 + 256; }
+inline bool small_graph_ok(int64_t N, int64_t B, const mlcgb_schnet_weights *w) {
+    return N > 0 && B > 0 && N <= kMaskNodes && N <= kSmallNodes && B <= kMaskStructs && w->hidden == 128 && w->filters == 128 && w->conv_out == 128 &&
+           w->num_blocks >= 1 && w->num_blocks <= kMaxBlocks;
+}
+int small_graph_start(const SmallForward &f, const SmallGraph &g, cudaStream_t st);    // graph, distances, embedding, lin1 of the first block
+// interaction.cu: mlcgb_schnet_energy_forces / _eval_counted (grad_sign -1 / 1) behind it
+int schnet_eval_small(const void *pos, const int64_t *types, int64_t N, int64_t B, const SmallGraph &g, const mlcgb_rbf_spec *rbf, int conv_cutoff_kind,
+                      double conv_lower, double conv_upper, const mlcgb_schnet_weights *w, int precision, void *workspace, size_t workspace_bytes,
+                      void *energy, void *grad_pos, float grad_sign, int32_t *status, cudaStream_t st);
 int small_start(const SmallForward &f, cudaStream_t st);    // distances, embedding, lin1 of the first block
 int small_forward(const SmallForward &f, cudaStream_t st);  // the blocks, the output network and, if wanted, the force pass down to s of block 1
 int small_finish(const SmallForward &f, const int32_t *twin, const int64_t *struct_ptr, float *energy, float *grad, float sign, cudaStream_t st);

@@ -485,6 +485,8 @@ class SchNet(torch.nn.Module):
             return None
         n_atoms, ptr = sizes_or_pointer(data)
         N, seen = data.pos.shape[0], self.__dict__.get("_mlcgb_edges_per_bead", 0.0)
+        if not seen and not training and N <= 2048:       # (nothing to go by: every bead sees its whole structure, or forty others)
+            seen = min((N - 1) / (ptr.numel() - 1 if n_atoms is None else max(n_atoms.numel(), 1)), 40.0)
         res = get_backend().schnet_from_positions(data.pos, self._types(data), n_atoms, ptr, float(self.rbf_layer.cutoff.cutoff_upper),
                                                   int(self.max_num_neighbors), *setup, forces, 1.03 * seen * N + 64 if seen else 0, training)
         if res is None:
@@ -559,12 +561,15 @@ class SchNet(torch.nn.Module):
         be = get_backend()
         pos = data.pos.detach().contiguous()
         N, cap = pos.shape[0], int(self.edge_capacity)
+        n_atoms, ptr = sizes_or_pointer(data)
+        upper, most = float(self.rbf_layer.cutoff.cutoff_upper), int(self.max_num_neighbors)
         key = (N, cap, pos.device)
         cached = self.__dict__.get("_mlcgb_rows")
         if cached is None or cached[0] != key:       # stale entries of earlier graphs stay valid point indices for the same N
             cached = self.__dict__["_mlcgb_rows"] = (key, torch.zeros((2, cap), dtype=torch.int32, device=pos.device))
-        n_atoms, ptr = sizes_or_pointer(data)
-        res = be.graph_capacity(_as_3d(pos), ptr, n_atoms, float(self.rbf_layer.cutoff.cutoff_upper), self.max_num_neighbors, cap, cached[1])
+        if pos.shape[1] == 3 and be.schnet_fixed_ok(N, ptr.numel() - 1 if n_atoms is None else n_atoms.numel(), setup[2]):
+            return be.schnet_fixed(pos, self._types(data), n_atoms, ptr, upper, most, *setup, forces, cached[1])
+        res = be.graph_capacity(_as_3d(pos), ptr, n_atoms, upper, most, cap, cached[1])
         plan, ptr = EdgePlan.from_graph(res, N, symmetric=True), res["ptr"]
         spec, conv_cut, weights, precision = setup
         return be.schnet_eval(pos, self._types(data), ptr, plan, spec, conv_cut, weights, precision, want_grad=True, counts=res["counts"],

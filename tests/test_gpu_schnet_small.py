@@ -51,6 +51,51 @@ def test_evaluation_from_positions_keeps_up_with_changing_sizes():
         assert torch.equal(got["energy"], want["energy"]) and torch.equal(got["forces"], want["forces"]), sizes
 
 
+@pytest.mark.parametrize("sizes", [[2], [3, 1], [31, 33], [64] * 8, [1] * 1000 + [20], [1024, 1023], [2047], [2048], [1] * 2000 + [48], [2049], [1, 0, 4]])
+def test_graph_made_inside_the_evaluation(sizes):
+    """Up to 2048 beads the lists are made by the evaluation's first two launches, ahead of the host's look at the edge count or without
+    one: the numbers are those of the evaluation on a given list, bit by bit, for workspaces that are too small, exact and larger;
+    a list cut short leaves the route."""
+    from mlcg_b200.backend import get_backend
+    torch.manual_seed(0)
+    cut = bnn.CosineCutoff(0.0, 6.0)
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, 32, trainable=False), cut, [128], embedding_size=5, num_interactions=2).eval().to(DEV)
+    model, be, n = bnn.GradientsOut(net, "forces").eval(), get_backend(), sum(sizes)
+    gen = torch.Generator().manual_seed(n)
+    pos, types_ = (torch.rand(n, 3, generator=gen) * 2.5 * max(sizes) ** (1 / 3)).to(DEV), torch.randint(0, 5, (n,), generator=gen).to(DEV)
+    batch = torch.repeat_interleave(torch.arange(len(sizes)), torch.tensor(sizes)).to(DEV)
+    make = lambda **kw: mlcg_b200.AtomicData(pos=pos.clone(), atom_types=types_, batch=batch, **kw)  # noqa: E731
+    by_size = dict(n_atoms=torch.tensor(sizes, device=DEV))
+    given = make(**by_size)
+    given.neighbor_list = net.neighbor_list(given, 6.0)
+    E = given.neighbor_list["SchNet"]["index_mapping"].shape[1]
+    want = model(given).out["SchNet"]
+    for guess in (0.0, (E - 2) / n / 1.04, E / n, 3 * E / n):
+        for kw in (by_size, {}):
+            net.__dict__["_mlcgb_edges_per_bead"] = max(guess, 0.0)
+            got = model(make(**kw)).out["SchNet"]
+            assert torch.equal(got["energy"], want["energy"]) and torch.equal(got["forces"], want["forces"]), guess
+    for cap in (E, E + 2, 3 * E):
+        bnn.set_edge_capacity(model, cap)
+        got = model(make(**by_size)).out["SchNet"]
+        be.check_pending()
+        assert torch.equal(got["energy"], want["energy"]) and torch.equal(got["forces"], want["forces"]), cap
+    bnn.set_edge_capacity(model, E - 2)
+    if E > 2:
+        model(make(**by_size))
+        with pytest.raises(RuntimeError, match="capacity"):
+            be.check_pending()
+    bnn.set_edge_capacity(model, None)
+    if max(sizes) > 8:
+        net.max_num_neighbors = 3
+        cut_short = model(make(**by_size)).out["SchNet"]
+        given = make(**by_size)
+        given.neighbor_list = net.neighbor_list(given, 6.0, 3)
+        want = model(given).out["SchNet"]
+        assert torch.equal(cut_short["energy"], want["energy"]) and torch.equal(cut_short["forces"], want["forces"])
+    be.check_pending()
+
+
 @pytest.mark.parametrize("sizes", [[40, 30], [2500]])
 def test_weights_written_by_the_launch_before(sizes):
     """A call whose first kernels read weights sees what the kernel launched just before it wrote to them, and so does one product
