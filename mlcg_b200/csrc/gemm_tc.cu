@@ -954,25 +954,44 @@ int tn_jobs_launch(const TnJobs &jobs, int n, int32_t *status, cudaStream_t st) 
     return check_launch();
 }
 
-// dst[i] = sum over parts of src[part * stride + i], in their order; entry blockIdx.y
-__global__ void partial_sums_kernel(const __grid_constant__ PartialSums sums) {
+// dst[i] = sum over parts of src[part * stride + i]; entry blockIdx.y.  A block takes 32 elements, a warp an eighth of the parts, and the
+// eighths are added in their order: bound by the latency of a thread's chain of loads, which is 592 parts long for the embedding table
+// (one thread per element: 49 us for the sums of a 256 x 73 step).
+constexpr int kSumWarps = 8;
+__global__ void __launch_bounds__(kSumWarps * 32) partial_sums_kernel(const __grid_constant__ PartialSums sums) {
+    __shared__ float s_part[kSumWarps][32];
     const PartialSum &s = sums.sum[blockIdx.y];
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < s.n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, z0 = s.parts * warp / kSumWarps, z1 = s.parts * (warp + 1) / kSumWarps;
+    for (int64_t i0 = (int64_t)blockIdx.x * 32; i0 < s.n; i0 += (int64_t)gridDim.x * 32) {
+        const int64_t i = i0 + lane;
         float v = 0.f;
-        int z = 0;
-        for (; z + 8 <= s.parts; z += 8) {
+        if (i < s.n) {
+            int z = z0;
+            for (; z + 8 <= z1; z += 8) {
+                float x[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) x[u] = __ldg(s.src + (z + u) * s.stride + i);
+#pragma unroll
+                for (int u = 0; u < 8; u++) v += x[u];
+            }
             float x[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) x[u] = __ldg(s.src + (z + u) * s.stride + i);
+            for (int u = 0; u < 8; u++) x[u] = z + u < z1 ? __ldg(s.src + (z + u) * s.stride + i) : 0.f;
 #pragma unroll
             for (int u = 0; u < 8; u++) v += x[u];
         }
-        for (; z < s.parts; z++) v += __ldg(s.src + z * s.stride + i);
-        s.dst[i] = v;
+        s_part[warp][lane] = v;
+        __syncthreads();
+        if (warp == 0 && i < s.n) {
+#pragma unroll
+            for (int w = 1; w < kSumWarps; w++) v += s_part[w][lane];
+            s.dst[i] = v;
+        }
+        __syncthreads();
     }
 }
 int partial_sums_launch(const PartialSums &sums, int n, cudaStream_t st) {
-    partial_sums_kernel<<<dim3(64, n), 256, 0, st>>>(sums);
+    partial_sums_kernel<<<dim3(128, n), kSumWarps * 32, 0, st>>>(sums);
     return check_launch();
 }
 
