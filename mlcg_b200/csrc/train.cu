@@ -101,7 +101,7 @@ struct TrainBackward {
 static TrainForward train_forward_layout(int64_t N, int64_t E, int64_t P, int64_t Wh, int64_t L) {
     TrainForward o;
     int64_t at = 0;
-    auto take = [&](int64_t n) { const int64_t r = at; at += (n + 3) & ~(int64_t)3; return r; };
+    auto take = [&](int64_t n) { const int64_t r = at; at += (n + 63) & ~(int64_t)63; return r; };      // (arrays on 256-byte boundaries)
     const int64_t hidden = (int64_t)(mlcgb_filter_hidden_bytes(P) / sizeof(float));
     o.pos = take(3 * N);
     o.d = take(E); o.gd = take(E); o.en = take(N); o.ah = take(N * Wh); o.zmax = take(L);
@@ -118,7 +118,7 @@ static TrainForward train_forward_layout(int64_t N, int64_t E, int64_t P, int64_
 static TrainBackward train_backward_layout(int64_t N, int64_t E, int64_t P, int64_t R, int64_t Wh, int64_t L, int64_t T) {
     TrainBackward o;
     int64_t at = 0;
-    auto take = [&](int64_t n) { const int64_t r = at; at += (n + 3) & ~(int64_t)3; return r; };
+    auto take = [&](int64_t n) { const int64_t r = at; at += (n + 63) & ~(int64_t)63; return r; };      // (arrays on 256-byte boundaries)
     const int64_t jobs = 3 * L + 2;
     const int64_t tiles = 2 * ((N + 127) / 128);
     o.node_parts = (int)(kNumSM / jobs < 1 ? 1 : kNumSM / jobs);
