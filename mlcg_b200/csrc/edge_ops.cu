@@ -312,11 +312,11 @@ edge_distance_bwd_kernel(const T *__restrict__ pos, const T *__restrict__ g, con
     }
 }
 
-// Forces of a symmetric centre-sorted list (the in-edges of a node are the reverses of its out-edges) and the per-structure sums of
-// the node energies in one launch: a warp per node, then a warp per structure
+// Forces of a symmetric centre-sorted list (the in-edges of a node are the reverses of its out-edges) from the derivative of every pair,
+// and the per-structure sums of the node energies in one launch: a warp per node, then a warp per structure
 __global__ void __launch_bounds__(256)
-finish_kernel(const float *__restrict__ pos, const float *__restrict__ g, const float *__restrict__ d, const int32_t *__restrict__ row1,
-              const int64_t *__restrict__ ptr, const int32_t *__restrict__ twin, int64_t N, float *__restrict__ gpos, float sign, const float *__restrict__ en,
+finish_kernel(const float *__restrict__ pos, const float *__restrict__ pair_g, const float *__restrict__ d, const int32_t *__restrict__ row1,
+              const int64_t *__restrict__ ptr, const int32_t *__restrict__ pair_of, int64_t N, float *__restrict__ gpos, float sign, const float *__restrict__ en,
               const int64_t *__restrict__ struct_ptr, int64_t B, float *__restrict__ energy) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -333,7 +333,7 @@ finish_kernel(const float *__restrict__ pos, const float *__restrict__ g, const 
         const float x = pos[n * 3], y = pos[n * 3 + 1], z = pos[n * 3 + 2];
         for (int64_t k = ptr[n] + lane; k < ptr[n + 1]; k += 32) {
             const int64_t j = row1[k];
-            const float dk = d[k], w = dk > 0.f ? sign * (g[k] + g[twin[k]]) / dk : 0.f;     // (coinciding beads: the norm's subgradient 0)
+            const float dk = d[k], w = dk > 0.f ? sign * pair_g[pair_of[k]] / dk : 0.f;     // (coinciding beads: the norm's subgradient 0)
             s0 = fmaf(w, x - pos[j * 3], s0);
             s1 = fmaf(w, y - pos[j * 3 + 1], s1);
             s2 = fmaf(w, z - pos[j * 3 + 2], s2);
@@ -343,10 +343,10 @@ finish_kernel(const float *__restrict__ pos, const float *__restrict__ g, const 
     }
 }
 
-int finish_launch(const float *pos, const float *g, const float *d, const int32_t *row1, const int64_t *ptr, const int32_t *twin, int64_t N, float *gpos,
+int finish_launch(const float *pos, const float *pair_g, const float *d, const int32_t *row1, const int64_t *ptr, const int32_t *pair_of, int64_t N, float *gpos,
                   float sign, const float *en, const int64_t *struct_ptr, int64_t B, float *energy, cudaStream_t st) {
     TimelineScope timeline_scope("finish", st);
-    launch_pdl(finish_kernel, dim3(grid_for((N + B) * 32, 256)), dim3(256), 0, st, pos, g, d, row1, ptr, twin, N, gpos, sign, en, struct_ptr, B, energy);
+    launch_pdl(finish_kernel, dim3(grid_for((N + B) * 32, 256)), dim3(256), 0, st, pos, pair_g, d, row1, ptr, pair_of, N, gpos, sign, en, struct_ptr, B, energy);
     return check_launch();
 }
 

@@ -10,7 +10,7 @@
 // `force` is the step of the force pass that used to be an aggregation and a backward pass of the filter network: gd of a pair is
 // s[(i,j)] + s[(j,i)], with x = lin1 features and a = gradient of the aggregate.  Bound by the L2: per edge 1.5 KB (force) or
 // 2 KB (tangent) of rows, of which W and W' come from HBM once.
-#include "common.cuh"
+#include "schnet_internal.cuh"
 
 namespace mlcgb {
 
@@ -141,6 +141,75 @@ seg_vd_kernel(const float *__restrict__ a, const float *__restrict__ x, const fl
         if (MODE != kSegDot)
             reinterpret_cast<float4 *>(out)[n * 32 + lane] = make_float4(acc0.x + acc1.x, acc0.y + acc1.y, acc0.z + acc1.z, acc0.w + acc1.w);
     }
+}
+
+// One dot product per pair (seg_pair_dot): a warp takes the upper edges of its node, whose pairs and rows of W' are consecutive, four
+// at a time in registers.  Per pair one row of W' and two node rows cross the first-level pipe where the two directed edges of the
+// kernel above took four, and the sums of the other blocks are added here, once per pair, instead of per edge with the forces.  Dot
+// products of 545 k pairs inside an evaluation 114 us by edges, 94 like this; 128 k pairs 39 and 29; 94 k pairs 39 and 27.
+constexpr int kPairWarps = 4;
+__global__ void __launch_bounds__(kPairWarps * 32, 6)
+seg_pair_dot_kernel(const float *__restrict__ a, const float *__restrict__ x, const float *__restrict__ Wd, const int64_t *__restrict__ ptr,
+                    const int32_t *__restrict__ nbr, const int32_t *__restrict__ pair_of, const int32_t *__restrict__ twin, const float *__restrict__ s,
+                    int64_t N, float *__restrict__ sp) {
+    const int lane = threadIdx.x & 31;
+    const char *a_lane = reinterpret_cast<const char *>(a) + lane * 16, *x_lane = reinterpret_cast<const char *>(x) + lane * 16,
+               *w_lane = reinterpret_cast<const char *>(Wd) + lane * 16;
+    auto row = [](const char *base, int64_t r) { return __ldg(reinterpret_cast<const float4 *>(base + r * 512)); };
+    const int64_t n = (int64_t)blockIdx.x * kPairWarps + (threadIdx.x >> 5);
+    if (n >= N) return;
+    const int64_t k0 = ptr[n], k1 = ptr[n + 1];
+    if (k0 == k1) return;
+    const float4 xi = row(x_lane, n), ai = row(a_lane, n);
+    for (int64_t c0 = k0; c0 < k1; c0 += 32) {
+        const bool in = c0 + lane < k1;
+        const int32_t my_j = in ? nbr[c0 + lane] : 0;
+        const unsigned upper = __ballot_sync(0xffffffffu, in && my_j > n);
+        if (!upper) continue;
+        const int first = __ffs(upper) - 1, len = first + __popc(upper);       // (neighbours ascend)
+        const bool mine = lane >= first && lane < len;
+        int32_t my_p = 0;
+        float my_s = 0.f;
+        if (mine) {
+            my_p = pair_of[c0 + lane];
+            if (s) my_s = s[c0 + lane] + s[twin[c0 + lane]];
+        }
+        for (int g = first; g < len; g += 4) {
+            float4 w[4], aj[4], xj[4];
+            float dot[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int t = g + u < len ? g + u : len - 1;
+                const int64_t j = __shfl_sync(0xffffffffu, my_j, t);
+                w[u] = row(w_lane, __shfl_sync(0xffffffffu, my_p, t));
+                aj[u] = row(a_lane, j);
+                xj[u] = row(x_lane, j);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                dot[u] = fmaf(fmaf(xi.x, aj[u].x, xj[u].x * ai.x), w[u].x, fmaf(fmaf(xi.y, aj[u].y, xj[u].y * ai.y), w[u].y,
+                         fmaf(fmaf(xi.z, aj[u].z, xj[u].z * ai.z), w[u].z, fmaf(xi.w, aj[u].w, xj[u].w * ai.w) * w[u].w)));
+            // (the four sums as in the kernel above: sum u is left in lanes 8 u .. 8 u + 7)
+            const bool up = lane & 16, up2 = lane & 8;
+            const float d0 = (up ? dot[2] : dot[0]) + __shfl_xor_sync(0xffffffffu, up ? dot[0] : dot[2], 16);
+            const float d1 = (up ? dot[3] : dot[1]) + __shfl_xor_sync(0xffffffffu, up ? dot[1] : dot[3], 16);
+            float d = (up2 ? d1 : d0) + __shfl_xor_sync(0xffffffffu, up2 ? d0 : d1, 8);
+            d += __shfl_xor_sync(0xffffffffu, d, 4);
+            d += __shfl_xor_sync(0xffffffffu, d, 2);
+            d += __shfl_xor_sync(0xffffffffu, d, 1);
+            const float got = __shfl_sync(0xffffffffu, d, ((lane - g) & 3) * 8);
+            if (lane >= g && lane < g + 4) my_s += got;
+        }
+        if (mine) sp[my_p] = my_s;
+    }
+}
+
+int seg_pair_dot(const float *a, const float *x, const float *Wd, const int64_t *ptr, const int32_t *nbr, const int32_t *pair_of, const int32_t *twin,
+                 const float *s, int64_t N, float *sp, cudaStream_t st) {
+    TimelineScope timeline_scope("seg_pair_dot", st);
+    if (int rc = prefer_l1<seg_pair_dot_kernel>()) return rc;
+    seg_pair_dot_kernel<<<(unsigned)((N + kPairWarps - 1) / kPairWarps), kPairWarps * 32, 0, st>>>(a, x, Wd, ptr, nbr, pair_of, twin, s, N, sp);
+    return check_launch();
 }
 
 // dd[e] = d(distance of e)/dt when the positions move along sign v: (pos[j] - pos[i]) . (v[j] - v[i]) / d, zero where the beads coincide

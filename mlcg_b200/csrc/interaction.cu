@@ -169,7 +169,7 @@ static int node_layers_backward(const float *g, const mlcgb_schnet_block &w, con
 static inline int64_t up64(int64_t n) { return (n + 63) & ~(int64_t)63; }
 
 struct SchnetLayout {                                                        // offsets in floats
-    int64_t d, x[2], g[2], agg, gy, gxl, ah, en, gd, W, Wd, wstride, block0, block_stride, xl_off, a_off, total;
+    int64_t d, x[2], g[2], agg, gy, gxl, ah, en, gd, gp, W, Wd, wstride, block0, block_stride, xl_off, a_off, total;
 };
 static SchnetLayout schnet_layout(int64_t N, int64_t E, int64_t P, int64_t H, int64_t F, int64_t H2, int64_t Wh, int64_t L) {
     SchnetLayout o;
@@ -180,7 +180,7 @@ static SchnetLayout schnet_layout(int64_t N, int64_t E, int64_t P, int64_t H, in
     o.g[0] = take(N * H); o.g[1] = take(N * H);
     o.agg = take(N * F); o.gy = take(N * H2); o.gxl = take(N * F);
     o.ah = take(N * Wh); o.en = take(N);
-    o.gd = take(E);
+    o.gd = take(E); o.gp = take(P);
     o.wstride = padded_rows(P) * F;
     o.W = take(L * o.wstride); o.Wd = take(L * o.wstride);                   // filter rows of all blocks, and their distance derivatives
     o.xl_off = 0; o.a_off = up64(N * F);
@@ -304,15 +304,17 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
         rc = node_layers_backward(g, bw, blk + lay.a_off, N, H, F, H2, ws + lay.gy, gagg, status, stream);
         if (rc) return rc;
         // s[e] of every block adds up in one array: the last block sets it, the others add
-        rc = mlcgb_seg_force(gagg, blk + lay.xl_off, ws + lay.W + l * lay.wstride, ws + lay.Wd + l * lay.wstride, offsets, row1, pair_of, N, F,
-                             l > 0 ? gxl : nullptr, ws + lay.gd,
+        if (l == 0) {
+            if ((rc = seg_pair_dot(gagg, blk + lay.xl_off, ws + lay.Wd, offsets, row1, pair_of, twin, L > 1 ? ws + lay.gd : nullptr, N, ws + lay.gp, st))) return rc;
+            break;
+        }
+        rc = mlcgb_seg_force(gagg, blk + lay.xl_off, ws + lay.W + l * lay.wstride, ws + lay.Wd + l * lay.wstride, offsets, row1, pair_of, N, F, gxl, ws + lay.gd,
                              l != L - 1, stream);
         if (rc) return rc;
-        if (l > 0) rc = mlcgb_gemm_tc_fused(1, gxl, bw.lin1_w, nullptr, g, 2, N, H, F, gnext, status, stream);
-        if (rc) return rc;
+        if ((rc = mlcgb_gemm_tc_fused(1, gxl, bw.lin1_w, nullptr, g, 2, N, H, F, gnext, status, stream))) return rc;
         gcur ^= 1;
     }
-    return finish_launch((const float *)pos, ws + lay.gd, d, row1, offsets, twin, N, (float *)grad_pos, grad_sign, ws + lay.en, struct_ptr, B, (float *)energy, st);
+    return finish_launch((const float *)pos, ws + lay.gp, d, row1, offsets, pair_of, N, (float *)grad_pos, grad_sign, ws + lay.en, struct_ptr, B, (float *)energy, st);
 }
 
 }  // extern "C"

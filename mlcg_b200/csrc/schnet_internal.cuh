@@ -84,9 +84,13 @@ struct SmallBackward {
 };
 int small_backward(const SmallForward &f, const SmallBackward &b, cudaStream_t st);
 
-// edge_ops.cu: position gradients (times sign: -1 gives forces) from per-edge derivatives of the energy (g[e] + g[reverse] belongs to a
-// pair) and energies, in one launch
-int finish_launch(const float *pos, const float *g, const float *d, const int32_t *row1, const int64_t *ptr, const int32_t *twin, int64_t N, float *gpos,
+// edge_vd.cu: the last dot products of a force pass, one per pair: sp[p] = sum_f (x[i] a[j] + x[j] a[i]) W'[p] + s[(i,j)] + s[(j,i)], the
+// sums of the blocks before (NULL: none)
+int seg_pair_dot(const float *a, const float *x, const float *Wd, const int64_t *ptr, const int32_t *nbr, const int32_t *pair_of, const int32_t *twin,
+                 const float *s, int64_t N, float *sp, cudaStream_t st);
+// edge_ops.cu: position gradients (times sign: -1 gives forces) from the energy's derivative with respect to each pair's distance, and
+// energies, in one launch
+int finish_launch(const float *pos, const float *pair_g, const float *d, const int32_t *row1, const int64_t *ptr, const int32_t *pair_of, int64_t N, float *gpos,
                   float sign, const float *en, const int64_t *struct_ptr, int64_t B, float *energy, cudaStream_t st);
 
 }  // namespace mlcgb

@@ -88,7 +88,7 @@ train_begin_kernel(const float *__restrict__ pos, int64_t n, float *__restrict__
 constexpr int64_t kH = 128;
 
 struct TrainForward {                                 // offsets in floats
-    int64_t pos, d, gd, en, ah, zmax, W, Wd, Hs, Zs, wstride, hstride, block0, stride, total;      // W .. Zs: of all blocks
+    int64_t pos, d, gd, gp, en, ah, zmax, W, Wd, Hs, Zs, wstride, hstride, block0, stride, total;      // W .. Zs: of all blocks
     int64_t x, xl, agg, a, gu, gagg, gxl, g;          // of a block; g: the gradient of the block's output
 };
 struct TrainBackward {
@@ -104,7 +104,7 @@ static TrainForward train_forward_layout(int64_t N, int64_t E, int64_t P, int64_
     auto take = [&](int64_t n) { const int64_t r = at; at += (n + 63) & ~(int64_t)63; return r; };      // (arrays on 256-byte boundaries)
     const int64_t hidden = (int64_t)(mlcgb_filter_hidden_bytes(P) / sizeof(float));
     o.pos = take(3 * N);
-    o.d = take(E); o.gd = take(E); o.en = take(N); o.ah = take(N * Wh); o.zmax = take(L);
+    o.d = take(E); o.gd = take(E); o.gp = take(P); o.en = take(N); o.ah = take(N * Wh); o.zmax = take(L);
     o.wstride = padded_rows(P) * kH;
     o.hstride = hidden;
     o.W = take(L * o.wstride); o.Wd = take(L * o.wstride); o.Hs = take(L * hidden); o.Zs = take(L * hidden);
@@ -232,12 +232,16 @@ int mlcgb_schnet_train_forward(const void *pos, const int64_t *types, const int6
         const mlcgb_schnet_block &bw = w->blocks[l];
         float *b = blk(l);
         if ((rc = mlcgb_gemm_tc_chain2(1, b + o.g, bw.lin_w, nullptr, bw.lin2_w, nullptr, b + o.a, N, b + o.gu, b + o.gagg, status, stream))) return rc;
-        if ((rc = mlcgb_seg_force(b + o.gagg, b + o.xl, ws + o.W + l * o.wstride, ws + o.Wd + l * o.wstride, offsets, row1, pair_of, N, kH, l > 0 ? b + o.gxl : nullptr, ws + o.gd, l != L - 1,
+        if (l == 0) {
+            if ((rc = seg_pair_dot(b + o.gagg, b + o.xl, ws + o.Wd, offsets, row1, pair_of, twin, L > 1 ? ws + o.gd : nullptr, N, ws + o.gp, st))) return rc;
+            break;
+        }
+        if ((rc = mlcgb_seg_force(b + o.gagg, b + o.xl, ws + o.W + l * o.wstride, ws + o.Wd + l * o.wstride, offsets, row1, pair_of, N, kH, b + o.gxl, ws + o.gd, l != L - 1,
                                   stream)))
             return rc;
-        if (l > 0 && (rc = mlcgb_gemm_tc_fused(1, b + o.gxl, bw.lin1_w, nullptr, b + o.g, 2, N, kH, kH, blk(l - 1) + o.g, status, stream))) return rc;
+        if ((rc = mlcgb_gemm_tc_fused(1, b + o.gxl, bw.lin1_w, nullptr, b + o.g, 2, N, kH, kH, blk(l - 1) + o.g, status, stream))) return rc;
     }
-    return finish_launch((const float *)pos, ws + o.gd, d, row1, offsets, twin, N, (float *)grad_pos, negate ? -1.f : 1.f, ws + o.en, struct_ptr, B, (float *)energy, st);
+    return finish_launch((const float *)pos, ws + o.gp, d, row1, offsets, pair_of, N, (float *)grad_pos, negate ? -1.f : 1.f, ws + o.en, struct_ptr, B, (float *)energy, st);
 }
 
 int mlcgb_schnet_train_backward(const int64_t *types, const int64_t *struct_ptr, int64_t N, int64_t B, const int32_t *row0,

@@ -163,3 +163,28 @@ def test_recordings_of_one_model_stand_by_themselves():
             assert torch.equal(got[0], e) and torch.equal(got[1], g)
     fields[0].check()
     assert all(bool((j == 7).all()) for j in junk)
+
+
+@pytest.mark.parametrize("blocks", [1, 2])
+def test_large_batches_with_nodes_of_every_degree(blocks):
+    """Above the small batches' limit the last dot products are taken per pair: beads without neighbours, with one, and with several
+    chunks of 32, the first upper neighbour anywhere in a chunk."""
+    gen = torch.Generator().manual_seed(blocks)
+    torch.manual_seed(2)
+    upper, sizes = 6.0, [2200, 1, 2, 110, 150]
+    cut = bnn.CosineCutoff(0.0, upper)
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, 32, trainable=False), cut, [128], hidden_channels=128, embedding_size=6, num_filters=128,
+                             num_interactions=blocks)
+    parts = [torch.rand(n, 3, generator=gen) * side for n, side in zip(sizes, (60.0, 1.0, 100.0, 9.0, 12.0))]
+    parts[2] = torch.tensor([[0.0, 0.0, 0.0], [3.0, 0.0, 0.0]])
+    pos = torch.cat(parts)
+    types_, batch = torch.randint(0, 6, (sum(sizes),), generator=gen), torch.arange(len(sizes)).repeat_interleave(torch.tensor(sizes))
+    e_x, f_x, _ = _oracle(net, "expnormal", upper, blocks, pos, types_, batch, len(sizes), torch.float64)
+    net = net.to(DEV).eval()
+    data = mlcg_b200.AtomicData(pos=pos.to(DEV), atom_types=types_.to(DEV), batch=batch.to(DEV), n_atoms=torch.tensor(sizes).to(DEV))
+    degrees = net.neighbor_list(data, upper)["SchNet"]["index_mapping"][0].bincount(minlength=sum(sizes))
+    assert int(degrees.min()) == 0 and int((degrees == 1).sum()) > 0 and int(degrees.max()) > 64
+    out = bnn.GradientsOut(net, "forces").eval()(data).out["SchNet"]
+    assert torch.allclose(out["energy"].cpu().double(), e_x, rtol=E_RTOL, atol=E_RTOL * float(e_x.abs().max()))
+    # (dense clusters: forces of hundreds, to the same number of digits as elsewhere)
+    assert float((out["forces"].cpu().double() - f_x).abs().max()) < F_ATOL * max(1.0, float(f_x.abs().max()) / 10)
