@@ -275,8 +275,8 @@ __global__ void edge_distance_kernel(const T *__restrict__ pos, const int32_t *_
             d[e] = T(0);
             continue;
         }
-        const T dx = pos[b * 3] - pos[a * 3], dy = pos[b * 3 + 1] - pos[a * 3 + 1], dz = pos[b * 3 + 2] - pos[a * 3 + 2];
-        d[e] = sqrt(dx * dx + dy * dy + dz * dz);
+        // (rounded as the graph kernels round it, which write the distances of their own lists)
+        d[e] = sqrt(dist2_rn(pos[a * 3], pos[a * 3 + 1], pos[a * 3 + 2], pos[b * 3], pos[b * 3 + 1], pos[b * 3 + 2]));
     }
 }
 

@@ -131,18 +131,19 @@ int mlcgb_schnet_evaluate(const void *pos, const int64_t *types, const int64_t *
     auto *row0 = (int32_t *)at, *row1 = (int32_t *)(at + row), *twin = (int32_t *)(at + 2 * row), *pair_of = (int32_t *)(at + 3 * row),
          *sel = (int32_t *)(at + 4 * row);
     const size_t lists = list_bytes(E);
-    int rc = mlcgb_graph_finish(pos, MLCGB_F32, ptr, N, B, r, 0, nullptr, nullptr, g, G.graph, offsets, E, nullptr, nullptr, nullptr, row0, row1, twin, sel,
+    // (the distances go straight to where the evaluation wants them)
+    char *distances = at + lists + (training ? train_distances_at(N, E, w->head_width, w->num_blocks) : 0);
+    int rc = mlcgb_graph_finish(pos, MLCGB_F32, ptr, N, B, r, 0, nullptr, nullptr, g, G.graph, offsets, E, nullptr, distances, nullptr, row0, row1, twin, sel,
                                 pair_of, host[3] != 0, status, stream);
     if (rc) return rc;
     ChainScope chain;
     if (training)
         rc = precision ? MLCGB_E_ARG
-                       : mlcgb_schnet_train_forward(pos, types, ptr, N, B, row0, row1, offsets, sel, pair_of, twin, E, E / 2, rbf, conv_cutoff_kind,
-                                                    conv_lower, conv_upper, w, negate, at + lists, workspace_bytes - lists, energy, grad_pos, status, stream);
+                       : schnet_train_forward(pos, types, ptr, N, B, row0, row1, offsets, sel, pair_of, twin, E, E / 2, rbf, conv_cutoff_kind, conv_lower, conv_upper,
+                                              w, negate, true, at + lists, workspace_bytes - lists, energy, grad_pos, status, stream);
     else
-        rc = (negate ? mlcgb_schnet_energy_forces : mlcgb_schnet_eval_counted)(pos, types, ptr, N, B, row0, row1, offsets, sel, pair_of, twin, E, E / 2,
-                                                                               nullptr, rbf, conv_cutoff_kind, conv_lower, conv_upper, w, precision, at + lists,
-                                                                               workspace_bytes - lists, energy, grad_pos, status, stream);
+        rc = schnet_eval_distances(pos, types, ptr, N, B, row0, row1, offsets, sel, pair_of, twin, E, rbf, conv_cutoff_kind, conv_lower, conv_upper, w, precision,
+                                   at + lists, workspace_bytes - lists, energy, grad_pos, negate ? -1.f : 1.f, status, stream);
     if (rc == MLCGB_OK) host[4] = MLCGB_EVALUATE_DONE;
     return rc;
 }

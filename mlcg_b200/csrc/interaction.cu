@@ -175,7 +175,7 @@ static SchnetLayout schnet_layout(int64_t N, int64_t E, int64_t P, int64_t H, in
     SchnetLayout o;
     int64_t at = 0;
     auto take = [&](int64_t n) { const int64_t r = at; at += up64(n); return r; };
-    o.d = take(E);
+    o.d = take(E);                                                           // (first: schnet_eval_distances)
     o.x[0] = take(N * H); o.x[1] = take(N * H);
     o.g[0] = take(N * H); o.g[1] = take(N * H);
     o.agg = take(N * F); o.gy = take(N * H2); o.gxl = take(N * F);
@@ -219,7 +219,7 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
                               const int32_t *pair_of, const int32_t *twin, int64_t E, int64_t P, const int64_t *counts,
                               const mlcgb_rbf_spec *rbf, int conv_cutoff_kind, double conv_lower, double conv_upper,
                               const mlcgb_schnet_weights *w, int precision, void *workspace, size_t workspace_bytes, void *energy,
-                              void *grad_pos, float grad_sign, int32_t *status, void *stream, const SmallGraph *graph = nullptr) {
+                              void *grad_pos, float grad_sign, int32_t *status, void *stream, const SmallGraph *graph = nullptr, bool have_distances = false) {
     const int64_t *pairs_dev = counts ? counts + 1 : nullptr;
     if (N < 0 || B < 0 || E < 0 || P < 0 || !w || !status || !energy || !struct_ptr) return MLCGB_E_ARG;
     if (B == 0) return MLCGB_OK;
@@ -263,7 +263,7 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
         if ((rc = small_forward(f, st))) return rc;
         return small_finish(f, twin, struct_ptr, (float *)energy, (float *)grad_pos, grad_sign, st);
     }
-    if ((rc = mlcgb_edge_distance(pos, MLCGB_F32, row0, row1, E, N, d, status, stream))) return rc;
+    if (!have_distances && (rc = mlcgb_edge_distance(pos, MLCGB_F32, row0, row1, E, N, d, status, stream))) return rc;
     {
         TimelineScope timeline_scope("embedding", stream);
         launch_pdl(embedding_rows_kernel, dim3(grid_for(N * (H >> 2), 256)), dim3(256), 0, st, (const float *)w->embedding, types, N, H, w->num_types, ws + lay.x[0], status);
@@ -318,6 +318,14 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
 }
 
 }  // extern "C"
+
+int mlcgb::schnet_eval_distances(const void *pos, const int64_t *types, const int64_t *struct_ptr, int64_t N, int64_t B, const int32_t *row0, const int32_t *row1,
+                                 const int64_t *offsets, const int32_t *sel, const int32_t *pair_of, const int32_t *twin, int64_t E, const mlcgb_rbf_spec *rbf,
+                                 int conv_cutoff_kind, double conv_lower, double conv_upper, const mlcgb_schnet_weights *w, int precision, void *workspace,
+                                 size_t workspace_bytes, void *energy, void *grad_pos, float grad_sign, int32_t *status, void *stream) {
+    return schnet_eval_impl(pos, types, struct_ptr, N, B, row0, row1, offsets, sel, pair_of, twin, E, E / 2, nullptr, rbf, conv_cutoff_kind, conv_lower,
+                            conv_upper, w, precision, workspace, workspace_bytes, energy, grad_pos, grad_sign, status, stream, nullptr, true);
+}
 
 int mlcgb::schnet_eval_small(const void *pos, const int64_t *types, int64_t N, int64_t B, const SmallGraph &g, const mlcgb_rbf_spec *rbf, int conv_cutoff_kind,
                              double conv_lower, double conv_upper, const mlcgb_schnet_weights *w, int precision, void *workspace, size_t workspace_bytes,

@@ -84,6 +84,18 @@ struct SmallBackward {
 };
 int small_backward(const SmallForward &f, const SmallBackward &b, cudaStream_t st);
 
+// The whole-model sequences on lists whose distances already lie in the workspace, at its start / at train_distances_at() bytes of it
+// (mlcgb_schnet_energy_forces / _eval_counted with grad_sign -1 / 1, mlcgb_schnet_train_forward)
+int schnet_eval_distances(const void *pos, const int64_t *types, const int64_t *struct_ptr, int64_t N, int64_t B, const int32_t *row0, const int32_t *row1,
+                          const int64_t *offsets, const int32_t *sel, const int32_t *pair_of, const int32_t *twin, int64_t E, const mlcgb_rbf_spec *rbf,
+                          int conv_cutoff_kind, double conv_lower, double conv_upper, const mlcgb_schnet_weights *w, int precision, void *workspace,
+                          size_t workspace_bytes, void *energy, void *grad_pos, float grad_sign, int32_t *status, void *stream);
+size_t train_distances_at(int64_t N, int64_t E, int64_t head_width, int64_t num_blocks);
+int schnet_train_forward(const void *pos, const int64_t *types, const int64_t *struct_ptr, int64_t N, int64_t B, const int32_t *row0, const int32_t *row1,
+                         const int64_t *offsets, const int32_t *sel, const int32_t *pair_of, const int32_t *twin, int64_t E, int64_t P, const mlcgb_rbf_spec *rbf,
+                         int conv_cutoff_kind, double conv_lower, double conv_upper, const mlcgb_schnet_weights *w, int negate, bool have_distances,
+                         void *workspace, size_t workspace_bytes, void *energy, void *grad_pos, int32_t *status, void *stream);
+
 // edge_vd.cu: the last dot products of a force pass, one per pair: sp[p] = sum_f (x[i] a[j] + x[j] a[i]) W'[p] + s[(i,j)] + s[(j,i)], the
 // sums of the blocks before (NULL: none)
 int seg_pair_dot(const float *a, const float *x, const float *Wd, const int64_t *ptr, const int32_t *nbr, const int32_t *pair_of, const int32_t *twin,

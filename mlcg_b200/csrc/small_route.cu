@@ -440,8 +440,7 @@ small_start_kernel(const float *__restrict__ pos, const int64_t *__restrict__ ty
         if (i < 0 || i >= N || j < 0 || j >= N) {
             atomicOr(status, (int)kBadIndex);
         } else {
-            const float dx = pos[3 * j] - pos[3 * i], dy = pos[3 * j + 1] - pos[3 * i + 1], dz = pos[3 * j + 2] - pos[3 * i + 2];
-            v = sqrtf(dx * dx + dy * dy + dz * dz);
+            v = sqrtf(dist2_rn(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], pos[3 * j], pos[3 * j + 1], pos[3 * j + 2]));
         }
         d[e] = v;
     }
@@ -616,7 +615,7 @@ small_graph_fill_kernel(const float *__restrict__ pos, const SmallGraph g, int64
                 if (!(bits >> lane & 1u) || rank >= kept) continue;
                 const int slot = off + rank, j = lo + (w0 + w) * 32 + lane;
                 const uint2 rev = g.masks[(int64_t)j * words + (il >> 5)];
-                const float dx = pos[3 * j] - xi, dy = pos[3 * j + 1] - yi, dz = pos[3 * j + 2] - zi;
+                const float d2 = dist2_rn(xi, yi, zi, pos[3 * j], pos[3 * j + 1], pos[3 * j + 2]);
                 const int rank_j = (int)rev.x + __popc(rev.y & ((1u << (il & 31)) - 1u));
                 const int off_j = s_off[j], kept_j = s_off[j + 1] - off_j, up_j = s_uoff[j + 1] - s_uoff[j];
                 const int p = j > i ? uo + (rank - nlower) : s_uoff[j] + (rank_j - (kept_j - up_j));
@@ -626,7 +625,7 @@ small_graph_fill_kernel(const float *__restrict__ pos, const SmallGraph g, int64
                 g.row1[slot] = j;
                 g.twin[slot] = ok ? off_j + rank_j : slot;
                 g.pair_of[slot] = ok ? p : 0;
-                d[slot] = sqrtf(dx * dx + dy * dy + dz * dz);
+                d[slot] = sqrtf(d2);
                 if (ok && j > i) g.sel[p] = slot;
             }
         }

@@ -163,6 +163,10 @@ static SmallForward small_view(const TrainForward &o, float *ws, const void *pos
     return f;
 }
 
+size_t train_distances_at(int64_t N, int64_t E, int64_t head_width, int64_t num_blocks) {
+    return sizeof(float) * (size_t)train_forward_layout(N, E, E / 2, head_width, num_blocks).d;
+}
+
 }  // namespace mlcgb
 
 using namespace mlcgb;
@@ -176,11 +180,13 @@ size_t mlcgb_schnet_train_workspace_bytes(int backward, int64_t N, int64_t E, in
                                              : train_forward_layout(N, E, P, head_width, num_blocks).total);
 }
 
-int mlcgb_schnet_train_forward(const void *pos, const int64_t *types, const int64_t *struct_ptr, int64_t N, int64_t B, const int32_t *row0,
+}  // extern "C"
+
+int mlcgb::schnet_train_forward(const void *pos, const int64_t *types, const int64_t *struct_ptr, int64_t N, int64_t B, const int32_t *row0,
                                const int32_t *row1, const int64_t *offsets, const int32_t *sel, const int32_t *pair_of, const int32_t *twin,
                                int64_t E, int64_t P, const mlcgb_rbf_spec *rbf, int conv_cutoff_kind, double conv_lower, double conv_upper,
-                               const mlcgb_schnet_weights *w, int negate, void *workspace, size_t workspace_bytes, void *energy, void *grad_pos,
-                               int32_t *status, void *stream) {
+                               const mlcgb_schnet_weights *w, int negate, bool have_distances, void *workspace, size_t workspace_bytes, void *energy,
+                               void *grad_pos, int32_t *status, void *stream) {
     if (!rbf || !w || N <= 0 || B <= 0 || E <= 0 || 2 * P != E) return MLCGB_E_ARG;
     if (!pos || !types || !struct_ptr || !row0 || !row1 || !offsets || !sel || !pair_of || !twin || !workspace || !energy || !grad_pos || !status)
         return MLCGB_E_ARG;
@@ -204,7 +210,7 @@ int mlcgb_schnet_train_forward(const void *pos, const int64_t *types, const int6
         if (!rs) rs = small_forward(f, st);
         return rs ? rs : small_finish(f, twin, struct_ptr, (float *)energy, (float *)grad_pos, negate ? -1.f : 1.f, st);
     }
-    int rc = mlcgb_edge_distance(pos, MLCGB_F32, row0, row1, E, N, d, status, stream);
+    int rc = have_distances ? MLCGB_OK : mlcgb_edge_distance(pos, MLCGB_F32, row0, row1, E, N, d, status, stream);
     if (rc) return rc;
     {
         TimelineScope timeline_scope("embedding", stream);
@@ -242,6 +248,17 @@ int mlcgb_schnet_train_forward(const void *pos, const int64_t *types, const int6
         if ((rc = mlcgb_gemm_tc_fused(1, b + o.gxl, bw.lin1_w, nullptr, b + o.g, 2, N, kH, kH, blk(l - 1) + o.g, status, stream))) return rc;
     }
     return finish_launch((const float *)pos, ws + o.gp, d, row1, offsets, pair_of, N, (float *)grad_pos, negate ? -1.f : 1.f, ws + o.en, struct_ptr, B, (float *)energy, st);
+}
+
+extern "C" {
+
+int mlcgb_schnet_train_forward(const void *pos, const int64_t *types, const int64_t *struct_ptr, int64_t N, int64_t B, const int32_t *row0,
+                               const int32_t *row1, const int64_t *offsets, const int32_t *sel, const int32_t *pair_of, const int32_t *twin,
+                               int64_t E, int64_t P, const mlcgb_rbf_spec *rbf, int conv_cutoff_kind, double conv_lower, double conv_upper,
+                               const mlcgb_schnet_weights *w, int negate, void *workspace, size_t workspace_bytes, void *energy, void *grad_pos,
+                               int32_t *status, void *stream) {
+    return schnet_train_forward(pos, types, struct_ptr, N, B, row0, row1, offsets, sel, pair_of, twin, E, P, rbf, conv_cutoff_kind, conv_lower, conv_upper, w,
+                                negate, false, workspace, workspace_bytes, energy, grad_pos, status, stream);
 }
 
 int mlcgb_schnet_train_backward(const int64_t *types, const int64_t *struct_ptr, int64_t N, int64_t B, const int32_t *row0,

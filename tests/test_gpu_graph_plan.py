@@ -97,3 +97,31 @@ def test_counts_read_by_several_threads():
 
     with ThreadPoolExecutor(4) as pool:
         assert all(pool.map(run, range(4)))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("sizes", [[3, 0, 5] * 400, [0] * 40 + [768] * 3 + [0] * 3, [1] * 2100, [2] * 1025, [767, 768, 768], [64, 31, 33] * 1100, [700] * 3 + [769], [1000, 600, 500, 1] ])
+def test_bit_rows_of_whole_batches(sizes, dtype):
+    """Batches of structures that all fit a bit row are counted and scanned in three launches (structures found by a warp among 1, 32, 33 and
+    more boundaries, parts of 32 points, blocks of 1024); one larger structure sends the batch the other way."""
+    rng = np.random.default_rng(len(sizes) + sizes[0])
+    ptr = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    assert 2048 < ptr[-1] <= 768 * len(sizes)
+    pos = (rng.random((int(ptr[-1]), 3)) * max(sizes) ** (1 / 3) * 2.0).astype(dtype)
+    be, t = get_backend(), torch.as_tensor(pos, device=DEV)
+    want = radius_ref.radius_graph_c(pos, ptr, 4.0, 1000, False, "cluster")
+    for given in (dict(ptr=torch.as_tensor(ptr, device=DEV)), dict(ptr=None, n_atoms=torch.as_tensor(sizes, dtype=torch.int64, device=DEV))):
+        res = be.radius_graph(t, given.pop("ptr"), 4.0, 1000, False, 1, want_distance=True, want_plan=True, **given)
+        assert torch.equal(res["ptr"].cpu(), torch.as_tensor(ptr)) and res["status"] == 0
+        assert torch.equal(res["edge_index"].cpu(), torch.from_numpy(want))
+        if want.shape[1]:
+            twin, sel, pair_of, status = be.pair_plan(res["row0"], res["row1"], res["offsets"], len(pos), fresh_status=True)
+            assert int(status[0]) == 0
+            assert torch.equal(res["twin"], twin) and torch.equal(res["sel"], sel) and torch.equal(res["pair_of"], pair_of)
+    for loop, rule, cap in ((True, 1, 1000), (False, 1, 3), (False, 0, 3)):
+        res = be.radius_graph(t, torch.as_tensor(ptr, device=DEV), 4.0, cap, loop, rule)
+        cut = radius_ref.radius_graph_c(pos, ptr, 4.0, cap, loop, "cluster" if rule else "native")
+        assert torch.equal(res["edge_index"].cpu(), torch.from_numpy(cut))
+        # (the cluster rule counts the point itself among its cap + 1: a list is cut short where it lost somebody)
+        assert bool(res["status"] & 1) == (cut.shape[1] < want.shape[1] + (len(pos) if loop else 0))
+    be.check_pending()
