@@ -592,12 +592,27 @@ typedef struct {
     const uint16_t *offsets;
     const void *slice_params;
 } mlcgb_prior_list;
+/* What an mlcgb_prior_list is made of, from the list as the neighbour-list dictionary holds it: idx [order,M] = mapping (an index outside
+ * [0,N) becomes -1 and sets status bit 1), params [n_params,M] = tables[q] ([num_types]^order, contiguous) at the types [N] of the
+ * term's beads (tables NULL: not written; `given` [n_params,M] are the parameters).  host_out (order 2 only, NULL: not wanted; the call then
+ * waits for the result and must not be captured): [0] = runs of equal first bead, [1] = 1 where the list holds (j, i) with the same
+ * parameters for every (i, j) (compared by the sum of 64-bit hashes).  starts [runs]: first term of each run, from the workspace that
+ * the call before left. */
+#define MLCGB_MAX_PRIOR_TABLES 32
+size_t mlcgb_prior_list_workspace_bytes(int64_t M);
+int mlcgb_prior_list_make(const int64_t *mapping, int order, int64_t M, const int64_t *types, int64_t N, int64_t num_types, int n_params,
+                          const void *const *tables /* host */, int dtype, const void *given, int32_t *idx, void *params, void *workspace,
+                          size_t workspace_bytes, int64_t *host_out /* [2] */, int32_t *status, void *stream);
+int mlcgb_prior_list_starts(const int32_t *first /* idx */, int64_t M, const void *workspace, size_t workspace_bytes, int64_t *starts, void *stream);
 /* The slices of a pair list idx [2,M] whose runs of equal first bead begin at starts [n_runs].  With slice_params NULL: slices =
  * {longest run, -, least, largest second bead} of each; then, with step0 = exclusive sums of (longest + 3) / 4 and steps their total,
  * the four arrays of mlcgb_prior_list (largest - least < 65536 in every slice). */
 int mlcgb_pair_slices(const int32_t *idx, const void *params, int dtype, int n_params, int64_t M, const int64_t *starts, int64_t n_runs,
                       int64_t steps, const int64_t *step0, int32_t *slices, int32_t *beads, uint16_t *offsets, void *slice_params,
                       void *stream);
+/* step0 [n_slices] of what the first of its two calls left in slices; host_out: all steps, slots of lanes without a run / 4, least second
+ * bead, largest span.  Waits for the result. */
+int mlcgb_pair_slices_plan(const int32_t *slices, int64_t n_slices, int64_t n_runs, int64_t *step0, int64_t *host_out /* [4] */, void *stream);
 size_t mlcgb_prior_eval_workspace_bytes(int n_lists, int64_t N, int64_t B, int dtype);
 int mlcgb_prior_eval(int n_lists, const mlcgb_prior_list *lists /* host */, const void *pos /* [N,3] */, int dtype,
                      const int64_t *batch /* [N] or NULL */, int64_t N, int64_t B, void *energy /* [n_lists,B] */,

@@ -43,6 +43,7 @@ class PriorListStruct(ctypes.Structure):
                 ("steps", c_i64), ("slices", c_vp), ("slice_beads", c_vp), ("offsets", c_vp), ("slice_params", c_vp)]
 
 
+MAX_PRIOR_TABLES = 32           # MLCGB_MAX_PRIOR_TABLES
 MAX_PRIOR_SEGMENTS = 8
 VERSION = 201                  # MLCGB_VERSION of the header that the tables below follow
 EVALUATE_DONE, EVALUATE_MORE = 1, 2
@@ -141,6 +142,10 @@ SIGNATURES = {
     "mlcgb_langevin_first_half": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_int, c_i64, c_dbl, c_dbl, c_dbl, c_vp]),
     "mlcgb_langevin_second_half": (c_int, [c_vp, c_vp, c_vp, c_int, c_i64, c_dbl, c_vp]),
     "mlcgb_prior_terms": (c_int, [c_int, c_vp, c_int, c_vp, c_vp, c_vp, c_int, c_i64, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp]),
+    "mlcgb_prior_list_workspace_bytes": (c_sz, [c_i64]),
+    "mlcgb_prior_list_make": (c_int, [c_vp, c_int, c_i64, c_vp, c_i64, c_i64, c_int, c_vp, c_int, c_vp, c_vp, c_vp, c_vp, c_sz, c_vp, c_vp, c_vp]),
+    "mlcgb_prior_list_starts": (c_int, [c_vp, c_i64, c_vp, c_sz, c_vp, c_vp]),
+    "mlcgb_pair_slices_plan": (c_int, [c_vp, c_i64, c_i64, c_vp, c_vp, c_vp]),
     "mlcgb_pair_slices": (c_int, [c_vp, c_vp, c_int, c_int, c_i64, c_vp, c_i64, c_i64] + [c_vp] * 6),
     "mlcgb_prior_eval_workspace_bytes": (c_sz, [c_int, c_i64, c_i64, c_int]),
     "mlcgb_prior_eval": (c_int, [c_int, ctypes.POINTER(PriorListStruct), c_vp, c_int, c_vp, c_i64, c_i64, c_vp, c_vp, c_int, c_vp, c_vp, c_int, c_vp, c_sz, c_vp,

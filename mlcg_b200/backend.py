@@ -1086,6 +1086,36 @@ class CudaBackend:
         return energy, grad
 
 
+    def prior_list(self, mapping, types, tables, params, n_beads, pairs):
+        """``(idx int32 [order, M], params [P, M], symmetric, starts)`` of an index list as the neighbour-list dictionary holds it (int64
+        [order, M]).  ``tables``: the parameters by the types of a term's beads, each [types] * order of one float dtype, or None where
+        ``params`` are given.  ``pairs`` (order 2): whether the list holds every term's reverse with the same parameters, and then the
+        first terms of its runs of equal first bead, where these are at least eight terms long on average (else None)."""
+        _need_cuda(mapping, types, params, *(tables or ()))
+        mapping, types = mapping.contiguous(), types.contiguous()
+        order, M = mapping.shape
+        dev, like = mapping.device, params if tables is None else tables[0]
+        if tables is None:
+            params, P, kinds = params.contiguous(), params.shape[0], 1
+        else:
+            P, kinds = len(tables), like.shape[0]
+        with _on(dev):
+            idx = torch.empty((order, M), dtype=torch.int32, device=dev)
+            out = params if tables is None else torch.empty((P, M), dtype=like.dtype, device=dev)
+            pairs = bool(pairs) and M > 0 and M % 2 == 0
+            wsb = self.lib.mlcgb_prior_list_workspace_bytes(M) if pairs else 0
+            ws = torch.empty(wsb, dtype=torch.uint8, device=dev) if pairs else None
+            host = (ctypes.c_int64 * 2)()
+            self._run("prior_list", self.lib.mlcgb_prior_list_make, (
+                _ptr(mapping), order, M, _ptr(types), n_beads, kinds, P, None if tables is None else (ctypes.c_void_p * P)(*(t.data_ptr() for t in tables)),
+                _dt(like), _ptr(params), _ptr(idx), None if tables is None else _ptr(out), _ptr(ws), wsb, host if pairs else None,
+                _ptr(self._sticky_status(dev)), _stream()), nbytes=M * (12 * order + P * like.element_size()))
+            starts = None
+            if host[1] and M >= 8 * host[0] and M < 2 ** 31:
+                starts = torch.empty(host[0], dtype=torch.int64, device=dev)
+                self._run("prior_list_starts", self.lib.mlcgb_prior_list_starts, (_ptr(idx), M, _ptr(ws), wsb, _ptr(starts), _stream()))
+        return idx, out, bool(host[1]), starts
+
     def pair_slices(self, idx, params, starts, worth):
         """The slices of a pair list (int32 [2, M], runs of equal first bead from ``starts`` on) as ``mlcgb_prior_list`` takes them:
         ``(slices, beads, offsets, params)``; None where the second beads of a slice lie too far apart or ``worth(slots)`` says that
@@ -1094,22 +1124,21 @@ class CudaBackend:
         idx, params, starts = idx.contiguous(), params.contiguous(), starts.contiguous()
         M, R, dev = idx.shape[1], starts.numel(), idx.device
         n = (R + 31) // 32
-        slices = torch.empty((n, 4), dtype=torch.int32, device=dev)
         with _on(dev):
+            slices = torch.empty((n, 4), dtype=torch.int32, device=dev)
+            step0 = torch.empty(n, dtype=torch.int64, device=dev)
             common = (_ptr(idx), _ptr(params), _dt(params), params.shape[0], M, _ptr(starts), R)
+            host = (ctypes.c_int64 * 4)()
             self._run("pair_slices", self.lib.mlcgb_pair_slices, common + (0, None, _ptr(slices), None, None, None, _stream()))
-            steps = (slices[:, 0].to(torch.int64) + 3) // 4
-            ends = torch.cumsum(steps, 0)
-            last = R - 32 * (n - 1)                    # runs of the last slice
-            total, unused, low, span = torch.stack([ends[-1], steps[-1] * (32 - last), slices[:, 2].min().to(torch.int64),
-                                                    (slices[:, 3] - slices[:, 2]).max().to(torch.int64)]).tolist()
+            self._run("pair_slices_plan", self.lib.mlcgb_pair_slices_plan, (_ptr(slices), n, R, _ptr(step0), host, _stream()))
+            total, unused, low, span = host
             if low < 0 or span >= 2 ** 16 or total >= 2 ** 31 or not worth(4 * (32 * total - unused)):
                 return None
             beads = torch.empty((n, 32), dtype=torch.int32, device=dev)
             offsets = torch.empty((total, 32, 4), dtype=torch.uint16, device=dev)
             packed = torch.empty((params.shape[0], total, 32, 4), dtype=params.dtype, device=dev)
             self._run("pair_slices", self.lib.mlcgb_pair_slices, common + (
-                total, _ptr(ends - steps), _ptr(slices), _ptr(beads), _ptr(offsets), _ptr(packed), _stream()))
+                total, _ptr(step0), _ptr(slices), _ptr(beads), _ptr(offsets), _ptr(packed), _stream()))
         return slices, beads, offsets, packed
 
     def prior_eval(self, lists, pos, batch, B, deterministic=True, forces=False, totals=False):

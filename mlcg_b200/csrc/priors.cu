@@ -3,6 +3,7 @@
 // the warp when all 32 terms belong to the same structure (the common case, lists are ordered by
 // structure), gradients go out as floating-point atomics.
 #include "common.cuh"
+#include "small_graph.cuh"
 
 #include <type_traits>
 
@@ -387,55 +388,251 @@ prior_slices_kernel(const __grid_constant__ PriorSegments seg, int parts, const 
     if (beside_terms) pdl_wait();
 }
 
-// The slices of a list (mlcgb_pair_slices): a warp per slice, a lane per run.  `out` NULL: {longest run, -, least, largest second
-// bead} of every slice; else the slice's steps are written out.
-template <typename T>
+// ---- what is made of a list on its first evaluation: 32-bit indices, the parameters of its terms from the tables of bead types, whether
+//      a pair list holds the reverse of every term, where its runs of equal first bead begin, and its slices.  A pass over the list
+//      for each of gather, starts and slices (two): bound by the memory it streams.  Gathered and sorted by library calls (two sorts
+//      of all keys for the reverses) the lists of 1024 chains of 268 beads, 73 M terms, took 17 ms, like this 1.8 with the evaluation.
+constexpr int kGatherThreads = 256, kGatherTerms = 8, kChunk = kGatherThreads * kGatherTerms;
+struct PriorTables { const void *p[MLCGB_MAX_PRIOR_TABLES]; };
+
+// finaliser of MurmurHash3 (Austin Appleby, public domain): every bit of the input moves every bit of the output
+__device__ __forceinline__ uint64_t mix64(uint64_t k) {
+    k ^= k >> 33; k *= 0xff51afd7ed558ccdull;
+    k ^= k >> 33; k *= 0xc4ceb9fe1a85ec53ull;
+    return k ^ k >> 33;
+}
+__device__ __forceinline__ uint64_t value_bits(float v) { return __float_as_uint(v + 0.f); }           // (-0 and 0 are the same parameter)
+__device__ __forceinline__ uint64_t value_bits(double v) { return (uint64_t)__double_as_longlong(v + 0.0); }
+
+// PAIR: `difference` gains the sum over the terms of hash(i, j, parameters) - hash(j, i, parameters), modulo 2^64: zero where the list is
+// the same set of terms reversed, and not zero otherwise but for one chance in 2^64; counts[chunk] = runs that begin in it
+template <typename T, int ORDER, bool PAIR>
+__global__ void __launch_bounds__(kGatherThreads)
+prior_gather_kernel(const int64_t *__restrict__ mapping, int64_t M, const int64_t *__restrict__ types, int64_t N, int64_t num_types, int n_params,
+                    const __grid_constant__ PriorTables tables, const T *__restrict__ given, int32_t *__restrict__ idx, T *__restrict__ params,
+                    unsigned long long *__restrict__ difference, int32_t *__restrict__ counts, int32_t *__restrict__ status) {
+    int runs = 0;
+    uint64_t diff = 0;
+    const int64_t t0 = (int64_t)blockIdx.x * kChunk + threadIdx.x;
+#pragma unroll 4
+    for (int u = 0; u < kGatherTerms; u++) {
+        const int64_t t = t0 + u * kGatherThreads;
+        if (t >= M) break;
+        int64_t at[ORDER], entry = 0;
+#pragma unroll
+        for (int o = 0; o < ORDER; o++) at[o] = mapping[(int64_t)o * M + t];
+        if (PAIR) runs += t == 0 || mapping[t - 1] != at[0];
+#pragma unroll
+        for (int o = 0; o < ORDER; o++) {
+            if (at[o] < 0 || at[o] >= N) {                   // (reported, and again by the evaluation, which leaves the term out)
+                atomicOr(status, (int)kBadIndex);
+                at[o] = -1;
+            }
+            idx[(int64_t)o * M + t] = (int32_t)at[o];
+        }
+        if (!given) {
+#pragma unroll
+            for (int o = 0; o < ORDER; o++) {
+                int64_t ty = at[o] < 0 ? 0 : __ldg(types + at[o]);
+                if (ty < 0) ty += num_types;                 // (as indexing a table does)
+                if (ty < 0 || ty >= num_types) {
+                    atomicOr(status, (int)kBadIndex);
+                    ty = 0;
+                }
+                entry = entry * num_types + ty;
+            }
+        }
+        uint64_t h = 0;
+        for (int q = 0; q < n_params; q++) {
+            const T v = given ? given[(int64_t)q * M + t] : __ldg((const T *)tables.p[q] + entry);
+            if (!given) params[(int64_t)q * M + t] = v;
+            if (PAIR) h = mix64(h + value_bits(v) + 1);
+        }
+        if (PAIR) {
+            const uint64_t i = (uint32_t)at[0], j = (uint32_t)at[1];
+            diff += mix64(h ^ (i << 32 | j)) - mix64(h ^ (j << 32 | i));
+        }
+    }
+    if constexpr (PAIR) {
+        __shared__ int s_runs[kGatherThreads / 32];
+        __shared__ uint64_t s_diff[kGatherThreads / 32];
+        runs = warp_sum(runs);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) diff += __shfl_xor_sync(0xffffffffu, diff, o);
+        if ((threadIdx.x & 31) == 0) { s_runs[threadIdx.x >> 5] = runs; s_diff[threadIdx.x >> 5] = diff; }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < kGatherThreads / 32; w++) { runs += s_runs[w]; diff += s_diff[w]; }
+            counts[blockIdx.x] = runs;
+            if (diff) atomicAdd(difference, (unsigned long long)diff);
+        }
+    }
+}
+
+// exclusive sums of n values by one block of 1024 threads, thread t holding `per` consecutive ones of each round: f(k) the value, g(k, sum before)
+template <typename F, typename G>
+__device__ __forceinline__ int64_t block_sums_before(int64_t n, F &&f, G &&g) {
+    __shared__ int64_t s_warp[32], s_total;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t carry = 0;
+    for (int64_t k0 = 0; k0 < n; k0 += 1024) {
+        const int64_t k = k0 + threadIdx.x;
+        const int64_t v = k < n ? f(k) : 0;
+        int64_t inc = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        if (lane == 31) s_warp[warp] = inc;
+        __syncthreads();
+        if (warp == 0) {
+            const int64_t w = s_warp[lane];
+            int64_t wi = w;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int64_t t = __shfl_up_sync(0xffffffffu, wi, o);
+                if (lane >= o) wi += t;
+            }
+            s_warp[lane] = wi - w;
+            if (lane == 31) s_total = wi;
+        }
+        __syncthreads();
+        if (k < n) g(k, carry + s_warp[warp] + inc - v);
+        carry += s_total;
+        __syncthreads();
+    }
+    return carry;
+}
+
+__global__ void __launch_bounds__(1024) run_offsets_kernel(const int32_t *__restrict__ counts, int64_t n, const unsigned long long *__restrict__ difference,
+                                                           int64_t *__restrict__ before, Publish pub) {
+    const int64_t runs = block_sums_before(n, [&](int64_t k) { return (int64_t)counts[k]; }, [&](int64_t k, int64_t v) { before[k] = v; });
+    if (threadIdx.x == 0) publish(pub, runs, *difference != 0);
+}
+
+// starts[r] = first term of run r (chunks and counts as above)
+__global__ void __launch_bounds__(kGatherThreads)
+run_starts_kernel(const int32_t *__restrict__ first, int64_t M, const int64_t *__restrict__ before, int64_t *__restrict__ starts) {
+    __shared__ int s_warp[kGatherThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t at = before[blockIdx.x];
+    for (int u = 0; u < kGatherTerms; u++) {
+        const int64_t t = (int64_t)blockIdx.x * kChunk + u * kGatherThreads + threadIdx.x;
+        const bool head = t < M && (t == 0 || first[t - 1] != first[t]);
+        const unsigned heads = __ballot_sync(0xffffffffu, head);
+        if (lane == 0) s_warp[warp] = __popc(heads);
+        __syncthreads();
+        int mine = __popc(heads & lanemask_lt()), all = 0;
+        for (int w = 0; w < kGatherThreads / 32; w++) {
+            mine += w < warp ? s_warp[w] : 0;
+            all += s_warp[w];
+        }
+        if (head) starts[at + mine] = t;
+        at += all;
+        __syncthreads();
+    }
+}
+
+// The slices of a list (mlcgb_pair_slices), a warp each.  First {longest run, -, least, largest second bead} of every slice: its terms are
+// consecutive, whatever their runs.
 __global__ void __launch_bounds__(256)
-pair_slices_kernel(const int32_t *__restrict__ idx, const T *__restrict__ params, int n_params, int64_t M, const int64_t *__restrict__ starts, int64_t n_runs,
-                   int64_t n_slices, int64_t steps, const int64_t *__restrict__ step0, int4 *__restrict__ slices, int32_t *__restrict__ beads,
-                   uint2 *__restrict__ offsets, typename Vec4<T>::type *__restrict__ out) {
-    using V = typename Vec4<T>::type;
+pair_slices_kernel(const int32_t *__restrict__ idx, int64_t M, const int64_t *__restrict__ starts, int64_t n_runs, int64_t n_slices, int4 *__restrict__ slices) {
     const int lane = threadIdx.x & 31;
     for (int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < n_slices; w += (int64_t)gridDim.x * (blockDim.x >> 5)) {
-        const int64_t run = w * 32 + lane;
+        const int64_t run = w * 32 + lane, end = (w + 1) * 32 < n_runs ? starts[(w + 1) * 32] : M;
+        const int64_t k0 = run < n_runs ? starts[run] : end, k1 = __shfl_down_sync(0xffffffffu, k0, 1);
+        int longest = (int)((lane == 31 ? end : k1) - k0), lo = 0x7fffffff, hi = -0x7fffffff - 1;
+        for (int64_t k = __shfl_sync(0xffffffffu, k0, 0) + lane; k < end; k += 32) {
+            const int j = idx[M + k];
+            lo = min(lo, j);
+            hi = max(hi, j);
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+            longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+        }
+        if (lane == 0) slices[w] = make_int4(longest, 0, lo, hi);
+    }
+}
+
+// first step of every slice; to the host: all steps, lanes without a run times the last slice's steps, least second bead, largest span
+__global__ void __launch_bounds__(1024) slices_plan_kernel(const int4 *__restrict__ slices, int64_t n_slices, int64_t n_runs, int64_t *__restrict__ step0, Publish pub) {
+    __shared__ int s_low, s_span;
+    if (threadIdx.x == 0) { s_low = 0x7fffffff; s_span = 0; }
+    int low = 0x7fffffff;
+    unsigned span = 0;
+    const int64_t total = block_sums_before(
+        n_slices,
+        [&](int64_t k) {
+            const int4 h = slices[k];
+            low = min(low, h.z);
+            span = max(span, (unsigned)min((int64_t)h.w - h.z, (int64_t)0x7fffffff));
+            return (int64_t)((h.x + 3) / 4);
+        },
+        [&](int64_t k, int64_t v) { step0[k] = v; });
+    atomicMin(&s_low, low);
+    atomicMax(&s_span, (int)span);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        volatile int64_t *h = pub.host;
+        h[1] = total;
+        h[2] = (slices[n_slices - 1].x + 3) / 4 * (32 * n_slices - n_runs);
+        h[3] = s_low;
+        h[4] = s_span;
+        __threadfence_system();
+        h[0] = pub.seq;
+    }
+}
+
+// The steps of a slice: the terms of 32 runs, read run by run in rows of 32 and turned over in shared memory.
+template <typename T> constexpr int kPackWarps = sizeof(T) == 4 ? 8 : 4;
+template <typename T> constexpr int kPackPitch = sizeof(T) == 4 ? 36 : 34;      // (128-bit reads along a row by eight lanes meet no bank twice)
+template <typename T>
+__global__ void __launch_bounds__(kPackWarps<T> * 32)
+pair_slices_pack_kernel(const int32_t *__restrict__ idx, const T *__restrict__ params, int n_params, int64_t M, const int64_t *__restrict__ starts,
+                        int64_t n_runs, int64_t n_slices, int64_t steps, const int64_t *__restrict__ step0, int4 *__restrict__ slices,
+                        int32_t *__restrict__ beads, uint2 *__restrict__ offsets, typename Vec4<T>::type *__restrict__ out) {
+    using V = typename Vec4<T>::type;
+    __shared__ __align__(32) T s_tile[kPackWarps<T>][32][kPackPitch<T>];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto tile = s_tile[warp];
+    for (int64_t w = (int64_t)blockIdx.x * kPackWarps<T> + warp; w < n_slices; w += (int64_t)gridDim.x * kPackWarps<T>) {
+        const int64_t run = w * 32 + lane, end = (w + 1) * 32 < n_runs ? starts[(w + 1) * 32] : M;
         const bool mine = run < n_runs;
-        const int64_t k0 = starts[mine ? run : w * 32], k1 = mine ? (run + 1 < n_runs ? starts[run + 1] : M) : k0;   // (no run: the slice's first bead, no terms)
-        const int len = (int)(k1 - k0);
-        if (!out) {
-            int lo = idx[M + k0], hi = lo, longest = len;
-            for (int64_t k = k0; k < k1; k++) {
-                const int j = idx[M + k];
-                lo = min(lo, j);
-                hi = max(hi, j);
-            }
-#pragma unroll
-            for (int o = 16; o; o >>= 1) {
-                lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-                hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-                longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
-            }
-            if (lane == 0) slices[w] = make_int4(longest, 0, lo, hi);
-            continue;
-        }
+        const int64_t begin = starts[w * 32];
+        const int at = (int)((mine ? starts[run] : end) - begin);                  // of this lane's run, from the slice's first term
+        const int next = __shfl_down_sync(0xffffffffu, at, 1), len = (lane == 31 ? (int)(end - begin) : next) - at;
         const int4 h = slices[w];
-        const int n = (h.x + 3) >> 2, base = h.z, filler = idx[M + k0] - base;
+        const int n = (h.x + 3) >> 2, base = h.z;
+        const int filler = (mine ? idx[M + begin + at] : idx[M + begin]) - base;     // (no run: the slice's first second bead)
         const int64_t first = step0[w];
-        for (int g = 0; g < n; g++) {
-            int j[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) j[u] = 4 * g + u < len ? idx[M + k0 + 4 * g + u] - base : filler;
-            const int64_t at = (first + g) * 32 + lane;
-            offsets[at] = make_uint2((uint32_t)j[0] | (uint32_t)j[1] << 16, (uint32_t)j[2] | (uint32_t)j[3] << 16);
-            for (int q = 0; q < n_params; q++) {
-                T v[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) v[u] = 4 * g + u < len ? params[(int64_t)q * M + k0 + 4 * g + u] : T(0);
-                V x;
-                x.x = v[0]; x.y = v[1]; x.z = v[2]; x.w = v[3];
-                out[(int64_t)q * steps * 32 + at] = x;
+        for (int q = -1; q < n_params; q++) {                                    // the second beads, then the parameters
+            for (int g0 = 0; g0 < n; g0 += 8) {
+                __syncwarp();
+#pragma unroll 8
+                for (int r = 0; r < 32; r++) {
+                    const int a = __shfl_sync(0xffffffffu, at, r), l = __shfl_sync(0xffffffffu, len, r), c = 4 * g0 + lane;
+                    const int fill = __shfl_sync(0xffffffffu, filler, r);
+                    const int64_t k = begin + a + c;
+                    if (q < 0) reinterpret_cast<int *>(&tile[r][0])[lane] = c < l ? idx[M + k] - base : fill;
+                    else tile[r][lane] = c < l ? params[(int64_t)q * M + k] : T(0);
+                }
+                __syncwarp();
+                for (int g = g0; g < n && g < g0 + 8; g++) {
+                    const int64_t to = (first + g) * 32 + lane;
+                    if (q < 0) {
+                        const int4 j = reinterpret_cast<const int4 *>(&tile[lane][0])[g - g0];
+                        offsets[to] = make_uint2((uint32_t)j.x | (uint32_t)j.y << 16, (uint32_t)j.z | (uint32_t)j.w << 16);
+                    } else {
+                        out[(int64_t)q * steps * 32 + to] = reinterpret_cast<const V *>(&tile[lane][0])[g - g0];
+                    }
+                }
             }
         }
-        beads[run] = mine ? idx[k0] : ~idx[k0];
+        beads[run] = mine ? idx[begin + at] : ~idx[begin];
         __syncwarp();
         if (lane == 0) slices[w] = make_int4((int)first, n, base, h.w - base);
     }
@@ -614,18 +811,92 @@ extern "C" int mlcgb_prior_terms(int kind, const void *pos, int dtype, const int
 
 static inline size_t prior_bead_bytes(int64_t N, int dtype) { return ((size_t)N * (dtype == MLCGB_F32 ? 16 : 32) + 255) / 256 * 256; }
 
+extern "C" size_t mlcgb_prior_list_workspace_bytes(int64_t M) {
+    if (M < 0) return 0;
+    return 256 + (size_t)((M + kChunk - 1) / kChunk) * 16;
+}
+
+extern "C" int mlcgb_prior_list_make(const int64_t *mapping, int order, int64_t M, const int64_t *types, int64_t N, int64_t num_types, int n_params,
+                                     const void *const *tables, int dtype, const void *given, int32_t *idx, void *params, void *workspace,
+                                     size_t workspace_bytes, int64_t *host_out, int32_t *status, void *stream) {
+    TimelineScope timeline_scope("prior_list", stream);
+    if (order < 2 || order > 4 || M < 0 || N < 0 || n_params < 0 || !status || (host_out && order != 2)) return MLCGB_E_ARG;
+    if (n_params > MLCGB_MAX_PRIOR_TABLES && tables) return MLCGB_E_LIMIT;
+    if (host_out) host_out[0] = host_out[1] = 0;
+    if (M == 0) return MLCGB_OK;
+    if (!mapping || !idx || (!tables && n_params && !given) || (tables && (!types || !params || num_types < 1))) return MLCGB_E_ARG;
+    if (host_out && (!workspace || workspace_bytes < mlcgb_prior_list_workspace_bytes(M) || ((uintptr_t)workspace & 7))) return MLCGB_E_WORKSPACE;
+    PriorTables t = {};
+    for (int q = 0; tables && q < n_params; q++)
+        if (!(t.p[q] = tables[q])) return MLCGB_E_ARG;
+    auto st = (cudaStream_t)stream;
+    const int64_t chunks = (M + kChunk - 1) / kChunk;
+    if (chunks >= (int64_t)1 << 31) return MLCGB_E_LIMIT;
+    auto *difference = (unsigned long long *)workspace;
+    auto *before = (int64_t *)((char *)workspace + 256);
+    auto *counts = (int32_t *)(before + chunks);
+    Publish pub;
+    if (host_out) {
+        if (int rc = publish_begin(&pub)) return rc;
+        cudaMemsetAsync(difference, 0, 8, st);
+    }
+    int rc = MLCGB_DISPATCH_DTYPE(dtype, [&] {
+        const auto *in = tables ? nullptr : (const scalar_t *)given;
+        const bool rows = tables || given;
+        auto go = [&](auto kern) {
+            kern<<<(unsigned)chunks, kGatherThreads, 0, st>>>(mapping, M, types, N, num_types, rows ? n_params : 0, t, in, idx, (scalar_t *)params, difference, counts, status);
+        };
+        if (order == 2 && host_out) go(prior_gather_kernel<scalar_t, 2, true>);
+        else if (order == 2) go(prior_gather_kernel<scalar_t, 2, false>);
+        else if (order == 3) go(prior_gather_kernel<scalar_t, 3, false>);
+        else go(prior_gather_kernel<scalar_t, 4, false>);
+        return check_launch();
+    });
+    if (rc || !host_out) return rc;
+    run_offsets_kernel<<<1, 1024, 0, st>>>(counts, chunks, difference, before, pub);
+    if ((rc = check_launch()) || (rc = publish_wait(pub, st))) return rc;
+    host_out[0] = pub.host[1];
+    host_out[1] = pub.host[2] == 0;
+    return MLCGB_OK;
+}
+
+extern "C" int mlcgb_prior_list_starts(const int32_t *first, int64_t M, const void *workspace, size_t workspace_bytes, int64_t *starts, void *stream) {
+    if (M < 0) return MLCGB_E_ARG;
+    if (M == 0) return MLCGB_OK;
+    if (!first || !workspace || !starts) return MLCGB_E_ARG;
+    if (workspace_bytes < mlcgb_prior_list_workspace_bytes(M)) return MLCGB_E_WORKSPACE;
+    run_starts_kernel<<<(unsigned)((M + kChunk - 1) / kChunk), kGatherThreads, 0, (cudaStream_t)stream>>>(first, M, (const int64_t *)((const char *)workspace + 256), starts);
+    return check_launch();
+}
+
 extern "C" int mlcgb_pair_slices(const int32_t *idx, const void *params, int dtype, int n_params, int64_t M, const int64_t *starts, int64_t n_runs,
                                  int64_t steps, const int64_t *step0, int32_t *slices, int32_t *beads, uint16_t *offsets, void *slice_params,
                                  void *stream) {
     if (!idx || !starts || !slices || M <= 0 || n_runs <= 0 || M >= (int64_t)1 << 31) return MLCGB_E_ARG;
     if (slice_params && (!params || n_params < 1 || !step0 || !beads || !offsets || steps <= 0)) return MLCGB_E_ARG;
     const int64_t n = (n_runs + 31) / 32;
+    auto st = (cudaStream_t)stream;
+    if (!slice_params) {
+        pair_slices_kernel<<<grid_for(n, 8, 16), 256, 0, st>>>(idx, M, starts, n_runs, n, (int4 *)slices);
+        return check_launch();
+    }
     return MLCGB_DISPATCH_DTYPE(dtype, [&] {
-        pair_slices_kernel<scalar_t><<<grid_for(n, 8, 16), 256, 0, (cudaStream_t)stream>>>(idx, (const scalar_t *)params, n_params, M, starts, n_runs, n, steps, step0,
-                                                                                         (int4 *)slices, beads, (uint2 *)offsets,
-                                                                                         (typename Vec4<scalar_t>::type *)slice_params);
+        pair_slices_pack_kernel<scalar_t><<<grid_for(n, kPackWarps<scalar_t>, 16), kPackWarps<scalar_t> * 32, 0, st>>>(
+            idx, (const scalar_t *)params, n_params, M, starts, n_runs, n, steps, step0, (int4 *)slices, beads, (uint2 *)offsets,
+            (typename Vec4<scalar_t>::type *)slice_params);
         return check_launch();
     });
+}
+
+extern "C" int mlcgb_pair_slices_plan(const int32_t *slices, int64_t n_slices, int64_t n_runs, int64_t *step0, int64_t *host_out, void *stream) {
+    if (!slices || !step0 || !host_out || n_slices <= 0 || n_runs <= 32 * (n_slices - 1) || n_runs > 32 * n_slices) return MLCGB_E_ARG;
+    Publish pub;
+    if (int rc = publish_begin(&pub)) return rc;
+    slices_plan_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>((const int4 *)slices, n_slices, n_runs, step0, pub);
+    if (int rc = check_launch()) return rc;
+    if (int rc = publish_wait(pub, (cudaStream_t)stream)) return rc;
+    for (int i = 0; i < 4; i++) host_out[i] = pub.host[1 + i];
+    return MLCGB_OK;
 }
 
 extern "C" size_t mlcgb_prior_eval_workspace_bytes(int n_lists, int64_t N, int64_t B, int dtype) {

@@ -90,3 +90,63 @@ def test_pair_slices_of_beads_that_lie_far_apart():
     assert _pair_slices(pairs, params) is not None
     pairs[1, 0] = 65528 + 65536
     assert _pair_slices(pairs, params) is None
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("beads,B", [(2, 1), (9, 1), (33, 2), (46, 1), (64, 33), (180, 3)])
+def test_lists_made_from_tables(beads, B, dtype):
+    """Indices, parameters, run starts and the comparison with the reversed list of one pass (chunks of 2048 terms), for complete pair
+    lists, and for those with a term lost, doubled, replaced or of another parameter than its reverse."""
+    from mlcg_b200.backend import get_backend
+    be, gen, n = get_backend(), torch.Generator().manual_seed(beads), beads * B
+    i = torch.arange(beads)
+    one = torch.cartesian_prod(i, i).t()
+    one = one[:, one[0] != one[1]]
+    pairs = torch.cat([one + b * beads for b in range(B)], dim=1).to(DEV)
+    M = pairs.shape[1]
+    types = torch.randint(0, 5, (n,), generator=gen).to(DEV)
+    table = torch.rand(5, 5, generator=gen, dtype=dtype).to(DEV)
+    even, odd = table + table.t(), table
+    idx, params, symmetric, starts = be.prior_list(pairs, types, [even, even * 2], None, n, True)
+    assert torch.equal(idx.long(), pairs) and torch.equal(params, torch.stack([even[types[pairs[0]], types[pairs[1]]] * f for f in (1, 2)]))
+    assert symmetric and (starts is None) == (beads < 9)
+    if starts is not None:
+        assert torch.equal(starts, torch.arange(0, M, beads - 1, device=DEV))
+        slices, where, offsets, packed = _pair_slices(idx, params, starts)
+        first = slices[:, 0].tolist()
+        for run in (0, 31, 32, n - 1):
+            if run < n:
+                w, lane = run // 32, run % 32
+                rows = slice(first[w], first[w] + int(slices[w, 1]))
+                assert int(where[w, lane]) == run
+                got = offsets[rows, lane].flatten()[: beads - 1].long() + int(slices[w, 2])
+                assert torch.equal(got, pairs[1, run * (beads - 1): (run + 1) * (beads - 1)])
+                assert torch.equal(packed[:, rows, lane].flatten(1)[:, : beads - 1], params[:, run * (beads - 1): (run + 1) * (beads - 1)])
+    assert be.prior_list(pairs, types, None, params, n, True)[2]
+    if len(torch.unique(types)) > 1 and beads > 2:
+        assert not be.prior_list(pairs, types, [odd], None, n, True)[2]
+        for at in (0, M // 2, M - 1):
+            broken = pairs.clone()
+            broken[:, at] = broken[:, at - 1]                      # one term lost, another one twice
+            assert not be.prior_list(broken, types, [even], None, n, True)[2]
+            given = params.clone()
+            given[0, at] = given[0, at] * 1.5
+            assert not be.prior_list(pairs, types, None, given, n, True)[2]
+    for order in (3, 4):
+        terms = torch.randint(0, n, (order, 2049), generator=gen).to(DEV)
+        tables = [torch.rand(*([5] * order), generator=gen, dtype=dtype).to(DEV) for _ in range(3)]
+        idx, params, symmetric, starts = be.prior_list(terms, types, tables, None, n, False)
+        assert torch.equal(idx.long(), terms) and not symmetric and starts is None
+        assert torch.equal(params, torch.stack([t[tuple(types[terms[o]] for o in range(order))] for t in tables]))
+    be.check_pending()
+
+
+def test_a_bead_that_does_not_exist_is_reported():
+    from mlcg_b200.backend import get_backend
+    be = get_backend()
+    types, table = torch.zeros(4, dtype=torch.int64, device=DEV), torch.ones(1, 1, device=DEV)
+    idx, _, symmetric, _ = be.prior_list(torch.tensor([[0, 1, 4, 2], [1, 0, 2, 4]], device=DEV), types, [table], None, 4, True)
+    assert idx.tolist() == [[0, 1, -1, 2], [1, 0, 2, -1]]
+    status = be._sticky_status(torch.device(DEV))
+    assert int(status[0]) & 2
+    status.zero_()
