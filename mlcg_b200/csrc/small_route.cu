@@ -122,17 +122,39 @@ struct SmallTile {
 // Aggregation of the tile's nodes, 16 / RT warps per node (a contiguous part of its edges each), eight edges in flight per lane:
 //   FORCE    sum_j a[j] W[p], s[e] (+)= xi a[j] W'[p]        TANGENT  sum_j a[j] W[p] + b[j] dd W'[p]  (a NULL: zero)     PLAIN  sum_j a[j] W[p]
 enum { kAggPlain = 0, kAggForce = 1, kAggTangent = 2 };
-template <int MODE, int RT>
-__device__ __forceinline__ void small_aggregate(const SmallNet &p, const SmallTile<RT> &t, float *S) {
+
+// A warp's part of its row's edges, and of the first 32 of them the neighbours and pairs
+struct SmallEdges {
+    int64_t k0, k1;
+    int32_t j, p;
+};
+template <int RT>
+__device__ __forceinline__ SmallEdges small_edges(const SmallNet &p, const SmallTile<RT> &t) {
     constexpr int WPR = 16 / RT;
-    const int row = t.warp / WPR, part = t.warp % WPR, lane = t.lane;
+    const int part = t.warp % WPR;
+    const int64_t n = t.n0 + t.warp / WPR;
+    SmallEdges e = {0, 0, 0, 0};
+    if (n >= p.N) return e;
+    // (past the first-level cache: this may run before the wait for the kernel in front, where that cache may hold the lists of another call)
+    const int64_t b0 = __ldcg(p.ptr + n), b1 = __ldcg(p.ptr + n + 1), per = (b1 - b0 + WPR - 1) / WPR;
+    e.k0 = b0 + part * per;
+    e.k1 = e.k0 + per < b1 ? e.k0 + per : b1;
+    if (e.k0 + t.lane < e.k1) {
+        e.j = __ldcg(p.nbr + e.k0 + t.lane);
+        e.p = __ldcg(p.pair_of + e.k0 + t.lane);
+    }
+    return e;
+}
+
+template <int MODE, int RT>
+__device__ __forceinline__ void small_aggregate(const SmallNet &p, const SmallTile<RT> &t, float *S, const SmallEdges &ed) {
+    constexpr int WPR = 16 / RT;
+    const int row = t.warp / WPR, lane = t.lane;
     const int64_t n = t.n0 + row;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 *red = reinterpret_cast<float4 *>(t.x);                     // [16][32]
     if (n < p.N) {
-        const int64_t b0 = p.ptr[n], b1 = p.ptr[n + 1];
-        const int64_t per = (b1 - b0 + WPR - 1) / WPR;
-        const int64_t k0 = b0 + part * per, k1 = k0 + per < b1 ? k0 + per : b1;
+        const int64_t k0 = ed.k0, k1 = ed.k1;
         const float4 *a4 = reinterpret_cast<const float4 *>(p.in_a) + lane, *b4 = reinterpret_cast<const float4 *>(p.in_b) + lane;
         const float4 *W4 = reinterpret_cast<const float4 *>(p.W) + lane, *Wd4 = reinterpret_cast<const float4 *>(p.Wd) + lane;
         const float4 xi = MODE == kAggForce ? b4[n * 32] : acc;
@@ -140,11 +162,13 @@ __device__ __forceinline__ void small_aggregate(const SmallNet &p, const SmallTi
         constexpr int U = MODE == kAggPlain ? 8 : 4;
         for (int64_t c0 = k0; c0 < k1; c0 += 32) {                     // lane t holds edge c0 + t
             const int len = (int)(k1 - c0 < 32 ? k1 - c0 : 32);
-            int32_t my_j = 0, my_p = 0;
+            int32_t my_j = ed.j, my_p = ed.p;
             float my_d = 0.f;
             if (lane < len) {
-                my_j = p.nbr[c0 + lane];
-                my_p = p.pair_of[c0 + lane];
+                if (c0 > k0) {
+                    my_j = p.nbr[c0 + lane];
+                    my_p = p.pair_of[c0 + lane];
+                }
                 if (MODE == kAggTangent) my_d = p.dd[c0 + lane];
             }
             for (int g = 0; g < len; g += U) {
@@ -219,12 +243,27 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
     if (p.w[1]) t.fetch(1, p.w[1], 128);
     if (p.w[2]) t.fetch(2, p.w[2], kLast ? p.Wh : 128);
     asm volatile("cp.async.commit_group;" ::: "memory");
+    // What does not come from the kernel in front is read before the wait for it, a latency of the second-level cache each: biases and the
+    // lists of the first tile (the kernel in front began behind those that made the lists).  What does, and is wanted after a layer,
+    // is read under the aggregation (64 x 10 beads replayed: 64 -> 60.5 us).
+    constexpr bool kForward = KIND == kSmFwd || KIND == kSmFwdLast;
+    const float b2 = kForward ? p.b2[t.c] : 0.f, b3 = kForward ? p.b3[t.c] : 0.f;
+    const float bh = KIND == kSmFwdLast && t.c < p.Wh ? p.bh[t.c] : 0.f, wo = kLast && t.c < p.Wh ? p.wo[t.c] : 0.f;
+    t.n0 = (int64_t)blockIdx.x * RT;
+    SmallEdges ed = small_edges(p, t);
     pdl_wait();
     pdl_launch_dependents();
     float *S0 = t.rows(0), *S1 = t.rows(1);
     bool ready = false;
-    for (t.n0 = (int64_t)blockIdx.x * RT; t.n0 < p.N; t.n0 += (int64_t)gridDim.x * RT) {
-        small_aggregate<KIND == kSmFwd || KIND == kSmFwdLast ? kAggPlain : (KIND == kSmBwd ? kAggForce : kAggTangent), RT>(p, t, S0);
+    for (; t.n0 < p.N; t.n0 += (int64_t)gridDim.x * RT) {
+        if (ready) ed = small_edges(p, t);
+        float res[RO], act[RO];
+#pragma unroll
+        for (int i = 0; i < RO; i++) {
+            res[i] = p.res ? t.get(p.res, i) : 0.f;
+            act[i] = kForward || KIND == kSmRevFirst ? 0.f : t.get(p.act, i);
+        }
+        small_aggregate<kForward ? kAggPlain : (KIND == kSmBwd ? kAggForce : kAggTangent), RT>(p, t, S0, ed);
         if (!ready) {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();
@@ -235,14 +274,14 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
             t.template layer<true>(S0, t.slot(0), v);                  // lin2 + tanh
 #pragma unroll
             for (int i = 0; i < RO; i++) {
-                a[i] = tc::tanh_ex2(v[i] + p.b2[t.c]);
+                a[i] = tc::tanh_ex2(v[i] + b2);
                 t.put(p.o_act, i, a[i]);
             }
             t.hand_on(S1, a);
             t.template layer<true>(S1, t.slot(1), v);                  // lin + residual
 #pragma unroll
             for (int i = 0; i < RO; i++) {
-                v[i] += p.b3[t.c] + t.get(p.res, i);
+                v[i] += b3 + res[i];
                 t.put(p.o_x, i, v[i]);
             }
             t.hand_on(S0, v);
@@ -251,7 +290,6 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
 #pragma unroll
                 for (int i = 0; i < RO; i++) t.put(p.o_next, i, v[i]);
             } else {
-                const float bh = t.c < p.Wh ? p.bh[t.c] : 0.f, wo = t.c < p.Wh ? p.wo[t.c] : 0.f;
                 float y[RO];
 #pragma unroll
                 for (int i = 0; i < RO; i++) {
@@ -289,15 +327,14 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
             t.template layer<false>(S0, t.slot(0), v);                 // lin1^T + residual
 #pragma unroll
             for (int i = 0; i < RO; i++) {
-                v[i] += t.get(p.res, i);
+                v[i] += res[i];
                 t.put(p.o_g, i, v[i]);
             }
             t.hand_on(S1, v);
             t.template layer<false>(S1, t.slot(1), v);                 // lin^T, tanh' of the block below
 #pragma unroll
             for (int i = 0; i < RO; i++) {
-                const float aa = t.get(p.act, i);
-                v[i] *= fmaf(-aa, aa, 1.f);
+                v[i] *= fmaf(-act[i], act[i], 1.f);
                 t.put(p.o_gu, i, v[i]);
             }
             t.hand_on(S0, v);
@@ -308,7 +345,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
             t.template layer<true>(S0, t.slot(0), v);
 #pragma unroll
             for (int i = 0; i < RO; i++) {
-                a[i] = t.get(p.act, i);
+                a[i] = act[i];
                 q[i] = -2.f * a[i] * v[i] * t.get(p.gu, i);
                 v[i] *= fmaf(-a[i], a[i], 1.f);
                 t.put(p.o_act, i, v[i]);
@@ -318,7 +355,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
             t.template layer<true>(S1, t.slot(1), v);
 #pragma unroll
             for (int i = 0; i < RO; i++) {
-                if (p.res) v[i] += t.get(p.res, i);
+                v[i] += res[i];
                 t.put(p.o_x, i, v[i]);
             }
             t.hand_on(S0, v);
@@ -327,7 +364,6 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
 #pragma unroll
                 for (int i = 0; i < RO; i++) t.put(p.o_next, i, v[i]);
             } else {
-                const float wo = t.c < p.Wh ? p.wo[t.c] : 0.f;
 #pragma unroll
                 for (int i = 0; i < RO; i++) {
                     const int64_t n = t.node(i);
@@ -371,7 +407,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
             t.template layer<false>(S0, t.slot(0), v);
 #pragma unroll
             for (int i = 0; i < RO; i++) {
-                v[i] += t.get(p.res, i);
+                v[i] += res[i];
                 t.put(p.o_g, i, v[i]);
             }
             if (KIND == kSmRev) {
@@ -379,8 +415,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 t.template layer<false>(S1, t.slot(1), v);
 #pragma unroll
                 for (int i = 0; i < RO; i++) {
-                    const float aa = t.get(p.act, i);
-                    v[i] = fmaf(v[i], fmaf(-aa, aa, 1.f), t.get(p.q, i));
+                    v[i] = fmaf(v[i], fmaf(-act[i], act[i], 1.f), t.get(p.q, i));
                     t.put(p.o_ub, i, v[i]);
                 }
                 t.hand_on(S0, v);
@@ -641,6 +676,20 @@ small_finish_kernel(const float *__restrict__ pos, const float *__restrict__ d, 
                     const float *__restrict__ en, const int64_t *__restrict__ struct_ptr, int64_t B, float *__restrict__ energy) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    // (lists, distances and the first block's rows lie there long before the kernel in front is done)
+    int64_t k0 = 0, k1 = 0;
+    int32_t first_j = 0, first_p = 0, first_t = 0;
+    float first_d = 0.f;
+    if (grad && warp < N) {
+        k0 = __ldcg(ptr + warp);
+        k1 = __ldcg(ptr + warp + 1);
+        if (k0 + lane < k1) {
+            first_j = __ldcg(nbr + k0 + lane);
+            first_p = __ldcg(pair_of + k0 + lane);
+            if (s) first_t = __ldcg(twin + k0 + lane);
+            first_d = __ldcg(d + k0 + lane);
+        }
+    }
     pdl_wait();
     for (int64_t n = warp; n < N + B; n += nwarps) {
         if (n >= N) {
@@ -652,19 +701,23 @@ small_finish_kernel(const float *__restrict__ pos, const float *__restrict__ d, 
             continue;
         }
         if (!grad) continue;
-        const int64_t k0 = ptr[n], k1 = ptr[n + 1];
+        if (n != warp) { k0 = ptr[n]; k1 = ptr[n + 1]; }
         const float4 *g4 = reinterpret_cast<const float4 *>(gagg) + lane, *x4 = reinterpret_cast<const float4 *>(xl) + lane;
         const float4 *Wd4 = reinterpret_cast<const float4 *>(Wd) + lane;
         const float4 gi = g4[n * 32], xi = x4[n * 32];
         float s0 = 0.f, s1 = 0.f, s2 = 0.f;
         for (int64_t c0 = k0; c0 < k1; c0 += 32) {
             const int len = (int)(k1 - c0 < 32 ? k1 - c0 : 32);
-            int32_t my_j = 0, my_p = 0;
-            float my_s = 0.f;
+            int32_t my_j = first_j, my_p = first_p, my_t = first_t;
+            float my_s = 0.f, my_d = first_d;
             if (lane < len) {
-                my_j = nbr[c0 + lane];
-                my_p = pair_of[c0 + lane];
-                if (s) my_s = s[c0 + lane] + s[twin[c0 + lane]];
+                if (n != warp || c0 > k0) {
+                    my_j = nbr[c0 + lane];
+                    my_p = pair_of[c0 + lane];
+                    if (s) my_t = twin[c0 + lane];
+                    my_d = d[c0 + lane];
+                }
+                if (s) my_s = s[c0 + lane] + s[my_t];
             }
             for (int g = 0; g < len; g += 4) {
                 float dot[4];
@@ -690,8 +743,7 @@ small_finish_kernel(const float *__restrict__ pos, const float *__restrict__ d, 
                 if (lane >= g && lane < g + 4 && lane < len) my_s += mine;
             }
             if (lane < len) {
-                const float dk = d[c0 + lane];
-                const float w = dk > 0.f ? sign * my_s / dk : 0.f;
+                const float w = my_d > 0.f ? sign * my_s / my_d : 0.f;
                 const int64_t j = my_j;
                 s0 = fmaf(w, pos[3 * n] - pos[3 * j], s0);
                 s1 = fmaf(w, pos[3 * n + 1] - pos[3 * j + 1], s1);
