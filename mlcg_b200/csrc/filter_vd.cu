@@ -19,7 +19,9 @@
 // fp32 in shared memory).
 // Bound by instruction issue and latency at one CTA per SM.  With the four GEMMs of a tile in turn on two accumulators every pass
 // waited for the one before: three launches over 553 k pairs took 757 us, like this 684, and with the arithmetic between the GEMMs
-// in pairs (two operations an instruction) 662 (bf16: 470, 441).
+// in pairs (two operations an instruction) 662 (bf16: 470, 441), without the part of the basis that is zero and with the per-row values
+// made where a product is waited for 624 (bf16: 410).  A tile takes 12 100 cycles: tanh 2100, the two stores 1700, phi' 1300 and phi
+// 1450, the derivative operand 2000, waiting for products and other warps 2800; the products themselves 4600.
 // Replaces the backward GEMM kernel in the force pass (filter_tc.cu): per block, forward + backward took 0.16 + 0.25 ms.
 #include "filter_common.cuh"
 #include "schnet_internal.cuh"
@@ -38,8 +40,9 @@ struct FilterVdParams {
     float *zmax;         // with Zd: largest |z'| (to be zero before; non-negative floats order like their bits)
 };
 
-// per-row values of four tiles behind the shared layout of the filter kernels
-template <bool SPLIT> constexpr int kVdSmem = FilterSmem<SPLIT>::kExtra + 16384 + (SPLIT ? 0 : 32768) + 1024;
+// per-row values of six tiles behind the shared layout of the filter kernels
+constexpr int kRowSlots = 6, kRowBytes = kRowSlots * 4096;
+template <bool SPLIT> constexpr int kVdSmem = FilterSmem<SPLIT>::kExtra + kRowBytes + (SPLIT ? 0 : 32768) + 1024;
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(kTcThreads + 32, 1)
@@ -72,6 +75,8 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
     const float wscale = SPLIT ? kWScale : 1.f;
     const float unscale = 1.f / wscale;
 
+    uint8_t *s_live = smem + L::kMisc + L::kRed2;      // [tile & 1][16 warps]: the warp's part of the tile's phi is not all zero
+
     const uint32_t tmem = filter_setup<SPLIT>(p, smem, Kpad1, 512);
     if (tid == 0) {
         for (int i = 0; i < 4; i++) {
@@ -82,6 +87,18 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
     float slope = 0.f;               // steepest basis function: |d g_k / dt| <= sqrt(2 ln2 w_k / e) where g_k = 2^(-w_k (t - c_k)^2)
     for (int k = 0; k < R; k++) slope = fmaxf(slope, fabsf(s_tab[k].y));
     slope = 0.7142f * sqrtf(slope);
+    // Where this quarter's functions are not zero as operands.  At w (t - c)^2 > 36 a function is below 2^-36: zero as a pair of fp16 (below
+    // 2^-25), and so is its derivative on the scale of its row (below 16 (z / 0.6065 + 1) 2^-36 < 2^-28 at z = 7.1 widths).  Exp-normal
+    // functions crowd the short distances that no bead comes to: of 128 over 15 A those beyond the 45th are zero at 4 A and more,
+    // over 10 A those beyond the 29th.  A warp whose 32 rows are all outside stores zeros, and the first GEMMs leave a quarter of K out that
+    // is zero in the whole tile: the same sums, bit by bit.
+    float near_lo = INFINITY, near_hi = -INFINITY;
+    for (int k = col0; k < col0 + 32 && k < R; k++) {
+        const float2 cw = s_tab[k];
+        const float reach = cw.y > 0.f ? sqrtf(36.f / cw.y) : INFINITY;
+        near_lo = fminf(near_lo, cw.x - reach);
+        near_hi = fmaxf(near_hi, cw.x + reach);
+    }
     __syncthreads();
     pdl_wait();                      // set-up done (weights only); from here on the distances of the previous kernels are read
     pdl_launch_dependents();
@@ -111,16 +128,36 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
             }
             __syncwarp();
         };
+        const auto gemm1 = [&](uint32_t d, uint32_t ta, uint32_t quarters, uint32_t done) {
+            if (elected) {
+                issue_gemm_ts_quarters<SPLIT>(d, ta, b1_hi, b1_lo, quarters ? quarters : 1u);
+                mma_commit(done);
+            }
+            __syncwarp();
+        };
+        const auto live_quarters = [&](uint32_t parity) {      // of the tile whose phi has been signalled
+            const unsigned w = __ballot_sync(0xffffffffu, lane < 16 && *reinterpret_cast<volatile uint8_t *>(s_live + parity * 16 + lane));
+            return (w & 0xfu ? 1u : 0u) | (w & 0xf0u ? 2u : 0u) | (w & 0xf00u ? 4u : 0u) | (w & 0xf000u ? 8u : 0u);
+        };
         uint32_t tV = tmem, tA = tmem + 128, tQ = tmem + 256;
         const uint32_t tR = tmem + 384;
-        if (n_local > 0) gemm(r1v, 0, tA, tV, b1_hi, b1_lo, Kpad1 / 16, c1v);
+        uint32_t quarters = 0, next = 0;
+        if (n_local > 0) {
+            await(r1v, 0);
+            next = live_quarters(0);
+            gemm1(tA, tV, next, c1v);
+        }
         for (int64_t j = 0; j < n_local; j++) {
             const uint32_t par = (uint32_t)(j & 1);
+            quarters = next;
             gemm(r2v, par, tA, tV, b2_hi, b2_lo, kF / 16, c2v);
-            gemm(r1d, par, tR, tQ, b1_hi, b1_lo, Kpad1 / 16, c1d);
+            await(r1d, par);
+            gemm1(tR, tQ, quarters, c1d);
             if (j + 1 < n_local) {
                 await(c1d, par);                       // phi' has been read: its block takes the next tile's values
-                gemm(r1v, par ^ 1, tQ, tA, b1_hi, b1_lo, Kpad1 / 16, c1v);
+                await(r1v, par ^ 1);
+                next = live_quarters(par ^ 1);
+                gemm1(tQ, tA, next, c1v);
             }
             gemm(r2d, par, tR, tV, b2_hi, b2_lo, kF / 16, c2d);
             const uint32_t old = tV;
@@ -132,14 +169,12 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
         uint32_t tV = t_lane, tA = t_lane + 128, tQ = t_lane + 256;
         const uint32_t tR = t_lane + 384;
         // fp32 hidden values of the bf16 mode (thread-private): chunks 0..3 in the operand region that it leaves free, 4..7 behind the rows
-        float4 *const h_lo = reinterpret_cast<float4 *>(smem + L::kA) + tid, *const h_hi = reinterpret_cast<float4 *>(smem + L::kExtra + 16384) + tid;
+        float4 *const h_lo = reinterpret_cast<float4 *>(smem + L::kA) + tid, *const h_hi = reinterpret_cast<float4 *>(smem + L::kExtra + kRowBytes) + tid;
         const bool same_env = p.conv.cutoff_kind == p.rbf.cutoff_kind && p.conv.lower == p.rbf.lower && p.conv.upper == p.rbf.upper;
-        auto load_d = [&](int64_t tile) {
-            const int64_t k = tile * kRows + r;
-            return k < nE ? p.d[p.sel ? (int64_t)p.sel[k] : k] : 1.f;
-        };
         // per-row values of a tile.  The four threads of a row (one per quarter) each work them out for one of the next four tiles and
-        // share them: every thread for every tile took a fifth of the kernel's instructions
+        // share them: every thread for every tile took a fifth of the kernel's instructions.  That is done in the third of four tiles, where
+        // the second value GEMM would be waited for, into slots that nobody reads any more by then (six, and the barrier before the
+        // tile's next operand in between); the edge and its distance are fetched two tiles ahead of their use each.
         struct Scalars { float t, dt, e0, e1, c0, c1, s1, l2e; };
         auto scalars = [&](float de) {
             Scalars s;
@@ -159,20 +194,23 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
             s.l2e = log2f(s.e0);
             return s;
         };
-        float4 *const s_rows = reinterpret_cast<float4 *>(smem + L::kExtra);       // [4 tiles][2][128]
+        float4 *const s_rows = reinterpret_cast<float4 *>(smem + L::kExtra);       // [6 tiles][2][128]
         auto row_group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(2 + (warp & 3)) : "memory"); };
-        float d_ahead = 1.f;                                         // distance of the tile this thread prepares next
-        auto fetch = [&](int64_t tile) { d_ahead = tile < ntiles ? load_d(tile) : 1.f; };
-        auto prepare = [&](int64_t group_tile) {                     // the four tiles from group_tile on
-            row_group_sync();                                        // (the four before are done with)
-            const Scalars s = scalars(d_ahead);
-            s_rows[(qt * 2) * 128 + r] = make_float4(s.t, s.dt, s.e0, s.e1);
-            s_rows[(qt * 2 + 1) * 128 + r] = make_float4(s.c0, s.c1, s.s1, s.l2e);
-            fetch(group_tile + (4 + qt) * step);
-            row_group_sync();
+        // of the tile that this thread prepares next: its edge (-1: no row), then the edge's distance
+        auto fetch_edge = [&](int64_t n) {
+            const int64_t k = (first + (n + qt) * step) * kRows + r;
+            return k < nE ? (p.sel ? __ldg(p.sel + k) : (int32_t)k) : -1;       // (lists have fewer than 2^31 edges)
         };
-        auto read_scalars = [&](int slot) {
-            const float4 a = s_rows[(slot * 2) * 128 + r], b = s_rows[(slot * 2 + 1) * 128 + r];
+        auto fetch_d = [&](int32_t edge) { return edge < 0 ? 1.f : __ldg(p.d + edge); };
+        auto prepare = [&](int64_t n, float d) {                     // tile n + qt of this block
+            const Scalars s = scalars(d);
+            float4 *row = s_rows + (int)((uint32_t)(n + qt) % (uint32_t)kRowSlots) * 256 + r;
+            row[0] = make_float4(s.t, s.dt, s.e0, s.e1);
+            row[128] = make_float4(s.c0, s.c1, s.s1, s.l2e);
+        };
+        auto read_scalars = [&](int64_t n) {
+            const float4 *row = s_rows + (int)((uint32_t)n % (uint32_t)kRowSlots) * 256 + r;
+            const float4 a = row[0], b = row[128];
             return Scalars{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
         };
         auto signal = [&](uint32_t bar) {
@@ -180,8 +218,17 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
             __syncwarp();
             if (lane == 0) mbar_arrive(bar);
         };
-        auto basis = [&](const Scalars &s, uint32_t ta) {
-            if (col0 < Kpad1) {
+        auto store_zeros = [&](uint32_t ta) {
+            tmem_zero16(ta + (col0 >> 1));
+            if (SPLIT) tmem_zero16(ta + 64 + (col0 >> 1));
+        };
+        // (rows past the end count as far away; a distance that is not a number does not)
+        auto basis = [&](const Scalars &s, uint32_t ta, int64_t n, int64_t tile) {
+            const bool live = __any_sync(0xffffffffu, !(s.t <= near_lo) && !(s.t >= near_hi) && tile * kRows + r < nE);
+            if (lane == 0) s_live[(n & 1) * 16 + warp] = live;
+            if (!live) {
+                if (col0 < Kpad1) store_zeros(ta);
+            } else if (col0 < Kpad1) {
                 const float l2a = s.l2e;
                 float x[32];
                 const float4 *tab4 = reinterpret_cast<const float4 *>(s_tab + col0);   // two (centre, width) pairs per 128-bit read
@@ -195,10 +242,13 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
                 store_a_tmem<SPLIT, kPackAsIs>(ta, col0, x, 1.f);
             }
             tmem_wait_st();
+            return live;
         };
         // phi'_k = g_k (env' - env 2 ln2 w_k (t - c_k) t'); columns at or beyond R: exactly 0
-        auto basis_derivative = [&](const Scalars &s) {
-            if (col0 < Kpad1) {
+        auto basis_derivative = [&](const Scalars &s, bool live) {
+            if (!live) {
+                if (col0 < Kpad1) store_zeros(tQ);
+            } else if (col0 < Kpad1) {
                 const float m2 = -2.f * kLn2 * s.dt * s.e0;
                 float x[32];
                 const float4 *tab4 = reinterpret_cast<const float4 *>(s_tab + col0);
@@ -237,16 +287,22 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
         };
 
         float zmax = 0.f;
+        int32_t edge_ahead = -1;
+        float d_ahead = 1.f;
+        bool live = false, live_next = false;                       // this warp's part of phi, this tile and the next
         float f_prev = 0.f;                                         // factor of the derivative rows whose GEMM is in flight
         if (n_local > 0) {
-            fetch(first + qt * step);
-            prepare(first);
-            basis(read_scalars(0), tV);
+            prepare(0, fetch_d(fetch_edge(0)));
+            edge_ahead = fetch_edge(4);
+            row_group_sync();
+            live_next = basis(read_scalars(0), tV, 0, first);
             signal(r1v);
         }
         int64_t tile = first;
         for (int64_t n = 0; n < n_local; n++, tile += step) {
             const uint32_t par = (uint32_t)(n & 1);
+            live = live_next;
+            if ((n & 3) == 0) d_ahead = fetch_d(edge_ahead);
             // ---- hidden layer
             await(c1v, par);
             {
@@ -269,18 +325,21 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
                 await(c2d, par ^ 1);
                 store_rows(&dmap, tile - step, tR, f_prev);
             }
-            const Scalars sc = read_scalars((int)(n & 3));
-            basis_derivative(sc);
+            const Scalars sc = read_scalars(n);
+            basis_derivative(sc, live);
             signal(r1d);
+            if ((n & 3) == 2 && n + 2 < n_local) {
+                prepare(n + 2, d_ahead);
+                edge_ahead = fetch_edge(n + 6);
+            }
             await(c2v, par);
             store_rows(&wmap, tile, tA, sc.c0 * unscale);
             if (n + 1 < n_local) {
                 // (the next tile's operand overwrites the accumulator just read: by all four quarters of the row)
                 tc_fence_before();
-                if (((n + 1) & 3) == 0) prepare(tile + step);
-                else row_group_sync();
+                row_group_sync();
                 tc_fence_after();
-                basis(read_scalars((int)((n + 1) & 3)), tA);
+                live_next = basis(read_scalars(n + 1), tA, n + 1, tile + step);
                 signal(r1v);
             }
             // ---- second operand of the derivatives, in place of h

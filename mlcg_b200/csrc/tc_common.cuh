@@ -254,6 +254,9 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
         "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};\n" ::"r"(taddr), "r"(0u) : "memory");
+}
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Two fp32 operations in one instruction, each rounded like the scalar one.  The element-wise phases between the GEMMs are bound by
@@ -409,6 +412,35 @@ __device__ __forceinline__ void issue_gemm_ts(uint32_t tmem_d, uint32_t ta, uint
             mma_f16_ts(tmem_d, ta + 64 + ks * 8, b_mn ? kstep_mnmajor(dbh, ks) : kstep_kmajor(dbh, ks), idesc, 1u);
         }
     for (int ks = 0; ks < ksteps; ks++) mma_f16_ts(tmem_d, ta + ks * 8, b_mn ? kstep_mnmajor(dbh, ks) : kstep_kmajor(dbh, ks), idesc, SPLIT || ks > 0 ? 1u : 0u);
+}
+
+// The same (K-major B) over the 32-element quarters of K whose bit is set: the A operand is zero in the others
+template <bool SPLIT>
+__device__ __forceinline__ void issue_gemm_ts_quarters(uint32_t tmem_d, uint32_t ta, uint32_t b_hi, uint32_t b_lo, uint32_t live) {
+    const uint32_t idesc = instr_desc(SPLIT ? 0 : 1, 0, 128);
+    const uint64_t dbh = desc_kmajor(b_hi), dbl = desc_kmajor(b_lo);
+    uint32_t more = 0u;
+    if (SPLIT) {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (live >> q & 1u) {
+#pragma unroll
+                for (int ks = 2 * q; ks < 2 * q + 2; ks++) {
+                    mma_f16_ts(tmem_d, ta + ks * 8, kstep_kmajor(dbl, ks), idesc, more);
+                    more = 1u;
+                    mma_f16_ts(tmem_d, ta + 64 + ks * 8, kstep_kmajor(dbh, ks), idesc, 1u);
+                }
+            }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if (live >> q & 1u) {
+#pragma unroll
+            for (int ks = 2 * q; ks < 2 * q + 2; ks++) {
+                mma_f16_ts(tmem_d, ta + ks * 8, kstep_kmajor(dbh, ks), idesc, more);
+                more = 1u;
+            }
+        }
 }
 
 // tanh through exp2: tanh z = sign(z) (1 - 2 / (2^{2 log2(e) |z|} + 1)); 2^x overflowing to inf gives exactly 1.

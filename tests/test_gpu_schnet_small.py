@@ -188,3 +188,30 @@ def test_large_batches_with_nodes_of_every_degree(blocks):
     assert torch.allclose(out["energy"].cpu().double(), e_x, rtol=E_RTOL, atol=E_RTOL * float(e_x.abs().max()))
     # (dense clusters: forces of hundreds, to the same number of digits as elsewhere)
     assert float((out["forces"].cpu().double() - f_x).abs().max()) < F_ATOL * max(1.0, float(f_x.abs().max()) / 10)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+@pytest.mark.parametrize("basis,num_rbf,upper", [("expnormal", 128, 10.0), ("expnormal", 100, 15.0), ("gaussian", 128, 15.0), ("gaussian", 33, 30.0)])
+def test_distances_on_both_sides_of_the_basis_that_is_zero(basis, num_rbf, upper, precision):
+    """Pairs of two beads at distances from almost nothing to beyond the cutoff: quarters of the basis that are zero for a warp, for a tile,
+    or for none, tiles of one kind and mixed ones, several tiles per block."""
+    torch.manual_seed(4)
+    cut = bnn.CosineCutoff(0.0, upper)
+    kind = {"expnormal": bnn.ExpNormalBasis, "gaussian": bnn.GaussianBasis}[basis]
+    net = bnn.StandardSchNet(kind(cut, num_rbf, trainable=False), cut, [128], hidden_channels=128, embedding_size=4, num_filters=128, num_interactions=1)
+    pairs = 900
+    gen = torch.Generator().manual_seed(5)
+    d = torch.cat([torch.linspace(0.05, 1.02 * upper, pairs - 300), torch.full((150,), 0.9 * upper), torch.full((150,), 0.3)])
+    d[300:450] = d[300:450][torch.randperm(150, generator=gen)]
+    pos = torch.zeros(2 * pairs, 3)
+    pos[1::2, 0] = d
+    types_, batch = torch.randint(0, 4, (2 * pairs,), generator=gen), torch.arange(pairs).repeat_interleave(2)
+    e_x, f_x, _ = _oracle(net, basis, upper, 1, pos, types_, batch, pairs, torch.float64)
+    bnn.set_filter_precision(net.to(DEV).eval(), precision)
+    out = bnn.GradientsOut(net, "forces").eval()(mlcg_b200.AtomicData(pos=pos.to(DEV), atom_types=types_.to(DEV), batch=batch.to(DEV),
+                                                                      n_atoms=torch.full((pairs,), 2).to(DEV))).out["SchNet"]
+    e, f = out["energy"].cpu().double(), out["forces"].cpu().double()
+    if precision == "fp32":
+        assert torch.allclose(e, e_x, rtol=E_RTOL, atol=E_RTOL * float(e_x.abs().max())) and float((f - f_x).abs().max()) < F_ATOL
+    else:
+        assert float((f - f_x).norm() / f_x.norm()) < 1e-2
