@@ -189,3 +189,24 @@ def check(code: int, what: str):
         msg = lib.mlcgb_strerror(code).decode()
         extra = f" (cudaError {lib.mlcgb_last_cuda_error()})" if code == -3 else ""
         raise RuntimeError(f"mlcg_b200: {what} failed: {msg}{extra}")
+
+
+_native_module = None
+
+
+def native():
+    """The host side of the hot calls (``csrc/host.cpp``), with the library's entry points handed over once it is loaded; raises
+    :class:`ExtensionMissing` where it has not been built."""
+    global _native_module
+    if _native_module is None:
+        try:
+            from . import _native
+        except ImportError as exc:
+            raise ExtensionMissing(f"{os.path.join(_HERE, '_native.so')} cannot be loaded ({exc}); build it with `python -m mlcg_b200.build`") from exc
+        _native_module = _native
+    return _native_module
+
+
+def bind_native(lib):
+    native().bind(*(ctypes.cast(getattr(lib, name), c_vp).value for name in ("mlcgb_schnet_evaluate", "mlcgb_schnet_evaluate_workspace_bytes",
+                                                                              "mlcgb_prior_eval", "mlcgb_prior_eval_workspace_bytes")))

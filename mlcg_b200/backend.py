@@ -206,6 +206,8 @@ class CudaBackend:
 
     def __init__(self):
         self.lib = _lib.load()
+        _lib.bind_native(self.lib)
+        self.native = _lib.native()
         self.profiler = None
         self._status = {}
         self.tensor_core_gemm = True   # float32 GEMMs of qualifying shape run on tcgen05 (fp32-equivalent products)
@@ -873,31 +875,17 @@ class CudaBackend:
         [N,3], edge count, None)``; None for a list without edges or cut short.  ``n_atoms`` or ``ptr`` (the other None); ``edges``: a
         guess at the edge count that sizes the workspace (too low costs a second call).  ``training``: the forward pass of
         :meth:`schnet_train_forward` (forces), its state as the last value."""
-        _need_cuda(pos, types, n_atoms, ptr)
         w, _keep = weights
-        pos = pos.detach().contiguous()
-        N, dev = pos.shape[0], pos.device
-        B = ptr.numel() - 1 if n_atoms is None else n_atoms.numel()
+        dev = pos.device
         s, keep = self._spec(spec, torch.float32)
         pend = self._take_pending(dev)
         status = self._sticky_status(dev)
-        lib, ref, size = self.lib, ctypes.byref(w), self.lib.mlcgb_schnet_evaluate_workspace_bytes
         with _on(dev):
-            energy = torch.empty(B, dtype=torch.float32, device=dev)
-            grad = torch.empty((N, 3), dtype=torch.float32, device=dev)
-            gb, wsb = size(N, B, -1, 0, ref, 0), size(N, B, max(int(edges), 0), spec.num_rbf, ref, training)
-            graph_ws, ws = torch.empty(gb, dtype=torch.uint8, device=dev), torch.empty(wsb, dtype=torch.uint8, device=dev)
-            host = (ctypes.c_int64 * 5)()
-            while True:
-                _lib.check(lib.mlcgb_schnet_evaluate(
-                    pos.data_ptr(), types.data_ptr(), _ptr(n_atoms), _ptr(ptr), N, B, r, max_num_neighbors, ctypes.byref(s), conv_cut[0], conv_cut[1],
-                    conv_cut[2], ref, precision, int(forces), training, graph_ws.data_ptr(), gb, ws.data_ptr(), wsb, energy.data_ptr(), grad.data_ptr(),
-                    pend[0][0].data_ptr() if pend else None, status.data_ptr(), host, _stream()), "schnet_evaluate")
-                if host[4] != _lib.EVALUATE_MORE:
-                    break
-                del ws
-                wsb = size(N, B, host[0], spec.num_rbf, ref, training)
-                ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
+            code, host, energy, grad, ws, graph_ws = self.native.evaluate(
+                pos, types, n_atoms, ptr, r, max_num_neighbors, ctypes.addressof(s), conv_cut[0], conv_cut[1], conv_cut[2], ctypes.addressof(w), precision,
+                forces, training, max(int(edges), 0), pend[0][0] if pend else None, status, _stream())
+        if code:
+            _lib.check(code, "schnet_evaluate")
         if pend and host[2]:
             self._raise_pending([int(host[2])], pend)
         if host[4] != _lib.EVALUATE_DONE:
@@ -906,10 +894,11 @@ class CudaBackend:
         self.defer_status(status, "SchNet force matching" if training else "SchNet evaluation")
         if not training:
             return energy, grad, E, None
+        N, B, ref = grad.shape[0], energy.shape[0], ctypes.byref(w)
         at = (ctypes.c_int64 * 8)()
-        lib.mlcgb_schnet_evaluate_lists(N, B, E, at)
+        self.lib.mlcgb_schnet_evaluate_lists(N, B, E, at)
         places = ((0, 0), (4, at[0]) if ptr is None else (5, 0), (3, at[2]), (3, at[3]), (4, at[1]), (3, at[6]), (3, at[5]), (3, at[7]), (3, at[4]), (1, 0), (2, 0))
-        ws = ws[:size(N, B, E, spec.num_rbf, ref, 1)]          # (saved with the size that its edges ask for, not that of the guess)
+        ws = ws[:self.lib.mlcgb_schnet_evaluate_workspace_bytes(N, B, E, spec.num_rbf, ref, 1)]          # (saved with the size that its edges ask for, not that of the guess)
         return energy, grad, E, ForceMatchingState(N, B, E, (types, spec.p0, spec.p1, ws, graph_ws, ptr), places, spec, conv_cut, weights)
 
     def schnet_fixed_ok(self, N, B, weights) -> bool:
@@ -975,7 +964,7 @@ class CudaBackend:
         views of one buffer in the order of the packed weights (``None`` for the output network's second bias).  ``saved``, ``params``:
         the buffers of the state and the weights (without the absent ones) as the autograd node's saved tensors hand them back."""
         wstruct, (_, tensors, live, addresses) = state.weights
-        if tuple([t.data_ptr() for t in params]) != addresses:       # (moved by a saved-tensor hook)
+        if self.native.pointers(list(params)) != addresses:          # (moved by a saved-tensor hook)
             moved = iter([t.contiguous() for t in params])
             weights = [None if t is None else next(moved) for t in tensors]
             wstruct, _keep = weights_struct(wstruct, weights)
@@ -995,7 +984,7 @@ class CudaBackend:
                 ctypes.byref(wstruct), 1, _ptr(gE), _ptr(gF), forward_ws, ws.data_ptr(), wsb, ctypes.byref(gs), status.data_ptr(), _stream()),
                 "schnet_train_backward")
         self.defer_status(status, "SchNet force matching")
-        views = iter(torch._C._nn.unflatten_dense_tensors(flat, live))        # (behind the launches: the device is busy by now)
+        views = iter(self.native.views(flat, live))                  # (behind the launches: the device is busy by now)
         return [None if t is None or k == 4 else next(views) for k, t in enumerate(tensors)]
 
     # ------------------------------------------------------------------ fused filter network (tensor cores)
@@ -1147,51 +1136,22 @@ class CudaBackend:
         ``mlcgb_prior_list`` describes them (at most ``_lib.MAX_PRIOR_SEGMENTS``).  Returns ``(energy [n, B], dE/dpos [n, N, 3])``, one row / block
         per list (``forces``: the negative gradient), and with ``totals`` their sums ``(energy [B], gradient [N, 3])`` over the lists.
         ``deterministic``: sums formed as 64-bit fixed-point integers (bit-identical from run to run)."""
-        _need_cuda(pos, batch)
         n = len(lists)
         if n == 0 or n > _lib.MAX_PRIOR_SEGMENTS:
             raise ValueError(f"between 1 and {_lib.MAX_PRIOR_SEGMENTS} prior lists per launch")
-        pos = pos.detach().contiguous()
-        N, dev, dt = pos.shape[0], pos.device, _dt(pos)
-        if batch is not None:
-            batch = batch.to(torch.int64).contiguous()
-            if batch.numel() != N:
-                raise ValueError("batch must have one entry per bead")
-        arr = (_lib.PriorListStruct * n)()
-        keep = []
-        M_total = moved = 0
-        for k, (kind, idx, params, symmetric, sliced) in enumerate(lists):
-            a = arr[k]
-            if sliced is not None:
-                slices, beads, offsets, params = sliced
-                _need_cuda(pos, *sliced)
-                M, per_term = offsets.shape[0] * 128, 2
-                a.n_slices, a.steps, a.slices, a.slice_beads = slices.shape[0], offsets.shape[0], slices.data_ptr(), beads.data_ptr()
-                a.offsets, a.slice_params = offsets.data_ptr(), params.data_ptr()
-            else:
-                _need_cuda(pos, idx, params)
-                if idx.dtype != torch.int32:
-                    raise TypeError("prior lists take int32 indices")
-                idx, params = idx.contiguous(), params.contiguous()
-                M, per_term = idx.shape[1], 4 * idx.shape[0]
-                keep += [idx, params]
-                a.idx, a.params = idx.data_ptr(), params.data_ptr()
-            if params.dtype != pos.dtype:
-                raise TypeError("prior lists take parameters of the positions' dtype")
-            a.kind, a.n_params, a.symmetric, a.M = kind, params.shape[0], bool(symmetric), M
-            M_total += M
-            moved += M * (params.shape[0] * pos.element_size() + per_term)
-        rows = n + 1 if totals else n
-        buf = torch.empty(rows * (3 * N + B), dtype=pos.dtype, device=dev)
-        grad, energy = buf[: rows * 3 * N].view(rows, N, 3), buf[rows * 3 * N:].view(rows, B)
-        status = self._sticky_status(dev)
+        _dt(pos)
+        dev, prof = pos.device, self.profiler
+        if prof is not None:
+            terms = [l[4][2].numel() if l[4] is not None else l[1].shape[1] for l in lists]
+            moved = sum(m * ((l[4][3] if l[4] is not None else l[2]).shape[0] * pos.element_size() + (2 if l[4] is not None else 4 * l[1].shape[0]))
+                        for m, l in zip(terms, lists))
+            event = prof.begin("prior_eval", 4, moved + 2 * pos.numel() * pos.element_size(), 40 * sum(terms))
         with _on(dev):
-            wsb = self.lib.mlcgb_prior_eval_workspace_bytes(n, N, B, dt)
-            ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
-            self._run("prior_eval", self.lib.mlcgb_prior_eval,
-                      (n, arr, _ptr(pos), dt, _ptr(batch), N, B, energy.data_ptr(), grad.data_ptr(), int(forces), energy[n].data_ptr() if totals else None,
-                       grad[n].data_ptr() if totals else None, 1 if deterministic else 0, _ptr(ws), wsb, _ptr(status), _stream()),
-                      launches=4, nbytes=moved + 2 * pos.numel() * pos.element_size(), flops=40 * M_total)
+            code, energy, grad = self.native.prior_eval(lists, pos, batch, B, bool(deterministic), bool(forces), bool(totals), self._sticky_status(dev), _stream())
+        if code:
+            _lib.check(code, "prior_eval")
+        if prof is not None:
+            prof.end("prior_eval", event)
         return energy, grad
 
 

@@ -9,6 +9,7 @@ from typing import Final, List
 
 import torch
 
+from .._lib import native
 from ..autograd import (attach_plan, EdgeDiff, EdgeDistanceOnce, EdgePlan, FusedFilterConv, FusedInteraction, PairSelect, RowScale, SchNetEval, SchNetForceMatching, SegIn, SegmentSum, SegPair,
                         edge_distances, plan_of)
 from ..autograd import tanh as tanh_op
@@ -369,9 +370,9 @@ class SchNet(torch.nn.Module):
     def packed_weights(self, layers=None):
         """``mlcgb_schnet_weights`` over the current parameters (rebuilt whenever a parameter's storage has moved), or None."""
         tensors = (self._layers() if layers is None else layers).weights()
-        if tensors is None or not all([t is None or t.is_contiguous() for t in tensors]):
+        key = None if tensors is None else native().pointers(tensors)       # (None: a weight that is not contiguous)
+        if key is None:
             return None
-        key = tuple([t.data_ptr() for t in tensors if t is not None])
         packed = self.__dict__.get("_mlcgb_packed")
         if packed is not None and packed[0] == key:
             return packed[1]

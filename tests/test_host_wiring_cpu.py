@@ -419,3 +419,23 @@ def test_condensed_priors_equal_the_reference_s(golden_condensed_priors):
     assert torch.allclose(out.out["forces"], g["forces"], rtol=1e-4, atol=1e-4 * float(g["forces"].abs().max()))
     for k, e in g["per_model_energy"].items():
         assert torch.allclose(out.out[k]["energy"], e, rtol=1e-5, atol=1e-4)
+
+
+def test_native_descriptions_of_tensors():
+    """What kept weights and lists are recognised by: an address, a version, a shape or a stride that changes is seen."""
+    from mlcg_b200 import _lib
+    n = _lib.native()
+    a, b = torch.arange(12.0).view(3, 4), torch.arange(5)
+    assert n.pointers([a, None, b]) == n.pointers([a, b]) and len(n.pointers([a, b])) == 16
+    assert n.pointers([a.t(), b]) is None and n.pointers([a, b]) != n.pointers([b, a])
+    seen = {n.layouts((a, b)), n.layouts((a.t(), b)), n.layouts((a.view(4, 3), b)), n.layouts((a[:2], b)), n.layouts((a,)), n.layouts((a, b + 0))}
+    a.add_(1.0)
+    seen.add(n.layouts((a, b)))
+    assert len(seen) == 7 and n.layouts((a, b)) in seen
+    like = [torch.empty(2, 3), torch.empty(4), torch.empty(()), torch.empty(1, 1)]
+    flat = torch.arange(12.0)
+    got = n.views(flat, like)
+    assert [g.shape for g in got] == [t.shape for t in like] and all(g.is_contiguous() for g in got)
+    assert torch.equal(torch.cat([g.flatten() for g in got]), flat)
+    with pytest.raises(TypeError):
+        n.pointers([3])
