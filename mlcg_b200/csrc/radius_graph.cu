@@ -2226,16 +2226,15 @@ extern "C" int mlcgb_radius_graph_static(const void *pos, int dtype, const int64
 namespace mlcgb {
 
 
-// Larger batches whose structures have at most 768 points on average: those that do go the same way (mask_rows_kernel); in a batch of
-// large structures the bit rows (192 bytes per point) would be room for nothing.  Graph and plan of 40 000 points in structures of
-// one size, us, bit rows : cells,
-//   points            400        576        768       1024
-//   uniform, 10 A     117 : 165  135 : 161  154 : 157  173 : 168
-//   chains, 12 A       85 : 210   89 : 184   93 : 229   98 : 211
-//   chains, 15 A, f64  93 : 198   99 : 498  105 : 993  116 : 1257
-// In a uniform cube the two meet at the limit; chains, which crowd few cells of their grid, would still gain up to the 1024 points that
-// a warp's row of bits can hold.
-constexpr int kMaskWordsPerRow = 24;
+// Larger batches whose structures have at most 1024 points on average: those that do go the same way (mask_rows_kernel), 1024 points
+// being what a warp's row of bits can hold; in a batch of large structures the bit rows (256 bytes per point) would be room for
+// nothing.  Lists and distances of 40 000 points in structures of one size, uniform, 10 A, us, bit rows : cells,
+//   points              800        900       1000
+//   float32           164 : 165  172 : 159  181 : 167
+//   float64           188 : 408  200 : 498  212 : 475
+//   ragged, 10.5 A    126 : 206 (float32), 139 : 438 (float64)
+// and chains, which crowd few cells of their grid, gain more than any of these.
+constexpr int kMaskWordsPerRow = 32;
 static inline bool mask_rows_route(int64_t N, int64_t B) { return N > kMaskNodes && N <= 32 * kMaskWordsPerRow * B; }
 
 struct GraphLayout {
@@ -2675,6 +2674,17 @@ rows_scan_kernel(const int32_t *__restrict__ deg, const int32_t *__restrict__ up
     }
 }
 
+// Distances of a list whose edges the cell kernels have written: those work through chains of dependent loads, and positions fetched in
+// them made 242 us of 172 (58 structures of up to 793 points in float64, 1.9 M edges); here 20.
+template <typename T, typename I>
+__global__ void __launch_bounds__(256)
+list_distance_kernel(const T *__restrict__ pos, const I *__restrict__ row0, const I *__restrict__ row1, int64_t E, T *__restrict__ distance) {
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t a = row0[e], b = row1[e];
+        distance[e] = sqrt(dist2_rn(pos[a * 3], pos[a * 3 + 1], pos[a * 3 + 2], pos[b * 3], pos[b * 3 + 1], pos[b * 3 + 2]));
+    }
+}
+
 // cellparam NULL: every structure has bit rows
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -3103,27 +3113,36 @@ int mlcgb_graph_finish(const void *pos, int dtype, const int64_t *ptr, int64_t N
     ex.ptr = ptr_exclude_pair_xs;
     auto st = (cudaStream_t)stream;
     char *w = (char *)workspace;
-    FillOut out{edge_index, edge_index ? edge_index + E : nullptr, mapping_batch, distance, row0, row1};
+    const FillOut everything{edge_index, edge_index ? edge_index + E : nullptr, mapping_batch, distance, row0, row1};
     return MLCGB_DISPATCH_DTYPE(dtype, [&] {
-        if (mask_route(N, B, ex)) return mask_fill_launch<scalar_t>(pos, ptr, N, B, w, L, offsets, out, twin, sel, pair_of, sticky_status, st);
+        if (mask_route(N, B, ex)) return mask_fill_launch<scalar_t>(pos, ptr, N, B, w, L, offsets, everything, twin, sel, pair_of, sticky_status, st);
         const bool rows = !ex.ptr && mask_rows_route(N, B), cells = !rows || with_cells;
         const WsLayout W = ws_layout(N, B, dtype);
         char *cw = w + L.cells;
         const auto *struct_of = (const int32_t *)(cw + W.struct_of);
         const auto *cellparam = (const CellParam *)(cw + W.cellparam);
         const auto *seg = (const int4 *)(w + L.seg);
+        FillOut out = everything;
+        if (cells) out.distance = nullptr;
+        auto distances = [&] {
+            if (!cells || !distance) return;
+            if (row0) list_distance_kernel<scalar_t, int32_t><<<grid_for(E, 256), 256, 0, st>>>((const scalar_t *)pos, row0, row1, E, (scalar_t *)distance);
+            else list_distance_kernel<scalar_t, int64_t><<<grid_for(E, 256), 256, 0, st>>>((const scalar_t *)pos, edge_index, edge_index + E, E, (scalar_t *)distance);
+        };
         if (cells) {
             const int rl = radius_launch<scalar_t>(false, true, pos, ptr, N, B, r, 0, loop, 0, cw, W.total, dtype, nullptr, const_cast<int64_t *>(offsets), out,
                                                    (int32_t *)(w + L.header), st, ex, rows ? kMaskMax : kBruteMax, rows ? 2 : 0);
             if (rl) return rl;
             if (twin && ((uintptr_t)row1 & 31) != 0) {
                 if (rows) return MLCGB_E_ARG;
+                distances();
                 return mlcgb_pair_plan(row0, row1, offsets, E, N, w + L.upper, L.seg - L.upper, twin, sel, pair_of, sticky_status, stream);
             }
         }
         if (rows)
             mask_rows_fill_kernel<scalar_t><<<grid_for(N * 32, 256), 256, 0, st>>>((const scalar_t *)pos, ptr, struct_of, cells ? cellparam : nullptr, N, (const uint2 *)(w + L.masks),
                                                                                  seg, offsets, out, twin, sel, pair_of);
+        distances();
         if (twin && cells) {
             // two structures of up to 4600 points fit an SM together; for larger ones a block takes the whole of it
             const bool walk = B >= kTransposeBatch;

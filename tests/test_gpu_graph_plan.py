@@ -100,13 +100,14 @@ def test_counts_read_by_several_threads():
 
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
-@pytest.mark.parametrize("sizes", [[3, 0, 5] * 400, [0] * 40 + [768] * 3 + [0] * 3, [1] * 2100, [2] * 1025, [767, 768, 768], [64, 31, 33] * 1100, [700] * 3 + [769], [1000, 600, 500, 1] ])
+@pytest.mark.parametrize("sizes", [[3, 0, 5] * 400, [0] * 40 + [768] * 3 + [0] * 3, [1] * 2100, [2] * 1025, [767, 768, 768], [64, 31, 33] * 1100, [700] * 3 + [769], [1000, 600, 500, 1],
+                                   [0] * 40 + [1024] * 3 + [0] * 3, [1023, 1024, 1024, 33], [900] * 3 + [1025]])
 def test_bit_rows_of_whole_batches(sizes, dtype):
     """Batches of structures that all fit a bit row are counted and scanned in three launches (structures found by a warp among 1, 32, 33 and
     more boundaries, parts of 32 points, blocks of 1024); one larger structure sends the batch the other way."""
     rng = np.random.default_rng(len(sizes) + sizes[0])
     ptr = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
-    assert 2048 < ptr[-1] <= 768 * len(sizes)
+    assert 2048 < ptr[-1] <= 1024 * len(sizes)
     pos = (rng.random((int(ptr[-1]), 3)) * max(sizes) ** (1 / 3) * 2.0).astype(dtype)
     be, t = get_backend(), torch.as_tensor(pos, device=DEV)
     want = radius_ref.radius_graph_c(pos, ptr, 4.0, 1000, False, "cluster")
