@@ -110,6 +110,19 @@ def test_dense_and_uneven_structures(dtype, loop):
         check_against_oracle(pos, ptr, r, 9, loop, "native")
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n,r,shape", [(1100, 12.0, (1, 1, 1)), (2500, 10.5, (1, 1, 1)), (4000, 12.0, (1, 1, 1)), (3000, 15.0, (1, 1, 1)), (3000, 21.0, (1, 1, 1)),
+                                       (3000, 12.0, (4, 0.5, 0.5)), (3000, 12.0, (0.2, 2.2, 2.2)), (3000, 12.0, (30, 0.01, 0.01))])
+def test_blocks_of_cells_about_a_stage_large(n, r, shape, dtype):
+    """Blocks are made smaller where their candidates would not fit a stage; from about 14 A on at this density even those of one cell
+    hold more."""
+    rng = np.random.default_rng(n)
+    ptr = np.array([0, n, n, 2 * n + 7], np.int64)
+    pos = (rng.random((2 * n + 7, 3)) * np.array(shape) * (n * 54.0) ** (1 / 3) - 7.0).astype(dtype)      # (54 cubic Angstrom a point)
+    for max_nn, loop in ((1000, False), (40, True)):
+        check_against_oracle(pos, ptr, r, max_nn, loop)
+
+
 def test_structure_larger_than_one_bitmask_window():
     rng = np.random.default_rng(1)
     sizes = [20000, 9000]
