@@ -9,6 +9,7 @@
 // hi*hi + hi*lo + lo*hi with fp32 accumulation in tensor memory, like the fused eval-mode kernels.
 // Rows of A (NT/NN) are scaled by a power of two so that their largest magnitude sits in [8,16);
 // TN scales each 128-edge tile of A and of B by one power of two and accumulates the tiles in registers.
+#include "schnet_internal.cuh"
 #include "tc_common.cuh"
 #include "tensor_map.cuh"
 #include "tn_jobs.cuh"
@@ -91,6 +92,14 @@ __device__ __forceinline__ void prefetch_tile_to_boxes(uint8_t *stage, const flo
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 __device__ __forceinline__ void wait_prefetch() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// a weight's image (schnet_internal.cuh) into its place in shared memory, by one thread that has just set up `bar`
+__device__ __forceinline__ void fetch_image(uint32_t dst, const uint8_t *image, uint32_t bar) {
+    tc::fence_async_smem();
+    tc::mbar_expect_bytes(bar, (uint32_t)kWeightImage);
+    tc::bulk_load(dst, image, 32768, bar);
+    tc::bulk_load(dst + 32768, image + 32768, 32768, bar);
+}
 
 // ------------------------------------------------------------------------------------------------ NT / NN
 template <int MODE>   // 0 NT, 1 NN
@@ -224,7 +233,8 @@ enum { kEpiNone = 0, kEpiTanh = 1, kEpiAdd = 2, kEpiTanhGrad = 3, kProTanhGradVe
 template <int MODE>   // 0 NT, 1 NN
 __global__ void __launch_bounds__(kGT, 1)
 gemm_tc_rows_pipe_kernel(const float *__restrict__ A, const float *__restrict__ B, const float *__restrict__ bias, int64_t E, int N, int K,
-                         const float *__restrict__ aux, int epi, const __grid_constant__ CUtensorMap cmap, int32_t *__restrict__ status) {
+                         const float *__restrict__ aux, int epi, const __grid_constant__ CUtensorMap cmap, const uint8_t *__restrict__ image,
+                         int32_t *__restrict__ status) {
     using namespace tc;
     using L = GemmTcSmem;
     extern __shared__ uint8_t smem_raw[];
@@ -234,8 +244,8 @@ gemm_tc_rows_pipe_kernel(const float *__restrict__ A, const float *__restrict__ 
     float *s_red = reinterpret_cast<float *>(smem + L::kMisc);
     float *s_bias = s_red + 512;
     float *s_vec = s_bias + 128;                                     // input-transform vector (EPI 4)
-    uint64_t *s_bar = reinterpret_cast<uint64_t *>(s_vec + 128);     // two barriers, one per accumulator
-    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(s_bar + 2);
+    uint64_t *s_bar = reinterpret_cast<uint64_t *>(s_vec + 128);     // two barriers, one per accumulator; the weight's
+    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(s_bar + 3);
     int *s_err = reinterpret_cast<int *>(s_tmem + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5;
@@ -245,7 +255,7 @@ gemm_tc_rows_pipe_kernel(const float *__restrict__ A, const float *__restrict__ 
     const int64_t step = gridDim.x, t0 = blockIdx.x;
     const int wrows = MODE == 0 ? N : K, wcols = MODE == 0 ? K : N;
     const int wpad = wcols <= 64 ? 64 : 128;
-    if (load_weight_tile<true>(sB_hi, sB_lo, B, wrows, wcols, wpad, kWS) && blockIdx.x == 0) atomicOr(status, (int)kWeightRange);
+    if (!image && load_weight_tile<true>(sB_hi, sB_lo, B, wrows, wcols, wpad, kWS) && blockIdx.x == 0) atomicOr(status, (int)kWeightRange);
     if (tid < 128) {
         s_bias[tid] = (bias && tid < N) ? bias[tid] : 0.f;
         s_vec[tid] = (epi == kProTanhGradVec && tid < K) ? aux[tid] : 0.f;      // (a parameter vector, not a result of the kernels before)
@@ -254,7 +264,9 @@ gemm_tc_rows_pipe_kernel(const float *__restrict__ A, const float *__restrict__ 
     if (tid == 0) {
         mbar_init(bar0, 1);
         mbar_init(bar0 + 8, 1);
+        mbar_init(bar0 + 16, 1);
         *s_err = 0;
+        if (image) fetch_image(smem_u32(sB_hi), image, bar0 + 16);
     }
     __syncwarp();
     if (warp == 0) tmem_alloc(smem_u32(s_tmem), 512);
@@ -271,6 +283,7 @@ gemm_tc_rows_pipe_kernel(const float *__restrict__ A, const float *__restrict__ 
     const int nmma = MODE == 0 ? 128 : wpad;
     const uint32_t b_hi = smem_u32(sB_hi), b_lo = smem_u32(sB_lo);
     uint32_t phase_bits = 0;          // bit b: parity the next wait on barrier b looks for
+    bool have_weight = !image;
 
     // the tile that has landed in the input stage: row scale, operand store, MMAs into accumulator `buf`; then the copy of
     // tile `following` (if any) into the stage.  Returns the row's scale.
@@ -299,6 +312,8 @@ gemm_tc_rows_pipe_kernel(const float *__restrict__ A, const float *__restrict__ 
         tc_fence_before();
         __syncthreads();
         if (warp == 0 && elect_one()) {
+            if (!have_weight && !mbar_wait(bar0 + 16, 0)) *s_err = 1;
+            have_weight = true;
             tc_fence_after();
             issue_gemm_ts<true>(tmem + buf * 128, ta, b_hi, b_lo, ksteps, MODE, nmma);
             mma_commit(bar0 + 8 * buf);
@@ -386,7 +401,7 @@ __global__ void __launch_bounds__(kGT, 1)
 gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa, const float *__restrict__ ba, const float *__restrict__ Wb,
                       const float *__restrict__ bb, const float *__restrict__ aux, int64_t E, float *__restrict__ mid_out,
                       float *__restrict__ C, int32_t *__restrict__ status, const float *__restrict__ ext0, const float *__restrict__ ext1,
-                      float *__restrict__ q_out) {
+                      float *__restrict__ q_out, const uint8_t *__restrict__ image_a, const uint8_t *__restrict__ image_b) {
     using namespace tc;
     using L = ChainSmem;
     constexpr bool BWD = KIND == kChainBwd || KIND == kChainRev;
@@ -399,15 +414,17 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
     float *s_red = reinterpret_cast<float *>(smem + L::kMisc);
     float *s_ba = s_red + 512, *s_bb = s_ba + 128;
     uint64_t *s_bar = reinterpret_cast<uint64_t *>(s_bb + 128);
-    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(s_bar + 1);
+    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(s_bar + 3);                // (barriers of the GEMMs, of Wa and of Wb)
     int *s_err = reinterpret_cast<int *>(s_tmem + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int r = tid & 127, qt = tid >> 7, col0 = qt * 32;
     constexpr float kWS = 64.f;
-    bool range = load_weight_tile<true>(sWa_hi, sWa_lo, Wa, W, W, W, kWS);
-    range = load_weight_tile<true>(sWb_hi, sWb_lo, Wb, W, W, W, kWS) || range;
-    if (range && blockIdx.x == 0) atomicOr(status, (int)kWeightRange);
+    if (!image_a) {
+        bool range = load_weight_tile<true>(sWa_hi, sWa_lo, Wa, W, W, W, kWS);
+        range = load_weight_tile<true>(sWb_hi, sWb_lo, Wb, W, W, W, kWS) || range;
+        if (range && blockIdx.x == 0) atomicOr(status, (int)kWeightRange);
+    }
     if (tid < 128) {
         s_ba[tid] = ba ? ba[tid] : 0.f;
         s_bb[tid] = bb ? bb[tid] : 0.f;
@@ -415,7 +432,13 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
     const uint32_t bar = smem_u32(s_bar);
     if (tid == 0) {
         mbar_init(bar, 1);
+        mbar_init(bar + 8, 1);
+        mbar_init(bar + 16, 1);
         *s_err = 0;
+        if (image_a) {
+            fetch_image(smem_u32(sWa_hi), image_a, bar + 8);
+            fetch_image(smem_u32(sWb_hi), image_b, bar + 16);
+        }
     }
     __syncwarp();
     if (warp == 0) tmem_alloc(smem_u32(s_tmem), 256);
@@ -449,8 +472,11 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
         __syncthreads();
         return sc;
     };
+    int arrived = image_a ? 0 : 2;                  // weight images that have
     auto gemm = [&](uint8_t *w_hi, uint8_t *w_lo) {
         if (warp == 0 && elect_one()) {
+            if (arrived < 2 && !mbar_wait(bar + 8 + 8 * arrived, 0)) *s_err = 1;
+            arrived++;
             tc_fence_after();
             issue_gemm_ts<true>(tmem, ta, smem_u32(w_hi), smem_u32(w_lo), W / 16, MODE, W);
             mma_commit(bar);
@@ -1008,7 +1034,7 @@ static int set_smem(Kern kern, bool *done) {
 
 // Pipelined row-wise kernel; MLCGB_E_LIMIT when its conditions on shape and alignment do not hold.
 static int rows_pipe_launch(int mode, const void *A, const void *B, const void *bias, const void *aux, int epi, int64_t M, int64_t N, int64_t K,
-                            void *C, int32_t *status, cudaStream_t st) {
+                            void *C, const uint8_t *image, int32_t *status, cudaStream_t st) {
     CUtensorMap cmap;
     if ((K & 3) != 0 || ((uintptr_t)A & 15) != 0 || (aux && epi != kProTanhGradVec && ((uintptr_t)aux & 15) != 0) || !make_rows_map(&cmap, (float *)C, M, N))
         return MLCGB_E_LIMIT;
@@ -1018,18 +1044,18 @@ static int rows_pipe_launch(int mode, const void *A, const void *B, const void *
     if (mode == 0) {
         if (int rc = set_smem(gemm_tc_rows_pipe_kernel<0>, p0)) return rc;
         launch_with_weights(gemm_tc_rows_pipe_kernel<0>, dim3(grid), dim3(kGT), GemmTcSmem::kTotal, st, (const float *)A, (const float *)B, (const float *)bias, M,
-                   (int)N, (int)K, (const float *)aux, epi, cmap, status);
+                   (int)N, (int)K, (const float *)aux, epi, cmap, image, status);
     } else {
         if (int rc = set_smem(gemm_tc_rows_pipe_kernel<1>, p1)) return rc;
         launch_with_weights(gemm_tc_rows_pipe_kernel<1>, dim3(grid), dim3(kGT), GemmTcSmem::kTotal, st, (const float *)A, (const float *)B, (const float *)bias, M,
-                   (int)N, (int)K, (const float *)aux, epi, cmap, status);
+                   (int)N, (int)K, (const float *)aux, epi, cmap, image, status);
     }
     return check_launch();
 }
 
 template <int KIND>
 static int chain2_launch(const void *A, const void *Wa, const void *ba, const void *Wb, const void *bb, const void *aux, int64_t M, void *mid_out,
-                         void *C, const void *ext0, const void *ext1, void *q_out, int32_t *status, cudaStream_t st) {
+                         void *C, const void *ext0, const void *ext1, void *q_out, const uint8_t *image_a, const uint8_t *image_b, int32_t *status, cudaStream_t st) {
     const int64_t ntiles = (M + tc::kRows - 1) / tc::kRows;
     const int grid = (int)(ntiles < kNumSM ? ntiles : kNumSM);
     static bool done[64] = {false};
@@ -1042,8 +1068,43 @@ static int chain2_launch(const void *A, const void *Wa, const void *ba, const vo
     }
     launch_with_weights(gemm_tc_chain2_kernel<KIND>, dim3(grid), dim3(kGT), ChainSmem::kTotal, st, (const float *)A, (const float *)Wa, (const float *)ba,
                (const float *)Wb, (const float *)bb, (const float *)aux, M, (float *)mid_out, (float *)C, status, (const float *)ext0,
-               (const float *)ext1, (float *)q_out);
+               (const float *)ext1, (float *)q_out, image_a, image_b);
     return check_launch();
+}
+
+int gemm_fused(int mode, const void *A, const void *B, const void *bias, const void *aux, int epilogue, int64_t M, int64_t N, int64_t K, void *C,
+               const uint8_t *image, int32_t *status, void *stream) {
+    TimelineScope timeline_scope("gemm_tc_fused", stream);
+    if ((mode != 0 && mode != 1) || epilogue < 0 || epilogue > 4 || !status) return MLCGB_E_ARG;
+    if ((epilogue == kEpiAdd || epilogue == kEpiTanhGrad || epilogue == kProTanhGradVec) && !aux) return MLCGB_E_ARG;
+    if (!mlcgb_gemm_tc_supported(mode, M, N, K)) return MLCGB_E_LIMIT;
+    if (M == 0) return MLCGB_OK;
+    if (!A || !B || !C) return MLCGB_E_ARG;
+    return rows_pipe_launch(mode, A, B, bias, aux, epilogue, M, N, K, C, image, status, (cudaStream_t)stream);
+}
+
+int gemm_chain2(int backward, const void *A, const void *Wa, const void *ba, const void *Wb, const void *bb, const void *aux, int64_t M, void *mid_out,
+                void *C, const uint8_t *image_a, const uint8_t *image_b, int32_t *status, void *stream) {
+    TimelineScope timeline_scope("gemm_tc_chain2", stream);
+    if (M < 0 || !status) return MLCGB_E_ARG;
+    if (M == 0) return MLCGB_OK;
+    if (!A || !Wa || !Wb || !aux || !C || (!backward && !mid_out)) return MLCGB_E_ARG;
+    if ((((uintptr_t)A | (uintptr_t)aux | (uintptr_t)C | (uintptr_t)mid_out) & 15) != 0) return MLCGB_E_LIMIT;
+    const auto st = (cudaStream_t)stream;
+    return backward ? chain2_launch<kChainBwd>(A, Wa, ba, Wb, bb, aux, M, mid_out, C, nullptr, nullptr, nullptr, image_a, image_b, status, st)
+                    : chain2_launch<kChainFwd>(A, Wa, ba, Wb, bb, aux, M, mid_out, C, nullptr, nullptr, nullptr, image_a, image_b, status, st);
+}
+
+int gemm_chain2_tangent(int reverse, const void *A, const void *Wa, const void *Wb, const void *a, const void *gu, const void *aux, int64_t M, void *q,
+                        void *mid_out, void *C, const uint8_t *image_a, const uint8_t *image_b, int32_t *status, void *stream) {
+    TimelineScope timeline_scope("gemm_tc_chain2_tangent", stream);
+    if (M < 0 || !status) return MLCGB_E_ARG;
+    if (M == 0) return MLCGB_OK;
+    if (!A || !Wa || !Wb || !a || !q || !mid_out || !C || (!reverse && !gu)) return MLCGB_E_ARG;
+    if ((((uintptr_t)A | (uintptr_t)a | (uintptr_t)gu | (uintptr_t)aux | (uintptr_t)q | (uintptr_t)mid_out | (uintptr_t)C) & 15) != 0) return MLCGB_E_LIMIT;
+    const auto st = (cudaStream_t)stream;
+    if (reverse) return chain2_launch<kChainRev>(A, Wa, nullptr, Wb, nullptr, a, M, mid_out, C, q, nullptr, nullptr, image_a, image_b, status, st);
+    return chain2_launch<kChainTan>(A, Wa, nullptr, Wb, nullptr, aux, M, mid_out, C, a, gu, q, image_a, image_b, status, st);
 }
 
 }  // namespace mlcgb
@@ -1054,37 +1115,17 @@ extern "C" {
 
 int mlcgb_gemm_tc_fused(int mode, const void *A, const void *B, const void *bias, const void *aux, int epilogue, int64_t M, int64_t N,
                         int64_t K, void *C, int32_t *status, void *stream) {
-    TimelineScope timeline_scope("gemm_tc_fused", stream);
-    if ((mode != 0 && mode != 1) || epilogue < 0 || epilogue > 4 || !status) return MLCGB_E_ARG;
-    if ((epilogue == kEpiAdd || epilogue == kEpiTanhGrad || epilogue == kProTanhGradVec) && !aux) return MLCGB_E_ARG;
-    if (!mlcgb_gemm_tc_supported(mode, M, N, K)) return MLCGB_E_LIMIT;
-    if (M == 0) return MLCGB_OK;
-    if (!A || !B || !C) return MLCGB_E_ARG;
-    return rows_pipe_launch(mode, A, B, bias, aux, epilogue, M, N, K, C, status, (cudaStream_t)stream);
+    return gemm_fused(mode, A, B, bias, aux, epilogue, M, N, K, C, nullptr, status, stream);
 }
-
 
 int mlcgb_gemm_tc_chain2(int backward, const void *A, const void *Wa, const void *ba, const void *Wb, const void *bb, const void *aux,
                          int64_t M, void *mid_out, void *C, int32_t *status, void *stream) {
-    TimelineScope timeline_scope("gemm_tc_chain2", stream);
-    if (M < 0 || !status) return MLCGB_E_ARG;
-    if (M == 0) return MLCGB_OK;
-    if (!A || !Wa || !Wb || !aux || !C || (!backward && !mid_out)) return MLCGB_E_ARG;
-    if ((((uintptr_t)A | (uintptr_t)aux | (uintptr_t)C | (uintptr_t)mid_out) & 15) != 0) return MLCGB_E_LIMIT;
-    const auto kind = backward ? kChainBwd : kChainFwd;
-    return kind == kChainBwd ? chain2_launch<kChainBwd>(A, Wa, ba, Wb, bb, aux, M, mid_out, C, nullptr, nullptr, nullptr, status, (cudaStream_t)stream)
-                             : chain2_launch<kChainFwd>(A, Wa, ba, Wb, bb, aux, M, mid_out, C, nullptr, nullptr, nullptr, status, (cudaStream_t)stream);
+    return gemm_chain2(backward, A, Wa, ba, Wb, bb, aux, M, mid_out, C, nullptr, nullptr, status, stream);
 }
 
 int mlcgb_gemm_tc_chain2_tangent(int reverse, const void *A, const void *Wa, const void *Wb, const void *a, const void *gu, const void *aux,
                                  int64_t M, void *q, void *mid_out, void *C, int32_t *status, void *stream) {
-    TimelineScope timeline_scope("gemm_tc_chain2_tangent", stream);
-    if (M < 0 || !status) return MLCGB_E_ARG;
-    if (M == 0) return MLCGB_OK;
-    if (!A || !Wa || !Wb || !a || !q || !mid_out || !C || (!reverse && !gu)) return MLCGB_E_ARG;
-    if ((((uintptr_t)A | (uintptr_t)a | (uintptr_t)gu | (uintptr_t)aux | (uintptr_t)q | (uintptr_t)mid_out | (uintptr_t)C) & 15) != 0) return MLCGB_E_LIMIT;
-    if (reverse) return chain2_launch<kChainRev>(A, Wa, nullptr, Wb, nullptr, a, M, mid_out, C, q, nullptr, nullptr, status, (cudaStream_t)stream);
-    return chain2_launch<kChainTan>(A, Wa, nullptr, Wb, nullptr, aux, M, mid_out, C, a, gu, q, status, (cudaStream_t)stream);
+    return gemm_chain2_tangent(reverse, A, Wa, Wb, a, gu, aux, M, q, mid_out, C, nullptr, nullptr, status, stream);
 }
 
 int mlcgb_gemm_tc_tn_colsum(const void *A, const void *B, int64_t K, int64_t M, int64_t N, void *C, void *colsum, void *workspace,
@@ -1124,7 +1165,7 @@ int mlcgb_gemm_tc(int mode, const void *A, const void *B, const void *bias, int6
     if (mode == 0 || mode == 1) {
         const int64_t ntiles = (M + tc::kRows - 1) / tc::kRows;
         const int grid = (int)(ntiles < kNumSM ? ntiles : kNumSM);
-        const int rc = rows_pipe_launch(mode, A, B, bias, nullptr, kEpiNone, M, N, K, C, status, st);
+        const int rc = rows_pipe_launch(mode, A, B, bias, nullptr, kEpiNone, M, N, K, C, nullptr, status, st);
         if (rc != MLCGB_E_LIMIT) return rc;            // else: shapes or alignment the pipelined kernel does not take
         if (mode == 0) {
             if (int rc = set_smem(gemm_tc_rows_kernel<0>, c0)) return rc;

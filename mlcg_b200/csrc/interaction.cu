@@ -5,6 +5,7 @@
 // row per unordered pair); everything else goes through the individual entry points.
 #include "common.cuh"
 #include "schnet_internal.cuh"
+#include "tc_common.cuh"
 
 using namespace mlcgb;
 
@@ -119,11 +120,28 @@ static int interaction_backward_counted(const void *g, const void *a, const void
 // ------------------------------------------------------------------------------------------------
 namespace mlcgb {
 
-__global__ void embedding_rows_kernel(const float *__restrict__ table, const int64_t *__restrict__ types, int64_t N, int64_t H, int64_t T,
-                                      float *__restrict__ x, int32_t *__restrict__ status) {
-    const int64_t Hv = H >> 2, total = N * Hv;
+// Rows of the embedding table, and in front of them eight blocks per weight image, 16 of its rows each
+__global__ void __launch_bounds__(256)
+embedding_rows_kernel(const float *__restrict__ table, const int64_t *__restrict__ types, int64_t N, int64_t H, int64_t T, float *__restrict__ x,
+                      const __grid_constant__ WeightImages im, int32_t *__restrict__ status) {
     pdl_wait();
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+    if ((int)blockIdx.x < 8 * im.n) {
+        const int k = blockIdx.x >> 3;
+        uint8_t *hi = im.dst + k * kWeightImage;
+        float most = 0.f;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int row = (blockIdx.x & 7) * 16 + u * 8 + (threadIdx.x >> 5), col = (threadIdx.x & 31) * 4;
+            const float *src = im.src[k] + row * 128 + col;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row < im.rows[k]) v = ((uintptr_t)src & 15) == 0 ? *reinterpret_cast<const float4 *>(src) : make_float4(src[0], src[1], src[2], src[3]);
+            most = fmaxf(most, tc::put_weight4<true>(hi, hi + kWeightImage / 2, row, col, v, 64.f));
+        }
+        if (!(most * 64.f <= 32768.f)) atomicOr(status, (int)kWeightRange);
+        return;
+    }
+    const int64_t Hv = H >> 2, total = N * Hv, first = blockIdx.x - 8 * im.n, blocks = gridDim.x - 8 * im.n;
+    for (int64_t t = first * blockDim.x + threadIdx.x; t < total; t += blocks * blockDim.x) {
         const int64_t n = t / Hv, c = t - n * Hv;
         int64_t ty = types[n];
         if (ty < 0 || ty >= T) {
@@ -132,6 +150,25 @@ __global__ void embedding_rows_kernel(const float *__restrict__ table, const int
         }
         reinterpret_cast<float4 *>(x)[t] = __ldg(reinterpret_cast<const float4 *>(table + ty * H) + c);
     }
+}
+
+int embedding_launch(const mlcgb_schnet_weights *w, const int64_t *types, int64_t N, float *x, void *images, int32_t *status, cudaStream_t st) {
+    TimelineScope timeline_scope("embedding", st);
+    WeightImages im;
+    im.n = 0;
+    im.dst = (uint8_t *)images;
+    auto add = [&](const void *src, int64_t rows) { im.src[im.n] = (const float *)src; im.rows[im.n++] = (int)rows; };
+    if (images) {
+        for (int64_t l = 0; l < w->num_blocks; l++) {
+            add(w->blocks[l].lin1_w, 128);
+            add(w->blocks[l].lin2_w, 128);
+            add(w->blocks[l].lin_w, 128);
+        }
+        add(w->head_W, w->head_width);
+    }
+    launch_pdl(embedding_rows_kernel, dim3(8 * im.n + grid_for(N * (w->hidden >> 2), 256)), dim3(256), 0, st, (const float *)w->embedding, types, N, w->hidden,
+               w->num_types, x, im, status);
+    return check_launch();
 }
 
 // e[n] = sum_f a[n,f] w[f] + b: the last Linear layer of the output network (one output); one warp per node
@@ -150,16 +187,19 @@ __global__ void head_out_kernel(const float *__restrict__ a, const float *__rest
 
 // tanh(agg W2^T + b2) -> a,  x + a W3^T + b3 -> out; one kernel where all widths are 128
 static int node_layers_forward(const float *agg, const mlcgb_schnet_block &w, const float *x, int64_t N, int64_t H, int64_t F, int64_t H2, float *a,
-                               float *out, int32_t *status, void *stream) {
-    if (H == 128 && F == 128 && H2 == 128) return mlcgb_gemm_tc_chain2(0, agg, w.lin2_w, w.lin2_b, w.lin_w, w.lin_b, x, N, a, out, status, stream);
+                               float *out, const uint8_t *images, int32_t *status, void *stream) {
+    if (H == 128 && F == 128 && H2 == 128)
+        return gemm_chain2(0, agg, w.lin2_w, w.lin2_b, w.lin_w, w.lin_b, x, N, a, out, images ? images + kLin2 * kWeightImage : nullptr,
+                           images ? images + kLin * kWeightImage : nullptr, status, stream);
     int rc = mlcgb_gemm_tc_fused(0, agg, w.lin2_w, w.lin2_b, nullptr, 1, N, H2, F, a, status, stream);
     return rc ? rc : mlcgb_gemm_tc_fused(0, a, w.lin_w, w.lin_b, x, 2, N, H, H2, out, status, stream);
 }
 // ((g W3) (1 - a^2)) W2 -> gagg
 static int node_layers_backward(const float *g, const mlcgb_schnet_block &w, const float *a, int64_t N, int64_t H, int64_t F, int64_t H2, float *gy,
-                                float *gagg, int32_t *status, void *stream) {
+                                float *gagg, const uint8_t *images, int32_t *status, void *stream) {
     if (H == 128 && F == 128 && H2 == 128)
-        return mlcgb_gemm_tc_chain2(1, g, w.lin_w, nullptr, w.lin2_w, nullptr, a, N, nullptr, gagg, status, stream);
+        return gemm_chain2(1, g, w.lin_w, nullptr, w.lin2_w, nullptr, a, N, nullptr, gagg, images ? images + kLin * kWeightImage : nullptr,
+                           images ? images + kLin2 * kWeightImage : nullptr, status, stream);
     int rc = mlcgb_gemm_tc_fused(1, g, w.lin_w, nullptr, a, 3, N, H2, H, gy, status, stream);
     return rc ? rc : mlcgb_gemm_tc_fused(1, gy, w.lin2_w, nullptr, nullptr, 0, N, F, H2, gagg, status, stream);
 }
@@ -169,7 +209,7 @@ static int node_layers_backward(const float *g, const mlcgb_schnet_block &w, con
 static inline int64_t up64(int64_t n) { return (n + 63) & ~(int64_t)63; }
 
 struct SchnetLayout {                                                        // offsets in floats
-    int64_t d, x[2], g[2], agg, gy, gxl, ah, en, gd, gp, W, Wd, wstride, block0, block_stride, xl_off, a_off, total;
+    int64_t d, x[2], g[2], agg, gy, gxl, ah, en, gd, gp, images, W, Wd, wstride, block0, block_stride, xl_off, a_off, total;   // images -1: none
 };
 static SchnetLayout schnet_layout(int64_t N, int64_t E, int64_t P, int64_t H, int64_t F, int64_t H2, int64_t Wh, int64_t L) {
     SchnetLayout o;
@@ -181,6 +221,7 @@ static SchnetLayout schnet_layout(int64_t N, int64_t E, int64_t P, int64_t H, in
     o.agg = take(N * F); o.gy = take(N * H2); o.gxl = take(N * F);
     o.ah = take(N * Wh); o.en = take(N);
     o.gd = take(E); o.gp = take(P);
+    o.images = N > kSmallNodes && H == 128 && F == 128 && H2 == 128 && L <= kMaxBlocks ? take(weight_images_floats(L)) : -1;
     o.wstride = padded_rows(P) * F;
     o.W = take(L * o.wstride); o.Wd = take(L * o.wstride);                   // filter rows of all blocks, and their distance derivatives
     o.xl_off = 0; o.a_off = up64(N * F);
@@ -264,27 +305,27 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
         return small_finish(f, twin, struct_ptr, (float *)energy, (float *)grad_pos, grad_sign, st);
     }
     if (!have_distances && (rc = mlcgb_edge_distance(pos, MLCGB_F32, row0, row1, E, N, d, status, stream))) return rc;
-    {
-        TimelineScope timeline_scope("embedding", stream);
-        launch_pdl(embedding_rows_kernel, dim3(grid_for(N * (H >> 2), 256)), dim3(256), 0, st, (const float *)w->embedding, types, N, H, w->num_types, ws + lay.x[0], status);
-    }
+    // (the kernel behind the one that makes them converts its weight itself: it reads it before it waits for that one)
+    const uint8_t *images = lay.images >= 0 && ((uintptr_t)ws & 15) == 0 ? (const uint8_t *)(ws + lay.images) : nullptr;
+    auto image = [&](int64_t k) { return images ? images + k * kWeightImage : nullptr; };
+    if ((rc = embedding_launch(w, types, N, ws + lay.x[0], (void *)images, status, st))) return rc;
     ChainScope chain;
     int cur = 0;
     for (int64_t l = 0; l < L; l++) {
         const mlcgb_schnet_block &bw = w->blocks[l];
         float *blk = ws + lay.block0 + l * lay.block_stride;
         float *xin = ws + lay.x[cur], *xout = ws + lay.x[cur ^ 1], *xl = blk + lay.xl_off, *a = blk + lay.a_off, *agg = ws + lay.agg;
-        rc = mlcgb_gemm_tc_fused(0, xin, bw.lin1_w, nullptr, nullptr, 0, N, F, H, xl, status, stream);
+        rc = gemm_fused(0, xin, bw.lin1_w, nullptr, nullptr, 0, N, F, H, xl, l > 0 ? image(3 * l + kLin1) : nullptr, status, stream);
         if (rc) return rc;
         if ((rc = filters(l, 1))) return rc;        // (block by block: what is written last is read first, some of it out of the L2)
         rc = mlcgb_seg_mul_sum(xl, ws + lay.W + l * lay.wstride, MLCGB_F32, offsets, row1, pair_of, N, P, F, agg, stream);
         if (rc) return rc;
-        rc = node_layers_forward(agg, bw, xin, N, H, F, H2, a, xout, status, stream);
+        rc = node_layers_forward(agg, bw, xin, N, H, F, H2, a, xout, image(3 * l), status, stream);
         if (rc) return rc;
         cur ^= 1;
     }
     // output network: tanh(x W^T + b) . w_out (+ b_out), summed per structure
-    rc = mlcgb_gemm_tc_fused(0, ws + lay.x[cur], w->head_W, w->head_b, nullptr, 1, N, Wh, H, ws + lay.ah, status, stream);
+    rc = gemm_fused(0, ws + lay.x[cur], w->head_W, w->head_b, nullptr, 1, N, Wh, H, ws + lay.ah, image(3 * L), status, stream);
     if (rc) return rc;
     {
         TimelineScope timeline_scope("head_out", stream);
@@ -295,13 +336,13 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
     // force pass: d(sum of energies)/d(pos)
     // through the output network: g = (w_out * (1 - a^2)) head_W, the factor applied as the GEMM reads its input tile
     int gcur = 0;
-    rc = mlcgb_gemm_tc_fused(1, ws + lay.ah, w->head_W, nullptr, w->head_out, 4, N, H, Wh, ws + lay.g[gcur], status, stream);
+    rc = gemm_fused(1, ws + lay.ah, w->head_W, nullptr, w->head_out, 4, N, H, Wh, ws + lay.g[gcur], image(3 * L), status, stream);
     if (rc) return rc;
     for (int64_t l = L - 1; l >= 0; l--) {
         const mlcgb_schnet_block &bw = w->blocks[l];
         float *blk = ws + lay.block0 + l * lay.block_stride;
         float *g = ws + lay.g[gcur], *gnext = ws + lay.g[gcur ^ 1], *gagg = ws + lay.agg, *gxl = ws + lay.gxl;
-        rc = node_layers_backward(g, bw, blk + lay.a_off, N, H, F, H2, ws + lay.gy, gagg, status, stream);
+        rc = node_layers_backward(g, bw, blk + lay.a_off, N, H, F, H2, ws + lay.gy, gagg, image(3 * l), status, stream);
         if (rc) return rc;
         // s[e] of every block adds up in one array: the last block sets it, the others add
         if (l == 0) {
@@ -311,7 +352,7 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
         rc = mlcgb_seg_force(gagg, blk + lay.xl_off, ws + lay.W + l * lay.wstride, ws + lay.Wd + l * lay.wstride, offsets, row1, pair_of, N, F, gxl, ws + lay.gd,
                              l != L - 1, stream);
         if (rc) return rc;
-        if ((rc = mlcgb_gemm_tc_fused(1, gxl, bw.lin1_w, nullptr, g, 2, N, H, F, gnext, status, stream))) return rc;
+        if ((rc = gemm_fused(1, gxl, bw.lin1_w, nullptr, g, 2, N, H, F, gnext, image(3 * l + kLin1), status, stream))) return rc;
         gcur ^= 1;
     }
     return finish_launch((const float *)pos, ws + lay.gp, d, row1, offsets, pair_of, N, (float *)grad_pos, grad_sign, ws + lay.en, struct_ptr, B, (float *)energy, st);

@@ -73,6 +73,16 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar_saddr) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_saddr) : "memory");
 }
 
+// `bytes` (a multiple of 16, both addresses 16-byte aligned) from global to shared memory; completes on the barrier, which expects them
+__device__ __forceinline__ void mbar_expect_bytes(uint32_t bar_saddr, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_saddr), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst_saddr, const void *src, uint32_t bytes, uint32_t bar_saddr) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_saddr),
+                 "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(bar_saddr)
+                 : "memory");
+}
+
 // Waits for the phase with the given parity; gives up after kSpinLimit polls and returns false.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar_saddr, uint32_t parity) {
     for (uint32_t it = 0; it < kSpinLimit; ++it) {
@@ -165,6 +175,22 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) 
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// Four consecutive elements of a weight's row n, scaled, into the tile (and its low part); returns the largest unscaled magnitude
+template <bool SPLIT>
+__device__ __forceinline__ float put_weight4(uint8_t *hi, uint8_t *lo, int n, int k, float4 w, float scale) {
+    const uint32_t off = elem_offset(n, k);
+    if (SPLIT) {
+        const __half2 a0 = __floats2half2_rn(w.x * scale, w.y * scale), a1 = __floats2half2_rn(w.z * scale, w.w * scale);
+        const float2 f0 = __half22float2(a0), f1 = __half22float2(a1);
+        const __half2 c0 = __floats2half2_rn(w.x * scale - f0.x, w.y * scale - f0.y), c1 = __floats2half2_rn(w.z * scale - f1.x, w.w * scale - f1.y);
+        *reinterpret_cast<uint2 *>(hi + off) = make_uint2(*reinterpret_cast<const uint32_t *>(&a0), *reinterpret_cast<const uint32_t *>(&a1));
+        *reinterpret_cast<uint2 *>(lo + off) = make_uint2(*reinterpret_cast<const uint32_t *>(&c0), *reinterpret_cast<const uint32_t *>(&c1));
+    } else {
+        const __nv_bfloat162 a0 = __floats2bfloat162_rn(w.x * scale, w.y * scale), a1 = __floats2bfloat162_rn(w.z * scale, w.w * scale);
+        *reinterpret_cast<uint2 *>(hi + off) = make_uint2(*reinterpret_cast<const uint32_t *>(&a0), *reinterpret_cast<const uint32_t *>(&a1));
+    }
+    return fmaxf(fmaxf(fabsf(w.x), fabsf(w.y)), fmaxf(fabsf(w.z), fabsf(w.w)));
+}
 // Fill a [128][Kpad] weight tile (and its low part) from a row-major fp32 matrix src[rows][K], scaled by `scale`.
 // Four consecutive K elements of a row are 8 contiguous bytes of the swizzled tile, so with K % 4 == 0 and a 16-byte
 // aligned source every thread moves float4 -> 8 bytes, with all its loads issued before the first conversion.
@@ -174,20 +200,7 @@ template <bool SPLIT>
 __device__ __forceinline__ bool load_weight_tile(uint8_t *hi, uint8_t *lo, const float *__restrict__ src, int rows, int K, int Kpad,
                                                  float scale) {
     float wmax = 0.f;
-    auto put4 = [&](int n, int k, float4 w) {
-        wmax = fmaxf(fmaxf(wmax, fmaxf(fabsf(w.x), fabsf(w.y))), fmaxf(fabsf(w.z), fabsf(w.w)));
-        const uint32_t off = elem_offset(n, k);
-        if (SPLIT) {
-            const __half2 a0 = __floats2half2_rn(w.x * scale, w.y * scale), a1 = __floats2half2_rn(w.z * scale, w.w * scale);
-            const float2 f0 = __half22float2(a0), f1 = __half22float2(a1);
-            const __half2 c0 = __floats2half2_rn(w.x * scale - f0.x, w.y * scale - f0.y), c1 = __floats2half2_rn(w.z * scale - f1.x, w.w * scale - f1.y);
-            *reinterpret_cast<uint2 *>(hi + off) = make_uint2(*reinterpret_cast<const uint32_t *>(&a0), *reinterpret_cast<const uint32_t *>(&a1));
-            *reinterpret_cast<uint2 *>(lo + off) = make_uint2(*reinterpret_cast<const uint32_t *>(&c0), *reinterpret_cast<const uint32_t *>(&c1));
-        } else {
-            const __nv_bfloat162 a0 = __floats2bfloat162_rn(w.x * scale, w.y * scale), a1 = __floats2bfloat162_rn(w.z * scale, w.w * scale);
-            *reinterpret_cast<uint2 *>(hi + off) = make_uint2(*reinterpret_cast<const uint32_t *>(&a0), *reinterpret_cast<const uint32_t *>(&a1));
-        }
-    };
+    auto put4 = [&](int n, int k, float4 w) { wmax = fmaxf(wmax, put_weight4<SPLIT>(hi, lo, n, k, w, scale)); };
     const int qpr = Kpad >> 2, nquads = kRows * qpr;          // quads per row, quads in the tile
     if ((K & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
         constexpr int kBatch = 8;

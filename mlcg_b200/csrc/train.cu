@@ -14,7 +14,6 @@
 
 namespace mlcgb {
 
-__global__ void embedding_rows_kernel(const float *table, const int64_t *types, int64_t N, int64_t H, int64_t T, float *x, int32_t *status);
 __global__ void head_out_kernel(const float *a, const float *w, const float *b, int64_t N, int64_t F, float *e);
 
 // Output network e = wo . tanh(y), its tangent along yt, and gE (per structure, NULL: zero); one warp per node:
@@ -88,7 +87,7 @@ train_begin_kernel(const float *__restrict__ pos, int64_t n, float *__restrict__
 constexpr int64_t kH = 128;
 
 struct TrainForward {                                 // offsets in floats
-    int64_t pos, d, gd, gp, en, ah, zmax, W, Wd, Hs, Zs, wstride, hstride, block0, stride, total;      // W .. Zs: of all blocks
+    int64_t pos, d, gd, gp, en, ah, zmax, images, W, Wd, Hs, Zs, wstride, hstride, block0, stride, total;      // W .. Zs: of all blocks
     int64_t x, xl, agg, a, gu, gagg, gxl, g;          // of a block; g: the gradient of the block's output
 };
 struct TrainBackward {
@@ -105,6 +104,7 @@ static TrainForward train_forward_layout(int64_t N, int64_t E, int64_t P, int64_
     const int64_t hidden = (int64_t)(mlcgb_filter_hidden_bytes(P) / sizeof(float));
     o.pos = take(3 * N);
     o.d = take(E); o.gd = take(E); o.gp = take(P); o.en = take(N); o.ah = take(N * Wh); o.zmax = take(L);
+    o.images = N > kSmallNodes ? take(weight_images_floats(L)) : -1;
     o.wstride = padded_rows(P) * kH;
     o.hstride = hidden;
     o.W = take(L * o.wstride); o.Wd = take(L * o.wstride); o.Hs = take(L * hidden); o.Zs = take(L * hidden);
@@ -212,32 +212,30 @@ int mlcgb::schnet_train_forward(const void *pos, const int64_t *types, const int
     }
     int rc = have_distances ? MLCGB_OK : mlcgb_edge_distance(pos, MLCGB_F32, row0, row1, E, N, d, status, stream);
     if (rc) return rc;
-    {
-        TimelineScope timeline_scope("embedding", stream);
-        launch_pdl(embedding_rows_kernel, dim3(grid_for(N * (kH >> 2), 256)), dim3(256), 0, st, (const float *)w->embedding, types, N, kH, w->num_types,
-                   blk(0) + o.x, status);
-    }
+    const uint8_t *images = ((uintptr_t)ws & 15) == 0 ? (const uint8_t *)(ws + o.images) : nullptr;
+    auto image = [&](int64_t k) { return images ? images + k * kWeightImage : nullptr; };
+    if ((rc = embedding_launch(w, types, N, blk(0) + o.x, (void *)images, status, st))) return rc;
     for (int64_t l = 0; l < L; l++) {
         const mlcgb_schnet_block &bw = w->blocks[l];
         float *b = blk(l), *xout = l + 1 < L ? blk(l + 1) + o.x : ws + o.block0 + L * o.stride;
-        if ((rc = mlcgb_gemm_tc_fused(0, b + o.x, bw.lin1_w, nullptr, nullptr, 0, N, kH, kH, b + o.xl, status, stream))) return rc;
+        if ((rc = gemm_fused(0, b + o.x, bw.lin1_w, nullptr, nullptr, 0, N, kH, kH, b + o.xl, l > 0 ? image(3 * l + kLin1) : nullptr, status, stream))) return rc;
         if ((rc = filters(l, 1))) return rc;
         if ((rc = mlcgb_seg_mul_sum(b + o.xl, ws + o.W + l * o.wstride, MLCGB_F32, offsets, row1, pair_of, N, P, kH, b + o.agg, stream))) return rc;
-        if ((rc = mlcgb_gemm_tc_chain2(0, b + o.agg, bw.lin2_w, bw.lin2_b, bw.lin_w, bw.lin_b, b + o.x, N, b + o.a, xout, status, stream))) return rc;
+        if ((rc = gemm_chain2(0, b + o.agg, bw.lin2_w, bw.lin2_b, bw.lin_w, bw.lin_b, b + o.x, N, b + o.a, xout, image(3 * l + kLin2), image(3 * l + kLin), status, stream))) return rc;
     }
     float *xL = ws + o.block0 + L * o.stride, *ah = ws + o.ah;
-    if ((rc = mlcgb_gemm_tc_fused(0, xL, w->head_W, w->head_b, nullptr, 1, N, Wh, kH, ah, status, stream))) return rc;
+    if ((rc = gemm_fused(0, xL, w->head_W, w->head_b, nullptr, 1, N, Wh, kH, ah, image(3 * L), status, stream))) return rc;
     {
         TimelineScope timeline_scope("head_out", stream);
         launch_pdl(head_out_kernel, dim3(grid_for(N * 32, 256)), dim3(256), 0, st, (const float *)ah, (const float *)w->head_out, (const float *)w->head_out_b, N,
                    Wh, ws + o.en);
     }
     // force pass; block l's g is the gradient of its output
-    if ((rc = mlcgb_gemm_tc_fused(1, ah, w->head_W, nullptr, w->head_out, 4, N, kH, Wh, blk(L - 1) + o.g, status, stream))) return rc;
+    if ((rc = gemm_fused(1, ah, w->head_W, nullptr, w->head_out, 4, N, kH, Wh, blk(L - 1) + o.g, image(3 * L), status, stream))) return rc;
     for (int64_t l = L - 1; l >= 0; l--) {
         const mlcgb_schnet_block &bw = w->blocks[l];
         float *b = blk(l);
-        if ((rc = mlcgb_gemm_tc_chain2(1, b + o.g, bw.lin_w, nullptr, bw.lin2_w, nullptr, b + o.a, N, b + o.gu, b + o.gagg, status, stream))) return rc;
+        if ((rc = gemm_chain2(1, b + o.g, bw.lin_w, nullptr, bw.lin2_w, nullptr, b + o.a, N, b + o.gu, b + o.gagg, image(3 * l + kLin), image(3 * l + kLin2), status, stream))) return rc;
         if (l == 0) {
             if ((rc = seg_pair_dot(b + o.gagg, b + o.xl, ws + o.Wd, offsets, row1, pair_of, twin, L > 1 ? ws + o.gd : nullptr, N, ws + o.gp, st))) return rc;
             break;
@@ -245,7 +243,7 @@ int mlcgb::schnet_train_forward(const void *pos, const int64_t *types, const int
         if ((rc = mlcgb_seg_force(b + o.gagg, b + o.xl, ws + o.W + l * o.wstride, ws + o.Wd + l * o.wstride, offsets, row1, pair_of, N, kH, b + o.gxl, ws + o.gd, l != L - 1,
                                   stream)))
             return rc;
-        if ((rc = mlcgb_gemm_tc_fused(1, b + o.gxl, bw.lin1_w, nullptr, b + o.g, 2, N, kH, kH, blk(l - 1) + o.g, status, stream))) return rc;
+        if ((rc = gemm_fused(1, b + o.gxl, bw.lin1_w, nullptr, b + o.g, 2, N, kH, kH, blk(l - 1) + o.g, image(3 * l + kLin1), status, stream))) return rc;
     }
     return finish_launch((const float *)pos, ws + o.gp, d, row1, offsets, pair_of, N, (float *)grad_pos, negate ? -1.f : 1.f, ws + o.en, struct_ptr, B, (float *)energy, st);
 }
@@ -296,35 +294,39 @@ int mlcgb_schnet_train_backward(const int64_t *types, const int64_t *struct_ptr,
         sb.xb[0] = xb0;
         if ((rc = small_backward(f, sb, st))) return rc;
     } else {
+        const uint8_t *images = ((uintptr_t)fw & 15) == 0 ? (const uint8_t *)(fw + o.images) : nullptr;
+        auto image = [&](int64_t k) { return images ? images + k * kWeightImage : nullptr; };
         // ---- along the tangent
         for (int64_t l = 0; l < L; l++) {
             const mlcgb_schnet_block &bw = w->blocks[l];
             const float *f = fblk(l), *xt_in = l > 0 ? blk(l - 1) + v.xt : nullptr;
             float *b = blk(l);
-            if (l > 0 && (rc = mlcgb_gemm_tc_fused(0, xt_in, bw.lin1_w, nullptr, nullptr, 0, N, kH, kH, b + v.xlt, status, stream))) return rc;
+            if (l > 0 && (rc = gemm_fused(0, xt_in, bw.lin1_w, nullptr, nullptr, 0, N, kH, kH, b + v.xlt, image(3 * l + kLin1), status, stream))) return rc;
             if ((rc = mlcgb_seg_tangent(l > 0 ? b + v.xlt : nullptr, f + o.xl, fw + o.W + l * o.wstride, fw + o.Wd + l * o.wstride, dd, offsets, row1, pair_of, N, kH, b + v.aggt, stream))) return rc;
-            if ((rc = mlcgb_gemm_tc_chain2_tangent(0, b + v.aggt, bw.lin2_w, bw.lin_w, f + o.a, f + o.gu, xt_in, N, b + v.q, b + v.at, b + v.xt, status, stream)))
+            if ((rc = gemm_chain2_tangent(0, b + v.aggt, bw.lin2_w, bw.lin_w, f + o.a, f + o.gu, xt_in, N, b + v.q, b + v.at, b + v.xt, image(3 * l + kLin2),
+                                          image(3 * l + kLin), status, stream)))
                 return rc;
         }
         // ---- output network
         const float *ah = fw + o.ah;
         float *yt = ws + v.yt;
-        if ((rc = mlcgb_gemm_tc_fused(0, blk(L - 1) + v.xt, w->head_W, nullptr, nullptr, 0, N, Wh, kH, yt, status, stream))) return rc;
+        if ((rc = gemm_fused(0, blk(L - 1) + v.xt, w->head_W, nullptr, nullptr, 0, N, Wh, kH, yt, image(3 * L), status, stream))) return rc;
         {
             TimelineScope timeline_scope("head_grad", stream);
             launch_pdl(head_grad_kernel, dim3(grid_for(N * 32, 256)), dim3(256), 0, st, ah, (const float *)yt, (const float *)w->head_out, (const float *)gE,
                        struct_ptr, N, B, Wh, yb, gy, r);
         }
-        if ((rc = mlcgb_gemm_tc_fused(1, yb, w->head_W, nullptr, nullptr, 0, N, kH, Wh, blk(L - 1) + v.xb, status, stream))) return rc;
+        if ((rc = gemm_fused(1, yb, w->head_W, nullptr, nullptr, 0, N, kH, Wh, blk(L - 1) + v.xb, image(3 * L), status, stream))) return rc;
         // ---- and back
         for (int64_t l = L - 1; l >= 0; l--) {
             const mlcgb_schnet_block &bw = w->blocks[l];
             const float *f = fblk(l);
             float *b = blk(l);
-            if ((rc = mlcgb_gemm_tc_chain2_tangent(1, b + v.xb, bw.lin_w, bw.lin2_w, f + o.a, nullptr, nullptr, N, b + v.q, b + v.ub, b + v.agb, status, stream)))
+            if ((rc = gemm_chain2_tangent(1, b + v.xb, bw.lin_w, bw.lin2_w, f + o.a, nullptr, nullptr, N, b + v.q, b + v.ub, b + v.agb, image(3 * l + kLin),
+                                          image(3 * l + kLin2), status, stream)))
                 return rc;
             if ((rc = mlcgb_seg_tangent(b + v.agb, f + o.gagg, fw + o.W + l * o.wstride, fw + o.Wd + l * o.wstride, dd, offsets, row1, pair_of, N, kH, b + v.xlb, stream))) return rc;
-            if ((rc = mlcgb_gemm_tc_fused(1, b + v.xlb, bw.lin1_w, nullptr, b + v.xb, 2, N, kH, kH, l > 0 ? blk(l - 1) + v.xb : xb0, status, stream))) return rc;
+            if ((rc = gemm_fused(1, b + v.xlb, bw.lin1_w, nullptr, b + v.xb, 2, N, kH, kH, l > 0 ? blk(l - 1) + v.xb : xb0, image(3 * l + kLin1), status, stream))) return rc;
         }
     }
     // ---- the filter networks
