@@ -108,14 +108,16 @@ __device__ __forceinline__ void edge_arg(float d, const RbfDev<float> &s, float 
 
 // Shared set-up of both kernels: weight tiles, bias, basis table, barrier, tensor memory.
 template <bool SPLIT>
-__device__ __forceinline__ uint32_t filter_setup(const FilterFwdParams &p, uint8_t *smem, int Kpad1, uint32_t tmem_cols) {
+__device__ __forceinline__ uint32_t filter_setup(const FilterFwdParams &p, uint8_t *smem, int Kpad1, uint32_t tmem_cols, bool have_weights = false) {
     using namespace tc;
     using L = FilterSmem<SPLIT>;
     const int tid = threadIdx.x, warp = tid >> 5;
     const float wscale = SPLIT ? kWScale : 1.f;
-    const bool over1 = load_weight_tile<SPLIT>(smem + L::kB1, smem + L::kB1 + 32768, p.A1, kF, p.rbf.R, Kpad1, wscale);
-    const bool over2 = load_weight_tile<SPLIT>(smem + L::kB2, smem + L::kB2 + 32768, p.A2, kF, kF, kF, wscale);
-    if ((over1 || over2) && blockIdx.x == 0) atomicOr(p.status, (int)kWeightRange);
+    if (!have_weights) {
+        const bool over1 = load_weight_tile<SPLIT>(smem + L::kB1, smem + L::kB1 + 32768, p.A1, kF, p.rbf.R, Kpad1, wscale);
+        const bool over2 = load_weight_tile<SPLIT>(smem + L::kB2, smem + L::kB2 + 32768, p.A2, kF, kF, kF, wscale);
+        if ((over1 || over2) && blockIdx.x == 0) atomicOr(p.status, (int)kWeightRange);
+    }
     float *s_b1 = reinterpret_cast<float *>(smem + L::kMisc + L::kBias);
     float2 *s_tab = reinterpret_cast<float2 *>(smem + L::kMisc + L::kTable);
     if (tid < kF) {

@@ -37,6 +37,7 @@ struct FilterVdParams {
     int64_t block_rows, block_hidden;    // rows / kept floats between the blocks' results
     float *Wd;           // [E][kF] derivatives
     float *Zd;           // z' kept for the weight gradients in hidden_offset() order, or NULL
+    const uint8_t *images;               // of the blocks' weights, two each (schnet_internal.cuh), or NULL
     float *zmax;         // with Zd: largest |z'| (to be zero before; non-negative floats order like their bits)
 };
 
@@ -77,7 +78,15 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
 
     uint8_t *s_live = smem + L::kMisc + L::kRed2;      // [tile & 1][16 warps]: the warp's part of the tile's phi is not all zero
 
-    const uint32_t tmem = filter_setup<SPLIT>(p, smem, Kpad1, 512);
+    const uint32_t wbar = bars + 64;                   // both weights' images have arrived
+    const bool images = SPLIT && q.images;
+    if (images && tid == 0) {
+        mbar_init(wbar, 2);
+        const uint8_t *image = q.images + blockIdx.y * 2 * kWeightImage;
+        fetch_image(smem_u32(smem + L::kB1), image, wbar);
+        fetch_image(smem_u32(smem + L::kB2), image + kWeightImage, wbar);
+    }
+    const uint32_t tmem = filter_setup<SPLIT>(p, smem, Kpad1, 512, images);
     if (tid == 0) {
         for (int i = 0; i < 4; i++) {
             mbar_init(bars + 8 * i, kTcThreads / 32);
@@ -142,6 +151,7 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
         uint32_t tV = tmem, tA = tmem + 128, tQ = tmem + 256;
         const uint32_t tR = tmem + 384;
         uint32_t quarters = 0, next = 0;
+        if (images) await(wbar, 0);                    // (whether or not there is a tile: the block outlives its copies)
         if (n_local > 0) {
             await(r1v, 0);
             next = live_quarters(0);
@@ -445,7 +455,7 @@ static int filter_vd_launch(const FilterVdParams &q, int64_t num_blocks, cudaStr
 
 int filter_vd_blocks(const float *d, int64_t P, const int64_t *rows_dev, const int32_t *sel, const mlcgb_rbf_spec *rbf, int conv_cutoff_kind,
                      double conv_lower, double conv_upper, const mlcgb_schnet_block *blocks, int64_t num_blocks, int precision, float *W, float *Wd,
-                     float *hs, float *zs, float *zmax, int32_t *status, cudaStream_t st) {
+                     float *hs, float *zs, float *zmax, const uint8_t *images, int32_t *status, cudaStream_t st) {
     TimelineScope timeline_scope("filter_value_derivative", st);
     if (int rc = check_spec(rbf, 1)) return rc;
     if (P < 0 || !status || (precision != 0 && precision != 1) || (conv_cutoff_kind != 0 && conv_cutoff_kind != 1)) return MLCGB_E_ARG;
@@ -476,6 +486,7 @@ int filter_vd_blocks(const float *d, int64_t P, const int64_t *rows_dev, const i
     q.Wd = Wd;
     q.Zd = zs;
     q.zmax = zmax;
+    q.images = images;
     return precision == 0 ? filter_vd_launch<true>(q, num_blocks, st) : filter_vd_launch<false>(q, num_blocks, st);
 }
 

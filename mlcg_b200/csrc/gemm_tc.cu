@@ -93,14 +93,6 @@ __device__ __forceinline__ void prefetch_tile_to_boxes(uint8_t *stage, const flo
 }
 __device__ __forceinline__ void wait_prefetch() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// a weight's image (schnet_internal.cuh) into its place in shared memory, by one thread that has just set up `bar`
-__device__ __forceinline__ void fetch_image(uint32_t dst, const uint8_t *image, uint32_t bar) {
-    tc::fence_async_smem();
-    tc::mbar_expect_bytes(bar, (uint32_t)kWeightImage);
-    tc::bulk_load(dst, image, 32768, bar);
-    tc::bulk_load(dst + 32768, image + 32768, 32768, bar);
-}
-
 // ------------------------------------------------------------------------------------------------ NT / NN
 template <int MODE>   // 0 NT, 1 NN
 __global__ void __launch_bounds__(kGT, 1)

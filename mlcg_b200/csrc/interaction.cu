@@ -126,15 +126,20 @@ embedding_rows_kernel(const float *__restrict__ table, const int64_t *__restrict
                       const __grid_constant__ WeightImages im, int32_t *__restrict__ status) {
     pdl_wait();
     if ((int)blockIdx.x < 8 * im.n) {
-        const int k = blockIdx.x >> 3;
+        const int k = blockIdx.x >> 3, cols = im.cols[k], pad = cols <= 64 ? 64 : 128;
         uint8_t *hi = im.dst + k * kWeightImage;
         float most = 0.f;
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const int row = (blockIdx.x & 7) * 16 + u * 8 + (threadIdx.x >> 5), col = (threadIdx.x & 31) * 4;
-            const float *src = im.src[k] + row * 128 + col;
+            if (col >= pad) continue;
+            const float *src = im.src[k] + row * cols + col;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (row < im.rows[k]) v = ((uintptr_t)src & 15) == 0 ? *reinterpret_cast<const float4 *>(src) : make_float4(src[0], src[1], src[2], src[3]);
+            if (row < im.rows[k]) {
+                if (col + 4 <= cols && ((uintptr_t)src & 15) == 0) v = *reinterpret_cast<const float4 *>(src);
+                else
+                    v = make_float4(col < cols ? src[0] : 0.f, col + 1 < cols ? src[1] : 0.f, col + 2 < cols ? src[2] : 0.f, col + 3 < cols ? src[3] : 0.f);
+            }
             most = fmaxf(most, tc::put_weight4<true>(hi, hi + kWeightImage / 2, row, col, v, 64.f));
         }
         if (!(most * 64.f <= 32768.f)) atomicOr(status, (int)kWeightRange);
@@ -152,12 +157,16 @@ embedding_rows_kernel(const float *__restrict__ table, const int64_t *__restrict
     }
 }
 
-int embedding_launch(const mlcgb_schnet_weights *w, const int64_t *types, int64_t N, float *x, void *images, int32_t *status, cudaStream_t st) {
+int embedding_launch(const mlcgb_schnet_weights *w, const int64_t *types, int64_t N, float *x, void *images, int num_rbf, int32_t *status, cudaStream_t st) {
     TimelineScope timeline_scope("embedding", st);
     WeightImages im;
     im.n = 0;
     im.dst = (uint8_t *)images;
-    auto add = [&](const void *src, int64_t rows) { im.src[im.n] = (const float *)src; im.rows[im.n++] = (int)rows; };
+    auto add = [&](const void *src, int64_t rows, int cols = 128) {          // (a weight that is not there is refused by the kernel that takes it)
+        im.src[im.n] = (const float *)src;
+        im.rows[im.n] = (int16_t)(src ? rows : 0);
+        im.cols[im.n++] = (int16_t)cols;
+    };
     if (images) {
         for (int64_t l = 0; l < w->num_blocks; l++) {
             add(w->blocks[l].lin1_w, 128);
@@ -165,6 +174,10 @@ int embedding_launch(const mlcgb_schnet_weights *w, const int64_t *types, int64_
             add(w->blocks[l].lin_w, 128);
         }
         add(w->head_W, w->head_width);
+        for (int64_t l = 0; l < w->num_blocks && num_rbf; l++) {
+            add(w->blocks[l].filter_w1, 128, num_rbf);
+            add(w->blocks[l].filter_w2, 128);
+        }
     }
     launch_pdl(embedding_rows_kernel, dim3(8 * im.n + grid_for(N * (w->hidden >> 2), 256)), dim3(256), 0, st, (const float *)w->embedding, types, N, w->hidden,
                w->num_types, x, im, status);
@@ -274,11 +287,15 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
     auto st = (cudaStream_t)stream;
     float *d = ws + lay.d;
     int rc;
+    // (the kernel behind the one that makes them converts its weight itself: it reads it before it waits for that one)
+    const uint8_t *images = lay.images >= 0 && ((uintptr_t)ws & 15) == 0 ? (const uint8_t *)(ws + lay.images) : nullptr;
+    auto image = [&](int64_t k) { return images ? images + k * kWeightImage : nullptr; };
+    const bool filter_images = images && grad_pos && P > 0 && precision == 0 && rbf && rbf->num_rbf <= 128;
     auto filters = [&](int64_t l, int64_t n) {                               // of blocks l .. l + n - 1, with derivatives where a force pass follows
         float *W = ws + lay.W + l * lay.wstride;
         if (grad_pos)
             return filter_vd_blocks(d, P, pairs_dev, sel, rbf, conv_cutoff_kind, conv_lower, conv_upper, w->blocks + l, n, precision, W,
-                                    ws + lay.Wd + l * lay.wstride, nullptr, nullptr, nullptr, status, st);
+                                    ws + lay.Wd + l * lay.wstride, nullptr, nullptr, nullptr, filter_images ? image(3 * L + 1 + 2 * l) : nullptr, status, st);
         int rf = MLCGB_OK;
         for (int64_t k = l; k < l + n && !rf; k++)
             rf = mlcgb_filter_forward_counted(d, P, pairs_dev, sel, nullptr, rbf, conv_cutoff_kind, conv_lower, conv_upper, w->blocks[k].filter_w1,
@@ -305,10 +322,7 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
         return small_finish(f, twin, struct_ptr, (float *)energy, (float *)grad_pos, grad_sign, st);
     }
     if (!have_distances && (rc = mlcgb_edge_distance(pos, MLCGB_F32, row0, row1, E, N, d, status, stream))) return rc;
-    // (the kernel behind the one that makes them converts its weight itself: it reads it before it waits for that one)
-    const uint8_t *images = lay.images >= 0 && ((uintptr_t)ws & 15) == 0 ? (const uint8_t *)(ws + lay.images) : nullptr;
-    auto image = [&](int64_t k) { return images ? images + k * kWeightImage : nullptr; };
-    if ((rc = embedding_launch(w, types, N, ws + lay.x[0], (void *)images, status, st))) return rc;
+    if ((rc = embedding_launch(w, types, N, ws + lay.x[0], (void *)images, filter_images ? rbf->num_rbf : 0, status, st))) return rc;
     ChainScope chain;
     int cur = 0;
     for (int64_t l = 0; l < L; l++) {

@@ -10,20 +10,22 @@ constexpr int kMaxBlocks = 10;             // interaction blocks of the whole-mo
 // rows kept per block where all blocks' filter rows share one matrix: whole 128-row tiles
 inline int64_t padded_rows(int64_t P) { return (P + 127) / 128 * 128; }
 
-// The weights of the node layers as the tensor-core kernels hold them: fp16 pairs in the layout of a 128 x 128 operand tile (high part,
-// low part), 64 KB each.  Made once per evaluation or step beside the embedding (interaction.cu); a kernel then fetches them with two
-// bulk copies that arrive under its first tile instead of 128 KB of loads, conversions and stores in every one of its CTAs.
+// Weights as the tensor-core kernels hold them: fp16 pairs in the layout of a 128-row operand tile (high part, low part), 64 KB each.
+// Made once per evaluation or step beside the embedding (interaction.cu); a kernel then fetches them with bulk copies that arrive under
+// its first tile instead of 64 KB of loads, conversions and stores per weight in every one of its CTAs.
 constexpr int64_t kWeightImage = 65536;
-enum { kLin1 = 0, kLin2 = 1, kLin = 2 };   // of block l: image 3 l + one of these; the output network's first layer follows the blocks'
+enum { kLin1 = 0, kLin2 = 1, kLin = 2 };   // image 3 l + one of these: of block l; 3 L: the output network's first layer; 3 L + 1 + 2 l: filter_w1, filter_w2
+constexpr int kMaxImages = 5 * kMaxBlocks + 1;
 struct WeightImages {
-    const float *src[3 * kMaxBlocks + 1];
-    int rows[3 * kMaxBlocks + 1];          // (columns: 128)
+    const float *src[kMaxImages];
+    int16_t rows[kMaxImages], cols[kMaxImages];
     int n;
     uint8_t *dst;
 };
-inline int64_t weight_images_floats(int64_t num_blocks) { return (3 * num_blocks + 1) * (kWeightImage / 4); }
-// embedding rows of all nodes and, unless images is NULL (16-byte aligned, all widths 128 but the output network's), the weight images
-int embedding_launch(const mlcgb_schnet_weights *w, const int64_t *types, int64_t N, float *x, void *images, int32_t *status, cudaStream_t st);
+inline int64_t weight_images_floats(int64_t num_blocks) { return (5 * num_blocks + 1) * (kWeightImage / 4); }
+// embedding rows of all nodes and, unless images is NULL (16-byte aligned, all widths 128 but the output network's), the weight images,
+// the filter networks' (of num_rbf basis functions) too unless num_rbf is 0
+int embedding_launch(const mlcgb_schnet_weights *w, const int64_t *types, int64_t N, float *x, void *images, int num_rbf, int32_t *status, cudaStream_t st);
 // gemm_tc.cu: mlcgb_gemm_tc_fused, _chain2 and _chain2_tangent with the images of their weights (NULL: converted by the kernel)
 int gemm_fused(int mode, const void *A, const void *B, const void *bias, const void *aux, int epilogue, int64_t M, int64_t N, int64_t K, void *C,
                const uint8_t *image, int32_t *status, void *stream);
@@ -36,7 +38,7 @@ int gemm_chain2_tangent(int reverse, const void *A, const void *Wa, const void *
 // l * padded_rows(P) of W and Wd, its kept rows (or NULL) at l * mlcgb_filter_hidden_bytes(P) of hs and zs, its zmax at l.
 int filter_vd_blocks(const float *d, int64_t P, const int64_t *rows_dev, const int32_t *sel, const mlcgb_rbf_spec *rbf, int conv_cutoff_kind,
                      double conv_lower, double conv_upper, const mlcgb_schnet_block *blocks, int64_t num_blocks, int precision, float *W, float *Wd,
-                     float *hs, float *zs, float *zmax, int32_t *status, cudaStream_t st);
+                     float *hs, float *zs, float *zmax, const uint8_t *images, int32_t *status, cudaStream_t st);    // images: of blocks[0], NULL: none
 
 // filter_wgrad.cu: the weight gradients of all of them in one launch; xl, xt, gagg, agb per block
 struct FilterGradBlock {

@@ -83,6 +83,14 @@ __device__ __forceinline__ void bulk_load(uint32_t dst_saddr, const void *src, u
                  : "memory");
 }
 
+// a weight's image (64 KB, schnet_internal.cuh) into its place in shared memory, by the thread that has just set up `bar_saddr`
+__device__ __forceinline__ void fetch_image(uint32_t dst_saddr, const uint8_t *image, uint32_t bar_saddr) {
+    fence_async_smem();
+    mbar_expect_bytes(bar_saddr, 65536);
+    bulk_load(dst_saddr, image, 32768, bar_saddr);
+    bulk_load(dst_saddr + 32768, image + 32768, 32768, bar_saddr);
+}
+
 // Waits for the phase with the given parity; gives up after kSpinLimit polls and returns false.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar_saddr, uint32_t parity) {
     for (uint32_t it = 0; it < kSpinLimit; ++it) {

@@ -199,9 +199,11 @@ int mlcgb::schnet_train_forward(const void *pos, const int64_t *types, const int
     auto blk = [&](int64_t l) { return ws + o.block0 + l * o.stride; };
     train_begin_kernel<<<grid_for(3 * N, 256), 256, 0, st>>>((const float *)pos, 3 * N, ws + o.pos, ws + o.zmax, L);
     ChainScope chain;
+    const uint8_t *images = N > kSmallNodes && ((uintptr_t)ws & 15) == 0 ? (const uint8_t *)(ws + o.images) : nullptr;
+    auto image = [&](int64_t k) { return images ? images + k * kWeightImage : nullptr; };
     auto filters = [&](int64_t l, int64_t n) {
         return filter_vd_blocks(d, P, nullptr, sel, rbf, conv_cutoff_kind, conv_lower, conv_upper, w->blocks + l, n, 0, ws + o.W + l * o.wstride,
-                                ws + o.Wd + l * o.wstride, ws + o.Hs + l * o.hstride, ws + o.Zs + l * o.hstride, ws + o.zmax + l, status, st);
+                                ws + o.Wd + l * o.wstride, ws + o.Hs + l * o.hstride, ws + o.Zs + l * o.hstride, ws + o.zmax + l, image(3 * L + 1 + 2 * l), status, st);
     };
     if (N <= kSmallNodes) {
         const SmallForward f = small_view(o, ws, pos, types, row0, row1, pair_of, offsets, N, E, B, w, status);
@@ -212,9 +214,7 @@ int mlcgb::schnet_train_forward(const void *pos, const int64_t *types, const int
     }
     int rc = have_distances ? MLCGB_OK : mlcgb_edge_distance(pos, MLCGB_F32, row0, row1, E, N, d, status, stream);
     if (rc) return rc;
-    const uint8_t *images = ((uintptr_t)ws & 15) == 0 ? (const uint8_t *)(ws + o.images) : nullptr;
-    auto image = [&](int64_t k) { return images ? images + k * kWeightImage : nullptr; };
-    if ((rc = embedding_launch(w, types, N, blk(0) + o.x, (void *)images, status, st))) return rc;
+    if ((rc = embedding_launch(w, types, N, blk(0) + o.x, (void *)images, rbf->num_rbf, status, st))) return rc;
     for (int64_t l = 0; l < L; l++) {
         const mlcgb_schnet_block &bw = w->blocks[l];
         float *b = blk(l), *xout = l + 1 < L ? blk(l + 1) + o.x : ws + o.block0 + L * o.stride;
