@@ -972,38 +972,42 @@ int tn_jobs_launch(const TnJobs &jobs, int n, int32_t *status, cudaStream_t st) 
     return check_launch();
 }
 
-// dst[i] = sum over parts of src[part * stride + i]; entry blockIdx.y.  A block takes 32 elements, a warp an eighth of the parts, and the
-// eighths are added in their order: bound by the latency of a thread's chain of loads, which is 592 parts long for the embedding table
-// (one thread per element: 49 us for the sums of a 256 x 73 step).
+// dst[i] = sum over parts of src[part * stride + i]; entry blockIdx.y.  A block takes 128 elements, four a lane, a warp an eighth of the
+// parts, and the eighths are added in their order: bound by the latency of a thread's chain of loads, which is 592 parts long for the
+// embedding table (one thread per element: 49 us for the sums of a 256 x 73 step, one element per lane 29, now 20, the
+// longest chains first).
 constexpr int kSumWarps = 8;
 __global__ void __launch_bounds__(kSumWarps * 32) partial_sums_kernel(const __grid_constant__ PartialSums sums) {
-    __shared__ float s_part[kSumWarps][32];
+    __shared__ float4 s_part[kSumWarps][32];
     const PartialSum &s = sums.sum[blockIdx.y];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, z0 = s.parts * warp / kSumWarps, z1 = s.parts * (warp + 1) / kSumWarps;
-    for (int64_t i0 = (int64_t)blockIdx.x * 32; i0 < s.n; i0 += (int64_t)gridDim.x * 32) {
-        const int64_t i = i0 + lane;
-        float v = 0.f;
+    const bool whole = ((uintptr_t)s.dst & 15) == 0;
+    auto add = [](float4 &v, const float4 &x) { v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w; };
+    for (int64_t i0 = (int64_t)blockIdx.x * 128; i0 < s.n; i0 += (int64_t)gridDim.x * 128) {
+        const int64_t i = i0 + lane * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i < s.n) {
             int z = z0;
             for (; z + 8 <= z1; z += 8) {
-                float x[8];
+                float4 x[8];
 #pragma unroll
-                for (int u = 0; u < 8; u++) x[u] = __ldg(s.src + (z + u) * s.stride + i);
+                for (int u = 0; u < 8; u++) x[u] = __ldg(reinterpret_cast<const float4 *>(s.src + (z + u) * s.stride + i));
 #pragma unroll
-                for (int u = 0; u < 8; u++) v += x[u];
+                for (int u = 0; u < 8; u++) add(v, x[u]);
             }
-            float x[8];
+            float4 x[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) x[u] = z + u < z1 ? __ldg(s.src + (z + u) * s.stride + i) : 0.f;
+            for (int u = 0; u < 8; u++) x[u] = z + u < z1 ? __ldg(reinterpret_cast<const float4 *>(s.src + (z + u) * s.stride + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int u = 0; u < 8; u++) v += x[u];
+            for (int u = 0; u < 8; u++) add(v, x[u]);
         }
         s_part[warp][lane] = v;
         __syncthreads();
         if (warp == 0 && i < s.n) {
 #pragma unroll
-            for (int w = 1; w < kSumWarps; w++) v += s_part[w][lane];
-            s.dst[i] = v;
+            for (int w = 1; w < kSumWarps; w++) add(v, s_part[w][lane]);
+            if (whole) *reinterpret_cast<float4 *>(s.dst + i) = v;
+            else { s.dst[i] = v.x; s.dst[i + 1] = v.y; s.dst[i + 2] = v.z; s.dst[i + 3] = v.w; }
         }
         __syncthreads();
     }

@@ -342,6 +342,7 @@ int mlcgb_schnet_train_backward(const int64_t *types, const int64_t *struct_ptr,
     TnJobs jobs;
     PartialSums sums;
     int nj = 0, ns = 0;
+    sums.sum[ns++] = {ws + v.emb_part, (float *)grads->embedding, T * kH, (int)(T * kH), v.emb_grid * v.emb_groups};   // (the longest chains first)
     jobs.E = N;
     jobs.parts = v.node_parts;
     float *part = ws + v.node_part;
@@ -376,7 +377,6 @@ int mlcgb_schnet_train_backward(const int64_t *types, const int64_t *struct_ptr,
         }
         launch_pdl(embedding_grad_kernel, dim3(v.emb_grid), dim3(128 * v.emb_groups), (size_t)v.emb_groups * T * 512, st, (const float *)xb0, types, N, (int)T,
                    ws + v.emb_part);
-        sums.sum[ns++] = {ws + v.emb_part, (float *)grads->embedding, T * kH, (int)(T * kH), v.emb_grid * v.emb_groups};
         if ((rc = tn_jobs_launch(jobs, nj, status, st))) return rc;
         if ((rc = partial_sums_launch(sums, ns, st))) return rc;
     }

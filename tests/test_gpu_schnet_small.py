@@ -4,6 +4,7 @@ import torch
 
 import mlcg_b200
 from mlcg_b200 import nn as bnn
+from mlcg_b200.backend import get_backend
 
 from helpers import random_walk_chain
 from test_gpu_schnet import E_RTOL, F_ATOL, _oracle
@@ -187,6 +188,37 @@ def test_large_batches_with_nodes_of_every_degree(blocks):
     out = bnn.GradientsOut(net, "forces").eval()(data).out["SchNet"]
     assert torch.allclose(out["energy"].cpu().double(), e_x, rtol=E_RTOL, atol=E_RTOL * float(e_x.abs().max()))
     # (dense clusters: forces of hundreds, to the same number of digits as elsewhere)
+    assert float((out["forces"].cpu().double() - f_x).abs().max()) < F_ATOL * max(1.0, float(f_x.abs().max()) / 10)
+
+
+@pytest.mark.parametrize("num_rbf,head,shift,too_large", [(20, 128, 0, None), (33, 64, 1, None), (64, 36, 2, None), (65, 4, 0, None), (128, 128, 3, None),
+                                                          (50, 128, 0, "lin1"), (50, 128, 0, "filter2"), (50, 64, 0, "head")])
+def test_weights_as_operand_tiles_of_large_batches(num_rbf, head, shift, too_large):
+    """Above the small batches' limit the weights are made into operand tiles in front: of every width, at addresses of any alignment, and
+    those beyond the range of a pair of fp16 are reported."""
+    gen = torch.Generator().manual_seed(num_rbf)
+    torch.manual_seed(3)
+    upper, sizes = 8.0, [60] * 39 + [29]
+    cut = bnn.CosineCutoff(0.0, upper)
+    net = bnn.StandardSchNet(bnn.GaussianBasis(cut, num_rbf, trainable=False), cut, [head], hidden_channels=128, embedding_size=6, num_filters=128, num_interactions=2)
+    pos = torch.cat([torch.rand(n, 3, generator=gen) * 14.0 for n in sizes])
+    types_, batch = torch.randint(0, 6, (sum(sizes),), generator=gen), torch.arange(len(sizes)).repeat_interleave(torch.tensor(sizes))
+    e_x, f_x, _ = _oracle(net, "gaussian", upper, 2, pos, types_, batch, len(sizes), torch.float64)
+    net = net.to(DEV).eval()
+    layers = dict(lin1=net.interaction_blocks[1].conv.lin1, filter2=[m for m in net.interaction_blocks[0].conv.filter_network.modules() if hasattr(m, "weight")][-1],
+                  head=[m for m in net.output_network.modules() if hasattr(m, "weight")][0])
+    for name, p in net.named_parameters():
+        if "embedding" not in name:                    # (its rows are read in 16-byte pieces)
+            p.data = torch.cat([p.data.new_zeros(shift), p.data.flatten()])[shift:].view(p.shape)
+    if too_large:
+        layers[too_large].weight.data[3, 1] = 600.0
+    out = bnn.GradientsOut(net, "forces").eval()(mlcg_b200.AtomicData(pos=pos.to(DEV), atom_types=types_.to(DEV), batch=batch.to(DEV),
+                                                                      n_atoms=torch.tensor(sizes).to(DEV))).out["SchNet"]
+    if too_large:
+        with pytest.raises(RuntimeError):
+            get_backend().check_pending()
+        return
+    assert torch.allclose(out["energy"].cpu().double(), e_x, rtol=E_RTOL, atol=E_RTOL * float(e_x.abs().max()))
     assert float((out["forces"].cpu().double() - f_x).abs().max()) < F_ATOL * max(1.0, float(f_x.abs().max()) / 10)
 
 
