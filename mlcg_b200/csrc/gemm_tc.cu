@@ -379,21 +379,28 @@ gemm_tc_rows_pipe_kernel(const float *__restrict__ A, const float *__restrict__ 
 // and, for the weight gradients of a force-matching step, the same two along a tangent and back (a: the block's tanh outputs):
 //   TAN (NT, NT):  u = A Wa^T,  mid = (1 - a^2) u,  q_out = -2 a u gu               C = aux + mid Wb^T      (ext0 = a, ext1 = gu)
 //   REV (NN, NN):  mid = (A Wa) (1 - aux^2) + q                                     C = mid Wb              (ext0 = q)
-// All widths are 128.  Shared memory: both weight tiles as fp16 hi/lo pairs (2 x 64 KB) and one 64 KB stage through which
-// every tile enters and leaves in whole rows.  One accumulator and one operand block of tensor memory, used by both GEMMs of
-// a tile one after the other.
+// LINKED: a third layer on the tile while it is on the chip (ChainLink, schnet_internal.cuh): behind the forward kinds the next block's
+// first layer or the output network's, in front of the backward ones the transpose of the same; its result, the gradient of the block's
+// output, then leaves on the way.  There is no room for three weights: the first and the third take turns in one place, each fetched by
+// bulk copy as soon as the other's GEMM is over.
+// All widths are 128 (but the third layer's outer one).  Shared memory: two weight tiles as fp16 hi/lo pairs (2 x 64 KB) and one 64 KB
+// stage through which every tile enters and leaves in whole rows.  One accumulator and one operand block of tensor memory, used by the
+// GEMMs of a tile one after the other.
+// Bound by latency: a tile's layers follow one another at one CTA of 16 warps per SM, 20 % of the L2's and 30 % of the memory's rate.  A
+// layer in a kernel of its own pays for a launch, barriers and tensor memory, a tile's way in and out; on 16 000 rows that is 9 us where
+// it takes 3 here (evaluation of 96 x 268 ragged 556 -> 514 us, step of 256 x 73 1518 -> 1428, evaluation of 512 x 100 1705 -> 1680).
 struct ChainSmem {
     static constexpr int kWa = 0, kWb = 65536, kStage = 131072, kMisc = 196608;
     static constexpr int kTotal = kMisc + 4096 + 1024;
 };
 
 enum { kChainFwd = 0, kChainBwd = 1, kChainTan = 2, kChainRev = 3 };
-template <int KIND>
+template <int KIND, bool LINKED>
 __global__ void __launch_bounds__(kGT, 1)
 gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa, const float *__restrict__ ba, const float *__restrict__ Wb,
                       const float *__restrict__ bb, const float *__restrict__ aux, int64_t E, float *__restrict__ mid_out,
                       float *__restrict__ C, int32_t *__restrict__ status, const float *__restrict__ ext0, const float *__restrict__ ext1,
-                      float *__restrict__ q_out, const uint8_t *__restrict__ image_a, const uint8_t *__restrict__ image_b) {
+                      float *__restrict__ q_out, const uint8_t *__restrict__ image_a, const uint8_t *__restrict__ image_b, const ChainLink link) {
     using namespace tc;
     using L = ChainSmem;
     constexpr bool BWD = KIND == kChainBwd || KIND == kChainRev;
@@ -404,8 +411,8 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
     uint8_t *sWa_hi = smem + L::kWa, *sWa_lo = sWa_hi + 32768, *sWb_hi = smem + L::kWb, *sWb_lo = sWb_hi + 32768;
     uint8_t *stage = smem + L::kStage;
     float *s_red = reinterpret_cast<float *>(smem + L::kMisc);
-    float *s_ba = s_red + 512, *s_bb = s_ba + 128;
-    uint64_t *s_bar = reinterpret_cast<uint64_t *>(s_bb + 128);
+    float *s_ba = s_red + 512, *s_bb = s_ba + 128, *s_bc = s_bb + 128;         // biases; s_bc: of the third layer, or its vector
+    uint64_t *s_bar = reinterpret_cast<uint64_t *>(s_bc + 128);
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(s_bar + 3);                // (barriers of the GEMMs, of Wa and of Wb)
     int *s_err = reinterpret_cast<int *>(s_tmem + 1);
 
@@ -420,6 +427,10 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
     if (tid < 128) {
         s_ba[tid] = ba ? ba[tid] : 0.f;
         s_bb[tid] = bb ? bb[tid] : 0.f;
+        if (LINKED) {
+            const float *of = BWD ? link.vec : link.bias;
+            s_bc[tid] = of && tid < link.width ? of[tid] : 0.f;
+        }
     }
     const uint32_t bar = smem_u32(s_bar);
     if (tid == 0) {
@@ -428,7 +439,7 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
         mbar_init(bar + 16, 1);
         *s_err = 0;
         if (image_a) {
-            fetch_image(smem_u32(sWa_hi), image_a, bar + 8);
+            fetch_image(smem_u32(sWa_hi), LINKED && BWD ? link.image : image_a, bar + 8);
             fetch_image(smem_u32(sWb_hi), image_b, bar + 16);
         }
     }
@@ -446,7 +457,8 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
     const int64_t ntiles = (E + kRows - 1) / kRows;
     uint32_t phase = 0;
     bool failed = false;
-    if (blockIdx.x < ntiles) prefetch_tile_to_stage(stage, A, (int64_t)blockIdx.x * kRows, E, W);
+    const int in_cols = LINKED && BWD ? link.width : W;
+    if (blockIdx.x < ntiles) prefetch_tile_to_stage(stage, A, (int64_t)blockIdx.x * kRows, E, in_cols);
 
     // this thread's 32 values -> operand block (row-scaled fp16 pairs); returns the row's scale.  `fetch`: a tile to copy into
     // the stage as soon as everybody has read the current contents out of it (rows of `fetch` starting at `fetch_row0`)
@@ -464,15 +476,18 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
         __syncthreads();
         return sc;
     };
-    int arrived = image_a ? 0 : 2;                  // weight images that have
-    auto gemm = [&](uint8_t *w_hi, uint8_t *w_lo) {
+    // Both weights are there for good, or (LINKED) the first place holds two in turn, each fetched when the GEMM with the other is done:
+    // `parity` of the fetch that has to be over
+    auto gemm = [&](uint8_t *w_hi, uint32_t wbar, uint32_t parity) {
         if (warp == 0 && elect_one()) {
-            if (arrived < 2 && !mbar_wait(bar + 8 + 8 * arrived, 0)) *s_err = 1;
-            arrived++;
+            if (image_a && !mbar_wait(wbar, parity)) *s_err = 1;
             tc_fence_after();
-            issue_gemm_ts<true>(tmem, ta, smem_u32(w_hi), smem_u32(w_lo), W / 16, MODE, W);
+            issue_gemm_ts<true>(tmem, ta, smem_u32(w_hi), smem_u32(w_hi) + 32768, W / 16, MODE, W);
             mma_commit(bar);
         }
+    };
+    auto refill = [&](const uint8_t *image) {
+        if (LINKED && warp == 0 && elect_one()) fetch_image(smem_u32(sWa_hi), image, bar + 8);
     };
     auto await = [&]() {
         if (!failed && !mbar_wait(bar, phase)) failed = true;
@@ -480,14 +495,14 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
         tc_fence_after();
     };
     // rows of the stage -> global memory, whole rows by consecutive lanes, eight rows per warp in flight
-    auto store_stage = [&](float *dst, int64_t tile) {
+    auto store_stage = [&](float *dst, int64_t tile, int cols) {
         float4 v[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) v[i] = *gstage(stage, warp * 8 + i, lane);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             const int64_t gr = tile * kRows + warp * 8 + i;
-            if (gr < E) __stcs(reinterpret_cast<float4 *>(dst + gr * W) + lane, v[i]);
+            if (gr < E && (!LINKED || lane * 4 < cols)) __stcs(reinterpret_cast<float4 *>(dst + gr * cols) + lane, v[i]);
         }
     };
 
@@ -509,9 +524,45 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
             const float4 v = *gstage(stage, r, (col0 >> 2) + w);
             x[4 * w] = v.x; x[4 * w + 1] = v.y; x[4 * w + 2] = v.z; x[4 * w + 3] = v.w;
         }
-        const float sc1 = to_operand(x, BWD ? aux : nullptr, tile * kRows);      // BWD: the tanh outputs arrive under the first GEMM
-        gemm(sWa_hi, sWa_lo);
+        if (LINKED && BWD) {
+            if (link.vec) {
+#pragma unroll
+                for (int c = 0; c < 32; c++) x[c] = s_bc[col0 + c] * fmaf(-x[c], x[c], 1.f);
+            }
+            const float sc0 = to_operand(x, link.res, tile * kRows);
+            gemm(sWa_hi, bar + 8, 0);
+            await();
+            refill(image_a);
+            if (link.res) {
+                wait_prefetch();
+                __syncthreads();
+            }
+            float v[32];
+            tmem_ld32(tmem + lane_off + col0, v);
+            const float inv = 1.f / (sc0 * kWS);
+#pragma unroll
+            for (int w = 0; w < 8; w++) {
+                float4 o = make_float4(v[4 * w] * inv, v[4 * w + 1] * inv, v[4 * w + 2] * inv, v[4 * w + 3] * inv);
+                float4 *slot = gstage(stage, r, (col0 >> 2) + w);
+                if (link.res) {
+                    const float4 t4 = *slot;
+                    o = make_float4(o.x + t4.x, o.y + t4.y, o.z + t4.z, o.w + t4.w);
+                }
+                *slot = o;
+                x[4 * w] = o.x; x[4 * w + 1] = o.y; x[4 * w + 2] = o.z; x[4 * w + 3] = o.w;
+            }
+        }
+        // BWD: the tanh outputs arrive under the first GEMM, behind what leaves
+        const float sc1 = to_operand(x, BWD && !LINKED ? aux : nullptr, tile * kRows);
+        gemm(sWa_hi, bar + 8, LINKED && BWD ? 1 : 0);
+        if (LINKED && BWD) {
+            store_stage(link.out, tile, W);
+            __syncthreads();
+            prefetch_tile_to_stage(stage, aux, tile * kRows, E, W);
+        }
         await();
+        if (LINKED && !BWD) refill(link.image);
+        if (LINKED && BWD && tile + gridDim.x < ntiles) refill(link.image);
         if (BWD) {
             wait_prefetch();
             __syncthreads();
@@ -547,9 +598,9 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
             }
         }
         const float sc2 = to_operand(x, nullptr, 0);     // (the accumulator has been read, the first GEMM's operand consumed)
-        gemm(sWb_hi, sWb_lo);
+        gemm(sWb_hi, bar + 16, 0);
         if (!BWD || mid_out) {                       // under the second GEMM: mid leaves, the residual tile arrives
-            store_stage(mid_out, tile);
+            store_stage(mid_out, tile, W);
             __syncthreads();
             if (residual) prefetch_tile_to_stage(stage, aux, tile * kRows, E, W);
         }
@@ -572,14 +623,36 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
                     o = make_float4(o.x + t4.x, o.y + t4.y, o.z + t4.z, o.w + t4.w);
                 }
                 *slot = o;
+                if (LINKED && !BWD) { x[4 * w] = o.x; x[4 * w + 1] = o.y; x[4 * w + 2] = o.z; x[4 * w + 3] = o.w; }
+            }
+        }
+        const int64_t next = tile + gridDim.x;
+        if (LINKED && !BWD) {
+            const float sc3 = to_operand(x, nullptr, 0);
+            gemm(sWa_hi, bar + 8, 1);
+            store_stage(C, tile, W);
+            __syncthreads();
+            await();
+            if (next < ntiles) refill(image_a);
+            if (col0 < link.width) {
+                float v[32];
+                tmem_ld32(tmem + lane_off + col0, v);
+                const float inv = 1.f / (sc3 * kWS);
+#pragma unroll
+                for (int w = 0; w < 8; w++) {
+                    float4 o = make_float4(fmaf(v[4 * w], inv, s_bc[col0 + 4 * w]), fmaf(v[4 * w + 1], inv, s_bc[col0 + 4 * w + 1]),
+                                           fmaf(v[4 * w + 2], inv, s_bc[col0 + 4 * w + 2]), fmaf(v[4 * w + 3], inv, s_bc[col0 + 4 * w + 3]));
+                    if (link.tanh) o = make_float4(tanh_ex2(o.x), tanh_ex2(o.y), tanh_ex2(o.z), tanh_ex2(o.w));
+                    *gstage(stage, r, (col0 >> 2) + w) = o;
+                }
             }
         }
         tc_fence_before();
         __syncthreads();
-        store_stage(C, tile);
+        if (LINKED && !BWD) store_stage(link.out, tile, link.width);
+        else store_stage(C, tile, W);
         __syncthreads();                            // the stage is free for the next input tile
-        const int64_t next = tile + gridDim.x;
-        if (next < ntiles) prefetch_tile_to_stage(stage, A, next * kRows, E, W);
+        if (next < ntiles) prefetch_tile_to_stage(stage, A, next * kRows, E, in_cols);
     }
     wait_prefetch();
     if (failed) *s_err = 1;
@@ -1049,23 +1122,34 @@ static int rows_pipe_launch(int mode, const void *A, const void *B, const void *
     return check_launch();
 }
 
-template <int KIND>
-static int chain2_launch(const void *A, const void *Wa, const void *ba, const void *Wb, const void *bb, const void *aux, int64_t M, void *mid_out,
-                         void *C, const void *ext0, const void *ext1, void *q_out, const uint8_t *image_a, const uint8_t *image_b, int32_t *status, cudaStream_t st) {
+template <int KIND, bool LINKED>
+static int chain2_launch_as(const void *A, const void *Wa, const void *ba, const void *Wb, const void *bb, const void *aux, int64_t M, void *mid_out,
+                            void *C, const void *ext0, const void *ext1, void *q_out, const uint8_t *image_a, const uint8_t *image_b,
+                            const ChainLink &link, int32_t *status, cudaStream_t st) {
     const int64_t ntiles = (M + tc::kRows - 1) / tc::kRows;
     const int grid = (int)(ntiles < kNumSM ? ntiles : kNumSM);
     static bool done[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        if (cudaFuncSetAttribute(gemm_tc_chain2_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, ChainSmem::kTotal) != cudaSuccess)
+        if (cudaFuncSetAttribute(gemm_tc_chain2_kernel<KIND, LINKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, ChainSmem::kTotal) != cudaSuccess)
             return check_launch();
         done[dev] = true;
     }
-    launch_with_weights(gemm_tc_chain2_kernel<KIND>, dim3(grid), dim3(kGT), ChainSmem::kTotal, st, (const float *)A, (const float *)Wa, (const float *)ba,
+    launch_with_weights(gemm_tc_chain2_kernel<KIND, LINKED>, dim3(grid), dim3(kGT), ChainSmem::kTotal, st, (const float *)A, (const float *)Wa, (const float *)ba,
                (const float *)Wb, (const float *)bb, (const float *)aux, M, (float *)mid_out, (float *)C, status, (const float *)ext0,
-               (const float *)ext1, (float *)q_out, image_a, image_b);
+               (const float *)ext1, (float *)q_out, image_a, image_b, link);
     return check_launch();
+}
+template <int KIND>
+static int chain2_launch(const void *A, const void *Wa, const void *ba, const void *Wb, const void *bb, const void *aux, int64_t M, void *mid_out,
+                         void *C, const void *ext0, const void *ext1, void *q_out, const uint8_t *image_a, const uint8_t *image_b,
+                         const ChainLink *link, int32_t *status, cudaStream_t st) {
+    if (link) {
+        if (!link->image || !image_a || !image_b || !link->out) return MLCGB_E_ARG;
+        return chain2_launch_as<KIND, true>(A, Wa, ba, Wb, bb, aux, M, mid_out, C, ext0, ext1, q_out, image_a, image_b, *link, status, st);
+    }
+    return chain2_launch_as<KIND, false>(A, Wa, ba, Wb, bb, aux, M, mid_out, C, ext0, ext1, q_out, image_a, image_b, ChainLink{}, status, st);
 }
 
 int gemm_fused(int mode, const void *A, const void *B, const void *bias, const void *aux, int epilogue, int64_t M, int64_t N, int64_t K, void *C,
@@ -1080,27 +1164,27 @@ int gemm_fused(int mode, const void *A, const void *B, const void *bias, const v
 }
 
 int gemm_chain2(int backward, const void *A, const void *Wa, const void *ba, const void *Wb, const void *bb, const void *aux, int64_t M, void *mid_out,
-                void *C, const uint8_t *image_a, const uint8_t *image_b, int32_t *status, void *stream) {
+                void *C, const uint8_t *image_a, const uint8_t *image_b, const ChainLink *link, int32_t *status, void *stream) {
     TimelineScope timeline_scope("gemm_tc_chain2", stream);
     if (M < 0 || !status) return MLCGB_E_ARG;
     if (M == 0) return MLCGB_OK;
     if (!A || !Wa || !Wb || !aux || !C || (!backward && !mid_out)) return MLCGB_E_ARG;
     if ((((uintptr_t)A | (uintptr_t)aux | (uintptr_t)C | (uintptr_t)mid_out) & 15) != 0) return MLCGB_E_LIMIT;
     const auto st = (cudaStream_t)stream;
-    return backward ? chain2_launch<kChainBwd>(A, Wa, ba, Wb, bb, aux, M, mid_out, C, nullptr, nullptr, nullptr, image_a, image_b, status, st)
-                    : chain2_launch<kChainFwd>(A, Wa, ba, Wb, bb, aux, M, mid_out, C, nullptr, nullptr, nullptr, image_a, image_b, status, st);
+    return backward ? chain2_launch<kChainBwd>(A, Wa, ba, Wb, bb, aux, M, mid_out, C, nullptr, nullptr, nullptr, image_a, image_b, link, status, st)
+                    : chain2_launch<kChainFwd>(A, Wa, ba, Wb, bb, aux, M, mid_out, C, nullptr, nullptr, nullptr, image_a, image_b, link, status, st);
 }
 
 int gemm_chain2_tangent(int reverse, const void *A, const void *Wa, const void *Wb, const void *a, const void *gu, const void *aux, int64_t M, void *q,
-                        void *mid_out, void *C, const uint8_t *image_a, const uint8_t *image_b, int32_t *status, void *stream) {
+                        void *mid_out, void *C, const uint8_t *image_a, const uint8_t *image_b, const ChainLink *link, int32_t *status, void *stream) {
     TimelineScope timeline_scope("gemm_tc_chain2_tangent", stream);
     if (M < 0 || !status) return MLCGB_E_ARG;
     if (M == 0) return MLCGB_OK;
     if (!A || !Wa || !Wb || !a || !q || !mid_out || !C || (!reverse && !gu)) return MLCGB_E_ARG;
     if ((((uintptr_t)A | (uintptr_t)a | (uintptr_t)gu | (uintptr_t)aux | (uintptr_t)q | (uintptr_t)mid_out | (uintptr_t)C) & 15) != 0) return MLCGB_E_LIMIT;
     const auto st = (cudaStream_t)stream;
-    if (reverse) return chain2_launch<kChainRev>(A, Wa, nullptr, Wb, nullptr, a, M, mid_out, C, q, nullptr, nullptr, image_a, image_b, status, st);
-    return chain2_launch<kChainTan>(A, Wa, nullptr, Wb, nullptr, aux, M, mid_out, C, a, gu, q, image_a, image_b, status, st);
+    if (reverse) return chain2_launch<kChainRev>(A, Wa, nullptr, Wb, nullptr, a, M, mid_out, C, q, nullptr, nullptr, image_a, image_b, link, status, st);
+    return chain2_launch<kChainTan>(A, Wa, nullptr, Wb, nullptr, aux, M, mid_out, C, a, gu, q, image_a, image_b, link, status, st);
 }
 
 }  // namespace mlcgb
@@ -1116,12 +1200,12 @@ int mlcgb_gemm_tc_fused(int mode, const void *A, const void *B, const void *bias
 
 int mlcgb_gemm_tc_chain2(int backward, const void *A, const void *Wa, const void *ba, const void *Wb, const void *bb, const void *aux,
                          int64_t M, void *mid_out, void *C, int32_t *status, void *stream) {
-    return gemm_chain2(backward, A, Wa, ba, Wb, bb, aux, M, mid_out, C, nullptr, nullptr, status, stream);
+    return gemm_chain2(backward, A, Wa, ba, Wb, bb, aux, M, mid_out, C, nullptr, nullptr, nullptr, status, stream);
 }
 
 int mlcgb_gemm_tc_chain2_tangent(int reverse, const void *A, const void *Wa, const void *Wb, const void *a, const void *gu, const void *aux,
                                  int64_t M, void *q, void *mid_out, void *C, int32_t *status, void *stream) {
-    return gemm_chain2_tangent(reverse, A, Wa, Wb, a, gu, aux, M, q, mid_out, C, nullptr, nullptr, status, stream);
+    return gemm_chain2_tangent(reverse, A, Wa, Wb, a, gu, aux, M, q, mid_out, C, nullptr, nullptr, nullptr, status, stream);
 }
 
 int mlcgb_gemm_tc_tn_colsum(const void *A, const void *B, int64_t K, int64_t M, int64_t N, void *C, void *colsum, void *workspace,

@@ -200,19 +200,19 @@ __global__ void head_out_kernel(const float *__restrict__ a, const float *__rest
 
 // tanh(agg W2^T + b2) -> a,  x + a W3^T + b3 -> out; one kernel where all widths are 128
 static int node_layers_forward(const float *agg, const mlcgb_schnet_block &w, const float *x, int64_t N, int64_t H, int64_t F, int64_t H2, float *a,
-                               float *out, const uint8_t *images, int32_t *status, void *stream) {
+                               float *out, const uint8_t *images, const ChainLink *link, int32_t *status, void *stream) {
     if (H == 128 && F == 128 && H2 == 128)
         return gemm_chain2(0, agg, w.lin2_w, w.lin2_b, w.lin_w, w.lin_b, x, N, a, out, images ? images + kLin2 * kWeightImage : nullptr,
-                           images ? images + kLin * kWeightImage : nullptr, status, stream);
+                           images ? images + kLin * kWeightImage : nullptr, link, status, stream);
     int rc = mlcgb_gemm_tc_fused(0, agg, w.lin2_w, w.lin2_b, nullptr, 1, N, H2, F, a, status, stream);
     return rc ? rc : mlcgb_gemm_tc_fused(0, a, w.lin_w, w.lin_b, x, 2, N, H, H2, out, status, stream);
 }
 // ((g W3) (1 - a^2)) W2 -> gagg
 static int node_layers_backward(const float *g, const mlcgb_schnet_block &w, const float *a, int64_t N, int64_t H, int64_t F, int64_t H2, float *gy,
-                                float *gagg, const uint8_t *images, int32_t *status, void *stream) {
+                                float *gagg, const uint8_t *images, const ChainLink *link, int32_t *status, void *stream) {
     if (H == 128 && F == 128 && H2 == 128)
         return gemm_chain2(1, g, w.lin_w, nullptr, w.lin2_w, nullptr, a, N, nullptr, gagg, images ? images + kLin * kWeightImage : nullptr,
-                           images ? images + kLin2 * kWeightImage : nullptr, status, stream);
+                           images ? images + kLin2 * kWeightImage : nullptr, link, status, stream);
     int rc = mlcgb_gemm_tc_fused(1, g, w.lin_w, nullptr, a, 3, N, H2, H, gy, status, stream);
     return rc ? rc : mlcgb_gemm_tc_fused(1, gy, w.lin2_w, nullptr, nullptr, 0, N, F, H2, gagg, status, stream);
 }
@@ -329,18 +329,25 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
         const mlcgb_schnet_block &bw = w->blocks[l];
         float *blk = ws + lay.block0 + l * lay.block_stride;
         float *xin = ws + lay.x[cur], *xout = ws + lay.x[cur ^ 1], *xl = blk + lay.xl_off, *a = blk + lay.a_off, *agg = ws + lay.agg;
-        rc = gemm_fused(0, xin, bw.lin1_w, nullptr, nullptr, 0, N, F, H, xl, l > 0 ? image(3 * l + kLin1) : nullptr, status, stream);
-        if (rc) return rc;
+        if (l == 0 || !images) {                    // (else it came with the block before)
+            rc = gemm_fused(0, xin, bw.lin1_w, nullptr, nullptr, 0, N, F, H, xl, nullptr, status, stream);
+            if (rc) return rc;
+        }
         if ((rc = filters(l, 1))) return rc;        // (block by block: what is written last is read first, some of it out of the L2)
         rc = mlcgb_seg_mul_sum(xl, ws + lay.W + l * lay.wstride, MLCGB_F32, offsets, row1, pair_of, N, P, F, agg, stream);
         if (rc) return rc;
-        rc = node_layers_forward(agg, bw, xin, N, H, F, H2, a, xout, image(3 * l), status, stream);
+        // what follows on the same rows: the next block's first layer, or the output network's, tanh(x W^T + b)
+        const ChainLink link = l + 1 < L ? ChainLink{image(3 * (l + 1) + kLin1), nullptr, nullptr, nullptr, blk + lay.block_stride + lay.xl_off, 128, 0}
+                                         : ChainLink{image(3 * L), (const float *)w->head_b, nullptr, nullptr, ws + lay.ah, (int)Wh, 1};
+        rc = node_layers_forward(agg, bw, xin, N, H, F, H2, a, xout, image(3 * l), images ? &link : nullptr, status, stream);
         if (rc) return rc;
         cur ^= 1;
     }
     // output network: tanh(x W^T + b) . w_out (+ b_out), summed per structure
-    rc = gemm_fused(0, ws + lay.x[cur], w->head_W, w->head_b, nullptr, 1, N, Wh, H, ws + lay.ah, image(3 * L), status, stream);
-    if (rc) return rc;
+    if (!images) {
+        rc = gemm_fused(0, ws + lay.x[cur], w->head_W, w->head_b, nullptr, 1, N, Wh, H, ws + lay.ah, nullptr, status, stream);
+        if (rc) return rc;
+    }
     {
         TimelineScope timeline_scope("head_out", stream);
         launch_pdl(head_out_kernel, dim3(grid_for(N * 32, 256)), dim3(256), 0, st, (const float *)(ws + lay.ah), (const float *)w->head_out, (const float *)w->head_out_b, N, Wh, ws + lay.en);
@@ -350,13 +357,18 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
     // force pass: d(sum of energies)/d(pos)
     // through the output network: g = (w_out * (1 - a^2)) head_W, the factor applied as the GEMM reads its input tile
     int gcur = 0;
-    rc = gemm_fused(1, ws + lay.ah, w->head_W, nullptr, w->head_out, 4, N, H, Wh, ws + lay.g[gcur], image(3 * L), status, stream);
-    if (rc) return rc;
+    // (with images each block's node layers take the layer before them along, which makes their input g)
+    ChainLink link = {image(3 * L), nullptr, (const float *)w->head_out, nullptr, ws + lay.g[gcur], (int)Wh, 0};
+    if (!images) {
+        rc = gemm_fused(1, ws + lay.ah, w->head_W, nullptr, w->head_out, 4, N, H, Wh, ws + lay.g[gcur], nullptr, status, stream);
+        if (rc) return rc;
+    }
     for (int64_t l = L - 1; l >= 0; l--) {
         const mlcgb_schnet_block &bw = w->blocks[l];
         float *blk = ws + lay.block0 + l * lay.block_stride;
         float *g = ws + lay.g[gcur], *gnext = ws + lay.g[gcur ^ 1], *gagg = ws + lay.agg, *gxl = ws + lay.gxl;
-        rc = node_layers_backward(g, bw, blk + lay.a_off, N, H, F, H2, ws + lay.gy, gagg, image(3 * l), status, stream);
+        rc = node_layers_backward(!images ? g : l == L - 1 ? ws + lay.ah : gxl, bw, blk + lay.a_off, N, H, F, H2, ws + lay.gy, gagg, image(3 * l),
+                                  images ? &link : nullptr, status, stream);
         if (rc) return rc;
         // s[e] of every block adds up in one array: the last block sets it, the others add
         if (l == 0) {
@@ -366,7 +378,8 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
         rc = mlcgb_seg_force(gagg, blk + lay.xl_off, ws + lay.W + l * lay.wstride, ws + lay.Wd + l * lay.wstride, offsets, row1, pair_of, N, F, gxl, ws + lay.gd,
                              l != L - 1, stream);
         if (rc) return rc;
-        if ((rc = gemm_fused(1, gxl, bw.lin1_w, nullptr, g, 2, N, H, F, gnext, image(3 * l + kLin1), status, stream))) return rc;
+        if (!images && (rc = gemm_fused(1, gxl, bw.lin1_w, nullptr, g, 2, N, H, F, gnext, nullptr, status, stream))) return rc;
+        link = {image(3 * l + kLin1), nullptr, nullptr, g, gnext, 128, 0};
         gcur ^= 1;
     }
     return finish_launch((const float *)pos, ws + lay.gp, d, row1, offsets, pair_of, N, (float *)grad_pos, grad_sign, ws + lay.en, struct_ptr, B, (float *)energy, st);

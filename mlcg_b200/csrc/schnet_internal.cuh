@@ -29,10 +29,18 @@ int embedding_launch(const mlcgb_schnet_weights *w, const int64_t *types, int64_
 // gemm_tc.cu: mlcgb_gemm_tc_fused, _chain2 and _chain2_tangent with the images of their weights (NULL: converted by the kernel)
 int gemm_fused(int mode, const void *A, const void *B, const void *bias, const void *aux, int epilogue, int64_t M, int64_t N, int64_t K, void *C,
                const uint8_t *image, int32_t *status, void *stream);
+// A third layer on the same tile (needs the images of all three).  Forward kinds: behind the two, out[M][width] = C image^T + bias, through
+// tanh if wanted.  Backward kinds: in front of them, out = A image + res, A[M][width] replaced by vec (1 - A^2) where vec is given.
+struct ChainLink {
+    const uint8_t *image;
+    const float *bias, *vec, *res;         // NULL: none
+    float *out;
+    int width, tanh;
+};
 int gemm_chain2(int backward, const void *A, const void *Wa, const void *ba, const void *Wb, const void *bb, const void *aux, int64_t M, void *mid_out,
-                void *C, const uint8_t *image_a, const uint8_t *image_b, int32_t *status, void *stream);
+                void *C, const uint8_t *image_a, const uint8_t *image_b, const ChainLink *link, int32_t *status, void *stream);
 int gemm_chain2_tangent(int reverse, const void *A, const void *Wa, const void *Wb, const void *a, const void *gu, const void *aux, int64_t M, void *q,
-                        void *mid_out, void *C, const uint8_t *image_a, const uint8_t *image_b, int32_t *status, void *stream);
+                        void *mid_out, void *C, const uint8_t *image_a, const uint8_t *image_b, const ChainLink *link, int32_t *status, void *stream);
 
 // filter_vd.cu: filter rows and their derivatives of `num_blocks` blocks in one launch.  Block l's rows start at row
 // l * padded_rows(P) of W and Wd, its kept rows (or NULL) at l * mlcgb_filter_hidden_bytes(P) of hs and zs, its zmax at l.

@@ -218,24 +218,32 @@ int mlcgb::schnet_train_forward(const void *pos, const int64_t *types, const int
     for (int64_t l = 0; l < L; l++) {
         const mlcgb_schnet_block &bw = w->blocks[l];
         float *b = blk(l), *xout = l + 1 < L ? blk(l + 1) + o.x : ws + o.block0 + L * o.stride;
-        if ((rc = gemm_fused(0, b + o.x, bw.lin1_w, nullptr, nullptr, 0, N, kH, kH, b + o.xl, l > 0 ? image(3 * l + kLin1) : nullptr, status, stream))) return rc;
+        if ((l == 0 || !images) && (rc = gemm_fused(0, b + o.x, bw.lin1_w, nullptr, nullptr, 0, N, kH, kH, b + o.xl, nullptr, status, stream))) return rc;
         if ((rc = filters(l, 1))) return rc;
         if ((rc = mlcgb_seg_mul_sum(b + o.xl, ws + o.W + l * o.wstride, MLCGB_F32, offsets, row1, pair_of, N, P, kH, b + o.agg, stream))) return rc;
-        if ((rc = gemm_chain2(0, b + o.agg, bw.lin2_w, bw.lin2_b, bw.lin_w, bw.lin_b, b + o.x, N, b + o.a, xout, image(3 * l + kLin2), image(3 * l + kLin), status, stream))) return rc;
+        // (with images the layer that follows on the same rows, the next block's first or the output network's, comes along)
+        const ChainLink link = l + 1 < L ? ChainLink{image(3 * (l + 1) + kLin1), nullptr, nullptr, nullptr, blk(l + 1) + o.xl, (int)kH, 0}
+                                         : ChainLink{image(3 * L), (const float *)w->head_b, nullptr, nullptr, ws + o.ah, (int)Wh, 1};
+        if ((rc = gemm_chain2(0, b + o.agg, bw.lin2_w, bw.lin2_b, bw.lin_w, bw.lin_b, b + o.x, N, b + o.a, xout, image(3 * l + kLin2), image(3 * l + kLin),
+                              images ? &link : nullptr, status, stream)))
+            return rc;
     }
     float *xL = ws + o.block0 + L * o.stride, *ah = ws + o.ah;
-    if ((rc = gemm_fused(0, xL, w->head_W, w->head_b, nullptr, 1, N, Wh, kH, ah, image(3 * L), status, stream))) return rc;
+    if (!images && (rc = gemm_fused(0, xL, w->head_W, w->head_b, nullptr, 1, N, Wh, kH, ah, nullptr, status, stream))) return rc;
     {
         TimelineScope timeline_scope("head_out", stream);
         launch_pdl(head_out_kernel, dim3(grid_for(N * 32, 256)), dim3(256), 0, st, (const float *)ah, (const float *)w->head_out, (const float *)w->head_out_b, N,
                    Wh, ws + o.en);
     }
     // force pass; block l's g is the gradient of its output
-    if ((rc = gemm_fused(1, ah, w->head_W, nullptr, w->head_out, 4, N, kH, Wh, blk(L - 1) + o.g, image(3 * L), status, stream))) return rc;
+    if (!images && (rc = gemm_fused(1, ah, w->head_W, nullptr, w->head_out, 4, N, kH, Wh, blk(L - 1) + o.g, nullptr, status, stream))) return rc;
+    ChainLink link = {image(3 * L), nullptr, (const float *)w->head_out, nullptr, blk(L - 1) + o.g, (int)Wh, 0};      // (the layer in front of a block's, which makes its g)
     for (int64_t l = L - 1; l >= 0; l--) {
         const mlcgb_schnet_block &bw = w->blocks[l];
         float *b = blk(l);
-        if ((rc = gemm_chain2(1, b + o.g, bw.lin_w, nullptr, bw.lin2_w, nullptr, b + o.a, N, b + o.gu, b + o.gagg, image(3 * l + kLin), image(3 * l + kLin2), status, stream))) return rc;
+        if ((rc = gemm_chain2(1, !images ? b + o.g : l == L - 1 ? ah : blk(l + 1) + o.gxl, bw.lin_w, nullptr, bw.lin2_w, nullptr, b + o.a, N, b + o.gu, b + o.gagg,
+                              image(3 * l + kLin), image(3 * l + kLin2), images ? &link : nullptr, status, stream)))
+            return rc;
         if (l == 0) {
             if ((rc = seg_pair_dot(b + o.gagg, b + o.xl, ws + o.Wd, offsets, row1, pair_of, twin, L > 1 ? ws + o.gd : nullptr, N, ws + o.gp, st))) return rc;
             break;
@@ -243,7 +251,8 @@ int mlcgb::schnet_train_forward(const void *pos, const int64_t *types, const int
         if ((rc = mlcgb_seg_force(b + o.gagg, b + o.xl, ws + o.W + l * o.wstride, ws + o.Wd + l * o.wstride, offsets, row1, pair_of, N, kH, b + o.gxl, ws + o.gd, l != L - 1,
                                   stream)))
             return rc;
-        if ((rc = gemm_fused(1, b + o.gxl, bw.lin1_w, nullptr, b + o.g, 2, N, kH, kH, blk(l - 1) + o.g, image(3 * l + kLin1), status, stream))) return rc;
+        if (!images && (rc = gemm_fused(1, b + o.gxl, bw.lin1_w, nullptr, b + o.g, 2, N, kH, kH, blk(l - 1) + o.g, nullptr, status, stream))) return rc;
+        link = {image(3 * l + kLin1), nullptr, nullptr, b + o.g, blk(l - 1) + o.g, (int)kH, 0};
     }
     return finish_launch((const float *)pos, ws + o.gp, d, row1, offsets, pair_of, N, (float *)grad_pos, negate ? -1.f : 1.f, ws + o.en, struct_ptr, B, (float *)energy, st);
 }
@@ -301,32 +310,36 @@ int mlcgb_schnet_train_backward(const int64_t *types, const int64_t *struct_ptr,
             const mlcgb_schnet_block &bw = w->blocks[l];
             const float *f = fblk(l), *xt_in = l > 0 ? blk(l - 1) + v.xt : nullptr;
             float *b = blk(l);
-            if (l > 0 && (rc = gemm_fused(0, xt_in, bw.lin1_w, nullptr, nullptr, 0, N, kH, kH, b + v.xlt, image(3 * l + kLin1), status, stream))) return rc;
+            if (l > 0 && !images && (rc = gemm_fused(0, xt_in, bw.lin1_w, nullptr, nullptr, 0, N, kH, kH, b + v.xlt, nullptr, status, stream))) return rc;
             if ((rc = mlcgb_seg_tangent(l > 0 ? b + v.xlt : nullptr, f + o.xl, fw + o.W + l * o.wstride, fw + o.Wd + l * o.wstride, dd, offsets, row1, pair_of, N, kH, b + v.aggt, stream))) return rc;
+            const ChainLink link = l + 1 < L ? ChainLink{image(3 * (l + 1) + kLin1), nullptr, nullptr, nullptr, blk(l + 1) + v.xlt, (int)kH, 0}
+                                             : ChainLink{image(3 * L), nullptr, nullptr, nullptr, ws + v.yt, (int)Wh, 0};
             if ((rc = gemm_chain2_tangent(0, b + v.aggt, bw.lin2_w, bw.lin_w, f + o.a, f + o.gu, xt_in, N, b + v.q, b + v.at, b + v.xt, image(3 * l + kLin2),
-                                          image(3 * l + kLin), status, stream)))
+                                          image(3 * l + kLin), images ? &link : nullptr, status, stream)))
                 return rc;
         }
         // ---- output network
         const float *ah = fw + o.ah;
         float *yt = ws + v.yt;
-        if ((rc = gemm_fused(0, blk(L - 1) + v.xt, w->head_W, nullptr, nullptr, 0, N, Wh, kH, yt, image(3 * L), status, stream))) return rc;
+        if (!images && (rc = gemm_fused(0, blk(L - 1) + v.xt, w->head_W, nullptr, nullptr, 0, N, Wh, kH, yt, nullptr, status, stream))) return rc;
         {
             TimelineScope timeline_scope("head_grad", stream);
             launch_pdl(head_grad_kernel, dim3(grid_for(N * 32, 256)), dim3(256), 0, st, ah, (const float *)yt, (const float *)w->head_out, (const float *)gE,
                        struct_ptr, N, B, Wh, yb, gy, r);
         }
-        if ((rc = gemm_fused(1, yb, w->head_W, nullptr, nullptr, 0, N, kH, Wh, blk(L - 1) + v.xb, image(3 * L), status, stream))) return rc;
+        if (!images && (rc = gemm_fused(1, yb, w->head_W, nullptr, nullptr, 0, N, kH, Wh, blk(L - 1) + v.xb, nullptr, status, stream))) return rc;
+        ChainLink link = {image(3 * L), nullptr, nullptr, nullptr, blk(L - 1) + v.xb, (int)Wh, 0};
         // ---- and back
         for (int64_t l = L - 1; l >= 0; l--) {
             const mlcgb_schnet_block &bw = w->blocks[l];
             const float *f = fblk(l);
             float *b = blk(l);
-            if ((rc = gemm_chain2_tangent(1, b + v.xb, bw.lin_w, bw.lin2_w, f + o.a, nullptr, nullptr, N, b + v.q, b + v.ub, b + v.agb, image(3 * l + kLin),
-                                          image(3 * l + kLin2), status, stream)))
+            if ((rc = gemm_chain2_tangent(1, !images ? b + v.xb : l == L - 1 ? yb : blk(l + 1) + v.xlb, bw.lin_w, bw.lin2_w, f + o.a, nullptr, nullptr, N, b + v.q,
+                                          b + v.ub, b + v.agb, image(3 * l + kLin), image(3 * l + kLin2), images ? &link : nullptr, status, stream)))
                 return rc;
             if ((rc = mlcgb_seg_tangent(b + v.agb, f + o.gagg, fw + o.W + l * o.wstride, fw + o.Wd + l * o.wstride, dd, offsets, row1, pair_of, N, kH, b + v.xlb, stream))) return rc;
-            if ((rc = gemm_fused(1, b + v.xlb, bw.lin1_w, nullptr, b + v.xb, 2, N, kH, kH, l > 0 ? blk(l - 1) + v.xb : xb0, image(3 * l + kLin1), status, stream))) return rc;
+            if ((l == 0 || !images) && (rc = gemm_fused(1, b + v.xlb, bw.lin1_w, nullptr, b + v.xb, 2, N, kH, kH, l > 0 ? blk(l - 1) + v.xb : xb0, image(3 * l + kLin1), status, stream))) return rc;
+            if (l > 0) link = {image(3 * l + kLin1), nullptr, nullptr, b + v.xb, blk(l - 1) + v.xb, (int)kH, 0};
         }
     }
     // ---- the filter networks
