@@ -391,7 +391,7 @@ gemm_tc_rows_pipe_kernel(const float *__restrict__ A, const float *__restrict__ 
 // it takes 3 here (evaluation of 96 x 268 ragged 556 -> 514 us, step of 256 x 73 1518 -> 1428, evaluation of 512 x 100 1705 -> 1680).
 struct ChainSmem {
     static constexpr int kWa = 0, kWb = 65536, kStage = 131072, kMisc = 196608;
-    static constexpr int kTotal = kMisc + 4096 + 1024;
+    static constexpr int kTotal = kMisc + 4352 + 1024;      // (exchange and four vectors, 4 KB, then barriers)
 };
 
 enum { kChainFwd = 0, kChainBwd = 1, kChainTan = 2, kChainRev = 3 };
@@ -412,7 +412,8 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
     uint8_t *stage = smem + L::kStage;
     float *s_red = reinterpret_cast<float *>(smem + L::kMisc);
     float *s_ba = s_red + 512, *s_bb = s_ba + 128, *s_bc = s_bb + 128;         // biases; s_bc: of the third layer, or its vector
-    uint64_t *s_bar = reinterpret_cast<uint64_t *>(s_bc + 128);
+    float *s_dot = s_bc + 128;
+    uint64_t *s_bar = reinterpret_cast<uint64_t *>(s_dot + 128);
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(s_bar + 3);                // (barriers of the GEMMs, of Wa and of Wb)
     int *s_err = reinterpret_cast<int *>(s_tmem + 1);
 
@@ -430,6 +431,7 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
         if (LINKED) {
             const float *of = BWD ? link.vec : link.bias;
             s_bc[tid] = of && tid < link.width ? of[tid] : 0.f;
+            s_dot[tid] = !BWD && link.dot && tid < link.width ? link.dot_w[tid] : 0.f;
         }
     }
     const uint32_t bar = smem_u32(s_bar);
@@ -634,6 +636,7 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
             __syncthreads();
             await();
             if (next < ntiles) refill(image_a);
+            float dot = 0.f;
             if (col0 < link.width) {
                 float v[32];
                 tmem_ld32(tmem + lane_off + col0, v);
@@ -644,12 +647,19 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
                                            fmaf(v[4 * w + 2], inv, s_bc[col0 + 4 * w + 2]), fmaf(v[4 * w + 3], inv, s_bc[col0 + 4 * w + 3]));
                     if (link.tanh) o = make_float4(tanh_ex2(o.x), tanh_ex2(o.y), tanh_ex2(o.z), tanh_ex2(o.w));
                     *gstage(stage, r, (col0 >> 2) + w) = o;
+                    const float4 u = *reinterpret_cast<const float4 *>(s_dot + col0 + 4 * w);
+                    dot = fmaf(o.x, u.x, fmaf(o.y, u.y, fmaf(o.z, u.z, fmaf(o.w, u.w, dot))));
                 }
             }
+            s_red[qt * 128 + r] = dot;
         }
         tc_fence_before();
         __syncthreads();
-        if (LINKED && !BWD) store_stage(link.out, tile, link.width);
+        if (LINKED && !BWD) {
+            store_stage(link.out, tile, link.width);
+            if (link.dot && qt == 0 && tile * kRows + r < E)
+                link.dot[tile * kRows + r] = (s_red[r] + s_red[128 + r]) + (s_red[256 + r] + s_red[384 + r]) + (link.dot_b ? link.dot_b[0] : 0.f);
+        }
         else store_stage(C, tile, W);
         __syncthreads();                            // the stage is free for the next input tile
         if (next < ntiles) prefetch_tile_to_stage(stage, A, next * kRows, E, in_cols);

@@ -338,7 +338,8 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
         if (rc) return rc;
         // what follows on the same rows: the next block's first layer, or the output network's, tanh(x W^T + b)
         const ChainLink link = l + 1 < L ? ChainLink{image(3 * (l + 1) + kLin1), nullptr, nullptr, nullptr, blk + lay.block_stride + lay.xl_off, 128, 0}
-                                         : ChainLink{image(3 * L), (const float *)w->head_b, nullptr, nullptr, ws + lay.ah, (int)Wh, 1};
+                                         : ChainLink{image(3 * L), (const float *)w->head_b, nullptr, nullptr, ws + lay.ah, (int)Wh, 1, (const float *)w->head_out,
+                                                     (const float *)w->head_out_b, ws + lay.en};
         rc = node_layers_forward(agg, bw, xin, N, H, F, H2, a, xout, image(3 * l), images ? &link : nullptr, status, stream);
         if (rc) return rc;
         cur ^= 1;
@@ -347,8 +348,6 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
     if (!images) {
         rc = gemm_fused(0, ws + lay.x[cur], w->head_W, w->head_b, nullptr, 1, N, Wh, H, ws + lay.ah, nullptr, status, stream);
         if (rc) return rc;
-    }
-    {
         TimelineScope timeline_scope("head_out", stream);
         launch_pdl(head_out_kernel, dim3(grid_for(N * 32, 256)), dim3(256), 0, st, (const float *)(ws + lay.ah), (const float *)w->head_out, (const float *)w->head_out_b, N, Wh, ws + lay.en);
     }

@@ -30,12 +30,14 @@ int embedding_launch(const mlcgb_schnet_weights *w, const int64_t *types, int64_
 int gemm_fused(int mode, const void *A, const void *B, const void *bias, const void *aux, int epilogue, int64_t M, int64_t N, int64_t K, void *C,
                const uint8_t *image, int32_t *status, void *stream);
 // A third layer on the same tile (needs the images of all three).  Forward kinds: behind the two, out[M][width] = C image^T + bias, through
-// tanh if wanted.  Backward kinds: in front of them, out = A image + res, A[M][width] replaced by vec (1 - A^2) where vec is given.
+// tanh if wanted, and dot[M] = out . dot_w + dot_b (the output network's last layer) where dot is given.  Backward kinds: in front of them, out = A image + res, A[M][width] replaced by vec (1 - A^2) where vec is given.
 struct ChainLink {
     const uint8_t *image;
     const float *bias, *vec, *res;         // NULL: none
     float *out;
     int width, tanh;
+    const float *dot_w, *dot_b;            // dot_b NULL: zero
+    float *dot;
 };
 int gemm_chain2(int backward, const void *A, const void *Wa, const void *ba, const void *Wb, const void *bb, const void *aux, int64_t M, void *mid_out,
                 void *C, const uint8_t *image_a, const uint8_t *image_b, const ChainLink *link, int32_t *status, void *stream);

@@ -223,14 +223,15 @@ int mlcgb::schnet_train_forward(const void *pos, const int64_t *types, const int
         if ((rc = mlcgb_seg_mul_sum(b + o.xl, ws + o.W + l * o.wstride, MLCGB_F32, offsets, row1, pair_of, N, P, kH, b + o.agg, stream))) return rc;
         // (with images the layer that follows on the same rows, the next block's first or the output network's, comes along)
         const ChainLink link = l + 1 < L ? ChainLink{image(3 * (l + 1) + kLin1), nullptr, nullptr, nullptr, blk(l + 1) + o.xl, (int)kH, 0}
-                                         : ChainLink{image(3 * L), (const float *)w->head_b, nullptr, nullptr, ws + o.ah, (int)Wh, 1};
+                                         : ChainLink{image(3 * L), (const float *)w->head_b, nullptr, nullptr, ws + o.ah, (int)Wh, 1, (const float *)w->head_out,
+                                                     (const float *)w->head_out_b, ws + o.en};
         if ((rc = gemm_chain2(0, b + o.agg, bw.lin2_w, bw.lin2_b, bw.lin_w, bw.lin_b, b + o.x, N, b + o.a, xout, image(3 * l + kLin2), image(3 * l + kLin),
                               images ? &link : nullptr, status, stream)))
             return rc;
     }
     float *xL = ws + o.block0 + L * o.stride, *ah = ws + o.ah;
     if (!images && (rc = gemm_fused(0, xL, w->head_W, w->head_b, nullptr, 1, N, Wh, kH, ah, nullptr, status, stream))) return rc;
-    {
+    if (!images) {
         TimelineScope timeline_scope("head_out", stream);
         launch_pdl(head_out_kernel, dim3(grid_for(N * 32, 256)), dim3(256), 0, st, (const float *)ah, (const float *)w->head_out, (const float *)w->head_out_b, N,
                    Wh, ws + o.en);
