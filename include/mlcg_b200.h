@@ -108,7 +108,7 @@ int mlcgb_radius_fill_excl(const void *pos, int dtype, const int64_t *ptr, int64
  * outputs with torch and a host read, src/opt_radius/mlcg_opt_radius/radius.cu:236-241,288-292); it exists
  * for callers that may not allocate device memory at the point of the call: a force routine invoked from
  * inside another program's integration loop, a plug-in whose host owns all of the GPU's memory, a thread
- * that must stay off the allocator's locks.  The cell-list scratch is a fixed 9.5 MiB array inside the
+ * that must stay off the allocator's locks.  The cell-list scratch is a fixed 8.5 MiB array inside the
  * library image (every GPU that loads the library holds it until the process exits); the limits are
  * N <= 65536 points and B <= 8192 structures, and larger inputs return MLCGB_E_LIMIT.
  *   deg[N], offsets[N+1] and edge_index[2, capacity] are the caller's; row 0 starts at edge_index, row 1 at

@@ -53,11 +53,12 @@ constexpr int kTransposePair = 4600;   // structures up to this size share an SM
 // layer), 2 by the bit-mask kernels, 0 by the warp kernels.
 struct CellParam { int gx, gy, gz, use_cells, reach, tile, ngroups, pad; };
 
-// Candidates of a stage of the block kernels.  In float64 that leaves an SM seven warps, but the tests are bound by the float64 pipe;
-// with half the stage, and twice the blocks per SM, nearly all blocks went through the filling kernel from 8 A on at 54 cubic
-// Angstrom per point (15 x 4000 points, 8 A: 558 us, now 214; 12 A: 1610, now 384).
-constexpr int kBlkCap = 768;
-constexpr int kHitWords = kBlkCap / 32;                    // block kernels: words of a centre's hit mask
+// Candidates of a stage of the block kernels.  In float64 that leaves an SM eight warps, but the tests are bound by the float64 pipe;
+// with 384, and more blocks per SM, nearly all blocks went through the filling kernel from 8 A on at 54 cubic Angstrom per point
+// (15 x 4000 points, 8 A: 558 us, now 211; 12 A: 1610, now 480).  640: a point's workspace is then as large as in float32.
+template <typename T> struct BlkCap { static constexpr int value = 768; };
+template <> struct BlkCap<double> { static constexpr int value = 640; };
+template <typename T> struct HitWords { static constexpr int value = BlkCap<T>::value / 32; };    // words of a centre's hit mask
 constexpr int kBlkMaxBY = 8;                               // block kernels: rows of cells in a block, at most
 constexpr int kBlkTargetCentres = 24;                      // mean number of centres per block the block's size aims at
 
@@ -85,7 +86,7 @@ static WsLayout ws_layout(int64_t N, int64_t B, int dtype) {
     L.struct_of = o;   o += align256((size_t)N * 4);
     L.bsum = o;        o += align256((size_t)((N + kScanBlock - 1) / kScanBlock + 1) * 8);
     L.group_ptr = o;   o += align256((size_t)(B + 4) * 4);
-    L.hits = o;        o += align256((size_t)N * kHitWords * 4);   // hit words per point
+    L.hits = o;        o += align256((size_t)N * (dtype == MLCGB_F64 ? HitWords<double>::value : HitWords<float>::value) * 4);   // hit words per point
     L.cidx = o;        o += align256((size_t)N * 4);                      // local index of every cell-sorted point (= spos[].w, compact)
     L.item_flag = o;   o += align256((size_t)N);                          // per work item (at most one per cell, cells <= points): 1 = no hit masks
     L.total = o;
@@ -194,7 +195,7 @@ build_cells_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, i
                 // Smaller where its candidates, at the mean density (the last cells of an axis are only partly inside the box), would
                 // not fit a stage: such a block leaves no masks and is tested twice more, in windows, by the filling kernel.  15 x 4000
                 // uniform points at 10.5 A, 24 centres a block and 750 candidates: 609 us, with 15 centres 232; at 12 A 925 and 327.
-                const double most = kBlkCap - 2 * sqrt((double)kBlkCap);
+                const double most = BlkCap<T>::value - 2 * sqrt((double)BlkCap<T>::value);
                 double full = (double)n;
                 for (int a = 0; a < 3; a++) full /= fmax(ext[a] / h, 1.0);
                 auto candidates = [&] {
@@ -709,7 +710,7 @@ __device__ __forceinline__ void write_sources(unsigned short *src, const ItemRun
 
 template <typename T>
 struct CountSmem {
-    static constexpr int kCap = kBlkCap;
+    static constexpr int kCap = BlkCap<T>::value;
     static constexpr size_t cand = 0;                                         // V4<T>[kCap]: staged candidates
     static constexpr size_t src = cand + (size_t)kCap * sizeof(V4<T>);        // u16[kCap]: where the candidates of a stage come from
     static constexpr size_t ssrc = src + (size_t)kCap * 2;                    // u16[kCap]: the same in ascending order of index
@@ -774,14 +775,14 @@ __device__ __forceinline__ void mark_and_rank(const int32_t *__restrict__ ci, co
 // under the neighbour-cap rule comes from the same words (hits before / after the centre's own place).  An item with more
 // candidates is counted in windows, as they come, sets the flag word after the work-item prefix and leaves no masks.
 template <typename T>
-__global__ void __launch_bounds__(32, 12)                  // (shared memory allows 12 one-warp blocks per SM, in float64 7)
+__global__ void __launch_bounds__(32, 12)                  // (shared memory allows 12 one-warp blocks per SM, in float64 8)
 neighbours_block_count_kernel(const int64_t *__restrict__ ptr, int64_t B, T r2, int64_t max_nn, int loop, int rule,
                               const V4<T> *__restrict__ spos, const CellParam *__restrict__ cellparam,
                               const int32_t *__restrict__ cell_start, int32_t *__restrict__ group_ptr, int32_t *__restrict__ deg,
                               const int32_t *__restrict__ cidx, unsigned *__restrict__ hits, unsigned char *__restrict__ item_flag,
                               int32_t *__restrict__ status, int32_t *__restrict__ upper /* or NULL */) {
     using S = CountSmem<T>;
-    constexpr int kCap = S::kCap, kPerLane = kCap / 32, kWords = kHitWords;
+    constexpr int kCap = S::kCap, kPerLane = kCap / 32, kWords = HitWords<T>::value;
     extern __shared__ __align__(32) unsigned char blk_smem[];
     const int lane = threadIdx.x;
     V4<T> *cand = reinterpret_cast<V4<T> *>(blk_smem + S::cand);
@@ -995,7 +996,7 @@ constexpr int kFillListStride = kFillList + 2;             // (in 16-bit entries
 
 template <typename T>
 struct FillSmem {
-    static constexpr int kCap = kBlkCap;
+    static constexpr int kCap = BlkCap<T>::value;
     static constexpr size_t cand = 0;                                          // V4<T>[kCap]: staged candidates, ascending
     static constexpr size_t hits = cand + (size_t)kCap * sizeof(V4<T>);        // u16[kFillWarps][32][kFillListStride]
     static constexpr size_t hits_bytes = (size_t)kFillWarps * 32 * kFillListStride * 2;
@@ -1314,7 +1315,7 @@ constexpr int kExpListStride = kExpList + 2;               // (16-bit entries: a
 
 template <typename T>
 struct ExpandSmem {
-    static constexpr int kCap = kBlkCap;
+    static constexpr int kCap = BlkCap<T>::value;
     static constexpr size_t sidx = 0;                                          // u16[kCap]: the candidates' local indices, ascending
     static constexpr size_t src = sidx + (size_t)kCap * 2;                     // u16[kCap]: where the candidates come from
     static constexpr size_t mask = src + (size_t)kCap * 2;                     // u32[kCapBits / 32]
@@ -1336,7 +1337,7 @@ neighbours_block_expand_kernel(const T *__restrict__ pos, const int64_t *__restr
                                const int32_t *__restrict__ cidx, const unsigned *__restrict__ hits, const int64_t *__restrict__ offsets,
                                FillOut out) {
     using S = ExpandSmem<T>;
-    constexpr int kCap = S::kCap, kWords = kHitWords;
+    constexpr int kCap = S::kCap, kWords = HitWords<T>::value;
     extern __shared__ __align__(32) unsigned char blk_smem[];
     const int lane = threadIdx.x;
     unsigned short *src = reinterpret_cast<unsigned short *>(blk_smem + S::src);
@@ -2149,7 +2150,7 @@ int mlcgb_pair_index(const int32_t *sel, const int32_t *twin, int64_t P, int32_t
 namespace mlcgb {
 constexpr int64_t kStaticMaxPoints = 65536;
 constexpr int64_t kStaticMaxStructures = 8192;
-constexpr size_t kStaticScratchBytes = (size_t)19 << 19;  // 9.5 MB >= ws_layout(65536, 8192, float64).total = 9 831 424 (float32: 8 782 848)
+constexpr size_t kStaticScratchBytes = (size_t)17 << 19;  // 8.5 MB >= ws_layout(65536, 8192).total = 8 782 848
 static __device__ __align__(256) unsigned char g_radius_scratch[kStaticScratchBytes];
 
 constexpr int kMaxDevices = 64;
