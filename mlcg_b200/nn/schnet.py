@@ -44,6 +44,9 @@ class _Layers:
         self._children = [m._modules for m in modules if m._modules]
         self._found = [child for c in self._children for child in c.values()]
         self._states = [m.__dict__ for m in modules if m is not net]       # (its own would tie a knot: `net` holds this object)
+        # (a tanh has no mode; the one in the default arguments is shared by every model made with them: a model in training took the others
+        # off their one-call route, 512 x 100 beads 1.65 -> 2.53 ms)
+        self._modes = [m.__dict__ for m in modules if m is not net and type(m) is not torch.nn.Tanh]
         basis = net.rbf_layer
         self._basis = [m._parameters for m in _all_modules(basis)]
         self._basis_tensors = (basis._parameters, basis._buffers)
@@ -71,7 +74,7 @@ class _Layers:
 
     def in_mode(self, training: bool) -> bool:
         """Whether all modules are in the same mode as the model (each takes its weights as constants or not by its own)."""
-        return all([d["training"] is training for d in self._states])
+        return all([d["training"] is training for d in self._modes])
 
     def trained_basis(self) -> bool:
         return any([t is not None and t.requires_grad for p in self._basis for t in p.values()])

@@ -439,3 +439,15 @@ def test_native_descriptions_of_tensors():
     assert torch.equal(torch.cat([g.flatten() for g in got]), flat)
     with pytest.raises(TypeError):
         n.pointers([3])
+
+
+def test_a_shared_activation_has_no_mode():
+    """Models made with the default arguments share their activation: one of them in training leaves the others in their own mode."""
+    def make():
+        cut = bnn.CosineCutoff(0.0, 8.0)
+        return bnn.StandardSchNet(bnn.GaussianBasis(cut, 20, trainable=False), cut, [128], embedding_size=4, num_interactions=2)
+    a, b = make().eval(), make().train()
+    assert a.interaction_blocks[0].activation is b.interaction_blocks[0].activation
+    assert a._layers().in_mode(False) and b._layers().in_mode(True)
+    a.interaction_blocks[1].conv.lin1.train()
+    assert not a._layers().in_mode(False)
