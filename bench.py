@@ -668,11 +668,15 @@ def kernel_work(name, E, P, N, F, R):
         return P * (8 * F + 4), 4 * E * F * (R + F)
     if name == "seg_mul_sum":           # one filter row per pair, neighbour index and pair index per edge, node rows in and out
         return P * F * 4 + 8 * E + 2 * N * F * 4 + 8 * N, 2 * E * F
-    if name == "seg_force":             # mean of its launches: a filter and a derivative row per pair (the first block's dot product: the latter
-        #                                 alone), two indices and a dot product per edge (read too where it adds), two node rows in, one out
+    if name == "seg_force":             # a filter and a derivative row per pair, two indices and a dot product per edge (read too where it adds:
+        #                                 in all blocks but the last), two node rows in, one out
         L = WORKLOAD["interactions"]
-        rows, nodes, dots = (2 * L - 1) / L, (3 * L - 1) / L, (2 * L - 1) / L
-        return rows * P * F * 4 + (8 + 4 * dots) * E + nodes * N * F * 4 + 8 * N, (4 * L - 2) / L * E * F
+        dots = (2 * L - 3) / (L - 1)
+        return 2 * P * F * 4 + (8 + 4 * dots) * E + 3 * N * F * 4 + 8 * N, 4 * E * F
+    if name == "seg_pair_dot":          # the first block's: a derivative row, three indices and two dot products per pair in, one out; two node rows in
+        return P * (F * 4 + 24) + 2 * N * F * 4 + 8 * N, 4 * E * F
+    if name == "gemm_tc_chain2":        # three node layers on a tile: three node rows in, two out (or the other way round), three weights
+        return (5 * N * F + 3 * F * F) * 4, 6 * N * F * F
     if name.startswith("gemm_tc"):      # node-sized Linear layers, 128 wide
         return (2 * N * F + F * F) * 4, 2 * N * F * F
     if name == "radius_graph_capacity":
@@ -961,12 +965,12 @@ def run_ours(args):
     # kernels of the library per evaluation on the route the timed region takes (one library call for the model): radius graph 12
     # (structure boundaries, cells, work-item scan, count by the block kernel and by the warp kernel, three scan kernels, clamp to
     # the capacity, fill by the expanding kernel, the testing block kernel and the warp kernel), reverse-edge map / pair selection /
-    # pair index 5 (count of upper edges, three scan kernels, plan), distances 1, embedding 1, four per block forward (lin1, filter
-    # values and derivatives, aggregation, the two chained layers), output network 2 (layer + tanh, dot product), its derivative 1,
-    # three per block backward (chained layers, aggregation with the distance gradients, lin1 with the residual; two for the first
-    # block, whose input gradient nobody needs), forces and per-structure energies 1
+    # pair index 5 (count of upper edges, three scan kernels, plan), distances 1, embedding and weight tiles 1, lin1 of the first
+    # block 1, three per block forward (filter values and derivatives, aggregation, node layers up to the next block's lin1 or the
+    # output network), two per block backward (node layers, aggregation with the distance gradients or dot products alone), forces and
+    # per-structure energies 1
     L = WORKLOAD["interactions"]
-    launches_timed = args.steps * (12 + 5 + 1 + 1 + 4 * L + 2 + 1 + 3 * (L - 1) + 2 + 1)
+    launches_timed = args.steps * (12 + 5 + 1 + 1 + 1 + 3 * L + 2 * L + 1)
     value = world * B * args.steps / (ms_total / 1e3)
     h2d = pos_h.numel() * 4 + types_h.numel() * 8 + batch_h.numel() * 8
     d2h = B * 4 + pos_h.numel() * 4
