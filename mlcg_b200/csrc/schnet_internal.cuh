@@ -61,11 +61,11 @@ int filter_wgrad_parts(int64_t P, int64_t num_blocks);      // partial sums per 
 
 // small_route.cu: see there.  All widths 128 but the output network's.
 // 148 SMs x 16 rows: two passes of eight rows per SM.  Chains of 100 beads, three blocks, 12 A, us, this route : the tensor-core
-// kernels, a replayed evaluation and the kernels of a force-matching step (timed launch by launch),
-//   beads       600        1200       2000       2400       3200       4000       6400
-//   evaluation  107 : 234  159 : 249  198 : 263  253 : 280  297 : 311  355 : 305  515 : 385
-//   step        145 : 379  203 : 399  236 : 408  271 : 410  301 : 432  368 : 468  527 : 532
-// The line lies where a third pass begins; the routes meet at about 3500 beads for the evaluation and 6400 for the step.
+// kernels, an evaluation and the kernels of a force-matching step,
+//   beads       1200       2000       2400       3200       4000
+//   evaluation  146 : 198  164 : 209  217 : 224  258 : 250  322 : 258
+//   step        407 : 525  493 : 566  570 : 590  660 : 647  803 : 696
+// The line lies where a third pass begins; the routes meet at about 2800 beads.
 constexpr int64_t kSmallNodes = 2368;
 struct SmallForward {                      // per node unless said otherwise; NULL: not wanted
     const float *pos;
