@@ -414,6 +414,7 @@ prior_gather_kernel(const int64_t *__restrict__ mapping, int64_t M, const int64_
     int runs = 0;
     uint64_t diff = 0;
     const int64_t t0 = (int64_t)blockIdx.x * kChunk + threadIdx.x;
+    const auto written = [&](int64_t bead) { return bead < 0 || bead >= N ? -1 : (int32_t)bead; };
 #pragma unroll 4
     for (int u = 0; u < kGatherTerms; u++) {
         const int64_t t = t0 + u * kGatherThreads;
@@ -421,14 +422,16 @@ prior_gather_kernel(const int64_t *__restrict__ mapping, int64_t M, const int64_
         int64_t at[ORDER], entry = 0;
 #pragma unroll
         for (int o = 0; o < ORDER; o++) at[o] = mapping[(int64_t)o * M + t];
-        if (PAIR) runs += t == 0 || mapping[t - 1] != at[0];
+        // (by what is written, where run_starts_kernel looks for them: neighbouring beads that do not exist are one run)
+        if (PAIR) runs += t == 0 || written(mapping[t - 1]) != written(at[0]);
 #pragma unroll
         for (int o = 0; o < ORDER; o++) {
-            if (at[o] < 0 || at[o] >= N) {                   // (reported, and again by the evaluation, which leaves the term out)
+            const int32_t bead = written(at[o]);
+            if (bead < 0) {                                  // (reported, and again by the evaluation, which leaves the term out)
                 atomicOr(status, (int)kBadIndex);
                 at[o] = -1;
             }
-            idx[(int64_t)o * M + t] = (int32_t)at[o];
+            idx[(int64_t)o * M + t] = bead;
         }
         if (!given) {
 #pragma unroll

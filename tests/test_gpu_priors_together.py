@@ -150,3 +150,24 @@ def test_a_bead_that_does_not_exist_is_reported():
     status = be._sticky_status(torch.device(DEV))
     assert int(status[0]) & 2
     status.zero_()
+
+
+@pytest.mark.parametrize("there,missing", [(36, 64), (33, 31), (100, 1), (0, 64)])
+def test_run_starts_of_a_list_for_a_longer_chain(there, missing):
+    """A complete pair list over beads of which the last ones do not exist: as many run starts as runs are counted, and each where the
+    written list has one (looked at on the host before anything reads through them); no slices."""
+    from mlcg_b200.backend import get_backend
+    be, n = get_backend(), there + missing
+    i = torch.arange(n)
+    pairs = torch.cartesian_prod(i, i).t()
+    pairs = pairs[:, pairs[0] != pairs[1]].contiguous().to(DEV)
+    types, table = torch.zeros(max(there, 1), dtype=torch.int64, device=DEV), torch.ones(1, 1, device=DEV)
+    idx, params, symmetric, starts = be.prior_list(pairs, types, [table], None, there, True)
+    first = idx[0].cpu()
+    assert torch.equal(first, torch.where(pairs[0] < there, pairs[0], -1).cpu().to(torch.int32))
+    heads = [0] + (torch.nonzero(first[1:] != first[:-1]).flatten() + 1).tolist()
+    assert symmetric and starts.tolist() == heads and len(heads) == there + 1
+    assert _pair_slices(idx, params, starts) is None
+    status = be._sticky_status(torch.device(DEV))
+    assert int(status[0]) & 2
+    status.zero_()
