@@ -1083,6 +1083,8 @@ class CudaBackend:
         _need_cuda(mapping, types, params, *(tables or ()))
         mapping, types = mapping.contiguous(), types.contiguous()
         order, M = mapping.shape
+        if tables is not None:
+            n_beads = min(n_beads, types.numel())        # (a bead without a type is one that does not exist)
         dev, like = mapping.device, params if tables is None else tables[0]
         if tables is None:
             params, P, kinds = params.contiguous(), params.shape[0], 1

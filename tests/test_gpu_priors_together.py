@@ -171,3 +171,37 @@ def test_run_starts_of_a_list_for_a_longer_chain(there, missing):
     status = be._sticky_status(torch.device(DEV))
     assert int(status[0]) & 2
     status.zero_()
+
+
+@pytest.mark.parametrize("order,pairs", [(2, True), (2, False), (3, False), (4, False)])
+def test_types_that_end_before_the_beads_do(order, pairs):
+    """Beads past the end of the types are reported and left out; nothing is looked up behind the types."""
+    from mlcg_b200.backend import get_backend
+    be, n, typed = get_backend(), 40, 7
+    mapping = torch.randint(0, typed, (order, 500), generator=torch.Generator().manual_seed(order)).to(DEV)
+    mapping[order - 1, 100:] = torch.arange(400, device=DEV) % n
+    types = torch.zeros(n, dtype=torch.int64, device=DEV)[:typed].clone()
+    tables = [torch.full((1,) * order, 3.0, device=DEV)]
+    idx, params, _, _ = be.prior_list(mapping, types, tables, None, n, pairs)
+    assert torch.equal(idx.long(), torch.where(mapping < typed, mapping, -1)) and torch.equal(params, torch.full_like(params, 3.0))
+    status = be._sticky_status(torch.device(DEV))
+    assert int(status[0]) & 2
+    status.zero_()
+
+
+def test_a_list_is_made_again_for_more_beads():
+    """A list first met with beads missing is not kept for the call that has them."""
+    data, priors = prior_setup(40, 2, 4, torch.Generator().manual_seed(4))
+    data, p = data.to(DEV), priors["repulsion"].to(DEV).eval()
+    data.pos = torch.cat([random_walk_chain(40, torch.Generator().manual_seed(5), min_dist=3.0) for _ in range(2)]).float().to(DEV)
+    want, pos, batch = _evaluate_together([p], data, forces=True)[0]["repulsion"], data.pos, data.batch
+    p.__dict__.pop("_mlcgb_list")
+    data.pos, data.batch = pos[:60], batch[:60]
+    _evaluate_together([p], data, forces=True)
+    from mlcg_b200.backend import get_backend
+    status = get_backend()._sticky_status(torch.device(DEV))
+    assert int(status[0]) & 2
+    status.zero_()
+    data.pos, data.batch = pos, batch
+    got = _evaluate_together([p], data, forces=True)[0]["repulsion"]
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and int(status[0]) == 0
