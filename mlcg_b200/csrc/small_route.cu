@@ -767,17 +767,18 @@ static int small_configure(Kern kern, size_t bytes, bool *done) {
 }
 
 template <int KIND, int RT>
-static int small_launch_rt(const SmallNet &p, cudaStream_t st) {
+static int small_launch_rt(const SmallNet &p, bool early, cudaStream_t st) {
     static bool done[64] = {false};
     if (int rc = small_configure(small_block_kernel<KIND, RT>, SmallSmem<RT>::kBytes, done)) return rc;
     const int64_t tiles = (p.N + RT - 1) / RT;
-    launch_with_weights(small_block_kernel<KIND, RT>, dim3((unsigned)(tiles < kNumSM ? tiles : kNumSM)), dim3(kST), SmallSmem<RT>::kBytes, st, p);
+    launch_early(early, small_block_kernel<KIND, RT>, dim3((unsigned)(tiles < kNumSM ? tiles : kNumSM)), dim3(kST), SmallSmem<RT>::kBytes, st, p);
     return check_launch();
 }
 template <int KIND>
-static int small_launch(const SmallNet &p, cudaStream_t st) {
+static int small_launch(const SmallNet &p, cudaStream_t st, bool early = true) {
     TimelineScope timeline_scope("small_block", st);
-    return p.N <= 4 * kNumSM ? small_launch_rt<KIND, 4>(p, st) : small_launch_rt<KIND, 8>(p, st);
+    early = early && g_chain_depth > 0;                                // (weights are read before the wait, as launch_with_weights() has it)
+    return p.N <= 4 * kNumSM ? small_launch_rt<KIND, 4>(p, early, st) : small_launch_rt<KIND, 8>(p, early, st);
 }
 
 int small_start(const SmallForward &f, cudaStream_t st) {
@@ -839,16 +840,19 @@ int small_forward(const SmallForward &f, cudaStream_t st) {
         p.o_agg = f.agg[l];
         p.o_act = f.a[l];
         p.o_x = f.x[l + 1];
+        // The lists are read before the wait, which is sound behind a kernel that has waited for those that made them: the filters, or a
+        // link.  Lists without room for an edge have no filters, and the first link would stand behind the kernel that writes the offsets.
+        const bool early = l > 0 || f.E > 0;
         if (l + 1 < L) {
             p.o_next = f.xl[l + 1];
-            if (int rc = small_launch<kSmFwd>(p, st)) return rc;
+            if (int rc = small_launch<kSmFwd>(p, st, early)) return rc;
         } else {
             p.o_ah = f.ah;
             p.o_en = f.en;
             p.o_g = f.g[l];
             p.o_gu = f.gu[l];
             p.o_gagg = f.want_grad ? f.gagg[l] : nullptr;
-            if (int rc = small_launch<kSmFwdLast>(p, st)) return rc;
+            if (int rc = small_launch<kSmFwdLast>(p, st, early)) return rc;
         }
     }
     for (int64_t l = L - 1; l > 0 && f.want_grad; l--) {

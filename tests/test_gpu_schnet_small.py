@@ -247,3 +247,34 @@ def test_distances_on_both_sides_of_the_basis_that_is_zero(basis, num_rbf, upper
         assert torch.allclose(e, e_x, rtol=E_RTOL, atol=E_RTOL * float(e_x.abs().max())) and float((f - f_x).abs().max()) < F_ATOL
     else:
         assert float((f - f_x).norm() / f_x.norm()) < 1e-2
+
+
+@pytest.mark.parametrize("sizes,box,edges", [([1, 1, 1], 1.0, 0), ([4, 3], 3.0, 18), ([600, 1, 700], 3000.0, None), ([2048], 6000.0, None)])
+def test_lists_without_room_for_an_edge(sizes, box, edges):
+    """A fixed capacity of 0: beads alone get their energies, and every edge is reported.  Between the calls the workspaces hold lists of
+    another batch, so that a link which reads them too early would read those."""
+    import ctypes
+    torch.manual_seed(0)
+    cut = bnn.CosineCutoff(0.0, 6.0)
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, 32, trainable=False), cut, [128], embedding_size=5, num_interactions=2).eval().to(DEV)
+    be, lib, n, gen = get_backend(), get_backend().lib, sum(sizes), torch.Generator().manual_seed(7)
+    pos, types_ = (torch.rand(n, 3, generator=gen) * box).to(DEV), torch.randint(0, 5, (n,), generator=gen).to(DEV)
+    n_atoms = torch.tensor(sizes, device=DEV)
+    spec, conv_cut, (w, _keep), precision = net._whole_model_setup(pos)
+    s, keep = be._spec(spec, torch.float32)
+    size = lib.mlcgb_schnet_evaluate_workspace_bytes
+    gb, wsb = size(n, len(sizes), -1, 0, ctypes.byref(w), 0), size(n, len(sizes), 0, spec.num_rbf, ctypes.byref(w), 0)
+    status, per_type = be._sticky_status(torch.device(DEV)), None
+    alone = bnn.GradientsOut(net, "forces").eval()(mlcg_b200.AtomicData(pos=torch.arange(5, device=DEV)[:, None] * torch.full((1, 3), 50.0, device=DEV), atom_types=torch.arange(5, device=DEV),
+                                                                      batch=torch.arange(5, device=DEV), n_atoms=torch.ones(5, dtype=torch.int64, device=DEV)))
+    per_type = alone.out["SchNet"]["energy"]
+    want = torch.zeros(len(sizes), device=DEV).index_add_(0, torch.repeat_interleave(torch.arange(len(sizes), device=DEV), n_atoms), per_type[types_])
+    for fill in (0, 1, 0x7f):
+        graph_ws, ws = (torch.full((b,), fill, dtype=torch.uint8, device=DEV) for b in (gb, wsb))
+        energy, grad = torch.empty(len(sizes), device=DEV), torch.empty(n, 3, device=DEV)
+        code = lib.mlcgb_schnet_evaluate_fixed(pos.data_ptr(), types_.data_ptr(), n_atoms.data_ptr(), None, n, len(sizes), 6.0, 1000, ctypes.byref(s), conv_cut[0],
+                                               conv_cut[1], conv_cut[2], ctypes.byref(w), precision, 1, 0, None, graph_ws.data_ptr(), gb, ws.data_ptr(), wsb,
+                                               energy.data_ptr(), grad.data_ptr(), status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert code == 0 and int(status[0]) == (32 if edges else 0)
+        status.zero_()
+        assert torch.allclose(energy, want, rtol=1e-5, atol=1e-5 * float(want.abs().max())) and not grad.any()
