@@ -483,19 +483,30 @@ class SchNet(torch.nn.Module):
                                          want_grad=True, forces=forces)
 
     def _from_positions(self, data, setup, forces, training=False):
-        """Graph and evaluation in one call, its workspace sized by the edges per bead of the call before and a margin (a size only:
-        a call that needs more says so and is continued): ``(energy, gradient or forces, training state)`` or None."""
+        """Graph and evaluation in one call: ``(energy, gradient or forces, training state)`` or None.  The workspace is sized by the edges
+        per bead of calls before, a size only: a call that needs more says so and is made again.  For a batch whose graph is made inside the
+        evaluation (up to 2048 beads) that is a whole evaluation, so it takes the most that any such call had and a quarter: one model on
+        four batches of 35 to 268 beads a chain in turn took 137 us each by the call before (117 with the graph in front of the
+        evaluation), like this 90.  Others have only counted their edges by then and go by the call before, their workspaces being large."""
         if data.pos.shape[1] != 3:
             return None
         n_atoms, ptr = sizes_or_pointer(data)
-        N, seen = data.pos.shape[0], self.__dict__.get("_mlcgb_edges_per_bead", 0.0)
-        if not seen and not training and N <= 2048:       # (nothing to go by: every bead sees its whole structure, or forty others)
+        N, kept = data.pos.shape[0], self.__dict__
+        inside = not training and N <= 2048
+        seen = kept.get("_mlcgb_edges_per_bead", 0.0)
+        if not inside:
+            seen = kept.get("_mlcgb_edges_per_bead_large", seen)
+        elif not seen:                                    # (nothing to go by: every bead sees its whole structure, or forty others)
             seen = min((N - 1) / (ptr.numel() - 1 if n_atoms is None else max(n_atoms.numel(), 1)), 40.0)
+        room = (1.25 if inside else 1.03) * seen * N + 64 if seen else 0
         res = get_backend().schnet_from_positions(data.pos, self._types(data), n_atoms, ptr, float(self.rbf_layer.cutoff.cutoff_upper),
-                                                  int(self.max_num_neighbors), *setup, forces, 1.03 * seen * N + 64 if seen else 0, training)
+                                                  int(self.max_num_neighbors), *setup, forces, room, training)
         if res is None:
             return None
-        self.__dict__["_mlcgb_edges_per_bead"] = res[2] / N
+        if inside:
+            kept["_mlcgb_edges_per_bead"] = max(kept.get("_mlcgb_edges_per_bead", 0.0), res[2] / N)
+        else:
+            kept["_mlcgb_edges_per_bead_large"] = res[2] / N
         return res[0], res[1], res[3]
 
     def energy_and_forces_training(self, data):

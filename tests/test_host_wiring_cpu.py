@@ -451,3 +451,33 @@ def test_a_shared_activation_has_no_mode():
     assert a._layers().in_mode(False) and b._layers().in_mode(True)
     a.interaction_blocks[1].conv.lin1.train()
     assert not a._layers().in_mode(False)
+
+
+def test_room_for_the_edges_of_proteins_in_turn(golden, monkeypatch):
+    """Small batches of different density, one after another by one model: each is asked for with too little room once at most, a denser
+    protein in between or not; large batches and training steps go by the call before, whatever the small ones had."""
+    net = schnet_from_case(golden["schnet_expnormal_f32"])
+    asked = []
+
+    def from_positions(pos, types, n_atoms, ptr, r, most, forces, edges, training):
+        asked.append(edges)
+        return None, None, per_bead * pos.shape[0], None
+
+    monkeypatch.setattr(backend._backend, "schnet_from_positions", from_positions, raising=False)
+
+    def call(n, training=False):
+        data = mlcg_b200.AtomicData(pos=torch.zeros(n, 3), atom_types=torch.zeros(n, dtype=torch.long), n_atoms=torch.tensor([n]))
+        net._from_positions(data, (), True, training)
+        return asked[-1] >= per_bead * n
+
+    missed = 0
+    for _ in range(3):
+        for n, per_bead in ((73, 36.0), (160, 58.0), (35, 20.0), (268, 71.0), (1000, 71.0 * 1.24), (10, 9.0)):
+            missed += not call(n)
+    assert missed == 1                       # (58 a bead when they were new)
+    for n, training in ((5000, False), (5000, False), (500, True)):
+        per_bead = 12.0
+        call(n, training)
+    assert asked[-2] == 1.03 * 12.0 * 5000 + 64 and asked[-1] == 1.03 * 12.0 * 500 + 64
+    per_bead = 80.0
+    assert call(1000)
