@@ -1680,18 +1680,15 @@ __global__ void pair_plan_kernel(const int32_t *__restrict__ row0, const int32_t
             continue;
         }
         twin[e] = t;
-        if (b > a) {
-            const int64_t p = uoff[a] + (e - (offsets[a + 1] - upper[a]));
-            if (p >= (nE >> 1)) {              // more upper than lower edges: not symmetric
-                atomicOr(status, (int)kAsymmetric);
-                pair_of[e] = 0;
-                continue;
-            }
-            sel[p] = (int32_t)e;
-            pair_of[e] = (int32_t)p;
-        } else {
-            pair_of[e] = (int32_t)(uoff[b] + (t - (offsets[b + 1] - upper[b])));
+        const int up = b > a ? a : b;          // the row that holds the pair's upper edge, in its tail
+        const int64_t p = uoff[up] + ((b > a ? e : t) - (offsets[up + 1] - upper[up]));
+        if (p < 0 || p >= (nE >> 1)) {         // a row out of order, or more upper than lower edges: not symmetric
+            atomicOr(status, (int)kAsymmetric);
+            pair_of[e] = 0;
+            continue;
         }
+        if (b > a) sel[p] = (int32_t)e;
+        pair_of[e] = (int32_t)p;
     }
 }
 

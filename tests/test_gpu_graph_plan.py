@@ -126,3 +126,44 @@ def test_bit_rows_of_whole_batches(sizes, dtype):
         # (the cluster rule counts the point itself among its cap + 1: a list is cut short where it lost somebody)
         assert bool(res["status"] & 1) == (cut.shape[1] < want.shape[1] + (len(pos) if loop else 0))
     be.check_pending()
+
+
+@pytest.mark.parametrize("how", ["rows shuffled", "rows reversed", "cut in the middle", "upper halves alone", "other centres"])
+def test_a_list_without_a_plan_is_reported_and_stays_inside(how):
+    """mlcgb_pair_plan of lists that are not what it takes: status bit 2, and every entry is an index, none of it outside the arrays."""
+    be, n, gen = get_backend(), 300, torch.Generator().manual_seed(3)
+    pos = (torch.rand(n, 3, generator=gen) * 12).to(DEV)
+    ref = be.radius_graph(pos, torch.tensor([0, n], device=DEV), 4.0, 1000, False, 1)
+    row0, row1, offsets = ref["row0"].cpu(), ref["row1"].cpu(), ref["offsets"].cpu()
+    ends = offsets.tolist()
+    if how == "rows shuffled":
+        row1 = torch.cat([row1[a:b][torch.randperm(b - a, generator=gen)] for a, b in zip(ends, ends[1:])])
+    elif how == "rows reversed":
+        row1 = torch.cat([row1[a:b].flip(0) for a, b in zip(ends, ends[1:])])
+    elif how == "cut in the middle":
+        keep = ends[n // 2] // 2 * 2
+        row0, row1, offsets = row0[:keep], row1[:keep], offsets.clamp(max=keep)
+    elif how == "upper halves alone":
+        up = row0 < row1
+        row0, row1 = row0[up], row1[up]
+        offsets = torch.cat([torch.zeros(1, dtype=torch.int64), torch.bincount(row0.long(), minlength=n).cumsum(0)])
+        if row0.numel() % 2:
+            row0, row1, offsets = row0[:-1], row1[:-1], offsets.clamp(max=row0.numel() - 1)
+    else:
+        row0 = row0.flip(0)
+    E = row0.numel()
+    rows, offsets = torch.stack([row0, row1]).contiguous().to(DEV), offsets.to(DEV)
+    guard, mark = 4096, -7
+    sizes = (E, E // 2, E)
+    bufs = [torch.full((guard + k + guard,), mark, dtype=torch.int32, device=DEV) for k in sizes]
+    for b, k in zip(bufs, sizes):
+        b[guard:guard + k] = 0
+    status, wsb = torch.zeros(4, dtype=torch.int32, device=DEV), be.lib.mlcgb_pair_plan_workspace_bytes(n)
+    ws = torch.empty(wsb, dtype=torch.uint8, device=DEV)
+    assert be.lib.mlcgb_pair_plan(rows[0].data_ptr(), rows[1].data_ptr(), offsets.data_ptr(), E, n, ws.data_ptr(), wsb, *(b[guard:].data_ptr() for b in bufs),
+                                  status.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    assert int(status[0]) & 4
+    for b, k, most in zip(bufs, sizes, (E, E, E // 2)):
+        inside = b[guard:guard + k]
+        assert int(inside.min()) >= 0 and int(inside.max()) < most
+        assert bool((b[:guard] == mark).all()) and bool((b[guard + k:] == mark).all())
