@@ -19,7 +19,7 @@ from typing import Optional
 
 import torch
 
-from .backend import RbfSpec, get_backend
+from .backend import RbfSpec, get_backend, lasting
 
 
 @dataclass
@@ -48,7 +48,8 @@ class EdgePlan:
             return None
         if self._half is None:
             # exactly E/2 edges have row0 < row1, so the size is known without reading the device
-            self._half = torch.nonzero_static(self.row0 < self.row1, size=self.E // 2).flatten().to(torch.int32)
+            with lasting():
+                self._half = torch.nonzero_static(self.row0 < self.row1, size=self.E // 2).flatten().to(torch.int32)
         return self._half
 
     def pair_index(self) -> Optional[torch.Tensor]:
@@ -57,7 +58,8 @@ class EdgePlan:
         if sel is None:
             return None
         if self._pair_of is None:
-            self._pair_of = get_backend().pair_index(sel, self.perm_in)
+            with lasting():
+                self._pair_of = get_backend().pair_index(sel, self.perm_in)
         return self._pair_of
 
     def pair_rows(self):
@@ -66,8 +68,9 @@ class EdgePlan:
         if sel is None:
             return None
         if self._pair_rows is None:
-            idx = sel.long()
-            self._pair_rows = (self.row0.index_select(0, idx).contiguous(), self.row1.index_select(0, idx).contiguous())
+            with lasting():
+                idx = sel.long()
+                self._pair_rows = (self.row0.index_select(0, idx).contiguous(), self.row1.index_select(0, idx).contiguous())
         return self._pair_rows
 
     @staticmethod
@@ -140,8 +143,9 @@ class DeferredPlan:
         recording = cuda and torch.cuda.is_current_stream_capturing()
         if self._made is not None and self._stream == stream and not recording:
             return self._made
-        row0, row1 = self.index.to(torch.int32).unbind(0)
-        plan = EdgePlan.from_centre_sorted(row0, row1, self.offsets, self.N, self.symmetric, self.loops)
+        with lasting():
+            row0, row1 = self.index.to(torch.int32).unbind(0)
+            plan = EdgePlan.from_centre_sorted(row0, row1, self.offsets, self.N, self.symmetric, self.loops)
         if not recording:
             self._made, self._stream = plan, stream
         return plan
@@ -169,7 +173,8 @@ def plan_of(edge_index: torch.Tensor, N: int) -> EdgePlan:
     """The plan travelling with an edge list built by this package, else one derived on the spot."""
     plan = attached_plan(edge_index)
     if plan is None or plan.N != N or plan.E != edge_index.shape[1]:
-        plan = EdgePlan.from_edge_index(edge_index, N)
+        with lasting():
+            plan = EdgePlan.from_edge_index(edge_index, N)
         attach_plan(edge_index, plan)
     return plan
 

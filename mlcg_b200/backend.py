@@ -4,6 +4,7 @@ Every operator of the package goes through the object returned by :func:`get_bac
 back end is :class:`CudaBackend`; it refuses tensors that are not on a CUDA device, and constructing it
 raises if ``libmlcg_b200.so`` is missing.
 """
+import contextlib
 import ctypes
 from dataclasses import dataclass
 from typing import Optional
@@ -114,6 +115,18 @@ class _NoGuard:
 
 
 _NO_GUARD = _NoGuard()
+
+
+@contextlib.contextmanager
+def _outside_inference():
+    with torch.inference_mode(False), torch.no_grad():
+        yield
+
+
+def lasting():
+    """The mode in which what is kept for later calls is made, whatever the caller's: a tensor made under ``torch.inference_mode()`` has no
+    count of the writes to it and can enter no graph outside."""
+    return _outside_inference() if torch.is_inference_mode_enabled() else _NO_GUARD
 
 
 def _on(device):

@@ -11,7 +11,7 @@ from typing import Dict, Mapping, Optional, Tuple
 import torch
 
 from .autograd import DeferredPlan, EdgePlan, attach_plan, carried_plan, edge_distances
-from .backend import STATUS_TRUNCATED, get_backend
+from .backend import STATUS_TRUNCATED, get_backend, lasting
 
 RULE_NATIVE, RULE_CLUSTER = 0, 1
 
@@ -46,10 +46,11 @@ def _graph(x, r, ptr, loop, max_num_neighbors, rule, want_distance=False, exclud
     if getattr(be, "plans_with_graph", False):         # the pair plan comes with the graph
         more = dict(want_plan=True, want_index=want_index, n_atoms=n_atoms)
         ptr = None if n_atoms is not None else ptr
-    res = be.radius_graph(_as_3d(x), ptr, r, max_num_neighbors, loop, rule, want_distance=want_distance, want_batch=want_batch, exclude=exclude, **more)
-    truncated = bool(res["status"] & STATUS_TRUNCATED)
-    # an exclusion list need not hold both directions of a pair: such a graph is not taken to be symmetric
-    plan = EdgePlan.from_graph(res, x.shape[0], symmetric=not truncated and exclude is None, loops=bool(loop))
+    with lasting():                                     # (the list and its plan stay together, and a list counts the writes to it)
+        res = be.radius_graph(_as_3d(x), ptr, r, max_num_neighbors, loop, rule, want_distance=want_distance, want_batch=want_batch, exclude=exclude, **more)
+        truncated = bool(res["status"] & STATUS_TRUNCATED)
+        # an exclusion list need not hold both directions of a pair: such a graph is not taken to be symmetric
+        plan = EdgePlan.from_graph(res, x.shape[0], symmetric=not truncated and exclude is None, loops=bool(loop))
     if res["edge_index"] is not None:
         attach_plan(res["edge_index"], plan)
     if res.get("ptr") is None:
@@ -63,15 +64,16 @@ def _edges(x, r, batch, batch_size, ptr, loop, max_num_neighbors, rule, want_dis
     rows with the list: 1815 us for 65 M edges, without them 1004).  Structures from ``ptr``, or from ``batch`` and ``batch_size``."""
     be, N = get_backend(), x.shape[0]
     small = getattr(be, "small_graph_points", 0)
-    if ptr is None and 0 < N <= small and exclude is None and batch_size is None and (batch is None or batch.numel() == N):
-        res = be.radius_graph_small(_as_3d(x), None if batch is None else batch.to(torch.int64), r, max_num_neighbors, loop, rule, want_distance)
-    else:
-        more = {"want_rows": False} if small else {}
-        ptr = _structure_ptr(x, batch, batch_size) if ptr is None else ptr
-        res = be.radius_graph(_as_3d(x), ptr, r, max_num_neighbors, loop, rule, want_distance=want_distance, want_batch=False, exclude=exclude, **more)
-    # an exclusion list need not hold both directions of a pair: such a graph is not taken to be symmetric
-    symmetric = exclude is None and not res["status"] & STATUS_TRUNCATED
-    return attach_plan(res["edge_index"], DeferredPlan(res["edge_index"], res["offsets"], N, symmetric, bool(loop))), res["distance"]
+    with lasting():                                     # (a plan made later has to know whether the list was written to)
+        if ptr is None and 0 < N <= small and exclude is None and batch_size is None and (batch is None or batch.numel() == N):
+            res = be.radius_graph_small(_as_3d(x), None if batch is None else batch.to(torch.int64), r, max_num_neighbors, loop, rule, want_distance)
+        else:
+            more = {"want_rows": False} if small else {}
+            ptr = _structure_ptr(x, batch, batch_size) if ptr is None else ptr
+            res = be.radius_graph(_as_3d(x), ptr, r, max_num_neighbors, loop, rule, want_distance=want_distance, want_batch=False, exclude=exclude, **more)
+        # an exclusion list need not hold both directions of a pair: such a graph is not taken to be symmetric
+        symmetric = exclude is None and not res["status"] & STATUS_TRUNCATED
+        return attach_plan(res["edge_index"], DeferredPlan(res["edge_index"], res["offsets"], N, symmetric, bool(loop))), res["distance"]
 
 
 def _differentiated(x) -> bool:

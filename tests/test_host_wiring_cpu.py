@@ -481,3 +481,43 @@ def test_room_for_the_edges_of_proteins_in_turn(golden, monkeypatch):
     assert asked[-2] == 1.03 * 12.0 * 5000 + 64 and asked[-1] == 1.03 * 12.0 * 500 + 64
     per_bead = 80.0
     assert call(1000)
+
+
+@pytest.mark.parametrize("make", ["radius_graph", "radius_distance", "neighbor_list", "from_outside"])
+def test_lists_of_inference_mode(golden, make):
+    """Lists made, first used or written to under ``torch.inference_mode()``: their plans are those of the edges they hold, and what is
+    kept of them is of use outside."""
+    c = golden["schnet_gaussian_f32"]
+    net, data = schnet_from_case(c), data_from_case(c)
+    pos, batch, upper, N = data.pos, data.batch, float(c["upper"]), data.pos.shape[0]
+
+    def fresh():
+        if make == "radius_distance":
+            return mlcg_b200.neighbor_list.radius_distance(pos, upper, batch, max_num_neighbors=1000)[1]
+        if make == "neighbor_list":
+            return net.neighbor_list(data, upper)["SchNet"]["index_mapping"]
+        return mlcg_b200.radius_graph(pos, upper, batch, max_num_neighbors=1000, flow="target_to_source")
+
+    want = fresh().clone()
+    for made_inside in (True, False):
+        if make == "from_outside":
+            edges = want.clone()
+        else:
+            with torch.inference_mode(made_inside):
+                edges = fresh()
+        assert torch.equal(edges, want)
+        with torch.inference_mode():
+            plan = ag.plan_of(edges, N)
+            assert plan.symmetric == (make != "from_outside")
+            parts = (plan.row0, plan.row1, plan.ptr_out, plan.perm_in, plan.nbr_in) + ((plan.half_selection(), plan.pair_index(), *plan.pair_rows()) if plan.symmetric else ())
+        assert ag.plan_of(edges, N) is plan and not any(t.is_inference() for t in parts)
+        # written to before its first use, and once more after it
+        if make != "from_outside":
+            with torch.inference_mode(made_inside):
+                edges = fresh()
+        for first in (0, 16):
+            with torch.inference_mode():
+                edges[:, first:first + 8] = edges[:, first + 8:first + 16].clone()
+                plan = ag.plan_of(edges, N)
+            assert torch.equal(plan.row0.long(), edges[0]) and torch.equal(plan.row1.long(), edges[1]) and not plan.symmetric
+            assert torch.equal(plan.ptr_in[1:] - plan.ptr_in[:-1], torch.bincount(edges[1], minlength=N))
