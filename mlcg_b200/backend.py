@@ -561,7 +561,8 @@ class CudaBackend:
         """One status array per device for kernels whose status is only ever checked lazily (bits accumulate)."""
         st = self._status.get(dev)
         if st is None:
-            st = self._status[dev] = torch.zeros(4, dtype=torch.int32, device=dev)
+            with lasting():
+                st = self._status[dev] = torch.zeros(4, dtype=torch.int32, device=dev)
         return st
 
     def edge_distance(self, pos, row0, row1):

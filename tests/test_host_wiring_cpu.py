@@ -521,3 +521,13 @@ def test_lists_of_inference_mode(golden, make):
                 plan = ag.plan_of(edges, N)
             assert torch.equal(plan.row0.long(), edges[0]) and torch.equal(plan.row1.long(), edges[1]) and not plan.symmetric
             assert torch.equal(plan.ptr_in[1:] - plan.ptr_in[:-1], torch.bincount(edges[1], minlength=N))
+
+
+def test_prior_parameters_kept_in_inference_mode_are_of_use_in_training():
+    data, priors = prior_setup(12, 2, 3, torch.Generator().manual_seed(6))
+    data.pos.requires_grad_(True)
+    for k, p in priors.items():
+        with torch.inference_mode():
+            p.eval()._cached_params(data)
+        energy = p.train()(data).out[k]["energy"]
+        assert bool(torch.autograd.grad(energy.sum(), data.pos)[0].isfinite().all())
