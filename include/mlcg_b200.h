@@ -11,7 +11,8 @@
  *     Data-dependent conditions are reported through a 4-word device `status` array the caller zeroes:
  *     status[0] bit 0 = a centre had more neighbours than max_num_neighbors (list truncated),
  *     status[0] bit 1 = an index was out of range and the element was skipped,
- *     status[0] bit 2 = an edge had no reverse partner (graph not symmetric).
+ *     status[0] bit 2 = an edge had no reverse partner (graph not symmetric),
+ *     status[0] bit 6 = a list that is being prepared names a bead or a bead type that does not exist.
  *   - `stream` is a cudaStream_t passed as void*.
  *
  * Each entry point names the reference interface it stands in for (path inside the mlcg repository).
@@ -593,7 +594,7 @@ typedef struct {
     const void *slice_params;
 } mlcgb_prior_list;
 /* What an mlcgb_prior_list is made of, from the list as the neighbour-list dictionary holds it: idx [order,M] = mapping (an index outside
- * [0,N) becomes -1 and sets status bit 1), params [n_params,M] = tables[q] ([num_types]^order, contiguous) at the types [N] of the
+ * [0,N) becomes -1 and sets status bit 1; one outside [-N,N), or a type outside the tables, which is taken as 0, bit 6 too), params [n_params,M] = tables[q] ([num_types]^order, contiguous) at the types [N] of the
  * term's beads (tables NULL: not written; `given` [n_params,M] are the parameters).  host_out (order 2 only, NULL: not wanted; the call then
  * waits for the result and must not be captured): [0] = runs of equal first bead, [1] = 1 where the list holds (j, i) with the same
  * parameters for every (i, j) (compared by the sum of 64-bit hashes).  starts [runs]: first term of each run, from the workspace that

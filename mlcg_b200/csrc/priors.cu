@@ -428,7 +428,7 @@ prior_gather_kernel(const int64_t *__restrict__ mapping, int64_t M, const int64_
         for (int o = 0; o < ORDER; o++) {
             const int32_t bead = written(at[o]);
             if (bead < 0) {                                  // (reported, and again by the evaluation, which leaves the term out)
-                atomicOr(status, (int)kBadIndex);
+                atomicOr(status, (int)kBadIndex | (at[o] >= N || at[o] < -N ? (int)kNotThere : 0));
                 at[o] = -1;
             }
             idx[(int64_t)o * M + t] = bead;
@@ -439,7 +439,7 @@ prior_gather_kernel(const int64_t *__restrict__ mapping, int64_t M, const int64_
                 int64_t ty = at[o] < 0 ? 0 : __ldg(types + at[o]);
                 if (ty < 0) ty += num_types;                 // (as indexing a table does)
                 if (ty < 0 || ty >= num_types) {
-                    atomicOr(status, (int)kBadIndex);
+                    atomicOr(status, (int)kBadIndex | (int)kNotThere);
                     ty = 0;
                 }
                 entry = entry * num_types + ty;

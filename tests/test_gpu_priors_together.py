@@ -189,19 +189,21 @@ def test_types_that_end_before_the_beads_do(order, pairs):
     status.zero_()
 
 
-def test_a_list_is_made_again_for_more_beads():
-    """A list first met with beads missing is not kept for the call that has them."""
+@pytest.mark.parametrize("name", ["bonds", "angles", "dihedrals", "repulsion"])
+def test_lists_for_other_data_are_refused(name):
+    """A list for a longer chain than the data, and beads of a type that the tables do not have: an error at the first call and at the
+    next one, and the list is made again, whole, for data that fit."""
     data, priors = prior_setup(40, 2, 4, torch.Generator().manual_seed(4))
-    data, p = data.to(DEV), priors["repulsion"].to(DEV).eval()
+    data, p = data.to(DEV), priors[name].to(DEV).eval()
     data.pos = torch.cat([random_walk_chain(40, torch.Generator().manual_seed(5), min_dist=3.0) for _ in range(2)]).float().to(DEV)
-    want, pos, batch = _evaluate_together([p], data, forces=True)[0]["repulsion"], data.pos, data.batch
-    p.__dict__.pop("_mlcgb_list")
-    data.pos, data.batch = pos[:60], batch[:60]
-    _evaluate_together([p], data, forces=True)
+    want, pos, batch, types = _evaluate_together([p], data, forces=True)[0][name], data.pos, data.batch, data.atom_types
     from mlcg_b200.backend import get_backend
     status = get_backend()._sticky_status(torch.device(DEV))
-    assert int(status[0]) & 2
-    status.zero_()
-    data.pos, data.batch = pos, batch
-    got = _evaluate_together([p], data, forces=True)[0]["repulsion"]
-    assert all(torch.equal(a, b) for a, b in zip(got, want)) and int(status[0]) == 0
+    for other in ((pos[:60], batch[:60], types), (pos, batch, types[:60]), (pos, batch, torch.where(torch.arange(80, device=DEV) == 70, 4, types))):
+        data.pos, data.batch, data.atom_types = other
+        for _ in range(2):
+            with pytest.raises(IndexError, match="does not exist"):
+                _evaluate_together([p], data, forces=True)
+        data.pos, data.batch, data.atom_types = pos, batch, types
+        got = _evaluate_together([p], data, forces=True)[0][name]
+        assert all(torch.equal(a, b) for a, b in zip(got, want)) and int(status[0]) == 0
