@@ -1121,15 +1121,16 @@ class CudaBackend:
                 self._run("prior_list_starts", self.lib.mlcgb_prior_list_starts, (_ptr(idx), M, _ptr(ws), wsb, _ptr(starts), _stream()))
         return idx, out, bool(host[1]), starts
 
-    def refuse_missing(self, dev, what):
-        """Raise where :meth:`prior_list` has met a bead or a type that does not exist (a host read; not while recording)."""
+    def lists_name_missing(self, dev) -> bool:
+        """Whether :meth:`prior_list` has met a bead or a type that does not exist since this was asked last (a host read; not while
+        recording)."""
         if torch.cuda.is_current_stream_capturing():
-            return
+            return False
         status = self._sticky_status(dev)
         word = int(status[0])
         if word & STATUS_NOT_THERE:
             status[0] = word & ~(STATUS_NOT_THERE | STATUS_BAD_INDEX)
-            raise IndexError(f"mlcg_b200: {what}: the list names a bead, or a bead has a type, that does not exist")
+        return bool(word & STATUS_NOT_THERE)
 
     def pair_slices(self, idx, params, starts, worth):
         """The slices of a pair list (int32 [2, M], runs of equal first bead from ``starts`` on) as ``mlcgb_prior_list`` takes them:
