@@ -46,8 +46,9 @@ int mlcgb_last_cuda_error(void); /* cudaError_t of the last failed launch on thi
  *   200  mlcgb_prior_list: run_ptr, n_runs gone, the slice fields new.  mlcgb_prior_eval: the int32 struct_of became batch (int64 or
  *        NULL), negate and the totals are new, fixed_point = 0 writes its outputs too (it added to them), the workspace is wanted in
  *        both modes and mlcgb_prior_eval_workspace_bytes takes the dtype where it took fixed_point.  mlcgb_gemm_tc_chain2 with
- *        backward = 1 writes mid_out unless it is NULL. */
-#define MLCGB_VERSION 201
+ *        backward = 1 writes mid_out unless it is NULL.
+ *   300  mlcgb_prior_list_make: host_out has three values. */
+#define MLCGB_VERSION 300
 int mlcgb_version(void);
 
 /* Device time per entry point, without a profiler.  No counterpart in the reference (mlcg times whole steps on the host).
@@ -597,13 +598,13 @@ typedef struct {
  * [0,N) becomes -1 and sets status bit 1; one outside [-N,N), or a type outside the tables, which is taken as 0, bit 6 too), params [n_params,M] = tables[q] ([num_types]^order, contiguous) at the types [N] of the
  * term's beads (tables NULL: not written; `given` [n_params,M] are the parameters).  host_out (order 2 only, NULL: not wanted; the call then
  * waits for the result and must not be captured): [0] = runs of equal first bead, [1] = 1 where the list holds (j, i) with the same
- * parameters for every (i, j) (compared by the sum of 64-bit hashes).  starts [runs]: first term of each run, from the workspace that
+ * parameters for every (i, j) (compared by the sum of 64-bit hashes), [2] = status[0] behind the call.  starts [runs]: first term of each run, from the workspace that
  * the call before left. */
 #define MLCGB_MAX_PRIOR_TABLES 32
 size_t mlcgb_prior_list_workspace_bytes(int64_t M);
 int mlcgb_prior_list_make(const int64_t *mapping, int order, int64_t M, const int64_t *types, int64_t N, int64_t num_types, int n_params,
                           const void *const *tables /* host */, int dtype, const void *given, int32_t *idx, void *params, void *workspace,
-                          size_t workspace_bytes, int64_t *host_out /* [2] */, int32_t *status, void *stream);
+                          size_t workspace_bytes, int64_t *host_out /* [3] */, int32_t *status, void *stream);
 int mlcgb_prior_list_starts(const int32_t *first /* idx */, int64_t M, const void *workspace, size_t workspace_bytes, int64_t *starts, void *stream);
 /* The slices of a pair list idx [2,M] whose runs of equal first bead begin at starts [n_runs].  With slice_params NULL: slices =
  * {longest run, -, least, largest second bead} of each; then, with step0 = exclusive sums of (longest + 3) / 4 and steps their total,

@@ -45,7 +45,7 @@ class PriorListStruct(ctypes.Structure):
 
 MAX_PRIOR_TABLES = 32           # MLCGB_MAX_PRIOR_TABLES
 MAX_PRIOR_SEGMENTS = 8
-VERSION = 201                  # MLCGB_VERSION of the header that the tables below follow
+VERSION = 300                  # MLCGB_VERSION of the header that the tables below follow
 EVALUATE_DONE, EVALUATE_MORE = 1, 2
 
 # name -> (restype, argtypes); one entry per symbol declared in include/mlcg_b200.h

@@ -6,6 +6,7 @@ raises if ``libmlcg_b200.so`` is missing.
 """
 import contextlib
 import ctypes
+import threading
 from dataclasses import dataclass
 from typing import Optional
 
@@ -222,7 +223,7 @@ class CudaBackend:
         _lib.bind_native(self.lib)
         self.native = _lib.native()
         self.profiler = None
-        self._status = {}
+        self._status, self._lists = {}, threading.local()
         self.tensor_core_gemm = True   # float32 GEMMs of qualifying shape run on tcgen05 (fp32-equivalent products)
         self._pending = []      # (status tensor, what) of kernels whose status word has not been read yet
 
@@ -1110,7 +1111,7 @@ class CudaBackend:
             pairs = bool(pairs) and M > 0 and M % 2 == 0
             wsb = self.lib.mlcgb_prior_list_workspace_bytes(M) if pairs else 0
             ws = torch.empty(wsb, dtype=torch.uint8, device=dev) if pairs else None
-            host = (ctypes.c_int64 * 2)()
+            host = (ctypes.c_int64 * 3)()
             self._run("prior_list", self.lib.mlcgb_prior_list_make, (
                 _ptr(mapping), order, M, _ptr(types), n_beads, kinds, P, None if tables is None else (ctypes.c_void_p * P)(*(t.data_ptr() for t in tables)),
                 _dt(like), _ptr(params), _ptr(idx), None if tables is None else _ptr(out), _ptr(ws), wsb, host if pairs else None,
@@ -1119,15 +1120,18 @@ class CudaBackend:
             if host[1] and M >= 8 * host[0] and M < 2 ** 31:
                 starts = torch.empty(host[0], dtype=torch.int64, device=dev)
                 self._run("prior_list_starts", self.lib.mlcgb_prior_list_starts, (_ptr(idx), M, _ptr(ws), wsb, _ptr(starts), _stream()))
+        # what the status word says of the lists made so far: known to the host (a pair list), or to be read
+        self._lists.word = int(host[2]) if pairs else None
         return idx, out, bool(host[1]), starts
 
     def lists_name_missing(self, dev) -> bool:
-        """Whether :meth:`prior_list` has met a bead or a type that does not exist since this was asked last (a host read; not while
-        recording)."""
+        """Whether :meth:`prior_list` has met a bead or a type that does not exist since this was asked last (a host read unless the last list
+        was a pair list, whose call has waited; not while recording)."""
         if torch.cuda.is_current_stream_capturing():
             return False
-        status = self._sticky_status(dev)
-        word = int(status[0])
+        status, word = self._sticky_status(dev), getattr(self._lists, "word", None)
+        if word is None or word & STATUS_NOT_THERE:
+            word = int(status[0])
         if word & STATUS_NOT_THERE:
             status[0] = word & ~(STATUS_NOT_THERE | STATUS_BAD_INDEX)
         return bool(word & STATUS_NOT_THERE)
