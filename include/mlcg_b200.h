@@ -183,6 +183,15 @@ int mlcgb_pair_plan(const int32_t *row0, const int32_t *row1, const int64_t *off
                     void *workspace, size_t workspace_bytes, int32_t *twin /* [E] */, int32_t *sel /* [E/2] */,
                     int32_t *pair_of /* [E] */, int32_t *status, void *stream);
 
+/* 32-bit rows and pair plan of a list as the radius graph hands it out: edge_index [2,E] int64, complete (symmetric, not cut short),
+ * without loops, centre-major with ascending neighbours, E even; offsets as its count left them.  ptr [B+1]: the structure boundaries it
+ * was made with, or NULL (then, and up to 2048 points, every reverse is found by bisection).  row1 on a 32-byte boundary, else as without
+ * ptr.  A list that is none of that sets status bits 1 and 2; the outputs are then no plan, but valid indices. */
+size_t mlcgb_list_plan_workspace_bytes(int64_t N);
+int mlcgb_list_plan(const int64_t *edge_index, const int64_t *offsets /* [N+1] */, const int64_t *ptr, int64_t B, int64_t E, int64_t N, void *workspace,
+                    size_t workspace_bytes, int32_t *row0 /* [E] */, int32_t *row1 /* [E] */, int32_t *twin /* [E] */, int32_t *sel /* [E/2] */,
+                    int32_t *pair_of /* [E] */, int32_t *status, void *stream);
+
 /* ------------------------------------------------------------------------------------------------
  * Edge geometry.  compute_distances, src/mlcg/geometry/internal_coordinates.py:72-100, split into
  * its linear part dr = pos[row1] - pos[row0] and that part's transpose (used by every derivative).

@@ -67,6 +67,8 @@ SIGNATURES = {
                                           ctypes.POINTER(c_i64), c_vp, c_vp]),
     "mlcgb_edge_twin": (c_int, [c_vp, c_vp, c_vp, c_i64, c_i64, c_vp, c_vp, c_vp]),
     "mlcgb_pair_plan_workspace_bytes": (c_sz, [c_i64]),
+    "mlcgb_list_plan_workspace_bytes": (c_sz, [c_i64]),
+    "mlcgb_list_plan": (c_int, [c_vp, c_vp, c_vp, c_i64, c_i64, c_i64, c_vp, c_sz] + [c_vp] * 7),
     "mlcgb_pair_plan": (c_int, [c_vp, c_vp, c_vp, c_i64, c_i64, c_vp, c_sz, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "mlcgb_pair_index": (c_int, [c_vp, c_vp, c_i64, c_vp, c_vp]),
     "mlcgb_edge_diff": (c_int, [c_vp, c_int, c_vp, c_vp, c_i64, c_i64, c_vp, c_vp, c_vp]),

@@ -130,22 +130,27 @@ class DeferredPlan:
     kept for the stream that it was made on (another one makes its own, there is no order between the two) and never out of a
     recording, whose buffers hold nothing until it is replayed."""
 
-    __slots__ = ("index", "offsets", "N", "symmetric", "loops", "_made", "_stream")
+    __slots__ = ("index", "offsets", "ptr", "N", "symmetric", "loops", "_made", "_stream")
 
-    def __init__(self, edge_index: torch.Tensor, offsets: torch.Tensor, N: int, symmetric: bool, loops: bool):
-        # (an alias: the list carries this object, which must not hold the list)
-        self.index, self.offsets, self.N, self.symmetric, self.loops = edge_index.detach(), offsets, N, symmetric, loops
+    def __init__(self, edge_index: torch.Tensor, offsets: torch.Tensor, ptr: Optional[torch.Tensor], N: int, symmetric: bool, loops: bool):
+        # (an alias: the list carries this object, which must not hold the list; ptr: the structure boundaries, None where they are the caller's)
+        self.index, self.offsets, self.ptr, self.N, self.symmetric, self.loops = edge_index.detach(), offsets, ptr, N, symmetric, loops
         self._made = self._stream = None
 
     def plan(self) -> EdgePlan:
         cuda = self.index.is_cuda
-        stream = torch.cuda.current_stream(self.index.device).cuda_stream if cuda else 0
+        stream = torch._C._cuda_getCurrentRawStream(self.index.get_device()) if cuda else 0
         recording = cuda and torch.cuda.is_current_stream_capturing()
         if self._made is not None and self._stream == stream and not recording:
             return self._made
         with lasting():
-            row0, row1 = self.index.to(torch.int32).unbind(0)
-            plan = EdgePlan.from_centre_sorted(row0, row1, self.offsets, self.N, self.symmetric, self.loops)
+            be, E = get_backend(), self.index.shape[1]
+            if self.symmetric and not self.loops and E % 2 == 0 and 0 < E < 1 << 31 and hasattr(be, "list_plan"):
+                row0, row1, twin, sel, pair_of = be.list_plan(self.index, self.offsets, self.ptr, self.N)
+                plan = EdgePlan(self.N, E, row0, row1, self.offsets, None, row1, self.offsets, twin, row1, True, False, sel, pair_of)
+            else:
+                row0, row1 = self.index.to(torch.int32).unbind(0)
+                plan = EdgePlan.from_centre_sorted(row0, row1, self.offsets, self.N, self.symmetric, self.loops)
         if not recording:
             self._made, self._stream = plan, stream
         return plan

@@ -539,6 +539,22 @@ class CudaBackend:
                                                                _ptr(status), _stream()), launches=5, nbytes=28 * E + 20 * N)
         return twin, sel, pair_of, status
 
+    def list_plan(self, edge_index, offsets, ptr, N):
+        """``(row0, row1, twin, sel, pair_of)``, all int32, of a complete, loop-free list (int64 [2, E], E even and not 0) as
+        :meth:`radius_graph` returns it with its offsets and the structure boundaries (or None) it was made with.  A list that is none is
+        reported through the accumulating status words."""
+        _need_cuda(edge_index, offsets, ptr)
+        E, dev = edge_index.shape[1], edge_index.device
+        with _on(dev):
+            pad = -E % 8            # (row1 on a 32-byte boundary)
+            r0, _, r1, twin, pair_of, sel = torch.empty(4 * E + pad + E // 2, dtype=torch.int32, device=dev).split((E, pad, E, E, E, E // 2))
+            wsb = self.lib.mlcgb_list_plan_workspace_bytes(N)
+            ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
+            self._run("list_plan", self.lib.mlcgb_list_plan, (
+                _ptr(edge_index), _ptr(offsets), _ptr(ptr), 0 if ptr is None else ptr.numel() - 1, E, N, _ptr(ws), wsb, _ptr(r0), _ptr(r1), _ptr(twin), _ptr(sel),
+                _ptr(pair_of), _ptr(self._sticky_status(dev)), _stream()), launches=5, nbytes=46 * E + 20 * N)
+        return r0, r1, twin, sel, pair_of
+
     def pair_index(self, sel, twin):
         """pair_of[e] = k for the k-th selected edge and for its reverse."""
         _need_cuda(sel, twin)

@@ -1696,7 +1696,8 @@ __global__ void pair_plan_kernel(const int32_t *__restrict__ row0, const int32_t
 // falls among b's lower or upper neighbours if those are spread evenly over the structure, eight entries (one 32-byte sector)
 // at a time, and only then by bisection.  `seg` of a node is {first edge, lower edges, upper edges, pairs before}: one load.  A block
 // takes consecutive nodes, so that the seg entries of its structure stay in the L1.  65 M edges of 4000-point structures: the
-// bisection above took 1.80 ms, seven dependent loads per edge.
+// bisection above took 1.80 ms, seven dependent loads per edge.  cellparam NULL: every structure that pair_transpose_kernel can take is
+// its own.  A list that turns out to be none is reported, and every index written stays inside its array.
 __global__ void __launch_bounds__(256)
 pair_plan_search_kernel(const int32_t *__restrict__ row1, const int4 *__restrict__ seg, const int32_t *__restrict__ struct_of,
                         const int64_t *__restrict__ ptr, const CellParam *__restrict__ cellparam, const int32_t *__restrict__ others, int transpose_max,
@@ -1708,7 +1709,7 @@ pair_plan_search_kernel(const int32_t *__restrict__ row1, const int4 *__restrict
         for (int64_t ai = n0 + warp; ai < n0 + kNodes && ai < N; ai += 8) {
             const int a = (int)ai;
             const int4 sa = seg[a];
-            const int st = struct_of[a], s0 = (int)ptr[st], s1 = (int)ptr[st + 1], tile = cellparam[st].tile;
+            const int st = struct_of[a], s0 = (int)ptr[st], s1 = (int)ptr[st + 1], tile = cellparam ? cellparam[st].tile : s1 - s0 > kBruteMax;
             if (tile == 2 || (tile == 1 && s1 - s0 <= transpose_max)) continue;      // (structures of the kernels below)
             const int deg = sa.y + sa.z;
             for (int q = lane; q < deg; q += 32) {
@@ -1747,16 +1748,16 @@ pair_plan_search_kernel(const int32_t *__restrict__ row1, const int4 *__restrict
                     // a near miss is almost always in the next sector; further off, bisect
                     guess = round == 0 ? (a < first ? hi - 1 : lo) : (lo + hi) >> 1;
                 }
-                if (t < 0) {
+                const int p = up ? sa.w + (q - sa.y) : sb.w + (t - sb.x - sb.y);
+                if (t < 0 || p < 0 || p >= (E >> 1)) {
                     atomicOr(status, (int)kAsymmetric);
                     twin[e] = e;
                     pair_of[e] = 0;
                     continue;
                 }
-                const int p = up ? sa.w + (q - sa.y) : sb.w + (t - sb.x - sb.y);
                 twin[e] = t;
                 pair_of[e] = p;
-                if (up && p < (E >> 1)) sel[p] = e;
+                if (up) sel[p] = e;
             }
         }
     }
@@ -2645,7 +2646,7 @@ mask_rows_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, int
 }
 
 // offsets and `seg` from the degrees: a block adds up the parts before its 1024 points itself; the last one hands the edge count to the
-// host (with -1 cells: not counted, the batch holds larger structures)
+// host (with -1 cells: not counted, the batch holds larger structures).  header NULL: nobody waits
 __global__ void __launch_bounds__(kScanBlock)
 rows_scan_kernel(const int32_t *__restrict__ deg, const int32_t *__restrict__ upper, const int2 *__restrict__ parts, int64_t N, int64_t *__restrict__ offsets,
                  int4 *__restrict__ seg, const int32_t *__restrict__ header, Publish pub) {
@@ -2654,7 +2655,7 @@ rows_scan_kernel(const int32_t *__restrict__ deg, const int32_t *__restrict__ up
     pdl_wait();
     const bool last = blockIdx.x == gridDim.x - 1;
     pub.cells_known = true;
-    if (header[8]) {
+    if (header && header[8]) {
         if (last && threadIdx.x == 0) {
             *reinterpret_cast<volatile int64_t *>(pub.host + 4) = -1;
             publish(pub, 0, 0);
@@ -2674,14 +2675,57 @@ rows_scan_kernel(const int32_t *__restrict__ deg, const int32_t *__restrict__ up
     block_exclusive_scan(bu, s_warp, &before_u);
     const int64_t ed = before_d + block_exclusive_scan(d, s_warp, &total_d);
     if (last && threadIdx.x == 0) {                    // (as early as it is known)
-        *reinterpret_cast<volatile int64_t *>(pub.host + 4) = 0;
-        publish(pub, before_d + total_d, *reinterpret_cast<const volatile int32_t *>(header));
+        if (header) {
+            *reinterpret_cast<volatile int64_t *>(pub.host + 4) = 0;
+            publish(pub, before_d + total_d, *reinterpret_cast<const volatile int32_t *>(header));
+        }
         offsets[N] = before_d + total_d;
     }
     const int64_t eu = before_u + block_exclusive_scan(u, s_warp, nullptr);
     if (i < N) {
         offsets[i] = ed;
         seg[i] = make_int4((int)ed, d - u, u, (int)eu);      // (read for plans only, which have fewer than 2^31 edges)
+    }
+}
+
+// 32-bit rows of a list that was handed out with int64 rows, and per centre its degree and its upper edges, a warp each; their sums of 32
+// centres for rows_scan_kernel.  An entry that is not an edge of its centre (the list was written to behind its owner's back) is reported
+// and becomes a loop, which no plan has; sel starts as zeros.  Bound by the stream: 65 M edges 361 us for 1.7 GB.
+__global__ void __launch_bounds__(256)
+list_rows_kernel(const int64_t *__restrict__ index, int64_t E, const int64_t *__restrict__ offsets, int64_t N, int32_t *__restrict__ row0,
+                 int32_t *__restrict__ row1, int32_t *__restrict__ deg, int32_t *__restrict__ upper, int2 *__restrict__ parts, int32_t *__restrict__ sel, int32_t *__restrict__ status) {
+    __shared__ int s_deg[8], s_upper[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int sum_deg = 0, sum_upper = 0;
+    for (int u = 0; u < 4; u++) {
+        const int64_t i = (int64_t)blockIdx.x * 32 + warp * 4 + u;
+        if (i >= N) break;
+        const int64_t k0 = offsets[i], k1 = offsets[i + 1];
+        int up = 0;
+#pragma unroll 2
+        for (int64_t k = k0 + lane; k < k1; k += 32) {
+            const int64_t c = index[k], j = index[E + k];
+            const bool ok = c == i && j >= 0 && j < N;
+            if (!ok) atomicOr(status, (int)kBadIndex | (int)kAsymmetric);
+            row0[k] = (int32_t)i;
+            row1[k] = (int32_t)(ok ? j : i);
+            if (!(k & 1)) sel[k >> 1] = 0;
+            up += ok && j > i;
+        }
+        up = warp_sum(up);
+        if (lane == 0) {
+            deg[i] = (int32_t)(k1 - k0);
+            upper[i] = up;
+        }
+        sum_deg += (int)(k1 - k0);
+        sum_upper += up;
+    }
+    if (lane == 0) { s_deg[warp] = sum_deg; s_upper[warp] = sum_upper; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int2 v = make_int2(0, 0);
+        for (int w = 0; w < 8; w++) { v.x += s_deg[w]; v.y += s_upper[w]; }
+        parts[blockIdx.x] = v;
     }
 }
 
@@ -2753,16 +2797,19 @@ constexpr int kTrWarps = 8, kTrRows = 4, kTrChunks = 3;
 // structures of 3000 points 82 us of walking against 55 us, at 47 of 4000 points 165 against 198.
 constexpr int64_t kTransposeBatch = 48;
 static inline int transpose_smem(int max_n) { return max_n * (8 + 2 * kTrWarps) + 64; }
+// CHECK: of a list that was out of our hands.  What is not a list of its structure's points in both directions is reported, and every
+// index written stays inside its array (65 M edges: 110 us, so the lists of the same call do without)
+template <bool CHECK>
 __global__ void __launch_bounds__(kTrWarps * 32)
-pair_transpose_kernel(const int32_t *__restrict__ row1, const int4 *__restrict__ seg, const CellParam *__restrict__ cellparam,
-                      const int64_t *__restrict__ ptr, int64_t B, int parts, int max_n, int32_t *__restrict__ twin, int32_t *__restrict__ sel,
-                      int32_t *__restrict__ pair_of) {
+pair_transpose_kernel(const int32_t *__restrict__ row1, const int4 *__restrict__ seg, const CellParam *__restrict__ cellparam /* NULL: as above */,
+                      const int64_t *__restrict__ ptr, int64_t B, int64_t P, int parts, int max_n, int32_t *__restrict__ twin, int32_t *__restrict__ sel,
+                      int32_t *__restrict__ pair_of, int32_t *__restrict__ status) {
     extern __shared__ uint32_t s_tr[];                 // [n] first edge of a row, [n] pair - edge of its lower entries, [warps][n] counters
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int64_t item = blockIdx.x; item < B * parts; item += gridDim.x) {
         const int64_t b = item / parts;
         const int lo = (int)ptr[b], n = (int)(ptr[b + 1] - ptr[b]), first_range = (int)(item % parts) * kTrWarps, ranges = parts * kTrWarps;
-        if (cellparam[b].tile != 1 || n > max_n) continue;
+        if ((cellparam ? cellparam[b].tile != 1 : n <= kBruteMax) || n > max_n) continue;
         const int stride = (n + 1) & ~1;
         int *s_off = reinterpret_cast<int *>(s_tr), *s_d = s_off + stride;
         uint16_t *cnt = reinterpret_cast<uint16_t *>(s_d + stride), *mine = cnt + warp * stride;
@@ -2855,15 +2902,22 @@ pair_transpose_kernel(const int32_t *__restrict__ row1, const int4 *__restrict__
             }
         };
         walk([&](int a, const int4 &s, int q, int k) {
+            const int e = s.x + q;
+            if (CHECK && (unsigned)k >= (unsigned)n) {
+                atomicOr(status, (int)kAsymmetric);
+                twin[e] = e;
+                pair_of[e] = 0;
+                return;
+            }
             const int r = mine[k];
             mine[k] = (uint16_t)(r + 1);
-            const int e = s.x + q, t = s_off[k] + r;
-            int p;
-            if (k > a) {
-                p = s.w + (q - s.y);
+            int t = s_off[k] + r, p = k > a ? s.w + (q - s.y) : t + s_d[k];
+            if (CHECK && (t >= end || (unsigned)p >= (unsigned)P)) {
+                atomicOr(status, (int)kAsymmetric);
+                t = e;
+                p = 0;
+            } else if (k > a) {
                 sel[p] = e;
-            } else {
-                p = t + s_d[k];
             }
             twin[e] = t;
             pair_of[e] = p;
@@ -2917,6 +2971,37 @@ __global__ void __launch_bounds__(kScanBlock) scan2_apply_kernel(const int32_t *
         offsets[i] = ed;
         seg[i] = make_int4((int)ed, d - u, u, (int)eu);      // (read for plans only, which have fewer than 2^31 edges)
     }
+}
+
+// Pairs of structures that have no bit rows: by counting where there are enough of them, by search for the rest.  `others` as
+// pair_plan_search_kernel has it, small_done: the structures without a cell grid have their pairs.  CHECK: see pair_transpose_kernel
+template <bool CHECK>
+static int large_plans(const int32_t *row1, const int4 *seg, const int32_t *struct_of, const int64_t *ptr, const CellParam *cellparam, const int32_t *others,
+                       bool small_done, int64_t N, int64_t B, int64_t E, int32_t *twin, int32_t *sel, int32_t *pair_of, int32_t *status, cudaStream_t st) {
+    // two structures of up to 4600 points fit an SM together; for larger ones a block takes the whole of it
+    const bool walk = B >= kTransposeBatch;
+    const int max_n = !walk ? 0 : N <= kTransposePair * B ? kTransposePair : kCapBits;
+    if (walk) {
+        static bool done[64] = {false};
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev >= 0 && dev < 64 && !done[dev]) {
+            if (cudaFuncSetAttribute(pair_transpose_kernel<CHECK>, cudaFuncAttributeMaxDynamicSharedMemorySize, transpose_smem(kCapBits)) != cudaSuccess)
+                return check_launch();
+            done[dev] = true;
+        }
+        // two blocks an SM: where that leaves some idle, structures are cut into parts (each pays for its own start counters)
+        const int64_t want = 2 * (int64_t)kNumSM / B;
+        const int parts = (int)(want < 1 ? 1 : want);
+        pair_transpose_kernel<CHECK><<<grid_for(B * parts, 1, 2), kTrWarps * 32, transpose_smem(max_n), st>>>(row1, seg, cellparam, ptr, B, E >> 1, parts, max_n, twin, sel,
+                                                                                                      pair_of, status);
+    }
+    if (!small_done || N > max_n) {              // structures too small for a cell grid, too large for the counters or too few
+        const int nodes = N >= (int64_t)kNumSM * 16 * 64 ? 64 : 8;
+        pair_plan_search_kernel<<<grid_for(N, nodes, 16), 256, 0, st>>>(row1, seg, struct_of, ptr, cellparam, walk ? others : nullptr, max_n, nodes, E, N, twin, sel,
+                                                                      pair_of, status);
+    }
+    return check_launch();
 }
 
 template <typename T, bool BATCH = false>
@@ -3154,34 +3239,61 @@ int mlcgb_graph_finish(const void *pos, int dtype, const int64_t *ptr, int64_t N
             mask_rows_fill_kernel<scalar_t><<<grid_for(N * 32, 256), 256, 0, st>>>((const scalar_t *)pos, ptr, struct_of, cells ? cellparam : nullptr, N, (const uint2 *)(w + L.masks),
                                                                                  seg, offsets, out, twin, sel, pair_of);
         distances();
-        if (twin && cells) {
-            // two structures of up to 4600 points fit an SM together; for larger ones a block takes the whole of it
-            const bool walk = B >= kTransposeBatch;
-            const int max_n = !walk ? 0 : N <= kTransposePair * B ? kTransposePair : kCapBits;
-            if (walk) {
-                static bool done[64] = {false};
-                int dev = 0;
-                cudaGetDevice(&dev);
-                if (dev >= 0 && dev < 64 && !done[dev]) {
-                    if (cudaFuncSetAttribute(pair_transpose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, transpose_smem(kCapBits)) != cudaSuccess)
-                        return check_launch();
-                    done[dev] = true;
-                }
-                // two blocks an SM: where that leaves some idle, structures are cut into parts (each pays for its own start counters)
-                const int64_t want = 2 * (int64_t)kNumSM / B;
-                const int parts = (int)(want < 1 ? 1 : want);
-                pair_transpose_kernel<<<grid_for(B * parts, 1, 2), kTrWarps * 32, transpose_smem(max_n), st>>>(row1, seg, cellparam, ptr, B, parts, max_n, twin,
-                                                                                                      sel, pair_of);
-            }
-            if (!rows || N > max_n) {            // structures too small for a cell grid, too large for the counters or too few
-                const auto *others = walk && N > (rows ? kMaskMax : kBruteMax) ? (const int32_t *)(cw + W.group_ptr) + B + 1 : nullptr;
-                const int nodes = N >= (int64_t)kNumSM * 16 * 64 ? 64 : 8;
-                pair_plan_search_kernel<<<grid_for(N, nodes, 16), 256, 0, st>>>(row1, seg, struct_of, ptr, cellparam, others, max_n, nodes, E, N, twin, sel,
-                                                                              pair_of, sticky_status);
-            }
-        }
+        if (twin && cells)
+            return large_plans<false>(row1, seg, struct_of, ptr, cellparam, N > (rows ? kMaskMax : kBruteMax) ? (const int32_t *)(cw + W.group_ptr) + B + 1 : nullptr, rows, N, B,
+                               E, twin, sel, pair_of, sticky_status, st);
         return check_launch();
     });
+}
+
+struct ListPlanLayout {
+    size_t deg, upper, uoff, bsum, seg, struct_of, parts, total;
+};
+static ListPlanLayout list_plan_layout(int64_t N) {
+    ListPlanLayout L;
+    size_t o = 0;
+    L.deg = o;       o += align256((size_t)N * 4);
+    L.upper = o;     o += align256((size_t)N * 4);
+    L.uoff = o;      o += align256((size_t)(N + 1) * 8);
+    L.bsum = o;      o += align256((size_t)((N + kScanBlock - 1) / kScanBlock + 1) * 8);
+    L.seg = o;       o += align256((size_t)N * 16);
+    L.struct_of = o; o += align256((size_t)N * 4);
+    L.parts = o;     o += align256((size_t)((N + 31) / 32) * 8);
+    L.total = o;
+    return L;
+}
+
+size_t mlcgb_list_plan_workspace_bytes(int64_t N) {
+    if (N < 0) return 0;
+    return list_plan_layout(N).total;
+}
+
+int mlcgb_list_plan(const int64_t *edge_index, const int64_t *offsets, const int64_t *ptr, int64_t B, int64_t E, int64_t N, void *workspace,
+                    size_t workspace_bytes, int32_t *row0, int32_t *row1, int32_t *twin, int32_t *sel, int32_t *pair_of, int32_t *status, void *stream) {
+    TimelineScope timeline_scope("list_plan", stream);
+    if (E < 0 || N < 0 || (E & 1) || !status || (ptr && B <= 0)) return MLCGB_E_ARG;
+    if (E == 0) return MLCGB_OK;
+    if (!edge_index || !offsets || !row0 || !row1 || !twin || !sel || !pair_of || !workspace || N == 0) return MLCGB_E_ARG;
+    if (E >= (int64_t)1 << 31 || N >= (int64_t)1 << 31) return MLCGB_E_LIMIT;
+    const ListPlanLayout L = list_plan_layout(N);
+    if (workspace_bytes < L.total) return MLCGB_E_WORKSPACE;
+    auto st = (cudaStream_t)stream;
+    char *w = (char *)workspace;
+    auto *deg = (int32_t *)(w + L.deg), *upper = (int32_t *)(w + L.upper), *struct_of = (int32_t *)(w + L.struct_of);
+    auto *uoff = (int64_t *)(w + L.uoff);
+    auto *seg = (int4 *)(w + L.seg);
+    auto *parts = (int2 *)(w + L.parts);
+    const bool structures = ptr && N > kMaskNodes && ((uintptr_t)row1 & 31) == 0;
+    list_rows_kernel<<<(unsigned)((N + 31) / 32), 256, 0, st>>>(edge_index, E, offsets, N, row0, row1, deg, upper, parts, sel, status);
+    if (structures) {
+        rows_scan_kernel<<<(unsigned)((N + kScanBlock - 1) / kScanBlock), kScanBlock, 0, st>>>(deg, upper, parts, N, uoff, seg, nullptr, Publish{});
+        cudaMemsetAsync(struct_of, 0, (size_t)N * 4, st);                    // (points of no structure)
+        struct_of_kernel<<<grid_for(B, 1, 8), 256, 0, st>>>(ptr, B, struct_of);
+        return large_plans<true>(row1, seg, struct_of, ptr, nullptr, nullptr, false, N, B, E, twin, sel, pair_of, status, st);
+    }
+    launch_scan(upper, N, (int64_t *)(w + L.bsum), uoff, st);
+    pair_plan_kernel<<<grid_for(E, 256), 256, 0, st>>>(row0, row1, offsets, upper, uoff, E, N, twin, sel, pair_of, status);
+    return check_launch();
 }
 
 int mlcgb_graph_capacity(const void *pos, int dtype, const int64_t *n_atoms, int64_t *ptr, int64_t N, int64_t B, double r, int64_t max_nn, int rule,

@@ -167,3 +167,59 @@ def test_a_list_without_a_plan_is_reported_and_stays_inside(how):
         inside = b[guard:guard + k]
         assert int(inside.min()) >= 0 and int(inside.max()) < most
         assert bool((b[:guard] == mark).all()) and bool((b[guard + k:] == mark).all())
+
+
+@pytest.mark.parametrize("sizes", [[2], [31, 0, 33], [2048], [2049], [1] * 2000 + [60], [384, 385] * 30, [700] * 4, [768, 5, 0, 1200], [4600, 4601, 10, 385], [385] * 47, [385] * 48, [8192, 5000],
+                                   [8193, 300], [8193] + [20] * 60, [100] * 30])
+def test_plan_of_a_list_given_later(sizes):
+    """The plan made of a list when it is first used is the one that the separate entry point gives, whatever the route to it."""
+    from mlcg_b200 import radius_graph
+    from mlcg_b200.autograd import plan_of
+    from mlcg_b200.neighbor_list import radius_cuda
+    gen, be, n = torch.Generator().manual_seed(len(sizes) + sizes[0]), get_backend(), sum(sizes)
+    pos = (torch.rand(n, 3, generator=gen) * max(sizes) ** (1 / 3) * 2.0).to(DEV)
+    batch = torch.repeat_interleave(torch.arange(len(sizes)), torch.tensor(sizes)).to(DEV)
+    ptr = torch.tensor([0] + sizes, device=DEV).cumsum(0)
+    for edges in (radius_graph(pos, 4.0, batch, max_num_neighbors=1000, flow="target_to_source"), radius_cuda(pos, ptr, 4.0, 1000, True)[0]):
+        plan = plan_of(edges, n)
+        assert torch.equal(torch.stack([plan.row0, plan.row1]).long(), edges) and plan.symmetric
+        if edges.shape[1] == 0:
+            continue
+        offsets = torch.cat([torch.zeros(1, dtype=torch.int64, device=DEV), torch.bincount(edges[0], minlength=n).cumsum(0)])
+        twin, sel, pair_of, status = be.pair_plan(plan.row0.clone(), plan.row1.clone(), offsets, n, fresh_status=True)
+        assert int(status[0]) == 0 and torch.equal(plan.ptr_out, offsets)
+        assert torch.equal(plan.perm_in, twin) and torch.equal(plan.half_selection(), sel) and torch.equal(plan.pair_index(), pair_of)
+        assert plan_of(edges, n) is plan
+    be.check_pending()
+    assert int(be._sticky_status(torch.device(DEV))[0]) == 0
+
+
+@pytest.mark.parametrize("sizes", [[300], [400] * 60, [3000, 100]])
+@pytest.mark.parametrize("how", ["shuffled", "another structure", "other centres", "no bead", "one named by all"])
+def test_a_list_changed_behind_its_version_is_reported(sizes, how):
+    """Writes that a list does not count (``.data``) before its plan is made: reported, and every entry of the plan is an index."""
+    from mlcg_b200 import radius_graph
+    from mlcg_b200.autograd import plan_of
+    gen, be, n = torch.Generator().manual_seed(5), get_backend(), sum(sizes)
+    pos = (torch.rand(n, 3, generator=gen) * max(sizes) ** (1 / 3) * 2.0).to(DEV)
+    batch = torch.repeat_interleave(torch.arange(len(sizes)), torch.tensor(sizes)).to(DEV)
+    edges = radius_graph(pos, 4.0, batch, max_num_neighbors=1000, flow="target_to_source")
+    E = edges.shape[1]
+    if how == "shuffled":
+        edges.data[1] = edges[1][torch.randperm(E, generator=gen).to(DEV)]
+    elif how == "another structure":
+        edges.data[1] = (edges[1] + sizes[0] // 2 + 1) % n
+    elif how == "other centres":
+        edges.data[0] = edges[0].flip(0)
+    elif how == "no bead":
+        edges.data[1, ::7] = n + 5
+        edges.data[1, 3::7] = -1
+    else:
+        edges.data[1] = sizes[0] // 2
+    status = be._sticky_status(torch.device(DEV))
+    status.zero_()
+    plan = plan_of(edges, n)
+    assert int(status[0]) & 4
+    status.zero_()
+    for t, most in ((plan.row0, n), (plan.row1, n), (plan.perm_in, E), (plan.half_selection(), E), (plan.pair_index(), E // 2)):
+        assert int(t.min()) >= 0 and int(t.max()) < most
