@@ -91,6 +91,11 @@ __device__ __forceinline__ float ex2_fast(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+__device__ __forceinline__ float min_nan(float x, float y) {      // (fminf gives the number where one of the two is none)
+    float m;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(x), "f"(y));
+    return m;
+}
 // Per-edge part of the basis: value t(d) the basis functions are centred on and its derivative.
 //   Gaussian:   g_k = exp(coeff (d - offset_k)^2)                 t = d,                 t' = 1
 //   exp-normal: g_k = exp(-beta_k (u - mean_k)^2), u = exp(alpha (lower - d)):  t = u,   t' = -alpha u
@@ -163,7 +168,7 @@ __device__ __forceinline__ void tanh_row32(float (&v)[NC], const float *s_b1s, i
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 zz[i] = tc::fma2(make_float2(v[4 * q + 2 * i], v[4 * q + 2 * i + 1]), both(unscale2), make_float2(bb[2 * i], bb[2 * i + 1]));
-                den[i] = tc::add2(make_float2(ex2_fast(fminf(fabsf(zz[i].x), 30.f)), ex2_fast(fminf(fabsf(zz[i].y), 30.f))), both(1.f));
+                den[i] = tc::add2(make_float2(ex2_fast(min_nan(fabsf(zz[i].x), 30.f)), ex2_fast(min_nan(fabsf(zz[i].y), 30.f))), both(1.f));
             }
             // (products of the first and of the second of each pair, so that the pairs stay pairs)
             const float2 p = tc::mul2(den[0], den[1]);

@@ -278,3 +278,30 @@ def test_lists_without_room_for_an_edge(sizes, box, edges):
         assert code == 0 and int(status[0]) == (32 if edges else 0)
         status.zero_()
         assert torch.allclose(energy, want, rtol=1e-5, atol=1e-5 * float(want.abs().max())) and not grad.any()
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+@pytest.mark.parametrize("num_rbf", [128, 50, 33])
+@pytest.mark.parametrize("copies", [3, 600])
+def test_a_weight_that_is_not_a_number_reaches_the_results(copies, num_rbf, precision):
+    """Energies and forces are no numbers either, in batches of both routes."""
+    torch.manual_seed(4)
+    cut = bnn.CosineCutoff(0.0, 10.0)
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, num_rbf, trainable=False), cut, [128], hidden_channels=128, embedding_size=4, num_filters=128, num_interactions=2)
+    model = bnn.GradientsOut(bnn.set_filter_precision(net.to(DEV).eval(), precision), "forces").eval()
+    pos = random_walk_chain(5, torch.Generator().manual_seed(1), min_dist=3.8).repeat(copies, 1).to(DEV)
+    batch = torch.arange(copies, device=DEV).repeat_interleave(5)
+    data = lambda: mlcg_b200.AtomicData(pos=pos.clone(), atom_types=torch.zeros(5 * copies, dtype=torch.int64, device=DEV), batch=batch,  # noqa: E731
+                                        n_atoms=torch.full((copies,), 5, device=DEV))
+    want = model(data()).out["SchNet"]
+    assert bool(want["energy"].isfinite().all() and want["forces"].isfinite().all())
+    layers = net.interaction_blocks[1].conv.filter_network.layers
+    for weight, places in ((layers[0].bias, ((5,),)), (layers[2].weight, ((3, 64),))):
+        for at in places:
+            before = weight.data[at].clone()
+            weight.data[at] = float("nan")
+            out = model(data()).out["SchNet"]
+            assert bool(out["energy"].isnan().all()) and bool(out["forces"].isnan().all()), (tuple(weight.shape), at)
+            weight.data[at] = before
+    again = model(data()).out["SchNet"]
+    assert torch.equal(again["energy"], want["energy"]) and torch.equal(again["forces"], want["forces"])
