@@ -119,7 +119,7 @@ __device__ __forceinline__ uint32_t filter_setup(const FilterFwdParams &p, uint8
     const int tid = threadIdx.x, warp = tid >> 5;
     const float wscale = SPLIT ? kWScale : 1.f;
     if (!have_weights) {
-        const bool over1 = load_weight_tile<SPLIT>(smem + L::kB1, smem + L::kB1 + 32768, p.A1, kF, p.rbf.R, Kpad1, wscale);
+        const bool over1 = load_weight_tile<SPLIT>(smem + L::kB1, smem + L::kB1 + 32768, p.A1, kF, p.rbf.R, Kpad1, wscale, true);
         const bool over2 = load_weight_tile<SPLIT>(smem + L::kB2, smem + L::kB2 + 32768, p.A2, kF, kF, kF, wscale);
         if ((over1 || over2) && blockIdx.x == 0) atomicOr(p.status, (int)kWeightRange);
     }

@@ -100,7 +100,9 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
     // 2^-25), and so is its derivative on the scale of its row (below 16 (z / 0.6065 + 1) 2^-36 < 2^-28 at z = 7.1 widths).  Exp-normal
     // functions crowd the short distances that no bead comes to: of 128 over 15 A those beyond the 45th are zero at 4 A and more,
     // over 10 A those beyond the 29th.  A warp whose 32 rows are all outside stores zeros, and the first GEMMs leave a quarter of K out that
-    // is zero in the whole tile: the same sums, bit by bit.
+    // is zero in the whole tile: the same sums, bit by bit, in the mode of fp16 pairs.  The operands of the bf16 mode
+    // reach further down: there the values left out are below 2^-36 where its rounding of the others is 2^-9 of them.  A weight that is not a
+    // number is so in its whole row (spread_nan) and reaches the sums through the quarter that is always there.
     float near_lo = INFINITY, near_hi = -INFINITY;
     for (int k = col0; k < col0 + 32 && k < R; k++) {
         const float2 cw = s_tab[k];

@@ -129,18 +129,19 @@ embedding_rows_kernel(const float *__restrict__ table, const int64_t *__restrict
         const int k = blockIdx.x >> 3, cols = im.cols[k], pad = cols <= 64 ? 64 : 128;
         uint8_t *hi = im.dst + k * kWeightImage;
         float most = 0.f;
+        const bool first_layer = k >= im.first_filter && ((k - im.first_filter) & 1) == 0;
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const int row = (blockIdx.x & 7) * 16 + u * 8 + (threadIdx.x >> 5), col = (threadIdx.x & 31) * 4;
-            if (col >= pad) continue;
             const float *src = im.src[k] + row * cols + col;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (row < im.rows[k]) {
+            if (row < im.rows[k] && col < pad) {
                 if (col + 4 <= cols && ((uintptr_t)src & 15) == 0) v = *reinterpret_cast<const float4 *>(src);
                 else
                     v = make_float4(col < cols ? src[0] : 0.f, col + 1 < cols ? src[1] : 0.f, col + 2 < cols ? src[2] : 0.f, col + 3 < cols ? src[3] : 0.f);
             }
-            most = fmaxf(most, tc::put_weight4<true>(hi, hi + kWeightImage / 2, row, col, v, 64.f));
+            if (first_layer) v = tc::spread_nan(v, 32);
+            if (col < pad) most = fmaxf(most, tc::put_weight4<true>(hi, hi + kWeightImage / 2, row, col, v, 64.f));
         }
         if (!(most * 64.f <= 32768.f)) atomicOr(status, (int)kWeightRange);
         return;
@@ -175,6 +176,7 @@ int embedding_launch(const mlcgb_schnet_weights *w, const int64_t *types, int64_
     TimelineScope timeline_scope("embedding", st);
     WeightImages im;
     im.n = 0;
+    im.first_filter = kMaxImages;
     im.dst = (uint8_t *)images;
     auto add = [&](const void *src, int64_t rows, int cols = 128) {          // (a weight that is not there is refused by the kernel that takes it)
         im.src[im.n] = (const float *)src;
@@ -188,6 +190,7 @@ int embedding_launch(const mlcgb_schnet_weights *w, const int64_t *types, int64_
             add(w->blocks[l].lin_w, 128);
         }
         add(w->head_W, w->head_width);
+        im.first_filter = im.n;
         for (int64_t l = 0; l < w->num_blocks && num_rbf; l++) {
             add(w->blocks[l].filter_w1, 128, num_rbf);
             add(w->blocks[l].filter_w2, 128);

@@ -19,7 +19,7 @@ constexpr int kMaxImages = 5 * kMaxBlocks + 1;
 struct WeightImages {
     const float *src[kMaxImages];
     int16_t rows[kMaxImages], cols[kMaxImages];
-    int n;
+    int n, first_filter;                   // (of the filters' weights; every other one from there on is a filter_w1)
     uint8_t *dst;
 };
 inline int64_t weight_images_floats(int64_t num_blocks) { return (5 * num_blocks + 1) * (kWeightImage / 4); }

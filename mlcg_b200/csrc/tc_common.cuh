@@ -199,14 +199,25 @@ __device__ __forceinline__ float put_weight4(uint8_t *hi, uint8_t *lo, int n, in
     }
     return fmaxf(fmaxf(fabsf(w.x), fabsf(w.y)), fmaxf(fabsf(w.z), fabsf(w.w)));
 }
+// A quad of a weight's row, `lanes` lanes a row: not a number anywhere in the row makes the whole row so.  A GEMM that leaves out the part of
+// K where its other operand is zero then gives what the whole one gives.  By all lanes of a warp.
+__device__ __forceinline__ float4 spread_nan(float4 w, int lanes) {
+    const float s = (w.x + w.y) + (w.z + w.w);
+    const bool bad = s != s && (w.x != w.x || w.y != w.y || w.z != w.z || w.w != w.w);
+    const unsigned all = __ballot_sync(0xffffffffu, bad), row = lanes == 32 ? all : all >> (threadIdx.x & 16) & 0xffffu;
+    if (row == 0) return w;
+    const float nan = __int_as_float(0x7fffffff);
+    return make_float4(nan, nan, nan, nan);
+}
 // Fill a [128][Kpad] weight tile (and its low part) from a row-major fp32 matrix src[rows][K], scaled by `scale`.
 // Four consecutive K elements of a row are 8 contiguous bytes of the swizzled tile, so with K % 4 == 0 and a 16-byte
 // aligned source every thread moves float4 -> 8 bytes, with all its loads issued before the first conversion.
 // Returns true if this thread saw a scaled weight too large for a 16-bit operand (|w * scale| > 32768 with fp16 pairs):
-// the caller reports it through its status word instead of computing with infinities.
+// the caller reports it through its status word instead of computing with infinities.  A weight that is not a number is not reported:
+// it makes results that are none (`spread`: see above; Kpad 64 or 128, whole warps).
 template <bool SPLIT>
 __device__ __forceinline__ bool load_weight_tile(uint8_t *hi, uint8_t *lo, const float *__restrict__ src, int rows, int K, int Kpad,
-                                                 float scale) {
+                                                 float scale, bool spread = false) {
     float wmax = 0.f;
     auto put4 = [&](int n, int k, float4 w) { wmax = fmaxf(wmax, put_weight4<SPLIT>(hi, lo, n, k, w, scale)); };
     const int qpr = Kpad >> 2, nquads = kRows * qpr;          // quads per row, quads in the tile
@@ -219,6 +230,10 @@ __device__ __forceinline__ bool load_weight_tile(uint8_t *hi, uint8_t *lo, const
                 const int qd = base + u * blockDim.x;
                 const int n = qd / qpr, k = (qd - n * qpr) << 2;
                 w[u] = (qd < nquads && n < rows && k < K) ? __ldg(reinterpret_cast<const float4 *>(src + (int64_t)n * K + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            if (spread) {
+#pragma unroll
+                for (int u = 0; u < kBatch; u++) w[u] = spread_nan(w[u], qpr);
             }
 #pragma unroll
             for (int u = 0; u < kBatch; u++) {
@@ -236,9 +251,10 @@ __device__ __forceinline__ bool load_weight_tile(uint8_t *hi, uint8_t *lo, const
         float v[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) v[j] = (n < rows && k + j < K) ? src[(int64_t)n * K + k + j] : 0.f;
-        put4(n, k, make_float4(v[0], v[1], v[2], v[3]));
+        const float4 w = make_float4(v[0], v[1], v[2], v[3]);
+        put4(n, k, spread ? spread_nan(w, qpr) : w);
     }
-    return SPLIT && !(wmax * scale <= 32768.f);     // (also true for NaN weights)
+    return SPLIT && !(wmax * scale <= 32768.f);
 }
 
 // ---- A operand in tensor memory -----------------------------------------------------------------------

@@ -284,7 +284,8 @@ def test_lists_without_room_for_an_edge(sizes, box, edges):
 @pytest.mark.parametrize("num_rbf", [128, 50, 33])
 @pytest.mark.parametrize("copies", [3, 600])
 def test_a_weight_that_is_not_a_number_reaches_the_results(copies, num_rbf, precision):
-    """Energies and forces are no numbers either, in batches of both routes."""
+    """Also where it stands in a column of the filter network's first layer that the basis does not reach: energies and forces are no
+    numbers either, in batches of both routes."""
     torch.manual_seed(4)
     cut = bnn.CosineCutoff(0.0, 10.0)
     net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, num_rbf, trainable=False), cut, [128], hidden_channels=128, embedding_size=4, num_filters=128, num_interactions=2)
@@ -296,7 +297,7 @@ def test_a_weight_that_is_not_a_number_reaches_the_results(copies, num_rbf, prec
     want = model(data()).out["SchNet"]
     assert bool(want["energy"].isfinite().all() and want["forces"].isfinite().all())
     layers = net.interaction_blocks[1].conv.filter_network.layers
-    for weight, places in ((layers[0].bias, ((5,),)), (layers[2].weight, ((3, 64),))):
+    for weight, places in ((layers[0].weight, ((0, 0), (17, num_rbf - 1), (127, num_rbf // 2))), (layers[0].bias, ((5,),)), (layers[2].weight, ((3, 64),))):
         for at in places:
             before = weight.data[at].clone()
             weight.data[at] = float("nan")
