@@ -47,7 +47,8 @@ int mlcgb_last_cuda_error(void); /* cudaError_t of the last failed launch on thi
  *        NULL), negate and the totals are new, fixed_point = 0 writes its outputs too (it added to them), the workspace is wanted in
  *        both modes and mlcgb_prior_eval_workspace_bytes takes the dtype where it took fixed_point.  mlcgb_gemm_tc_chain2 with
  *        backward = 1 writes mid_out unless it is NULL.
- *   300  mlcgb_prior_list_make: host_out has three values. */
+ *   300  mlcgb_prior_list_make: host_out has three values.  mlcgb_seg_force wants its first output.  mlcgb_batch_structures is gone
+ *        (mlcgb_batch_boundaries). */
 #define MLCGB_VERSION 300
 int mlcgb_version(void);
 
@@ -150,9 +151,8 @@ int mlcgb_pair_index(const int32_t *sel /* [P] */, const int32_t *twin /* [E] */
  *   graph_capacity: both without a host read into buffers of `capacity` edges (an even number), counts as in
  *     mlcgb_radius_graph_capacity; index entries past the live ones are left as they were.
  * N, B > 0.  Excluded pairs go with rule 0 and are given to both calls. */
-/* Structures of a sorted batch vector (batch[N-1] + 1), read on the host as above. */
-int mlcgb_batch_structures(const int64_t *batch, int64_t N, int64_t *host_out, void *stream);
-/* The same and the boundaries ptr [most + 1] of up to `most` structures, in one launch (more of them: mlcgb_batch_to_ptr). */
+/* Structures of a sorted batch vector (batch[N-1] + 1), read on the host as above, and the boundaries ptr [most + 1] of up to `most`
+ * structures, in one launch (more of them: mlcgb_batch_to_ptr). */
 int mlcgb_batch_boundaries(const int64_t *batch, int64_t N, int64_t most, int64_t *ptr, int64_t *host_out, void *stream);
 /* graph_begin / graph_finish for up to 2048 points given with their batch vector (sorted; NULL: one structure): edges and distances
  * (or NULL), no plan.  Workspace: mlcgb_graph_workspace_bytes(N, 1, dtype). */
@@ -374,7 +374,7 @@ int mlcgb_tanh_grad(int mode, const void *G, const void *g, const void *y, int d
 
 /* Aggregations over filter rows W [P,F], one per unordered pair, and their distance derivatives Wd = dW/dd (float32, F = 128,
  * symmetric centre-sorted list ptr / nbr with its pair index pair_of):
- *   seg_force:    out[i] = sum_j a[j] W[p] (out NULL: not wanted),  s[e] = (accumulate ? s[e] : 0) + sum_f (x[i] a[j] Wd[p])_f
+ *   seg_force:    out[i] = sum_j a[j] W[p],  s[e] = (accumulate ? s[e] : 0) + sum_f (x[i] a[j] Wd[p])_f
  *   seg_tangent:  out[i] = sum_j a[j] W[p] + b[j] (dd[e] Wd[p])   (a NULL: zero)
  *   edge_tangent: dd[e] = change of the distance of edge e when the positions move along v */
 int mlcgb_seg_force(const void *a, const void *x, const void *W, const void *Wd, const int64_t *ptr, const int32_t *nbr, const int32_t *pair_of,

@@ -110,7 +110,6 @@ SIGNATURES = {
                                           c_dbl, c_vp, c_int, c_vp, c_sz, c_vp, c_vp, c_vp, c_vp]),
     "mlcgb_schnet_energy_forces": (c_int, [c_vp, c_vp, c_vp, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_i64, c_i64, c_vp, c_vp, c_int, c_dbl,
                                            c_dbl, c_vp, c_int, c_vp, c_sz, c_vp, c_vp, c_vp, c_vp]),
-    "mlcgb_batch_structures": (c_int, [c_vp, c_i64, c_vp, c_vp]),
     "mlcgb_schnet_evaluate_workspace_bytes": (c_sz, [c_i64] * 4 + [ctypes.POINTER(SchnetWeightsStruct), c_int]),
     "mlcgb_schnet_evaluate_lists": (None, [c_i64, c_i64, c_i64, c_vp]),
     "mlcgb_schnet_evaluate": (c_int, [c_vp, c_vp, c_vp, c_vp, c_i64, c_i64, c_dbl, c_i64, ctypes.POINTER(RbfSpecStruct), c_int, c_dbl, c_dbl,

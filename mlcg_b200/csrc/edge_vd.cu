@@ -4,7 +4,6 @@
 // 16 bytes of a row: no synchronisation beyond the copy groups), node rows through registers.  Sums in edge order, no atomics.
 //
 //   force    out[i] = sum_j a[j] W[p]          s[e] (+)= sum_f (x[i] a[j] W'[p])_f          e = (i, j), p = its pair
-//   dot      the second of these alone
 //   tangent  out[i] = sum_j a[j] W[p] + b[j] (dd[e] W'[p])
 //
 // `force` is the step of the force pass that used to be an aggregation and a backward pass of the filter network: gd of a pair is
@@ -14,13 +13,13 @@
 
 namespace mlcgb {
 
-enum { kSegForce = 0, kSegDot = 1, kSegTangent = 2, kSegTangentRows = 3 };     // the last: tangent with a = 0
+enum { kSegForce = 0, kSegTangent = 1, kSegTangentRows = 2 };     // the last: tangent with a = 0
 constexpr int kVdWarps = 8;
 // Rows in flight per warp and blocks per SM.  The rings take first-level cache from the node rows, which are read again and again
 // while a structure is worked on: eight rows (or pairs of rows) and three blocks took 313 us for three `force` launches over 1.1 M
-// edges, 131 us for a `dot`; four and four blocks 286 and 114.  A tangent holds too much in registers for four blocks (324 against 297).
-template <int MODE> constexpr int kVdSlots = MODE == kSegForce || MODE == kSegDot ? 4 : 8;
-template <int MODE> constexpr int kVdBlocks = MODE == kSegForce || MODE == kSegDot ? 4 : 3;
+// edges; four and four blocks 286.  A tangent holds too much in registers for four blocks (324 against 297).
+template <int MODE> constexpr int kVdSlots = MODE == kSegForce ? 4 : 8;
+template <int MODE> constexpr int kVdBlocks = MODE == kSegForce ? 4 : 3;
 
 __device__ __forceinline__ void fma4(float4 &acc, const float4 &a, const float4 &b) {
     acc.x = fmaf(a.x, b.x, acc.x); acc.y = fmaf(a.y, b.y, acc.y); acc.z = fmaf(a.z, b.z, acc.z); acc.w = fmaf(a.w, b.w, acc.w);
@@ -138,8 +137,7 @@ seg_vd_kernel(const float *__restrict__ a, const float *__restrict__ x, const fl
                 __syncwarp();
             }
         }
-        if (MODE != kSegDot)
-            reinterpret_cast<float4 *>(out)[n * 32 + lane] = make_float4(acc0.x + acc1.x, acc0.y + acc1.y, acc0.z + acc1.z, acc0.w + acc1.w);
+        reinterpret_cast<float4 *>(out)[n * 32 + lane] = make_float4(acc0.x + acc1.x, acc0.y + acc1.y, acc0.z + acc1.z, acc0.w + acc1.w);
     }
 }
 
@@ -253,9 +251,8 @@ int mlcgb_seg_force(const void *a, const void *x, const void *W, const void *Wd,
     if (N < 0) return MLCGB_E_ARG;
     if (F != 128) return MLCGB_E_LIMIT;
     if (N == 0) return MLCGB_OK;
-    if (!a || !x || !ptr) return MLCGB_E_ARG;
-    if (out) return seg_vd_launch<kSegForce>(a, x, W, Wd, ptr, nbr, pair_of, N, out, s, accumulate, (cudaStream_t)stream);
-    return seg_vd_launch<kSegDot>(a, x, W, Wd, ptr, nbr, pair_of, N, out, s, accumulate, (cudaStream_t)stream);
+    if (!a || !x || !ptr || !out) return MLCGB_E_ARG;
+    return seg_vd_launch<kSegForce>(a, x, W, Wd, ptr, nbr, pair_of, N, out, s, accumulate, (cudaStream_t)stream);
 }
 
 int mlcgb_seg_tangent(const void *a, const void *b, const void *W, const void *Wd, const void *dd, const int64_t *ptr, const int32_t *nbr,

@@ -2270,9 +2270,7 @@ static GraphLayout graph_layout(int64_t N, int64_t B, int dtype) {
 }
 static inline bool mask_route(int64_t N, int64_t B, const Exclusion &ex) { return N <= kMaskNodes && B <= kMaskStructs && !ex.ptr; }
 
-__global__ void last_of_kernel(const int64_t *__restrict__ last, Publish p) { publish(p, *last, 0); }
-
-// The same and the boundaries, for up to `most` structures: the host reads on while they are looked for
+// The last entry of a batch vector to the host, and the boundaries of up to `most` structures: the host reads on while they are looked for
 __global__ void batch_boundaries_kernel(const int64_t *__restrict__ batch, int64_t N, int64_t most, int64_t *__restrict__ ptr, Publish p) {
     const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, last = batch[N - 1];
     if (b == 0) publish(p, last, 0);
@@ -3064,18 +3062,6 @@ int publish_wait(const Publish &p, cudaStream_t st) { return wait_published(p.se
 }  // namespace mlcgb
 
 extern "C" {
-
-int mlcgb_batch_structures(const int64_t *batch, int64_t N, int64_t *host_out, void *stream) {
-    if (N <= 0 || !batch || !host_out) return MLCGB_E_ARG;
-    auto st = (cudaStream_t)stream;
-    Publish pub;
-    if (int rc = publish_begin(&pub)) return rc;
-    last_of_kernel<<<1, 1, 0, st>>>(batch + N - 1, pub);
-    if (int rc = check_launch()) return rc;
-    if (int rc = publish_wait(pub, st)) return rc;
-    *host_out = pub.host[1] + 1;
-    return MLCGB_OK;
-}
 
 int mlcgb_batch_boundaries(const int64_t *batch, int64_t N, int64_t most, int64_t *ptr, int64_t *host_out, void *stream) {
     if (N <= 0 || most < 0 || !batch || !ptr || !host_out) return MLCGB_E_ARG;
