@@ -2338,53 +2338,14 @@ mask_count_kernel(const T *__restrict__ pos, const int64_t *__restrict__ sizes, 
             lo = s_ptr[b];
             hi = min(s_ptr[b + 1], (int)N);
         }
-        const int n = hi - lo, il = i - lo;
-        const T xi = pos[3 * ci], yi = pos[3 * ci + 1], zi = pos[3 * ci + 2];
-        unsigned m0 = 0, m1 = 0;                       // words `lane` and `32 + lane` of the row
-        for (int jb = 0; jb < n; jb += 32) {
-            const int j = jb + lane;
-            bool hit = false;
-            if (j < n) {
-                const T *q = pos + 3 * ((int64_t)lo + j);
-                hit = dist2_rn(xi, yi, zi, q[0], q[1], q[2]) < r2;
-            }
-            const unsigned bal = __ballot_sync(0xffffffffu, hit);
-            const int w = jb >> 5;
-            if (w == lane) m0 = bal;
-            if (w == lane + 32) m1 = bal;
-        }
-        const int sw = il >> 5;                        // the centre's own word and bit
-        const unsigned own = sw < 32 ? __shfl_sync(0xffffffffu, m0, sw) : __shfl_sync(0xffffffffu, m1, sw & 31);
-        const int self_hit = own >> (il & 31) & 1;
-        if (!loop && self_hit) {
-            if (lane == sw) m0 &= ~(1u << (il & 31));
-            if (lane + 32 == sw) m1 &= ~(1u << (il & 31));
-        }
-        int p0 = __popc(m0), p1 = __popc(m1);
-        const int c0 = p0, c1 = p1;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t0 = __shfl_up_sync(0xffffffffu, p0, o), t1 = __shfl_up_sync(0xffffffffu, p1, o);
-            if (lane >= o) { p0 += t0; p1 += t1; }
-        }
-        const int first = __shfl_sync(0xffffffffu, p0, 31), total_hits = first + __shfl_sync(0xffffffffu, p1, 31);
-        p0 -= c0;                                      // hits before the word
-        p1 += first - c1;
-        uint2 *row = masks + ci * words;
-        const int nw = (n + 31) >> 5;
-        if (lane < nw) row[lane] = make_uint2((unsigned)p0, m0);
-        if (lane + 32 < nw) row[lane + 32] = make_uint2((unsigned)p1, m1);
-        // hits before the centre
-        const unsigned below = (1u << (il & 31)) - 1u;
-        const int nlo0 = p0 + __popc(m0 & below), nlo1 = p1 + __popc(m1 & below);
-        const int nlo = sw < 32 ? __shfl_sync(0xffffffffu, nlo0, sw) : __shfl_sync(0xffffffffu, nlo1, sw & 31);
+        const RowHits h = row_of_bits<T>(pos, ci, lo, hi - lo, r2, loop, masks + ci * words, lane);
         if (lane == 0) {
-            const int64_t total = total_hits;          // (with loop: the centre itself among them)
+            const int64_t total = h.total;             // (with loop: the centre itself among them)
             int64_t k;
-            if (!loop && rule == MLCGB_RULE_CLUSTER && self_hit && nlo >= max_nn + 1) k = max_nn + 1;
+            if (!loop && rule == MLCGB_RULE_CLUSTER && h.own && h.before_own >= max_nn + 1) k = max_nn + 1;
             else k = total < max_nn ? total : max_nn;
             deg[i] = (int32_t)k;
-            upper[i] = (int32_t)(k > nlo ? k - nlo : 0);
+            upper[i] = (int32_t)(k > h.before_own ? k - h.before_own : 0);
             if (k < total) atomicOr(status, (int)kTruncated);
         }
     }
@@ -2451,9 +2412,16 @@ mask_fill_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, int
     __shared__ int s_ptr[BATCH ? 1 : kMaskStructs + 1];
     if constexpr (!BATCH) load_boundaries<256>(s_ptr, nullptr, const_cast<int64_t *>(ptr), B);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned lt = lanemask_lt();
     const int64_t P = offsets[N] >> 1;
     if (twin && (offsets[N] & 1) && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(sticky, (int)kAsymmetric);
+    struct {
+        const int64_t *offsets;
+        const int32_t *upper, *uoff;
+        __device__ int64_t first(int k) const { return offsets[k]; }
+        __device__ int kept(int k) const { return (int)(offsets[k + 1] - offsets[k]); }
+        __device__ int lower(int k) const { return kept(k) - upper[k]; }
+        __device__ int64_t pairs(int k) const { return uoff[k]; }
+    } const at = {offsets, upper, uoff};
     for (int64_t ci = (int64_t)blockIdx.x * 8 + warp; ci < N; ci += (int64_t)gridDim.x * 8) {
         const int i = (int)ci;
         int b = 0, lo = 0, hi = (int)N;
@@ -2464,38 +2432,22 @@ mask_fill_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, int
             lo = s_ptr[b];
             hi = min(s_ptr[b + 1], (int)N);
         }
-        const int n = hi - lo, il = i - lo;
         const int64_t off = offsets[i];
-        const int kept = (int)(offsets[i + 1] - off), nw = (n + 31) >> 5;
+        const int kept = (int)(offsets[i + 1] - off);
         if (kept == 0) continue;
-        const int up = upper[i], nlower = kept - up, uo = uoff[i];
-        const uint2 *row = masks + ci * words;
-        for (int w0 = 0; w0 < nw; w0 += 32) {
-            const uint2 mine = w0 + lane < nw ? row[w0 + lane] : make_uint2(0u, 0u);
-            const int take = nw - w0 < 32 ? nw - w0 : 32;
-            for (int w = 0; w < take; w++) {
-                const unsigned bits = __shfl_sync(0xffffffffu, mine.y, w);
-                const int rank = (int)__shfl_sync(0xffffffffu, mine.x, w) + __popc(bits & lt);
-                const int jl = (w0 + w) * 32 + lane;
-                if (!(bits >> lane & 1u) || rank >= kept) continue;
-                const int64_t slot = off + rank, j = lo + jl;
-                T d2 = T(0);
-                if (out.distance) d2 = dist2_rn(pos[3 * ci], pos[3 * ci + 1], pos[3 * ci + 2], pos[3 * j], pos[3 * j + 1], pos[3 * j + 2]);
-                emit_edge<T>(out, slot, i, j, b, d2);
-                if (!twin) continue;
-                const uint2 rev = masks[j * words + (il >> 5)];
-                const int rank_j = (int)rev.x + __popc(rev.y & ((1u << (il & 31)) - 1u));
-                const int64_t off_j = offsets[j];
-                const int kept_j = (int)(offsets[j + 1] - off_j);
-                const int64_t p = j > i ? (int64_t)uo + (rank - nlower) : (int64_t)uoff[j] + (rank_j - (kept_j - upper[j]));
-                // not a valid plan (a list was cut short): reported, and every index written stays inside its array
-                const bool ok = rank_j < kept_j && (rev.y >> (il & 31) & 1u) && i != j && p >= 0 && p < P;
-                if (!ok) atomicOr(sticky, (int)kAsymmetric);
-                twin[slot] = (int32_t)(ok ? off_j + rank_j : slot);
-                pair_of[slot] = (int32_t)(ok ? p : 0);
-                if (ok && j > i) sel[p] = (int32_t)slot;
-            }
-        }
+        each_hit(masks + ci * words, (hi - lo + 31) >> 5, kept, lane, [&](int rank, int jl) {
+            const int64_t slot = off + rank, j = lo + jl;
+            T d2 = T(0);
+            if (out.distance) d2 = dist2_rn(pos[3 * ci], pos[3 * ci + 1], pos[3 * ci + 2], pos[3 * j], pos[3 * j + 1], pos[3 * j + 2]);
+            emit_edge<T>(out, slot, i, j, b, d2);
+            if (!twin) return;
+            const PairPlace place = pair_place(masks, words, i, i - lo, (int)j, rank, P, at);
+            // not a valid plan (a list was cut short): reported, and every index written stays inside its array
+            if (!place.ok) atomicOr(sticky, (int)kAsymmetric);
+            twin[slot] = (int32_t)(place.ok ? place.twin : slot);
+            pair_of[slot] = (int32_t)(place.ok ? place.pair : 0);
+            if (place.ok && j > i) sel[place.pair] = (int32_t)slot;
+        });
     }
 }
 

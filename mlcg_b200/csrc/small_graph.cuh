@@ -67,6 +67,82 @@ __device__ __forceinline__ int structure_of(const int *s_ptr, int64_t B, int i) 
     return lo;
 }
 
+// ---- rows of bits: a warp tests the points of a centre's structure and keeps its hits, {hits before the word, word} per 32 points
+struct RowHits {
+    int total, before_own;                     // hits (without the centre unless `loop`), and those of points before it
+    bool own;                                  // the centre is within its own cutoff
+};
+// centre ci of the structure [lo, lo + n), n <= 2048, by the whole warp
+template <typename T>
+__device__ __forceinline__ RowHits row_of_bits(const T *__restrict__ pos, int64_t ci, int lo, int n, T r2, bool loop, uint2 *__restrict__ row, int lane) {
+    static_assert(kMaskNodes <= 64 * 32, "two words per lane");
+    const T xi = pos[3 * ci], yi = pos[3 * ci + 1], zi = pos[3 * ci + 2];
+    unsigned m0 = 0, m1 = 0;                   // words `lane` and `32 + lane` of the row
+    for (int jb = 0; jb < n; jb += 32) {
+        const int j = jb + lane;
+        bool hit = false;
+        if (j < n) {
+            const T *q = pos + 3 * ((int64_t)lo + j);
+            hit = dist2_rn(xi, yi, zi, q[0], q[1], q[2]) < r2;
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, hit);
+        const int w = jb >> 5;
+        if (w == lane) m0 = bal;
+        if (w == lane + 32) m1 = bal;
+    }
+    const int il = (int)ci - lo, sw = il >> 5;         // the centre's own word and bit
+    const unsigned own = sw < 32 ? __shfl_sync(0xffffffffu, m0, sw) : __shfl_sync(0xffffffffu, m1, sw & 31);
+    const bool self_hit = own >> (il & 31) & 1;
+    if (!loop && self_hit) {
+        if (lane == sw) m0 &= ~(1u << (il & 31));
+        if (lane + 32 == sw) m1 &= ~(1u << (il & 31));
+    }
+    int p0 = __popc(m0), p1 = __popc(m1);
+    const int c0 = p0, c1 = p1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t0 = __shfl_up_sync(0xffffffffu, p0, o), t1 = __shfl_up_sync(0xffffffffu, p1, o);
+        if (lane >= o) { p0 += t0; p1 += t1; }
+    }
+    const int first = __shfl_sync(0xffffffffu, p0, 31), total = first + __shfl_sync(0xffffffffu, p1, 31);
+    p0 -= c0;                                          // hits before the word
+    p1 += first - c1;
+    const int nw = (n + 31) >> 5;
+    if (lane < nw) row[lane] = make_uint2((unsigned)p0, m0);
+    if (lane + 32 < nw) row[lane + 32] = make_uint2((unsigned)p1, m1);
+    const unsigned below = (1u << (il & 31)) - 1u;
+    const int nlo0 = p0 + __popc(m0 & below), nlo1 = p1 + __popc(m1 & below);
+    const int nlo = sw < 32 ? __shfl_sync(0xffffffffu, nlo0, sw) : __shfl_sync(0xffffffffu, nlo1, sw & 31);
+    return {total, nlo, self_hit};
+}
+// f(rank, local index) for the first `kept` hits of a row of nw words, lane by lane
+template <typename F>
+__device__ __forceinline__ void each_hit(const uint2 *__restrict__ row, int nw, int kept, int lane, F &&f) {
+    const unsigned lt = lanemask_lt();
+    for (int w0 = 0; w0 < nw; w0 += 32) {
+        const uint2 mine = w0 + lane < nw ? row[w0 + lane] : make_uint2(0u, 0u);
+        for (unsigned live = __ballot_sync(0xffffffffu, mine.y != 0u); live; live &= live - 1) {
+            const int w = __ffs(live) - 1;
+            const unsigned bits = __shfl_sync(0xffffffffu, mine.y, w);
+            const int rank = (int)__shfl_sync(0xffffffffu, mine.x, w) + __popc(bits & lt);
+            if ((bits >> lane & 1u) && rank < kept) f(rank, (w0 + w) * 32 + lane);
+        }
+    }
+}
+// The reverse of the edge (i, j) that is hit `rank` of its row, and the pair of the two: from j's row at the word of i (local index il).
+// `at`: first edge, kept edges, lower ones among them and pairs before of a row.  Not ok where the list holds no plan (cut short, or sizes
+// that do not add up); every index is inside its array if it is.
+struct PairPlace {
+    int64_t twin, pair;
+    bool ok;
+};
+template <typename At>
+__device__ __forceinline__ PairPlace pair_place(const uint2 *__restrict__ masks, int words, int i, int il, int j, int rank, int64_t P, const At &at) {
+    const uint2 rev = masks[(int64_t)j * words + (il >> 5)];
+    const int rank_j = (int)rev.x + __popc(rev.y & ((1u << (il & 31)) - 1u));
+    const int64_t p = j > i ? at.pairs(i) + (rank - at.lower(i)) : at.pairs(j) + (rank_j - at.lower(j));
+    return {at.first(j) + rank_j, p, rank_j >= 0 && rank_j < at.kept(j) && (rev.y >> (il & 31) & 1u) && i != j && p >= 0 && p < P};
+}
 
 // radius_graph.cu: the calling thread's line of mapped memory for the next published result, and the wait for it
 int publish_begin(Publish *p);

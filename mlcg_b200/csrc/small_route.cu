@@ -527,52 +527,14 @@ small_graph_count_kernel(const float *__restrict__ pos, const SmallGraph g, int6
     load_boundaries<kST>(s_ptr, g.sizes, g.ptr, B);
     const int64_t ci = (int64_t)blockIdx.x * (kST / 32) + warp;
     if (ci >= N) return;
-    const int words = (int)((N + 31) >> 5);
-    const int i = (int)ci, b = structure_of(s_ptr, B, i), lo = s_ptr[b], n = min(s_ptr[b + 1], (int)N) - lo, il = i - lo;
-    const float xi = pos[3 * ci], yi = pos[3 * ci + 1], zi = pos[3 * ci + 2];
-    unsigned m0 = 0, m1 = 0;                           // words `lane` and `32 + lane` of the row
-    for (int jb = 0; jb < n; jb += 32) {
-        const int j = jb + lane;
-        bool hit = false;
-        if (j < n) {
-            const float *q = pos + 3 * ((int64_t)lo + j);
-            hit = dist2_rn(xi, yi, zi, q[0], q[1], q[2]) < r2;
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, hit);
-        const int w = jb >> 5;
-        if (w == lane) m0 = bal;
-        if (w == lane + 32) m1 = bal;
-    }
-    const int sw = il >> 5;                            // the bead's own word and bit
-    const unsigned own = sw < 32 ? __shfl_sync(0xffffffffu, m0, sw) : __shfl_sync(0xffffffffu, m1, sw & 31);
-    const int self_hit = own >> (il & 31) & 1;
-    if (self_hit) {
-        if (lane == sw) m0 &= ~(1u << (il & 31));
-        if (lane + 32 == sw) m1 &= ~(1u << (il & 31));
-    }
-    int p0 = __popc(m0), p1 = __popc(m1);
-    const int c0 = p0, c1 = p1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t0 = __shfl_up_sync(0xffffffffu, p0, o), t1 = __shfl_up_sync(0xffffffffu, p1, o);
-        if (lane >= o) { p0 += t0; p1 += t1; }
-    }
-    const int first = __shfl_sync(0xffffffffu, p0, 31), total = first + __shfl_sync(0xffffffffu, p1, 31);
-    p0 -= c0;                                          // hits before the word
-    p1 += first - c1;
-    uint2 *row = g.masks + ci * words;
-    const int nw = (n + 31) >> 5;
-    if (lane < nw) row[lane] = make_uint2((unsigned)p0, m0);
-    if (lane + 32 < nw) row[lane + 32] = make_uint2((unsigned)p1, m1);
-    const unsigned below = (1u << (il & 31)) - 1u;
-    const int nlo0 = p0 + __popc(m0 & below), nlo1 = p1 + __popc(m1 & below);
-    const int nlo = sw < 32 ? __shfl_sync(0xffffffffu, nlo0, sw) : __shfl_sync(0xffffffffu, nlo1, sw & 31);
+    const int i = (int)ci, b = structure_of(s_ptr, B, i), lo = s_ptr[b], n = min(s_ptr[b + 1], (int)N) - lo;
+    const RowHits h = row_of_bits<float>(pos, ci, lo, n, r2, false, g.masks + ci * ((N + 31) >> 5), lane);
     if (lane == 0) {
         // (the cluster rule keeps max_nn + 1 of a bead whose own index comes after as many hits)
-        const int64_t most = self_hit && nlo >= g.max_nn + 1 ? g.max_nn + 1 : g.max_nn;
-        const int k = total < most ? total : (int)most;
-        g.deg[i] = k | (k < total ? kDegCut : 0);
-        g.upper[i] = k > nlo ? k - nlo : 0;
+        const int64_t most = h.own && h.before_own >= g.max_nn + 1 ? g.max_nn + 1 : g.max_nn;
+        const int k = h.total < most ? h.total : (int)most;
+        g.deg[i] = k | (k < h.total ? kDegCut : 0);
+        g.upper[i] = k > h.before_own ? k - h.before_own : 0;
     }
 }
 
@@ -632,38 +594,31 @@ small_graph_fill_kernel(const float *__restrict__ pos, const SmallGraph g, int64
     }
     if (bad) return;
     __syncthreads();
-    const int words = (n_all + 31) >> 5, P = (int)(total >> 1);
-    const unsigned lt = lanemask_lt();
+    const int words = (n_all + 31) >> 5;
+    struct {
+        const int *off, *uoff;
+        __device__ int64_t first(int k) const { return off[k]; }
+        __device__ int kept(int k) const { return off[k + 1] - off[k]; }
+        __device__ int lower(int k) const { return kept(k) - (uoff[k + 1] - uoff[k]); }
+        __device__ int64_t pairs(int k) const { return uoff[k]; }
+    } const at = {s_off, s_uoff};
     for (int i = blockIdx.x * (kFillThreads / 32) + warp; i < n_all; i += gridDim.x * (kFillThreads / 32)) {
-        const int b = structure_of(s_ptr, B, i), lo = s_ptr[b], n = min(s_ptr[b + 1], n_all) - lo, il = i - lo;
-        const int off = s_off[i], kept = s_off[i + 1] - off, nw = (n + 31) >> 5;
+        const int b = structure_of(s_ptr, B, i), lo = s_ptr[b], n = min(s_ptr[b + 1], n_all) - lo;
+        const int off = s_off[i], kept = s_off[i + 1] - off;
         if (kept == 0) continue;
-        const int up = s_uoff[i + 1] - s_uoff[i], nlower = kept - up, uo = s_uoff[i];
-        const uint2 *row = g.masks + (int64_t)i * words;
         const float xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
-        for (int w0 = 0; w0 < nw; w0 += 32) {
-            const uint2 mine = w0 + lane < nw ? row[w0 + lane] : make_uint2(0u, 0u);
-            for (unsigned live = __ballot_sync(0xffffffffu, mine.y != 0u); live; live &= live - 1) {
-                const int w = __ffs(live) - 1;
-                const unsigned bits = __shfl_sync(0xffffffffu, mine.y, w);
-                const int rank = (int)__shfl_sync(0xffffffffu, mine.x, w) + __popc(bits & lt);
-                if (!(bits >> lane & 1u) || rank >= kept) continue;
-                const int slot = off + rank, j = lo + (w0 + w) * 32 + lane;
-                const uint2 rev = g.masks[(int64_t)j * words + (il >> 5)];
-                const float d2 = dist2_rn(xi, yi, zi, pos[3 * j], pos[3 * j + 1], pos[3 * j + 2]);
-                const int rank_j = (int)rev.x + __popc(rev.y & ((1u << (il & 31)) - 1u));
-                const int off_j = s_off[j], kept_j = s_off[j + 1] - off_j, up_j = s_uoff[j + 1] - s_uoff[j];
-                const int p = j > i ? uo + (rank - nlower) : s_uoff[j] + (rank_j - (kept_j - up_j));
-                // (structure sizes that do not add up: reported, and every index written stays inside its array)
-                const bool ok = rank_j >= 0 && rank_j < kept_j && (rev.y >> (il & 31) & 1u) && i != j && p >= 0 && p < P;
-                if (!ok) atomicOr(status, (int)kAsymmetric);
-                g.row1[slot] = j;
-                g.twin[slot] = ok ? off_j + rank_j : slot;
-                g.pair_of[slot] = ok ? p : 0;
-                d[slot] = sqrtf(d2);
-                if (ok && j > i) g.sel[p] = slot;
-            }
-        }
+        each_hit(g.masks + (int64_t)i * words, (n + 31) >> 5, kept, lane, [&](int rank, int jl) {
+            const int slot = off + rank, j = lo + jl;
+            const float d2 = dist2_rn(xi, yi, zi, pos[3 * j], pos[3 * j + 1], pos[3 * j + 2]);
+            const PairPlace place = pair_place(g.masks, words, i, i - lo, j, rank, total >> 1, at);
+            // (structure sizes that do not add up: reported, and every index written stays inside its array)
+            if (!place.ok) atomicOr(status, (int)kAsymmetric);
+            g.row1[slot] = j;
+            g.twin[slot] = place.ok ? (int)place.twin : slot;
+            g.pair_of[slot] = place.ok ? (int)place.pair : 0;
+            d[slot] = sqrtf(d2);
+            if (place.ok && j > i) g.sel[place.pair] = slot;
+        });
     }
 }
 
