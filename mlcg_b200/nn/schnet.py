@@ -493,7 +493,7 @@ class SchNet(torch.nn.Module):
         n_atoms, ptr = sizes_or_pointer(data)
         N, kept = data.pos.shape[0], self.__dict__
         inside = not training and N <= 2048
-        seen = kept.get("_mlcgb_edges_per_bead", 0.0)
+        seen = most = kept.get("_mlcgb_edges_per_bead", 0.0)
         if not inside:
             seen = kept.get("_mlcgb_edges_per_bead_large", seen)
         elif not seen:                                    # (nothing to go by: every bead sees its whole structure, or forty others)
@@ -503,10 +503,10 @@ class SchNet(torch.nn.Module):
                                                   int(self.max_num_neighbors), *setup, forces, room, training)
         if res is None:
             return None
-        if inside:
-            kept["_mlcgb_edges_per_bead"] = max(kept.get("_mlcgb_edges_per_bead", 0.0), res[2] / N)
-        else:
+        if not inside:
             kept["_mlcgb_edges_per_bead_large"] = res[2] / N
+        elif res[2] > most * N:
+            kept["_mlcgb_edges_per_bead"] = res[2] / N
         return res[0], res[1], res[3]
 
     def energy_and_forces_training(self, data):
