@@ -1,7 +1,7 @@
 // The host side of the calls that a small batch waits for: addresses and layouts of lists of tensors, outputs and workspaces, and the
 // library calls themselves, without a Python object per argument.  Of the 68 us of host time for an evaluation of 64 x 10 beads 21 went
 // around the library call (now 61 us, the kernels take 60), of a step of Langevin dynamics of 54 beads with four priors 228 are 168
-// now, of a force-matching step of 12 x 100 beads 590 are 554.  Nothing here computes: the library's entry points come as addresses,
+// now, of a force-matching step of 12 x 100 beads 590 are 554 (its spread from run to run is as large).  Nothing here computes: the library's entry points come as addresses,
 // from the copy that the ctypes binding has loaded.
 #include <torch/extension.h>
 

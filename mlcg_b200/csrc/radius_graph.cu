@@ -2240,12 +2240,16 @@ namespace mlcgb {
 
 // Larger batches whose structures have at most 1024 points on average: those that do go the same way (mask_rows_kernel), 1024 points
 // being what a warp's row of bits can hold; in a batch of large structures the bit rows (256 bytes per point) would be room for
-// nothing.  Lists and distances of 40 000 points in structures of one size, uniform, 10 A, us, bit rows : cells,
-//   points              800        900       1000
-//   float32           164 : 165  172 : 159  181 : 167
-//   float64           188 : 408  200 : 498  212 : 475
-//   ragged, 10.5 A    126 : 206 (float32), 139 : 438 (float64)
-// and chains, which crowd few cells of their grid, gain more than any of these.
+// nothing.  40 000 points in structures of one size, uniform at 54 cubic Angstrom each or chains, us, bit rows : cells,
+//                        edges                              with distances
+//   points, cutoff     8 A       10 A      12 A      chain, 10 A     8 A       10 A      12 A
+//   float32   800   130 : 139  144 : 160  156 : 243  101 : 199   148 : 143  160 : 164  166 : 243
+//            1000   140 : 140  158 : 161  175 : 282  105 : 242   161 : 143  181 : 166  190 : 280
+//   float64   800   139 : 152  154 : 202  170 : 328  109 : 216   170 : 157  184 : 211  192 : 333
+//            1000   153 : 155  173 : 197  190 : 349  116 : 263   188 : 160  209 : 206  221 : 355
+// So the cells keep what is uniform, of 800 points or more, at 8 to 10 A and wants distances (up to 17 % faster there), and lose up to eight
+// times on the rest (chains at 15 A): the batch's shape is not known when the route is chosen, and chains are what this package is for.
+// A batch that holds a larger structure all the same is counted twice (60 structures of up to 1300 points: 240 us instead of 218).
 constexpr int kMaskWordsPerRow = 32;
 static inline bool mask_rows_route(int64_t N, int64_t B) { return N > kMaskNodes && N <= 32 * kMaskWordsPerRow * B; }
 
