@@ -215,6 +215,11 @@ class KernelProfiler:
         return sum(v["launches"] for v in self.stats.values())
 
 
+class _Lists(threading.local):
+    made = 0            # prior lists prepared by this thread
+    word = None         # the status word behind the last of them, where its call has waited
+
+
 class CudaBackend:
     name = "cuda"
 
@@ -223,7 +228,7 @@ class CudaBackend:
         _lib.bind_native(self.lib)
         self.native = _lib.native()
         self.profiler = None
-        self._status, self._lists = {}, threading.local()
+        self._status, self.lists = {}, _Lists()
         self.tensor_core_gemm = True   # float32 GEMMs of qualifying shape run on tcgen05 (fp32-equivalent products)
         self._pending = []      # (status tensor, what) of kernels whose status word has not been read yet
 
@@ -1137,7 +1142,8 @@ class CudaBackend:
                 starts = torch.empty(host[0], dtype=torch.int64, device=dev)
                 self._run("prior_list_starts", self.lib.mlcgb_prior_list_starts, (_ptr(idx), M, _ptr(ws), wsb, _ptr(starts), _stream()))
         # what the status word says of the lists made so far: known to the host (a pair list), or to be read
-        self._lists.word = int(host[2]) if pairs else None
+        self.lists.made += 1
+        self.lists.word = int(host[2]) if pairs else None
         return idx, out, bool(host[1]), starts
 
     def lists_name_missing(self, dev) -> bool:
@@ -1145,7 +1151,7 @@ class CudaBackend:
         was a pair list, whose call has waited; not while recording)."""
         if torch.cuda.is_current_stream_capturing():
             return False
-        status, word = self._sticky_status(dev), getattr(self._lists, "word", None)
+        status, word = self._sticky_status(dev), self.lists.word
         if word is None or word & STATUS_NOT_THERE:
             word = int(status[0])
         if word & STATUS_NOT_THERE:

@@ -60,10 +60,11 @@ py::object pointers(const py::list &list) {
     return py::bytes(reinterpret_cast<const char *>(at.data()), at.size() * sizeof(void *));
 }
 
-// address, in-place version, shape and strides of every tensor of a sequence, as bytes
-py::bytes layouts(const py::tuple &list) {
+// address, in-place version, shape and strides of every tensor of a sequence, as bytes; in front of them dtype, device and length of `like`
+py::bytes layouts(const py::tuple &list, const c10::optional<at::Tensor> &like) {
     std::vector<int64_t> v;
-    v.reserve(8 * list.size());
+    v.reserve(8 * list.size() + 4);
+    if (like) v = {(int64_t)like->scalar_type(), (int64_t)like->device().type(), (int64_t)like->device().index(), like->size(0)};
     for (py::handle h : list) {
         const at::Tensor &t = tensor_of(h.ptr());
         v.push_back(reinterpret_cast<int64_t>(t.data_ptr()));
@@ -194,7 +195,7 @@ py::tuple prior_eval(const py::list &lists, const at::Tensor &pos_in, const c10:
 PYBIND11_MODULE(_native, m) {
     m.def("bind", &bind);
     m.def("pointers", &pointers);
-    m.def("layouts", &layouts);
+    m.def("layouts", &layouts, py::arg("list"), py::arg("like") = py::none());
     m.def("views", &views);
     m.def("evaluate", &evaluate);
     m.def("prior_eval", &prior_eval);
