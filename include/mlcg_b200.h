@@ -12,7 +12,8 @@
  *     status[0] bit 0 = a centre had more neighbours than max_num_neighbors (list truncated),
  *     status[0] bit 1 = an index was out of range and the element was skipped,
  *     status[0] bit 2 = an edge had no reverse partner (graph not symmetric),
- *     status[0] bit 6 = a list that is being prepared names a bead or a bead type that does not exist.
+ *     status[0] bit 6 = a list that is being prepared names a bead or a bead type that does not exist,
+ *     status[0] bit 7 = structure sizes do not add up to the points (the last structure then takes what the others leave).
  *   - `stream` is a cudaStream_t passed as void*.
  *
  * Each entry point names the reference interface it stands in for (path inside the mlcg repository).
@@ -517,7 +518,7 @@ int mlcgb_schnet_energy_forces(const void *pos, const int64_t *types, const int6
  * workspaces (mlcgb_schnet_evaluate_lists names the places).  host [5]: the four values of mlcgb_graph_begin and an outcome (0 before the first call):
  *   MLCGB_EVALUATE_DONE     energy and grad_pos are on their way
  *   MLCGB_EVALUATE_MORE     the workspace is too small for host[0] edges: call again, everything but the workspace as it was
- *   MLCGB_EVALUATE_NO_PLAN  nothing evaluated: no edges, or a list cut short by max_nn */
+ *   MLCGB_EVALUATE_NO_PLAN  nothing evaluated: no edges, a list cut short by max_nn, or sizes that do not add up (host[1]) */
 #define MLCGB_EVALUATE_DONE 1
 #define MLCGB_EVALUATE_MORE 2
 #define MLCGB_EVALUATE_NO_PLAN 3

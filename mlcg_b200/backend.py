@@ -16,7 +16,7 @@ import torch
 from . import _lib
 
 _DT = {torch.float32: 0, torch.float64: 1}
-STATUS_TRUNCATED, STATUS_BAD_INDEX, STATUS_ASYMMETRIC, STATUS_NOT_THERE = 1, 2, 4, 64
+STATUS_TRUNCATED, STATUS_BAD_INDEX, STATUS_ASYMMETRIC, STATUS_NOT_THERE, STATUS_SIZES = 1, 2, 4, 64, 128
 
 
 @dataclass(frozen=True)
@@ -153,6 +153,8 @@ def _need_cuda(*ts):
 
 def _raise_for_status(word: int, what: str) -> None:
     """Status bits the tensor-core kernels set (read lazily, with the next unavoidable host read)."""
+    if word & STATUS_SIZES:
+        raise ValueError(f"mlcg_b200: {what}: n_atoms does not add up to the positions")
     if word & 8:
         raise RuntimeError(f"mlcg_b200: {what}: a tensor-core wait ran out; results are incomplete")
     if word & 32:
@@ -263,7 +265,7 @@ class CudaBackend:
     def _raise_pending(words, pending):
         """Raise for the first status word that reports a failure; the words are cleared first, so one failure is reported
         once and later evaluations start clean."""
-        bad = [(w, what) for w, (_, what) in zip(words, pending) if w & (4 | 8 | 16 | 32)]
+        bad = [(w, what) for w, (_, what) in zip(words, pending) if w & (4 | 8 | 16 | 32 | STATUS_SIZES)]
         if bad:
             for st, _ in pending:
                 st.zero_()
@@ -391,6 +393,8 @@ class CudaBackend:
             E, st = host[0], int(host[1])
             if pend and host[2]:
                 self._raise_pending([int(host[2])], pend)
+            if st & STATUS_SIZES:
+                _raise_for_status(st, "radius graph")
             plan = want_plan and not loop and exclude is None and not st & STATUS_TRUNCATED and 0 < E < 1 << 31 and E % 2 == 0
             ei = torch.empty((2, E), dtype=torch.int64, device=dev) if want_index else None
             dist = torch.empty(E, dtype=pos.dtype, device=dev) if want_distance else None
@@ -922,6 +926,9 @@ class CudaBackend:
                 forces, training, max(int(edges), 0), pend[0][0] if pend else None, status, _stream())
         if code:
             _lib.check(code, "schnet_evaluate")
+        if host[1] & STATUS_SIZES:
+            status.bitwise_and_(~STATUS_SIZES)
+            _raise_for_status(host[1], "radius graph")
         if pend and host[2]:
             self._raise_pending([int(host[2])], pend)
         if host[4] != _lib.EVALUATE_DONE:

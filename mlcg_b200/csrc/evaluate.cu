@@ -111,7 +111,7 @@ int mlcgb_schnet_evaluate(const void *pos, const int64_t *types, const int64_t *
                                 (char *)workspace, workspace_bytes, energy, grad_pos, pub, status, (cudaStream_t)stream);
             if (rc || (rc = publish_wait(pub, (cudaStream_t)stream))) return rc;
             for (int i = 0; i < 4; i++) host[i] = pub.host[1 + i];
-            host[4] = (host[1] & kTruncated) || host[0] <= 0 || (host[0] & 1) ? MLCGB_EVALUATE_NO_PLAN : host[0] > 2 * lo ? MLCGB_EVALUATE_MORE : MLCGB_EVALUATE_DONE;
+            host[4] = (host[1] & (kTruncated | kSizes)) || host[0] <= 0 || (host[0] & 1) ? MLCGB_EVALUATE_NO_PLAN : host[0] > 2 * lo ? MLCGB_EVALUATE_MORE : MLCGB_EVALUATE_DONE;
             return MLCGB_OK;
         }
     }
@@ -122,7 +122,7 @@ int mlcgb_schnet_evaluate(const void *pos, const int64_t *types, const int64_t *
     }
     const int64_t E = host[0];
     host[4] = MLCGB_EVALUATE_NO_PLAN;
-    if ((host[1] & kTruncated) || E <= 0 || (E & 1) || E >= (int64_t)1 << 31) return MLCGB_OK;
+    if ((host[1] & (kTruncated | kSizes)) || E <= 0 || (E & 1) || E >= (int64_t)1 << 31) return MLCGB_OK;
     host[4] = MLCGB_EVALUATE_MORE;
     if (!workspace || workspace_bytes < mlcgb_schnet_evaluate_workspace_bytes(N, B, E, rbf->num_rbf, w, training)) return MLCGB_OK;
     if ((uintptr_t)workspace & 255) return MLCGB_E_ARG;

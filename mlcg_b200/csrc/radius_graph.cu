@@ -2282,18 +2282,24 @@ __global__ void batch_boundaries_kernel(const int64_t *__restrict__ batch, int64
     ptr[b] = first_at_least(batch, N, b);
 }
 
-__global__ void __launch_bounds__(kScanBlock) sizes_to_ptr_kernel(const int64_t *__restrict__ sizes, int64_t B, int64_t *__restrict__ ptr) {
+__global__ void __launch_bounds__(kScanBlock) sizes_to_ptr_kernel(const int64_t *__restrict__ sizes, int64_t B, int64_t N, int64_t *__restrict__ ptr,
+                                                                  int32_t *__restrict__ status) {
     __shared__ int64_t s_warp[33];
     int64_t carry = 0;
     for (int64_t b0 = 0; b0 < B; b0 += kScanBlock) {
         const int64_t b = b0 + threadIdx.x;
         int64_t total;
-        const int64_t ex = block_exclusive_scan(b < B ? sizes[b] : 0, s_warp, &total);
-        if (b < B) ptr[b] = carry + ex;
+        const int64_t size = b < B ? sizes[b] : 0, n = usable_size(size, N);
+        if (n != size) atomicOr(status, (int)kSizes);
+        const int64_t ex = block_exclusive_scan(n, s_warp, &total);
+        if (b < B) ptr[b] = carry + ex < N ? carry + ex : N;
         carry += total;
         __syncthreads();
     }
-    if (threadIdx.x == 0) ptr[B] = carry;
+    if (threadIdx.x == 0) {
+        ptr[B] = N;
+        if (carry != N) atomicOr(status, (int)kSizes);
+    }
 }
 
 // The structure of point i as the run of its entry in a sorted batch vector of at most kMaskNodes points, by the whole warp: 32 probes,
@@ -2330,7 +2336,7 @@ mask_count_kernel(const T *__restrict__ pos, const int64_t *__restrict__ sizes, 
                   int64_t capacity /* < 0: none */, int64_t *__restrict__ counts, int32_t *__restrict__ sticky, Publish pub) {
     __shared__ int s_ptr[BATCH ? 1 : kMaskStructs + 1];
     __shared__ int s_last, s_wd[8], s_wu[8];
-    if constexpr (!BATCH) load_boundaries<256>(s_ptr, sizes, ptr, B);
+    if constexpr (!BATCH) load_boundaries<256>(s_ptr, sizes, ptr, B, (int)N, status);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int64_t ci = (int64_t)blockIdx.x * 8 + warp; ci < N; ci += (int64_t)gridDim.x * 8) {
         const int i = (int)ci;
@@ -2414,7 +2420,7 @@ mask_fill_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, int
                  const int32_t *__restrict__ upper, const int32_t *__restrict__ uoff, const int64_t *__restrict__ offsets, FillOut out,
                  int32_t *__restrict__ twin, int32_t *__restrict__ sel, int32_t *__restrict__ pair_of, int32_t *__restrict__ sticky) {
     __shared__ int s_ptr[BATCH ? 1 : kMaskStructs + 1];
-    if constexpr (!BATCH) load_boundaries<256>(s_ptr, nullptr, const_cast<int64_t *>(ptr), B);
+    if constexpr (!BATCH) load_boundaries<256>(s_ptr, nullptr, const_cast<int64_t *>(ptr), B, (int)N, sticky);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t P = offsets[N] >> 1;
     if (twin && (offsets[N] & 1) && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(sticky, (int)kAsymmetric);
@@ -2476,27 +2482,29 @@ __device__ __forceinline__ int64_t structure_at(const int64_t *__restrict__ ptr,
     return lo;
 }
 
-// boundaries from the sizes (or as they are), the status words cleared, and whether a structure is too large
+// boundaries from the sizes (or as they are), the status words cleared, and whether a structure is too large (as the last one may be where
+// the sizes do not add up)
 __global__ void __launch_bounds__(kScanBlock)
-rows_begin_kernel(const int64_t *__restrict__ sizes, int64_t B, int64_t *__restrict__ ptr, int32_t *__restrict__ header) {
+rows_begin_kernel(const int64_t *__restrict__ sizes, int64_t B, int64_t N, int64_t *__restrict__ ptr, int32_t *__restrict__ header) {
     __shared__ int64_t s_warp[33];
     pdl_launch_dependents();
     int64_t carry = 0;
-    bool large = false;
+    bool large = false, odd = false;
     for (int64_t b0 = 0; b0 < B; b0 += kScanBlock) {
         const int64_t b = b0 + threadIdx.x;
-        const int64_t n = b < B ? (sizes ? sizes[b] : ptr[b + 1] - ptr[b]) : 0;
+        const int64_t size = b < B ? (sizes ? sizes[b] : ptr[b + 1] - ptr[b]) : 0, n = sizes ? usable_size(size, N) : size;
         large |= n > kMaskMax;
+        odd |= n != size;
         if (!sizes) continue;
         int64_t total;
         const int64_t ex = block_exclusive_scan(n, s_warp, &total);
-        if (b < B) ptr[b] = carry + ex;
+        if (b < B) ptr[b] = carry + ex < N ? carry + ex : N;
         carry += total;
         __syncthreads();
     }
-    if (sizes && threadIdx.x == 0) ptr[B] = carry;
-    const int any = __syncthreads_or(large);
-    if (threadIdx.x < 8) header[threadIdx.x] = 0;
+    if (sizes && threadIdx.x == 0) ptr[B] = N;
+    const int wrong = __syncthreads_or(odd || (sizes && carry != N)), any = __syncthreads_or(large) || wrong;
+    if (threadIdx.x < 8) header[threadIdx.x] = threadIdx.x == 0 && wrong ? kSizes : 0;
     if (threadIdx.x == 0) header[8] = any;
 }
 
@@ -2612,7 +2620,7 @@ rows_scan_kernel(const int32_t *__restrict__ deg, const int32_t *__restrict__ up
     if (header && header[8]) {
         if (last && threadIdx.x == 0) {
             *reinterpret_cast<volatile int64_t *>(pub.host + 4) = -1;
-            publish(pub, 0, 0);
+            publish(pub, 0, header[0]);
         }
         return;
     }
@@ -3091,11 +3099,12 @@ int mlcgb_graph_begin(const void *pos, int dtype, const int64_t *n_atoms, int64_
     if (int rc = publish_begin(&pub)) return rc;
     pub.pending = pending_status;
     const bool rows = !ex.ptr && !mask_route(N, B, ex) && mask_rows_route(N, B);
+    int64_t sizes = 0;                         // (what the first count of a batch that is counted twice has to say of them)
     const WsLayout W = ws_layout(N, B, dtype);
     char *cw = w + L.cells;
     auto *deg = (int32_t *)(w + L.deg), *upper = (int32_t *)(w + L.upper), *status = (int32_t *)(w + L.header);
     if (rows) {
-        rows_begin_kernel<<<1, kScanBlock, 0, st>>>(n_atoms, B, ptr, status);
+        rows_begin_kernel<<<1, kScanBlock, 0, st>>>(n_atoms, B, N, ptr, status);
         int rc = MLCGB_DISPATCH_DTYPE(dtype, [&] {
             launch_pdl(mask_rows_kernel<scalar_t, true>, dim3((unsigned)((N + 31) / 32)), dim3(256), 0, st, (const scalar_t *)pos, (const int64_t *)ptr,
                        (int32_t *)(cw + W.struct_of), (const CellParam *)nullptr, N, (scalar_t)(r * r), max_nn, loop, rule, (uint2 *)(w + L.masks), deg, upper, status, B,
@@ -3107,13 +3116,14 @@ int mlcgb_graph_begin(const void *pos, int dtype, const int64_t *n_atoms, int64_
         if (rc || (rc = publish_wait(pub, st))) return rc;
         for (int i = 0; i < 4; i++) host_out[i] = pub.host[1 + i];
         if (host_out[3] >= 0) return MLCGB_OK;
+        sizes = host_out[1] & kSizes;
         if ((rc = publish_begin(&pub))) return rc;
     }
     cudaMemsetAsync(w + L.header, 0, 32, st);
     int rc = MLCGB_DISPATCH_DTYPE(dtype, [&] {
         if (mask_route(N, B, ex))
             return mask_count_launch<scalar_t>(pos, n_atoms, ptr, N, B, r, max_nn, loop, rule, w, L, offsets, -1, nullptr, nullptr, pub, st);
-        if (n_atoms && !rows) sizes_to_ptr_kernel<<<1, kScanBlock, 0, st>>>(n_atoms, B, ptr);
+        if (n_atoms && !rows) sizes_to_ptr_kernel<<<1, kScanBlock, 0, st>>>(n_atoms, B, N, ptr, status);
         const int rl = radius_launch<scalar_t>(false, false, pos, ptr, N, B, r, max_nn, loop, rule, cw, W.total, dtype, deg, offsets, FillOut{}, status, st, ex,
                                                rows ? kMaskMax : kBruteMax, rows ? 2 : 0, upper);
         if (rl) return rl;
@@ -3131,6 +3141,7 @@ int mlcgb_graph_begin(const void *pos, int dtype, const int64_t *n_atoms, int64_
     if (rc) return rc;
     if ((rc = publish_wait(pub, st))) return rc;
     for (int i = 0; i < 4; i++) host_out[i] = pub.host[1 + i];
+    host_out[1] |= sizes;
     return MLCGB_OK;
 }
 
@@ -3252,7 +3263,7 @@ int mlcgb_graph_capacity(const void *pos, int dtype, const int64_t *n_atoms, int
     // a list that did not fit has fewer upper edges than pairs: the kernels that read sel behind it still need valid edges
     if (capacity > 0) cudaMemsetAsync(sel, 0, (size_t)(capacity / 2) * 4, st);
     if (!mask_route(N, B, Exclusion{})) {
-        if (n_atoms) sizes_to_ptr_kernel<<<1, kScanBlock, 0, st>>>(n_atoms, B, ptr);
+        if (n_atoms) sizes_to_ptr_kernel<<<1, kScanBlock, 0, st>>>(n_atoms, B, N, ptr, sticky_status);
         int rc = mlcgb_radius_graph_capacity(pos, dtype, ptr, N, B, r, max_nn, 0, rule, w + L.cells, ws_layout(N, B, dtype).total, (int32_t *)(w + L.deg),
                                              offsets, capacity, nullptr, row0, row1, counts, sticky_status, stream);
         if (rc || capacity == 0) return rc;

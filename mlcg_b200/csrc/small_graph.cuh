@@ -24,9 +24,13 @@ __device__ __forceinline__ void publish(const Publish &p, int64_t edges, int sta
     h[0] = p.seq;
 }
 
+// A structure's size as the kernels take it.  Sizes that do not add up to the points are reported (kSizes), and the boundaries made of them
+// are those of N points all the same, ascending: the last structure begins where the others end and takes what is left.
+__device__ __forceinline__ int64_t usable_size(int64_t size, int64_t N) { return size < 0 ? 0 : size < N ? size : N; }
+
 // structure boundaries into shared memory: from the sizes (whose prefix sums block 0 also writes out) or from ptr
 template <int NT /* threads of the block */>
-__device__ __forceinline__ void load_boundaries(int *s_ptr, const int64_t *sizes, int64_t *ptr, int64_t B) {
+__device__ __forceinline__ void load_boundaries(int *s_ptr, const int64_t *sizes, int64_t *ptr, int64_t B, int N, int32_t *status) {
     __shared__ int s_part[NT / 32];
     if (!sizes) {
         for (int b = threadIdx.x; b <= B; b += NT) s_ptr[b] = (int)ptr[b];
@@ -37,7 +41,9 @@ __device__ __forceinline__ void load_boundaries(int *s_ptr, const int64_t *sizes
     int carry = 0;
     for (int64_t b0 = 0; b0 < B; b0 += NT) {
         const int64_t b = b0 + threadIdx.x;
-        const int v = b < B ? (int)sizes[b] : 0;
+        const int64_t size = b < B ? sizes[b] : 0;
+        const int v = (int)usable_size(size, N);
+        if (v != size && blockIdx.x == 0) atomicOr(status, (int)kSizes);
         int inc = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -48,11 +54,14 @@ __device__ __forceinline__ void load_boundaries(int *s_ptr, const int64_t *sizes
         __syncthreads();
         int before = carry;
         for (int w = 0; w < warp; w++) before += s_part[w];
-        if (b < B) s_ptr[b] = before + inc - v;
+        if (b < B) s_ptr[b] = min(before + inc - v, N);
         for (int w = 0; w < NT / 32; w++) carry += s_part[w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) s_ptr[B] = carry;
+    if (threadIdx.x == 0) {
+        s_ptr[B] = N;
+        if (carry != N && blockIdx.x == 0) atomicOr(status, (int)kSizes);
+    }
     __syncthreads();
     if (blockIdx.x == 0)
         for (int b = threadIdx.x; b <= B; b += NT) ptr[b] = s_ptr[b];

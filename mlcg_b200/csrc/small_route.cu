@@ -524,7 +524,7 @@ small_graph_count_kernel(const float *__restrict__ pos, const SmallGraph g, int6
         }
         return;
     }
-    load_boundaries<kST>(s_ptr, g.sizes, g.ptr, B);
+    load_boundaries<kST>(s_ptr, g.sizes, g.ptr, B, (int)N, status);
     const int64_t ci = (int64_t)blockIdx.x * (kST / 32) + warp;
     if (ci >= N) return;
     const int i = (int)ci, b = structure_of(s_ptr, B, i), lo = s_ptr[b], n = min(s_ptr[b + 1], (int)N) - lo;
@@ -585,7 +585,8 @@ small_graph_fill_kernel(const float *__restrict__ pos, const SmallGraph g, int64
         if (threadIdx.x == 0) {
             g.counts[0] = bad ? 0 : total;
             g.counts[1] = bad ? 0 : total >> 1;
-            if (g.pub.host) publish(g.pub, total, cut ? (int)kTruncated : 0);
+            const int sizes = *reinterpret_cast<volatile int32_t *>(status) & kSizes;
+            if (g.pub.host) publish(g.pub, total, (cut ? (int)kTruncated : 0) | sizes);
             else if (bad) atomicOr(status, (cut ? (int)kTruncated : 0) | (total > g.capacity ? (int)kCapacity : 0) | (total & 1 ? (int)kAsymmetric : 0));
         }
         if (i0 <= n_all) g.offsets[i0] = bad ? 0 : e0;

@@ -223,3 +223,50 @@ def test_a_list_changed_behind_its_version_is_reported(sizes, how):
     status.zero_()
     for t, most in ((plan.row0, n), (plan.row1, n), (plan.perm_in, E), (plan.half_selection(), E), (plan.pair_index(), E // 2)):
         assert int(t.min()) >= 0 and int(t.max()) < most
+
+
+@pytest.mark.parametrize("sizes", [[40, 30], [900, 900, 600], [1000, 1500, 700], [3000, 100], [20] * 150])
+@pytest.mark.parametrize("given", ["one short", "many short", "one over", "far over", "one below zero", "one beyond all"])
+def test_sizes_that_do_not_add_up(sizes, given):
+    """``n_atoms`` of another batch, on every route of the graph: an error, and the call after it has its own result."""
+    import mlcg_b200
+    from mlcg_b200 import nn as bnn
+    be, n, gen = get_backend(), sum(sizes), torch.Generator().manual_seed(2)
+    pos = (torch.rand(n, 3, generator=gen) * max(sizes) ** (1 / 3) * 2.5).to(DEV)
+    right = torch.tensor(sizes, device=DEV)
+    wrong = right.clone()
+    if given == "one short":
+        wrong[-1] -= 1
+    elif given == "many short":
+        wrong = wrong // 3
+    elif given == "one over":
+        wrong[0] += 1
+    elif given == "far over":
+        wrong *= 1000
+    elif given == "one below zero":
+        wrong[-1] = -5
+    else:
+        wrong[0] = 2 ** 40
+    torch.manual_seed(0)
+    cut = bnn.CosineCutoff(0.0, 4.0)
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, 32, trainable=False), cut, [128], embedding_size=5, num_interactions=2).eval().to(DEV)
+    model, types = bnn.GradientsOut(net, "forces").eval(), torch.zeros(n, dtype=torch.int64, device=DEV)
+    data = lambda s: mlcg_b200.AtomicData(pos=pos.clone(), atom_types=types, batch=torch.repeat_interleave(torch.arange(len(sizes), device=DEV), right), n_atoms=s)  # noqa: E731
+    graph = lambda s: be.radius_graph(pos, None, 4.0, 1000, False, 1, n_atoms=s, want_plan=True)  # noqa: E731
+    want, out = graph(right), model(data(right)).out["SchNet"]
+    with pytest.raises(ValueError, match="does not add up"):
+        graph(wrong)
+    with pytest.raises(ValueError, match="does not add up"):
+        model(data(wrong))
+    bnn.set_edge_capacity(model, want["row0"].numel() * 2)
+    with pytest.raises(ValueError, match="does not add up"):
+        model(data(wrong))
+        be.check_pending()
+    fixed = model(data(right)).out["SchNet"]
+    be.check_pending()
+    bnn.set_edge_capacity(model, None)
+    got, again = graph(right), model(data(right)).out["SchNet"]
+    be.check_pending()
+    assert torch.equal(got["edge_index"], want["edge_index"]) and torch.equal(got["twin"], want["twin"])
+    assert torch.equal(again["energy"], out["energy"]) and torch.equal(again["forces"], out["forces"])
+    assert torch.allclose(fixed["energy"], out["energy"], rtol=1e-5, atol=1e-5 * float(out["energy"].abs().max()))
