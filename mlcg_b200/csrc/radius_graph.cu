@@ -2451,7 +2451,7 @@ mask_fill_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, int
             if (out.distance) d2 = dist2_rn(pos[3 * ci], pos[3 * ci + 1], pos[3 * ci + 2], pos[3 * j], pos[3 * j + 1], pos[3 * j + 2]);
             emit_edge<T>(out, slot, i, j, b, d2);
             if (!twin) return;
-            const PairPlace place = pair_place(masks, words, i, i - lo, (int)j, rank, P, at);
+            const auto place = pair_place(masks, words, i, i - lo, (int)j, rank, P, at);
             // not a valid plan (a list was cut short): reported, and every index written stays inside its array
             if (!place.ok) atomicOr(sticky, (int)kAsymmetric);
             twin[slot] = (int32_t)(place.ok ? place.twin : slot);

@@ -141,15 +141,15 @@ __device__ __forceinline__ void each_hit(const uint2 *__restrict__ row, int nw, 
 // The reverse of the edge (i, j) that is hit `rank` of its row, and the pair of the two: from j's row at the word of i (local index il).
 // `at`: first edge, kept edges, lower ones among them and pairs before of a row.  Not ok where the list holds no plan (cut short, or sizes
 // that do not add up); every index is inside its array if it is.
-struct PairPlace {
-    int64_t twin, pair;
+template <typename I> struct PairPlace {
+    I twin, pair;
     bool ok;
 };
-template <typename At>
-__device__ __forceinline__ PairPlace pair_place(const uint2 *__restrict__ masks, int words, int i, int il, int j, int rank, int64_t P, const At &at) {
+template <typename I, typename At>
+__device__ __forceinline__ PairPlace<I> pair_place(const uint2 *__restrict__ masks, int words, int i, int il, int j, int rank, I P, const At &at) {
     const uint2 rev = masks[(int64_t)j * words + (il >> 5)];
     const int rank_j = (int)rev.x + __popc(rev.y & ((1u << (il & 31)) - 1u));
-    const int64_t p = j > i ? at.pairs(i) + (rank - at.lower(i)) : at.pairs(j) + (rank_j - at.lower(j));
+    const I p = j > i ? at.pairs(i) + (rank - at.lower(i)) : at.pairs(j) + (rank_j - at.lower(j));
     return {at.first(j) + rank_j, p, rank_j >= 0 && rank_j < at.kept(j) && (rev.y >> (il & 31) & 1u) && i != j && p >= 0 && p < P};
 }
 

@@ -546,6 +546,7 @@ small_graph_fill_kernel(const float *__restrict__ pos, const SmallGraph g, int64
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_all = (int)N;
     pdl_launch_dependents();
     pdl_wait();
+    const int sizes = blockIdx.x == 0 && threadIdx.x == 0 ? __ldcg(status) & kSizes : 0;      // (what the count found)
     for (int b = threadIdx.x; b <= B; b += kFillThreads) s_ptr[b] = (int)g.ptr[b];
     static_assert(kMaskNodes == 2 * kFillThreads, "two beads per thread");
     const int i0 = 2 * threadIdx.x;
@@ -585,7 +586,6 @@ small_graph_fill_kernel(const float *__restrict__ pos, const SmallGraph g, int64
         if (threadIdx.x == 0) {
             g.counts[0] = bad ? 0 : total;
             g.counts[1] = bad ? 0 : total >> 1;
-            const int sizes = *reinterpret_cast<volatile int32_t *>(status) & kSizes;
             if (g.pub.host) publish(g.pub, total, (cut ? (int)kTruncated : 0) | sizes);
             else if (bad) atomicOr(status, (cut ? (int)kTruncated : 0) | (total > g.capacity ? (int)kCapacity : 0) | (total & 1 ? (int)kAsymmetric : 0));
         }
@@ -595,28 +595,28 @@ small_graph_fill_kernel(const float *__restrict__ pos, const SmallGraph g, int64
     }
     if (bad) return;
     __syncthreads();
-    const int words = (n_all + 31) >> 5;
+    const int words = (n_all + 31) >> 5, P = (int)(total >> 1);
     struct {
         const int *off, *uoff;
-        __device__ int64_t first(int k) const { return off[k]; }
+        __device__ int first(int k) const { return off[k]; }
         __device__ int kept(int k) const { return off[k + 1] - off[k]; }
         __device__ int lower(int k) const { return kept(k) - (uoff[k + 1] - uoff[k]); }
-        __device__ int64_t pairs(int k) const { return uoff[k]; }
+        __device__ int pairs(int k) const { return uoff[k]; }
     } const at = {s_off, s_uoff};
     for (int i = blockIdx.x * (kFillThreads / 32) + warp; i < n_all; i += gridDim.x * (kFillThreads / 32)) {
-        const int b = structure_of(s_ptr, B, i), lo = s_ptr[b], n = min(s_ptr[b + 1], n_all) - lo;
+        const int b = structure_of(s_ptr, B, i), lo = s_ptr[b], n = min(s_ptr[b + 1], n_all) - lo, il = i - lo;
         const int off = s_off[i], kept = s_off[i + 1] - off;
         if (kept == 0) continue;
         const float xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
         each_hit(g.masks + (int64_t)i * words, (n + 31) >> 5, kept, lane, [&](int rank, int jl) {
             const int slot = off + rank, j = lo + jl;
             const float d2 = dist2_rn(xi, yi, zi, pos[3 * j], pos[3 * j + 1], pos[3 * j + 2]);
-            const PairPlace place = pair_place(g.masks, words, i, i - lo, j, rank, total >> 1, at);
+            const auto place = pair_place(g.masks, words, i, il, j, rank, P, at);
             // (structure sizes that do not add up: reported, and every index written stays inside its array)
             if (!place.ok) atomicOr(status, (int)kAsymmetric);
             g.row1[slot] = j;
-            g.twin[slot] = place.ok ? (int)place.twin : slot;
-            g.pair_of[slot] = place.ok ? (int)place.pair : 0;
+            g.twin[slot] = place.ok ? place.twin : slot;
+            g.pair_of[slot] = place.ok ? place.pair : 0;
             d[slot] = sqrtf(d2);
             if (place.ok && j > i) g.sel[place.pair] = slot;
         });

@@ -201,9 +201,12 @@ __device__ __forceinline__ float put_weight4(uint8_t *hi, uint8_t *lo, int n, in
 }
 // A quad of a weight's row, `lanes` lanes a row: not a number anywhere in the row makes the whole row so.  A GEMM that leaves out the part of
 // K where its other operand is zero then gives what the whole one gives.  By all lanes of a warp.
-__device__ __forceinline__ float4 spread_nan(float4 w, int lanes) {
+__device__ __forceinline__ bool maybe_nan(float4 w) {       // (also of infinities of both signs)
     const float s = (w.x + w.y) + (w.z + w.w);
-    const bool bad = s != s && (w.x != w.x || w.y != w.y || w.z != w.z || w.w != w.w);
+    return s != s;
+}
+__device__ __forceinline__ float4 spread_nan(float4 w, int lanes) {
+    const bool bad = w.x != w.x || w.y != w.y || w.z != w.z || w.w != w.w;
     const unsigned all = __ballot_sync(0xffffffffu, bad), row = lanes == 32 ? all : all >> (threadIdx.x & 16) & 0xffffu;
     if (row == 0) return w;
     const float nan = __int_as_float(0x7fffffff);
@@ -232,8 +235,13 @@ __device__ __forceinline__ bool load_weight_tile(uint8_t *hi, uint8_t *lo, const
                 w[u] = (qd < nquads && n < rows && k < K) ? __ldg(reinterpret_cast<const float4 *>(src + (int64_t)n * K + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
             if (spread) {
+                bool some = false;
 #pragma unroll
-                for (int u = 0; u < kBatch; u++) w[u] = spread_nan(w[u], qpr);
+                for (int u = 0; u < kBatch; u++) some |= maybe_nan(w[u]);
+                if (__any_sync(0xffffffffu, some)) {
+#pragma unroll
+                    for (int u = 0; u < kBatch; u++) w[u] = spread_nan(w[u], qpr);
+                }
             }
 #pragma unroll
             for (int u = 0; u < kBatch; u++) {

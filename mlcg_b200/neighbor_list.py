@@ -63,18 +63,21 @@ def _edges(x, r, batch, batch_size, ptr, loop, max_num_neighbors, rule, want_dis
     """``(edge_index, distance | None)`` for callers that return edges: their plan is made if an operator is given the list.  Structures from
     ``ptr``, or from ``batch`` and ``batch_size``.  A list, a list and then its plan, and both in one go as it was before, us:
     64 x 10 points 37, 68, 80; 256 x 73 (0.6 M edges) 72, 126, 108; 96 x 268 (1.8 M) 83, 157, 130; 256 x 4000 (65 M) 1005, 2180, 1815."""
+    if torch.is_inference_mode_enabled():               # (a plan made later has to know whether the list was written to)
+        with lasting():
+            return _edges(x, r, batch, batch_size, ptr, loop, max_num_neighbors, rule, want_distance, exclude)
     be, N, bounds = get_backend(), x.shape[0], None
     small = getattr(be, "small_graph_points", 0)
-    with lasting():                                     # (a plan made later has to know whether the list was written to)
-        if ptr is None and 0 < N <= small and exclude is None and batch_size is None and (batch is None or batch.numel() == N):
-            res = be.radius_graph_small(_as_3d(x), None if batch is None else batch.to(torch.int64), r, max_num_neighbors, loop, rule, want_distance)
-        else:
-            more = {"want_rows": False} if small else {}
-            bounds = _structure_ptr(x, batch, batch_size) if ptr is None else None
-            res = be.radius_graph(_as_3d(x), bounds if ptr is None else ptr, r, max_num_neighbors, loop, rule, want_distance=want_distance, want_batch=False, exclude=exclude, **more)
-        # an exclusion list need not hold both directions of a pair: such a graph is not taken to be symmetric
-        symmetric = exclude is None and not res["status"] & STATUS_TRUNCATED
-        return attach_plan(res["edge_index"], DeferredPlan(res["edge_index"], res["offsets"], bounds, N, symmetric, bool(loop))), res["distance"]
+    if ptr is None and 0 < N <= small and exclude is None and batch_size is None and (batch is None or batch.numel() == N):
+        res = be.radius_graph_small(_as_3d(x), None if batch is None else batch.to(torch.int64), r, max_num_neighbors, loop, rule, want_distance)
+    else:
+        more = {"want_rows": False} if small else {}
+        if ptr is None:
+            ptr = bounds = _structure_ptr(x, batch, batch_size)
+        res = be.radius_graph(_as_3d(x), ptr, r, max_num_neighbors, loop, rule, want_distance=want_distance, want_batch=False, exclude=exclude, **more)
+    # an exclusion list need not hold both directions of a pair: such a graph is not taken to be symmetric
+    symmetric = exclude is None and not res["status"] & STATUS_TRUNCATED
+    return attach_plan(res["edge_index"], DeferredPlan(res["edge_index"], res["offsets"], bounds, N, symmetric, bool(loop))), res["distance"]
 
 
 def _differentiated(x) -> bool:
