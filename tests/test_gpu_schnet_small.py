@@ -306,3 +306,24 @@ def test_a_weight_that_is_not_a_number_reaches_the_results(copies, num_rbf, prec
             weight.data[at] = before
     again = model(data()).out["SchNet"]
     assert torch.equal(again["energy"], want["energy"]) and torch.equal(again["forces"], want["forces"])
+
+
+@pytest.mark.parametrize("sizes", [[2049], [1500, 1400], [100] * 30])
+def test_room_of_large_batches(sizes):
+    """Above 2048 beads the workspace goes by the call before: one that is too small, exact or larger gives the evaluation of a given list."""
+    torch.manual_seed(0)
+    cut = bnn.CosineCutoff(0.0, 6.0)
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, 32, trainable=False), cut, [128], embedding_size=5, num_interactions=2).eval().to(DEV)
+    model, n, gen = bnn.GradientsOut(net, "forces").eval(), sum(sizes), torch.Generator().manual_seed(1)
+    pos, types_ = (torch.rand(n, 3, generator=gen) * 2.5 * max(sizes) ** (1 / 3)).to(DEV), torch.randint(0, 5, (n,), generator=gen).to(DEV)
+    make = lambda: mlcg_b200.AtomicData(pos=pos.clone(), atom_types=types_, batch=torch.repeat_interleave(torch.arange(len(sizes)), torch.tensor(sizes)).to(DEV),  # noqa: E731
+                                        n_atoms=torch.tensor(sizes, device=DEV))
+    given = make()
+    given.neighbor_list = net.neighbor_list(given, 6.0)
+    E = given.neighbor_list["SchNet"]["index_mapping"].shape[1]
+    want = model(given).out["SchNet"]
+    for guess in (0.0, (E - 2) / n / 1.04, E / n, 3 * E / n):
+        net.__dict__["_mlcgb_edges_per_bead_large"] = guess
+        got = model(make()).out["SchNet"]
+        assert torch.equal(got["energy"], want["energy"]) and torch.equal(got["forces"], want["forces"]), guess
+        assert net.__dict__["_mlcgb_edges_per_bead_large"] == E / n
