@@ -130,11 +130,12 @@ class DeferredPlan:
     kept for the stream that it was made on (another one makes its own, there is no order between the two) and never out of a
     recording, whose buffers hold nothing until it is replayed."""
 
-    __slots__ = ("index", "offsets", "ptr", "N", "symmetric", "loops", "_made", "_stream")
+    __slots__ = ("index", "offsets", "ptr", "N", "symmetric", "loops", "_home", "_made", "_stream")
 
     def __init__(self, edge_index: torch.Tensor, offsets: torch.Tensor, ptr: Optional[torch.Tensor], N: int, symmetric: bool, loops: bool):
         # (an alias: the list carries this object, which must not hold the list; ptr: the structure boundaries, None where they are the caller's)
         self.index, self.offsets, self.ptr, self.N, self.symmetric, self.loops = edge_index.detach(), offsets, ptr, N, symmetric, loops
+        self._home = torch._C._cuda_getCurrentRawStream(edge_index.get_device()) if edge_index.is_cuda else 0
         self._made = self._stream = None
 
     def plan(self) -> EdgePlan:
@@ -143,6 +144,10 @@ class DeferredPlan:
         recording = cuda and torch.cuda.is_current_stream_capturing()
         if self._made is not None and self._stream == stream and not recording:
             return self._made
+        if stream != self._home and not recording:      # (read there: their memory is not to be given to others while that stream is behind)
+            for t in (self.index, self.offsets, self.ptr):
+                if t is not None:
+                    t.record_stream(torch.cuda.current_stream(t.device))
         with lasting():
             be, E = get_backend(), self.index.shape[1]
             if self.symmetric and not self.loops and E % 2 == 0 and 0 < E < 1 << 31 and hasattr(be, "list_plan"):

@@ -270,3 +270,33 @@ def test_sizes_that_do_not_add_up(sizes, given):
     assert torch.equal(got["edge_index"], want["edge_index"]) and torch.equal(got["twin"], want["twin"])
     assert torch.equal(again["energy"], out["energy"]) and torch.equal(again["forces"], out["forces"])
     assert torch.allclose(fixed["energy"], out["energy"], rtol=1e-5, atol=1e-5 * float(out["energy"].abs().max()))
+
+
+@pytest.mark.parametrize("sizes", [[300], [73] * 60])
+def test_a_plan_asked_for_on_another_stream(sizes):
+    """The list goes out of use while the stream that makes its plan is still behind: its memory is not given to others before."""
+    from mlcg_b200 import radius_graph
+    from mlcg_b200.autograd import plan_of
+    gen, be, n = torch.Generator().manual_seed(8), get_backend(), sum(sizes)
+    pos = (torch.rand(n, 3, generator=gen) * 9).to(DEV)
+    batch = torch.repeat_interleave(torch.arange(len(sizes)), torch.tensor(sizes)).to(DEV)
+    make = lambda: radius_graph(pos, 4.0, batch, max_num_neighbors=1000, flow="target_to_source")  # noqa: E731
+    want_edges = make().clone()
+    want = plan_of(make(), n)
+    want = [t.clone() for t in (want.row0, want.row1, want.ptr_out, want.perm_in, want.half_selection(), want.pair_index())]
+    side = torch.cuda.Stream()
+    for _ in range(3):
+        edges = make()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(20_000_000)                  # (about 10 ms)
+            plan = plan_of(edges, n)
+        sizes_held = [edges.numel() * 8, (n + 1) * 8, (len(sizes) + 1) * 8]
+        del edges
+        held = [torch.full((k,), 0x7f, dtype=torch.uint8, device=DEV) for k in sizes_held for _ in range(4)]
+        torch.cuda.synchronize()
+        got = (plan.row0, plan.row1, plan.ptr_out, plan.perm_in, plan.half_selection(), plan.pair_index())
+        assert all(torch.equal(a, b) for a, b in zip(got, want)) and len(held) == 12
+        del plan, got, held
+    assert torch.equal(make(), want_edges)
+    be.check_pending()
