@@ -14,6 +14,7 @@ Bilinear family on a fixed edge list (row 0 = centre, row 1 = neighbour)::
     SegOut(a, V)[m] = sum_{e: row0(e)=m} a[row1(e)] * V[e]      its transpose
     EdgeMul(a, b)[e] = a[row0(e)] * b[row1(e)]
 """
+import weakref
 from dataclasses import dataclass
 from typing import Optional
 
@@ -161,16 +162,32 @@ class DeferredPlan:
         return plan
 
 
+class _Carried:
+    """A plan on the list that it is of, and the count of writes to the list that it goes with (None: a list without one).  Copies of the list
+    have counts of their own, and so none of the plan; in a file it is an empty set, which every mode of ``torch.load`` takes."""
+
+    __slots__ = ("plan", "version", "owner")
+
+    def __init__(self, plan, edge_index: torch.Tensor):
+        self.plan, self.owner = plan, weakref.ref(edge_index)
+        self.version = None if edge_index.is_inference() else edge_index._version
+
+    def __reduce__(self):
+        return set, ()
+
+
 def attach_plan(edge_index: torch.Tensor, plan) -> torch.Tensor:
     """``plan``: an :class:`EdgePlan` or a :class:`DeferredPlan`."""
-    edge_index._mlcgb_plan = plan, None if edge_index.is_inference() else edge_index._version
+    edge_index._mlcgb_plan = _Carried(plan, edge_index)
     return edge_index
 
 
 def carried_plan(edge_index: torch.Tensor):
     """What :func:`attach_plan` left with an edge list, None where the list has been written to since."""
-    plan, version = getattr(edge_index, "_mlcgb_plan", (None, None))
-    return plan if version is None or version == edge_index._version else None
+    carried = getattr(edge_index, "_mlcgb_plan", None)
+    if type(carried) is not _Carried or carried.owner() is not edge_index:
+        return None
+    return carried.plan if carried.version is None or carried.version == edge_index._version else None
 
 
 def attached_plan(edge_index: torch.Tensor) -> Optional[EdgePlan]:

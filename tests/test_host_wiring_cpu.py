@@ -531,3 +531,33 @@ def test_prior_parameters_kept_in_inference_mode_are_of_use_in_training():
             p.eval()._cached_params(data)
         energy = p.train()(data).out[k]["energy"]
         assert bool(torch.autograd.grad(energy.sum(), data.pos)[0].isfinite().all())
+
+
+@pytest.mark.parametrize("how", ["deepcopy", "copy", "file", "file, weights only"])
+def test_copies_of_a_list_have_plans_of_their_own(how):
+    """A copy of a list that was written to is planned for the edges it holds, also where its count of writes is the one that the other
+    list's plan was made for; a list on file is a tensor."""
+    import copy
+    import io
+
+    def again(t):
+        if how in ("copy", "deepcopy"):
+            return getattr(copy, how)(t)
+        file = io.BytesIO()
+        torch.save(t, file)
+        file.seek(0)
+        return torch.load(file, weights_only="only" in how)
+
+    pos = torch.rand(20, 3, generator=torch.Generator().manual_seed(1)) * 5
+    edges = mlcg_b200.radius_graph(pos, 3.0, max_num_neighbors=100, flow="target_to_source")
+    assert ag.plan_of(edges, 20).symmetric
+    copied = again(edges)
+    assert torch.equal(copied, edges) and torch.equal(ag.plan_of(copied, 20).row1.long(), edges[1])
+    for _ in range(4):
+        copied[:, :4] = copied[:, 4:8].clone()
+        copied = again(copied)
+        plan = ag.plan_of(copied, 20)
+        assert torch.equal(plan.row0.long(), copied[0]) and torch.equal(plan.row1.long(), copied[1])
+    other = again(copied)
+    copied[:, :4] = copied[:, 8:12].clone()
+    assert torch.equal(ag.plan_of(other, 20).row1.long(), other[1])
