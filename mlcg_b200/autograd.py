@@ -131,20 +131,21 @@ class DeferredPlan:
     kept for the stream that it was made on (another one makes its own, there is no order between the two) and never out of a
     recording, whose buffers hold nothing until it is replayed."""
 
-    __slots__ = ("index", "offsets", "ptr", "N", "symmetric", "loops", "_home", "_made", "_stream")
+    __slots__ = ("index", "offsets", "ptr", "N", "symmetric", "loops", "_home", "_made")
 
     def __init__(self, edge_index: torch.Tensor, offsets: torch.Tensor, ptr: Optional[torch.Tensor], N: int, symmetric: bool, loops: bool):
         # (an alias: the list carries this object, which must not hold the list; ptr: the structure boundaries, None where they are the caller's)
         self.index, self.offsets, self.ptr, self.N, self.symmetric, self.loops = edge_index.detach(), offsets, ptr, N, symmetric, loops
         self._home = torch._C._cuda_getCurrentRawStream(edge_index.get_device()) if edge_index.is_cuda else 0
-        self._made = self._stream = None
+        self._made = None, None             # (the plan and its stream, in one: threads may ask at the same time)
 
     def plan(self) -> EdgePlan:
         cuda = self.index.is_cuda
         stream = torch._C._cuda_getCurrentRawStream(self.index.get_device()) if cuda else 0
         recording = cuda and torch.cuda.is_current_stream_capturing()
-        if self._made is not None and self._stream == stream and not recording:
-            return self._made
+        made, of = self._made
+        if made is not None and of == stream and not recording:
+            return made
         if stream != self._home and not recording:      # (read there: their memory is not to be given to others while that stream is behind)
             for t in (self.index, self.offsets, self.ptr):
                 if t is not None:
@@ -158,7 +159,7 @@ class DeferredPlan:
                 row0, row1 = self.index.to(torch.int32).unbind(0)
                 plan = EdgePlan.from_centre_sorted(row0, row1, self.offsets, self.N, self.symmetric, self.loops)
         if not recording:
-            self._made, self._stream = plan, stream
+            self._made = plan, stream
         return plan
 
 
