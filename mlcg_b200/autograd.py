@@ -127,36 +127,39 @@ def _ptr_from_index(idx: torch.Tensor, N: int) -> torch.Tensor:
 
 
 class DeferredPlan:
-    """The plan of a centre-sorted list whose caller asked for the edges alone: made when an operator is first given the list.  It is
-    kept for the stream that it was made on (another one makes its own, there is no order between the two) and never out of a
-    recording, whose buffers hold nothing until it is replayed."""
+    """The plan of a centre-sorted list (int64 [2, E]) whose caller asked for the edges alone: made when an operator is first given the list.
+    It is kept for the stream that it was made on (another one makes its own, there is no order between the two) and never out of a
+    recording, whose buffers hold nothing until it is replayed.  Holds the offsets and boundaries of the list (None: the caller's), not the list."""
 
-    __slots__ = ("index", "offsets", "ptr", "N", "symmetric", "loops", "_home", "_made")
+    __slots__ = ("offsets", "ptr", "N", "E", "symmetric", "loops", "_home", "_made")
 
     def __init__(self, edge_index: torch.Tensor, offsets: torch.Tensor, ptr: Optional[torch.Tensor], N: int, symmetric: bool, loops: bool):
-        # (an alias: the list carries this object, which must not hold the list; ptr: the structure boundaries, None where they are the caller's)
-        self.index, self.offsets, self.ptr, self.N, self.symmetric, self.loops = edge_index.detach(), offsets, ptr, N, symmetric, loops
+        self.offsets, self.ptr, self.N, self.E, self.symmetric, self.loops = offsets, ptr, N, edge_index.shape[1], symmetric, loops
         self._home = torch._C._cuda_getCurrentRawStream(edge_index.get_device()) if edge_index.is_cuda else 0
         self._made = None, None             # (the plan and its stream, in one: threads may ask at the same time)
 
-    def plan(self) -> EdgePlan:
-        cuda = self.index.is_cuda
-        stream = torch._C._cuda_getCurrentRawStream(self.index.get_device()) if cuda else 0
-        recording = cuda and torch.cuda.is_current_stream_capturing()
+    def plan(self, edge_index: torch.Tensor) -> Optional[EdgePlan]:
+        """Of the list as it was handed out (None for one that has been given another shape)."""
+        E = self.E
+        if edge_index.shape != (2, E):
+            return None
+        stream, recording = 0, False
+        if edge_index.is_cuda:
+            stream, recording = torch._C._cuda_getCurrentRawStream(edge_index.get_device()), torch.cuda.is_current_stream_capturing()
         made, of = self._made
         if made is not None and of == stream and not recording:
             return made
         if stream != self._home and not recording:      # (read there: their memory is not to be given to others while that stream is behind)
-            for t in (self.index, self.offsets, self.ptr):
+            for t in (edge_index, self.offsets, self.ptr):
                 if t is not None:
                     t.record_stream(torch.cuda.current_stream(t.device))
         with lasting():
-            be, E = get_backend(), self.index.shape[1]
+            be = get_backend()
             if self.symmetric and not self.loops and E % 2 == 0 and 0 < E < 1 << 31 and hasattr(be, "list_plan"):
-                row0, row1, twin, sel, pair_of = be.list_plan(self.index, self.offsets, self.ptr, self.N)
+                row0, row1, twin, sel, pair_of = be.list_plan(edge_index.contiguous(), self.offsets, self.ptr, self.N)
                 plan = EdgePlan(self.N, E, row0, row1, self.offsets, None, row1, self.offsets, twin, row1, True, False, sel, pair_of)
             else:
-                row0, row1 = self.index.to(torch.int32).unbind(0)
+                row0, row1 = edge_index.to(torch.int32).unbind(0)
                 plan = EdgePlan.from_centre_sorted(row0, row1, self.offsets, self.N, self.symmetric, self.loops)
         if not recording:
             self._made = plan, stream
@@ -194,7 +197,7 @@ def carried_plan(edge_index: torch.Tensor):
 def attached_plan(edge_index: torch.Tensor) -> Optional[EdgePlan]:
     """The plan that travels with an edge list, None where the list has been written to since."""
     plan = carried_plan(edge_index)
-    return plan.plan() if isinstance(plan, DeferredPlan) else plan
+    return plan.plan(edge_index) if isinstance(plan, DeferredPlan) else plan
 
 
 def plan_of(edge_index: torch.Tensor, N: int) -> EdgePlan:
