@@ -1596,10 +1596,15 @@ __device__ __forceinline__ int64_t first_at_least(const int64_t *__restrict__ ba
     }
     return lo;
 }
+// Where structure b of B begins.  Every point has a structure, whatever the vector holds: where bisection goes right for an index it does
+// for a larger one, so the boundaries of an unsorted vector ascend too, and the first and the last are those of all points.
+__device__ __forceinline__ int64_t boundary(const int64_t *__restrict__ batch, int64_t N, int64_t b, int64_t B) {
+    return b <= 0 ? 0 : b >= B ? N : first_at_least(batch, N, b);
+}
 __global__ void batch_to_ptr_kernel(const int64_t *__restrict__ batch, int64_t N, int64_t B, int64_t *__restrict__ ptr) {
     const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (b > B) return;
-    ptr[b] = first_at_least(batch, N, b);
+    ptr[b] = boundary(batch, N, b, B);
 }
 
 __global__ void edge_twin_kernel(const int32_t *__restrict__ row0, const int32_t *__restrict__ row1,
@@ -2279,7 +2284,7 @@ __global__ void batch_boundaries_kernel(const int64_t *__restrict__ batch, int64
     const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, last = batch[N - 1];
     if (b == 0) publish(p, last, 0);
     if (b > last + 1 || b > most) return;
-    ptr[b] = first_at_least(batch, N, b);
+    ptr[b] = boundary(batch, N, b, last + 1);
 }
 
 __global__ void __launch_bounds__(kScanBlock) sizes_to_ptr_kernel(const int64_t *__restrict__ sizes, int64_t B, int64_t N, int64_t *__restrict__ ptr,

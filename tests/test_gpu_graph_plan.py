@@ -300,3 +300,29 @@ def test_a_plan_asked_for_on_another_stream(sizes):
         del plan, got, held
     assert torch.equal(make(), want_edges)
     be.check_pending()
+
+
+@pytest.mark.parametrize("n", [300, 3000, 9000])
+@pytest.mark.parametrize("how", ["last first", "shuffled", "below zero", "size too small", "size too large"])
+def test_batch_vectors_that_are_not_sorted(n, how):
+    """Undefined neighbours, but of points that are there: boundaries that ascend from 0 to N, edges inside it, and a call after it that is right."""
+    from mlcg_b200 import radius_graph
+    gen, be = torch.Generator().manual_seed(n), get_backend()
+    pos = (torch.rand(n, 3, generator=gen) * n ** (1 / 3) * 1.5).to(DEV)
+    sorted_batch = torch.sort(torch.randint(0, max(n // 700, 2), (n,), generator=gen))[0].to(DEV)
+    want = radius_graph(pos, 3.0, sorted_batch, max_num_neighbors=1000)
+    batch, more = sorted_batch.clone(), {}
+    if how == "last first":
+        batch = batch.flip(0)
+    elif how == "shuffled":
+        batch = batch[torch.randperm(n, generator=gen).to(DEV)]
+    elif how == "below zero":
+        batch -= 1
+    else:
+        more = dict(batch_size=int(batch.max()) + (0 if how == "size too small" else 5))
+    ptr = be.batch_to_ptr(batch, more["batch_size"]) if more else be.batch_boundaries(batch)
+    assert int(ptr[0]) == 0 and int(ptr[-1]) == n * (ptr.numel() > 1) and bool((ptr[1:] >= ptr[:-1]).all())
+    if ptr.numel() > 1:
+        edges = radius_graph(pos, 3.0, batch, max_num_neighbors=1000, **more)
+        assert edges.numel() == 0 or (int(edges.min()) >= 0 and int(edges.max()) < n and not bool((edges[0] == edges[1]).any()))
+    assert torch.equal(radius_graph(pos, 3.0, sorted_batch, max_num_neighbors=1000), want)
