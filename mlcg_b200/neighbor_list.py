@@ -176,11 +176,11 @@ def validate_neighborlist(inp: Mapping) -> bool:
 
 
 def sizes_or_pointer(data):
-    """``(n_atoms, None)`` where the structure sizes lie on the device of the positions as the kernels take them, else
-    ``(None, structure pointer)``."""
+    """``(n_atoms, None)`` where there are structure sizes (the kernels that take them check them), else ``(None, structure pointer)``."""
     n_atoms, pos = getattr(data, "n_atoms", None), data.pos
-    if (n_atoms is not None and torch.is_tensor(n_atoms) and n_atoms.dim() == 1 and n_atoms.dtype == torch.int64 and n_atoms.device == pos.device
-            and n_atoms.is_contiguous() and getattr(get_backend(), "plans_with_graph", False)):
+    if n_atoms is not None and torch.is_tensor(n_atoms) and n_atoms.dim() == 1 and getattr(get_backend(), "plans_with_graph", False):
+        if n_atoms.dtype != torch.int64 or n_atoms.device != pos.device or not n_atoms.is_contiguous():
+            n_atoms = n_atoms.to(device=pos.device, dtype=torch.int64).contiguous()
         return n_atoms, None
     return None, structure_pointer(data)
 
