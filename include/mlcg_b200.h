@@ -2,8 +2,8 @@
  * mlcg_b200 — C ABI of the B200 (sm_100a) kernels behind mlcg's coarse-grained force-field hot path.
  *
  * Conventions
- *   - Every pointer is a DEVICE pointer unless the comment says "host". The library never allocates,
- *     frees or synchronises (one entry point, mlcgb_radius_graph_static, waits for its stream once and says so):
+ *   - Every pointer is a DEVICE pointer unless the comment says "host". The library allocates and frees no
+ *     device memory and waits for the device only where an entry point hands a result to the host and says so:
  *     the caller owns inputs, outputs and workspaces and passes the stream.
  *   - `dtype`: 0 = float32, 1 = float64 (the type of positions and of every floating tensor of a call).
  *   - Node tensors are row-major [N, F]; edge tensors are row-major [E, F]; index rows are contiguous.
