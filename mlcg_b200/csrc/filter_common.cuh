@@ -151,6 +151,15 @@ __device__ __forceinline__ uint32_t filter_setup(const FilterFwdParams &p, uint8
     return *s_tmem;
 }
 
+// Largest |w_k| of the basis table, by all lanes of a warp
+__device__ __forceinline__ float table_max_width(const float2 *s_tab, int R, int lane) {
+    float w = 0.f;
+    for (int k = lane; k < R; k += 32) w = fmaxf(w, fabsf(s_tab[k].y));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) w = fmaxf(w, __shfl_xor_sync(0xffffffffu, w, o));
+    return w;
+}
+
 // h = tanh(z) for this thread's accumulator values, z = v * unscale + b1, through exp2: tanh z = sign(z) (1 - 2/(2^{|zz|} + 1)),
 // zz = 2 log2(e) z.  |zz| is clamped at 30, where the result has long rounded to 1, so that four denominators can share one
 // reciprocal (1/A = B C D / (A B C D), ...): five special-function operations per four values instead of eight — this phase

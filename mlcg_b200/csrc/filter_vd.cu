@@ -93,9 +93,9 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
             mbar_init(bars + 32 + 8 * i, 1);
         }
     }
-    float slope = 0.f;               // steepest basis function: |d g_k / dt| <= sqrt(2 ln2 w_k / e) where g_k = 2^(-w_k (t - c_k)^2)
-    for (int k = 0; k < R; k++) slope = fmaxf(slope, fabsf(s_tab[k].y));
-    slope = 0.7142f * sqrtf(slope);
+    // steepest basis function: |d g_k / dt| <= sqrt(2 ln2 w_k / e) where g_k = 2^(-w_k (t - c_k)^2).  (A lane looks at its share of the
+    // table here and below: every thread going through all of it took 4 of the 8-10 us of a CTA's set-up.)
+    const float slope = 0.7142f * sqrtf(table_max_width(s_tab, R, lane));
     // Where this quarter's functions are not zero as operands.  At w (t - c)^2 > 36 a function is below 2^-36: zero as a pair of fp16 (below
     // 2^-25), and so is its derivative on the scale of its row (below 16 (z / 0.6065 + 1) 2^-36 < 2^-28 at z = 7.1 widths).  Exp-normal
     // functions crowd the short distances that no bead comes to: of 128 over 15 A those beyond the 45th are zero at 4 A and more,
@@ -104,11 +104,16 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
     // reach further down: there the values left out are below 2^-36 where its rounding of the others is 2^-9 of them.  A weight that is not a
     // number is so in its whole row (spread_nan) and reaches the sums through the quarter that is always there.
     float near_lo = INFINITY, near_hi = -INFINITY;
-    for (int k = col0; k < col0 + 32 && k < R; k++) {
-        const float2 cw = s_tab[k];
+    if (col0 + lane < R) {
+        const float2 cw = s_tab[col0 + lane];
         const float reach = cw.y > 0.f ? sqrtf(36.f / cw.y) : INFINITY;
         near_lo = fminf(near_lo, cw.x - reach);
         near_hi = fmaxf(near_hi, cw.x + reach);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        near_lo = fminf(near_lo, __shfl_xor_sync(0xffffffffu, near_lo, o));
+        near_hi = fmaxf(near_hi, __shfl_xor_sync(0xffffffffu, near_hi, o));
     }
     __syncthreads();
     pdl_wait();                      // set-up done (weights only); from here on the distances of the previous kernels are read

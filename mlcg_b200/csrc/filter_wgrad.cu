@@ -88,8 +88,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) filter_wgrad_kernel(const __gri
     const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t a2_hi = smem_u32(smem + L::kA2), a2_lo = a2_hi + 32768, x_hi = smem_u32(X), x_lo = x_hi + 32768, y_hi = smem_u32(Y), y_lo = y_hi + 32768;
 
-    float slope = 0.f;
-    for (int k = 0; k < R; k++) slope = fmaxf(slope, fabsf(s_tab[k].y));
+    const float slope = table_max_width(s_tab, R, lane);
     // right operands: |h|, |phi| <= 1, |h'| <= |z'|, and a bound on |phi'|
     const float env1 = q.rbf.cutoff_kind == 0 ? 0.f : 3.1416f / (q.rbf.lower > 0.f ? q.rbf.upper - q.rbf.lower : 2.f * q.rbf.upper);
     const float phi1 = 0.7142f * sqrtf(slope) * (q.rbf.kind == 0 ? 1.f : fabsf(q.rbf.alpha) * expf(fmaxf(q.rbf.alpha * q.rbf.lower, 0.f))) + fabsf(env1);

@@ -223,7 +223,7 @@ __device__ __forceinline__ bool load_weight_tile(uint8_t *hi, uint8_t *lo, const
                                                  float scale, bool spread = false) {
     float wmax = 0.f;
     auto put4 = [&](int n, int k, float4 w) { wmax = fmaxf(wmax, put_weight4<SPLIT>(hi, lo, n, k, w, scale)); };
-    const int qpr = Kpad >> 2, nquads = kRows * qpr;          // quads per row, quads in the tile
+    const int lg = Kpad == 128 ? 5 : 4, qpr = 1 << lg, nquads = kRows * qpr;          // quads per row (Kpad is 64 or 128), quads in the tile
     if ((K & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
         constexpr int kBatch = 8;
         for (int base = threadIdx.x; base < nquads; base += kBatch * blockDim.x) {
@@ -231,7 +231,7 @@ __device__ __forceinline__ bool load_weight_tile(uint8_t *hi, uint8_t *lo, const
 #pragma unroll
             for (int u = 0; u < kBatch; u++) {
                 const int qd = base + u * blockDim.x;
-                const int n = qd / qpr, k = (qd - n * qpr) << 2;
+                const int n = qd >> lg, k = (qd & (qpr - 1)) << 2;
                 w[u] = (qd < nquads && n < rows && k < K) ? __ldg(reinterpret_cast<const float4 *>(src + (int64_t)n * K + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
             if (spread) {
@@ -246,16 +246,13 @@ __device__ __forceinline__ bool load_weight_tile(uint8_t *hi, uint8_t *lo, const
 #pragma unroll
             for (int u = 0; u < kBatch; u++) {
                 const int qd = base + u * blockDim.x;
-                if (qd < nquads) {
-                    const int n = qd / qpr;
-                    put4(n, (qd - n * qpr) << 2, w[u]);
-                }
+                if (qd < nquads) put4(qd >> lg, (qd & (qpr - 1)) << 2, w[u]);
             }
         }
         return SPLIT && !(wmax * scale <= 32768.f);
     }
     for (int qd = threadIdx.x; qd < nquads; qd += blockDim.x) {
-        const int n = qd / qpr, k = (qd - n * qpr) << 2;
+        const int n = qd >> lg, k = (qd & (qpr - 1)) << 2;
         float v[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) v[j] = (n < rows && k + j < K) ? src[(int64_t)n * K + k + j] : 0.f;
