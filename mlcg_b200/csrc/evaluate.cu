@@ -44,7 +44,7 @@ int evaluate_small(const void *pos, const int64_t *types, const int64_t *n_atoms
     s.row1 = row1 ? row1 : (int32_t *)(at + row);      // (places as below, without row0)
     s.twin = (int32_t *)(at + 2 * row);
     s.pair_of = (int32_t *)(at + 3 * row);
-    s.sel = (int32_t *)(at + 4 * row);
+    s.pair_d = (float *)(at + 4 * row);
     s.offsets = (int64_t *)(g + G.offsets);
     s.pub = pub;
     return schnet_eval_small(pos, types, N, B, s, rbf, conv_cutoff_kind, conv_lower, conv_upper, w, precision, at + lists, bytes - lists, energy, grad_pos,

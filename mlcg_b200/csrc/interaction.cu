@@ -297,7 +297,7 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
     const int64_t H = w->hidden, F = w->filters, H2 = w->conv_out, Wh = w->head_width, L = w->num_blocks;
     if (F != 128 || H > 128 || H2 > 128 || Wh > 128 || (H & 3) || (H2 & 3) || (Wh & 3) || L < 1) return MLCGB_E_LIMIT;
     if (!pos || !types || !offsets || !w->embedding || !w->blocks || !w->head_W || !w->head_b || !w->head_out || !workspace) return MLCGB_E_ARG;
-    if (E > 0 && ((!row0 && !graph) || !row1 || !sel || !pair_of || !twin || 2 * P != E)) return MLCGB_E_ARG;
+    if (E > 0 && ((!row0 && !graph) || !row1 || (!sel && !graph) || !pair_of || !twin || 2 * P != E)) return MLCGB_E_ARG;
     const SchnetLayout lay = schnet_layout(N, E, P, H, F, H2, Wh, L);
     if (workspace_bytes < (size_t)lay.total * sizeof(float)) return MLCGB_E_WORKSPACE;
     float *ws = (float *)workspace;
@@ -311,7 +311,7 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
     auto filters = [&](int64_t l, int64_t n) {                               // of blocks l .. l + n - 1, with derivatives where a force pass follows
         float *W = ws + lay.W + l * lay.wstride;
         if (grad_pos)
-            return filter_vd_blocks(d, P, pairs_dev, sel, rbf, conv_cutoff_kind, conv_lower, conv_upper, w->blocks + l, n, precision, W,
+            return filter_vd_blocks(graph ? graph->pair_d : d, P, pairs_dev, graph ? nullptr : sel, rbf, conv_cutoff_kind, conv_lower, conv_upper, w->blocks + l, n, precision, W,
                                     ws + lay.Wd + l * lay.wstride, nullptr, nullptr, nullptr, filter_images ? image(3 * L + 1 + 2 * l) : nullptr, status, st);
         int rf = MLCGB_OK;
         for (int64_t k = l; k < l + n && !rf; k++)
@@ -415,7 +415,7 @@ int mlcgb::schnet_eval_small(const void *pos, const int64_t *types, int64_t N, i
                              double conv_lower, double conv_upper, const mlcgb_schnet_weights *w, int precision, void *workspace, size_t workspace_bytes,
                              void *energy, void *grad_pos, float grad_sign, int32_t *status, cudaStream_t st) {
     if (!grad_pos || !small_graph_ok(N, B, w)) return MLCGB_E_LIMIT;
-    return schnet_eval_impl(pos, types, g.ptr, N, B, nullptr, g.row1, g.offsets, g.sel, g.pair_of, g.twin, g.capacity, g.capacity / 2, g.counts, rbf,
+    return schnet_eval_impl(pos, types, g.ptr, N, B, nullptr, g.row1, g.offsets, nullptr, g.pair_of, g.twin, g.capacity, g.capacity / 2, g.counts, rbf,
                             conv_cutoff_kind, conv_lower, conv_upper, w, precision, workspace, workspace_bytes, energy, grad_pos, grad_sign, status, st, &g);
 }
 

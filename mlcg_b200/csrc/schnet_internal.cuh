@@ -91,7 +91,8 @@ struct SmallGraph {
     int64_t max_nn, capacity;
     uint2 *masks;                          // [N][(N + 31) / 32]
     int32_t *deg, *upper;                  // [N]
-    int32_t *row1, *twin, *pair_of, *sel;  // [capacity], sel [capacity / 2]
+    int32_t *row1, *twin, *pair_of;        // [capacity]
+    float *pair_d;                         // [capacity / 2]: distances of the pairs, which the filters read in order
     int64_t *offsets, *counts;             // [N + 1]; {edges, pairs}
     Publish pub;                           // host NULL: reported in the evaluation's status word
 };

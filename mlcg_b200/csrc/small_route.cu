@@ -2,15 +2,15 @@
 //
 // At these sizes an evaluation is a chain of dependent launches, and what counts is how long one link takes.  A tensor-core kernel
 // over node rows takes 8-11 us for its only tile (a 128-row tile on one SM: fp16 conversion, two exchanges and 1400 cycles of
-// issue per GEMM, and 32 columns of epilogue per thread), whatever the batch.  Here a CTA takes 8 rows (4 where that still
-// gives every SM at most one tile), so the rows spread over the chip, and one kernel does a whole link: the aggregation of its
+// issue per GEMM, and 32 columns of epilogue per thread), whatever the batch.  Here a CTA takes 1 to 8 rows (small_rows()),
+// so the rows spread over the chip, and one kernel does a whole link: the aggregation of its
 // nodes, the Linear layers behind it up to the next aggregation, activations and residuals between them, in plain fp32:
 //   forward, block l   agg -> lin2, tanh -> lin, + x -> lin1 of block l+1       (last block: output network, its gradient and
 //                                                                                 the first step of the force pass instead)
 //   force pass         gagg -> aggregation + edge dot products -> lin1^T, + g -> lin^T, tanh' -> lin2^T of block l-1
 // and the two along a tangent and back that a force-matching step adds.  Weights (three 64 KB matrices) are copied to shared
-// memory before the kernel waits for its predecessor.  A 128-column layer over 8 rows is 1300 issue slots per scheduler (four
-// k-ranges by 128 columns; partial sums through shared memory).  Launches per evaluation of L blocks: 2 L + 3 where the tensor-core
+// memory while the kernel waits for its predecessor, each waited for in front of its layer (SmallTile says how a layer is split; a
+// column and 32 k per thread over tiles of 4 or 8 rows: 61.4 us an evaluation of 64 x 10 beads, like this 52).  Launches per evaluation of L blocks: 2 L + 3 where the tensor-core
 // sequence takes 7 L + 7; one evaluation of 64 x 10 beads, two blocks: 154 us of kernels before.
 // For many more rows per SM the tensor-core kernels are the faster ones (figures at kSmallNodes).
 #include "schnet_internal.cuh"
@@ -46,67 +46,109 @@ struct SmallSmem {
     static constexpr int kS = 3 * kWFloats;                                 // two row tiles [RT][128]
     static constexpr int kX = kS + 2 * RT * 128;                            // partial sums [4][RT][128]; the aggregation's [16][128]
     static constexpr int kXFloats = 16 * 128 > 4 * RT * 128 ? 16 * 128 : 4 * RT * 128;
-    static constexpr int kDot = kX + kXFloats;                              // [16 warps][4]... dot products of four edges
-    static constexpr size_t kBytes = sizeof(float) * (kDot + 64);
+    static constexpr size_t kBytes = sizeof(float) * (kX + kXFloats);
 };
 
 __device__ __forceinline__ void fma4s(float4 &acc, const float4 &a, const float4 &b) {
     acc.x = fmaf(a.x, b.x, acc.x); acc.y = fmaf(a.y, b.y, acc.y); acc.z = fmaf(a.z, b.z, acc.z); acc.w = fmaf(a.w, b.w, acc.w);
 }
+template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// What a thread multiplies with in a layer: 16 k of two columns, w[4 i + j] and w[16 + 4 i + j] at k = 32 kq + 8 i + 4 kh + j
+struct SmallWeights { float w[32]; };
+
+// A layer over RT rows: warp = 32 columns (warp & 3) by a quarter of k (kq = warp >> 2); lane = two columns (lane & 15) by half of every
+// eight k (kh = lane >> 4).  What bounds it is what shared memory hands to registers: a broadcast 128-bit read takes two cycles like any
+// 256 bytes, so a second column per thread halves the rows' share (256 -> 128 cycles a row and layer), and the halves of k meet in one
+// exchange a row.  (Measured on one SM: broadcast 128-bit reads 2.1 cycles a warp, full ones 4.0; packed multiplications no faster than plain.)
 template <int RT>
 struct SmallTile {
-    static constexpr int RO = RT / 4;         // rows a thread holds after a layer: rows kq * RO + i, column c
+    static constexpr int RO = (RT + 3) / 4;   // rows a thread holds after a layer: rows rq + 4 i, column c
     float *smem, *x;
-    int tid, c, kq, lane, warp;
+    int tid, c, rq, lane, warp;
     int64_t n0, N;
 
+    __device__ __forceinline__ SmallTile(float4 *base, int at_x, int64_t N_)
+        : smem(reinterpret_cast<float *>(base)), x(smem + at_x), tid(threadIdx.x), c(threadIdx.x & 127), rq(threadIdx.x >> 7), lane(threadIdx.x & 31),
+          warp(threadIdx.x >> 5), n0(0), N(N_) {}
     __device__ __forceinline__ float *slot(int i) const { return smem + SmallSmem<RT>::kW + i * SmallSmem<RT>::kWFloats; }
     __device__ __forceinline__ float *rows(int i) const { return smem + SmallSmem<RT>::kS + i * RT * 128; }
-    // matrix [rows][128] -> slot, asynchronously; rows past the end zero
+    // matrix [rows][128] -> slot, asynchronously, a group of copies of its own; rows past the end zero
     __device__ __forceinline__ void fetch(int i, const float *src, int nrows) const {
         const uint32_t base = tc::smem_u32(slot(i));
+        if (src) {
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int idx = tid + u * kST, row = idx >> 5, ch = idx & 31;
-            const int nbytes = row < nrows ? 16 : 0;
-            const float *g = row < nrows ? src + row * 128 + ch * 4 : src;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + (row * kWPitch + ch * 4) * 4), "l"(g), "r"(nbytes) : "memory");
+            for (int u = 0; u < 8; u++) {
+                const int idx = tid + u * kST, row = idx >> 5, ch = idx & 31;
+                const int nbytes = row < nrows ? 16 : 0;
+                const float *g = row < nrows ? src + row * 128 + ch * 4 : src;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + (row * kWPitch + ch * 4) * 4), "l"(g), "r"(nbytes) : "memory");
+            }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    // v[i] = sum_k S[row][k] W(k, c): NT: W stored [c][k], else [k][c].  Ends with every thread past its reads of S.
+    // NT: columns lane & 15 and 16 more, W stored [c][k]; else neighbouring columns, W stored [k][c]: no bank is met twice either way
+    template <bool NT> __device__ __forceinline__ int column() const { return (warp & 3) * 32 + (NT ? (lane & 15) : 2 * (lane & 15)); }
     template <bool NT>
-    __device__ __forceinline__ void layer(const float *S, const float *Wm, float (&v)[RO]) const {
-        float acc[RT];
+    __device__ __forceinline__ SmallWeights weights(const float *Wm) const {
+        SmallWeights r;
+        const int c0 = column<NT>(), k0 = (warp >> 2) * 32 + (lane >> 4) * 4;
 #pragma unroll
-        for (int r = 0; r < RT; r++) acc[r] = 0.f;
-        const int k0 = kq * 32;
-#pragma unroll
-        for (int kk = 0; kk < 32; kk += 4) {
-            float w[4];
+        for (int i = 0; i < 4; i++) {
+            const int k = k0 + 8 * i;
             if (NT) {
-                const float4 w4 = *reinterpret_cast<const float4 *>(Wm + c * kWPitch + k0 + kk);
-                w[0] = w4.x; w[1] = w4.y; w[2] = w4.z; w[3] = w4.w;
+                const float4 a = *reinterpret_cast<const float4 *>(Wm + c0 * kWPitch + k), b = *reinterpret_cast<const float4 *>(Wm + (c0 + 16) * kWPitch + k);
+                r.w[4 * i] = a.x; r.w[4 * i + 1] = a.y; r.w[4 * i + 2] = a.z; r.w[4 * i + 3] = a.w;
+                r.w[16 + 4 * i] = b.x; r.w[17 + 4 * i] = b.y; r.w[18 + 4 * i] = b.z; r.w[19 + 4 * i] = b.w;
             } else {
 #pragma unroll
-                for (int j = 0; j < 4; j++) w[j] = Wm[(k0 + kk + j) * kWPitch + c];
-            }
-#pragma unroll
-            for (int r = 0; r < RT; r++) {
-                const float4 a = *reinterpret_cast<const float4 *>(S + r * 128 + k0 + kk);
-                acc[r] = fmaf(a.x, w[0], fmaf(a.y, w[1], fmaf(a.z, w[2], fmaf(a.w, w[3], acc[r]))));
+                for (int j = 0; j < 4; j++) {
+                    const float2 a = *reinterpret_cast<const float2 *>(Wm + (k + j) * kWPitch + c0);
+                    r.w[4 * i + j] = a.x;
+                    r.w[16 + 4 * i + j] = a.y;
+                }
             }
         }
+        return r;
+    }
+    // v[i] = sum_k S[row][k] W(k, c).  Ends with every thread past its reads of S.
+    template <bool NT>
+    __device__ __forceinline__ void multiply(const float *S, const SmallWeights &m, float (&v)[RO]) const {
+        const int kh = lane >> 4, k0 = (warp >> 2) * 32 + kh * 4;
+        float acc[RT][2];
 #pragma unroll
-        for (int r = 0; r < RT; r++) x[(kq * RT + r) * 128 + c] = acc[r];
+        for (int r = 0; r < RT; r++) acc[r][0] = acc[r][1] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+#pragma unroll
+            for (int r = 0; r < RT; r++) {
+                const float4 a = *reinterpret_cast<const float4 *>(S + r * 128 + k0 + 8 * i);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const float *w = m.w + 16 * h + 4 * i;
+                    acc[r][h] = fmaf(a.x, w[0], fmaf(a.y, w[1], fmaf(a.z, w[2], fmaf(a.w, w[3], acc[r][h]))));
+                }
+            }
+        }
+        const int col = column<NT>() + (NT ? 16 * kh : kh);
+#pragma unroll
+        for (int r = 0; r < RT; r++) {
+            const float mine = kh ? acc[r][1] : acc[r][0], other = kh ? acc[r][0] : acc[r][1];
+            x[((warp >> 2) * RT + r) * 128 + col] = mine + __shfl_xor_sync(0xffffffffu, other, 16);
+        }
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < RO; i++) {
-            const int r = kq * RO + i;
-            v[i] = (x[r * 128 + c] + x[(RT + r) * 128 + c]) + (x[(2 * RT + r) * 128 + c] + x[(3 * RT + r) * 128 + c]);
+            const int r = rq + 4 * i;
+            v[i] = 0.f;
+            if (r < RT) v[i] = (x[r * 128 + c] + x[(RT + r) * 128 + c]) + (x[(2 * RT + r) * 128 + c] + x[(3 * RT + r) * 128 + c]);
         }
     }
-    __device__ __forceinline__ int64_t node(int i) const { return n0 + kq * RO + i; }
+    template <bool NT>
+    __device__ __forceinline__ void layer(const float *S, const float *Wm, float (&v)[RO]) const {
+        multiply<NT>(S, weights<NT>(Wm), v);
+    }
+    __device__ __forceinline__ int64_t node(int i) const { return rq + 4 * i < RT ? n0 + rq + 4 * i : N; }      // (N: none)
     __device__ __forceinline__ float get(const float *p, int i) const { return node(i) < N ? p[node(i) * 128 + c] : 0.f; }
     __device__ __forceinline__ void put(float *p, int i, float v) const {
         if (p && node(i) < N) p[node(i) * 128 + c] = v;
@@ -114,7 +156,8 @@ struct SmallTile {
     // values -> row tile for the next layer; every thread sees it after
     __device__ __forceinline__ void hand_on(float *S, const float (&v)[RO]) const {
 #pragma unroll
-        for (int i = 0; i < RO; i++) S[(kq * RO + i) * 128 + c] = v[i];
+        for (int i = 0; i < RO; i++)
+            if (rq + 4 * i < RT) S[(rq + 4 * i) * 128 + c] = v[i];
         __syncthreads();
     }
 };
@@ -134,7 +177,7 @@ __device__ __forceinline__ SmallEdges small_edges(const SmallNet &p, const Small
     const int part = t.warp % WPR;
     const int64_t n = t.n0 + t.warp / WPR;
     SmallEdges e = {0, 0, 0, 0};
-    if (n >= p.N) return e;
+    if (n >= p.N || t.warp >= RT * WPR) return e;
     // (past the first-level cache: this may run before the wait for the kernel in front, where that cache may hold the lists of another call)
     const int64_t b0 = __ldcg(p.ptr + n), b1 = __ldcg(p.ptr + n + 1), per = (b1 - b0 + WPR - 1) / WPR;
     e.k0 = b0 + part * per;
@@ -148,12 +191,12 @@ __device__ __forceinline__ SmallEdges small_edges(const SmallNet &p, const Small
 
 template <int MODE, int RT>
 __device__ __forceinline__ void small_aggregate(const SmallNet &p, const SmallTile<RT> &t, float *S, const SmallEdges &ed) {
-    constexpr int WPR = 16 / RT;
+    constexpr int WPR = 16 / RT;                                       // (warps that have no row are idle)
     const int row = t.warp / WPR, lane = t.lane;
     const int64_t n = t.n0 + row;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 *red = reinterpret_cast<float4 *>(t.x);                     // [16][32]
-    if (n < p.N) {
+    if (n < p.N && row < RT) {
         const int64_t k0 = ed.k0, k1 = ed.k1;
         const float4 *a4 = reinterpret_cast<const float4 *>(p.in_a) + lane, *b4 = reinterpret_cast<const float4 *>(p.in_b) + lane;
         const float4 *W4 = reinterpret_cast<const float4 *>(p.W) + lane, *Wd4 = reinterpret_cast<const float4 *>(p.Wd) + lane;
@@ -233,16 +276,11 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
     extern __shared__ float4 small_smem[];
     using T = SmallTile<RT>;
     constexpr int RO = T::RO;
-    T t;
-    t.smem = reinterpret_cast<float *>(small_smem);
-    t.x = t.smem + SmallSmem<RT>::kX;
-    t.tid = threadIdx.x; t.c = threadIdx.x & 127; t.kq = threadIdx.x >> 7; t.lane = threadIdx.x & 31; t.warp = threadIdx.x >> 5;
-    t.N = p.N;
+    T t(small_smem, SmallSmem<RT>::kX, p.N);
     constexpr bool kLast = KIND == kSmFwdLast || KIND == kSmTanLast;
-    if (p.w[0]) t.fetch(0, p.w[0], 128);
-    if (p.w[1]) t.fetch(1, p.w[1], 128);
-    if (p.w[2]) t.fetch(2, p.w[2], kLast ? p.Wh : 128);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    t.fetch(0, p.w[0], 128);
+    t.fetch(1, p.w[1], 128);
+    t.fetch(2, p.w[2], kLast ? p.Wh : 128);
     // What does not come from the kernel in front is read before the wait for it, a latency of the second-level cache each: biases and the
     // lists of the first tile (the kernel in front began behind those that made the lists).  What does, and is wanted after a layer,
     // is read under the aggregation (64 x 10 beads replayed: 64 -> 60.5 us).
@@ -263,12 +301,9 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
             res[i] = p.res ? t.get(p.res, i) : 0.f;
             act[i] = kForward || KIND == kSmRevFirst ? 0.f : t.get(p.act, i);
         }
+        copies_wait<2>();                                              // (a matrix is waited for in front of the barrier before its layer)
         small_aggregate<kForward ? kAggPlain : (KIND == kSmBwd ? kAggForce : kAggTangent), RT>(p, t, S0, ed);
-        if (!ready) {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            __syncthreads();
-            ready = true;
-        }
+        ready = true;
         float v[RO], a[RO], q[RO];
         if (KIND == kSmFwd || KIND == kSmFwdLast) {
             t.template layer<true>(S0, t.slot(0), v);                  // lin2 + tanh
@@ -277,6 +312,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 a[i] = tc::tanh_ex2(v[i] + b2);
                 t.put(p.o_act, i, a[i]);
             }
+            copies_wait<1>();
             t.hand_on(S1, a);
             t.template layer<true>(S1, t.slot(1), v);                  // lin + residual
 #pragma unroll
@@ -284,6 +320,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 v[i] += b3 + res[i];
                 t.put(p.o_x, i, v[i]);
             }
+            copies_wait<0>();
             t.hand_on(S0, v);
             t.template layer<true>(S0, t.slot(2), v);                  // lin1 of the next block | output network
             if (KIND == kSmFwd) {
@@ -330,6 +367,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 v[i] += res[i];
                 t.put(p.o_g, i, v[i]);
             }
+            copies_wait<1>();
             t.hand_on(S1, v);
             t.template layer<false>(S1, t.slot(1), v);                 // lin^T, tanh' of the block below
 #pragma unroll
@@ -337,6 +375,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 v[i] *= fmaf(-act[i], act[i], 1.f);
                 t.put(p.o_gu, i, v[i]);
             }
+            copies_wait<0>();
             t.hand_on(S0, v);
             t.template layer<false>(S0, t.slot(2), v);                 // lin2^T
 #pragma unroll
@@ -351,6 +390,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 t.put(p.o_act, i, v[i]);
                 if (KIND == kSmTan) t.put(p.o_q, i, q[i]);
             }
+            copies_wait<1>();
             t.hand_on(S1, v);
             t.template layer<true>(S1, t.slot(1), v);
 #pragma unroll
@@ -358,6 +398,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 v[i] += res[i];
                 t.put(p.o_x, i, v[i]);
             }
+            copies_wait<0>();
             t.hand_on(S0, v);
             t.template layer<true>(S0, t.slot(2), v);
             if (KIND == kSmTan) {
@@ -411,6 +452,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 t.put(p.o_g, i, v[i]);
             }
             if (KIND == kSmRev) {
+                copies_wait<1>();
                 t.hand_on(S1, v);
                 t.template layer<false>(S1, t.slot(1), v);
 #pragma unroll
@@ -418,6 +460,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                     v[i] = fmaf(v[i], fmaf(-act[i], act[i], 1.f), t.get(p.q, i));
                     t.put(p.o_ub, i, v[i]);
                 }
+                copies_wait<0>();
                 t.hand_on(S0, v);
                 t.template layer<false>(S0, t.slot(2), v);
 #pragma unroll
@@ -426,7 +469,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
         }
         __syncthreads();                                               // the tile buffers are free for the next rows
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    copies_wait<0>();
 }
 
 // Embedding rows and lin1 of the first block, eight nodes
@@ -460,13 +503,8 @@ small_start_kernel(const float *__restrict__ pos, const int64_t *__restrict__ ty
                    float *__restrict__ x, float *__restrict__ xl, int32_t *__restrict__ status) {
     extern __shared__ float4 small_smem[];
     constexpr int RT = 8;
-    SmallTile<RT> t;
-    t.smem = reinterpret_cast<float *>(small_smem);
-    t.x = t.smem + SmallSmem<RT>::kX;
-    t.tid = threadIdx.x; t.c = threadIdx.x & 127; t.kq = threadIdx.x >> 7; t.lane = threadIdx.x & 31; t.warp = threadIdx.x >> 5;
-    t.N = N;
+    SmallTile<RT> t(small_smem, SmallSmem<RT>::kX, N);
     t.fetch(0, W1, 128);
-    asm volatile("cp.async.commit_group;" ::: "memory");
     pdl_wait();
     pdl_launch_dependents();
     for (int64_t e = (int64_t)blockIdx.x * kST + threadIdx.x; e < E; e += (int64_t)gridDim.x * kST) {
@@ -479,7 +517,7 @@ small_start_kernel(const float *__restrict__ pos, const int64_t *__restrict__ ty
         }
         d[e] = v;
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    copies_wait<0>();
     for (t.n0 = (int64_t)blockIdx.x * RT; t.n0 < N; t.n0 += (int64_t)gridDim.x * RT) {
         __syncthreads();
         embedding_rows(t, t.rows(0), types, num_types, table, x, xl, status);
@@ -510,14 +548,9 @@ small_graph_count_kernel(const float *__restrict__ pos, const SmallGraph g, int6
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if ((int)blockIdx.x >= count_blocks) {
-        SmallTile<8> t;
-        t.smem = reinterpret_cast<float *>(small_smem);
-        t.x = t.smem + SmallStartSmem::kX;
-        t.tid = threadIdx.x; t.c = threadIdx.x & 127; t.kq = threadIdx.x >> 7; t.lane = lane; t.warp = warp;
-        t.N = N;
+        SmallTile<8> t(small_smem, SmallStartSmem::kX, N);
         t.fetch(0, W1, 128);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        copies_wait<0>();
         for (t.n0 = (int64_t)(blockIdx.x - count_blocks) * 8; t.n0 < N; t.n0 += (int64_t)(gridDim.x - count_blocks) * 8) {
             __syncthreads();
             embedding_rows(t, t.smem + SmallStartSmem::kS, types, num_types, table, x, xl, status);
@@ -546,7 +579,9 @@ small_graph_fill_kernel(const float *__restrict__ pos, const SmallGraph g, int64
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_all = (int)N;
     pdl_launch_dependents();
     pdl_wait();
-    const int sizes = blockIdx.x == 0 && threadIdx.x == 0 ? __ldcg(status) & kSizes : 0;      // (what the count found)
+    // (the host's line is written by a block of its own: its system-wide fence held a block with edges up for 2.5 us)
+    const bool publishes = g.pub.host && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0;
+    const int sizes = publishes ? __ldcg(status) & kSizes : 0;                                // (what the count found)
     for (int b = threadIdx.x; b <= B; b += kFillThreads) s_ptr[b] = (int)g.ptr[b];
     static_assert(kMaskNodes == 2 * kFillThreads, "two beads per thread");
     const int i0 = 2 * threadIdx.x;
@@ -586,13 +621,13 @@ small_graph_fill_kernel(const float *__restrict__ pos, const SmallGraph g, int64
         if (threadIdx.x == 0) {
             g.counts[0] = bad ? 0 : total;
             g.counts[1] = bad ? 0 : total >> 1;
-            if (g.pub.host) publish(g.pub, total, (cut ? (int)kTruncated : 0) | sizes);
-            else if (bad) atomicOr(status, (cut ? (int)kTruncated : 0) | (total > g.capacity ? (int)kCapacity : 0) | (total & 1 ? (int)kAsymmetric : 0));
+            if (!g.pub.host && bad) atomicOr(status, (cut ? (int)kTruncated : 0) | (total > g.capacity ? (int)kCapacity : 0) | (total & 1 ? (int)kAsymmetric : 0));
         }
         if (i0 <= n_all) g.offsets[i0] = bad ? 0 : e0;
         if (i0 + 1 <= n_all) g.offsets[i0 + 1] = bad ? 0 : e0 + k0;
         if (i0 + 2 == n_all) g.offsets[n_all] = bad ? 0 : total;
     }
+    if (publishes) publish(g.pub, total, (cut ? (int)kTruncated : 0) | sizes);
     if (bad) return;
     __syncthreads();
     const int words = (n_all + 31) >> 5, P = (int)(total >> 1);
@@ -617,62 +652,69 @@ small_graph_fill_kernel(const float *__restrict__ pos, const SmallGraph g, int64
             g.row1[slot] = j;
             g.twin[slot] = place.ok ? place.twin : slot;
             g.pair_of[slot] = place.ok ? place.pair : 0;
-            d[slot] = sqrtf(d2);
-            if (place.ok && j > i) g.sel[place.pair] = slot;
+            const float r = sqrtf(d2);
+            d[slot] = r;
+            if (place.ok && j > i) g.pair_d[place.pair] = r;
         });
     }
 }
 
-// Forces and energies: the dot products of the first block taken here in both directions (one node's edges per warp, so nothing is
-// written per edge), those of the other blocks read from s
-__global__ void __launch_bounds__(256)
+// Forces and energies: the dot products of the first block taken here in both directions (a node's edges by WPN warps, so nothing is
+// written per edge), those of the other blocks read from s.  A latency chain: with one warp per node, four edges at a time, it took
+// 4.5-4.9 us behind the last link, most of it the later edges' turns.
+constexpr int kFinishThreads = 256;
+template <int WPN>
+__global__ void __launch_bounds__(kFinishThreads)
 small_finish_kernel(const float *__restrict__ pos, const float *__restrict__ d, const float *__restrict__ gagg, const float *__restrict__ xl,
                     const float *__restrict__ Wd, const float *__restrict__ s, const int64_t *__restrict__ ptr, const int32_t *__restrict__ nbr,
-                    const int32_t *__restrict__ pair_of, const int32_t *__restrict__ twin, int64_t N, float *__restrict__ grad, float sign,
+                    const int32_t *__restrict__ pair_of, const int32_t *__restrict__ twin, int64_t N, int node_blocks, float *__restrict__ grad, float sign,
                     const float *__restrict__ en, const int64_t *__restrict__ struct_ptr, int64_t B, float *__restrict__ energy) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    // (lists, distances and the first block's rows lie there long before the kernel in front is done)
+    constexpr int kWarps = kFinishThreads / 32, kNodes = kWarps / WPN;
+    __shared__ float s_sum[kWarps][3];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if ((int)blockIdx.x >= node_blocks) {                                // energies, a warp per structure
+        const int64_t b = (int64_t)((int)blockIdx.x - node_blocks) * kWarps + warp;
+        if (b >= B) return;
+        const int64_t n0 = __ldcg(struct_ptr + b), n1 = __ldcg(struct_ptr + b + 1);
+        pdl_wait();
+        float e = 0.f;
+        for (int64_t k = n0 + lane; k < n1; k += 32) e += en[k];
+        e = warp_sum(e);
+        if (lane == 0) energy[b] = e;
+        return;
+    }
+    const int64_t n = (int64_t)blockIdx.x * kNodes + warp / WPN;
+    const bool mine = n < N;
+    // (lists, distances and positions lie there long before the kernel in front is done)
     int64_t k0 = 0, k1 = 0;
-    int32_t first_j = 0, first_p = 0, first_t = 0;
-    float first_d = 0.f;
-    if (grad && warp < N) {
-        k0 = __ldcg(ptr + warp);
-        k1 = __ldcg(ptr + warp + 1);
-        if (k0 + lane < k1) {
-            first_j = __ldcg(nbr + k0 + lane);
-            first_p = __ldcg(pair_of + k0 + lane);
-            if (s) first_t = __ldcg(twin + k0 + lane);
-            first_d = __ldcg(d + k0 + lane);
-        }
+    int32_t my_j = 0, my_p = 0, my_t = 0;
+    float my_d = 0.f, x = 0.f, y = 0.f, z = 0.f;
+    const auto edge = [&](int64_t k) {
+        my_j = __ldcg(nbr + k);
+        my_p = __ldcg(pair_of + k);
+        if (s) my_t = __ldcg(twin + k);
+        my_d = __ldcg(d + k);
+        x = pos[3 * n] - pos[3 * (int64_t)my_j];
+        y = pos[3 * n + 1] - pos[3 * (int64_t)my_j + 1];
+        z = pos[3 * n + 2] - pos[3 * (int64_t)my_j + 2];
+    };
+    if (mine) {
+        const int64_t b0 = __ldcg(ptr + n), b1 = __ldcg(ptr + n + 1), per = (b1 - b0 + WPN - 1) / WPN;
+        k0 = b0 + (warp % WPN) * per;
+        k1 = k0 + per < b1 ? k0 + per : b1;
+        if (k0 + lane < k1) edge(k0 + lane);
     }
     pdl_wait();
-    for (int64_t n = warp; n < N + B; n += nwarps) {
-        if (n >= N) {
-            const int64_t b = n - N;
-            float e = 0.f;
-            for (int64_t k = struct_ptr[b] + lane; k < struct_ptr[b + 1]; k += 32) e += en[k];
-            e = warp_sum(e);
-            if (lane == 0) energy[b] = e;
-            continue;
-        }
-        if (!grad) continue;
-        if (n != warp) { k0 = ptr[n]; k1 = ptr[n + 1]; }
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+    if (k0 < k1) {
         const float4 *g4 = reinterpret_cast<const float4 *>(gagg) + lane, *x4 = reinterpret_cast<const float4 *>(xl) + lane;
         const float4 *Wd4 = reinterpret_cast<const float4 *>(Wd) + lane;
         const float4 gi = g4[n * 32], xi = x4[n * 32];
-        float s0 = 0.f, s1 = 0.f, s2 = 0.f;
         for (int64_t c0 = k0; c0 < k1; c0 += 32) {
             const int len = (int)(k1 - c0 < 32 ? k1 - c0 : 32);
-            int32_t my_j = first_j, my_p = first_p, my_t = first_t;
-            float my_s = 0.f, my_d = first_d;
+            float my_s = 0.f;
             if (lane < len) {
-                if (n != warp || c0 > k0) {
-                    my_j = nbr[c0 + lane];
-                    my_p = pair_of[c0 + lane];
-                    if (s) my_t = twin[c0 + lane];
-                    my_d = d[c0 + lane];
-                }
+                if (c0 > k0) edge(c0 + lane);
                 if (s) my_s = s[c0 + lane] + s[my_t];
             }
             for (int g = 0; g < len; g += 4) {
@@ -695,19 +737,25 @@ small_finish_kernel(const float *__restrict__ pos, const float *__restrict__ d, 
                 v += __shfl_xor_sync(0xffffffffu, v, 2);
                 v += __shfl_xor_sync(0xffffffffu, v, 1);
                 // edge u of the four sits in lanes 8 (2 (u >> 1) + (u & 1)): to the lane that holds the edge
-                const float mine = __shfl_sync(0xffffffffu, v, (lane & 3) * 8);
-                if (lane >= g && lane < g + 4 && lane < len) my_s += mine;
+                const float got = __shfl_sync(0xffffffffu, v, (lane & 3) * 8);
+                if (lane >= g && lane < g + 4 && lane < len) my_s += got;
             }
             if (lane < len) {
                 const float w = my_d > 0.f ? sign * my_s / my_d : 0.f;
-                const int64_t j = my_j;
-                s0 = fmaf(w, pos[3 * n] - pos[3 * j], s0);
-                s1 = fmaf(w, pos[3 * n + 1] - pos[3 * j + 1], s1);
-                s2 = fmaf(w, pos[3 * n + 2] - pos[3 * j + 2], s2);
+                s0 = fmaf(w, x, s0);
+                s1 = fmaf(w, y, s1);
+                s2 = fmaf(w, z, s2);
             }
         }
         s0 = warp_sum(s0); s1 = warp_sum(s1); s2 = warp_sum(s2);
-        if (lane == 0) { grad[n * 3] = s0; grad[n * 3 + 1] = s1; grad[n * 3 + 2] = s2; }
+    }
+    if (lane == 0) { s_sum[warp][0] = s0; s_sum[warp][1] = s1; s_sum[warp][2] = s2; }
+    __syncthreads();
+    if (mine && warp % WPN == 0 && lane < 3) {
+        float v = s_sum[warp][lane];
+#pragma unroll
+        for (int k = 1; k < WPN; k++) v += s_sum[warp + k][lane];
+        grad[n * 3 + lane] = v;
     }
 }
 
@@ -722,6 +770,24 @@ static int small_configure(Kern kern, size_t bytes, bool *done) {
     return MLCGB_OK;
 }
 
+// Rows of a tile.  Fewer rows make a link shorter while the chip has an SM for every tile (one pass), and while it has two, one for the
+// link before, a tile's weights arrive under that link.  Chains of 12 A, three blocks, us an evaluation with tiles of
+//   beads     73 (10 A)   146    200    270    400    560   640 (10 a chain)   800   1000   1400   1700   2000
+//   1 row        46        59     67     73     91
+//   2            48        48     57     61     74     79     89
+//   3            50        50     53     59     65     75     76      90
+//   4            52        53     55     57     65     65     78      94     88    126    133
+//   6            57        59     61     67     72     67     67      81     97    121    124    160
+//   8            62        63     65     71     78     67     69      83     77    130    135    141
+// (9 of 640 beads, 72 tiles: 73; weights of two layers held in registers for one row a tile: 46.3 against 46.2)
+static int small_rows(int64_t N) {
+    constexpr int64_t kHalf = kNumSM / 2;
+    if (N <= 3 * kHalf) return (int)((N + kHalf - 1) / kHalf);
+    if (N <= 4 * kNumSM) return 4;
+    if (N <= 6 * kNumSM) return 6;
+    if (N <= 8 * kNumSM) return 8;
+    return N <= 12 * kNumSM ? 6 : 8;                                   // (two passes)
+}
 template <int KIND, int RT>
 static int small_launch_rt(const SmallNet &p, bool early, cudaStream_t st) {
     static bool done[64] = {false};
@@ -734,7 +800,14 @@ template <int KIND>
 static int small_launch(const SmallNet &p, cudaStream_t st, bool early = true) {
     TimelineScope timeline_scope("small_block", st);
     early = early && g_chain_depth > 0;                                // (weights are read before the wait, as launch_with_weights() has it)
-    return p.N <= 4 * kNumSM ? small_launch_rt<KIND, 4>(p, early, st) : small_launch_rt<KIND, 8>(p, early, st);
+    switch (small_rows(p.N)) {
+        case 0: case 1: return small_launch_rt<KIND, 1>(p, early, st);
+        case 2: return small_launch_rt<KIND, 2>(p, early, st);
+        case 3: return small_launch_rt<KIND, 3>(p, early, st);
+        case 4: return small_launch_rt<KIND, 4>(p, early, st);
+        case 6: return small_launch_rt<KIND, 6>(p, early, st);
+        default: return small_launch_rt<KIND, 8>(p, early, st);
+    }
 }
 
 int small_start(const SmallForward &f, cudaStream_t st) {
@@ -759,7 +832,8 @@ int small_graph_start(const SmallForward &f, const SmallGraph &g, cudaStream_t s
         f.pos, g, f.N, f.B, (float)(g.r * g.r), count_blocks, f.types, f.w->num_types, (const float *)f.w->embedding, (const float *)f.w->blocks[0].lin1_w, f.x[0],
         f.xl[0], f.status);
     if (int rc = check_launch()) return rc;
-    launch_pdl(small_graph_fill_kernel, dim3((unsigned)((f.N + kFillThreads / 32 - 1) / (kFillThreads / 32))), dim3(kFillThreads), 0, st, f.pos, g, f.N, f.B, f.d,
+    const unsigned fill_blocks = (unsigned)((f.N + kFillThreads / 32 - 1) / (kFillThreads / 32)) + (g.pub.host ? 1 : 0);
+    launch_pdl(small_graph_fill_kernel, dim3(fill_blocks), dim3(kFillThreads), 0, st, f.pos, g, f.N, f.B, f.d,
                f.status);
     return check_launch();
 }
@@ -833,9 +907,15 @@ int small_forward(const SmallForward &f, cudaStream_t st) {
 
 int small_finish(const SmallForward &f, const int32_t *twin, const int64_t *struct_ptr, float *energy, float *grad, float sign, cudaStream_t st) {
     TimelineScope timeline_scope("small_finish", st);
-    launch_pdl(small_finish_kernel, dim3(grid_for((f.N + f.B) * 32, 256)), dim3(256), 0, st, f.pos, (const float *)f.d, (const float *)f.gagg[0],
-               (const float *)f.xl[0], (const float *)f.Wd, (const float *)(f.w->num_blocks > 1 ? f.s : nullptr), f.ptr, f.row1, f.pair_of, twin, f.N,
-               f.want_grad ? grad : nullptr, sign, (const float *)f.en, struct_ptr, f.B, energy);
+    const auto go = [&](auto kern, int nodes) {                          // nodes per block
+        const int node_blocks = f.want_grad && grad ? (int)((f.N + nodes - 1) / nodes) : 0;
+        launch_pdl(kern, dim3((unsigned)(node_blocks + (f.B + kFinishThreads / 32 - 1) / (kFinishThreads / 32))), dim3(kFinishThreads), 0, st, f.pos,
+                   (const float *)f.d, (const float *)f.gagg[0], (const float *)f.xl[0], (const float *)f.Wd,
+                   (const float *)(f.w->num_blocks > 1 ? f.s : nullptr), f.ptr, f.row1, f.pair_of, twin, f.N, node_blocks, grad, sign, (const float *)f.en,
+                   struct_ptr, f.B, energy);
+    };
+    if (f.N <= 2 * kNumSM) go(small_finish_kernel<8>, kFinishThreads / 32 / 8);
+    else go(small_finish_kernel<4>, kFinishThreads / 32 / 4);
     return check_launch();
 }
 

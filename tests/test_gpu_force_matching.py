@@ -77,6 +77,13 @@ def test_step_against_float64(kind, R, upper, L, sizes, head, energies):
         assert float((p.grad.cpu().double() - g).abs().max()) <= 2e-5 * float(g.abs().max()) + 1e-9, n
 
 
+@pytest.mark.parametrize("beads", [74, 75, 148, 149, 222, 223, 592, 593, 888, 889, 1184, 1185, 1776, 1777, 2368])
+def test_tiles_of_every_height(beads):
+    """Small batches run in tiles of 1 to 8 rows by their number of beads: both sides of every line, forward and backward."""
+    sizes = [37] * (beads // 37) + [beads % 37] * (beads % 37 > 0)
+    test_step_against_float64("expnormal", 20, 7.0, 2, sizes, 128, True)
+
+
 def test_higher_derivatives_and_position_gradients_take_the_composable_operators():
     net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, [12, 9], 128, 5)
     net = net.to(DEV)
