@@ -4,6 +4,7 @@
 // structure), gradients go out as floating-point atomics.
 #include "common.cuh"
 #include "small_graph.cuh"
+#include "tc_common.cuh"
 
 #include <type_traits>
 
@@ -186,8 +187,8 @@ prior_kernel(const T *__restrict__ pos, const int64_t *__restrict__ mapping, con
 }
 
 // ------------------------------------------------------------------------------------------------
-// All prior classes of a model together, in four launches: a first one that widens the positions to one 16-byte (32-byte) record per
-// bead with its structure and clears the sums, one for the slices of pair lists, one for all other terms, a last one that turns the
+// All prior classes of a model together, in three launches: a first one that widens the positions to one 16-byte (32-byte) record per
+// bead with its structure and clears the sums, one for the slices of pair lists and all other terms, a last one that turns the
 // sums into energies and gradients (or forces) and adds up the lists.  Up to MLCGB_MAX_PRIOR_SEGMENTS lists; every list has its own
 // energy row and gradient block, so the caller still gets one energy / force set per prior, and the totals that SumOut forms
 // (src/mlcg/nn/gradients.py:111-117).  Indices are 32-bit; the structure of a term is that of its first bead.
@@ -196,7 +197,8 @@ prior_kernel(const T *__restrict__ pos, const int64_t *__restrict__ mapping, con
 //   FIXED: energies and gradients are accumulated as 64-bit fixed-point integers (integer addition is associative: the
 //   result does not depend on the order in which the threads arrive) and converted afterwards.
 // ------------------------------------------------------------------------------------------------
-constexpr int kSliceBlocks = 3;             // of prior_slices_kernel, float, each SM
+constexpr int kSliceWarps = 4, kSliceBlocks = 6;         // of prior_all_kernel; blocks each SM, float (5: 146 us, 7: the same with spills)
+template <typename T> constexpr int kSliceStage = sizeof(T) == 4 ? 3072 : 2304;    // bytes of half the steps on their way, each warp (1536: 149 us instead of 141)
 constexpr int kFixedShift = 36;          // fixed point: 2^-36 resolution, +-1.3e8 range
 
 struct PriorSegments {
@@ -278,8 +280,10 @@ __device__ __forceinline__ void run_accumulate(const A &acc, int64_t block0, int
 // 16-bit offset.  Energy and gradient stay in registers: one addition per bead and component, no scatter and no reduction across
 // lanes (the reverse terms of the list carry the other half of every pair's gradient).  In the lists of a topology the lanes of a
 // slice meet the same second bead at nearly the same step: a gather of positions is one or two cache lines.
-// Bound by the stream of terms, 6 bytes each.  One kernel for all lists with a warp per run (32-bit indices, three 4-byte loads a
-// position, a reduction a run) took 390 us for 72 M terms, this 116 us.
+// Bound by instruction issue (29 a term and warp) beside the stream of terms, 6 bytes each: of 134 us for 72 M terms and three lists of
+// single terms, the stream alone takes 75, with its arithmetic 95, the single terms 20 more, the first and the last launch 20.  With loads
+// two steps ahead in registers 155; with a warp per run in one kernel for all lists (32-bit indices, three 4-byte loads a position, a
+// reduction a run) the pair terms alone took 390.
 __device__ __forceinline__ float inv_sqrt(float x) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -287,26 +291,31 @@ __device__ __forceinline__ float inv_sqrt(float x) {
 }
 __device__ __forceinline__ double inv_sqrt(double x) { return rsqrt(x); }
 
-template <int KIND, typename T> struct PairStep {
-    uint2 j;
-    typename Vec4<T>::type a, b;
-    __device__ __forceinline__ void load(const uint2 *off, const T *pa, int64_t stride, int64_t at) {
-        using V = typename Vec4<T>::type;
-        j = __ldg(off + at);
-        a = *((const V *)pa + at);
-        if constexpr (KIND == 0) b = *((const V *)(pa + stride) + at);
-    }
+// A warp's steps on their way from memory: two stages of a few steps each, filled by the copy engine (steps lie one behind the other, so
+// a stage is one copy of offsets and one of each parameter), which takes neither issue slots nor the registers that loads ahead did.
+template <int KIND, typename T> struct PairStages {
+    using V = typename Vec4<T>::type;
+    static constexpr int kParams = KIND == 0 ? 2 : 1, kPar = 32 * (int)sizeof(V), kStep = 256 + kParams * kPar;
+    static constexpr int kSteps = kSliceStage<T> / kStep >= 4 ? 4 : kSliceStage<T> / kStep >= 2 ? 2 : 1, kBytes = kSteps * kStep;
+    static_assert(kBytes <= kSliceStage<T>, "half of a warp's part of the shared memory");
 };
+
+// b - a; the first two components in one instruction (141 -> 134 us for 72 M terms)
+__device__ __forceinline__ V3<float> difference(const float4 &b, const float4 &a) {
+    const float2 xy = tc::sub2(make_float2(b.x, b.y), make_float2(a.x, a.y));
+    return V3<float>{xy.x, xy.y, b.z - a.z};
+}
+__device__ __forceinline__ V3<double> difference(const double4 &b, const double4 &a) { return V3<double>{b.x - a.x, b.y - a.y, b.z - a.z}; }
 
 template <int KIND, typename T, typename A, typename Bead>
 __device__ __forceinline__ void prior_slices(const A &acc, const PriorSegments &seg, int s, int parts, const Bead *__restrict__ beads, int64_t N,
-                                             int64_t B, int32_t *status) {
+                                             int64_t B, int32_t *status, int block, int blocks, char *ring, uint32_t bars, int &turn, bool &failed) {
     const int lane = threadIdx.x & 31;
     const int64_t units = (int64_t)seg.n_slices[s] * parts;
     const int64_t steps = seg.steps[s], stride = steps * 128;
     const auto *off = (const uint2 *)seg.offsets[s];
     const T *pa = (const T *)seg.slice_params[s];
-    for (int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < units; w += (int64_t)gridDim.x * (blockDim.x >> 5)) {
+    for (int64_t w = (int64_t)block * kSliceWarps + (threadIdx.x >> 5); w < units; w += (int64_t)blocks * kSliceWarps) {
         const int slice = (int)(w / parts), part = (int)(w % parts);
         const int4 h = __ldg(seg.slices[s] + slice);             // {first step, steps, base, span}
         const int first = __ldg(seg.slice_beads[s] + (int64_t)slice * 32 + lane), c0 = first < 0 ? ~first : first;    // (~bead: an idle lane)
@@ -317,46 +326,83 @@ __device__ __forceinline__ void prior_slices(const A &acc, const PriorSegments &
         }
         const Bead b0 = beads[c0];
         const Bead *other = beads + h.z;
-        const V3<T> p0 = xyz<T>(b0);
-        int g = (int)((int64_t)h.y * part / parts);
-        const int g1 = (int)((int64_t)h.y * (part + 1) / parts);
-        if (g >= g1) continue;
+        using S = PairStages<KIND, T>;
+        using V = typename S::V;
+        // (a unit takes every `parts`-th stage: neighbouring warps read neighbouring memory)
+        const int all = (h.y + S::kSteps - 1) / S::kSteps, stages = (all - part + parts - 1) / parts;
+        if (part >= all) continue;
         T es = T(0);
+        float2 es2 = make_float2(0.f, 0.f);
         V3<T> gs{T(0), T(0), T(0)};
-        int64_t at = ((int64_t)h.x + g) * 32 + lane;
-        const auto step = [&](const PairStep<KIND, T> &now) {
-            const Bead bj[4] = {other[now.j.x & 0xffffu], other[now.j.x >> 16], other[now.j.y & 0xffffu], other[now.j.y >> 16]};
-            const T pa4[4] = {now.a.x, now.a.y, now.a.z, now.a.w};
+        const auto step = [&](const uint2 j, const auto &a, const auto &b) {
+            const Bead bj[4] = {other[j.x & 0xffffu], other[j.x >> 16], other[j.y & 0xffffu], other[j.y >> 16]};
+            const T pa4[4] = {a.x, a.y, a.z, a.w}, pb4[4] = {b.x, b.y, b.z, b.w};
+            V3<T> dr[4];
+            T inv_d[4], d2[4], f[4];                              // f: dE/dd / d; of a repulsion without its factor -6
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const V3<T> dr = sub(xyz<T>(bj[u]), p0);
-                const T d2 = dot(dr, dr), inv_d = inv_sqrt(d2);
-                T f;                                              // dE/dd / d; of a repulsion without its factor -6
-                if constexpr (KIND == 0) {
-                    const T k = u == 0 ? now.b.x : u == 1 ? now.b.y : u == 2 ? now.b.z : now.b.w, x = d2 * inv_d - pa4[u];
-                    es += k * x * x;
-                    f = T(2) * k * x * inv_d;
-                } else {
-                    const T q = pa4[u] * inv_d, rr = q * q, ee = rr * rr * rr;
-                    es += ee;
-                    f = ee * inv_d * inv_d;
-                }
-                gs.x += dr.x * f; gs.y += dr.y * f; gs.z += dr.z * f;
+                dr[u] = difference(bj[u], b0);
+                d2[u] = dot(dr[u], dr[u]);
+                inv_d[u] = inv_sqrt(d2[u]);
             }
+            if constexpr (KIND == 3 && sizeof(T) == 4) {          // two terms an instruction
+#pragma unroll
+                for (int u = 0; u < 4; u += 2) {
+                    const float2 inv = make_float2(inv_d[u], inv_d[u + 1]), q = tc::mul2(make_float2(pa4[u], pa4[u + 1]), inv), rr = tc::mul2(q, q),
+                                 ee = tc::mul2(tc::mul2(rr, rr), rr), ff = tc::mul2(tc::mul2(ee, inv), inv);
+                    es2 = tc::add2(es2, ee);
+                    f[u] = ff.x;
+                    f[u + 1] = ff.y;
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if constexpr (KIND == 0) {
+                        const T k = pb4[u], x = d2[u] * inv_d[u] - pa4[u];
+                        es += k * x * x;
+                        f[u] = T(2) * k * x * inv_d[u];
+                    } else {
+                        const T q = pa4[u] * inv_d[u], rr = q * q, ee = rr * rr * rr;
+                        es += ee;
+                        f[u] = ee * inv_d[u] * inv_d[u];
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) { gs.x += dr[u].x * f[u]; gs.y += dr[u].y * f[u]; gs.z += dr[u].z * f[u]; }
         };
-        // two steps ahead
-        PairStep<KIND, T> even, odd;
-        even.load(off, pa, stride, at);
-        if (g + 1 < g1) odd.load(off, pa, stride, at + 32);
-        for (; g < g1; g += 2, at += 64) {
-            PairStep<KIND, T> now = even;
-            if (g + 2 < g1) even.load(off, pa, stride, at + 64);
-            step(now);
-            if (g + 1 >= g1) break;
-            now = odd;
-            if (g + 3 < g1) odd.load(off, pa, stride, at + 96);
-            step(now);
+        const auto fetch = [&](int k) {                          // stage k of this unit, into half (turn + k) & 1
+            if (lane != 0 || k >= stages) return;
+            const int half = (turn + k) & 1, first_step = (part + k * parts) * S::kSteps, m = h.y - first_step < S::kSteps ? h.y - first_step : S::kSteps;
+            const uint32_t to = tc::smem_u32(ring + half * kSliceStage<T>), bar = bars + 8 * half;
+            const int64_t from = ((int64_t)h.x + first_step) * 32;
+            tc::mbar_expect_bytes(bar, (uint32_t)(m * S::kStep));
+            tc::bulk_load(to, off + from, (uint32_t)(m * 256), bar);
+#pragma unroll
+            for (int q = 0; q < S::kParams; q++)
+                tc::bulk_load(to + S::kSteps * (256 + q * S::kPar), (const V *)(pa + q * stride) + from, (uint32_t)(m * S::kPar), bar);
+        };
+        fetch(0);
+        fetch(1);
+        for (int k = 0; k < stages; k++) {
+            const int half = (turn + k) & 1, m = h.y - (part + k * parts) * S::kSteps;
+            if (!failed && !tc::mbar_wait(bars + 8 * half, (uint32_t)(turn + k) >> 1 & 1u)) failed = true;
+            const char *in = ring + half * kSliceStage<T>;
+            const auto steps = [&](int u) {
+                const V *par = reinterpret_cast<const V *>(in + S::kSteps * 256) + u * 32 + lane;
+                step(reinterpret_cast<const uint2 *>(in)[u * 32 + lane], par[0], par[KIND == 0 ? S::kSteps * 32 : 0]);
+            };
+            if (m >= S::kSteps) {
+#pragma unroll
+                for (int u = 0; u < S::kSteps; u++) steps(u);
+            } else {
+                for (int u = 0; u < m; u++) steps(u);
+            }
+            __syncwarp();
+            fetch(k + 2);
         }
+        turn += stages;
+        if constexpr (KIND == 3 && sizeof(T) == 4) es = es2.x + es2.y;
         const int mb = structure_of(b0);
         const bool mine = first >= 0 && mb >= 0;
         if (first >= 0 && mb < 0) atomicOr(status, (int)kBadIndex);
@@ -369,23 +415,6 @@ __device__ __forceinline__ void prior_slices(const A &acc, const PriorSegments &
             acc.energy((int64_t)s * B + mb, es);
         }
     }
-}
-
-template <typename T, bool FIXED>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? kSliceBlocks : 2)
-prior_slices_kernel(const __grid_constant__ PriorSegments seg, int parts, const typename Vec4<T>::type *__restrict__ beads, int64_t N, int64_t B,
-                    typename Accum<T, FIXED>::type *__restrict__ energy, typename Accum<T, FIXED>::type *__restrict__ grad,
-                    int32_t *__restrict__ status, int beside_terms) {
-    const Accum<T, FIXED> acc{energy, grad};
-    // beside_terms: the kernel before this one is prior_terms_kernel, which lets it start once the beads and the sums are there (its
-    // own wait is over): the two run side by side, and this one ends after that one
-    if (!beside_terms) pdl_wait();
-    for (int s = 0; s < seg.n; s++) {
-        if (seg.n_slices[s] == 0) continue;
-        if (seg.kind[s] == 0) prior_slices<0, T>(acc, seg, s, parts, beads, N, B, status);
-        else prior_slices<3, T>(acc, seg, s, parts, beads, N, B, status);
-    }
-    if (beside_terms) pdl_wait();
 }
 
 // ---- what is made of a list on its first evaluation: 32-bit indices, the parameters of its terms from the tables of bead types, whether
@@ -658,17 +687,13 @@ pair_slices_pack_kernel(const int32_t *__restrict__ idx, const T *__restrict__ p
 // of their double-precision chains and by the scattered additions.  Terms of a chain that follow one another in the list share beads
 // with their neighbours: a lane hands what it has for the beads that the next lane's term starts with over to that lane, so that a
 // torsion adds to one bead instead of four (47 -> 33 us for the three lists of 1024 chains of 268 beads, the shorter torsion included).
-template <typename T, bool FIXED>
-__global__ void __launch_bounds__(256)
-prior_terms_kernel(const __grid_constant__ PriorSegments seg, const typename Vec4<T>::type *__restrict__ beads, int64_t N, int64_t B,
-                   typename Accum<T, FIXED>::type *__restrict__ energy, typename Accum<T, FIXED>::type *__restrict__ grad, int32_t *__restrict__ status) {
+template <typename T, typename A>
+__device__ __forceinline__ void prior_terms(const A &acc, const PriorSegments &seg, const typename Vec4<T>::type *__restrict__ beads, int64_t N, int64_t B,
+                                            int32_t *status, int block, int blocks) {
     const int lane = threadIdx.x & 31;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t stride = (int64_t)blocks * blockDim.x;
     const int64_t vtotal = seg.vstart[seg.n];
-    Accum<T, FIXED> acc{energy, grad};
-    pdl_wait();
-    pdl_launch_dependents();
-    for (int64_t vbase = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; vbase < vtotal; vbase += stride) {
+    for (int64_t vbase = (int64_t)block * blockDim.x + threadIdx.x - lane; vbase < vtotal; vbase += stride) {
         int s = 0;
         while (s + 1 < seg.n && vbase >= seg.vstart[s + 1]) s++;               // warp-uniform: lists start on warp boundaries
         const int kind = seg.kind[s];
@@ -760,6 +785,43 @@ prior_terms_kernel(const __grid_constant__ PriorSegments seg, const typename Vec
             acc.energy(e_row + mb, e);
         }
     }
+}
+
+// All terms: blocks of slices and blocks of single terms, dealt evenly, so that every SM holds both: the slices use the issue slots that the
+// chains of double-precision operations leave.  In launches of their own the two hardly met (a launch starts when the last block of the
+// one before has, whatever the former allows): 143.5 us for the lists of 1024 chains of 268 beads, like this 141.
+template <typename T, bool FIXED>
+__global__ void __launch_bounds__(kSliceWarps * 32, sizeof(T) == 4 ? kSliceBlocks : 4)
+prior_all_kernel(const __grid_constant__ PriorSegments seg, int parts, int term_blocks, const typename Vec4<T>::type *__restrict__ beads, int64_t N, int64_t B,
+                 typename Accum<T, FIXED>::type *__restrict__ energy, typename Accum<T, FIXED>::type *__restrict__ grad, int32_t *__restrict__ status) {
+    __shared__ __align__(128) char s_ring[kSliceWarps][2 * kSliceStage<T>];
+    __shared__ uint64_t s_bar[kSliceWarps][2];
+    const Accum<T, FIXED> acc{energy, grad};
+    // term blocks before this one, and whether this is one
+    const int before = (int)((int64_t)blockIdx.x * term_blocks / gridDim.x), upto = (int)(((int64_t)blockIdx.x + 1) * term_blocks / gridDim.x);
+    if (upto > before) {
+        pdl_wait();
+        prior_terms<T>(acc, seg, beads, N, B, status, before, term_blocks);
+        return;
+    }
+    char *const ring = s_ring[threadIdx.x >> 5];
+    const uint32_t bars = tc::smem_u32(s_bar[threadIdx.x >> 5]);      // this warp's stages have arrived
+    if ((threadIdx.x & 31) == 0) {
+        tc::mbar_init(bars, 1);
+        tc::mbar_init(bars + 8, 1);
+        tc::fence_async_smem();
+    }
+    __syncwarp();
+    int turn = 0;                                                     // stages this warp has used
+    bool failed = false;
+    pdl_wait();
+    const int block = (int)blockIdx.x - before, blocks = (int)gridDim.x - term_blocks;
+    for (int s = 0; s < seg.n; s++) {
+        if (seg.n_slices[s] == 0) continue;
+        if (seg.kind[s] == 0) prior_slices<0, T>(acc, seg, s, parts, beads, N, B, status, block, blocks, ring, bars, turn, failed);
+        else prior_slices<3, T>(acc, seg, s, parts, beads, N, B, status, block, blocks, ring, bars, turn, failed);
+    }
+    if (failed) atomicOr(status, (int)kTensorWait);
 }
 
 template <typename T, typename A> __device__ __forceinline__ T sum_value(A v) {
@@ -970,13 +1032,12 @@ extern "C" int mlcgb_prior_eval(int n_lists, const mlcgb_prior_list *lists, cons
         auto *sums = (A *)((char *)workspace + prior_bead_bytes(N, dtype));
         A *se = sums, *sg = sums + (int64_t)n_lists * B;
         prior_begin_kernel<T, A><<<grid_for(N > n_sums / 4 ? N : n_sums / 4, 256, 8), 256, 0, st>>>((const T *)pos, batch, N, B, beads, sums, n_sums);
-        if (v) launch_pdl(prior_terms_kernel<T, FIXED>, dim3(grid_for(v, 256, 16)), dim3(256), 0, st, seg, beads, N, B, se, sg, status);
-        if (r) {
-            // a slice is cut into parts until the chip holds a few rounds of warps (48 each SM); sixteen parts of a step or two at most
-            const int64_t want = (2 * 48 * (int64_t)kNumSM + r - 1) / r;
-            const int parts = (int)(want > 16 ? 16 : want);
-            launch_pdl(prior_slices_kernel<T, FIXED>, dim3(grid_for(r * parts, 8, 48)), dim3(256), 0, st, seg, parts, beads, N, B, se, sg, status, v ? 1 : 0);
-        }
+        // a slice is cut into parts until the chip holds a few rounds of warps (48 each SM); sixteen parts of a step or two at most
+        const int64_t want = r ? (2 * 48 * (int64_t)kNumSM + r - 1) / r : 1;
+        const int parts = (int)(want > 16 ? 16 : want), slice_blocks = r ? grid_for(r * parts, kSliceWarps, 96) : 0,
+                  term_blocks = v ? grid_for(v, kSliceWarps * 32, 96) : 0;
+        if (slice_blocks + term_blocks)
+            launch_pdl(prior_all_kernel<T, FIXED>, dim3(slice_blocks + term_blocks), dim3(kSliceWarps * 32), 0, st, seg, parts, term_blocks, beads, N, B, se, sg, status);
         launch_pdl(prior_finish_kernel<T, A>, dim3(grid_for(B + 3 * N, 256, 8)), dim3(256), 0, st, sums, n_lists, N, B, (T)(negate ? -1 : 1), (T *)energy,
                    (T *)grad, (T *)total_energy, (T *)total_grad);
         return check_launch();

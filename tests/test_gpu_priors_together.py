@@ -3,6 +3,7 @@ float64 autograd over the differentiable terms."""
 import pytest
 import torch
 
+import mlcg_b200
 from helpers import prior_setup, random_walk_chain
 from mlcg_b200 import nn as bnn
 from mlcg_b200.nn.prior import _evaluate_together, _pair_slices
@@ -40,6 +41,36 @@ def test_forces_and_totals(n, B, dtype):
             e_sum, f_sum = e_sum + want.detach(), f_sum + f
         assert torch.allclose(energy.double(), e_sum, rtol=tol, atol=tol)
         assert float((forces.double() - f_sum).abs().max()) <= tol * (1 + float(f_sum.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("n,B", [(20, 3), (21, 40), (24, 2), (25, 1), (32, 5), (33, 70), (34, 3), (57, 4), (66, 2), (129, 1), (321, 3)])
+def test_slices_at_the_ends_of_stages(n, B, dtype):
+    """Sliced lists of bonds and of repulsion, every pair of a structure both ways: runs of n - 1 terms that end inside, at and behind a
+    stage of the copies, cut into parts that get no stage, one, or many."""
+    gen = torch.Generator().manual_seed(n)
+    every = torch.cartesian_prod(torch.arange(n), torch.arange(n)).t()
+    every = every[:, every[0] != every[1]]
+    mapping = torch.cat([every + k * n for k in range(B)], dim=1)
+    owner = torch.arange(B).repeat_interleave(every.shape[1])
+    priors = {"bonds": bnn.HarmonicBonds({(0, 0): {"k": 0.3, "x_0": 9.0}}), "repulsion": bnn.Repulsion({(0, 0): {"sigma": 3.5}})}
+    lists = {k: mlcg_b200.make_neighbor_list(k, 2, mapping, owner) for k in priors}
+    data = mlcg_b200.AtomicData(pos=torch.cat([random_walk_chain(n, gen, min_dist=3.0) for _ in range(B)]).to(dtype), atom_types=torch.zeros(n * B, dtype=torch.long),
+                                batch=torch.arange(B).repeat_interleave(n), n_atoms=torch.full((B,), n), neighbor_list=lists).to(DEV)
+    priors = {k: p.to(DEV).eval() for k, p in priors.items()}
+    assert all(p._cached_list(data)[4] is not None for p in priors.values())
+    each = _evaluate_together(list(priors.values()), data, forces=True)[0]
+    again = _evaluate_together(list(priors.values()), data, forces=True)[0]
+    pos = data.pos.double().requires_grad_(True)
+    # (float32: sums of n terms of the roundings that one term has, as above)
+    tol = 1e-5 if dtype == torch.float32 else 1e-9
+    for k, p in priors.items():
+        y = p._energy_terms(pos, lists[k]["index_mapping"].to(DEV), p._params(data).double())
+        want = torch.zeros(B, dtype=torch.float64, device=DEV).index_add_(0, owner.to(DEV), y)
+        f = -torch.autograd.grad(want.sum(), pos)[0]
+        assert torch.allclose(each[k][0].double(), want.detach(), rtol=tol, atol=tol), k
+        assert float((each[k][1].double() - f).abs().max()) <= tol * (1 + float(f.abs().max())), k
+        assert torch.equal(each[k][0], again[k][0]) and torch.equal(each[k][1], again[k][1]), k
 
 
 def test_a_sliced_list_is_kept_once():
