@@ -45,7 +45,7 @@ struct FilterVdParams {
 constexpr int kRowSlots = 6, kRowBytes = kRowSlots * 4096;
 template <bool SPLIT> constexpr int kVdSmem = FilterSmem<SPLIT>::kExtra + kRowBytes + (SPLIT ? 0 : 32768) + 1024;
 
-template <bool SPLIT>
+template <bool SPLIT, bool APART>
 __global__ void __launch_bounds__(kTcThreads + 32, 1)
 filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap dmap) {
     using namespace tc;
@@ -54,8 +54,11 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
     p.A1 = q.blk[blockIdx.y].A1;
     p.b1 = q.blk[blockIdx.y].b1;
     p.A2 = q.blk[blockIdx.y].A2;
-    float4 *const h_keep = p.H ? reinterpret_cast<float4 *>(p.H + blockIdx.y * q.block_hidden) : nullptr;
-    float4 *const z_keep = q.Zd ? reinterpret_cast<float4 *>(q.Zd + blockIdx.y * q.block_hidden) : nullptr;
+    // APART: a launch with few tiles gives each to two CTAs (blockIdx.z), one for the values and one for the derivatives, the first steps
+    // done in both: a chain of two GEMMs each instead of four in turn.
+    const bool values = !APART || blockIdx.z == 0, derivatives = !APART || blockIdx.z == 1;
+    float4 *const h_keep = p.H && values ? reinterpret_cast<float4 *>(p.H + blockIdx.y * q.block_hidden) : nullptr;
+    float4 *const z_keep = q.Zd && derivatives ? reinterpret_cast<float4 *>(q.Zd + blockIdx.y * q.block_hidden) : nullptr;
     const int row_base = (int)(blockIdx.y * q.block_rows);
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -167,7 +170,8 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
         for (int64_t j = 0; j < n_local; j++) {
             const uint32_t par = (uint32_t)(j & 1);
             quarters = next;
-            gemm(r2v, par, tA, tV, b2_hi, b2_lo, kF / 16, c2v);
+            if (values) gemm(r2v, par, tA, tV, b2_hi, b2_lo, kF / 16, c2v);
+            if (!derivatives) break;                   // (a tile of its own)
             await(r1d, par);
             gemm1(tR, tQ, quarters, c1d);
             if (j + 1 < n_local) {
@@ -284,7 +288,8 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
         };
         // accumulator x (this row's factor) -> stage -> rows of the mapped matrix, by the copy engine.  A warp stages and stores its own box of
         // 32 rows x 32 columns: no warp waits for another one here (one box of 128 rows for the block took two block-wide barriers)
-        auto store_rows = [&](const CUtensorMap *map, int64_t tile, uint32_t acc, float f) {
+        // (a tile of its own: by the lanes of the warp, which need not stay until the copy engine is done, nor the host describe the matrix)
+        auto store_rows = [&](const CUtensorMap *map, float *plain, int64_t tile, uint32_t acc, float f) {
             float v[32];
             tmem_ld32(acc + col0, v);
             if (lane == 0) bulk_wait_read<0>();                     // the copy before has read the stage
@@ -294,9 +299,19 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
                 const float2 lo = mul2(make_float2(v[4 * w], v[4 * w + 1]), both(f)), hi = mul2(make_float2(v[4 * w + 2], v[4 * w + 3]), both(f));
                 *box_chunk(stage, qt, r, w) = make_float4(lo.x, lo.y, hi.x, hi.y);
             }
+            const int64_t row = tile * kRows + 32 * (warp & 3);
+            if (APART) {
+                __syncwarp();
+                float4 *const to = reinterpret_cast<float4 *>(plain + (row_base + row) * kF + col0) + (lane & 7);
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const int k = 4 * i + (lane >> 3);
+                    if (row + k < nE) to[k * (kF / 4)] = *box_chunk(stage, qt, 32 * (warp & 3) + k, lane & 7);
+                }
+                return;
+            }
             fence_async_smem();
             __syncwarp();
-            const int64_t row = tile * kRows + 32 * (warp & 3);
             if (lane == 0 && row < nE) {
                 tensor_store_box(map, col0, row_base + (int)row, stage + qt * 16384 + (warp & 3) * 4096);
                 bulk_commit();
@@ -314,6 +329,10 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
             row_group_sync();
             live_next = basis(read_scalars(0), tV, 0, first);
             signal(r1v);
+            if (APART && derivatives) {
+                basis_derivative(read_scalars(0), live_next);
+                signal(r1d);
+            }
         }
         int64_t tile = first;
         for (int64_t n = 0; n < n_local; n++, tile += step) {
@@ -337,20 +356,25 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
                 }
                 tmem_wait_st();
             }
-            signal(r2v);
+            if (values) signal(r2v);
             if (n > 0) {
                 await(c2d, par ^ 1);
-                store_rows(&dmap, tile - step, tR, f_prev);
+                store_rows(&dmap, q.Wd, tile - step, tR, f_prev);
             }
             const Scalars sc = read_scalars(n);
-            basis_derivative(sc, live);
-            signal(r1d);
+            if (!APART) {
+                basis_derivative(sc, live);
+                signal(r1d);
+            }
             if ((n & 3) == 2 && n + 2 < n_local) {
                 prepare(n + 2, d_ahead);
                 edge_ahead = fetch_edge(n + 6);
             }
-            await(c2v, par);
-            store_rows(&wmap, tile, tA, sc.c0 * unscale);
+            if (values) {
+                await(c2v, par);
+                store_rows(&wmap, p.W, tile, tA, sc.c0 * unscale);
+                if (!derivatives) break;
+            }
             if (n + 1 < n_local) {
                 // (the next tile's operand overwrites the accumulator just read: by all four quarters of the row)
                 tc_fence_before();
@@ -422,9 +446,9 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
             tA = tQ;
             tQ = old;
         }
-        if (n_local > 0) {
+        if (n_local > 0 && derivatives) {
             await(c2d, (uint32_t)((n_local - 1) & 1));
-            store_rows(&dmap, tile - step, tR, f_prev);
+            store_rows(&dmap, q.Wd, tile - step, tR, f_prev);
         }
         if (z_keep) {
 #pragma unroll
@@ -441,22 +465,25 @@ filter_vd_kernel(FilterVdParams q, const __grid_constant__ CUtensorMap wmap, con
     if (warp == 0) tmem_free(tmem, 512);
 }
 
-template <bool SPLIT>
-static int filter_vd_launch(const FilterVdParams &q, int64_t num_blocks, cudaStream_t st) {
-    using L = FilterSmem<SPLIT>;
+template <bool SPLIT, bool APART>
+static int filter_vd_launch(const FilterVdParams &q, int64_t ntiles, int64_t num_blocks, cudaStream_t st) {
     static bool configured[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-        if (cudaFuncSetAttribute(filter_vd_kernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kVdSmem<SPLIT>) != cudaSuccess) return check_launch();
+        if (cudaFuncSetAttribute(filter_vd_kernel<SPLIT, APART>, cudaFuncAttributeMaxDynamicSharedMemorySize, kVdSmem<SPLIT>) != cudaSuccess) return check_launch();
         configured[dev] = true;
     }
-    CUtensorMap wmap, dmap;
+    CUtensorMap wmap = {}, dmap = {};
     const int64_t rows = (num_blocks - 1) * q.block_rows + q.f.E;
-    if (!make_rows_map(&wmap, q.f.W, rows, kF, 32) || !make_rows_map(&dmap, q.Wd, rows, kF, 32)) return MLCGB_E_LIMIT;
-    const int64_t ntiles = (q.f.E + tc::kRows - 1) / tc::kRows, per_block = num_blocks < kNumSM ? kNumSM / num_blocks : 1;
+    if (APART) {
+        if (((uintptr_t)q.f.W | (uintptr_t)q.Wd) % 16) return MLCGB_E_LIMIT;
+    } else if (!make_rows_map(&wmap, q.f.W, rows, kF, 32) || !make_rows_map(&dmap, q.Wd, rows, kF, 32)) {
+        return MLCGB_E_LIMIT;
+    }
+    const int64_t per_block = num_blocks < kNumSM ? kNumSM / num_blocks : 1;
     const int grid = (int)(ntiles < per_block ? ntiles : per_block);
-    launch_with_weights(filter_vd_kernel<SPLIT>, dim3(grid, (unsigned)num_blocks), dim3(kTcThreads + 32), kVdSmem<SPLIT>, st, q, wmap, dmap);
+    launch_with_weights(filter_vd_kernel<SPLIT, APART>, dim3(grid, (unsigned)num_blocks, APART ? 2 : 1), dim3(kTcThreads + 32), kVdSmem<SPLIT>, st, q, wmap, dmap);
     return check_launch();
 }
 
@@ -494,7 +521,11 @@ int filter_vd_blocks(const float *d, int64_t P, const int64_t *rows_dev, const i
     q.Zd = zs;
     q.zmax = zmax;
     q.images = images;
-    return precision == 0 ? filter_vd_launch<true>(q, num_blocks, st) : filter_vd_launch<false>(q, num_blocks, st);
+    // two CTAs a tile while the chip holds them all (64 x 10 beads, two blocks: 51.9 -> 50.5 us an evaluation, 52.3 -> 50.3 replayed)
+    const int64_t ntiles = (P + tc::kRows - 1) / tc::kRows;
+    if (2 * ntiles * num_blocks <= kNumSM)
+        return precision == 0 ? filter_vd_launch<true, true>(q, ntiles, num_blocks, st) : filter_vd_launch<false, true>(q, ntiles, num_blocks, st);
+    return precision == 0 ? filter_vd_launch<true, false>(q, ntiles, num_blocks, st) : filter_vd_launch<false, false>(q, ntiles, num_blocks, st);
 }
 
 }  // namespace mlcgb
