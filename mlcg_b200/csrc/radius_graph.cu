@@ -2715,7 +2715,6 @@ mask_rows_fill_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr
                       const int64_t *__restrict__ offsets, FillOut out, int32_t *__restrict__ twin, int32_t *__restrict__ sel,
                       int32_t *__restrict__ pair_of) {
     const int lane = threadIdx.x & 31;
-    const unsigned lt = lanemask_lt();
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < N; i += ((int64_t)gridDim.x * blockDim.x) >> 5) {
         const int b = struct_of[i];
         if (cellparam && cellparam[b].tile != 2) continue;
@@ -2723,17 +2722,12 @@ mask_rows_fill_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr
         const int n = (int)((ptr[b + 1] < N ? ptr[b + 1] : N) - lo), il = (int)(i - lo), nw = (n + 31) >> 5, kept = (int)(offsets[i + 1] - off);
         if (kept == 0) continue;
         const int4 si = seg[i];
-        const uint2 mine = lane < nw ? masks[i * kMaskWords + lane] : make_uint2(0u, 0u);
-        for (unsigned words = __ballot_sync(0xffffffffu, mine.y != 0u); words; words &= words - 1) {
-            const int w = __ffs(words) - 1;
-            const unsigned bits = __shfl_sync(0xffffffffu, mine.y, w);
-            const int rank = (int)__shfl_sync(0xffffffffu, mine.x, w) + __popc(bits & lt);
-            if (!(bits >> lane & 1u) || rank >= kept) continue;
-            const int64_t slot = off + rank, j = lo + w * 32 + lane;
+        each_hit(masks + i * kMaskWords, nw, kept, lane, [&](int rank, int jl) {
+            const int64_t slot = off + rank, j = lo + jl;
             T d2 = T(0);
             if (out.distance) d2 = dist2_rn(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], pos[3 * j], pos[3 * j + 1], pos[3 * j + 2]);
             emit_edge<T>(out, slot, i, j, b, d2);
-            if (!twin) continue;
+            if (!twin) return;
             // (a complete list: the reverse is there)
             const uint2 rev = masks[j * kMaskWords + (il >> 5)];
             const int rank_j = (int)rev.x + __popc(rev.y & ((1u << (il & 31)) - 1u));
@@ -2747,7 +2741,7 @@ mask_rows_fill_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr
             }
             twin[slot] = sj.x + rank_j;
             pair_of[slot] = p;
-        }
+        });
     }
 }
 

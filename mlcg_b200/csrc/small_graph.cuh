@@ -124,17 +124,41 @@ __device__ __forceinline__ RowHits row_of_bits(const T *__restrict__ pos, int64_
     const int nlo = sw < 32 ? __shfl_sync(0xffffffffu, nlo0, sw) : __shfl_sync(0xffffffffu, nlo1, sw & 31);
     return {total, nlo, self_hit};
 }
-// f(rank, local index) for the first `kept` hits of a row of nw words, lane by lane
+// The k-th set bit of a word that has more than k
+__device__ __forceinline__ int nth_bit(unsigned bits, int k) {
+    int at = 0;
+#pragma unroll
+    for (int half = 16; half; half >>= 1) {
+        const int c = __popc(bits & ((1u << half) - 1u));
+        const bool up = k >= c;
+        k -= up ? c : 0;
+        at += up ? half : 0;
+        bits >>= up ? half : 0;
+    }
+    return at;
+}
+// f(rank, local index) for the first `kept` hits of a row of nw words, 32 consecutive ranks at a time: a lane looks for the word of its rank
+// among the 32 of the warp, and for the bit in it.  (Word by word, the lanes of the word's bits at work, a row took as many turns as it
+// has words with a hit, most lanes idle: 37 structures of up to 700 points in float64 with distances 99 -> 81 us.)
 template <typename F>
 __device__ __forceinline__ void each_hit(const uint2 *__restrict__ row, int nw, int kept, int lane, F &&f) {
-    const unsigned lt = lanemask_lt();
     for (int w0 = 0; w0 < nw; w0 += 32) {
-        const uint2 mine = w0 + lane < nw ? row[w0 + lane] : make_uint2(0u, 0u);
-        for (unsigned live = __ballot_sync(0xffffffffu, mine.y != 0u); live; live &= live - 1) {
-            const int w = __ffs(live) - 1;
+        const bool there = w0 + lane < nw;
+        const uint2 mine = there ? row[w0 + lane] : make_uint2(0u, 0u);
+        const int first = (int)__shfl_sync(0xffffffffu, mine.x, 0), last = min(nw - w0, 32) - 1;
+        const int before = there ? (int)mine.x : 0x7fffffff;
+        const int end = min(kept, (int)__shfl_sync(0xffffffffu, mine.x + (unsigned)__popc(mine.y), last));
+        for (int k = first; k < end; k += 32) {
+            const int rank = k + lane;
+            int w = 0;                             // the last word with no more hits before it than the rank
+#pragma unroll
+            for (int step = 16; step; step >>= 1) {
+                const int b = __shfl_sync(0xffffffffu, before, w + step);
+                if (b <= rank) w += step;
+            }
             const unsigned bits = __shfl_sync(0xffffffffu, mine.y, w);
-            const int rank = (int)__shfl_sync(0xffffffffu, mine.x, w) + __popc(bits & lt);
-            if ((bits >> lane & 1u) && rank < kept) f(rank, (w0 + w) * 32 + lane);
+            const int b = __shfl_sync(0xffffffffu, before, w);
+            if (rank < end) f(rank, (w0 + w) * 32 + nth_bit(bits, rank - b));
         }
     }
 }
