@@ -383,42 +383,52 @@ gemm_tc_rows_pipe_kernel(const float *__restrict__ A, const float *__restrict__ 
 // first layer or the output network's, in front of the backward ones the transpose of the same; its result, the gradient of the block's
 // output, then leaves on the way.  There is no room for three weights: the first and the third take turns in one place, each fetched by
 // bulk copy as soon as the other's GEMM is over.
-// All widths are 128 (but the third layer's outer one).  Shared memory: two weight tiles as fp16 hi/lo pairs (2 x 64 KB) and one 64 KB
-// stage through which every tile enters and leaves in whole rows.  One accumulator and one operand block of tensor memory, used by the
+// All widths are 128 (but the third layer's outer one).  Shared memory: two weight tiles as fp16 hi/lo pairs (2 x 64 KB) and 64 KB of
+// boxes through which every tile enters and leaves.  One accumulator and one operand block of tensor memory, used by the
 // GEMMs of a tile one after the other.
-// Bound by latency: a tile's layers follow one another at one CTA of 16 warps per SM, 20 % of the L2's and 30 % of the memory's rate.  A
-// layer in a kernel of its own pays for a launch, barriers and tensor memory, a tile's way in and out; on 16 000 rows that is 9 us where
-// it takes 3 here (evaluation of 96 x 268 ragged 556 -> 514 us, step of 256 x 73 1518 -> 1428, evaluation of 512 x 100 1705 -> 1680).
+// Bound by latency: a tile's layers follow one another at one CTA per SM.  So nothing in a tile waits for more than it needs: a warp's
+// 32 x 32 part of every tile comes and goes through a box of its own (asynchronous copies and whole 128-byte pieces by its lanes), the
+// four warps of the same rows meet for the rows' largest entry, and all sixteen only at the operand, by arriving at a barrier that a
+// warp waits for which issues the products and fetches the weights.  With the whole tile in one stage and barriers of the CTA at every
+// turn of it (twelve a tile) a tile took 12-15 us: CHAINFIGURES.
+// A layer in a kernel of its own pays for a launch, barriers and tensor memory, a tile's way in and out.
 struct ChainSmem {
     static constexpr int kWa = 0, kWb = 65536, kStage = 131072, kMisc = 196608;
     static constexpr int kTotal = kMisc + 4352 + 1024;      // (exchange and four vectors, 4 KB, then barriers)
 };
+constexpr int kChainThreads = kGT + 32;                     // sixteen warps with a row and 32 columns a thread, and the issuing warp
+enum { kMapA, kMapAux, kMapRes, kMapExt, kMapMid, kMapC, kMapOut, kMapQ, kChainMaps };
+struct ChainMaps {
+    CUtensorMap m[kChainMaps];             // of the matrices that a launch has, boxes of 32 columns by box_rows
+    int box_rows;
+};
 
 enum { kChainFwd = 0, kChainBwd = 1, kChainTan = 2, kChainRev = 3 };
 template <int KIND, bool LINKED>
-__global__ void __launch_bounds__(kGT, 1)
-gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa, const float *__restrict__ ba, const float *__restrict__ Wb,
-                      const float *__restrict__ bb, const float *__restrict__ aux, int64_t E, float *__restrict__ mid_out,
-                      float *__restrict__ C, int32_t *__restrict__ status, const float *__restrict__ ext0, const float *__restrict__ ext1,
-                      float *__restrict__ q_out, const uint8_t *__restrict__ image_a, const uint8_t *__restrict__ image_b, const ChainLink link) {
+__global__ void __launch_bounds__(kChainThreads, 1)
+gemm_tc_chain2_kernel(const __grid_constant__ ChainMaps maps, const float *__restrict__ Wa, const float *__restrict__ ba, const float *__restrict__ Wb,
+                      const float *__restrict__ bb, int64_t E, int with_aux, int with_mid, int32_t *__restrict__ status, const float *__restrict__ ext,
+                      const uint8_t *__restrict__ image_a, const uint8_t *__restrict__ image_b, const ChainLink link) {
     using namespace tc;
     using L = ChainSmem;
     constexpr bool BWD = KIND == kChainBwd || KIND == kChainRev;
     constexpr int W = 128, MODE = BWD ? 1 : 0;
-    const bool residual = !BWD && (KIND == kChainFwd || aux != nullptr);
+    const bool residual = !BWD && with_aux;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint8_t *sWa_hi = smem + L::kWa, *sWa_lo = sWa_hi + 32768, *sWb_hi = smem + L::kWb, *sWb_lo = sWb_hi + 32768;
-    uint8_t *stage = smem + L::kStage;
     float *s_red = reinterpret_cast<float *>(smem + L::kMisc);
     float *s_ba = s_red + 512, *s_bb = s_ba + 128, *s_bc = s_bb + 128;         // biases; s_bc: of the third layer, or its vector
     float *s_dot = s_bc + 128;
     uint64_t *s_bar = reinterpret_cast<uint64_t *>(s_dot + 128);
-    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(s_bar + 3);                // (barriers of the GEMMs, of Wa and of Wb)
+    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(s_bar + 4);
     int *s_err = reinterpret_cast<int *>(s_tmem + 1);
+    // a GEMM is complete; the first and the second weight have arrived; an operand is written (one arrival per warp)
+    const uint32_t done = smem_u32(s_bar), have_a = done + 8, have_b = done + 16, ready = done + 24;
+    const uint32_t arrived = done + 48 + 8 * (threadIdx.x >> 5);               // a warp's box (behind the two words of s_tmem and s_err)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int r = tid & 127, qt = tid >> 7, col0 = qt * 32;
+    const int r = tid & 127, qt = (tid >> 7) & 3, col0 = qt * 32;
     constexpr float kWS = 64.f;
     if (!image_a) {
         bool range = load_weight_tile<true>(sWa_hi, sWa_lo, Wa, W, W, W, kWS);
@@ -434,15 +444,16 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
             s_dot[tid] = !BWD && link.dot && tid < link.width ? link.dot_w[tid] : 0.f;
         }
     }
-    const uint32_t bar = smem_u32(s_bar);
     if (tid == 0) {
-        mbar_init(bar, 1);
-        mbar_init(bar + 8, 1);
-        mbar_init(bar + 16, 1);
+        mbar_init(done, 1);
+        mbar_init(have_a, 1);
+        mbar_init(have_b, 1);
+        mbar_init(ready, kGT / 32);
+        for (int w = 0; w < kGT / 32; w++) mbar_init(done + 48 + 8 * w, 1);
         *s_err = 0;
         if (image_a) {
-            fetch_image(smem_u32(sWa_hi), LINKED && BWD ? link.image : image_a, bar + 8);
-            fetch_image(smem_u32(sWb_hi), image_b, bar + 16);
+            fetch_image(smem_u32(sWa_hi), LINKED && BWD ? link.image : image_a, have_a);
+            fetch_image(smem_u32(sWb_hi), image_b, have_b);
         }
     }
     __syncwarp();
@@ -454,217 +465,241 @@ gemm_tc_chain2_kernel(const float *__restrict__ A, const float *__restrict__ Wa,
     pdl_wait();                                    // set-up done (weights only); A and aux belong to the kernels before
     pdl_launch_dependents();
     const uint32_t tmem = *s_tmem;                 // accumulator at columns [0,128), operand at [128,256)
-    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t ta = tmem + 128;
     const int64_t ntiles = (E + kRows - 1) / kRows;
-    uint32_t phase = 0;
     bool failed = false;
-    const int in_cols = LINKED && BWD ? link.width : W;
-    if (blockIdx.x < ntiles) prefetch_tile_to_stage(stage, A, (int64_t)blockIdx.x * kRows, E, in_cols);
-
-    // this thread's 32 values -> operand block (row-scaled fp16 pairs); returns the row's scale.  `fetch`: a tile to copy into
-    // the stage as soon as everybody has read the current contents out of it (rows of `fetch` starting at `fetch_row0`)
-    auto to_operand = [&](const float (&x)[32], const float *fetch, int64_t fetch_row0) {
-        float rmax = 0.f;
-#pragma unroll
-        for (int c = 0; c < 32; c++) rmax = fmaxf(rmax, fabsf(x[c]));
-        s_red[qt * 128 + r] = rmax;
-        __syncthreads();
-        if (fetch) prefetch_tile_to_stage(stage, fetch, fetch_row0, E, W);
-        const float sc = row_scale(fmaxf(fmaxf(s_red[r], s_red[128 + r]), fmaxf(s_red[256 + r], s_red[384 + r])));
-        store_a_tmem<true>(ta + lane_off, col0, x, sc);
-        tmem_wait_st();
-        tc_fence_before();
-        __syncthreads();
-        return sc;
-    };
-    // Both weights are there for good, or (LINKED) the first place holds two in turn, each fetched when the GEMM with the other is done:
-    // `parity` of the fetch that has to be over
-    auto gemm = [&](uint8_t *w_hi, uint32_t wbar, uint32_t parity) {
-        if (warp == 0 && elect_one()) {
-            if (image_a && !mbar_wait(wbar, parity)) *s_err = 1;
-            tc_fence_after();
-            issue_gemm_ts<true>(tmem, ta, smem_u32(w_hi), smem_u32(w_hi) + 32768, W / 16, MODE, W);
-            mma_commit(bar);
-        }
-    };
-    auto refill = [&](const uint8_t *image) {
-        if (LINKED && warp == 0 && elect_one()) fetch_image(smem_u32(sWa_hi), image, bar + 8);
-    };
-    auto await = [&]() {
-        if (!failed && !mbar_wait(bar, phase)) failed = true;
-        phase ^= 1;
+    auto await = [&](uint32_t bar, uint32_t parity) {
+        if (!failed && !mbar_wait(bar, parity)) failed = true;
         tc_fence_after();
     };
-    // rows of the stage -> global memory, whole rows by consecutive lanes, eight rows per warp in flight
-    auto store_stage = [&](float *dst, int64_t tile, int cols) {
-        float4 v[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = *gstage(stage, warp * 8 + i, lane);
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int64_t gr = tile * kRows + warp * 8 + i;
-            if (gr < E && (!LINKED || lane * 4 < cols)) __stcs(reinterpret_cast<float4 *>(dst + gr * cols) + lane, v[i]);
-        }
-    };
 
-    // four columns of this thread's row of a matrix shaped like A (zero past the end); both halves of a 32-byte sector are used
-    auto own_row = [&](const float *src, int64_t tile, int w) {
-        const int64_t gr = tile * kRows + r;
-        return gr < E ? __ldg(reinterpret_cast<const float4 *>(src + gr * W + col0) + w) : make_float4(0.f, 0.f, 0.f, 0.f);
-    };
+    if (warp == kGT / 32) {
+        // ---- the issuing warp: products in the order of the layers.  The first place holds two weights in turn (LINKED), each fetched
+        // when the product with the other is done; `parity` of the fetch that has to be over
+        const bool elected = elect_one();
+        uint32_t n = 0;                            // products issued
+        auto gemm = [&](uint8_t *w_hi, uint32_t wbar, uint32_t parity) {
+            if (image_a) await(wbar, parity);
+            await(ready, n & 1);
+            if (elected) {
+                issue_gemm_ts<true>(tmem, tmem + 128, smem_u32(w_hi), smem_u32(w_hi) + 32768, W / 16, MODE, W);
+                mma_commit(done);
+            }
+            __syncwarp();
+            n++;
+        };
+        auto refill = [&](const uint8_t *image) {
+            await(done, (n - 1) & 1);
+            if (elected) fetch_image(smem_u32(sWa_hi), image, have_a);
+            __syncwarp();
+        };
+        for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+            const bool more = tile + gridDim.x < ntiles;
+            gemm(sWa_hi, have_a, 0);
+            if (LINKED && BWD) {
+                refill(image_a);
+                gemm(sWa_hi, have_a, 1);
+                if (more) refill(link.image);
+            }
+            if (LINKED && !BWD) refill(link.image);
+            gemm(sWb_hi, have_b, 0);
+            if (LINKED && !BWD) {
+                gemm(sWa_hi, have_a, 1);
+                if (more) refill(image_a);
+            }
+        }
+    } else {
+        const uint32_t acc = tmem + ((uint32_t)((warp & 3) * 32) << 16), ta = acc + 128;
+        uint8_t *const box = smem + L::kStage + warp * 4096;                    // [32 rows][128 bytes], 16-byte pieces in the 128-byte swizzle
+        const int row0 = 32 * (warp & 3);
+        auto piece = [&](int row, int w) { return reinterpret_cast<float4 *>(box + row * 128 + ((w ^ (row & 7)) << 4)); };
+        auto own = [&](int w) { return piece(lane, w); };                       // four columns of this thread's row
+        // the warp's part of a tile into its box (zeros past the end), once all lanes are past what they had to do there and what leaves has
+        // been read
+        uint32_t loads = 0;
+        auto load_box = [&](const CUtensorMap *map, int64_t tile) {
+            __syncwarp();
+            if (lane == 0) {
+                bulk_wait_read<0>();
+                mbar_expect_bytes(arrived, (uint32_t)maps.box_rows * 128u);
+                tensor_load_box(map, col0, (int)(tile * kRows) + row0, smem_u32(box), arrived);
+            }
+            loads++;
+        };
+        auto wait_box = [&]() { await(arrived, (loads - 1) & 1); };
+        // the box to its place; the next to write there waits for box_left()
+        auto store_box = [&](const CUtensorMap *map, int64_t tile) {
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                if (tile * kRows + row0 < E) tensor_store_box(map, col0, (int)(tile * kRows) + row0, box);
+                bulk_commit();
+            }
+        };
+        auto box_left = [&]() {
+            if (lane == 0) bulk_wait_read<0>();
+            __syncwarp();
+        };
+        auto row_group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + (warp & 3)) : "memory"); };
+        // this thread's 32 values -> operand block (row-scaled fp16 pairs); returns the row's scale.  (What the accumulator and the operand
+        // block held has been read and consumed: by this warp, and by the product that it has waited for.)
+        auto to_operand = [&](const float (&x)[32]) {
+            float rmax = 0.f;
+#pragma unroll
+            for (int c = 0; c < 32; c++) rmax = fmaxf(rmax, fabsf(x[c]));
+            s_red[qt * 128 + r] = rmax;
+            row_group_sync();
+            const float sc = row_scale(fmaxf(fmaxf(s_red[r], s_red[128 + r]), fmaxf(s_red[256 + r], s_red[384 + r])));
+            store_a_tmem<true>(ta, col0, x, sc);
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(ready);
+            return sc;
+        };
+        uint32_t phase = 0;
+        auto await_product = [&]() {
+            await(done, phase);
+            phase ^= 1;
+        };
+        // four columns of this thread's row of a matrix shaped like A (zero past the end); both halves of a 32-byte sector are used
+        auto own_row = [&](const float *src, int64_t tile, int w) {
+            const int64_t gr = tile * kRows + r;
+            return gr < E ? __ldg(reinterpret_cast<const float4 *>(src + gr * W + col0) + w) : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        if (blockIdx.x < ntiles) load_box(&maps.m[kMapA], blockIdx.x);
 
-    // Everything else that crosses to or from global memory goes through the stage in whole rows (a thread's own 32 columns of a
-    // row are 128 bytes: 32 separate lines per warp instruction if moved directly).  The stage holds, in turn: the input tile;
-    // BWD: the tile of tanh outputs; FWD: mid on its way out, then the residual tile; the output tile on its way out.
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        wait_prefetch();
-        __syncthreads();                            // the input tile has landed
-        float x[32];
-#pragma unroll
-        for (int w = 0; w < 8; w++) {
-            const float4 v = *gstage(stage, r, (col0 >> 2) + w);
-            x[4 * w] = v.x; x[4 * w + 1] = v.y; x[4 * w + 2] = v.z; x[4 * w + 3] = v.w;
-        }
-        if (LINKED && BWD) {
-            if (link.vec) {
-#pragma unroll
-                for (int c = 0; c < 32; c++) x[c] = s_bc[col0 + c] * fmaf(-x[c], x[c], 1.f);
-            }
-            const float sc0 = to_operand(x, link.res, tile * kRows);
-            gemm(sWa_hi, bar + 8, 0);
-            await();
-            refill(image_a);
-            if (link.res) {
-                wait_prefetch();
-                __syncthreads();
-            }
-            float v[32];
-            tmem_ld32(tmem + lane_off + col0, v);
-            const float inv = 1.f / (sc0 * kWS);
+        // The box holds, in turn: the input; BWD: what the third layer adds, its result on its way out, the tanh outputs, mid on its way out;
+        // TAN: a, then q on its way out; FWD: mid on its way out, then the residual; the output on its way out, and the third layer's.
+        for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+            float x[32];
+            wait_box();
 #pragma unroll
             for (int w = 0; w < 8; w++) {
-                float4 o = make_float4(v[4 * w] * inv, v[4 * w + 1] * inv, v[4 * w + 2] * inv, v[4 * w + 3] * inv);
-                float4 *slot = gstage(stage, r, (col0 >> 2) + w);
-                if (link.res) {
-                    const float4 t4 = *slot;
-                    o = make_float4(o.x + t4.x, o.y + t4.y, o.z + t4.z, o.w + t4.w);
-                }
-                *slot = o;
-                x[4 * w] = o.x; x[4 * w + 1] = o.y; x[4 * w + 2] = o.z; x[4 * w + 3] = o.w;
+                const float4 v = *own(w);
+                x[4 * w] = v.x; x[4 * w + 1] = v.y; x[4 * w + 2] = v.z; x[4 * w + 3] = v.w;
             }
-        }
-        // BWD: the tanh outputs arrive under the first GEMM, behind what leaves
-        const float sc1 = to_operand(x, BWD && !LINKED ? aux : nullptr, tile * kRows);
-        gemm(sWa_hi, bar + 8, LINKED && BWD ? 1 : 0);
-        if (LINKED && BWD) {
-            store_stage(link.out, tile, W);
-            __syncthreads();
-            prefetch_tile_to_stage(stage, aux, tile * kRows, E, W);
-        }
-        await();
-        if (LINKED && !BWD) refill(link.image);
-        if (LINKED && BWD && tile + gridDim.x < ntiles) refill(link.image);
-        if (BWD) {
-            wait_prefetch();
-            __syncthreads();
-        }
-        {
-            float v[32];
-            tmem_ld32(tmem + lane_off + col0, v);
-            const float inv = 1.f / (sc1 * kWS);
+            if (LINKED && BWD) {
+                if (link.res) load_box(&maps.m[kMapRes], tile);
+                if (link.vec) {
 #pragma unroll
-            for (int w = 0; w < 8; w++) {
-                float4 o = make_float4(fmaf(v[4 * w], inv, s_ba[col0 + 4 * w]), fmaf(v[4 * w + 1], inv, s_ba[col0 + 4 * w + 1]),
-                                       fmaf(v[4 * w + 2], inv, s_ba[col0 + 4 * w + 2]), fmaf(v[4 * w + 3], inv, s_ba[col0 + 4 * w + 3]));
-                float4 *slot = gstage(stage, r, (col0 >> 2) + w);
-                if (BWD) {
-                    const float4 t4 = *slot;
-                    o = make_float4(o.x * fmaf(-t4.x, t4.x, 1.f), o.y * fmaf(-t4.y, t4.y, 1.f), o.z * fmaf(-t4.z, t4.z, 1.f), o.w * fmaf(-t4.w, t4.w, 1.f));
-                    if (KIND == kChainRev) {
-                        const float4 q4 = own_row(ext0, tile, w);
-                        o = make_float4(o.x + q4.x, o.y + q4.y, o.z + q4.z, o.w + q4.w);
-                    }
-                    if (mid_out) *slot = o;
-                } else if (KIND == kChainTan) {
-                    const float4 a4 = own_row(ext0, tile, w), g4 = own_row(ext1, tile, w);
-                    const float4 q4 = make_float4(-2.f * a4.x * o.x * g4.x, -2.f * a4.y * o.y * g4.y, -2.f * a4.z * o.z * g4.z, -2.f * a4.w * o.w * g4.w);
-                    if (tile * kRows + r < E) *(reinterpret_cast<float4 *>(q_out + (tile * kRows + r) * W + col0) + w) = q4;
-                    o = make_float4(o.x * fmaf(-a4.x, a4.x, 1.f), o.y * fmaf(-a4.y, a4.y, 1.f), o.z * fmaf(-a4.z, a4.z, 1.f), o.w * fmaf(-a4.w, a4.w, 1.f));
-                    *slot = o;
-                } else {
-                    o = make_float4(tanh_ex2(o.x), tanh_ex2(o.y), tanh_ex2(o.z), tanh_ex2(o.w));
-                    *slot = o;                       // on its way to mid_out
+                    for (int c = 0; c < 32; c++) x[c] = s_bc[col0 + c] * fmaf(-x[c], x[c], 1.f);
                 }
-                x[4 * w] = o.x; x[4 * w + 1] = o.y; x[4 * w + 2] = o.z; x[4 * w + 3] = o.w;
-            }
-        }
-        const float sc2 = to_operand(x, nullptr, 0);     // (the accumulator has been read, the first GEMM's operand consumed)
-        gemm(sWb_hi, bar + 16, 0);
-        if (!BWD || mid_out) {                       // under the second GEMM: mid leaves, the residual tile arrives
-            store_stage(mid_out, tile, W);
-            __syncthreads();
-            if (residual) prefetch_tile_to_stage(stage, aux, tile * kRows, E, W);
-        }
-        await();
-        if (residual) {
-            wait_prefetch();
-            __syncthreads();
-        }
-        {
-            float v[32];
-            tmem_ld32(tmem + lane_off + col0, v);
-            const float inv = 1.f / (sc2 * kWS);
-#pragma unroll
-            for (int w = 0; w < 8; w++) {
-                float4 o = make_float4(fmaf(v[4 * w], inv, s_bb[col0 + 4 * w]), fmaf(v[4 * w + 1], inv, s_bb[col0 + 4 * w + 1]),
-                                       fmaf(v[4 * w + 2], inv, s_bb[col0 + 4 * w + 2]), fmaf(v[4 * w + 3], inv, s_bb[col0 + 4 * w + 3]));
-                float4 *slot = gstage(stage, r, (col0 >> 2) + w);
-                if (residual) {
-                    const float4 t4 = *slot;
-                    o = make_float4(o.x + t4.x, o.y + t4.y, o.z + t4.z, o.w + t4.w);
-                }
-                *slot = o;
-                if (LINKED && !BWD) { x[4 * w] = o.x; x[4 * w + 1] = o.y; x[4 * w + 2] = o.z; x[4 * w + 3] = o.w; }
-            }
-        }
-        const int64_t next = tile + gridDim.x;
-        if (LINKED && !BWD) {
-            const float sc3 = to_operand(x, nullptr, 0);
-            gemm(sWa_hi, bar + 8, 1);
-            store_stage(C, tile, W);
-            __syncthreads();
-            await();
-            if (next < ntiles) refill(image_a);
-            float dot = 0.f;
-            if (col0 < link.width) {
+                const float sc0 = to_operand(x);
+                await_product();
+                if (link.res) wait_box();
                 float v[32];
-                tmem_ld32(tmem + lane_off + col0, v);
-                const float inv = 1.f / (sc3 * kWS);
+                tmem_ld32(acc + col0, v);
+                const float inv = 1.f / (sc0 * kWS);
 #pragma unroll
                 for (int w = 0; w < 8; w++) {
-                    float4 o = make_float4(fmaf(v[4 * w], inv, s_bc[col0 + 4 * w]), fmaf(v[4 * w + 1], inv, s_bc[col0 + 4 * w + 1]),
-                                           fmaf(v[4 * w + 2], inv, s_bc[col0 + 4 * w + 2]), fmaf(v[4 * w + 3], inv, s_bc[col0 + 4 * w + 3]));
-                    if (link.tanh) o = make_float4(tanh_ex2(o.x), tanh_ex2(o.y), tanh_ex2(o.z), tanh_ex2(o.w));
-                    *gstage(stage, r, (col0 >> 2) + w) = o;
-                    const float4 u = *reinterpret_cast<const float4 *>(s_dot + col0 + 4 * w);
-                    dot = fmaf(o.x, u.x, fmaf(o.y, u.y, fmaf(o.z, u.z, fmaf(o.w, u.w, dot))));
+                    float4 o = make_float4(v[4 * w] * inv, v[4 * w + 1] * inv, v[4 * w + 2] * inv, v[4 * w + 3] * inv);
+                    if (link.res) {
+                        const float4 t4 = *own(w);
+                        o = make_float4(o.x + t4.x, o.y + t4.y, o.z + t4.z, o.w + t4.w);
+                    }
+                    *own(w) = o;
+                    x[4 * w] = o.x; x[4 * w + 1] = o.y; x[4 * w + 2] = o.z; x[4 * w + 3] = o.w;
                 }
             }
-            s_red[qt * 128 + r] = dot;
+            const float sc1 = to_operand(x);
+            if (LINKED && BWD) store_box(&maps.m[kMapOut], tile);
+            if (BWD) load_box(&maps.m[kMapAux], tile);
+            if (KIND == kChainTan) load_box(&maps.m[kMapExt], tile);
+            float4 e4[8];                            // (on their way under the product)
+            if (KIND == kChainTan || KIND == kChainRev) {
+#pragma unroll
+                for (int w = 0; w < 8; w++) e4[w] = own_row(ext, tile, w);
+            }
+            await_product();
+            if (BWD || KIND == kChainTan) wait_box();
+            {
+                float v[32];
+                tmem_ld32(acc + col0, v);
+                const float inv = 1.f / (sc1 * kWS);
+#pragma unroll
+                for (int w = 0; w < 8; w++) {
+                    float4 o = make_float4(fmaf(v[4 * w], inv, s_ba[col0 + 4 * w]), fmaf(v[4 * w + 1], inv, s_ba[col0 + 4 * w + 1]),
+                                           fmaf(v[4 * w + 2], inv, s_ba[col0 + 4 * w + 2]), fmaf(v[4 * w + 3], inv, s_ba[col0 + 4 * w + 3]));
+                    if (BWD) {
+                        const float4 t4 = *own(w);
+                        o = make_float4(o.x * fmaf(-t4.x, t4.x, 1.f), o.y * fmaf(-t4.y, t4.y, 1.f), o.z * fmaf(-t4.z, t4.z, 1.f), o.w * fmaf(-t4.w, t4.w, 1.f));
+                        if (KIND == kChainRev) o = make_float4(o.x + e4[w].x, o.y + e4[w].y, o.z + e4[w].z, o.w + e4[w].w);
+                        if (with_mid) *own(w) = o;
+                    } else if (KIND == kChainTan) {
+                        const float4 a4 = *own(w), g4 = e4[w];
+                        *own(w) = make_float4(-2.f * a4.x * o.x * g4.x, -2.f * a4.y * o.y * g4.y, -2.f * a4.z * o.z * g4.z, -2.f * a4.w * o.w * g4.w);
+                        o = make_float4(o.x * fmaf(-a4.x, a4.x, 1.f), o.y * fmaf(-a4.y, a4.y, 1.f), o.z * fmaf(-a4.z, a4.z, 1.f), o.w * fmaf(-a4.w, a4.w, 1.f));
+                    } else {
+                        o = make_float4(tanh_ex2(o.x), tanh_ex2(o.y), tanh_ex2(o.z), tanh_ex2(o.w));
+                        *own(w) = o;
+                    }
+                    x[4 * w] = o.x; x[4 * w + 1] = o.y; x[4 * w + 2] = o.z; x[4 * w + 3] = o.w;
+                }
+            }
+            const float sc2 = to_operand(x);         // under the second product: mid leaves, the residual arrives
+            if (KIND == kChainTan) {
+                store_box(&maps.m[kMapQ], tile);
+                box_left();
+#pragma unroll
+                for (int w = 0; w < 8; w++) *own(w) = make_float4(x[4 * w], x[4 * w + 1], x[4 * w + 2], x[4 * w + 3]);
+            }
+            if (!BWD || with_mid) store_box(&maps.m[kMapMid], tile);
+            if (residual) load_box(&maps.m[kMapAux], tile);
+            await_product();
+            if (residual) wait_box();
+            else box_left();
+            {
+                float v[32];
+                tmem_ld32(acc + col0, v);
+                const float inv = 1.f / (sc2 * kWS);
+#pragma unroll
+                for (int w = 0; w < 8; w++) {
+                    float4 o = make_float4(fmaf(v[4 * w], inv, s_bb[col0 + 4 * w]), fmaf(v[4 * w + 1], inv, s_bb[col0 + 4 * w + 1]),
+                                           fmaf(v[4 * w + 2], inv, s_bb[col0 + 4 * w + 2]), fmaf(v[4 * w + 3], inv, s_bb[col0 + 4 * w + 3]));
+                    if (residual) {
+                        const float4 t4 = *own(w);
+                        o = make_float4(o.x + t4.x, o.y + t4.y, o.z + t4.z, o.w + t4.w);
+                    }
+                    *own(w) = o;
+                    if (LINKED && !BWD) { x[4 * w] = o.x; x[4 * w + 1] = o.y; x[4 * w + 2] = o.z; x[4 * w + 3] = o.w; }
+                }
+            }
+            if (LINKED && !BWD) {
+                const float sc3 = to_operand(x);
+                store_box(&maps.m[kMapC], tile);
+                await_product();
+                float dot = 0.f;
+                if (col0 < link.width) {
+                    box_left();
+                    float v[32];
+                    tmem_ld32(acc + col0, v);
+                    const float inv = 1.f / (sc3 * kWS);
+#pragma unroll
+                    for (int w = 0; w < 8; w++) {
+                        float4 o = make_float4(fmaf(v[4 * w], inv, s_bc[col0 + 4 * w]), fmaf(v[4 * w + 1], inv, s_bc[col0 + 4 * w + 1]),
+                                               fmaf(v[4 * w + 2], inv, s_bc[col0 + 4 * w + 2]), fmaf(v[4 * w + 3], inv, s_bc[col0 + 4 * w + 3]));
+                        if (link.tanh) o = make_float4(tanh_ex2(o.x), tanh_ex2(o.y), tanh_ex2(o.z), tanh_ex2(o.w));
+                        *own(w) = o;
+                        const float4 u = *reinterpret_cast<const float4 *>(s_dot + col0 + 4 * w);
+                        dot = fmaf(o.x, u.x, fmaf(o.y, u.y, fmaf(o.z, u.z, fmaf(o.w, u.w, dot))));
+                    }
+                    store_box(&maps.m[kMapOut], tile);
+                }
+                if (link.dot) {
+                    s_red[qt * 128 + r] = dot;
+                    row_group_sync();
+                    if (qt == 0 && tile * kRows + r < E)
+                        link.dot[tile * kRows + r] = (s_red[r] + s_red[128 + r]) + (s_red[256 + r] + s_red[384 + r]) + (link.dot_b ? link.dot_b[0] : 0.f);
+                    row_group_sync();                // (before the next tile's rows exchange anything there)
+                }
+            } else {
+                store_box(&maps.m[kMapC], tile);
+            }
+            const int64_t next = tile + gridDim.x;
+            if (next < ntiles) load_box(&maps.m[kMapA], next);
         }
-        tc_fence_before();
-        __syncthreads();
-        if (LINKED && !BWD) {
-            store_stage(link.out, tile, link.width);
-            if (link.dot && qt == 0 && tile * kRows + r < E)
-                link.dot[tile * kRows + r] = (s_red[r] + s_red[128 + r]) + (s_red[256 + r] + s_red[384 + r]) + (link.dot_b ? link.dot_b[0] : 0.f);
-        }
-        else store_stage(C, tile, W);
-        __syncthreads();                            // the stage is free for the next input tile
-        if (next < ntiles) prefetch_tile_to_stage(stage, A, next * kRows, E, in_cols);
+        bulk_wait_all();
     }
-    wait_prefetch();
     if (failed) *s_err = 1;
     tc_fence_before();
     __syncthreads();
@@ -1146,9 +1181,15 @@ static int chain2_launch_as(const void *A, const void *Wa, const void *ba, const
             return check_launch();
         done[dev] = true;
     }
-    launch_with_weights(gemm_tc_chain2_kernel<KIND, LINKED>, dim3(grid), dim3(kGT), ChainSmem::kTotal, st, (const float *)A, (const float *)Wa, (const float *)ba,
-               (const float *)Wb, (const float *)bb, (const float *)aux, M, (float *)mid_out, (float *)C, status, (const float *)ext0,
-               (const float *)ext1, (float *)q_out, image_a, image_b, link);
+    ChainMaps maps = {};
+    maps.box_rows = (int)(M < 32 ? M : 32);
+    const auto map = [&](int k, const void *p, int64_t cols = 128) { return !p || make_rows_map(&maps.m[k], (float *)p, M, cols, 32); };
+    if (M >= (int64_t)1 << 31 || !map(kMapA, A, LINKED && (KIND == kChainBwd || KIND == kChainRev) ? link.width : 128) || !map(kMapAux, aux) ||
+        !map(kMapRes, link.res) || !map(kMapExt, KIND == kChainTan ? ext0 : nullptr) || !map(kMapMid, mid_out) || !map(kMapC, C) ||
+        !map(kMapOut, link.out, LINKED && KIND != kChainBwd && KIND != kChainRev ? link.width : 128) || !map(kMapQ, q_out))
+        return MLCGB_E_LIMIT;
+    launch_with_weights(gemm_tc_chain2_kernel<KIND, LINKED>, dim3(grid), dim3(kChainThreads), ChainSmem::kTotal, st, maps, (const float *)Wa, (const float *)ba,
+               (const float *)Wb, (const float *)bb, M, aux ? 1 : 0, mid_out ? 1 : 0, status, (const float *)(KIND == kChainTan ? ext1 : ext0), image_a, image_b, link);
     return check_launch();
 }
 template <int KIND>

@@ -52,6 +52,13 @@ __device__ __forceinline__ void tensor_store_box(const CUtensorMap *map, int x, 
                  "r"(y), "r"(tc::smem_u32(src_box))
                  : "memory");
 }
+// One box of a mapped matrix into shared memory (128-byte swizzle, as above), zeros past the end of the matrix; completes on the barrier,
+// which expects the whole box's bytes
+__device__ __forceinline__ void tensor_load_box(const CUtensorMap *map, int x, int y, uint32_t dst_saddr, uint32_t bar_saddr) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst_saddr),
+                 "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar_saddr)
+                 : "memory");
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // all but the newest `Pending` groups of this thread have finished reading shared memory
 template <int Pending>
