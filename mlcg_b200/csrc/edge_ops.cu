@@ -108,6 +108,47 @@ seg_mul_sum_kernel(const T *__restrict__ a, const T *__restrict__ V, const int64
 // and accumulation order are those of the kernel above: identical results.
 constexpr int kSegSlots = 8, kSegWarps = 8, kSegBlocks = 4;
 
+// What a warp that walks nodes n, n + step, ... needs of the lists before it can ask for rows: the edges of its node and the first 32 of them
+// (lane t holds edge k0 + t), asked for while it works on the node before; the bounds of the node after that one too.  With bounds,
+// neighbours and rows one after the other for every node, a launch over 1.1 M edges took 74 us, like this 70 (the force pass's
+// kernel, which needs the registers, does better without: 124 us of 147).
+template <bool PERM>
+struct NodeEdges {
+    const int64_t *ptr;
+    const int32_t *nbr, *eperm;
+    int64_t N, step;
+    int lane;
+    int64_t k0 = 0, next0 = 0;
+    int64_t len = 0, next_len = 0;
+    int32_t j = 0, e = 0;
+    __device__ __forceinline__ void bounds(int64_t n) {
+        if (n < N) {
+            next0 = ptr[n];
+            next_len = ptr[n + 1] - next0;
+        }
+    }
+    __device__ __forceinline__ void edges() {
+        k0 = next0;
+        len = next_len;
+        j = e = 0;
+        if (lane < len) {
+            j = nbr[k0 + lane];
+            if (PERM) e = eperm[k0 + lane];
+        }
+    }
+    __device__ __forceinline__ void start(int64_t n) {
+        bounds(n);
+        edges();
+        bounds(n + step);
+    }
+    __device__ __forceinline__ void next(int64_t n) {      // (node n has been taken)
+        if (n + step < N) {
+            edges();
+            bounds(n + 2 * step);
+        }
+    }
+};
+
 template <bool PERM>
 __global__ void __launch_bounds__(kSegWarps * 32, kSegBlocks)
 seg_mul_sum_async_kernel(const float *__restrict__ a, const float *__restrict__ V, const int64_t *__restrict__ ptr, const int32_t *__restrict__ nbr,
@@ -119,56 +160,62 @@ seg_mul_sum_async_kernel(const float *__restrict__ a, const float *__restrict__ 
     const float4 *a4 = reinterpret_cast<const float4 *>(a) + lane, *V4 = reinterpret_cast<const float4 *>(V) + lane;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    NodeEdges<PERM> ahead{ptr, nbr, eperm, N, nwarps, lane};
+    ahead.start(warp);
     for (int64_t n = warp; n < N; n += nwarps) {
-        const int64_t k0 = ptr[n], k1 = ptr[n + 1];
+        const int64_t k0 = ahead.k0, k1 = k0 + ahead.len;
+        const int32_t first_j = ahead.j, first_e = ahead.e;
+        ahead.next(n);
         float4 acc0 = make_float4(0.f, 0.f, 0.f, 0.f), acc1 = acc0;
         for (int64_t c0 = k0; c0 < k1; c0 += 32) {               // the row's edges, 32 at a time: lane t holds edge c0 + t
             const int len = (int)(k1 - c0 < 32 ? k1 - c0 : 32);
-            int32_t my_j = 0;
-            int64_t my_e = 0;
-            if (lane < len) {
+            int32_t my_j = first_j, my_e = PERM ? first_e : lane;    // (without a permutation the row of V from c0)
+            if (c0 > k0 && lane < len) {
                 my_j = nbr[c0 + lane];
-                my_e = PERM ? (int64_t)eperm[c0 + lane] : c0 + lane;
+                if (PERM) my_e = eperm[c0 + lane];
             }
-            const int ngroups = (len + 3) >> 2;
+            const float4 *Vc = PERM ? V4 : V4 + c0 * 32;
             // group g = edges 4g .. 4g+3 of the chunk -> slots (4g + u) % kSegSlots
             auto issue = [&](int g) {
-                if (g < ngroups) {
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const int t = 4 * g + u;
-                        const int64_t e = __shfl_sync(0xffffffffu, my_e, t & 31);
-                        if (t < len)
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring_addr + (uint32_t)((t % kSegSlots) * 512)), "l"(V4 + e * 32) : "memory");
-                    }
-                }
-                asm volatile("cp.async.commit_group;" ::: "memory");       // (an empty group keeps the count of pending groups fixed)
-            };
-#pragma unroll
-            for (int g = 0; g < kSegSlots / 4; g++) issue(g);
-            for (int g = 0; g < ngroups; g++) {
-                float4 x[4];
+                const uint32_t to = ring_addr + (uint32_t)(4 * g % kSegSlots) * 512u;
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     const int t = 4 * g + u;
-                    const int32_t j = __shfl_sync(0xffffffffu, my_j, t & 31);
-                    x[u] = t < len ? __ldg(a4 + (int64_t)j * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const int32_t e = __shfl_sync(0xffffffffu, my_e, t & 31);
+                    if (t < len)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + (uint32_t)(u * 512)), "l"(Vc + (int64_t)e * 32) : "memory");
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");       // (an empty group keeps the count of pending groups fixed)
+            };
+            const int whole = len >> 2;
+#pragma unroll
+            for (int g = 0; g < kSegSlots / 4; g++) issue(g);
+            for (int g = 0; g < whole; g++) {
+                float4 x[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) x[u] = __ldg(a4 + (int64_t)__shfl_sync(0xffffffffu, my_j, 4 * g + u) * 32);
+                asm volatile("cp.async.wait_group %0;" ::"n"(kSegSlots / 4 - 1) : "memory");
+                const float4 *slot = ring + (4 * g % kSegSlots) * 32;
+                const float4 v0 = slot[0], v1 = slot[32], v2 = slot[64], v3 = slot[96];
+                vfma(acc0, x[0], v0);
+                vfma(acc1, x[1], v1);
+                vfma(acc0, x[2], v2);
+                vfma(acc1, x[3], v3);
+                if (4 * (g + kSegSlots / 4) < len) issue(g + kSegSlots / 4);
+                else asm volatile("cp.async.commit_group;" ::: "memory");
+            }
+            if (len & 3) {                                       // the last edges of the row, one by one into the first sum
+                float4 x[3];
+#pragma unroll
+                for (int u = 0; u < 3; u++) {
+                    const int32_t j = __shfl_sync(0xffffffffu, my_j, (4 * whole + u) & 31);
+                    x[u] = 4 * whole + u < len ? __ldg(a4 + (int64_t)j * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
                 asm volatile("cp.async.wait_group %0;" ::"n"(kSegSlots / 4 - 1) : "memory");
-                const int full = 4 * g + 3 < len;
-                if (full) {
-                    const float4 v0 = ring[((4 * g) % kSegSlots) * 32], v1 = ring[((4 * g + 1) % kSegSlots) * 32];
-                    const float4 v2 = ring[((4 * g + 2) % kSegSlots) * 32], v3 = ring[((4 * g + 3) % kSegSlots) * 32];
-                    vfma(acc0, x[0], v0);
-                    vfma(acc1, x[1], v1);
-                    vfma(acc0, x[2], v2);
-                    vfma(acc1, x[3], v3);
-                } else {                                          // the last edges of the row, one by one into the first sum
+                const float4 *slot = ring + (4 * whole % kSegSlots) * 32;
 #pragma unroll
-                    for (int u = 0; u < 3; u++)
-                        if (4 * g + u < len) vfma(acc0, x[u], ring[((4 * g + u) % kSegSlots) * 32]);
-                }
-                issue(g + kSegSlots / 4);
+                for (int u = 0; u < 3; u++)
+                    if (4 * whole + u < len) vfma(acc0, x[u], slot[u * 32]);
             }
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }

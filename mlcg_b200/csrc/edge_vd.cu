@@ -11,6 +11,8 @@
 // 2 KB (tangent) of rows, of which W and W' come from HBM once.
 #include "schnet_internal.cuh"
 
+#include <type_traits>
+
 namespace mlcgb {
 
 enum { kSegForce = 0, kSegTangent = 1, kSegTangentRows = 2 };     // the last: tangent with a = 0
@@ -61,12 +63,13 @@ seg_vd_kernel(const float *__restrict__ a, const float *__restrict__ x, const fl
             // group g = edges 2g, 2g+1 of the chunk -> slots (2g + u) % kSlots
             auto issue = [&](int g) {
                 if (g < ngroups) {
+                    const uint32_t to = ring_addr + (uint32_t)((2 * g % kSlots) * kRows * 512);
 #pragma unroll
                     for (int u = 0; u < 2; u++) {
                         const int t = 2 * g + u;
                         const int64_t p = __shfl_sync(0xffffffffu, my_p, t & 31);
                         if (t < len) {
-                            const uint32_t dst = ring_addr + (uint32_t)((t % kSlots) * kRows * 512);
+                            const uint32_t dst = to + (uint32_t)(u * kRows * 512);
                             if (kValue) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(W4 + p * 32) : "memory");
                             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (kRows - 1) * 512), "l"(Wd4 + p * 32) : "memory");
                         }
@@ -76,8 +79,10 @@ seg_vd_kernel(const float *__restrict__ a, const float *__restrict__ x, const fl
             };
 #pragma unroll
             for (int g = 0; g < kSlots / 2; g++) issue(g);
-            // two groups (four edges) per step
-            for (int g = 0; g < ngroups; g += 2) {
+            // two groups (four edges) per step; of the last step perhaps some.  (Tangents: steps of whole groups without bounds, a step of
+            // 256 x 73 beads 1380 -> 1350 us; the force pass has no registers for both kinds of step: 124 -> 129 us a launch.)
+            auto step = [&](int g, auto whole) {
+                constexpr bool ALL = decltype(whole)::value;
                 float4 xa[4], xb[4];
                 float dd[4];
 #pragma unroll
@@ -85,18 +90,19 @@ seg_vd_kernel(const float *__restrict__ a, const float *__restrict__ x, const fl
                     const int t = 2 * g + u;
                     const int64_t j = __shfl_sync(0xffffffffu, my_j, t & 31);
                     if (kTan) dd[u] = __shfl_sync(0xffffffffu, my_s, t & 31);
-                    if (MODE != kSegTangentRows) xa[u] = t < len ? __ldg(a4 + j * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (kTan) xb[u] = t < len ? __ldg(x4 + j * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (MODE != kSegTangentRows) xa[u] = ALL || t < len ? __ldg(a4 + j * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (kTan) xb[u] = ALL || t < len ? __ldg(x4 + j * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
                 float dot[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     asm volatile("cp.async.wait_group %0;" ::"n"(kSlots / 2 - 1) : "memory");
+                    const float4 *slots = ring + (2 * (g + h) % kSlots) * kRows * 32;
 #pragma unroll
                     for (int v = 0; v < 2; v++) {
                         const int u = 2 * h + v, t = 2 * g + u;
-                        if (t < len) {
-                            const float4 *slot = ring + (t % kSlots) * kRows * 32;
+                        if (ALL || t < len) {
+                            const float4 *slot = slots + v * kRows * 32;
                             const float4 wd = slot[(kRows - 1) * 32];
                             if (kValue) {
                                 const float4 w = slot[0];
@@ -126,7 +132,11 @@ seg_vd_kernel(const float *__restrict__ a, const float *__restrict__ x, const fl
                     d += __shfl_xor_sync(0xffffffffu, d, 1);
                     if ((lane & 7) == 0) s_dot[(2 * g + (lane >> 4) * 2 + ((lane >> 3) & 1)) & 31] = d;
                 }
-            }
+            };
+            int g = 0;
+            if constexpr (kTan)
+                for (; 2 * g + 4 <= len; g += 2) step(g, std::true_type{});
+            for (; 2 * g < len; g += 2) step(g, std::false_type{});
             asm volatile("cp.async.wait_group 0;" ::: "memory");
             if (!kTan) {
                 __syncwarp();
