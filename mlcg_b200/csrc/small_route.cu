@@ -26,6 +26,7 @@ struct SmallNet {                             // pointers of one launch
     const float *b2, *b3, *bh, *wo, *bo;      // biases; output layer
     int64_t N, B;
     int Wh;
+    int32_t *status;
     const int64_t *ptr, *struct_ptr;
     const int32_t *nbr, *pair_of;
     const float *W, *Wd, *dd;
@@ -46,7 +47,8 @@ struct SmallSmem {
     static constexpr int kS = 3 * kWFloats;                                 // two row tiles [RT][128]
     static constexpr int kX = kS + 2 * RT * 128;                            // partial sums [4][RT][128]; the aggregation's [16][128]
     static constexpr int kXFloats = 16 * 128 > 4 * RT * 128 ? 16 * 128 : 4 * RT * 128;
-    static constexpr size_t kBytes = sizeof(float) * (kX + kXFloats);
+    static constexpr int kBar = kX + kXFloats;                              // a barrier per slot
+    static constexpr size_t kBytes = sizeof(float) * (kBar + 6);
 };
 
 __device__ __forceinline__ void fma4s(float4 &acc, const float4 &a, const float4 &b) {
@@ -67,12 +69,39 @@ struct SmallTile {
     float *smem, *x;
     int tid, c, rq, lane, warp;
     int64_t n0, N;
+    bool failed = false;                      // a matrix did not arrive
 
     __device__ __forceinline__ SmallTile(float4 *base, int at_x, int64_t N_)
         : smem(reinterpret_cast<float *>(base)), x(smem + at_x), tid(threadIdx.x), c(threadIdx.x & 127), rq(threadIdx.x >> 7), lane(threadIdx.x & 31),
           warp(threadIdx.x >> 5), n0(0), N(N_) {}
     __device__ __forceinline__ float *slot(int i) const { return smem + SmallSmem<RT>::kW + i * SmallSmem<RT>::kWFloats; }
     __device__ __forceinline__ float *rows(int i) const { return smem + SmallSmem<RT>::kS + i * RT * 128; }
+    // The matrices of a launch -> slots, by the copy engine, a row of 512 bytes at a time (by all threads; rows past the end zero).  (Copies of
+    // 16 bytes by all lanes kept a CTA that had to wait for its SM, beside the last one's links, from its lists for 1 us: 64 x 10 beads replayed 50.3 -> 48.6 us.)
+    __device__ __forceinline__ uint32_t bar(int i) const { return tc::smem_u32(smem + SmallSmem<RT>::kBar) + 8 * i; }
+    __device__ __forceinline__ void fetch_all(const float *const (&src)[3], int last_rows) const {
+        if (tid == 0) {
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                tc::mbar_init(bar(i), 1);
+                if (src[i]) tc::mbar_expect_bytes(bar(i), (uint32_t)(i == 2 ? last_rows : 128) * 512u);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const int row = warp * 8 + lane, rows = i == 2 ? last_rows : 128;
+            if (!src[i] || lane >= 8) continue;
+            if (row < rows) {
+                tc::bulk_load(tc::smem_u32(slot(i) + row * kWPitch), src[i] + row * 128, 512, bar(i));
+            } else {
+                for (int k = 0; k < 32; k++) reinterpret_cast<float4 *>(slot(i) + row * kWPitch)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+    }
+    __device__ __forceinline__ void arrived(int i) {
+        if (!failed && !tc::mbar_wait(bar(i), 0)) failed = true;
+    }
     // matrix [rows][128] -> slot, asynchronously, a group of copies of its own; rows past the end zero
     __device__ __forceinline__ void fetch(int i, const float *src, int nrows) const {
         const uint32_t base = tc::smem_u32(slot(i));
@@ -278,9 +307,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
     constexpr int RO = T::RO;
     T t(small_smem, SmallSmem<RT>::kX, p.N);
     constexpr bool kLast = KIND == kSmFwdLast || KIND == kSmTanLast;
-    t.fetch(0, p.w[0], 128);
-    t.fetch(1, p.w[1], 128);
-    t.fetch(2, p.w[2], kLast ? p.Wh : 128);
+    t.fetch_all(p.w, kLast ? p.Wh : 128);
     // What does not come from the kernel in front is read before the wait for it, a latency of the second-level cache each: biases and the
     // lists of the first tile (the kernel in front began behind those that made the lists).  What does, and is wanted after a layer,
     // is read under the aggregation (64 x 10 beads replayed: 64 -> 60.5 us).
@@ -301,8 +328,8 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
             res[i] = p.res ? t.get(p.res, i) : 0.f;
             act[i] = kForward || KIND == kSmRevFirst ? 0.f : t.get(p.act, i);
         }
-        copies_wait<2>();                                              // (a matrix is waited for in front of the barrier before its layer)
         small_aggregate<kForward ? kAggPlain : (KIND == kSmBwd ? kAggForce : kAggTangent), RT>(p, t, S0, ed);
+        t.arrived(0);                                                  // (a matrix is waited for in front of its layer)
         ready = true;
         float v[RO], a[RO], q[RO];
         if (KIND == kSmFwd || KIND == kSmFwdLast) {
@@ -312,7 +339,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 a[i] = tc::tanh_ex2(v[i] + b2);
                 t.put(p.o_act, i, a[i]);
             }
-            copies_wait<1>();
+            t.arrived(1);
             t.hand_on(S1, a);
             t.template layer<true>(S1, t.slot(1), v);                  // lin + residual
 #pragma unroll
@@ -320,7 +347,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 v[i] += b3 + res[i];
                 t.put(p.o_x, i, v[i]);
             }
-            copies_wait<0>();
+            t.arrived(2);
             t.hand_on(S0, v);
             t.template layer<true>(S0, t.slot(2), v);                  // lin1 of the next block | output network
             if (KIND == kSmFwd) {
@@ -367,7 +394,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 v[i] += res[i];
                 t.put(p.o_g, i, v[i]);
             }
-            copies_wait<1>();
+            t.arrived(1);
             t.hand_on(S1, v);
             t.template layer<false>(S1, t.slot(1), v);                 // lin^T, tanh' of the block below
 #pragma unroll
@@ -375,7 +402,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 v[i] *= fmaf(-act[i], act[i], 1.f);
                 t.put(p.o_gu, i, v[i]);
             }
-            copies_wait<0>();
+            t.arrived(2);
             t.hand_on(S0, v);
             t.template layer<false>(S0, t.slot(2), v);                 // lin2^T
 #pragma unroll
@@ -390,7 +417,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 t.put(p.o_act, i, v[i]);
                 if (KIND == kSmTan) t.put(p.o_q, i, q[i]);
             }
-            copies_wait<1>();
+            t.arrived(1);
             t.hand_on(S1, v);
             t.template layer<true>(S1, t.slot(1), v);
 #pragma unroll
@@ -398,7 +425,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 v[i] += res[i];
                 t.put(p.o_x, i, v[i]);
             }
-            copies_wait<0>();
+            t.arrived(2);
             t.hand_on(S0, v);
             t.template layer<true>(S0, t.slot(2), v);
             if (KIND == kSmTan) {
@@ -452,7 +479,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                 t.put(p.o_g, i, v[i]);
             }
             if (KIND == kSmRev) {
-                copies_wait<1>();
+                t.arrived(1);
                 t.hand_on(S1, v);
                 t.template layer<false>(S1, t.slot(1), v);
 #pragma unroll
@@ -460,7 +487,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
                     v[i] = fmaf(v[i], fmaf(-act[i], act[i], 1.f), t.get(p.q, i));
                     t.put(p.o_ub, i, v[i]);
                 }
-                copies_wait<0>();
+                t.arrived(2);
                 t.hand_on(S0, v);
                 t.template layer<false>(S0, t.slot(2), v);
 #pragma unroll
@@ -469,7 +496,7 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
         }
         __syncthreads();                                               // the tile buffers are free for the next rows
     }
-    copies_wait<0>();
+    if (t.failed) atomicOr(p.status, (int)kTensorWait);
 }
 
 // Embedding rows and lin1 of the first block, eight nodes
@@ -489,6 +516,7 @@ __device__ __forceinline__ void embedding_rows(SmallTile<8> &t, float *S, const 
         }
         reinterpret_cast<float4 *>(S)[t.warp * 32 + t.lane] = v;
     }
+    copies_wait<0>();                                                  // (the weight, under the two latencies of the rows)
     __syncthreads();
     float v[2];
     t.layer<true>(S, t.slot(0), v);
@@ -517,7 +545,6 @@ small_start_kernel(const float *__restrict__ pos, const int64_t *__restrict__ ty
         }
         d[e] = v;
     }
-    copies_wait<0>();
     for (t.n0 = (int64_t)blockIdx.x * RT; t.n0 < N; t.n0 += (int64_t)gridDim.x * RT) {
         __syncthreads();
         embedding_rows(t, t.rows(0), types, num_types, table, x, xl, status);
@@ -550,7 +577,6 @@ small_graph_count_kernel(const float *__restrict__ pos, const SmallGraph g, int6
     if ((int)blockIdx.x >= count_blocks) {
         SmallTile<8> t(small_smem, SmallStartSmem::kX, N);
         t.fetch(0, W1, 128);
-        copies_wait<0>();
         for (t.n0 = (int64_t)(blockIdx.x - count_blocks) * 8; t.n0 < N; t.n0 += (int64_t)(gridDim.x - count_blocks) * 8) {
             __syncthreads();
             embedding_rows(t, t.smem + SmallStartSmem::kS, types, num_types, table, x, xl, status);
@@ -843,6 +869,7 @@ static SmallNet small_net(const SmallForward &f, int64_t l) {
     p.N = f.N;
     p.B = f.B;
     p.Wh = (int)f.w->head_width;
+    p.status = f.status;
     p.ptr = f.ptr;
     p.nbr = f.row1;
     p.pair_of = f.pair_of;
