@@ -360,40 +360,56 @@ edge_distance_bwd_kernel(const T *__restrict__ pos, const T *__restrict__ g, con
 }
 
 // Forces of a symmetric centre-sorted list (the in-edges of a node are the reverses of its out-edges) from the derivative of every pair,
-// and the per-structure sums of the node energies in one launch: a warp per node, then a warp per structure
+// and the per-structure sums of the node energies in one launch: half a warp per node, then a warp per structure
 __global__ void __launch_bounds__(256)
 finish_kernel(const float *__restrict__ pos, const float *__restrict__ pair_g, const float *__restrict__ d, const int32_t *__restrict__ row1,
               const int64_t *__restrict__ ptr, const int32_t *__restrict__ pair_of, int64_t N, float *__restrict__ gpos, float sign, const float *__restrict__ en,
               const int64_t *__restrict__ struct_ptr, int64_t B, float *__restrict__ energy) {
-    const int lane = threadIdx.x & 31;
+    // Half a warp per node, two edges a lane and turn: a chain of three latencies (bounds, lists, rows of pairs and positions) whatever the
+    // number of lanes, so what counts is how many nodes are in it (a warp per node: 25.5 us for 51 200 nodes, like this 12.9).
+    const int lane = threadIdx.x & 31, sub = lane & 15;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t node_warps = (N + 1) / 2;
     pdl_wait();
-    for (int64_t n = warp; n < N + B; n += nwarps) {
+    for (int64_t item = warp; item < node_warps + B; item += nwarps) {
         float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-        if (n >= N) {
-            const int64_t b = n - N;
+        if (item >= node_warps) {
+            const int64_t b = item - node_warps;
             for (int64_t k = struct_ptr[b] + lane; k < struct_ptr[b + 1]; k += 32) s0 += en[k];
             s0 = warp_sum(s0);
             if (lane == 0) energy[b] = s0;
             continue;
         }
-        const float x = pos[n * 3], y = pos[n * 3 + 1], z = pos[n * 3 + 2];
-        for (int64_t k = ptr[n] + lane; k < ptr[n + 1]; k += 32) {
-            const int64_t j = row1[k];
-            const float dk = d[k], w = dk > 0.f ? sign * pair_g[pair_of[k]] / dk : 0.f;     // (coinciding beads: the norm's subgradient 0)
-            s0 = fmaf(w, x - pos[j * 3], s0);
-            s1 = fmaf(w, y - pos[j * 3 + 1], s1);
-            s2 = fmaf(w, z - pos[j * 3 + 2], s2);
+        const int64_t n = 2 * item + (lane >> 4);
+        int64_t k0 = 0, k1 = 0;
+        float x = 0.f, y = 0.f, z = 0.f;
+        if (n < N) {
+            k0 = ptr[n];
+            k1 = ptr[n + 1];
+            x = pos[n * 3]; y = pos[n * 3 + 1]; z = pos[n * 3 + 2];
         }
-        s0 = warp_sum(s0); s1 = warp_sum(s1); s2 = warp_sum(s2);
-        if (lane == 0) { gpos[n * 3] = s0; gpos[n * 3 + 1] = s1; gpos[n * 3 + 2] = s2; }
+        for (int64_t k = k0 + sub; k < k1; k += 32) {
+            const bool two = k + 16 < k1;
+            const int64_t k2 = two ? k + 16 : k, j0 = row1[k], j1 = row1[k2];
+            const float d0 = d[k], d1 = d[k2], g0 = pair_g[pair_of[k]], g1 = pair_g[pair_of[k2]];
+            const float x0 = pos[j0 * 3], y0 = pos[j0 * 3 + 1], z0 = pos[j0 * 3 + 2], x1 = pos[j1 * 3], y1 = pos[j1 * 3 + 1], z1 = pos[j1 * 3 + 2];
+            const float w0 = d0 > 0.f ? sign * g0 / d0 : 0.f, w1 = two && d1 > 0.f ? sign * g1 / d1 : 0.f;     // (coinciding beads: the norm's subgradient 0)
+            s0 = fmaf(w0, x - x0, s0); s1 = fmaf(w0, y - y0, s1); s2 = fmaf(w0, z - z0, s2);
+            if (two) { s0 = fmaf(w1, x - x1, s0); s1 = fmaf(w1, y - y1, s1); s2 = fmaf(w1, z - z1, s2); }
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+            s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+            s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+        }
+        if (sub == 0 && n < N) { gpos[n * 3] = s0; gpos[n * 3 + 1] = s1; gpos[n * 3 + 2] = s2; }
     }
 }
-
 int finish_launch(const float *pos, const float *pair_g, const float *d, const int32_t *row1, const int64_t *ptr, const int32_t *pair_of, int64_t N, float *gpos,
                   float sign, const float *en, const int64_t *struct_ptr, int64_t B, float *energy, cudaStream_t st) {
     TimelineScope timeline_scope("finish", st);
-    launch_pdl(finish_kernel, dim3(grid_for((N + B) * 32, 256)), dim3(256), 0, st, pos, pair_g, d, row1, ptr, pair_of, N, gpos, sign, en, struct_ptr, B, energy);
+    launch_pdl(finish_kernel, dim3(grid_for(((N + 1) / 2 + B) * 32, 256)), dim3(256), 0, st, pos, pair_g, d, row1, ptr, pair_of, N, gpos, sign, en, struct_ptr, B, energy);
     return check_launch();
 }
 

@@ -2716,13 +2716,17 @@ mask_rows_fill_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr
                       int32_t *__restrict__ pair_of) {
     const int lane = threadIdx.x & 31;
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < N; i += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+        // (all that hangs on the point alone is asked for at once, its words before it is known how many there are)
         const int b = struct_of[i];
-        if (cellparam && cellparam[b].tile != 2) continue;
-        const int64_t lo = ptr[b], off = offsets[i];
-        const int n = (int)((ptr[b + 1] < N ? ptr[b + 1] : N) - lo), il = (int)(i - lo), nw = (n + 31) >> 5, kept = (int)(offsets[i + 1] - off);
-        if (kept == 0) continue;
+        const int64_t off = offsets[i], next = offsets[i + 1];
         const int4 si = seg[i];
-        each_hit(masks + i * kMaskWords, nw, kept, lane, [&](int rank, int jl) {
+        const uint2 mine = masks[i * kMaskWords + lane];
+        if (cellparam && cellparam[b].tile != 2) continue;
+        const int64_t lo = ptr[b], hi = ptr[b + 1];
+        const int n = (int)((hi < N ? hi : N) - lo), il = (int)(i - lo), nw = (n + 31) >> 5, kept = (int)(next - off);
+        if (kept == 0) continue;
+        static_assert(kMaskWords == 32, "a word of the row per lane");
+        each_hit_of(mine, 0, nw, kept, lane, [&](int rank, int jl) {
             const int64_t slot = off + rank, j = lo + jl;
             T d2 = T(0);
             if (out.distance) d2 = dist2_rn(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], pos[3 * j], pos[3 * j + 1], pos[3 * j + 2]);

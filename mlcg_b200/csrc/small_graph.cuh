@@ -140,27 +140,30 @@ __device__ __forceinline__ int nth_bit(unsigned bits, int k) {
 // f(rank, local index) for the first `kept` hits of a row of nw words, 32 consecutive ranks at a time: a lane looks for the word of its rank
 // among the 32 of the warp, and for the bit in it.  (Word by word, the lanes of the word's bits at work, a row took as many turns as it
 // has words with a hit, most lanes idle: 37 structures of up to 700 points in float64 with distances 99 -> 81 us.)
+// each_hit_of: of up to 32 words from w0 on, of which lane t holds word w0 + t (whatever it holds beyond the row).
+template <typename F>
+__device__ __forceinline__ void each_hit_of(uint2 mine, int w0, int nw, int kept, int lane, F &&f) {
+    const bool there = w0 + lane < nw;
+    if (!there) mine = make_uint2(0u, 0u);
+    const int first = (int)__shfl_sync(0xffffffffu, mine.x, 0), last = min(nw - w0, 32) - 1;
+    const int before = there ? (int)mine.x : 0x7fffffff;
+    const int end = min(kept, (int)__shfl_sync(0xffffffffu, mine.x + (unsigned)__popc(mine.y), last));
+    for (int k = first; k < end; k += 32) {
+        const int rank = k + lane;
+        int w = 0;                                 // the last word with no more hits before it than the rank
+#pragma unroll
+        for (int step = 16; step; step >>= 1) {
+            const int b = __shfl_sync(0xffffffffu, before, w + step);
+            if (b <= rank) w += step;
+        }
+        const unsigned bits = __shfl_sync(0xffffffffu, mine.y, w);
+        const int b = __shfl_sync(0xffffffffu, before, w);
+        if (rank < end) f(rank, (w0 + w) * 32 + nth_bit(bits, rank - b));
+    }
+}
 template <typename F>
 __device__ __forceinline__ void each_hit(const uint2 *__restrict__ row, int nw, int kept, int lane, F &&f) {
-    for (int w0 = 0; w0 < nw; w0 += 32) {
-        const bool there = w0 + lane < nw;
-        const uint2 mine = there ? row[w0 + lane] : make_uint2(0u, 0u);
-        const int first = (int)__shfl_sync(0xffffffffu, mine.x, 0), last = min(nw - w0, 32) - 1;
-        const int before = there ? (int)mine.x : 0x7fffffff;
-        const int end = min(kept, (int)__shfl_sync(0xffffffffu, mine.x + (unsigned)__popc(mine.y), last));
-        for (int k = first; k < end; k += 32) {
-            const int rank = k + lane;
-            int w = 0;                             // the last word with no more hits before it than the rank
-#pragma unroll
-            for (int step = 16; step; step >>= 1) {
-                const int b = __shfl_sync(0xffffffffu, before, w + step);
-                if (b <= rank) w += step;
-            }
-            const unsigned bits = __shfl_sync(0xffffffffu, mine.y, w);
-            const int b = __shfl_sync(0xffffffffu, before, w);
-            if (rank < end) f(rank, (w0 + w) * 32 + nth_bit(bits, rank - b));
-        }
-    }
+    for (int w0 = 0; w0 < nw; w0 += 32) each_hit_of(w0 + lane < nw ? row[w0 + lane] : make_uint2(0u, 0u), w0, nw, kept, lane, f);
 }
 // The reverse of the edge (i, j) that is hit `rank` of its row, and the pair of the two: from j's row at the word of i (local index il).
 // `at`: first edge, kept edges, lower ones among them and pairs before of a row.  Not ok where the list holds no plan (cut short, or sizes
