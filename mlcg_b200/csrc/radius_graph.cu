@@ -2487,6 +2487,24 @@ __device__ __forceinline__ int64_t structure_at(const int64_t *__restrict__ ptr,
     return lo;
 }
 
+// The same with its boundaries, where structures are of similar sizes in one look at the 32 boundaries around the one that the point's place
+// suggests (three latencies otherwise, 18.2 -> 17.0 us for 512 x 100 points).
+__device__ __forceinline__ void structure_near(const int64_t *__restrict__ ptr, int64_t B, int64_t i, float per_point, int lane, int64_t &b, int64_t &lo,
+                                               int64_t &hi) {
+    const int64_t guess = (int64_t)((float)i * per_point) - 15, base = max(min(guess, B - 31), (int64_t)0);
+    const int64_t p = ptr[min(base + lane, B)];
+    const int c = __popc(__ballot_sync(0xffffffffu, p <= i));          // (boundaries ascend)
+    if (c > 0 && c < 32 && base + c <= B) {
+        b = base + c - 1;
+        lo = __shfl_sync(0xffffffffu, p, c - 1);
+        hi = __shfl_sync(0xffffffffu, p, c);
+    } else {
+        b = structure_at(ptr, B, i, lane);
+        lo = ptr[b];
+        hi = ptr[b + 1];
+    }
+}
+
 // boundaries from the sizes (or as they are), the status words cleared, and whether a structure is too large (as the last one may be where
 // the sizes do not add up)
 __global__ void __launch_bounds__(kScanBlock)
@@ -2523,6 +2541,7 @@ mask_rows_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, int
     const int lane = threadIdx.x & 31;
     const int64_t ngroups = (N + C - 1) / C;
     int sum_deg = 0, sum_upper = 0;                    // (lane 0: of the warp's centres)
+    const float per_point = (float)B / (float)N;
     if constexpr (ALL) {
         pdl_launch_dependents();
         pdl_wait();
@@ -2532,11 +2551,14 @@ mask_rows_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, int
     for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < ngroups; g += ((int64_t)gridDim.x * blockDim.x) >> 5) {
         const int64_t i0 = g * C, i1 = i0 + C < N ? i0 + C : N;
         for (int64_t c0 = i0; c0 < i1;) {              // the centres of one structure among them
-            int64_t b;
-            if constexpr (ALL) b = structure_at(ptr, B, c0, lane);
-            else b = struct_of[c0];
-            const int64_t lo = ptr[b];
-            int64_t hi = ptr[b + 1];
+            int64_t b, lo, hi;
+            if constexpr (ALL) {
+                structure_near(ptr, B, c0, per_point, lane, b, lo, hi);
+            } else {
+                b = struct_of[c0];
+                lo = ptr[b];
+                hi = ptr[b + 1];
+            }
             if (ALL && hi > N) hi = N;
             if (ALL && hi <= c0) {                     // (sizes that do not add up to N: points of no structure)
                 if (lane < (int)(i1 - c0)) { deg[c0 + lane] = upper[c0 + lane] = 0; struct_of[c0 + lane] = (int32_t)b; }
@@ -2617,8 +2639,10 @@ mask_rows_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, int
 __global__ void __launch_bounds__(kScanBlock)
 rows_scan_kernel(const int32_t *__restrict__ deg, const int32_t *__restrict__ upper, const int2 *__restrict__ parts, int64_t N, int64_t *__restrict__ offsets,
                  int4 *__restrict__ seg, const int32_t *__restrict__ header, Publish pub) {
-    static_assert(kScanBlock == 1024, "32 parts per block");
-    __shared__ int64_t s_warp[33];
+    static_assert(kScanBlock == 1024, "32 parts per block, 32 warps");
+    __shared__ int64_t s_before[2][32];                // sums of the parts before this block, by warp: degrees, upper degrees
+    __shared__ uint64_t s_own[32];                     // of this block's points: upper degrees above, degrees below (2^20 at most, or parts of a list of fewer than 2^31 edges)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     pdl_wait();
     const bool last = blockIdx.x == gridDim.x - 1;
     pub.cells_known = true;
@@ -2637,10 +2661,31 @@ rows_scan_kernel(const int32_t *__restrict__ deg, const int32_t *__restrict__ up
     }
     const int64_t i = (int64_t)blockIdx.x * kScanBlock + threadIdx.x;
     const int d = i < N ? deg[i] : 0, u = i < N ? upper[i] : 0;
-    int64_t before_d, before_u, total_d;
-    block_exclusive_scan(bd, s_warp, &before_d);
-    block_exclusive_scan(bu, s_warp, &before_u);
-    const int64_t ed = before_d + block_exclusive_scan(d, s_warp, &total_d);
+    // (one barrier: a scan and two sums by warps, then every warp over the warps' results; four scans of the block took 9.3 us for 51 200 points, like this 8.7)
+    const uint64_t own = (uint64_t)(uint32_t)u << 32 | (uint32_t)d;
+    uint64_t inc = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    bd = warp_sum(bd);
+    bu = warp_sum(bu);
+    if (lane == 31) {
+        s_own[warp] = inc;
+        s_before[0][warp] = bd;
+        s_before[1][warp] = bu;
+    }
+    __syncthreads();
+    uint64_t warps = s_own[lane];
+    const uint64_t mine = warps;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t t = __shfl_up_sync(0xffffffffu, warps, o);
+        if (lane >= o) warps += t;
+    }
+    const int64_t before_d = warp_sum(s_before[0][lane]), before_u = warp_sum(s_before[1][lane]);
+    const int64_t total_d = (int64_t)(uint32_t)__shfl_sync(0xffffffffu, warps, 31);
     if (last && threadIdx.x == 0) {                    // (as early as it is known)
         if (header) {
             *reinterpret_cast<volatile int64_t *>(pub.host + 4) = 0;
@@ -2648,7 +2693,8 @@ rows_scan_kernel(const int32_t *__restrict__ deg, const int32_t *__restrict__ up
         }
         offsets[N] = before_d + total_d;
     }
-    const int64_t eu = before_u + block_exclusive_scan(u, s_warp, nullptr);
+    const uint64_t at = __shfl_sync(0xffffffffu, warps - mine, warp) + inc - own;
+    const int64_t ed = before_d + (int64_t)(uint32_t)at, eu = before_u + (int64_t)(at >> 32);
     if (i < N) {
         offsets[i] = ed;
         seg[i] = make_int4((int)ed, d - u, u, (int)eu);      // (read for plans only, which have fewer than 2^31 edges)
