@@ -390,7 +390,8 @@ gemm_tc_rows_pipe_kernel(const float *__restrict__ A, const float *__restrict__ 
 // 32 x 32 part of every tile comes and goes through a box of its own (asynchronous copies and whole 128-byte pieces by its lanes), the
 // four warps of the same rows meet for the rows' largest entry, and all sixteen only at the operand, by arriving at a barrier that a
 // warp waits for which issues the products and fetches the weights.  With the whole tile in one stage and barriers of the CTA at every
-// turn of it (twelve a tile) a tile took 12-15 us: CHAINFIGURES.
+// turn of it (twelve a tile) a launch over 51200 rows (three tiles a CTA)
+// took 45.6 us forward and 42 back; it takes 42.9 and 38.5.
 // A layer in a kernel of its own pays for a launch, barriers and tensor memory, a tile's way in and out.
 struct ChainSmem {
     static constexpr int kWa = 0, kWb = 65536, kStage = 131072, kMisc = 196608;
@@ -514,9 +515,12 @@ gemm_tc_chain2_kernel(const __grid_constant__ ChainMaps maps, const float *__res
         auto piece = [&](int row, int w) { return reinterpret_cast<float4 *>(box + row * 128 + ((w ^ (row & 7)) << 4)); };
         auto own = [&](int w) { return piece(lane, w); };                       // four columns of this thread's row
         // the warp's part of a tile into its box (zeros past the end), once all lanes are past what they had to do there and what leaves has
-        // been read
+        // been read.  The fence is what keeps the copy behind the lanes' reads of what the box held: a __syncwarp() alone says that they
+        // have been issued, and a copy out of the second-level cache can overtake them (one evaluation of 3000 beads in 400 had rows of
+        // the wrong matrix)
         uint32_t loads = 0;
         auto load_box = [&](const CUtensorMap *map, int64_t tile) {
+            fence_async_smem();
             __syncwarp();
             if (lane == 0) {
                 bulk_wait_read<0>();
@@ -579,12 +583,12 @@ gemm_tc_chain2_kernel(const __grid_constant__ ChainMaps maps, const float *__res
                 x[4 * w] = v.x; x[4 * w + 1] = v.y; x[4 * w + 2] = v.z; x[4 * w + 3] = v.w;
             }
             if (LINKED && BWD) {
-                if (link.res) load_box(&maps.m[kMapRes], tile);
                 if (link.vec) {
 #pragma unroll
                     for (int c = 0; c < 32; c++) x[c] = s_bc[col0 + c] * fmaf(-x[c], x[c], 1.f);
                 }
                 const float sc0 = to_operand(x);
+                if (link.res) load_box(&maps.m[kMapRes], tile);      // (behind the last use of what the box held)
                 await_product();
                 if (link.res) wait_box();
                 float v[32];

@@ -308,6 +308,24 @@ def test_a_weight_that_is_not_a_number_reaches_the_results(copies, num_rbf, prec
     assert torch.equal(again["energy"], want["energy"]) and torch.equal(again["forces"], want["forces"])
 
 
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+def test_evaluations_repeat_bit_by_bit(precision):
+    """The node layers' parts of tiles are copied into places that have just been read: a copy that overtakes the reads shows up as rows of
+    the wrong matrix, once in some hundred evaluations of this batch (24 tiles of beads, two blocks)."""
+    torch.manual_seed(4)
+    cut = bnn.CosineCutoff(0.0, 10.0)
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, 128, trainable=False), cut, [128], hidden_channels=128, embedding_size=4, num_filters=128, num_interactions=2)
+    model = bnn.GradientsOut(bnn.set_filter_precision(net.to(DEV).eval(), precision), "forces").eval()
+    pos, batch = random_walk_chain(5, torch.Generator().manual_seed(1), min_dist=3.8).repeat(600, 1).to(DEV), torch.arange(600, device=DEV).repeat_interleave(5)
+    types_, sizes = torch.zeros(3000, dtype=torch.int64, device=DEV), torch.full((600,), 5, device=DEV)
+    step = lambda: model(mlcg_b200.AtomicData(pos=pos, atom_types=types_, batch=batch, n_atoms=sizes)).out["SchNet"]  # noqa: E731
+    want, differs = step(), torch.zeros((), dtype=torch.int64, device=DEV)
+    for _ in range(2000):
+        got = step()
+        differs += (got["forces"] != want["forces"]).any() | (got["energy"] != want["energy"]).any()
+    assert int(differs) == 0
+
+
 @pytest.mark.parametrize("sizes", [[2049], [1500, 1400], [100] * 30])
 def test_room_of_large_batches(sizes):
     """Above 2048 beads the workspace goes by the call before: one that is too small, exact or larger gives the evaluation of a given list."""
