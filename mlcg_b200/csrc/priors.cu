@@ -398,6 +398,7 @@ __device__ __forceinline__ void prior_slices(const A &acc, const PriorSegments &
             } else {
                 for (int u = 0; u < m; u++) steps(u);
             }
+            tc::fence_async_smem();                              // the next copy into this half stays behind the reads of it
             __syncwarp();
             fetch(k + 2);
         }
