@@ -128,6 +128,12 @@ def test_bit_rows_of_whole_batches(sizes, dtype):
     be.check_pending()
 
 
+@pytest.mark.parametrize("sizes", [[1] * 1500 + [700] * 2, [700] * 2 + [1] * 1500, [3] * 17 + [1000] * 2 + [0] * 60, [24] * 31 + [0] * 33 + [25] * 60, [100] * 30 + [0] * 300])
+def test_structures_far_from_where_their_points_suggest(sizes):
+    """The look at the 32 boundaries around a point's share of the batch: structures before, behind and outside of them."""
+    test_bit_rows_of_whole_batches(sizes, np.float32)
+
+
 @pytest.mark.parametrize("how", ["rows shuffled", "rows reversed", "cut in the middle", "upper halves alone", "other centres"])
 def test_a_list_without_a_plan_is_reported_and_stays_inside(how):
     """mlcgb_pair_plan of lists that are not what it takes: status bit 2, and every entry is an index, none of it outside the arrays."""

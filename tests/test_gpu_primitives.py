@@ -314,6 +314,13 @@ def test_two_chained_layers_equal_two_fused_gemms(M):
     get_backend().check_pending()
 
 
+@pytest.mark.parametrize("M", [1, 31, 32, 33, 127, 129, 148 * 128 + 1])
+def test_chained_layers_at_the_edges_of_boxes(M):
+    """A warp's part of a tile comes and goes through a box of 32 rows: one row, the last row of a box and the first of the next, of a tile,
+    and of a CTA's second tile."""
+    test_two_chained_layers_equal_two_fused_gemms(M)
+
+
 @pytest.mark.parametrize("with_perm", [False, True])
 def test_seg_mul_sum_rows_of_every_length(with_perm):
     """The float32 / 128-feature kernel (rows of V through a ring of asynchronous copies, sixteen per warp in flight): rows with

@@ -309,6 +309,30 @@ def test_a_weight_that_is_not_a_number_reaches_the_results(copies, num_rbf, prec
 
 
 @pytest.mark.parametrize("precision", ["fp32", "bf16"])
+@pytest.mark.parametrize("blocks", [1, 2, 3])
+def test_few_tiles_of_pairs_in_two_ctas_each(blocks, precision):
+    """With a tile of pairs for every second SM or less, values and derivatives of a tile go to two CTAs: 31 beads make 465 pairs (four tiles),
+    twenty times as many 73 tiles, forty times 146.  The same structure has the same numbers in each, but for the order in which the parts
+    of a bead's 30 edges are added up, which goes by the size of the batch: 30 roundings of the largest partial sum, taken as 32 times
+    the largest force."""
+    torch.manual_seed(blocks)
+    cut = bnn.CosineCutoff(0.0, 60.0)
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, 64, trainable=False), cut, [128], hidden_channels=128, embedding_size=4, num_filters=128, num_interactions=blocks)
+    model = bnn.GradientsOut(bnn.set_filter_precision(net.to(DEV).eval(), precision), "forces").eval()
+    one, types_ = torch.rand(31, 3, generator=torch.Generator().manual_seed(7)).mul(14.0).to(DEV), (torch.arange(31) % 4).to(DEV)
+    got = []
+    for copies in (1, 20, 40):
+        batch, sizes = torch.arange(copies, device=DEV).repeat_interleave(31), torch.full((copies,), 31, device=DEV)
+        out = model(mlcg_b200.AtomicData(pos=one.repeat(copies, 1), atom_types=types_.repeat(copies), batch=batch, n_atoms=sizes)).out["SchNet"]
+        forces = out["forces"].view(copies, 31, 3)
+        assert torch.equal(forces, forces[:1].expand_as(forces)) and torch.equal(out["energy"], out["energy"][:1].expand_as(out["energy"]))
+        got.append((out["energy"][0], forces[0]))
+    for energy, forces in got[1:]:
+        assert float((forces - got[0][1]).abs().max()) <= 30 * 2.0 ** -24 * 32 * float(got[0][1].abs().max())
+        assert torch.allclose(energy, got[0][0], rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
 def test_evaluations_repeat_bit_by_bit(precision):
     """The node layers' parts of tiles are copied into places that have just been read: a copy that overtakes the reads shows up as rows of
     the wrong matrix, once in some hundred evaluations of this batch (24 tiles of beads, two blocks)."""
