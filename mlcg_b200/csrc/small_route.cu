@@ -308,12 +308,13 @@ __global__ void __launch_bounds__(kST, 1) small_block_kernel(const __grid_consta
     T t(small_smem, SmallSmem<RT>::kX, p.N);
     constexpr bool kLast = KIND == kSmFwdLast || KIND == kSmTanLast;
     t.fetch_all(p.w, kLast ? p.Wh : 128);
-    // What does not come from the kernel in front is read before the wait for it, a latency of the second-level cache each: biases and the
+    // What does not come from the kernel in front is read before the wait for it, a latency of the second-level cache each (the first-level
+    // cache may hold what lay there in a call before): biases and the
     // lists of the first tile (the kernel in front began behind those that made the lists).  What does, and is wanted after a layer,
     // is read under the aggregation (64 x 10 beads replayed: 64 -> 60.5 us).
     constexpr bool kForward = KIND == kSmFwd || KIND == kSmFwdLast;
-    const float b2 = kForward ? p.b2[t.c] : 0.f, b3 = kForward ? p.b3[t.c] : 0.f;
-    const float bh = KIND == kSmFwdLast && t.c < p.Wh ? p.bh[t.c] : 0.f, wo = kLast && t.c < p.Wh ? p.wo[t.c] : 0.f;
+    const float b2 = kForward ? __ldcg(p.b2 + t.c) : 0.f, b3 = kForward ? __ldcg(p.b3 + t.c) : 0.f;
+    const float bh = KIND == kSmFwdLast && t.c < p.Wh ? __ldcg(p.bh + t.c) : 0.f, wo = kLast && t.c < p.Wh ? __ldcg(p.wo + t.c) : 0.f;
     t.n0 = (int64_t)blockIdx.x * RT;
     SmallEdges ed = small_edges(p, t);
     pdl_wait();
@@ -711,7 +712,8 @@ small_finish_kernel(const float *__restrict__ pos, const float *__restrict__ d, 
     }
     const int64_t n = (int64_t)blockIdx.x * kNodes + warp / WPN;
     const bool mine = n < N;
-    // (lists, distances and positions lie there long before the kernel in front is done)
+    // (lists, distances and positions lie there long before the kernel in front is done.  All of them past the first-level cache, as in
+    // small_edges(): a program that moves its positions in place leaves other coordinates at the same addresses)
     int64_t k0 = 0, k1 = 0;
     int32_t my_j = 0, my_p = 0, my_t = 0;
     float my_d = 0.f, x = 0.f, y = 0.f, z = 0.f;
@@ -720,9 +722,10 @@ small_finish_kernel(const float *__restrict__ pos, const float *__restrict__ d, 
         my_p = __ldcg(pair_of + k);
         if (s) my_t = __ldcg(twin + k);
         my_d = __ldcg(d + k);
-        x = pos[3 * n] - pos[3 * (int64_t)my_j];
-        y = pos[3 * n + 1] - pos[3 * (int64_t)my_j + 1];
-        z = pos[3 * n + 2] - pos[3 * (int64_t)my_j + 2];
+        const float *pi = pos + 3 * n, *pj = pos + 3 * (int64_t)my_j;
+        x = __ldcg(pi) - __ldcg(pj);
+        y = __ldcg(pi + 1) - __ldcg(pj + 1);
+        z = __ldcg(pi + 2) - __ldcg(pj + 2);
     };
     if (mine) {
         const int64_t b0 = __ldcg(ptr + n), b1 = __ldcg(ptr + n + 1), per = (b1 - b0 + WPN - 1) / WPN;

@@ -166,6 +166,51 @@ def test_recordings_of_one_model_stand_by_themselves():
     assert all(bool((j == 7).all()) for j in junk)
 
 
+@pytest.mark.parametrize("sizes", [[73], [10] * 64, [268] * 8])
+@pytest.mark.parametrize("blocks", [1, 2])
+def test_positions_and_biases_written_in_place_between_evaluations(sizes, blocks):
+    """One buffer of positions and one set of biases, overwritten between replays and between plain evaluations: kernels that start early
+    read what lies there now, not what an evaluation before has left in a cache."""
+    torch.manual_seed(blocks)
+    cut = bnn.CosineCutoff(0.0, 9.0)
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, 32, trainable=False), cut, [128], embedding_size=4, num_interactions=blocks)
+    model = bnn.GradientsOut(net.to(DEV), "forces").eval()
+    n, gen = sum(sizes), torch.Generator().manual_seed(len(sizes))
+    frames = [torch.cat([random_walk_chain(k, gen, min_dist=3.0) for k in sizes]).to(DEV) for _ in range(3)]
+    biases = [[torch.randn(p.shape, generator=gen).mul(0.1).to(DEV) for name, p in net.named_parameters() if name.endswith("bias")] for _ in frames]
+    here, kept = torch.empty(n, 3, device=DEV), [p for name, p in net.named_parameters() if name.endswith("bias")]
+    batch = torch.arange(len(sizes), device=DEV).repeat_interleave(torch.tensor(sizes, device=DEV))
+    make = lambda pos: mlcg_b200.AtomicData(pos=pos, atom_types=torch.arange(n, device=DEV) % 4, batch=batch, n_atoms=torch.tensor(sizes, device=DEV))  # noqa: E731
+
+    def write(k):
+        here.copy_(frames[k])
+        with torch.no_grad():
+            torch._foreach_copy_(kept, biases[k])
+
+    want = []
+    for k, frame in enumerate(frames):
+        write(k)
+        torch.cuda.synchronize()
+        out = model(make(frame.clone())).out["SchNet"]
+        want.append((out["energy"].clone(), out["forces"].clone()))
+        torch.cuda.synchronize()
+    field = None
+    if n >= 128:                            # (the fewest beads that a recording takes)
+        bnn.set_edge_capacity(model, 40 * n)
+        field = mlcg_b200.GraphedForceField(model, make(frames[0].clone()))
+        bnn.set_edge_capacity(model, None)
+    wrong = torch.zeros((), dtype=torch.int64, device=DEV)
+    for turn in range(300):
+        k = turn % 3
+        write(k)
+        out = model(make(here)).out["SchNet"]
+        pairs = [(out["energy"], out["forces"])] + ([] if field is None else [field(here)])
+        for e, f in pairs:
+            wrong += (e != want[k][0]).any() | (f != want[k][1]).any()
+    assert int(wrong) == 0
+    get_backend().check_pending()
+
+
 @pytest.mark.parametrize("blocks", [1, 2])
 def test_large_batches_with_nodes_of_every_degree(blocks):
     """Above the small batches' limit the last dot products are taken per pair: beads without neighbours, with one, and with several
