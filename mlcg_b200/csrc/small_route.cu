@@ -533,7 +533,8 @@ small_start_kernel(const float *__restrict__ pos, const int64_t *__restrict__ ty
     extern __shared__ float4 small_smem[];
     constexpr int RT = 8;
     SmallTile<RT> t(small_smem, SmallSmem<RT>::kX, N);
-    t.fetch(0, W1, 128);
+    // (a CTA of edges alone, where there are more than 64 to a bead, brings nothing: nothing would wait for it before the CTA is gone)
+    if ((int64_t)blockIdx.x * RT < N) t.fetch(0, W1, 128);
     pdl_wait();
     pdl_launch_dependents();
     for (int64_t e = (int64_t)blockIdx.x * kST + threadIdx.x; e < E; e += (int64_t)gridDim.x * kST) {
