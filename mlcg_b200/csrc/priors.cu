@@ -386,7 +386,12 @@ __device__ __forceinline__ void prior_slices(const A &acc, const PriorSegments &
         fetch(1);
         for (int k = 0; k < stages; k++) {
             const int half = (turn + k) & 1, m = h.y - (part + k * parts) * S::kSteps;
-            if (!failed && !tc::mbar_wait(bars + 8 * half, (uint32_t)(turn + k) >> 1 & 1u)) failed = true;
+            // (a copy that does not arrive: what lies there are no offsets.  The other half's is waited for too, so that none is on its way when the block leaves)
+            if (!__all_sync(0xffffffffu, tc::mbar_wait(bars + 8 * half, (uint32_t)(turn + k) >> 1 & 1u))) {
+                failed = true;
+                if (k + 1 < stages) tc::mbar_wait(bars + 8 * (half ^ 1), (uint32_t)(turn + k + 1) >> 1 & 1u);
+                return;
+            }
             const char *in = ring + half * kSliceStage<T>;
             const auto steps = [&](int u) {
                 const V *par = reinterpret_cast<const V *>(in + S::kSteps * 256) + u * 32 + lane;
@@ -818,7 +823,7 @@ prior_all_kernel(const __grid_constant__ PriorSegments seg, int parts, int term_
     pdl_wait();
     const int block = (int)blockIdx.x - before, blocks = (int)gridDim.x - term_blocks;
     for (int s = 0; s < seg.n; s++) {
-        if (seg.n_slices[s] == 0) continue;
+        if (seg.n_slices[s] == 0 || failed) continue;
         if (seg.kind[s] == 0) prior_slices<0, T>(acc, seg, s, parts, beads, N, B, status, block, blocks, ring, bars, turn, failed);
         else prior_slices<3, T>(acc, seg, s, parts, beads, N, B, status, block, blocks, ring, bars, turn, failed);
     }
