@@ -298,6 +298,7 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
     if (F != 128 || H > 128 || H2 > 128 || Wh > 128 || (H & 3) || (H2 & 3) || (Wh & 3) || L < 1) return MLCGB_E_LIMIT;
     if (!pos || !types || !offsets || !w->embedding || !w->blocks || !w->head_W || !w->head_b || !w->head_out || !workspace) return MLCGB_E_ARG;
     if (E > 0 && ((!row0 && !graph) || !row1 || (!sel && !graph) || !pair_of || !twin || 2 * P != E)) return MLCGB_E_ARG;
+    if ((uintptr_t)w->embedding & 15) return MLCGB_E_LIMIT;                  // (its rows are read in pieces of 16 bytes)
     const SchnetLayout lay = schnet_layout(N, E, P, H, F, H2, Wh, L);
     if (workspace_bytes < (size_t)lay.total * sizeof(float)) return MLCGB_E_WORKSPACE;
     float *ws = (float *)workspace;
@@ -319,7 +320,7 @@ static int schnet_eval_impl(const void *pos, const int64_t *types, const int64_t
                                               w->blocks[k].filter_b1, w->blocks[k].filter_w2, F, precision, W + (k - l) * lay.wstride, nullptr, status, stream);
         return rf;
     };
-    if (N <= kSmallNodes && L <= kMaxBlocks && H == 128 && H2 == 128) {      // one launch per link of the chain (small_route.cu)
+    if (H == 128 && H2 == 128 && small_route(N, w)) {                        // one launch per link of the chain (small_route.cu)
         SmallForward f = {};
         f.pos = (const float *)pos; f.types = types; f.row0 = row0; f.row1 = row1; f.pair_of = pair_of; f.ptr = offsets;
         f.N = N; f.E = E; f.B = B; f.w = w; f.d = d; f.W = ws + lay.W; f.Wd = grad_pos ? ws + lay.Wd : nullptr; f.wstride = lay.wstride;

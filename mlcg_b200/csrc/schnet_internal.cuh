@@ -67,6 +67,14 @@ int filter_wgrad_parts(int64_t P, int64_t num_blocks);      // partial sums per 
 //   step        407 : 525  493 : 566  570 : 590  660 : 647  803 : 696
 // The line lies where a third pass begins; the routes meet at about 2800 beads.
 constexpr int64_t kSmallNodes = 2368;
+// The chain of small_route.cu takes a batch (of a network whose widths are 128).  It brings its matrices in pieces of 16 bytes, so they have to lie on
+// such boundaries; weights that do not (parts of a larger buffer, say) take the kernels of larger batches, which convert them value by value.
+inline bool small_route(int64_t N, const mlcgb_schnet_weights *w) {
+    if (N > kSmallNodes || w->num_blocks < 1 || w->num_blocks > kMaxBlocks || !w->blocks) return false;
+    uintptr_t at = (uintptr_t)w->head_W;
+    for (int64_t l = 0; l < w->num_blocks; l++) at |= (uintptr_t)w->blocks[l].lin1_w | (uintptr_t)w->blocks[l].lin2_w | (uintptr_t)w->blocks[l].lin_w;
+    return (at & 15) == 0;
+}
 struct SmallForward {                      // per node unless said otherwise; NULL: not wanted
     const float *pos;
     const int64_t *types;
@@ -98,8 +106,7 @@ struct SmallGraph {
 };
 inline size_t small_graph_scratch(int64_t N) { return (size_t)N * ((N + 31) / 32) * 8 + (size_t)N * 8 + 256; }
 inline bool small_graph_ok(int64_t N, int64_t B, const mlcgb_schnet_weights *w) {
-    return N > 0 && B > 0 && N <= kMaskNodes && N <= kSmallNodes && B <= kMaskStructs && w->hidden == 128 && w->filters == 128 && w->conv_out == 128 &&
-           w->num_blocks >= 1 && w->num_blocks <= kMaxBlocks;
+    return N > 0 && B > 0 && N <= kMaskNodes && B <= kMaskStructs && w->hidden == 128 && w->filters == 128 && w->conv_out == 128 && small_route(N, w);
 }
 int small_graph_start(const SmallForward &f, const SmallGraph &g, cudaStream_t st);    // graph, distances, embedding, lin1 of the first block
 // interaction.cu: mlcgb_schnet_energy_forces / _eval_counted (grad_sign -1 / 1) behind it

@@ -190,7 +190,7 @@ int mlcgb::schnet_train_forward(const void *pos, const int64_t *types, const int
     if (!rbf || !w || N <= 0 || B <= 0 || E <= 0 || 2 * P != E) return MLCGB_E_ARG;
     if (!pos || !types || !struct_ptr || !row0 || !row1 || !offsets || !sel || !pair_of || !twin || !workspace || !energy || !grad_pos || !status)
         return MLCGB_E_ARG;
-    if (!train_supported(w, rbf->num_rbf)) return MLCGB_E_LIMIT;
+    if (!train_supported(w, rbf->num_rbf) || ((uintptr_t)w->embedding & 15)) return MLCGB_E_LIMIT;      // (the table's rows are read in pieces of 16 bytes)
     const int64_t Wh = w->head_width, L = w->num_blocks;
     const TrainForward o = train_forward_layout(N, E, P, Wh, L);
     if (workspace_bytes < (size_t)o.total * sizeof(float)) return MLCGB_E_WORKSPACE;
@@ -205,7 +205,7 @@ int mlcgb::schnet_train_forward(const void *pos, const int64_t *types, const int
         return filter_vd_blocks(d, P, nullptr, sel, rbf, conv_cutoff_kind, conv_lower, conv_upper, w->blocks + l, n, 0, ws + o.W + l * o.wstride,
                                 ws + o.Wd + l * o.wstride, ws + o.Hs + l * o.hstride, ws + o.Zs + l * o.hstride, ws + o.zmax + l, image(3 * L + 1 + 2 * l), status, st);
     };
-    if (N <= kSmallNodes) {
+    if (small_route(N, w)) {
         const SmallForward f = small_view(o, ws, pos, types, row0, row1, pair_of, offsets, N, E, B, w, status);
         int rs = small_start(f, st);
         if (!rs) rs = filters(0, L);
@@ -292,7 +292,7 @@ int mlcgb_schnet_train_backward(const int64_t *types, const int64_t *struct_ptr,
     if (rc) return rc;
     ChainScope chain;
     float *yb = ws + v.yb, *gy = ws + v.gy, *r = ws + v.r;
-    if (N <= kSmallNodes) {
+    if (small_route(N, w)) {
         const SmallForward f = small_view(o, const_cast<float *>(fw), pos, types, row0, row1, pair_of, offsets, N, E, B, w, status);
         SmallBackward sb = {};
         sb.dd = dd; sb.gE = (const float *)gE; sb.struct_ptr = struct_ptr; sb.yb = yb; sb.gy = gy; sb.r = r;
@@ -304,7 +304,7 @@ int mlcgb_schnet_train_backward(const int64_t *types, const int64_t *struct_ptr,
         sb.xb[0] = xb0;
         if ((rc = small_backward(f, sb, st))) return rc;
     } else {
-        const uint8_t *images = ((uintptr_t)fw & 15) == 0 ? (const uint8_t *)(fw + o.images) : nullptr;
+        const uint8_t *images = N > kSmallNodes && ((uintptr_t)fw & 15) == 0 ? (const uint8_t *)(fw + o.images) : nullptr;
         auto image = [&](int64_t k) { return images ? images + k * kWeightImage : nullptr; };
         // ---- along the tangent
         for (int64_t l = 0; l < L; l++) {

@@ -379,7 +379,8 @@ class SchNet(torch.nn.Module):
         packed = self.__dict__.get("_mlcgb_packed")
         if packed is not None and packed[0] == key:
             return packed[1]
-        ok = all(t is None or (t.is_cuda and t.dtype == torch.float32) for t in tensors)
+        # (rows of the embedding table are read in pieces of 16 bytes)
+        ok = all(t is None or (t.is_cuda and t.dtype == torch.float32) for t in tensors) and tensors[0].data_ptr() % 16 == 0
         H = self.embedding_layer.embedding_dim
         blocks = list(self.interaction_blocks)
         F, H2, Wh = blocks[0].conv.lin1.out_features, blocks[0].conv.lin2.out_features, self.output_network.layers[0].out_features
