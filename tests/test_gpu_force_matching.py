@@ -46,6 +46,51 @@ def _reference(net, kind, upper, L, pos, types_, batch, B, loss_of):
     return e.detach(), f.detach(), loss.detach(), dict(zip(sorted(names), grads))
 
 
+@pytest.mark.parametrize("kind,R,upper,L,sizes,head,energies", [
+    ("expnormal", 128, 10.0, 3, [73] * 6, 128, False),       # several tiles of pairs and nodes
+    ("gaussian", 50, 30.0, 2, [10] * 13, 128, True),         # a basis narrower than half a tile, energies in the loss
+    ("gaussian", 65, 9.0, 1, [5, 40, 23], 64, True),         # one block (no tangent into it), a narrow output network
+    ("expnormal", 20, 12.0, 2, [2], 128, False),             # one pair
+    ("expnormal", 64, 8.0, 3, [129, 1, 17], 32, True),       # a bead without neighbours
+    ("expnormal", 100, 11.0, 2, [300], 128, False),
+    ("gaussian", 50, 8.0, 2, [74] * 32 + [9], 96, True),     # more beads than the small route takes
+])
+def test_step_against_float64(kind, R, upper, L, sizes, head, energies):
+    net, pos, types_, batch, target = _setup(kind, R, upper, L, sizes, head, 3)
+    B = len(sizes)
+    loss_of = lambda e, f: ((f - target.to(f)) ** 2).mean() + (0.01 * (e ** 2).mean() if energies else 0.0)  # noqa: E731
+    e_x, f_x, loss_x, g_x = _reference(net, kind, upper, L, pos, types_, batch, B, loss_of)
+    net = net.to(DEV).train()
+    assert net._whole_model_setup(pos.to(DEV), training=True) is not None
+    data = lambda: mlcg_b200.AtomicData(pos=pos.to(DEV), atom_types=types_.to(DEV), batch=batch.to(DEV), n_atoms=torch.tensor(sizes).to(DEV))  # noqa: E731
+    out = bnn.GradientsOut(net, "forces").train()(data()).out["SchNet"]
+    assert type(out["forces"].grad_fn).__name__ == "SchNetForceMatchingBackward"
+    loss = loss_of(out["energy"], out["forces"])
+    loss.backward()
+    assert float((out["energy"].detach().cpu().double() - e_x).abs().max()) < 1e-5 * float(e_x.abs().max() + 1e-3)
+    assert float((out["forces"].detach().cpu().double() - f_x).abs().max()) < 1e-4
+    assert abs(float(loss.detach()) - float(loss_x)) < 1e-5 * float(loss_x)
+    for n, p in net.named_parameters():
+        g = g_x[n]
+        if g is None:
+            continue
+        assert float((p.grad.cpu().double() - g).abs().max()) <= 2e-5 * float(g.abs().max()) + 1e-9, n
+
+
+@pytest.mark.parametrize("beads", [74, 75, 148, 149, 222, 223, 592, 593, 888, 889, 1184, 1185, 1776, 1777, 2368])
+def test_tiles_of_every_height(beads):
+    """Small batches run in tiles of 1 to 8 rows by their number of beads: both sides of every line, forward and backward."""
+    sizes = [37] * (beads // 37) + [beads % 37] * (beads % 37 > 0)
+    test_step_against_float64("expnormal", 20, 7.0, 2, sizes, 128, True)
+
+
+@pytest.mark.parametrize("beads", [73, 200])
+def test_more_edges_than_the_tiles_of_beads_have_threads(beads):
+    """Above 64 edges a bead the first launch of a small step has CTAs of edges alone, which bring no weights: every pair of one chain."""
+    assert beads * (beads - 1) > 512 * ((beads + 7) // 8)
+    test_step_against_float64("gaussian", 64, {73: 40.0, 200: 95.0}[beads], 2, [beads], 128, True)
+
+
 def test_higher_derivatives_and_position_gradients_take_the_composable_operators():
     net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, [12, 9], 128, 5)
     net = net.to(DEV)
