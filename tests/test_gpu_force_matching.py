@@ -91,6 +91,44 @@ def test_more_edges_than_the_tiles_of_beads_have_threads(beads):
     test_step_against_float64("gaussian", 64, {73: 40.0, 200: 95.0}[beads], 2, [beads], 128, True)
 
 
+@pytest.mark.parametrize("copies,head", [(3789, 128), (7579, 96)])
+def test_linked_layers_over_several_tiles_each(copies, head):
+    """More tiles of 128 beads than the chip has SMs: 18945 beads, the last tile one row high, and two tiles for each and seven beads.  The same
+    structure over and over has the same energies and forces in every copy and every call, those of one copy alone, and the gradients of
+    one copy alone, in steps and in evaluations."""
+    net, pos, types_, _, target = _setup("expnormal", 32, 9.0, 3, [5], head, 11)
+    net = net.to(DEV)
+    model, n = bnn.GradientsOut(net, "forces"), 5
+
+    def data(k):
+        return mlcg_b200.AtomicData(pos=pos.repeat(k, 1).to(DEV), atom_types=types_.repeat(k).to(DEV), batch=torch.arange(k, device=DEV).repeat_interleave(n),
+                                    n_atoms=torch.full((k,), n, device=DEV))
+
+    def step(k):
+        model.train()
+        net.zero_grad()
+        out = model(data(k)).out["SchNet"]
+        assert type(out["forces"].grad_fn).__name__ == "SchNetForceMatchingBackward"
+        (((out["forces"] - target.repeat(k, 1).to(DEV)) ** 2).sum() / k + 0.01 * (out["energy"] ** 2).sum() / k).backward()
+        return out["energy"].detach().clone(), out["forces"].detach().clone(), [p.grad.clone() for p in net.parameters()]
+
+    def evaluation(k):
+        out = model.eval()(data(k)).out["SchNet"]
+        return out["energy"].clone(), out["forces"].clone()
+
+    for call, times in ((evaluation, 40), (step, 10)):
+        one, many = call(1), call(copies)
+        assert torch.equal(many[0], many[0][:1].expand(copies)) and torch.equal(many[1].view(copies, n, 3), many[1][:n].expand(copies, n, 3))
+        # (either within 1e-5 and 1e-4 of float64, and gradients within 2e-5 of the largest, as above)
+        assert torch.allclose(many[0][:1], one[0], rtol=2e-5, atol=2e-5) and float((many[1][:n] - one[1]).abs().max()) < 2e-4
+        for a, b in zip(*(x[2] if len(x) > 2 else [] for x in (many, one))):
+            assert float((a - b).abs().max()) <= 4e-5 * float(b.abs().max()) + 1e-9
+        for _ in range(times):
+            got = call(copies)
+            assert torch.equal(got[0], many[0]) and torch.equal(got[1], many[1])
+            assert all(torch.equal(a, b) for a, b in zip(*(x[2] if len(x) > 2 else [] for x in (got, many))))
+
+
 def test_higher_derivatives_and_position_gradients_take_the_composable_operators():
     net, pos, types_, batch, target = _setup("expnormal", 32, 9.0, 2, [12, 9], 128, 5)
     net = net.to(DEV)

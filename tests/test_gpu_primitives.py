@@ -321,6 +321,48 @@ def test_chained_layers_at_the_edges_of_boxes(M):
     test_two_chained_layers_equal_two_fused_gemms(M)
 
 
+@pytest.mark.parametrize("M", [1, 31, 32, 33, 129, 148 * 128 + 1])
+def test_tangent_layers_at_the_edges_of_boxes(M):
+    """mlcgb_gemm_tc_chain2_tangent, along the tangent with and without a residual and back, against float64; and the same bits in twenty
+    launches one behind the other."""
+    gen, be = torch.Generator().manual_seed(M), get_backend()
+    r = lambda *s: torch.randn(*s, generator=gen).to(DEV)  # noqa: E731
+    A, X, a, gu, Wa, Wb = r(M, 128), r(M, 128), torch.tanh(r(M, 128)), r(M, 128), r(128, 128) / 11, r(128, 128) / 11
+    status = be._sticky_status(A.device)
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def call(reverse, A, aux, q):
+        mid, C = torch.empty_like(A), torch.empty_like(A)
+        code = be.lib.mlcgb_gemm_tc_chain2_tangent(reverse, A.data_ptr(), Wa.data_ptr(), Wb.data_ptr(), a.data_ptr(), None if reverse else gu.data_ptr(),
+                                                   None if aux is None else aux.data_ptr(), M, q.data_ptr(), mid.data_ptr(), C.data_ptr(), status.data_ptr(), stream)
+        assert code == 0
+        return mid, C
+
+    def near(got, want):                      # (as a single layer is held to above; for the second of two, twice that)
+        assert float((got.double() - want).abs().max()) < 1e-5 * max(1.0, float(want.abs().max()))
+
+    a64, one = a.double(), 1 - a.double() ** 2
+    u = A.double() @ Wa.double().t()
+    for aux in (X, None):
+        q = torch.empty_like(A)
+        mid, C = call(0, A, aux, q)
+        near(mid, one * u)
+        near(q, -2 * a64 * u * gu.double())
+        near(C, (0 if aux is None else X.double()) + (one * u) @ Wb.double().t())
+        for _ in range(20):
+            again = torch.empty_like(q)
+            got = call(0, A, aux, again)
+            assert torch.equal(again, q) and torch.equal(got[0], mid) and torch.equal(got[1], C)
+    mid, C = call(1, A, None, X)              # (X in the place of q)
+    want = (A.double() @ Wa.double()) * one + X.double()
+    near(mid, want)
+    near(C, want @ Wb.double())
+    for _ in range(20):
+        got = call(1, A, None, X)
+        assert torch.equal(got[0], mid) and torch.equal(got[1], C)
+    be.check_pending()
+
+
 @pytest.mark.parametrize("with_perm", [False, True])
 def test_seg_mul_sum_rows_of_every_length(with_perm):
     """The float32 / 128-feature kernel (rows of V through a ring of asynchronous copies, sixteen per warp in flight): rows with

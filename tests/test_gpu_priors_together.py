@@ -73,6 +73,24 @@ def test_slices_at_the_ends_of_stages(n, B, dtype):
         assert torch.equal(each[k][0], again[k][0]) and torch.equal(each[k][1], again[k][1]), k
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_priors_repeat_bit_by_bit(dtype):
+    """Steps of pair terms are copied into places that have just been read: a copy that overtakes the reads shows up as terms of another step, now
+    and then.  (Sums are integers by default: nothing else may differ.)"""
+    data, priors = prior_setup(150, 20, 4, torch.Generator().manual_seed(5))
+    with torch.no_grad():                     # (its list is sliced)
+        priors["repulsion"].sigma.copy_(0.5 * (priors["repulsion"].sigma + priors["repulsion"].sigma.t()))
+    data.pos = torch.cat([random_walk_chain(150, torch.Generator().manual_seed(k), min_dist=3.0) for k in range(20)]).to(dtype)
+    data, priors = data.to(DEV), [p.to(DEV).eval() for p in priors.values()]
+    step = lambda: _evaluate_together(priors, data, forces=True)[0]  # noqa: E731
+    want, differs = {k: (v[0].clone(), v[1].clone()) for k, v in step().items()}, torch.zeros((), dtype=torch.int64, device=DEV)
+    assert any(p._cached_list(data)[4] is not None for p in priors)
+    for _ in range(1000):
+        for k, v in step().items():
+            differs += (v[0] != want[k][0]).any() | (v[1] != want[k][1]).any()
+    assert int(differs) == 0
+
+
 def test_a_sliced_list_is_kept_once():
     """The slices of a pair list take the place of the 32-bit list and of the gathered parameters: 6 bytes a term and the padding."""
     data, priors = prior_setup(150, 20, 4, torch.Generator().manual_seed(3))

@@ -418,6 +418,35 @@ def test_few_tiles_of_pairs_in_two_ctas_each(blocks, precision):
         assert torch.allclose(energy, got[0][0], rtol=1e-5, atol=1e-5)
 
 
+@pytest.mark.parametrize("blocks", [1, 2, 3])
+def test_filter_rows_of_two_ctas_are_those_of_one(blocks):
+    """The rows themselves: 40 copies of the 31 beads have 146 tiles of pairs, one CTA for each, and the first copy's rows and derivatives are, bit by bit,
+    those of the copy alone, in two CTAs a tile.  Read from the workspace of a step's forward pass (its arrays lie on 256-byte boundaries:
+    positions, edges, edges, pairs, beads, output network, one per block, then the rows of all blocks and their derivatives)."""
+    from mlcg_b200.autograd import plan_of
+    torch.manual_seed(blocks)
+    cut, head = bnn.CosineCutoff(0.0, 60.0), 64
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, 64, trainable=False), cut, [head], embedding_size=4, num_interactions=blocks).to(DEV).train()
+    one, types_ = torch.rand(31, 3, generator=torch.Generator().manual_seed(7)).mul(14.0).to(DEV), (torch.arange(31) % 4).to(DEV)
+    rows = []
+    for copies in (1, 40):
+        N, P = 31 * copies, 465 * copies
+        data = mlcg_b200.AtomicData(pos=one.repeat(copies, 1), atom_types=types_.repeat(copies), batch=torch.arange(copies, device=DEV).repeat_interleave(31),
+                                    n_atoms=torch.full((copies,), 31, device=DEV))
+        nl = net.neighbor_list(data, 60.0)["SchNet"]
+        plan = plan_of(nl["index_mapping"], N)
+        assert plan.E == 2 * P and N <= 2368
+        state = get_backend().schnet_train_forward(data.pos, data.atom_types, nl["_mlcgb_ptr"], plan, *net._whole_model_setup(data.pos, training=True)[:3])[2]
+        ws = state.tensors[state.places[state.NAMES.index("forward_ws")][0]].view(torch.float32)
+        at, stride = sum((k + 63) // 64 * 64 for k in (3 * N, 2 * P, 2 * P, P, N, N * head, blocks)), (P + 127) // 128 * 128 * 128
+        values, derivatives = (ws[at + k * blocks * stride: at + (k + 1) * blocks * stride].view(blocks, -1, 128)[:, :465] for k in (0, 1))
+        first = plan.half_selection()[:465]
+        rows.append((values.clone(), derivatives.clone(), plan.row0[first].clone(), plan.row1[first].clone()))
+    assert float(rows[0][0].abs().max()) > 0 and float(rows[0][1].abs().max()) > 0
+    assert all(torch.equal(a, b) for a, b in zip(*rows))
+    get_backend().check_pending()
+
+
 @pytest.mark.parametrize("precision", ["fp32", "bf16"])
 def test_evaluations_repeat_bit_by_bit(precision):
     """The node layers' parts of tiles are copied into places that have just been read: a copy that overtakes the reads shows up as rows of
