@@ -6,6 +6,7 @@
 #include "small_graph.cuh"
 #include "tc_common.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace mlcgb {
@@ -198,7 +199,7 @@ prior_kernel(const T *__restrict__ pos, const int64_t *__restrict__ mapping, con
 //   result does not depend on the order in which the threads arrive) and converted afterwards.
 // ------------------------------------------------------------------------------------------------
 constexpr int kSliceWarps = 4, kSliceBlocks = 6;         // of prior_all_kernel; blocks each SM, float (5: 146 us, 7: the same with spills)
-template <typename T> constexpr int kSliceStage = sizeof(T) == 4 ? 3072 : 2304;    // bytes of half the steps on their way, each warp (1536: 149 us instead of 141)
+template <typename T> constexpr int kSliceStage = sizeof(T) == 4 ? 3072 : 2560;    // bytes of half the steps on their way, each warp: four, in float64 two, of a repulsion
 constexpr int kFixedShift = 36;          // fixed point: 2^-36 resolution, +-1.3e8 range
 
 struct PriorSegments {
@@ -1038,9 +1039,21 @@ extern "C" int mlcgb_prior_eval(int n_lists, const mlcgb_prior_list *lists, cons
         auto *sums = (A *)((char *)workspace + prior_bead_bytes(N, dtype));
         A *se = sums, *sg = sums + (int64_t)n_lists * B;
         prior_begin_kernel<T, A><<<grid_for(N > n_sums / 4 ? N : n_sums / 4, 256, 8), 256, 0, st>>>((const T *)pos, batch, N, B, beads, sums, n_sums);
-        // a slice is cut into parts until the chip holds a few rounds of warps (48 each SM); sixteen parts of a step or two at most
-        const int64_t want = r ? (2 * 48 * (int64_t)kNumSM + r - 1) / r : 1;
-        const int parts = (int)(want > 16 ? 16 : want), slice_blocks = r ? grid_for(r * parts, kSliceWarps, 96) : 0,
+        // A slice is cut into parts until the chip holds a warp wherever it has room for one, into two at least (the last round of warps is shorter
+        // then) and into no more than an average slice has stages of copies, or sixteen: a part without a stage looks up its beads for nothing.
+        // us of device time, float32 / float64, aiming at 16, 24, 48 and 96 warps each SM:
+        //   chains          32 x 268    64 x 268    96 x 268    200 x 268   400 x 268    1024 x 73   1024 x 268
+        //   16              14.4, 20.6  17.9, 28.4  20.6, 38.7  35.8, 66.3  66.4, 126.6  25.1, 39.0  136.4, 269.4
+        //   24              20.1, 22.5  20.5, 26.5  21.8, 34.4  34.9, 63.6  59.8, 113.3  25.1, 39.0  136.2, 269.6
+        //   48              20.5, 23.0  26.2, 29.0  22.8, 36.9  36.2, 63.8  60.7, 111.1  32.6, 45.1  136.4, 269.5
+        //   96              20.5, 23.2  28.3, 31.2  32.9, 44.9  42.7, 69.7  69.8, 116.9  39.8, 60.2  134.0, 260.1 (the only one with two parts here)
+        const int64_t want = r ? (kSliceWarps * kSliceBlocks * (int64_t)kNumSM + r - 1) / r : 1;
+        int64_t stages = 1;
+        for (int i = 0; i < n_lists; i++) {
+            const int64_t a_stage = seg.kind[i] == 0 ? PairStages<0, T>::kSteps : PairStages<3, T>::kSteps;
+            if (seg.n_slices[i]) stages = std::max(stages, (seg.steps[i] + seg.n_slices[i] * a_stage - 1) / (seg.n_slices[i] * a_stage));
+        }
+        const int parts = (int)std::min(std::min(std::max(want, (int64_t)2), (int64_t)16), stages), slice_blocks = r ? grid_for(r * parts, kSliceWarps, 96) : 0,
                   term_blocks = v ? grid_for(v, kSliceWarps * 32, 96) : 0;
         if (slice_blocks + term_blocks)
             launch_pdl(prior_all_kernel<T, FIXED>, dim3(slice_blocks + term_blocks), dim3(kSliceWarps * 32), 0, st, seg, parts, term_blocks, beads, N, B, se, sg, status);
