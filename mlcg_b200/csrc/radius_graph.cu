@@ -2531,8 +2531,10 @@ rows_begin_kernel(const int64_t *__restrict__ sizes, int64_t B, int64_t N, int64
     if (threadIdx.x == 0) header[8] = any;
 }
 
+// (float32: 48 registers, as the look at 32 boundaries would take 61 and leave room for four blocks an SM: 20 structures of 1000 points, 625
+// blocks, 24.5 us instead of 21.2)
 template <typename T, bool ALL>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 0)
 mask_rows_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, int32_t *__restrict__ struct_of, const CellParam *__restrict__ cellparam,
                  int64_t N, T r2, int64_t max_nn, int loop, int rule, uint2 *__restrict__ masks, int32_t *__restrict__ deg, int32_t *__restrict__ upper,
                  int32_t *__restrict__ status, int64_t B, int2 *__restrict__ parts) {
