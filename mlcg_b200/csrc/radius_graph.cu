@@ -2450,12 +2450,12 @@ mask_fill_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, int
         const int64_t off = offsets[i];
         const int kept = (int)(offsets[i + 1] - off);
         if (kept == 0) continue;
-        each_hit(masks + ci * words, (hi - lo + 31) >> 5, kept, lane, [&](int rank, int jl) {
+        each_hit<BATCH ? kDense : kDensePlan>(masks + ci * words, (hi - lo + 31) >> 5, kept, lane, [&](int rank, int jl) {
             const int64_t slot = off + rank, j = lo + jl;
             T d2 = T(0);
             if (out.distance) d2 = dist2_rn(pos[3 * ci], pos[3 * ci + 1], pos[3 * ci + 2], pos[3 * j], pos[3 * j + 1], pos[3 * j + 2]);
             emit_edge<T>(out, slot, i, j, b, d2);
-            if (!twin) return;
+            if (BATCH || !twin) return;                // (a list by its batch vector comes without a plan)
             const auto place = pair_place(masks, words, i, i - lo, (int)j, rank, P, at);
             // not a valid plan (a list was cut short): reported, and every index written stays inside its array
             if (!place.ok) atomicOr(sticky, (int)kAsymmetric);
@@ -2756,7 +2756,7 @@ list_distance_kernel(const T *__restrict__ pos, const I *__restrict__ row0, cons
 }
 
 // cellparam NULL: every structure has bit rows
-template <typename T>
+template <typename T, bool PLAN>
 __global__ void __launch_bounds__(256)
 mask_rows_fill_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, const int32_t *__restrict__ struct_of,
                       const CellParam *__restrict__ cellparam, int64_t N, const uint2 *__restrict__ masks, const int4 *__restrict__ seg,
@@ -2767,19 +2767,19 @@ mask_rows_fill_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr
         // (all that hangs on the point alone is asked for at once, its words before it is known how many there are)
         const int b = struct_of[i];
         const int64_t off = offsets[i], next = offsets[i + 1];
-        const int4 si = seg[i];
+        const int4 si = PLAN ? seg[i] : make_int4(0, 0, 0, 0);
         const uint2 mine = masks[i * kMaskWords + lane];
         if (cellparam && cellparam[b].tile != 2) continue;
         const int64_t lo = ptr[b], hi = ptr[b + 1];
         const int n = (int)((hi < N ? hi : N) - lo), il = (int)(i - lo), nw = (n + 31) >> 5, kept = (int)(next - off);
         if (kept == 0) continue;
         static_assert(kMaskWords == 32, "a word of the row per lane");
-        each_hit_of(mine, 0, nw, kept, lane, [&](int rank, int jl) {
+        each_hit_of<PLAN ? kDensePlan : kDense>(mine, 0, nw, kept, lane, [&](int rank, int jl) {
             const int64_t slot = off + rank, j = lo + jl;
             T d2 = T(0);
             if (out.distance) d2 = dist2_rn(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], pos[3 * j], pos[3 * j + 1], pos[3 * j + 2]);
             emit_edge<T>(out, slot, i, j, b, d2);
-            if (!twin) return;
+            if constexpr (!PLAN) return;
             // (a complete list: the reverse is there)
             const uint2 rev = masks[j * kMaskWords + (il >> 5)];
             const int rank_j = (int)rev.x + __popc(rev.y & ((1u << (il & 31)) - 1u));
@@ -3239,9 +3239,11 @@ int mlcgb_graph_finish(const void *pos, int dtype, const int64_t *ptr, int64_t N
                 return mlcgb_pair_plan(row0, row1, offsets, E, N, w + L.upper, L.seg - L.upper, twin, sel, pair_of, sticky_status, stream);
             }
         }
-        if (rows)
-            mask_rows_fill_kernel<scalar_t><<<grid_for(N * 32, 256), 256, 0, st>>>((const scalar_t *)pos, ptr, struct_of, cells ? cellparam : nullptr, N, (const uint2 *)(w + L.masks),
-                                                                                 seg, offsets, out, twin, sel, pair_of);
+        if (rows) {
+            const auto kern = twin ? mask_rows_fill_kernel<scalar_t, true> : mask_rows_fill_kernel<scalar_t, false>;
+            kern<<<grid_for(N * 32, 256), 256, 0, st>>>((const scalar_t *)pos, ptr, struct_of, cells ? cellparam : nullptr, N, (const uint2 *)(w + L.masks), seg, offsets, out,
+                                                        twin, sel, pair_of);
+        }
         distances();
         if (twin && cells)
             return large_plans<false>(row1, seg, struct_of, ptr, cellparam, N > (rows ? kMaskMax : kBruteMax) ? (const int32_t *)(cw + W.group_ptr) + B + 1 : nullptr, rows, N, B,

@@ -124,6 +124,7 @@ __device__ __forceinline__ RowHits row_of_bits(const T *__restrict__ pos, int64_
     const int nlo = sw < 32 ? __shfl_sync(0xffffffffu, nlo0, sw) : __shfl_sync(0xffffffffu, nlo1, sw & 31);
     return {total, nlo, self_hit};
 }
+constexpr int kDense = 16, kDensePlan = 24;        // of each_hit()
 // The k-th set bit of a word that has more than k
 __device__ __forceinline__ int nth_bit(unsigned bits, int k) {
     int at = 0;
@@ -138,16 +139,30 @@ __device__ __forceinline__ int nth_bit(unsigned bits, int k) {
     return at;
 }
 // f(rank, local index) for the first `kept` hits of a row of nw words, 32 consecutive ranks at a time: a lane looks for the word of its rank
-// among the 32 of the warp, and for the bit in it.  (Word by word, the lanes of the word's bits at work, a row took as many turns as it
-// has words with a hit, most lanes idle: 37 structures of up to 700 points in float64 with distances 99 -> 81 us.)
+// among the 32 of the warp, and for the bit in it.  (Word by word, the lanes of the word's bits at work, a row takes as many turns as it
+// has words with a hit, most lanes idle: 37 structures of up to 700 points in float64 with distances 99 -> 81 us.)  Where the words
+// are full the two take the same number of turns and the search is what is left over: rows of more than DENSE hits for each word with one go
+// word by word.  64 structures of 1000 points, float32, us, by ranks alone : by words alone : these lines, a hit in so many of a word's 32,
+//   edges alone (16)       9  297 : 326 : 292      18  469 : 432 : 433      23  555 : 501 : 503      all  728 : 661 : 665
+//   with their plan (24)   9  287 : 381 : 284      18  490 : 579 : 490      23  605 : 672 : 612      all  872 : 850 : 855
 // each_hit_of: of up to 32 words from w0 on, of which lane t holds word w0 + t (whatever it holds beyond the row).
-template <typename F>
+template <int DENSE, typename F>
 __device__ __forceinline__ void each_hit_of(uint2 mine, int w0, int nw, int kept, int lane, F &&f) {
     const bool there = w0 + lane < nw;
     if (!there) mine = make_uint2(0u, 0u);
     const int first = (int)__shfl_sync(0xffffffffu, mine.x, 0), last = min(nw - w0, 32) - 1;
     const int before = there ? (int)mine.x : 0x7fffffff;
     const int end = min(kept, (int)__shfl_sync(0xffffffffu, mine.x + (unsigned)__popc(mine.y), last));
+    unsigned live = __ballot_sync(0xffffffffu, mine.y != 0u);
+    if (end - first > DENSE * __popc(live)) {
+        for (; live; live &= live - 1) {
+            const int w = __ffs(live) - 1;
+            const unsigned bits = __shfl_sync(0xffffffffu, mine.y, w);
+            const int rank = (int)__shfl_sync(0xffffffffu, mine.x, w) + __popc(bits & lanemask_lt());
+            if ((bits >> lane & 1u) && rank < kept) f(rank, (w0 + w) * 32 + lane);
+        }
+        return;
+    }
     for (int k = first; k < end; k += 32) {
         const int rank = k + lane;
         int w = 0;                                 // the last word with no more hits before it than the rank
@@ -161,9 +176,9 @@ __device__ __forceinline__ void each_hit_of(uint2 mine, int w0, int nw, int kept
         if (rank < end) f(rank, (w0 + w) * 32 + nth_bit(bits, rank - b));
     }
 }
-template <typename F>
+template <int DENSE, typename F>
 __device__ __forceinline__ void each_hit(const uint2 *__restrict__ row, int nw, int kept, int lane, F &&f) {
-    for (int w0 = 0; w0 < nw; w0 += 32) each_hit_of(w0 + lane < nw ? row[w0 + lane] : make_uint2(0u, 0u), w0, nw, kept, lane, f);
+    for (int w0 = 0; w0 < nw; w0 += 32) each_hit_of<DENSE>(w0 + lane < nw ? row[w0 + lane] : make_uint2(0u, 0u), w0, nw, kept, lane, f);
 }
 // The reverse of the edge (i, j) that is hit `rank` of its row, and the pair of the two: from j's row at the word of i (local index il).
 // `at`: first edge, kept edges, lower ones among them and pairs before of a row.  Not ok where the list holds no plan (cut short, or sizes

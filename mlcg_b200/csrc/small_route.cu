@@ -671,7 +671,7 @@ small_graph_fill_kernel(const float *__restrict__ pos, const SmallGraph g, int64
         const int off = s_off[i], kept = s_off[i + 1] - off;
         if (kept == 0) continue;
         const float xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
-        each_hit(g.masks + (int64_t)i * words, (n + 31) >> 5, kept, lane, [&](int rank, int jl) {
+        each_hit<kDensePlan>(g.masks + (int64_t)i * words, (n + 31) >> 5, kept, lane, [&](int rank, int jl) {
             const int slot = off + rank, j = lo + jl;
             const float d2 = dist2_rn(xi, yi, zi, pos[3 * j], pos[3 * j + 1], pos[3 * j + 2]);
             const auto place = pair_place(g.masks, words, i, il, j, rank, P, at);

@@ -134,6 +134,30 @@ def test_structures_far_from_where_their_points_suggest(sizes):
     test_bit_rows_of_whole_batches(sizes, np.float32)
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("r", [0.55, 0.7, 0.9, 2.0])
+@pytest.mark.parametrize("sizes", [[31, 32, 33, 64], [2000], [100] * 25, [33, 31] * 40, [1000, 900, 300], [1024, 65, 1024]])
+def test_rows_of_words_from_half_full_to_full(sizes, r, dtype):
+    """Rows with so many hits in a word that they are written word by word, rows just below, and both kinds in one row's words: edges, plans and rows
+    cut inside a word, against the oracle.  (Points of a unit cube; at 2 every pair.)"""
+    rng = np.random.default_rng(len(sizes))
+    ptr = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    pos = rng.random((int(ptr[-1]), 3)).astype(dtype)
+    be, t, p = get_backend(), torch.as_tensor(pos, device=DEV), torch.as_tensor(ptr, device=DEV)
+    batch = torch.repeat_interleave(torch.arange(len(sizes)), torch.tensor(sizes)).to(DEV)
+    want = torch.from_numpy(radius_ref.radius_graph_c(pos, ptr, r, 2000, False, "cluster"))
+    res = be.radius_graph(t, p, r, 2000, False, 1, want_distance=True, want_plan=True)
+    assert torch.equal(res["edge_index"].cpu(), want)
+    twin, sel, pair_of, status = be.pair_plan(res["row0"], res["row1"], res["offsets"], len(pos), fresh_status=True)
+    assert int(status[0]) == 0 and torch.equal(res["twin"], twin) and torch.equal(res["sel"], sel) and torch.equal(res["pair_of"], pair_of)
+    for loop, cap in ((False, 2000), (True, 2000), (False, 45), (True, 17)):
+        cut = torch.from_numpy(radius_ref.radius_graph_c(pos, ptr, r, cap, loop, "cluster"))
+        assert torch.equal(be.radius_graph(t, p, r, cap, loop, 1, want_plan=False)["edge_index"].cpu(), cut)
+        if len(pos) <= 2048:
+            assert torch.equal(be.radius_graph_small(t, batch, r, cap, loop, 1)["edge_index"].cpu(), cut)
+    be.check_pending()
+
+
 @pytest.mark.parametrize("how", ["rows shuffled", "rows reversed", "cut in the middle", "upper halves alone", "other centres"])
 def test_a_list_without_a_plan_is_reported_and_stays_inside(how):
     """mlcgb_pair_plan of lists that are not what it takes: status bit 2, and every entry is an index, none of it outside the arrays."""
