@@ -433,7 +433,7 @@ typedef struct {
     int64_t hidden, filters, conv_out, head_width; /* H, F, H2, width of the output network's hidden layer */
     int64_t num_blocks, num_types;
     const mlcgb_schnet_block *blocks;              /* host array [num_blocks] */
-    const void *embedding;                         /* [num_types, H] */
+    const void *embedding;                         /* [num_types, H], 16-byte aligned (MLCGB_E_LIMIT) */
     const void *head_W, *head_b;                   /* [head_width, H], [head_width] */
     const void *head_out, *head_out_b;             /* [head_width], [1] or NULL */
 } mlcgb_schnet_weights;

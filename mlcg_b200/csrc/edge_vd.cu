@@ -7,8 +7,9 @@
 //   tangent  out[i] = sum_j a[j] W[p] + b[j] (dd[e] W'[p])
 //
 // `force` is the step of the force pass that used to be an aggregation and a backward pass of the filter network: gd of a pair is
-// s[(i,j)] + s[(j,i)], with x = lin1 features and a = gradient of the aggregate.  Bound by the L2: per edge 1.5 KB (force) or
-// 2 KB (tangent) of rows, of which W and W' come from HBM once.
+// s[(i,j)] + s[(j,i)], with x = lin1 features and a = gradient of the aggregate.  Bound by rows in flight
+// and the first-level path: per edge 1.5 KB (force) or 2 KB (tangent) of rows, of which W and W' come from HBM once (force, 1.1 M edges: first
+// level 70 % of its throughput, L2 48 %, memory 65 %, issue slots 54 %).
 #include "schnet_internal.cuh"
 
 #include <type_traits>

@@ -198,8 +198,8 @@ prior_kernel(const T *__restrict__ pos, const int64_t *__restrict__ mapping, con
 //   FIXED: energies and gradients are accumulated as 64-bit fixed-point integers (integer addition is associative: the
 //   result does not depend on the order in which the threads arrive) and converted afterwards.
 // ------------------------------------------------------------------------------------------------
-constexpr int kSliceWarps = 4, kSliceBlocks = 6;         // of prior_all_kernel; blocks each SM, float (5: 146 us, 7: the same with spills)
-template <typename T> constexpr int kSliceStage = sizeof(T) == 4 ? 3072 : 2560;    // bytes of half the steps on their way, each warp: four, in float64 two, of a repulsion
+constexpr int kSliceWarps = 4, kSliceBlocks = 6;         // of prior_all_kernel; blocks each SM, float (5: 144.7 us instead of 133.5 for 1024 chains of 268 beads, 7: 141.6 with spills)
+template <typename T> constexpr int kSliceStage = sizeof(T) == 4 ? 3072 : 2560;    // bytes of half the steps on their way, each warp: four, in float64 two, of a repulsion (1536: 143.8 us instead of 133.5; float64 2304, one: 306 instead of 260)
 constexpr int kFixedShift = 36;          // fixed point: 2^-36 resolution, +-1.3e8 range
 
 struct PriorSegments {
@@ -281,9 +281,9 @@ __device__ __forceinline__ void run_accumulate(const A &acc, int64_t block0, int
 // 16-bit offset.  Energy and gradient stay in registers: one addition per bead and component, no scatter and no reduction across
 // lanes (the reverse terms of the list carry the other half of every pair's gradient).  In the lists of a topology the lanes of a
 // slice meet the same second bead at nearly the same step: a gather of positions is one or two cache lines.
-// Bound by instruction issue (29 a term and warp) beside the stream of terms, 6 bytes each: of 134 us for 72 M terms and three lists of
-// single terms, the stream alone takes 75, with its arithmetic 95, the single terms 20 more, the first and the last launch 20.  With loads
-// two steps ahead in registers 155; with a warp per run in one kernel for all lists (32-bit indices, three 4-byte loads a position, a
+// Bound by the stream of terms, 6 bytes each at half of the memory's rate, and by what its warps do meanwhile (29 instructions a term and warp, 60 %
+// of the issue slots): of 133.5 us for 72 M terms and three lists of single terms the first and the last launch take 12, the stream alone
+// 81, with its arithmetic 94, the single terms 27 more.  With loads two steps ahead in registers 155 (then); with a warp per run in one kernel for all lists (32-bit indices, three 4-byte loads a position, a
 // reduction a run) the pair terms alone took 390.
 __device__ __forceinline__ float inv_sqrt(float x) {
     float y;
@@ -301,7 +301,7 @@ template <int KIND, typename T> struct PairStages {
     static_assert(kBytes <= kSliceStage<T>, "half of a warp's part of the shared memory");
 };
 
-// b - a; the first two components in one instruction (141 -> 134 us for 72 M terms)
+// b - a; the first two components in one instruction (142.1 -> 133.5 us for 72 M terms)
 __device__ __forceinline__ V3<float> difference(const float4 &b, const float4 &a) {
     const float2 xy = tc::sub2(make_float2(b.x, b.y), make_float2(a.x, a.y));
     return V3<float>{xy.x, xy.y, b.z - a.z};
@@ -796,7 +796,7 @@ __device__ __forceinline__ void prior_terms(const A &acc, const PriorSegments &s
 
 // All terms: blocks of slices and blocks of single terms, dealt evenly, so that every SM holds both: the slices use the issue slots that the
 // chains of double-precision operations leave.  In launches of their own the two hardly met (a launch starts when the last block of the
-// one before has, whatever the former allows): 143.5 us for the lists of 1024 chains of 268 beads, like this 141.
+// one before has, whatever the former allows): 143.5 -> 141 us for the lists of 1024 chains of 268 beads when the launches were made one.
 template <typename T, bool FIXED>
 __global__ void __launch_bounds__(kSliceWarps * 32, sizeof(T) == 4 ? kSliceBlocks : 4)
 prior_all_kernel(const __grid_constant__ PriorSegments seg, int parts, int term_blocks, const typename Vec4<T>::type *__restrict__ beads, int64_t N, int64_t B,

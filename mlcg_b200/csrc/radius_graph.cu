@@ -2488,7 +2488,7 @@ __device__ __forceinline__ int64_t structure_at(const int64_t *__restrict__ ptr,
 }
 
 // The same with its boundaries, where structures are of similar sizes in one look at the 32 boundaries around the one that the point's place
-// suggests (three latencies otherwise, 18.2 -> 17.0 us for 512 x 100 points).
+// suggests (three latencies otherwise, 18.3 -> 17.5 us for 512 x 100 points).
 __device__ __forceinline__ void structure_near(const int64_t *__restrict__ ptr, int64_t B, int64_t i, float per_point, int lane, int64_t &b, int64_t &lo,
                                                int64_t &hi) {
     const int64_t guess = (int64_t)((float)i * per_point) - 15, base = max(min(guess, B - 31), (int64_t)0);
@@ -2531,8 +2531,9 @@ rows_begin_kernel(const int64_t *__restrict__ sizes, int64_t B, int64_t N, int64
     if (threadIdx.x == 0) header[8] = any;
 }
 
-// (float32: 48 registers, as the look at 32 boundaries would take 61 and leave room for four blocks an SM: 20 structures of 1000 points, 625
-// blocks, 24.5 us instead of 21.2)
+// (float32 in 48 registers, five blocks an SM.  The look at 32 boundaries would take 61, four blocks, which is the faster by 3-10 % where the
+// blocks divide well, 512 x 100 points 16.7 : 17.5 us, and the slower by 8-30 % where a fifth block would have held them all, 20 x 1000 25.0 : 21.4,
+// 22 x 1000 27.8 : 21.3)
 template <typename T, bool ALL>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 0)
 mask_rows_kernel(const T *__restrict__ pos, const int64_t *__restrict__ ptr, int32_t *__restrict__ struct_of, const CellParam *__restrict__ cellparam,

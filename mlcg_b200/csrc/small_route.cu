@@ -10,7 +10,8 @@
 //   force pass         gagg -> aggregation + edge dot products -> lin1^T, + g -> lin^T, tanh' -> lin2^T of block l-1
 // and the two along a tangent and back that a force-matching step adds.  Weights (three 64 KB matrices) are copied to shared
 // memory while the kernel waits for its predecessor, each waited for in front of its layer (SmallTile says how a layer is split; a
-// column and 32 k per thread over tiles of 4 or 8 rows: 61.4 us an evaluation of 64 x 10 beads, like this 52).  Launches per evaluation of L blocks: 2 L + 3 where the tensor-core
+// column and 32 k per thread over tiles of 4 or 8 rows: 61.4 us an evaluation of 64 x 10 beads, with the tiles below 52, and 49 with weights by the
+// copy engine and the filters in two CTAs a tile).  Launches per evaluation of L blocks: 2 L + 3 where the tensor-core
 // sequence takes 7 L + 7; one evaluation of 64 x 10 beads, two blocks: 154 us of kernels before.
 // For many more rows per SM the tensor-core kernels are the faster ones (figures at kSmallNodes).
 #include "schnet_internal.cuh"
@@ -689,7 +690,12 @@ small_graph_fill_kernel(const float *__restrict__ pos, const SmallGraph g, int64
 
 // Forces and energies: the dot products of the first block taken here in both directions (a node's edges by WPN warps, so nothing is
 // written per edge), those of the other blocks read from s.  A latency chain: with one warp per node, four edges at a time, it took
-// 4.5-4.9 us behind the last link, most of it the later edges' turns.
+// 4.5-4.9 us behind the last link, most of it the later edges' turns.  Eight warps a node or four (small_finish()), an evaluation replayed, us:
+//   beads   73    128    146    200    250    296    300    400    560    640 (10 a chain)   1000   1400   2000
+//   8      41.1   45.1   49.2   49.2   57.4   55.2   57.1   59.1   61.6   60.1               84.0   119.3  135.4
+//   4      43.0   45.6   50.8   51.0   58.0   55.5   57.5   60.0   61.6   58.0               82.2   116.8  131.4
+// (two: 2-4 us more up to 640 beads, 129.3 at 2000.)  They meet between 300 and 640 beads, the sooner the fewer
+// edges a bead has; the line lies at two beads an SM.
 constexpr int kFinishThreads = 256;
 template <int WPN>
 __global__ void __launch_bounds__(kFinishThreads)
@@ -810,6 +816,15 @@ static int small_configure(Kern kern, size_t bytes, bool *done) {
 //   6            57        59     61     67     72     67     67      81     97    121    124    160
 //   8            62        63     65     71     78     67     69      83     77    130    135    141
 // (9 of 640 beads, 72 tiles: 73; weights of two layers held in registers for one row a tile: 46.3 against 46.2)
+// The links of a training step go by the same line.  Kernels of a step (forward and backward) of the same chains, us:
+//   beads     73    146    200    270    400    560    640    800   1000   1184   1204   1400   1700   2000   2368
+//   1 row    123    137    164    172    210    250    274    338    413    458    488    535    649    732    828
+//   2        128    142    137    142    185    193    217    247    322    335    372    384    466    511    571
+//   3        135    151    143    145    153    197    185    220    298    304    316    366    408    455    512
+//   4        143    159    149    150    159    165    192    231    269    277    322    345    379    432    452
+//   6        158    180    168    168    176    183    160    196    290    305    321    322    363    425    449
+//   8        167    195    179    178    187    192    168    206    246    253    324    352    384    384    401
+// Where the two disagree (146 to 400 beads: a row less) the line costs a step 3-5 % of its kernels, which take a third of its time there.
 static int small_rows(int64_t N) {
     constexpr int64_t kHalf = kNumSM / 2;
     if (N <= 3 * kHalf) return (int)((N + kHalf - 1) / kHalf);
