@@ -188,7 +188,7 @@ prior_kernel(const T *__restrict__ pos, const int64_t *__restrict__ mapping, con
 }
 
 // ------------------------------------------------------------------------------------------------
-// All prior classes of a model together, in three launches: a first one that widens the positions to one 16-byte (32-byte) record per
+// All prior classes of a model together, in three launches (four where single terms are the larger part beside slices): a first one that widens the positions to one 16-byte (32-byte) record per
 // bead with its structure and clears the sums, one for the slices of pair lists and all other terms, a last one that turns the
 // sums into energies and gradients (or forces) and adds up the lists.  Up to MLCGB_MAX_PRIOR_SEGMENTS lists; every list has its own
 // energy row and gradient block, so the caller still gets one energy / force set per prior, and the totals that SumOut forms
@@ -794,6 +794,19 @@ __device__ __forceinline__ void prior_terms(const A &acc, const PriorSegments &s
     }
 }
 
+// Single terms in a launch of their own, where they are the larger part or the only one: without the stages' shared memory, which is taken from
+// the cache that their beads come through.  256 chains of 268 beads, us, in prior_all_kernel's blocks : like this: every pair one way (9 M terms, not
+// sliced) float32 331 : 278, float64 421 : 289; bonds, angles and dihedrals alone, 1024 chains, 40.6 : 39.0 and 55.4 : 45.1.
+template <typename T, bool FIXED>
+__global__ void __launch_bounds__(256)
+prior_terms_kernel(const __grid_constant__ PriorSegments seg, const typename Vec4<T>::type *__restrict__ beads, int64_t N, int64_t B,
+                   typename Accum<T, FIXED>::type *__restrict__ energy, typename Accum<T, FIXED>::type *__restrict__ grad, int32_t *__restrict__ status) {
+    const Accum<T, FIXED> acc{energy, grad};
+    pdl_wait();
+    pdl_launch_dependents();
+    prior_terms<T>(acc, seg, beads, N, B, status, (int)blockIdx.x, (int)gridDim.x);
+}
+
 // All terms: blocks of slices and blocks of single terms, dealt evenly, so that every SM holds both: the slices use the issue slots that the
 // chains of double-precision operations leave.  In launches of their own the two hardly met (a launch starts when the last block of the
 // one before has, whatever the former allows): 143.5 -> 141 us for the lists of 1024 chains of 268 beads when the launches were made one.
@@ -1048,13 +1061,17 @@ extern "C" int mlcgb_prior_eval(int n_lists, const mlcgb_prior_list *lists, cons
         //   48              20.5, 23.0  26.2, 29.0  22.8, 36.9  36.2, 63.8  60.7, 111.1  32.6, 45.1  136.4, 269.5
         //   96              20.5, 23.2  28.3, 31.2  32.9, 44.9  42.7, 69.7  69.8, 116.9  39.8, 60.2  134.0, 260.1 (the only one with two parts here)
         const int64_t want = r ? (kSliceWarps * kSliceBlocks * (int64_t)kNumSM + r - 1) / r : 1;
-        int64_t stages = 1;
+        int64_t stages = 1, in_slices = 0;
         for (int i = 0; i < n_lists; i++) {
             const int64_t a_stage = seg.kind[i] == 0 ? PairStages<0, T>::kSteps : PairStages<3, T>::kSteps;
-            if (seg.n_slices[i]) stages = std::max(stages, (seg.steps[i] + seg.n_slices[i] * a_stage - 1) / (seg.n_slices[i] * a_stage));
+            if (!seg.n_slices[i]) continue;
+            in_slices += 128 * seg.steps[i];
+            stages = std::max(stages, (seg.steps[i] + seg.n_slices[i] * a_stage - 1) / (seg.n_slices[i] * a_stage));
         }
+        const bool alone = v > in_slices;                // (prior_terms_kernel; beside a larger stream they cost least among its blocks)
         const int parts = (int)std::min(std::min(std::max(want, (int64_t)2), (int64_t)16), stages), slice_blocks = r ? grid_for(r * parts, kSliceWarps, 96) : 0,
-                  term_blocks = v ? grid_for(v, kSliceWarps * 32, 96) : 0;
+                  term_blocks = v && !alone ? grid_for(v, kSliceWarps * 32, 96) : 0;
+        if (v && alone) launch_pdl(prior_terms_kernel<T, FIXED>, dim3(grid_for(v, 256, 16)), dim3(256), 0, st, seg, beads, N, B, se, sg, status);
         if (slice_blocks + term_blocks)
             launch_pdl(prior_all_kernel<T, FIXED>, dim3(slice_blocks + term_blocks), dim3(kSliceWarps * 32), 0, st, seg, parts, term_blocks, beads, N, B, se, sg, status);
         launch_pdl(prior_finish_kernel<T, A>, dim3(grid_for(B + 3 * N, 256, 8)), dim3(256), 0, st, sums, n_lists, N, B, (T)(negate ? -1 : 1), (T *)energy,

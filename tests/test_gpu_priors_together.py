@@ -91,6 +91,35 @@ def test_priors_repeat_bit_by_bit(dtype):
     assert int(differs) == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("n", [21, 60, 130])
+def test_slices_beside_more_single_terms(n, dtype):
+    """A sliced list of bonds among twenty beads of a structure, every pair both ways, and a repulsion list of every pair one way, which is not
+    sliced: with more of the single terms than of the others they have a launch of their own (n above 29), else they share one."""
+    B, gen = 5, torch.Generator().manual_seed(n)
+    every = torch.cartesian_prod(torch.arange(20), torch.arange(20)).t()
+    both, half = every[:, every[0] != every[1]], torch.combinations(torch.arange(n)).t()
+    priors = {"bonds": bnn.HarmonicBonds({(0, 0): {"k": 0.3, "x_0": 9.0}}), "repulsion": bnn.Repulsion({(0, 0): {"sigma": 3.5}})}
+    lists, owner = {}, {}
+    for k, m in (("bonds", both), ("repulsion", half)):
+        owner[k] = torch.arange(B).repeat_interleave(m.shape[1])
+        lists[k] = mlcg_b200.make_neighbor_list(k, 2, torch.cat([m + b * n for b in range(B)], dim=1), owner[k])
+    data = mlcg_b200.AtomicData(pos=torch.cat([random_walk_chain(n, gen, min_dist=3.0) for _ in range(B)]).to(dtype), atom_types=torch.zeros(n * B, dtype=torch.long),
+                                batch=torch.arange(B).repeat_interleave(n), n_atoms=torch.full((B,), n), neighbor_list=lists).to(DEV)
+    priors = {k: p.to(DEV).eval() for k, p in priors.items()}
+    assert priors["bonds"]._cached_list(data)[4] is not None and priors["repulsion"]._cached_list(data)[4] is None
+    each = _evaluate_together(list(priors.values()), data, forces=True)[0]
+    again = _evaluate_together(list(priors.values()), data, forces=True)[0]
+    pos, tol = data.pos.double().requires_grad_(True), 1e-5 if dtype == torch.float32 else 1e-9          # (as above)
+    for k, p in priors.items():
+        y = p._energy_terms(pos, lists[k]["index_mapping"].to(DEV), p._params(data).double())
+        want = torch.zeros(B, dtype=torch.float64, device=DEV).index_add_(0, owner[k].to(DEV), y)
+        f = -torch.autograd.grad(want.sum(), pos)[0]
+        assert torch.allclose(each[k][0].double(), want.detach(), rtol=tol, atol=tol), k
+        assert float((each[k][1].double() - f).abs().max()) <= tol * (1 + float(f.abs().max())), k
+        assert torch.equal(each[k][0], again[k][0]) and torch.equal(each[k][1], again[k][1]), k
+
+
 def test_a_sliced_list_is_kept_once():
     """The slices of a pair list take the place of the 32-bit list and of the gathered parameters: 6 bytes a term and the padding."""
     data, priors = prior_setup(150, 20, 4, torch.Generator().manual_seed(3))
