@@ -252,6 +252,47 @@ def test_weights_at_any_address(sizes, shift, table):
         assert float((a - b).abs().max()) <= 4e-5 * float(b.abs().max()) + 1e-9
 
 
+@pytest.mark.parametrize("moved", ["forward", "backward"])
+def test_a_step_whose_weights_change_place(moved):
+    """Saved-tensor hooks that bring the weights back on other boundaries than the forward pass met: one pass by the chain of small batches, the
+    other by the kernels of larger ones, over one workspace."""
+    torch.manual_seed(3)
+    cut = bnn.CosineCutoff(0.0, 8.0)
+    net = bnn.StandardSchNet(bnn.ExpNormalBasis(cut, 33, trainable=False), cut, [64], embedding_size=5, num_interactions=3).to(DEV).train()
+    model, gen = bnn.GradientsOut(net, "forces"), torch.Generator().manual_seed(1)
+    pos, batch = torch.cat([random_walk_chain(60, gen, min_dist=3.0) for _ in range(4)]).to(DEV), torch.arange(4, device=DEV).repeat_interleave(60)
+    weights = [p for name, p in net.named_parameters() if "embedding" not in name]
+
+    def elsewhere(t, k):
+        return torch.cat([t.new_zeros(k), t.detach().flatten()])[k:].view(t.shape)
+
+    def step(pack, unpack):
+        net.zero_grad()
+        with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+            out = model(mlcg_b200.AtomicData(pos=pos, atom_types=torch.arange(240, device=DEV) % 5, batch=batch, n_atoms=torch.full((4,), 60, device=DEV))).out["SchNet"]
+            ((out["forces"] ** 2).mean() + 0.01 * (out["energy"] ** 2).mean()).backward()
+        assert type(out["forces"].grad_fn).__name__ == "SchNetForceMatchingBackward"
+        return [p.grad.clone() for p in net.parameters()]
+
+    want = step(lambda t: t, lambda t: t)
+    if moved == "forward":
+        for p in weights:
+            p.data = elsewhere(p.data, 1)
+    k, seen = int(moved == "backward"), []
+
+    def back(t):
+        if t.dtype == torch.float32 and any(t.shape == p.shape for p in weights):
+            seen.append(t.shape)
+            return elsewhere(t, k)
+        return t
+
+    got = step(lambda t: t, back)
+    assert len(seen) >= len(weights)
+    for a, b in zip(got, want):
+        assert float((a - b).abs().max()) <= 4e-5 * float(b.abs().max()) + 1e-9      # (either side within 2e-5, as above)
+    get_backend().check_pending()
+
+
 @pytest.mark.parametrize("blocks", [1, 2])
 def test_large_batches_with_nodes_of_every_degree(blocks):
     """Above the small batches' limit the last dot products are taken per pair: beads without neighbours, with one, and with several
